@@ -10,10 +10,13 @@
 // 512 TMEM columns with 16 tcgen05.mma M=64 N=256 K=16; 16 warps drain TMEM into whole 256-byte
 // row pieces of q_abs.
 //
-// Append blocks (present when the caller fuses the two steps): four new rows per block, the
-// bit-exact RMSNorm + RoPE + scatter of append_kernel (mla_kernels.cu), 128 threads per row.  They
-// share the launch because the append is a chain of dependent float additions that takes as long
-// as the absorb itself and needs only a handful of SMs.
+// Append blocks (present when the caller fuses the two steps): sixteen new rows per block, one warp
+// each, the bit-exact RMSNorm + RoPE + scatter of append_kernel (mla_kernels.cu).  They share the
+// launch because the append is a chain of dependent float additions that takes as long as the absorb
+// itself and needs only a handful of SMs.
+//
+// One launch serves `layers` consecutive layers of a step whose inputs are all at hand: with one row
+// per layer (16 heads, 27 layers) a launch per layer is 16 blocks on 148 SMs.
 #include "mla_launch.h"
 #include "mla_tc5.cuh"
 
@@ -36,15 +39,15 @@ constexpr int M_FAIL = 20;
 constexpr int MISC_BYTES = 64;
 constexpr int SMEM_BYTES = OFF_MISC + MISC_BYTES + 1024;   // + slack to round the base up to 1 KB
 constexpr int NUM_THREADS = 512;
-constexpr int APPEND_ROWS = NUM_THREADS / 128;  // rows per append block
+constexpr int APPEND_ROWS = NUM_THREADS / 32;   // rows per append block
 constexpr uint32_t TMEM_COLS = 512;
 
 
 struct AppendArgs {          // rows == 0: no append blocks in this launch
-    const void* kv_a;
-    void* pool;              // this layer's slice of the cache pool
-    uint64_t pool_slots;
-    const void* norm_w;
+    const void* kv_a;        // [layers][rows][576]
+    void* pool;              // the first layer's slice of the cache pool
+    uint64_t pool_slots;     // token slots per layer
+    const void* norm_w;      // [layers][512]
     const float* cos_sin;
     uint32_t cs_rows;
     float eps;
@@ -54,92 +57,79 @@ struct AppendArgs {          // rows == 0: no append blocks in this launch
     uint32_t wait_first;     // kv_a may be the output of the kernel just before this one in the stream
 };
 
-// One new cache row per 128 threads; every statement mirrors append_kernel (mla_kernels.cu), which
-// documents the reference's rounding sequence.  All threads of the block reach every barrier.
+// One new cache row per warp; every statement mirrors append_kernel (mla_kernels.cu), which documents the reference's
+// rounding sequence.  The row is normalised and rotated in place: every element (pair) has one lane.
+constexpr int APPEND_SMEM = APPEND_ROWS * (kRow * 2 + kRank * 4);
+static_assert(APPEND_SMEM <= SMEM_BYTES, "the append blocks live in the absorb blocks' shared memory");
 template <typename T>
-__device__ __forceinline__ void append_rows(const AppendArgs& a, uint32_t first_row, uint32_t* status)
+__device__ __forceinline__ void append_rows(const AppendArgs& a, uint32_t layer, uint32_t first_row, unsigned char* smem, uint32_t* status)
 {
-    __shared__ __align__(16) T xin[APPEND_ROWS][kRow];
-    __shared__ __align__(16) T xout[APPEND_ROWS][kRow];
-    __shared__ float sq[APPEND_ROWS][kRank];
-    __shared__ float rinv_s[APPEND_ROWS];
-    const uint32_t g = threadIdx.x / 128, tid = threadIdx.x % 128, r = first_row + g;
-    const T* kv_a = static_cast<const T*>(a.kv_a);
-    const T* norm_w = static_cast<const T*>(a.norm_w);
-    T* pool = static_cast<T*>(a.pool);
-    bool live = r < a.rows;
-    uint64_t slot = 0;
-    uint32_t pos = 0;
-    if (live) {
-        slot = a.row_slot[r];
-        pos = a.row_pos[r];
-        if (slot == ~uint64_t(0)) live = false;          // a query-only row: nothing to append
-        else if (slot >= a.pool_slots || pos >= a.cs_rows) {
-            if (tid == 0) atomicOr(status, ST_BAD_SLOT);
-            live = false;
-        }
+    const uint32_t g = threadIdx.x / 32, lane = threadIdx.x % 32, r = first_row + g;
+    float* sq = reinterpret_cast<float*>(smem) + g * kRank;
+    T* x = reinterpret_cast<T*>(smem + APPEND_ROWS * kRank * 4) + g * kRow;
+    if (r >= a.rows) return;
+    const uint64_t slot = a.row_slot[r];
+    const uint32_t pos = a.row_pos[r];
+    if (slot == ~uint64_t(0)) return;                    // a query-only row: nothing to append
+    if (slot >= a.pool_slots || pos >= a.cs_rows) {
+        if (lane == 0) atomicOr(status, ST_BAD_SLOT);
+        return;
     }
     constexpr int kChunks = kRow * 2 / 16;   // 72 x 16 bytes
-    // Every global load of the row is issued here, before the first barrier: the row itself, the rotation's cos/sin
-    // and this thread's four norm weights.  Left where they are used they would form a chain of three dependent
-    // round trips to memory (~1 us each) in a kernel whose whole budget is a few microseconds.
-    uint4 row_chunk = make_uint4(0, 0, 0, 0);
-    float cs = 0.0f, sn = 0.0f, nw[kRank / 128];
+    // Every global load of the row is issued here: the row itself, the rotation's cos/sin and this lane's norm weights.
+    // Left where they are used they would form a chain of three dependent round trips to memory (~1 us each) in a kernel
+    // whose whole budget is a few microseconds.
+    const uint4* src = reinterpret_cast<const uint4*>(static_cast<const T*>(a.kv_a) + (size_t(layer) * a.rows + r) * kRow);
+    const T* norm_w = static_cast<const T*>(a.norm_w) + size_t(layer) * kRank;
+    uint4 row_chunk[3];
+    float nw[kRank / 32];
 #pragma unroll
-    for (int k = 0; k < kRank / 128; k++) nw[k] = 0.0f;
-    if (live) {
-        if (tid < kChunks) row_chunk = reinterpret_cast<const uint4*>(kv_a + size_t(r) * kRow)[tid];
-        if (tid >= 32 && tid < 64) {
-            cs = a.cos_sin[size_t(pos) * kRope + (tid - 32)];
-            sn = a.cos_sin[size_t(pos) * kRope + 32 + (tid - 32)];
-        }
+    for (int k = 0; k < 3; k++) if (lane + 32 * k < uint32_t(kChunks)) row_chunk[k] = src[lane + 32 * k];
+    const float cs = a.cos_sin[size_t(pos) * kRope + lane], sn = a.cos_sin[size_t(pos) * kRope + 32 + lane];
 #pragma unroll
-        for (int k = 0; k < kRank / 128; k++) nw[k] = Elem<T>::to_f32(norm_w[tid + 128 * k]);
+    for (int k = 0; k < kRank / 32; k++) nw[k] = Elem<T>::to_f32(norm_w[lane + 32 * k]);
+#pragma unroll
+    for (int k = 0; k < 3; k++) if (lane + 32 * k < uint32_t(kChunks)) reinterpret_cast<uint4*>(x)[lane + 32 * k] = row_chunk[k];
+    __syncwarp();
+    float v[kRank / 32];
+#pragma unroll
+    for (int k = 0; k < kRank / 32; k++) {
+        v[k] = Elem<T>::to_f32(x[lane + 32 * k]);
+        sq[lane + 32 * k] = __fmul_rn(v[k], v[k]);
     }
-    if (live && tid < kChunks) reinterpret_cast<uint4*>(xin[g])[tid] = row_chunk;
-    __syncthreads();
-    if (live) {
-        for (int i = tid; i < kRank; i += 128) {
-            const float v = Elem<T>::to_f32(xin[g][i]);
-            sq[g][i] = __fmul_rn(v, v);
-        }
-        if (tid >= 32 && tid < 64) {
-            const int i = tid - 32;
-            const float x0 = Elem<T>::to_f32(xin[g][kRank + i]);
-            const float x1 = Elem<T>::to_f32(xin[g][kRank + 32 + i]);
-            xout[g][kRank + i]      = Elem<T>::from_f32(__fsub_rn(__fmul_rn(x0, cs), __fmul_rn(x1, sn)));
-            xout[g][kRank + 32 + i] = Elem<T>::from_f32(__fadd_rn(__fmul_rn(x1, cs), __fmul_rn(x0, sn)));
-        }
+    {
+        const float x0 = Elem<T>::to_f32(x[kRank + lane]), x1 = Elem<T>::to_f32(x[kRank + 32 + lane]);
+        x[kRank + lane]      = Elem<T>::from_f32(__fsub_rn(__fmul_rn(x0, cs), __fmul_rn(x1, sn)));
+        x[kRank + 32 + lane] = Elem<T>::from_f32(__fadd_rn(__fmul_rn(x1, cs), __fmul_rn(x0, sn)));
     }
-    __syncthreads();
-    if (live && tid == 0) {
+    __syncwarp();
+    float rinv = 0.0f;
+    if (lane == 0) {
         float ss = 0.0f;
-#pragma unroll 16
-        for (int i = 0; i < kRank; i++) ss = __fadd_rn(ss, sq[g][i]);
-        rinv_s[g] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, float(kRank)), a.eps)));
-    }
-    __syncthreads();
-    if (live) {
-        const float rinv = rinv_s[g];
-#pragma unroll
-        for (int k = 0; k < kRank / 128; k++) {
-            const int i = tid + 128 * k;
-            const float v = __fmul_rn(Elem<T>::to_f32(xin[g][i]), rinv);
-            xout[g][i] = Elem<T>::from_f32(__fmul_rn(v, nw[k]));
+#pragma unroll 4
+        for (int i = 0; i < kRank; i += 4) {
+            const float4 s4 = *reinterpret_cast<const float4*>(sq + i);
+            ss = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(ss, s4.x), s4.y), s4.z), s4.w);
         }
+        rinv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, float(kRank)), a.eps)));
     }
-    __syncthreads();
-    if (live && tid < kChunks)
-        reinterpret_cast<uint4*>(pool + slot * kRow)[tid] = reinterpret_cast<const uint4*>(xout[g])[tid];
+    rinv = __shfl_sync(0xffffffffu, rinv, 0);
+#pragma unroll
+    for (int k = 0; k < kRank / 32; k++) x[lane + 32 * k] = Elem<T>::from_f32(__fmul_rn(__fmul_rn(v[k], rinv), nw[k]));
+    __syncwarp();
+    uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(a.pool) + (size_t(layer) * a.pool_slots + slot) * kRow);
+#pragma unroll
+    for (int k = 0; k < 3; k++) if (lane + 32 * k < uint32_t(kChunks)) dst[lane + 32 * k] = reinterpret_cast<const uint4*>(x)[lane + 32 * k];
 }
 
 template <typename T>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict__ q, T* __restrict__ q_abs, uint32_t rows,
-                  uint32_t H, uint32_t absorb_blocks, const AppendArgs app, const float* __restrict__ q_cos_sin,
+                  uint32_t H, uint32_t layer0, uint32_t absorb_blocks, const AppendArgs app, const float* __restrict__ q_cos_sin,
                   const uint32_t* __restrict__ q_pos, const uint32_t* __restrict__ att_row, uint32_t cs_rows,
                   uint32_t* __restrict__ status)
 {
+    extern __shared__ unsigned char absorb_tc5_smem[];
     grid_launch_dependents();
     if (blockIdx.x >= absorb_blocks) {
         // Apart from kv_a the append touches nothing that an earlier kernel of the stream still reads or writes:
@@ -149,11 +139,11 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
         // handed over with the first layer's), the append works first and waits last; the wait then only keeps "this
         // kernel completes after its predecessors", which the kernels behind it rely on.
         if (app.wait_first) grid_dependency_wait();
-        append_rows<T>(app, (blockIdx.x - absorb_blocks) * APPEND_ROWS, status);
+        const uint32_t per_layer = (app.rows + APPEND_ROWS - 1) / APPEND_ROWS, b = blockIdx.x - absorb_blocks;
+        append_rows<T>(app, b / per_layer, (b % per_layer) * APPEND_ROWS, absorb_tc5_smem, status);
         if (!app.wait_first) grid_dependency_wait();
         return;
     }
-    extern __shared__ unsigned char absorb_tc5_smem[];
     const uint32_t raw = smem_u32(absorb_tc5_smem);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char* sm = absorb_tc5_smem + (base - raw);
@@ -162,7 +152,11 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + OFF_MISC + M_TMEM);
     volatile int* fail_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + M_FAIL);
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-    const uint32_t h = blockIdx.x % H, r0 = (blockIdx.x / H) * MT;
+    // head fastest, then row tile, then layer; virtual row layer * rows + r indexes q_abs (and q, unless att_row renames it)
+    const uint32_t row_tiles = (rows + MT - 1) / MT, rest = blockIdx.x / H;
+    const uint32_t h = blockIdx.x % H, r0 = (rest % row_tiles) * MT, li = rest / row_tiles;
+    q += size_t(li) * rows * H * kQDim;
+    q_abs += size_t(li) * rows * H * kRow;
 
     if (tid == 0) {
         *fail_flag = 0;
@@ -173,7 +167,7 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
         mbar_expect_tx(bar_w, W_BYTES);                      // W_UK_h^T: four boxes of 64 i x 256 d
 #pragma unroll 1
         for (int bx = 0; bx < 4; bx++)
-            tma_load_2d(sW + (bx / 2) * W_SUB + (bx % 2) * (W_SUB / 2), &map_w, bar_w, 64 * (bx / 2), int(h) * kRank + 256 * (bx % 2));
+            tma_load_2d(sW + (bx / 2) * W_SUB + (bx % 2) * (W_SUB / 2), &map_w, bar_w, 64 * (bx / 2), int((layer0 + li) * H + h) * kRank + 256 * (bx % 2));
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
@@ -291,27 +285,28 @@ int absorb_tc5_configure()
     return int(e);
 }
 
-// w_map: host CUtensorMap over this layer's W_UK^T ([H*512 d][128 i], box 64 i x 256 d, 128-byte swizzle).
-// With kv_a != nullptr the launch also appends the step's new rows to the layer's cache pool.  With rotate_q the
-// last 64 dims of every query head are rotated with the row's position (m.row_pos) before they are stored.
-int launch_absorb_tc5(int dtype, const void* q, const void* w_map, void* q_abs, uint32_t rows, uint32_t H, const void* kv_a,
+// w_map: host CUtensorMap over W_UK^T of all layers ([layers*H*512 d][128 i], box 64 i x 256 d, 128-byte swizzle).  q, q_abs
+// and (with kv_a != nullptr: the launch also appends) kv_a hold m.layers consecutive layers from layer0; layer_pool and
+// norm_w point at layer0's slices.  With rotate_q the last 64 dims of every query head are rotated with the row's
+// position (m.row_pos) before they are stored.
+int launch_absorb_tc5(int dtype, const void* q, const void* w_map, void* q_abs, uint32_t H, uint32_t layer0, const void* kv_a,
                       void* layer_pool, uint64_t pool_slots, const void* norm_w, const float* cos_sin, uint32_t cs_rows,
                       float eps, const StepMeta& m, bool rotate_q, bool append_waits, uint32_t* status, cudaStream_t st)
 {
-    if (rows == 0) return 0;
+    if (m.rows == 0) return 0;
     const CUtensorMap* map = static_cast<const CUtensorMap*>(w_map);
     AppendArgs app{};
     if (kv_a) app = AppendArgs{kv_a, layer_pool, pool_slots, norm_w, cos_sin, cs_rows, eps, m.app_pos, m.app_slot, m.app_rows, append_waits ? 1u : 0u};
-    const uint32_t absorb_blocks = H * ((rows + MT - 1) / MT);
-    const uint32_t append_blocks = (app.rows + APPEND_ROWS - 1) / APPEND_ROWS;
-    // append blocks carry the trailing indices; for decode batches all blocks are resident at once (H + rows/4 <= SMs)
+    const uint32_t absorb_blocks = m.layers * H * ((m.rows + MT - 1) / MT);
+    const uint32_t append_blocks = m.layers * ((app.rows + APPEND_ROWS - 1) / APPEND_ROWS);
+    // append blocks carry the trailing indices
     dim3 grid(absorb_blocks + append_blocks);
-    if (dtype == 0)
-        return int(launch_pdl(absorb_tc5_kernel<__half>, grid, dim3(NUM_THREADS), SMEM_BYTES, st, *map, static_cast<const __half*>(q),
-                              static_cast<__half*>(q_abs), rows, H, absorb_blocks, app, rotate_q ? cos_sin : nullptr, m.row_pos, m.att_row, cs_rows, status));
-    return int(launch_pdl(absorb_tc5_kernel<__nv_bfloat16>, grid, dim3(NUM_THREADS), SMEM_BYTES, st, *map,
-                          static_cast<const __nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(q_abs), rows, H, absorb_blocks, app,
-                          rotate_q ? cos_sin : nullptr, m.row_pos, m.att_row, cs_rows, status));
+    auto go = [&](auto kernel, auto* qp, auto* qa) {
+        return int(launch_pdl(kernel, grid, dim3(NUM_THREADS), SMEM_BYTES, st, *map, qp, qa, m.rows, H, layer0, absorb_blocks, app,
+                              rotate_q ? cos_sin : nullptr, m.row_pos, m.att_row, cs_rows, status));
+    };
+    if (dtype == 0) return go(absorb_tc5_kernel<__half>, static_cast<const __half*>(q), static_cast<__half*>(q_abs));
+    return go(absorb_tc5_kernel<__nv_bfloat16>, static_cast<const __nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(q_abs));
 }
 
 }  // namespace mla

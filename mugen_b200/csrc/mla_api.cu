@@ -23,20 +23,25 @@ namespace {
 
 thread_local std::string g_create_error;
 
-constexpr int kMetaRing = 4;
+constexpr int kMetaRing = 8;
 
-struct LayerW {
-    void* w_uk = nullptr;   // stored transposed per head: [h][512][128]
-    void* w_uk_rows = nullptr;   // as registered, (H*128) x 512: the prefill path expands keys with it
-    void* w_uv = nullptr;
-    void* norm = nullptr;
-    bool set = false;
-    // W_UV as ([H*128 outputs][512 dims]) with a box of 64 dims x 128 outputs, for the tcgen05 merge kernel
-    alignas(64) CUtensorMap w_uv_map;
-    // W_UK^T as ([H*512 d][128 i]) with a box of 64 i x 256 d, for the tcgen05 absorb kernel
-    alignas(64) CUtensorMap w_uk_map;
-    bool has_map = false;
+// a step row: one new token (or the query-only row of a sequence that takes none)
+struct RowSpec {
+    uint32_t seq_index;   // index into the step's sequence list
+    uint32_t attend_len;  // rows attended (0 allowed)
+    uint32_t pos;         // global position of the appended token
+    uint64_t slot;        // destination slot (all ones: nothing to append)
 };
+
+// Device metadata and kernel choice for a series of launches (see build_plan).
+struct Plan {
+    mla::StepMeta m{};
+    uint32_t kernel = 0;
+    uint32_t min_pages = 0, max_pages = 0;     // of any persistent worker
+    bool ready = false;
+};
+// the plans of a step live side by side in the device metadata buffer
+enum { kPlanStep = 0, kPlanRest, kPlanStack, kPlanStackTail, kPlanRegions };
 
 // projection weights of one layer's attention block (mla_set_block_weights), all in the storage type on the device
 struct BlockW {
@@ -46,7 +51,7 @@ struct BlockW {
 };
 
 struct MetaBuf {
-    void* host = nullptr;       // pinned
+    char* host = nullptr;       // pinned
     cudaEvent_t done = nullptr;
     bool in_flight = false;
 };
@@ -63,7 +68,13 @@ struct mla_ctx {
 
     char* pool = nullptr;           // [layers][n_pages*64][576] elements
     uint64_t pool_slots = 0;        // token slots per layer
-    std::vector<LayerW> layers;
+    // weights of all layers side by side, so that one tensor map (and one launch) reaches any run of layers
+    char* w_uk = nullptr;            // [layers][H][512][128]: W_UK transposed per head
+    char* w_uk_rows = nullptr;       // [layers][H*128][512]: as registered, the prefill path expands keys with it
+    char* w_uv = nullptr;            // [layers][H*128][512]
+    char* norm = nullptr;            // [layers][512]
+    std::vector<char> layer_set;     // weights registered
+    alignas(64) CUtensorMap w_uk_map, w_uv_map;
     std::vector<BlockW> blocks;
     // workspaces of the block projections, grown on demand: normalised hidden state, q_a, float K-slice partials,
     // and the block's q / kv_a / attention output when the library owns them (mla_step_block)
@@ -74,10 +85,10 @@ struct mla_ctx {
     uint32_t cs_rows = 0;           // positions filled so far
     uint32_t cs_cap = 0;
 
-    void* q_abs = nullptr;          // [max_rows][H][576]
-    float* recs = nullptr;          // [max_segs][H][514]
-    uint32_t max_segs = 0;
-    uint32_t workers = 1;
+    void* q_abs = nullptr;          // [ws_rows][H][576]
+    float* recs = nullptr;          // [rec_cap][514]
+    uint32_t ws_rows = 0;           // query rows a launch series may hold: max_rows, or a group of layers of fewer rows
+    size_t rec_cap = 0;
     uint32_t* status_dev = nullptr;
     // tensor maps of the tcgen05 attention kernels (make_tensor_maps; indices mla::kMap*)
     alignas(64) CUtensorMap tmaps[mla::kMapCount];
@@ -86,15 +97,17 @@ struct mla_ctx {
     MetaBuf ring[kMetaRing];
     int ring_next = 0;
     size_t meta_cap = 0;
-    char* meta_dev = nullptr;
-    mla::StepMeta meta{};
-    // A step that holds prefill chunks (sequences taking >= kPrefillMin new tokens) has a second plan: its query rows
-    // are the step's OTHER rows, the chunks go through the expanded-form prefill kernels (run_layer).  The explicit
-    // per-layer calls (mla_step_append / _attend / _attend_partial) keep using the first plan, in which every new token
-    // is a decode-style query row.
-    mla::StepMeta meta_b{};
-    bool has_plan_b = false;
-    struct Chunk { uint32_t seq_id, q_row0, n_new, start, base_pos; };
+    char* meta_dev = nullptr;       // [kPlanRegions][meta_cap]
+    char* meta_host = nullptr;      // [kMetaRing][meta_cap], page-locked
+    // Plans of the open step, made and uploaded by the first call that needs them.  `plan`: every new token is a decode-style
+    // query row, one layer at a time.  A step that holds prefill chunks (sequences taking >= kPrefillMin new tokens) also
+    // has `plan_rest`: its query rows are the step's OTHER rows, the chunks go through the expanded-form prefill kernels
+    // (run_layer); the explicit per-layer calls (mla_step_append / _attend / _attend_partial) keep using the first.
+    // `stack` / `stack_tail`: groups of layers of one mla_step_layers call.
+    Plan plan, plan_rest, stack, stack_tail;
+    bool has_chunks = false;
+    std::vector<RowSpec> rows;       // of the open step
+    struct Chunk { uint32_t tbl_off, q_row0, n_new, start, base_pos; };   // tbl_off: of its block table in the upload
     std::vector<Chunk> chunks;
     uint32_t step_rows = 0;          // rows of the step in the caller's q / kv_a / out tensors
     // prefill workspaces, grown on demand: gathered latent rows, expanded keys and values, rotated chunk queries
@@ -107,7 +120,7 @@ struct mla_ctx {
 
     // step state
     bool in_step = false;
-    std::vector<uint32_t> step_seqs, step_nnew, step_tbl_off;
+    std::vector<uint32_t> step_seqs, step_nnew;
 
     // optional per-launch timing of the attention kernel
     bool q_rope_in_kernel = false;  // queries arrive before their RoPE (mla_set_q_rope)
@@ -153,6 +166,11 @@ int pt_code(mla_ctx* c, int e)
 }
 
 size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
+
+// Sequences that take at least this many new tokens in a step go through the prefill kernels.
+constexpr uint32_t kPrefillMin = 64;
+// Most query rows and bytes of absorbed queries of a group of layers (step_layers_grouped).
+constexpr uint64_t kGroupRows = 1024, kGroupBytes = 48ull << 20;
 
 inline float half_bits_to_f32(uint16_t h) { return __half2float(__ushort_as_half(h)); }
 inline uint16_t f32_to_half_bits(float f) { return __half_as_ushort(__float2half_rn(f)); }
@@ -226,62 +244,92 @@ int ensure_rope_rows(mla_ctx* c, uint32_t upto, cudaStream_t st)
     return MLA_OK;
 }
 
-struct RowSpec {
-    uint32_t seq_index;   // index into the step's sequence list
-    uint32_t attend_len;  // rows attended (0 allowed)
-    uint32_t pos;         // global position of the appended token (append only)
-    uint64_t slot;        // destination slot (append only)
-};
-
-// Packs the step metadata, uploads it through the pinned ring and points c->meta (plan_b: c->meta_b) at it.
-// att_row: for each query row its row in the caller's tensors (plan_b only).
-int upload_meta(mla_ctx* c, const std::vector<uint32_t>& seq_ids, const std::vector<RowSpec>& rows,
-                bool with_segments, cudaStream_t st, bool plan_b = false, const std::vector<uint32_t>* att_row = nullptr)
+uint32_t workers_of(const mla_ctx* c, uint32_t kernel, uint32_t heads)
 {
-    const uint32_t R = uint32_t(rows.size()), S = uint32_t(seq_ids.size());
-    std::vector<uint32_t> lens(R);
-    for (uint32_t r = 0; r < R; r++) lens[r] = rows[r].attend_len;
-    std::vector<Segment> segs;
-    std::vector<uint32_t> row_seg_begin, cta_seg_begin;
-    if (with_segments) {
-        if (c->kernel == MLA_KERNEL_TCGEN05_PAIR128)
-            // a worker pays about five tiles' time per segment it starts (queries, pipeline fill, state drain: ~10 us)
-            mugen::mla::plan_min_makespan(lens, mla::kPage, c->workers, segs, row_seg_begin, cta_seg_begin, 2u, 5u);
-        else
-            mugen::mla::plan_balanced(lens, mla::kPage, c->workers, segs, row_seg_begin, cta_seg_begin, 1u);
-        if (segs.size() > c->max_segs)
-            return fail(c, MLA_ERR_CAPACITY, "step needs " + std::to_string(segs.size()) +
-                                                 " KV segments, workspace holds " + std::to_string(c->max_segs));
-    } else {
-        row_seg_begin.assign(R + 1, 0);
-        cta_seg_begin.assign(1, 0);
-    }
-    const uint32_t G = uint32_t(segs.size()), W = uint32_t(cta_seg_begin.size()) - 1;
-    if (with_segments) {
-        c->plan_workers = W;
-        c->plan_min_pages = ~0u;
-        c->plan_max_pages = 0;
-        for (uint32_t w = 0; w < W; w++) {
-            uint32_t pages = 0;
-            for (uint32_t g = cta_seg_begin[w]; g < cta_seg_begin[w + 1]; g++) pages += segs[g].page_end - segs[g].page_begin;
-            c->plan_min_pages = std::min(c->plan_min_pages, pages);
-            c->plan_max_pages = std::max(c->plan_max_pages, pages);
-        }
-        if (W == 0) c->plan_min_pages = 0;
-    }
+    if (kernel == MLA_KERNEL_TCGEN05_PAIR128) return std::max<uint32_t>(1, (c->sm_count / 2) / ((heads + 127) / 128));
+    if (kernel == MLA_KERNEL_TCGEN05) return std::max<uint32_t>(1, c->sm_count / ((heads + 63) / 64));
+    if (kernel == MLA_KERNEL_TCGEN05_T16) return std::max<uint32_t>(1, c->sm_count / ((heads + 15) / 16));
+    return std::max<uint32_t>(1, c->sm_count * 2 / ((heads + 15) / 16));
+}
+
+// The attention kernel for `heads` head rows over one stream of the cache.  128 rows go to the SM-pair kernel; up to 16
+// take the transposed tcgen05 form (tokens as rows, the heads as 16 columns); everything between fills (part of) the
+// 64-row tiles of the single-block kernel, which streams the cache once per 64 heads (measured at 32 heads, 64 sequences x
+// 8192 tokens: 128 us against 186 us for two passes of the 16-column form and 300 us for mma.sync).
+uint32_t kernel_for(const mla_ctx* c, uint32_t heads)
+{
+    if (c->cfg.kernel != MLA_KERNEL_AUTO) return c->cfg.kernel;
+    return (heads % 128 == 0 && c->sm_count % 2 == 0) ? uint32_t(MLA_KERNEL_TCGEN05_PAIR128)
+         : heads > 16 ? uint32_t(MLA_KERNEL_TCGEN05) : uint32_t(MLA_KERNEL_TCGEN05_T16);
+}
+
+size_t meta_capacity(const mla_ctx* c)
+{
+    const size_t R = c->cfg.max_rows, V = c->ws_rows, W = size_t(c->sm_count) * 2;
+    const size_t max_pages_per_seq = (size_t(c->cfg.max_seq_len) + mla::kPage - 1) / mla::kPage;
+    const size_t tbl_entries = std::min<size_t>(size_t(c->cfg.max_seqs) * max_pages_per_seq, c->cfg.n_pages) + 4;
+    return align16(R * 8) + 3 * align16(R * 4) + align16(tbl_entries * 4) + align16((W + V) * sizeof(mla::SegDesc)) +
+           align16(V * sizeof(mla::RowParts)) + align16((W + 1) * 4) + 256;
+}
+
+// Plans `layers` identical layers of query rows over the persistent attention workers, packs the metadata of the launch
+// series (new rows to append, query rows, block tables, segments) and uploads it through the page-locked ring into region
+// `region` of the device buffer, behind earlier work of `st`.
+//   app      the step's new rows, in the caller's row order (what the append writes)
+//   query    the query rows; nullptr: app.  att_row: their rows in the caller's tensors (with query only)
+//   layers   0: no attention (append or row copy only)
+int build_plan(mla_ctx* c, Plan& plan, int region, const std::vector<uint32_t>& seq_ids, const std::vector<RowSpec>& app,
+               const std::vector<RowSpec>* query, const std::vector<uint32_t>* att_row, uint32_t layers, cudaStream_t st)
+{
+    const std::vector<RowSpec>& rows = query ? *query : app;
+    const uint32_t A = uint32_t(app.size()), R = layers ? uint32_t(rows.size()) : 0, S = uint32_t(seq_ids.size()), H = c->cfg.n_heads;
+    plan = Plan{};
+    if (uint64_t(R) * layers > c->ws_rows)
+        return fail(c, MLA_ERR_CAPACITY, "step needs " + std::to_string(uint64_t(R) * layers) + " query rows, the workspace holds " +
+                                             std::to_string(c->ws_rows));
+    // block tables, sequence after sequence
     size_t tbl_total = 0;
     std::vector<uint32_t> tbl_off(S);
     for (uint32_t i = 0; i < S; i++) {
         tbl_off[i] = uint32_t(tbl_total);
         tbl_total += c->pt->seq(seq_ids[i])->pages.size();
     }
+    std::vector<Segment> segs;
+    std::vector<uint32_t> row_seg_begin{0}, cta_seg_begin{0};
+    plan.kernel = kernel_for(c, H);
+    if (R) {
+        std::vector<uint32_t> lens(size_t(R) * layers);
+        for (uint32_t r = 0; r < R; r++) lens[r] = rows[r].attend_len;
+        for (uint32_t l = 1; l < layers; l++) std::copy(lens.begin(), lens.begin() + R, lens.begin() + size_t(l) * R);
+        const uint32_t workers = workers_of(c, plan.kernel, H);
+        if (plan.kernel == MLA_KERNEL_TCGEN05_PAIR128)
+            // a worker pays about five tiles' time per segment it starts (queries, pipeline fill, state drain: ~10 us)
+            mugen::mla::plan_min_makespan(lens, mla::kPage, workers, segs, row_seg_begin, cta_seg_begin, 2u, 5u);
+        else
+            mugen::mla::plan_balanced(lens, mla::kPage, workers, segs, row_seg_begin, cta_seg_begin, 1u);
+        if (segs.size() * H > c->rec_cap)
+            return fail(c, MLA_ERR_CAPACITY, "step needs " + std::to_string(segs.size()) + " KV segments, more than the workspace holds");
+    }
+    const uint32_t G = uint32_t(segs.size()), W = uint32_t(cta_seg_begin.size()) - 1;
+    if (R) {
+        plan.min_pages = W ? ~0u : 0u;
+        for (uint32_t w = 0; w < W; w++) {
+            uint32_t pages = 0;
+            for (uint32_t g = cta_seg_begin[w]; g < cta_seg_begin[w + 1]; g++) pages += segs[g].page_end - segs[g].page_begin;
+            plan.min_pages = std::min(plan.min_pages, pages);
+            plan.max_pages = std::max(plan.max_pages, pages);
+        }
+        c->plan_workers = W;
+        c->plan_min_pages = plan.min_pages;
+        c->plan_max_pages = plan.max_pages;
+    }
     // layout
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off = align16(off + bytes); return o; };
-    const size_t o_slot = take(size_t(R) * 8), o_seq = take(size_t(R) * 4), o_len = take(size_t(R) * 4),
-                 o_pos = take(size_t(R) * 4), o_tblo = take(size_t(S) * 4), o_tbl = take(tbl_total * 4 + 4),
-                 o_sr = take(size_t(G) * 4), o_sb = take(size_t(G) * 4), o_se = take(size_t(G) * 4),
-                 o_rsb = take(size_t(R + 1) * 4), o_csb = take(size_t(W + 1) * 4), o_att = take(att_row ? size_t(R) * 4 : 0);
+    const size_t o_slot = take(size_t(A) * 8), o_apos = take(size_t(A) * 4), o_tbl = take(tbl_total * 4),
+                 o_pos = query ? take(size_t(R) * 4) : o_apos, o_att = take(att_row ? size_t(R) * 4 : 0),
+                 o_seg = take(size_t(G) * sizeof(mla::SegDesc)), o_parts = take(size_t(R) * layers * sizeof(mla::RowParts)),
+                 o_csb = take(size_t(W + 1) * 4);
     if (off > c->meta_cap)
         return fail(c, MLA_ERR_CAPACITY, "step metadata (" + std::to_string(off) + " B) exceeds the buffer (" +
                                              std::to_string(c->meta_cap) + " B)");
@@ -291,60 +339,74 @@ int upload_meta(mla_ctx* c, const std::vector<uint32_t>& seq_ids, const std::vec
         CU_TRY(c, cudaEventSynchronize(mb.done));
         mb.in_flight = false;
     }
-    char* h = static_cast<char*>(mb.host);
+    char* h = mb.host;
     auto* p_slot = reinterpret_cast<uint64_t*>(h + o_slot);
-    auto* p_seq = reinterpret_cast<uint32_t*>(h + o_seq);
-    auto* p_len = reinterpret_cast<uint32_t*>(h + o_len);
-    auto* p_pos = reinterpret_cast<uint32_t*>(h + o_pos);
-    for (uint32_t r = 0; r < R; r++) {
-        p_slot[r] = rows[r].slot;
-        p_seq[r] = rows[r].seq_index;
-        p_len[r] = rows[r].attend_len;
-        p_pos[r] = rows[r].pos;
-    }
-    std::memcpy(h + o_tblo, tbl_off.data(), size_t(S) * 4);
+    auto* p_apos = reinterpret_cast<uint32_t*>(h + o_apos);
+    for (uint32_t r = 0; r < A; r++) { p_slot[r] = app[r].slot; p_apos[r] = app[r].pos; }
     auto* p_tbl = reinterpret_cast<uint32_t*>(h + o_tbl);
     for (uint32_t i = 0; i < S; i++) {
         const auto& pg = c->pt->seq(seq_ids[i])->pages;
         std::memcpy(p_tbl + tbl_off[i], pg.data(), pg.size() * 4);
     }
-    auto* p_sr = reinterpret_cast<uint32_t*>(h + o_sr);
-    auto* p_sb = reinterpret_cast<uint32_t*>(h + o_sb);
-    auto* p_se = reinterpret_cast<uint32_t*>(h + o_se);
-    for (uint32_t g = 0; g < G; g++) {
-        p_sr[g] = segs[g].row;
-        p_sb[g] = segs[g].page_begin;
-        p_se[g] = segs[g].page_end;
+    if (query) {
+        auto* p_pos = reinterpret_cast<uint32_t*>(h + o_pos);
+        for (uint32_t r = 0; r < R; r++) p_pos[r] = rows[r].pos;
     }
-    std::memcpy(h + o_rsb, row_seg_begin.data(), size_t(R + 1) * 4);
-    std::memcpy(h + o_csb, cta_seg_begin.data(), size_t(W + 1) * 4);
     if (att_row) std::memcpy(h + o_att, att_row->data(), size_t(R) * 4);
-    char* d = c->meta_dev + (plan_b ? c->meta_cap : 0);
-    if (off) CU_TRY(c, cudaMemcpyAsync(d, h, off, cudaMemcpyHostToDevice, st));
+    auto* p_seg = reinterpret_cast<mla::SegDesc*>(h + o_seg);
+    for (uint32_t g = 0; g < G; g++) {
+        const RowSpec& rs = rows[segs[g].row % R];
+        const uint32_t tok0 = segs[g].page_begin * mla::kPage, tok1 = std::min(rs.attend_len, segs[g].page_end * uint32_t(mla::kPage));
+        const uint32_t n_tok = tok1 > tok0 ? tok1 - tok0 : 0;
+        p_seg[g] = mla::SegDesc{segs[g].row, tbl_off[rs.seq_index] + segs[g].page_begin, n_tok, segs[g].row / R, int32_t(n_tok), H, {0, 0}};
+    }
+    auto* p_parts = reinterpret_cast<mla::RowParts*>(h + o_parts);
+    for (uint32_t v = 0; v < R * layers; v++) p_parts[v] = mla::RowParts{row_seg_begin[v], row_seg_begin[v + 1], 0, 0};
+    std::memcpy(h + o_csb, cta_seg_begin.data(), size_t(W + 1) * 4);
+    char* d = c->meta_dev + size_t(region) * c->meta_cap;
+    CU_TRY(c, cudaMemcpyAsync(d, h, off, cudaMemcpyHostToDevice, st));
     CU_TRY(c, cudaEventRecord(mb.done, st));
     mb.in_flight = true;
 
-    mla::StepMeta& m = plan_b ? c->meta_b : c->meta;
-    m.row_slot = reinterpret_cast<const uint64_t*>(d + o_slot);
-    m.row_seq = reinterpret_cast<const uint32_t*>(d + o_seq);
-    m.row_len = reinterpret_cast<const uint32_t*>(d + o_len);
-    m.row_pos = reinterpret_cast<const uint32_t*>(d + o_pos);
-    m.seq_tbl_off = reinterpret_cast<const uint32_t*>(d + o_tblo);
+    mla::StepMeta& m = plan.m;
+    m.seg = reinterpret_cast<const mla::SegDesc*>(d + o_seg);
     m.tables = reinterpret_cast<const uint32_t*>(d + o_tbl);
-    m.seg_row = reinterpret_cast<const uint32_t*>(d + o_sr);
-    m.seg_page_begin = reinterpret_cast<const uint32_t*>(d + o_sb);
-    m.seg_page_end = reinterpret_cast<const uint32_t*>(d + o_se);
-    m.row_seg_begin = reinterpret_cast<const uint32_t*>(d + o_rsb);
     m.cta_seg_begin = reinterpret_cast<const uint32_t*>(d + o_csb);
+    m.parts = reinterpret_cast<const mla::RowParts*>(d + o_parts);
+    m.row_pos = reinterpret_cast<const uint32_t*>(d + o_pos);
     m.rows = R;
+    m.layers = layers ? layers : 1;
     m.segs = G;
     m.ctas = W;
-    // by default the rows to append are the query rows themselves
-    m.app_rows = R;
-    m.app_pos = m.row_pos;
-    m.app_slot = m.row_slot;
+    m.rec_stride = H;
+    m.app_rows = A;
+    m.app_pos = reinterpret_cast<const uint32_t*>(d + o_apos);
+    m.app_slot = reinterpret_cast<const uint64_t*>(d + o_slot);
     m.att_row = att_row ? reinterpret_cast<const uint32_t*>(d + o_att) : nullptr;
+    plan.ready = true;
     return MLA_OK;
+}
+
+// the open step's plan for one layer at a time
+int step_plan(mla_ctx* c, cudaStream_t st)
+{
+    return c->plan.ready ? int(MLA_OK) : build_plan(c, c->plan, kPlanStep, c->step_seqs, c->rows, nullptr, nullptr, 1, st);
+}
+
+// the plan of a step with prefill chunks: its decode-style rows are the query rows, all its rows are appended
+int rest_plan(mla_ctx* c, cudaStream_t st)
+{
+    if (c->plan_rest.ready) return MLA_OK;
+    std::vector<RowSpec> rest;
+    std::vector<uint32_t> att_row;
+    uint32_t r = 0;
+    for (uint32_t i = 0; i < c->step_nnew.size(); i++) {
+        const uint32_t cnt = std::max<uint32_t>(c->step_nnew[i], 1);
+        if (c->step_nnew[i] < kPrefillMin)
+            for (uint32_t t = 0; t < cnt; t++) { rest.push_back(c->rows[r + t]); att_row.push_back(r + t); }
+        r += cnt;
+    }
+    return build_plan(c, c->plan_rest, kPlanRest, c->step_seqs, c->rows, &rest, &att_row, 1, st);
 }
 
 char* layer_pool(mla_ctx* c, uint32_t layer)
@@ -355,71 +417,65 @@ char* layer_pool(mla_ctx* c, uint32_t layer)
 int check_layer(mla_ctx* c, uint32_t layer, bool need_weights)
 {
     if (layer >= c->cfg.n_layers) return fail(c, MLA_ERR_INVALID, "layer " + std::to_string(layer) + " out of range");
-    if (need_weights && !c->layers[layer].set)
+    if (need_weights && !c->layer_set[layer])
         return fail(c, MLA_ERR_STATE, "weights of layer " + std::to_string(layer) + " were never registered");
     return MLA_OK;
 }
 
-int run_append(mla_ctx* c, uint32_t layer, const void* kv_a, cudaStream_t st)
+// one layer's slices of the weights
+size_t weight_bytes(const mla_ctx* c) { return size_t(c->cfg.n_heads) * mla::kNope * mla::kRank * 2; }
+char* layer_norm(mla_ctx* c, uint32_t layer) { return c->norm + size_t(layer) * mla::kRank * 2; }
+
+int run_append(mla_ctx* c, uint32_t layer, const void* kv_a, const mla::StepMeta& m, cudaStream_t st)
 {
-    mla::launch_append(int(c->cfg.dtype), kv_a, layer_pool(c, layer), c->pool_slots, c->layers[layer].norm,
-                       c->cos_sin, c->cs_rows, c->cfg.rms_norm_eps, c->meta, c->status_dev, st);
-    c->launches += c->meta.app_rows ? 1 : 0;
+    mla::launch_append(int(c->cfg.dtype), kv_a, layer_pool(c, layer), c->pool_slots, layer_norm(c, layer),
+                       c->cos_sin, c->cs_rows, c->cfg.rms_norm_eps, m, c->status_dev, st);
+    c->launches += m.app_rows ? 1 : 0;
     CU_TRY(c, cudaGetLastError());
     return MLA_OK;
 }
 
-int run_merge(mla_ctx* c, uint32_t layer, const float* recs, const uint32_t* row_seg_begin, uint32_t n_parts, void* out,
-              float* exported, uint32_t rows, cudaStream_t st, const uint32_t* att_row = nullptr);
-
-// absorb -> split-KV attention -> merge (+ W_UV, or export of the merged partial state)
+// absorb -> split-KV attention -> merge (+ W_UV, or export of the merged partial state) of the plan's layers from `layer` on
 // With fused_kv_a the absorb launch also appends the step's new rows (the caller then skips run_append).
-int run_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, float* exported, cudaStream_t st,
-               const void* fused_kv_a = nullptr, bool kv_a_settled = false, bool plan_b = false)
+int run_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, float* exported, const Plan& p, cudaStream_t st,
+               const void* fused_kv_a = nullptr, bool kv_a_settled = false)
 {
-    const mla::StepMeta& m = plan_b ? c->meta_b : c->meta;
+    const mla::StepMeta& m = p.m;
     if (m.rows == 0) return MLA_OK;
     const uint32_t H = c->cfg.n_heads;
-    const LayerW& lw = c->layers[layer];
-    if (lw.has_map) {
-        const int ae = mla::launch_absorb_tc5(int(c->cfg.dtype), q, &lw.w_uk_map, c->q_abs, m.rows, H, fused_kv_a,
-                                              layer_pool(c, layer), c->pool_slots, lw.norm, c->cos_sin, c->cs_rows,
-                                              c->cfg.rms_norm_eps, m, c->q_rope_in_kernel, !kv_a_settled, c->status_dev, st);
-        if (ae != 0) return fail(c, MLA_ERR_CUDA, std::string("absorb launch: ") + cudaGetErrorString(cudaError_t(ae)));
-    } else {
-        if (fused_kv_a) return fail(c, MLA_ERR_STATE, "fused append needs the layer's tensor maps");
-        if (c->q_rope_in_kernel) return fail(c, MLA_ERR_UNSUPPORTED, "in-kernel q RoPE needs the layer's tensor maps");
-        if (m.att_row) return fail(c, MLA_ERR_UNSUPPORTED, "a step with prefill chunks needs the layer's tensor maps");
-        mla::launch_absorb(int(c->cfg.dtype), q, lw.w_uk, c->q_abs, m.rows, H, st);
-    }
+    const int dt = int(c->cfg.dtype);
+    const int ae = mla::launch_absorb_tc5(dt, q, &c->w_uk_map, c->q_abs, H, layer, fused_kv_a, layer_pool(c, layer), c->pool_slots,
+                                          layer_norm(c, layer), c->cos_sin, c->cs_rows, c->cfg.rms_norm_eps, m, c->q_rope_in_kernel,
+                                          !kv_a_settled, c->status_dev, st);
+    if (ae != 0) return fail(c, MLA_ERR_CUDA, std::string("absorb launch: ") + cudaGetErrorString(cudaError_t(ae)));
     int e;
     const bool timed = c->profiling && c->prof_used < c->prof_events.size() && (c->prof_seq++ % c->prof_stride) == 0;
     if (timed) CU_TRY(c, cudaEventRecord(c->prof_events[c->prof_used].first, st));
     // the W_UK the stream will want next: the following layer's (the first layer's after the last: the next step)
-    const LayerW& nlw = c->layers[(layer + 1) % c->cfg.n_layers];
-    const void* next_w = nlw.set ? nlw.w_uk : nullptr;
-    if (c->kernel == MLA_KERNEL_TCGEN05_PAIR128)
+    const uint32_t nl = (layer + m.layers) % c->cfg.n_layers;
+    const void* next_w = c->layer_set[nl] ? c->w_uk + nl * weight_bytes(c) : nullptr;
+    if (p.kernel == MLA_KERNEL_TCGEN05_PAIR128)
         // short work lists (few sequences on this GPU) are bound by load latency, not bandwidth: prefetch one tile ahead
-        e = mla::launch_decode_tc5_pair128(int(c->cfg.dtype), c->tmaps, layer_pool(c, layer), layer, c->cfg.n_pages, m, c->recs, H,
-                                           c->plan_max_pages <= 64 ? 1u : 0u, next_w, next_w ? uint32_t(size_t(H) * mla::kNope * mla::kRank * 2) : 0u,
-                                           c->status_dev, st);
-    else if (c->kernel == MLA_KERNEL_TCGEN05)
-        e = mla::launch_decode_tc5(int(c->cfg.dtype), c->tmaps, layer, c->cfg.n_pages, m, c->recs, H, c->status_dev, st);
-    else if (c->kernel == MLA_KERNEL_TCGEN05_T16)
-        e = mla::launch_decode_tc5_t16(int(c->cfg.dtype), c->tmaps, layer, c->cfg.n_pages, m, c->recs, H, c->status_dev, st);
+        e = mla::launch_decode_tc5_pair128(dt, c->tmaps, c->pool, layer, c->cfg.n_pages, m, c->recs, H, p.max_pages <= 64 ? 1u : 0u,
+                                           next_w, next_w ? uint32_t(weight_bytes(c)) : 0u, c->status_dev, st);
+    else if (p.kernel == MLA_KERNEL_TCGEN05)
+        e = mla::launch_decode_tc5(dt, c->tmaps, layer, c->cfg.n_pages, m, c->recs, H, c->status_dev, st);
+    else if (p.kernel == MLA_KERNEL_TCGEN05_T16)
+        e = mla::launch_decode_tc5_t16(dt, c->tmaps, layer, c->cfg.n_pages, m, c->recs, H, c->status_dev, st);
     else
-        e = mla::launch_decode_mma(int(c->cfg.dtype), c->q_abs, layer_pool(c, layer), c->cfg.n_pages, m,
-                                   c->recs, H, c->status_dev, st);
+        e = mla::launch_decode_mma(dt, c->q_abs, layer_pool(c, layer), c->cfg.n_pages, m, c->recs, H, c->status_dev, st);
     if (e != 0) return fail(c, MLA_ERR_CUDA, std::string("attention launch: ") + cudaGetErrorString(cudaError_t(e)));
     if (timed) CU_TRY(c, cudaEventRecord(c->prof_events[c->prof_used++].second, st));
-    if (int rc = run_merge(c, layer, c->recs, m.row_seg_begin, 0, out, exported, m.rows, st, m.att_row)) return rc;
+    if (exported) {
+        mla::launch_export_partial(c->recs, m, exported, H, st);
+    } else {
+        e = mla::launch_merge_tc5(dt, c->recs, m, 0, &c->w_uv_map, out, H, layer, c->status_dev, st);
+        if (e != 0) return fail(c, MLA_ERR_CUDA, std::string("merge launch: ") + cudaGetErrorString(cudaError_t(e)));
+    }
     c->launches += 3;
     CU_TRY(c, cudaGetLastError());
     return MLA_OK;
 }
-
-// Sequences that take at least this many new tokens in a step go through the prefill kernels.
-constexpr uint32_t kPrefillMin = 64;
 
 int grow_buf(mla_ctx* c, void** p, size_t* cap, size_t bytes)
 {
@@ -439,23 +495,20 @@ int grow_buf(mla_ctx* c, void** p, size_t* cap, size_t bytes)
 int run_chunks(mla_ctx* c, uint32_t layer, const void* q, void* out, cudaStream_t st)
 {
     const uint32_t H = c->cfg.n_heads;
-    const LayerW& lw = c->layers[layer];
     const int dt = int(c->cfg.dtype);
+    const char *w_uk = c->w_uk_rows + layer * weight_bytes(c), *w_uv = c->w_uv + layer * weight_bytes(c);
     for (const auto& ch : c->chunks) {
         const uint32_t total = ch.start + ch.n_new;
         if (int e = grow_buf(c, &c->pf_latent, &c->pf_latent_cap, size_t(total) * mla::kRow * 2)) return e;
         if (int e = grow_buf(c, &c->pf_kx, &c->pf_kx_cap, size_t(total) * H * mla::kNope * 2)) return e;
         if (int e = grow_buf(c, &c->pf_vx, &c->pf_vx_cap, size_t(total) * H * mla::kVDim * 2)) return e;
-        // the sequence's block table inside the first plan's upload
-        uint32_t si = 0;
-        for (; si < c->step_seqs.size(); si++) if (c->step_seqs[si] == ch.seq_id) break;
-        const uint32_t* table = c->meta.tables + c->step_tbl_off[si];
+        const uint32_t* table = c->plan_rest.m.tables + ch.tbl_off;
         int rc = mla::launch_gather_rows(layer_pool(c, layer), c->pool_slots, table, total, c->pf_latent, c->status_dev, st);
         if (rc) return fail(c, MLA_ERR_CUDA, std::string("gather launch: ") + cudaGetErrorString(cudaError_t(rc)));
-        rc = mla::launch_gemm_tc5(dt, c->pf_latent, mla::kRow, lw.w_uk_rows, mla::kRank, total, H * mla::kNope, mla::kRank, c->pf_kx,
+        rc = mla::launch_gemm_tc5(dt, c->pf_latent, mla::kRow, w_uk, mla::kRank, total, H * mla::kNope, mla::kRank, c->pf_kx,
                                   nullptr, 1, c->status_dev, st);
         if (rc == 0)
-            rc = mla::launch_gemm_tc5(dt, c->pf_latent, mla::kRow, lw.w_uv, mla::kRank, total, H * mla::kVDim, mla::kRank, c->pf_vx,
+            rc = mla::launch_gemm_tc5(dt, c->pf_latent, mla::kRow, w_uv, mla::kRank, total, H * mla::kVDim, mla::kRank, c->pf_vx,
                                       nullptr, 1, c->status_dev, st);
         if (rc) return fail(c, rc == -1 ? MLA_ERR_INVALID : MLA_ERR_CUDA, "key / value expansion launch failed");
         const void* qp = q;
@@ -484,18 +537,18 @@ int run_chunks(mla_ctx* c, uint32_t layer, const void* q, void* out, cudaStream_
 // kv_a_settled: kv_a was complete before the kernel launched just ahead of this layer's started (see launch_absorb_tc5).
 int run_layer(mla_ctx* c, uint32_t layer, const void* kv_a, const void* q, void* out, cudaStream_t st, bool kv_a_settled = false)
 {
-    if (c->has_plan_b) {
-        // decode-style rows through the second plan (their append covers ALL new rows of the step), then the chunks
-        if (c->meta_b.rows && c->layers[layer].has_map) {
-            if (int e = run_attend(c, layer, q, out, nullptr, st, kv_a, kv_a_settled, true)) return e;
+    if (c->has_chunks) {
+        // decode-style rows through their own plan (their append covers ALL new rows of the step), then the chunks
+        if (int e = rest_plan(c, st)) return e;
+        if (c->plan_rest.m.rows) {
+            if (int e = run_attend(c, layer, q, out, nullptr, c->plan_rest, st, kv_a, kv_a_settled)) return e;
         } else {
-            if (int e = run_append(c, layer, kv_a, st)) return e;
+            if (int e = run_append(c, layer, kv_a, c->plan_rest.m, st)) return e;
         }
         return run_chunks(c, layer, q, out, st);
     }
-    if (c->layers[layer].has_map) return run_attend(c, layer, q, out, nullptr, st, kv_a, kv_a_settled);
-    if (int e = run_append(c, layer, kv_a, st)) return e;
-    return run_attend(c, layer, q, out, nullptr, st);
+    if (int e = step_plan(c, st)) return e;
+    return run_attend(c, layer, q, out, nullptr, c->plan, st, kv_a, kv_a_settled);
 }
 
 using TensorMapEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -511,49 +564,6 @@ TensorMapEncodeFn tensor_map_encoder()
         qres != cudaDriverEntryPointSuccess)
         return nullptr;
     return reinterpret_cast<TensorMapEncodeFn>(fn);
-}
-
-int make_weight_map(mla_ctx* c, uint32_t layer)
-{
-    TensorMapEncodeFn enc = tensor_map_encoder();
-    if (!enc) return fail(c, MLA_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-    const CUtensorMapDataType dt = c->cfg.dtype == MLA_DTYPE_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
-                                                                 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    const cuuint64_t dims[2] = {cuuint64_t(mla::kRank), cuuint64_t(c->cfg.n_heads) * mla::kVDim};
-    const cuuint64_t strides[1] = {cuuint64_t(mla::kRank) * 2};
-    const cuuint32_t box[2] = {64, cuuint32_t(mla::kVDim)};
-    const cuuint32_t estr[2] = {1, 1};
-    LayerW& lw = c->layers[layer];
-    const CUresult r = enc(&lw.w_uv_map, dt, 2, lw.w_uv, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS)
-        return fail(c, MLA_ERR_CUDA, "cuTensorMapEncodeTiled(W_UV) failed with code " + std::to_string(int(r)));
-    const cuuint64_t kdims[2] = {cuuint64_t(mla::kNope), cuuint64_t(c->cfg.n_heads) * mla::kRank};
-    const cuuint64_t kstrides[1] = {cuuint64_t(mla::kNope) * 2};
-    const cuuint32_t kbox[2] = {64, 256};
-    const CUresult r2 = enc(&lw.w_uk_map, dt, 2, lw.w_uk, kdims, kstrides, kbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r2 != CUDA_SUCCESS)
-        return fail(c, MLA_ERR_CUDA, "cuTensorMapEncodeTiled(W_UK) failed with code " + std::to_string(int(r2)));
-    lw.has_map = true;
-    return MLA_OK;
-}
-
-// merge of the partial states + W_UV: tensor-core kernel, or the scalar one when the merged state is exported
-int run_merge(mla_ctx* c, uint32_t layer, const float* recs, const uint32_t* row_seg_begin, uint32_t n_parts, void* out,
-              float* exported, uint32_t rows, cudaStream_t st, const uint32_t* att_row)
-{
-    const LayerW& lw = c->layers[layer];
-    if (!exported && lw.has_map) {
-        const int e = mla::launch_merge_tc5(int(c->cfg.dtype), recs, row_seg_begin, n_parts, &lw.w_uv_map, out, rows,
-                                            c->cfg.n_heads, att_row, c->status_dev, st);
-        if (e != 0) return fail(c, MLA_ERR_CUDA, std::string("merge launch: ") + cudaGetErrorString(cudaError_t(e)));
-        return MLA_OK;
-    }
-    mla::launch_merge(int(c->cfg.dtype), recs, row_seg_begin, n_parts, lw.w_uv, out, exported, rows, c->cfg.n_heads, st, att_row);
-    return MLA_OK;
 }
 
 int make_tensor_maps(mla_ctx* c)
@@ -572,6 +582,21 @@ int make_tensor_maps(mla_ctx* c)
             return fail(c, MLA_ERR_CUDA, std::string("cuTensorMapEncodeTiled(") + what + ") failed with code " + std::to_string(int(r)));
         return MLA_OK;
     };
+    {   // W_UV of all layers as [layers*H*128 outputs][512 dims], boxes of 64 dims x 128 outputs (merge), and W_UK^T as
+        // [layers*H*512 d][128 i], boxes of 64 i x 256 d (absorb)
+        auto weights = [&](CUtensorMap* map, const char* what, void* basep, cuuint64_t inner, cuuint64_t outer, cuuint32_t box_rows) -> int {
+            const cuuint64_t dims[2] = {inner, outer}, strides[1] = {inner * 2};
+            const cuuint32_t box[2] = {64, box_rows};
+            const CUresult r = enc(map, dt, 2, basep, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            if (r != CUDA_SUCCESS)
+                return fail(c, MLA_ERR_CUDA, std::string("cuTensorMapEncodeTiled(") + what + ") failed with code " + std::to_string(int(r)));
+            return MLA_OK;
+        };
+        const cuuint64_t heads = cuuint64_t(c->cfg.n_layers) * c->cfg.n_heads;
+        if (int e = weights(&c->w_uv_map, "W_UV", c->w_uv, mla::kRank, heads * mla::kVDim, mla::kVDim)) return e;
+        if (int e = weights(&c->w_uk_map, "W_UK", c->w_uk, mla::kNope, heads * mla::kRank, 256)) return e;
+    }
     {   // cache pool: 576 values innermost, then the token slots of a layer, then layers;
         // box = 64 values (128 B, one swizzle row) x 64 tokens (one page)
         const cuuint64_t dims[3] = {cuuint64_t(mla::kRow), c->pool_slots, c->cfg.n_layers};
@@ -590,7 +615,7 @@ int make_tensor_maps(mla_ctx* c)
         if (int e = encode(mla::kMapPoolV, "cache pool, two chunks of a page", 4, c->pool, dims, strides, box_v)) return e;
         if (int e = encode(mla::kMapPoolPage, "cache pool, whole page", 4, c->pool, dims, strides, box_page)) return e;
         // 64 spare rows behind the queries: boxes of 64 head rows may start at the last row's heads
-        const cuuint64_t qdims[3] = {64, cuuint64_t(c->cfg.max_rows) * c->cfg.n_heads + 64, 9};
+        const cuuint64_t qdims[3] = {64, cuuint64_t(c->ws_rows) * c->cfg.n_heads + 64, 9};
         const cuuint64_t qstrides[2] = {cuuint64_t(mla::kRow) * 2, 128};
         const cuuint32_t qbox[3] = {64, 64, 9};
         if (int e = encode(mla::kMapQueries, "absorbed queries", 3, c->q_abs, qdims, qstrides, qbox)) return e;
@@ -648,21 +673,11 @@ int mla_create(const mla_config* cfg, mla_ctx** out)
     if (prop.major != 10)
         { cp->err = "this library is built for sm_100a only; device is sm_" + std::to_string(prop.major * 10 + prop.minor);
           return bail(MLA_ERR_UNSUPPORTED); }
-    // 128-head groups go to the SM-pair kernel; up to 16 heads take the transposed tcgen05 form (tokens as rows, the
-    // heads as 16 columns); everything between fills (part of) the 64-row tiles of the single-block kernel, which
-    // streams the cache once per 64 heads (measured at 32 heads, 64 sequences x 8192 tokens: 128 us against 186 us for
-    // two passes of the 16-column form and 300 us for mma.sync)
-    c->kernel = cfg->kernel != MLA_KERNEL_AUTO ? cfg->kernel
-              : (cfg->n_heads % 128 == 0 && c->sm_count % 2 == 0) ? uint32_t(MLA_KERNEL_TCGEN05_PAIR128)
-              : cfg->n_heads > 16 ? uint32_t(MLA_KERNEL_TCGEN05) : uint32_t(MLA_KERNEL_TCGEN05_T16);
+    c->kernel = kernel_for(cp, cfg->n_heads);
     const uint32_t H = cfg->n_heads;
-    if (c->kernel == MLA_KERNEL_TCGEN05_PAIR128) c->workers = std::max<uint32_t>(1, (c->sm_count / 2) / ((H + 127) / 128));
-    else if (c->kernel == MLA_KERNEL_TCGEN05) c->workers = std::max<uint32_t>(1, c->sm_count / ((H + 63) / 64));
-    else if (c->kernel == MLA_KERNEL_TCGEN05_T16) c->workers = std::max<uint32_t>(1, c->sm_count / ((H + 15) / 16));
-    else c->workers = std::max<uint32_t>(1, c->sm_count * 2 / ((H + 15) / 16));
 
     c->pt = std::make_unique<PageTable>(cfg->page_tokens, cfg->n_pages, cfg->max_seqs, cfg->max_seq_len);
-    c->layers.resize(cfg->n_layers);
+    c->layer_set.resize(cfg->n_layers, 0);
     c->blocks.resize(cfg->n_layers);
     c->pool_slots = uint64_t(cfg->n_pages) * cfg->page_tokens;
     const size_t pool_bytes = size_t(cfg->n_layers) * c->pool_slots * mla::kRow * 2;
@@ -670,31 +685,30 @@ int mla_create(const mla_config* cfg, mla_ctx** out)
     // zero-fill: rows past a sequence's end inside its last page are multiplied by P = 0 and
     // must therefore hold finite values
     CR_TRY(cudaMemset(c->pool, 0, pool_bytes));
-    for (auto& lw : c->layers) {
-        CR_TRY(cudaMalloc(&lw.w_uk, size_t(H) * mla::kNope * mla::kRank * 2));
-        CR_TRY(cudaMalloc(&lw.w_uk_rows, size_t(H) * mla::kNope * mla::kRank * 2));
-        CR_TRY(cudaMalloc(&lw.w_uv, size_t(H) * mla::kVDim * mla::kRank * 2));
-        CR_TRY(cudaMalloc(&lw.norm, mla::kRank * 2));
-    }
+    for (char** w : {&c->w_uk, &c->w_uk_rows, &c->w_uv}) CR_TRY(cudaMalloc(w, weight_bytes(cp) * cfg->n_layers));
+    CR_TRY(cudaMalloc(&c->norm, size_t(cfg->n_layers) * mla::kRank * 2));
     // rotary table: one row per position a sequence can reach
     c->cs_cap = std::max(cfg->max_seq_len, cfg->max_position);
     CR_TRY(cudaMalloc(&c->cos_sin, size_t(c->cs_cap) * mla::kRope * sizeof(float)));
-    const uint32_t R = c->cfg.max_rows;
+    // Workspace for the rows of one step, or of a group of layers when a step has few rows (step_layers_grouped): the
+    // absorbed queries of a group stay within kGroupBytes, so that they and the partial states stay in L2 between launches.
+    const uint64_t row_bytes = uint64_t(H) * mla::kRow * 2;
+    c->ws_rows = std::max<uint32_t>(c->cfg.max_rows, uint32_t(std::min<uint64_t>({uint64_t(c->cfg.max_rows) * cfg->n_layers, kGroupRows,
+                                                                                  std::max<uint64_t>(1, kGroupBytes / row_bytes)})));
     // 64 spare rows: the tcgen05 kernel fetches queries in boxes of 64 head rows
-    CR_TRY(cudaMalloc(&c->q_abs, (size_t(R) * H + 64) * mla::kRow * 2));
-    CR_TRY(cudaMemset(c->q_abs, 0, (size_t(R) * H + 64) * mla::kRow * 2));
-    c->max_segs = c->workers + R;
-    CR_TRY(cudaMalloc(&c->recs, size_t(c->max_segs) * H * mla::kPart * sizeof(float)));
+    CR_TRY(cudaMalloc(&c->q_abs, (size_t(c->ws_rows) * H + 64) * mla::kRow * 2));
+    CR_TRY(cudaMemset(c->q_abs, 0, (size_t(c->ws_rows) * H + 64) * mla::kRow * 2));
+    // a plan has at most one segment per row more than it has workers
+    c->rec_cap = (size_t(workers_of(cp, c->kernel, H)) + c->ws_rows) * H;
+    CR_TRY(cudaMalloc(&c->recs, c->rec_cap * mla::kPart * sizeof(float)));
     CR_TRY(cudaMalloc(&c->status_dev, sizeof(uint32_t)));
     CR_TRY(cudaMemset(c->status_dev, 0, sizeof(uint32_t)));
-    const size_t max_pages_per_seq = (size_t(cfg->max_seq_len) + cfg->page_tokens - 1) / cfg->page_tokens;
-    const size_t tbl_entries = std::min<size_t>(size_t(cfg->max_seqs) * max_pages_per_seq, cfg->n_pages) + 4;
-    c->meta_cap = align16(size_t(R) * 8) + 3 * align16(size_t(R) * 4) + align16(size_t(cfg->max_seqs) * 4) +
-                  align16(tbl_entries * 4 + 4) + 3 * align16(size_t(c->max_segs) * 4) +
-                  align16(size_t(R + 1) * 4) + align16(size_t(c->workers + 1) * 4) + align16(size_t(R) * 4) + 256;
-    CR_TRY(cudaMalloc(&c->meta_dev, 2 * c->meta_cap));                // the two plans of a step live side by side
-    for (auto& mb : c->ring) {
-        CR_TRY(cudaMallocHost(&mb.host, c->meta_cap));
+    c->meta_cap = meta_capacity(cp);
+    CR_TRY(cudaMalloc(&c->meta_dev, kPlanRegions * c->meta_cap));
+    CR_TRY(cudaMallocHost(&c->meta_host, kMetaRing * c->meta_cap));
+    for (int i = 0; i < kMetaRing; i++) {
+        MetaBuf& mb = c->ring[i];
+        mb.host = c->meta_host + i * c->meta_cap;
         CR_TRY(cudaEventCreateWithFlags(&mb.done, cudaEventDisableTiming));
     }
     if (int ce = mla::decode_mma_configure()) {
@@ -721,26 +735,18 @@ int mla_create(const mla_config* cfg, mla_ctx** out)
         cp->err = std::string("tcgen05 merge kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));
         return bail(MLA_ERR_CUDA);
     }
-    if (c->kernel == MLA_KERNEL_TCGEN05_PAIR128) {
-        if (int rc = make_tensor_maps(cp)) return bail(rc);
-        if (int ce = mla::decode_tc5_pair128_configure()) {
-            cp->err = std::string("tcgen05 pair128 kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));
-            return bail(MLA_ERR_CUDA);
-        }
+    if (int rc = make_tensor_maps(cp)) return bail(rc);
+    if (int ce = mla::decode_tc5_pair128_configure()) {
+        cp->err = std::string("tcgen05 pair128 kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));
+        return bail(MLA_ERR_CUDA);
     }
-    if (c->kernel == MLA_KERNEL_TCGEN05) {
-        if (int rc = make_tensor_maps(cp)) return bail(rc);
-        if (int ce = mla::decode_tc5_configure()) {
-            cp->err = std::string("tcgen05 kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));
-            return bail(MLA_ERR_CUDA);
-        }
+    if (int ce = mla::decode_tc5_configure()) {
+        cp->err = std::string("tcgen05 kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));
+        return bail(MLA_ERR_CUDA);
     }
-    if (c->kernel == MLA_KERNEL_TCGEN05_T16) {
-        if (int rc = make_tensor_maps(cp)) return bail(rc);
-        if (int ce = mla::decode_tc5_t16_configure()) {
-            cp->err = std::string("tcgen05 16-head kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));
-            return bail(MLA_ERR_CUDA);
-        }
+    if (int ce = mla::decode_tc5_t16_configure()) {
+        cp->err = std::string("tcgen05 16-head kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));
+        return bail(MLA_ERR_CUDA);
     }
 #undef CR_TRY
     *out = c.release();
@@ -753,7 +759,7 @@ void mla_destroy(mla_ctx* c)
     cudaSetDevice(c->cfg.device);
     cudaDeviceSynchronize();
     cudaFree(c->pool);
-    for (auto& lw : c->layers) { cudaFree(lw.w_uk); cudaFree(lw.w_uk_rows); cudaFree(lw.w_uv); cudaFree(lw.norm); }
+    cudaFree(c->w_uk); cudaFree(c->w_uk_rows); cudaFree(c->w_uv); cudaFree(c->norm);
     cudaFree(c->pf_latent); cudaFree(c->pf_kx); cudaFree(c->pf_vx); cudaFree(c->pf_q);
     cudaFree(c->cos_sin);
     cudaFree(c->q_abs);
@@ -761,9 +767,9 @@ void mla_destroy(mla_ctx* c)
     cudaFree(c->status_dev);
     cudaFree(c->meta_dev);
     for (auto& mb : c->ring) {
-        if (mb.host) cudaFreeHost(mb.host);
         if (mb.done) cudaEventDestroy(mb.done);
     }
+    if (c->meta_host) cudaFreeHost(c->meta_host);
     for (auto& pe : c->prof_events) { cudaEventDestroy(pe.first); cudaEventDestroy(pe.second); }
     if (c->h_in) cudaFreeHost(c->h_in);
     if (c->h_out) cudaFreeHost(c->h_out);
@@ -807,14 +813,13 @@ int mla_set_layer_weights(mla_ctx* c, uint32_t layer, const void* w_uk, const vo
             for (size_t i = 0; i < size_t(mla::kNope); i++)
                 for (size_t d = 0; d < size_t(mla::kRank); d++)
                     tr[(h * mla::kRank + d) * mla::kNope + i] = buf[(h * mla::kNope + i) * mla::kRank + d];
-        CU_TRY(c, cudaMemcpy(c->layers[layer].w_uk, tr.data(), tr.size() * 2, cudaMemcpyHostToDevice));
-        CU_TRY(c, cudaMemcpy(c->layers[layer].w_uk_rows, buf.data(), buf.size() * 2, cudaMemcpyHostToDevice));
+        CU_TRY(c, cudaMemcpy(c->w_uk + layer * weight_bytes(c), tr.data(), tr.size() * 2, cudaMemcpyHostToDevice));
+        CU_TRY(c, cudaMemcpy(c->w_uk_rows + layer * weight_bytes(c), buf.data(), buf.size() * 2, cudaMemcpyHostToDevice));
     }
     if (int e = decode_weights(c, w_uv, w_type, H * mla::kVDim, buf)) return e;
-    CU_TRY(c, cudaMemcpy(c->layers[layer].w_uv, buf.data(), buf.size() * 2, cudaMemcpyHostToDevice));
-    CU_TRY(c, cudaMemcpy(c->layers[layer].norm, kv_norm, mla::kRank * 2, cudaMemcpyHostToDevice));
-    if (int e = make_weight_map(c, layer)) return e;
-    c->layers[layer].set = true;
+    CU_TRY(c, cudaMemcpy(c->w_uv + layer * weight_bytes(c), buf.data(), buf.size() * 2, cudaMemcpyHostToDevice));
+    CU_TRY(c, cudaMemcpy(layer_norm(c, layer), kv_norm, mla::kRank * 2, cudaMemcpyHostToDevice));
+    c->layer_set[layer] = 1;
     return MLA_OK;
 }
 
@@ -914,8 +919,8 @@ int mla_append_rows(mla_ctx* c, uint32_t layer, uint32_t n, const uint32_t* seq_
         max_pos = std::max(max_pos, positions[r]);
     }
     if (n) if (int e = ensure_rope_rows(c, max_pos + 1, st)) return e;
-    if (int e = upload_meta(c, seqs, rows, false, st)) return e;
-    return run_append(c, layer, kv_a, st);
+    if (int e = build_plan(c, c->plan, kPlanStep, seqs, rows, nullptr, nullptr, 0, st)) return e;
+    return run_append(c, layer, kv_a, c->plan.m, st);
 }
 
 int mla_attend_rows(mla_ctx* c, uint32_t layer, uint32_t n, const uint32_t* seq_ids, const uint32_t* attend_lens,
@@ -945,8 +950,8 @@ int mla_attend_rows(mla_ctx* c, uint32_t layer, uint32_t n, const uint32_t* seq_
         max_pos = std::max(max_pos, qpos);
     }
     if (n && c->q_rope_in_kernel) if (int e = ensure_rope_rows(c, max_pos + 1, st)) return e;
-    if (int e = upload_meta(c, seqs, rows, true, st)) return e;
-    return run_attend(c, layer, q, out, nullptr, st);
+    if (int e = build_plan(c, c->plan, kPlanStep, seqs, rows, nullptr, nullptr, 1, st)) return e;
+    return run_attend(c, layer, q, out, nullptr, c->plan, st);
 }
 
 int mla_step_begin(mla_ctx* c, uint32_t n_seq, const uint32_t* seq_ids, const uint32_t* n_new, void* stream)
@@ -974,8 +979,13 @@ int mla_step_begin(mla_ctx* c, uint32_t n_seq, const uint32_t* seq_ids, const ui
         if (nn[i]) max_pos = std::max(max_pos, s->base_pos + s->len + nn[i] - 1);
     }
     if (total) if (int e = ensure_rope_rows(c, max_pos + 1, st)) return e;
-    std::vector<RowSpec> rows;
+    auto& rows = c->rows;
+    rows.clear();
     rows.reserve(total);
+    c->chunks.clear();
+    c->has_chunks = false;
+    c->step_new_rows = 0;
+    uint32_t tbl_off = 0;
     for (uint32_t i = 0; i < n_seq; i++) {
         const auto* s = c->pt->seq(seqs[i]);
         if (nn[i] == 0) {                                              // query-only row
@@ -984,48 +994,19 @@ int mla_step_begin(mla_ctx* c, uint32_t n_seq, const uint32_t* seq_ids, const ui
                                                     "(mla_set_q_rope(ctx, 0)) for KV-range shards that do not own the tail");
             rows.push_back({i, s->len, 0, ~uint64_t(0)});
         }
+        if (nn[i] >= kPrefillMin && c->kernel != MLA_KERNEL_MMA) {
+            c->chunks.push_back({tbl_off, uint32_t(rows.size()), nn[i], s->len, s->base_pos});
+            c->has_chunks = true;
+        }
         for (uint32_t t = 0; t < nn[i]; t++) {
             const uint32_t local = s->len + t;
             rows.push_back({i, local + 1, s->base_pos + local, c->pt->slot(seqs[i], local)});
         }
-    }
-    if (int e = upload_meta(c, seqs, rows, true, st)) return e;
-    c->step_new_rows = 0;
-    for (uint32_t i = 0; i < n_seq; i++) c->step_new_rows += nn[i];
-    // table offsets of the step's sequences inside the upload (the prefill path gathers rows through them)
-    c->step_tbl_off.resize(n_seq);
-    {
-        uint32_t o = 0;
-        for (uint32_t i = 0; i < n_seq; i++) { c->step_tbl_off[i] = o; o += uint32_t(c->pt->seq(seqs[i])->pages.size()); }
+        c->step_new_rows += nn[i];
+        tbl_off += uint32_t(s->pages.size());
     }
     c->step_rows = uint32_t(rows.size());
-    c->chunks.clear();
-    c->has_plan_b = false;
-    bool any_chunk = false;
-    for (uint32_t i = 0; i < n_seq; i++) any_chunk = any_chunk || nn[i] >= kPrefillMin;
-    if (any_chunk && c->kernel != MLA_KERNEL_MMA) {
-        std::vector<RowSpec> rows_b;
-        std::vector<uint32_t> att_row;
-        uint32_t r = 0;
-        for (uint32_t i = 0; i < n_seq; i++) {
-            const auto* sq = c->pt->seq(seqs[i]);
-            const uint32_t cnt = std::max<uint32_t>(nn[i], 1);
-            if (nn[i] >= kPrefillMin) {
-                c->chunks.push_back({seqs[i], r, nn[i], sq->len, sq->base_pos});
-            } else {
-                for (uint32_t t = 0; t < cnt; t++) { rows_b.push_back(rows[r + t]); att_row.push_back(r + t); }
-            }
-            r += cnt;
-        }
-        const uint32_t plan_workers = c->plan_workers, plan_min = c->plan_min_pages, plan_max = c->plan_max_pages;
-        if (int e = upload_meta(c, seqs, rows_b, true, st, true, &att_row)) return e;
-        (void)plan_workers; (void)plan_min; (void)plan_max;
-        // the append of the second plan still writes every new row of the step, in the caller's order
-        c->meta_b.app_rows = c->meta.rows;
-        c->meta_b.app_pos = c->meta.row_pos;
-        c->meta_b.app_slot = c->meta.row_slot;
-        c->has_plan_b = true;
-    }
+    c->plan.ready = c->plan_rest.ready = c->stack.ready = c->stack_tail.ready = false;
     c->step_seqs = std::move(seqs);
     c->step_nnew = std::move(nn);
     c->in_step = true;
@@ -1038,7 +1019,9 @@ int mla_step_append(mla_ctx* c, uint32_t layer, const void* kv_a, void* stream)
     USE_DEVICE(c);
     if (!c->in_step) return fail(c, MLA_ERR_STATE, "step_append outside step_begin/step_end");
     if (int e = check_layer(c, layer, true)) return e;
-    return run_append(c, layer, kv_a, static_cast<cudaStream_t>(stream));
+    auto st = static_cast<cudaStream_t>(stream);
+    if (int e = step_plan(c, st)) return e;
+    return run_append(c, layer, kv_a, c->plan.m, st);
 }
 
 int mla_step_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, void* stream)
@@ -1047,7 +1030,9 @@ int mla_step_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, void* 
     USE_DEVICE(c);
     if (!c->in_step) return fail(c, MLA_ERR_STATE, "step_attend outside step_begin/step_end");
     if (int e = check_layer(c, layer, true)) return e;
-    return run_attend(c, layer, q, out, nullptr, static_cast<cudaStream_t>(stream));
+    auto st = static_cast<cudaStream_t>(stream);
+    if (int e = step_plan(c, st)) return e;
+    return run_attend(c, layer, q, out, nullptr, c->plan, st);
 }
 
 int mla_step_layers(mla_ctx* c, uint32_t layer_begin, uint32_t n_layers, const void* kv_a, const void* q, void* out,
@@ -1058,11 +1043,30 @@ int mla_step_layers(mla_ctx* c, uint32_t layer_begin, uint32_t n_layers, const v
     if (!c->in_step) return fail(c, MLA_ERR_STATE, "step_layers outside step_begin/step_end");
     if (uint64_t(layer_begin) + n_layers > c->cfg.n_layers) return fail(c, MLA_ERR_INVALID, "layer range out of bounds");
     auto st = static_cast<cudaStream_t>(stream);
-    const size_t rows = c->meta.rows, H = c->cfg.n_heads;
+    const size_t rows = c->step_rows, H = c->cfg.n_heads;
     const size_t kv_b = rows * mla::kRow * 2, q_b = rows * H * mla::kQDim * 2, o_b = rows * H * mla::kVDim * 2;
+    for (uint32_t i = 0; i < n_layers; i++)
+        if (int e = check_layer(c, layer_begin + i, true)) return e;
+    // Layers whose inputs are all at hand need not queue up one behind the other: a group of them is ONE absorb, one
+    // attention and one merge launch, planned together, so that a step of few rows fills the machine.
+    uint32_t group = 1;
+    if (!c->has_chunks && rows && c->kernel != MLA_KERNEL_MMA) group = uint32_t(std::min<uint64_t>(n_layers, c->ws_rows / rows));
+    if (group > 1) {
+        const uint32_t n_groups = (n_layers + group - 1) / group;
+        group = (n_layers + n_groups - 1) / n_groups;
+        for (uint32_t i = 0; i < n_layers; i += group) {
+            const uint32_t n = std::min(group, n_layers - i);
+            Plan& p = n == group ? c->stack : c->stack_tail;
+            if (!p.ready || p.m.layers != n)
+                if (int e = build_plan(c, p, n == group ? kPlanStack : kPlanStackTail, c->step_seqs, c->rows, nullptr, nullptr, n, st)) return e;
+            if (int e = run_attend(c, layer_begin + i, static_cast<const char*>(q) + i * q_b, static_cast<char*>(out) + i * o_b, nullptr, p, st,
+                                   static_cast<const char*>(kv_a) + i * kv_b, i > 0))
+                return e;
+        }
+        return MLA_OK;
+    }
     for (uint32_t i = 0; i < n_layers; i++) {
         const uint32_t layer = layer_begin + i;
-        if (int e = check_layer(c, layer, true)) return e;
         // the caller's kv_a for ALL layers existed before this call: from the second layer on, the kernel ahead of the
         // layer's first launch is this library's own and kv_a was complete before it started
         if (int e = run_layer(c, layer, static_cast<const char*>(kv_a) + i * kv_b, static_cast<const char*>(q) + i * q_b,
@@ -1078,7 +1082,9 @@ int mla_step_attend_partial(mla_ctx* c, uint32_t layer, const void* q, float* pa
     USE_DEVICE(c);
     if (!c->in_step) return fail(c, MLA_ERR_STATE, "step_attend_partial outside step_begin/step_end");
     if (int e = check_layer(c, layer, true)) return e;
-    return run_attend(c, layer, q, nullptr, partial, static_cast<cudaStream_t>(stream));
+    auto st = static_cast<cudaStream_t>(stream);
+    if (int e = step_plan(c, st)) return e;
+    return run_attend(c, layer, q, nullptr, partial, c->plan, st);
 }
 
 int mla_step_layer_partial(mla_ctx* c, uint32_t layer, const void* kv_a, const void* q, float* partial, void* stream)
@@ -1087,15 +1093,12 @@ int mla_step_layer_partial(mla_ctx* c, uint32_t layer, const void* kv_a, const v
     USE_DEVICE(c);
     if (!c->in_step) return fail(c, MLA_ERR_STATE, "step_layer_partial outside step_begin/step_end");
     if (int e = check_layer(c, layer, true)) return e;
-    if (c->has_plan_b) return fail(c, MLA_ERR_UNSUPPORTED, "a step with prefill chunks has no partial form");
+    if (c->has_chunks) return fail(c, MLA_ERR_UNSUPPORTED, "a step with prefill chunks has no partial form");
     if (c->step_new_rows && !kv_a) return fail(c, MLA_ERR_INVALID, "the step appends rows on this GPU: kv_a is needed");
     auto st = static_cast<cudaStream_t>(stream);
     if (!c->step_new_rows) kv_a = nullptr;           // query-only rows: nothing to append, kv_a is never read
-    if (kv_a && !c->layers[layer].has_map) {
-        if (int e = run_append(c, layer, kv_a, st)) return e;
-        kv_a = nullptr;
-    }
-    return run_attend(c, layer, q, nullptr, partial, st, kv_a);
+    if (int e = step_plan(c, st)) return e;
+    return run_attend(c, layer, q, nullptr, partial, c->plan, st, kv_a);
 }
 
 int mla_merge_partials(mla_ctx* c, uint32_t layer, uint32_t n_parts, uint32_t rows, const float* partials,
@@ -1104,8 +1107,12 @@ int mla_merge_partials(mla_ctx* c, uint32_t layer, uint32_t n_parts, uint32_t ro
     if (!c || !partials || !out || n_parts == 0) return fail(c, MLA_ERR_INVALID, "null argument");
     USE_DEVICE(c);
     if (int e = check_layer(c, layer, true)) return e;
-    if (int rc = run_merge(c, layer, partials, nullptr, n_parts, out, nullptr, rows, static_cast<cudaStream_t>(stream)))
-        return rc;
+    mla::StepMeta m{};
+    m.rows = rows;
+    m.layers = 1;
+    const int e = mla::launch_merge_tc5(int(c->cfg.dtype), partials, m, n_parts, &c->w_uv_map, out, c->cfg.n_heads, layer, c->status_dev,
+                                        static_cast<cudaStream_t>(stream));
+    if (e != 0) return fail(c, MLA_ERR_CUDA, std::string("merge launch: ") + cudaGetErrorString(cudaError_t(e)));
     c->launches += rows ? 1 : 0;
     CU_TRY(c, cudaGetLastError());
     return MLA_OK;
@@ -1129,7 +1136,7 @@ int mla_step_layer_host(mla_ctx* c, uint32_t layer, const void* kv_a_host, const
     if (!c->in_step) return fail(c, MLA_ERR_STATE, "step_layer_host outside step_begin/step_end");
     if (int e = check_layer(c, layer, true)) return e;
     auto st = static_cast<cudaStream_t>(stream);
-    const size_t R = c->cfg.max_rows, H = c->cfg.n_heads, rows = c->meta.rows, L = c->cfg.n_layers;
+    const size_t R = c->cfg.max_rows, H = c->cfg.n_heads, rows = c->step_rows, L = c->cfg.n_layers;
     const size_t kv_cap = R * mla::kRow * 2, q_cap = R * H * mla::kQDim * 2, o_cap = R * H * mla::kVDim * 2;
     const size_t kv_b = rows * mla::kRow * 2, q_b = rows * H * mla::kQDim * 2, o_b = rows * H * mla::kVDim * 2;
     if (!c->d_kv) {
@@ -1213,8 +1220,9 @@ int mla_step_end(mla_ctx* c)
 int mla_step_info(const mla_ctx* c, uint32_t* rows, uint32_t* segments)
 {
     if (!c) return MLA_ERR_INVALID;
-    if (rows) *rows = c->meta.rows;
-    if (segments) *segments = c->meta.segs;
+    if (rows) *rows = c->step_rows;
+    // the segments of the step's (or the last explicit call's) one-layer plan, which exists once a layer has been launched
+    if (segments) *segments = c->plan.ready ? c->plan.m.segs : c->plan_rest.ready ? c->plan_rest.m.segs : c->stack.m.segs;
     return MLA_OK;
 }
 
@@ -1340,8 +1348,8 @@ int mla_write_rows(mla_ctx* c, uint32_t layer, uint32_t id, uint32_t row_begin, 
     auto st = static_cast<cudaStream_t>(stream);
     std::vector<uint32_t> seqs{id};
     std::vector<RowSpec> none;
-    if (int e = upload_meta(c, seqs, none, false, st)) return e;
-    mla::launch_write_rows(dev_rows, layer_pool(c, layer), c->pool_slots, c->meta.tables, row_begin, n,
+    if (int e = build_plan(c, c->plan, kPlanStep, seqs, none, nullptr, nullptr, 0, st)) return e;
+    mla::launch_write_rows(dev_rows, layer_pool(c, layer), c->pool_slots, c->plan.m.tables, row_begin, n,
                            c->status_dev, st);
     c->launches += n ? 1 : 0;
     CU_TRY(c, cudaGetLastError());
@@ -1479,7 +1487,7 @@ int mla_step_block(mla_ctx* c, uint32_t layer, void* hidden, void* stream)
     const BlockW* b = nullptr;
     if (int e = block_of(c, layer, &b)) return e;
     auto st = static_cast<cudaStream_t>(stream);
-    const uint32_t rows = c->meta.rows, H = c->cfg.n_heads;
+    const uint32_t rows = c->step_rows, H = c->cfg.n_heads;
     if (rows == 0) return MLA_OK;
     if (int e = grow(c, &c->blk_q, &c->blk_q_cap, size_t(rows) * H * mla::kQDim * 2)) return e;
     if (int e = grow(c, &c->blk_kv, &c->blk_kv_cap, size_t(rows) * mla::kRow * 2)) return e;

@@ -71,29 +71,54 @@ template <> struct Elem<__nv_bfloat16> {
     }
 };
 
-// Per-step metadata resident on the device (one upload per step, shared by all layers).
+// One KV segment of a plan: a run of whole pages of one sequence in one layer, attended by one query group.  A query
+// group is a run of consecutive step rows of the same sequence whose attend lengths grow by one per row (the new tokens
+// of a sequence in a step); its rows' heads lie side by side in the absorbed queries, so the attention kernels see
+// `heads` = rows x n_heads head rows over ONE stream of the pages.  32 bytes, read as two 16-byte loads.
+struct alignas(16) SegDesc {
+    uint32_t q_row;        // first row of the group among the plan's query rows (layer * rows + row)
+    uint32_t tbl;          // index in `tables` of the segment's first page
+    uint32_t n_tok;        // tokens of the segment that the group's LAST row may see (0: an empty segment)
+    uint32_t layer;        // relative to the first layer of the launch
+    int32_t  lim0;         // tokens of the segment that the group's first row may see (may be <= 0); row i: lim0 + i
+    uint32_t heads;        // live head rows of the group
+    uint32_t pad[2];
+};
+static_assert(sizeof(SegDesc) == 32, "read as two 16-byte loads");
+
+__device__ __forceinline__ SegDesc load_seg_desc(const SegDesc* seg) {
+    SegDesc s;
+    const uint4* p = reinterpret_cast<const uint4*>(seg);
+    const uint4 a = __ldg(p), b = __ldg(p + 1);
+    s.q_row = a.x; s.tbl = a.y; s.n_tok = a.z; s.layer = a.w;
+    s.lim0 = int32_t(b.x); s.heads = b.y;
+    return s;
+}
+// tokens of the segment that head row vh of its group may see
+__device__ __forceinline__ int seg_visible(const SegDesc& s, uint32_t vh, uint32_t H) {
+    return min(int(s.n_tok), s.lim0 + int(vh / H));
+}
+
+// Where a query row's partial states are: records (seg * rec_stride + rec_off + head) for seg in [begin, end).
+struct alignas(16) RowParts {
+    uint32_t begin, end, rec_off, pad;
+};
+
+// Metadata of one launch series resident on the device: `layers` consecutive layers of a step, `rows` query rows in each.
 struct StepMeta {
-    // query rows
-    const uint32_t* row_seq;        // [rows]  index into the step's sequence list
-    const uint32_t* row_len;        // [rows]  rows of the sequence this query attends
-    const uint32_t* row_pos;        // [rows]  global position of the appended token (RoPE)
-    const uint64_t* row_slot;       // [rows]  destination token slot of the appended token
-    // block tables
-    const uint32_t* seq_tbl_off;    // [seqs]  offset of the sequence's block table in `tables`
-    const uint32_t* tables;         // physical page ids
-    // split-KV segments
-    const uint32_t* seg_row;        // [segs]
-    const uint32_t* seg_page_begin; // [segs]
-    const uint32_t* seg_page_end;   // [segs]
-    const uint32_t* row_seg_begin;  // [rows+1]  a row's segments are contiguous
+    const SegDesc* seg;             // [segs]
+    const uint32_t* tables;         // physical page ids, sequence after sequence
     const uint32_t* cta_seg_begin;  // [ctas+1]  a persistent block's segments are contiguous
-    uint32_t rows, segs, ctas;
+    const RowParts* parts;          // [layers * rows]
+    const uint32_t* row_pos;        // [rows]  global position of the query row (RoPE)
+    uint32_t rows, layers, segs, ctas;
+    uint32_t rec_stride;            // partial-state records per segment (rows of the largest query group x n_heads)
     // The step's new tokens, in the caller's row order (kv_a rows): what the append writes.  Usually the same rows as
     // the query rows above; a step that routes long chunks to the prefill path keeps them here but not among the
     // query rows, which then carry the index of their row in the caller's q / out tensors.
     uint32_t app_rows;
     const uint32_t* app_pos;        // [app_rows]  global position (RoPE)
-    const uint64_t* app_slot;       // [app_rows]  destination token slot
+    const uint64_t* app_slot;       // [app_rows]  destination token slot (all ones: nothing to append)
     const uint32_t* att_row;        // [rows]  query row -> row of the caller's q / out (nullptr: the same index)
 };
 

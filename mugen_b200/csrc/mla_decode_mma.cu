@@ -81,13 +81,9 @@ decode_mma_kernel(const T* __restrict__ q_abs, const T* __restrict__ pool, uint3
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const uint32_t g = lane / 4, t4 = lane % 4;
 
-    const uint32_t row = m.seg_row[seg];
-    const uint32_t pb = m.seg_page_begin[seg], pe = m.seg_page_end[seg];
-    const uint32_t len = m.row_len[row];
-    const uint32_t* tbl = m.tables + m.seq_tbl_off[m.row_seq[row]];
-    const uint32_t tok_begin = pb * kPage;
-    const uint32_t tok_end = min(len, pe * kPage);
-    const uint32_t n_tok = tok_end > tok_begin ? tok_end - tok_begin : 0;
+    const SegDesc sd = load_seg_desc(m.seg + seg);      // a group of this kernel is always one row
+    const uint32_t row = sd.q_row, n_tok = sd.n_tok;
+    const uint32_t* tbl = m.tables + sd.tbl;
     const uint32_t n_tiles = (n_tok + TT - 1) / TT;
 
     // Q' fragments of this warp's 9 k-steps (A operand, row-major 16 x 16 per step).
@@ -108,7 +104,7 @@ decode_mma_kernel(const T* __restrict__ q_abs, const T* __restrict__ pool, uint3
 
     auto issue_tile = [&](uint32_t tile) {
         if (tile < n_tiles) {
-            const uint32_t tok = tok_begin + tile * TT;
+            const uint32_t tok = tile * TT;
             uint32_t page = tbl[tok / kPage];
             if (page >= n_pages) {
                 if (tid == 0) atomicOr(status, ST_BAD_PAGE);

@@ -65,18 +65,13 @@ enum { B_QFULL = 0, B_QEMPTY, B_KVFULL0, B_KVFULL1, B_KVEMPTY0, B_KVEMPTY1, B_SF
        B_SEMPTY0, B_SEMPTY1, B_PFULL, B_PEMPTY, B_OFULL, B_COUNT };
 
 
-struct SegInfo {
-    uint32_t row, page_begin, n_tiles, n_tok;
+struct SegInfo : SegDesc {
+    uint32_t n_tiles;
 };
 
 __device__ __forceinline__ SegInfo load_seg(const StepMeta& m, uint32_t seg) {
     SegInfo s;
-    s.row = m.seg_row[seg];
-    s.page_begin = m.seg_page_begin[seg];
-    const uint32_t pe = m.seg_page_end[seg];
-    const uint32_t len = m.row_len[s.row];
-    const uint32_t tb = s.page_begin * kPage, te = min(len, pe * kPage);
-    s.n_tok = te > tb ? te - tb : 0;
+    static_cast<SegDesc&>(s) = load_seg_desc(m.seg + seg);
     s.n_tiles = (s.n_tok + TILE - 1) / TILE;
     return s;
 }
@@ -84,7 +79,7 @@ __device__ __forceinline__ SegInfo load_seg(const StepMeta& m, uint32_t seg) {
 template <typename T>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 decode_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_q,
-                  uint32_t layer, uint32_t n_pages, StepMeta m, float* __restrict__ recs, uint32_t H,
+                  uint32_t layer0, uint32_t n_pages, StepMeta m, float* __restrict__ recs, uint32_t H,
                   float scale_log2, uint32_t* __restrict__ status)
 {
     extern __shared__ unsigned char smem_raw[];
@@ -141,25 +136,25 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_const
             bool ok = true;
             for (uint32_t seg = seg_begin; seg < seg_end && ok; seg++) {
                 const SegInfo s = load_seg(m, seg);
-                if (s.n_tiles == 0) continue;
+                if (s.n_tiles == 0 || s.heads <= h0) continue;
                 // Q' of this row's head group: 9 boxes of [64 heads][64 dims]
                 ok = mbar_wait(bar(B_QEMPTY), (nseg & 1) ^ 1, abort_flag, status);
                 if (!ok) break;
                 mbar_expect_tx(bar(B_QFULL), Q_BYTES);
-                tma_load_3d(sQ, &map_q, bar(B_QFULL), 0, int(s.row * H + h0), 0);          // all 9 sub-tiles in one box
-                const uint32_t* tbl = m.tables + m.seq_tbl_off[m.row_seq[s.row]];
+                tma_load_3d(sQ, &map_q, bar(B_QFULL), 0, int(s.q_row * H + h0), 0);          // all 9 sub-tiles in one box
+                const uint32_t* tbl = m.tables + s.tbl;
                 for (uint32_t j = 0; j < s.n_tiles; j++, t++) {
                     const uint32_t st = t % KV_STAGES;
                     ok = mbar_wait(bar(B_KVEMPTY0 + st), ((t / KV_STAGES) & 1) ^ 1, abort_flag, status);
                     if (!ok) break;
-                    uint32_t page = tbl[s.page_begin + j];
+                    uint32_t page = tbl[j];
                     if (page >= n_pages) {
                         atomicOr(status, ST_BAD_PAGE);
                         page = 0;
                     }
                     mbar_expect_tx(bar(B_KVFULL0 + st), KV_STAGE_BYTES);
                     const uint32_t dst = sKV + st * KV_STAGE_BYTES;
-                    tma_load_4d(dst, &map_kv, bar(B_KVFULL0 + st), 0, int(page * kPage), 0, int(layer));   // whole page
+                    tma_load_4d(dst, &map_kv, bar(B_KVFULL0 + st), 0, int(page * kPage), 0, int(layer0 + s.layer));   // whole page
                 }
                 nseg++;
             }
@@ -188,7 +183,7 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_const
         bool ok = true;
         for (uint32_t seg = seg_begin; seg < seg_end && ok; seg++) {
             const SegInfo s = load_seg(m, seg);
-            if (s.n_tiles == 0) continue;
+            if (s.n_tiles == 0 || s.heads <= h0) continue;
             if (is_qk) ok = mbar_wait(bar(B_QFULL), nseg & 1, abort_flag, status);
             for (uint32_t j = 0; j < s.n_tiles && ok; j++, t++) {
                 const uint32_t st = t % KV_STAGES;
@@ -278,12 +273,13 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_const
         bool stop = false;
         for (uint32_t seg = seg_begin; seg < seg_end && !stop; seg++) {
             const SegInfo s = load_seg(m, seg);
+            if (s.heads <= h0) continue;                      // a smaller group than the plan's largest: none of its rows here
             if (s.n_tiles == 0) {
                 // nothing to attend: the state of an empty range
                 const uint32_t st = tid - (NUM_THREADS - SOFTMAX_THREADS);
                 for (uint32_t h = 0; h < HG; h++) {
-                    if (h0 + h >= H) break;
-                    float* rc = recs + (size_t(seg) * H + h0 + h) * kPart;
+                    if (h0 + h >= s.heads) break;
+                    float* rc = recs + (size_t(seg) * m.rec_stride + h0 + h) * kPart;
                     for (uint32_t d = st; d < kRank; d += SOFTMAX_THREADS) rc[2 + d] = 0.0f;
                     if (st == 0) { rc[0] = -INFINITY; rc[1] = 0.0f; }
                 }
@@ -291,6 +287,7 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_const
             }
             m_a = m_b = -INFINITY;
             l_a = l_b = 0.0f;
+            const int lim_a = seg_visible(s, h0 + r_a, H), lim_b = seg_visible(s, h0 + r_b, H);
             for (uint32_t j = 0; j < s.n_tiles; j++, t++) {
                 const uint32_t sb = t & 1;
                 float* alpha_t = alpha_s + sb * HG;
@@ -318,15 +315,15 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_const
 #pragma unroll
                     for (int i = 0; i < 32; i++) sv[i] = 0u;
                 }
-                const uint32_t valid = min(uint32_t(TILE), s.n_tok - j * TILE);
+                const int valid_a = lim_a - int(j * TILE), valid_b = lim_b - int(j * TILE);
                 float mx_a = -INFINITY, mx_b = -INFINITY;
 #pragma unroll
                 for (int k = 0; k < 8; k++) {
 #pragma unroll
                     for (int e = 0; e < 2; e++) {
-                        const bool in = uint32_t(8 * k + 2 * qd + e) < valid;
-                        const float va = in ? __uint_as_float(sv[4 * k + e]) * scale_log2 : -INFINITY;
-                        const float vb = in ? __uint_as_float(sv[4 * k + 2 + e]) * scale_log2 : -INFINITY;
+                        const int tok = int(8 * k + 2 * qd + e);
+                        const float va = tok < valid_a ? __uint_as_float(sv[4 * k + e]) * scale_log2 : -INFINITY;
+                        const float vb = tok < valid_b ? __uint_as_float(sv[4 * k + 2 + e]) * scale_log2 : -INFINITY;
                         sv[4 * k + e] = __float_as_uint(va);
                         sv[4 * k + 2 + e] = __float_as_uint(vb);
                         mx_a = fmaxf(mx_a, va);
@@ -351,14 +348,16 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_const
                 // one barrier on the common path; a second one only to tell failure from rescale
                 bool any_need = group_or(need || fail);
                 if (any_need && group_or(fail)) { stop = true; break; }
+                // a row that has seen no token yet (a segment that only later rows of its group reach): p = 0
+                const float ma = m_a == -INFINITY ? 0.0f : m_a, mb = m_b == -INFINITY ? 0.0f : m_b;
                 float sum_a = 0.0f, sum_b = 0.0f;
                 uint32_t pk_a[8], pk_b[8];
 #pragma unroll
                 for (int k = 0; k < 8; k++) {
-                    const float a0 = fast_ex2(__uint_as_float(sv[4 * k]) - m_a);
-                    const float a1 = fast_ex2(__uint_as_float(sv[4 * k + 1]) - m_a);
-                    const float b0 = fast_ex2(__uint_as_float(sv[4 * k + 2]) - m_b);
-                    const float b1 = fast_ex2(__uint_as_float(sv[4 * k + 3]) - m_b);
+                    const float a0 = fast_ex2(__uint_as_float(sv[4 * k]) - ma);
+                    const float a1 = fast_ex2(__uint_as_float(sv[4 * k + 1]) - ma);
+                    const float b0 = fast_ex2(__uint_as_float(sv[4 * k + 2]) - mb);
+                    const float b1 = fast_ex2(__uint_as_float(sv[4 * k + 3]) - mb);
                     sum_a += a0 + a1;
                     sum_b += b0 + b1;
                     pk_a[k] = Elem<T>::pack2(a0, a1);
@@ -414,17 +413,17 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_const
                 const uint32_t hb = h0 + (c & 1) * 32;
 #pragma unroll
                 for (int i = 0; i < 32; i++) {
-                    if (hb + i < H) recs[(size_t(seg) * H + hb + i) * kPart + 2 + dim] = __uint_as_float(o[i]);
+                    if (hb + i < s.heads) recs[(size_t(seg) * m.rec_stride + hb + i) * kPart + 2 + dim] = __uint_as_float(o[i]);
                 }
             }
             if (qd == 0) {
-                if (h0 + r_a < H) {
-                    float* rc = recs + (size_t(seg) * H + h0 + r_a) * kPart;
+                if (h0 + r_a < s.heads) {
+                    float* rc = recs + (size_t(seg) * m.rec_stride + h0 + r_a) * kPart;
                     rc[0] = m_a;
                     rc[1] = l_a;
                 }
-                if (h0 + r_b < H) {
-                    float* rc = recs + (size_t(seg) * H + h0 + r_b) * kPart;
+                if (h0 + r_b < s.heads) {
+                    float* rc = recs + (size_t(seg) * m.rec_stride + h0 + r_b) * kPart;
                     rc[0] = m_b;
                     rc[1] = l_b;
                 }
@@ -454,18 +453,18 @@ int decode_tc5_configure()
     return int(e);
 }
 
-int launch_decode_tc5(int dtype, const void* tmaps, uint32_t layer, uint32_t n_pages, const StepMeta& m, float* recs,
+int launch_decode_tc5(int dtype, const void* tmaps, uint32_t layer0, uint32_t n_pages, const StepMeta& m, float* recs,
                       uint32_t H, uint32_t* status, cudaStream_t st)
 {
     if (m.ctas == 0) return 0;
     const CUtensorMap* maps = static_cast<const CUtensorMap*>(tmaps);
     const float scale_log2 = 1.4426950408889634f / sqrtf(float(kQDim));
-    dim3 grid(m.ctas, (H + HG - 1) / HG);
+    dim3 grid(m.ctas, (m.rec_stride + HG - 1) / HG);
     if (dtype == 0)
         return int(launch_pdl(decode_tc5_kernel<__half>, grid, dim3(NUM_THREADS), SMEM_BYTES, st, maps[kMapPoolPage], maps[kMapQueries],
-                              layer, n_pages, m, recs, H, scale_log2, status));
+                              layer0, n_pages, m, recs, H, scale_log2, status));
     return int(launch_pdl(decode_tc5_kernel<__nv_bfloat16>, grid, dim3(NUM_THREADS), SMEM_BYTES, st, maps[kMapPoolPage],
-                          maps[kMapQueries], layer, n_pages, m, recs, H, scale_log2, status));
+                          maps[kMapQueries], layer0, n_pages, m, recs, H, scale_log2, status));
 }
 
 }  // namespace mla

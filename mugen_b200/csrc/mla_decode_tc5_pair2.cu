@@ -98,17 +98,12 @@ enum { B_QFULL = 0, B_QEMPTY, B_KFULL, B_KEMPTY = B_KFULL + NSUB, B_VFULL = B_KE
 static_assert(B_COUNT * 8 <= M_TMEM, "barriers overflow their area");
 
 
-struct SegInfo {
-    uint32_t row, page_begin, n_pages, n_tiles, n_tok;
+struct SegInfo : SegDesc {
+    uint32_t n_pages, n_tiles;
 };
 __device__ __forceinline__ SegInfo load_seg(const StepMeta& m, uint32_t seg) {
     SegInfo s;
-    s.row = m.seg_row[seg];
-    s.page_begin = m.seg_page_begin[seg];
-    const uint32_t pe = m.seg_page_end[seg];
-    const uint32_t len = m.row_len[s.row];
-    const uint32_t tb = s.page_begin * kPage, te = min(len, pe * kPage);
-    s.n_tok = te > tb ? te - tb : 0;
+    static_cast<SegDesc&>(s) = load_seg_desc(m.seg + seg);
     s.n_pages = (s.n_tok + kPage - 1) / kPage;
     s.n_tiles = (s.n_pages + PAGES - 1) / PAGES;      // super-tiles
     return s;
@@ -117,8 +112,8 @@ __device__ __forceinline__ SegInfo load_seg(const StepMeta& m, uint32_t seg) {
 template <typename T>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __grid_constant__ CUtensorMap map_kv64,
-                          const __grid_constant__ CUtensorMap map_q, const unsigned char* __restrict__ pool_layer,
-                          uint32_t layer, uint32_t n_pages, StepMeta m, float* __restrict__ recs, uint32_t H,
+                          const __grid_constant__ CUtensorMap map_q, const unsigned char* __restrict__ pool,
+                          uint32_t layer0, uint32_t n_pages, StepMeta m, float* __restrict__ recs, uint32_t H,
                           float scale_log2, uint32_t prefetch_tiles, const unsigned char* __restrict__ next_weights,
                           uint32_t next_weights_bytes, uint32_t* __restrict__ status)
 {
@@ -186,14 +181,14 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     // The step's metadata was uploaded by a copy that the stream ordered before the step's first kernel, so it may be
-    // read ahead of the wait: the chain of dependent loads that describes the first segment (segment -> row -> table
-    // offset -> page ids) then overlaps the previous kernel's tail instead of delaying the first TMA.
+    // read ahead of the wait: the dependent loads that describe the first segment (descriptor -> page ids) then overlap
+    // the previous kernel's tail instead of delaying the first TMA.
     SegInfo seg0{};
     const uint32_t* tbl0 = nullptr;
     uint32_t page0[PAGES] = {0, 0};
     if (seg_begin < seg_end) {
         seg0 = load_seg(m, seg_begin);
-        tbl0 = m.tables + m.seq_tbl_off[m.row_seq[seg0.row]] + seg0.page_begin;
+        tbl0 = m.tables + seg0.tbl;
         if (seg0.n_tiles) {
 #pragma unroll
             for (int r = 0; r < PAGES; r++) page0[r] = tbl0[min(uint32_t(r), seg0.n_pages - 1)];
@@ -201,14 +196,17 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
     }
     auto seg_info = [&](uint32_t seg) -> SegInfo { return seg == seg_begin ? seg0 : load_seg(m, seg); };
     auto seg_table = [&](uint32_t seg, const SegInfo& si) -> const uint32_t* {
-        return seg == seg_begin ? tbl0 : m.tables + m.seq_tbl_off[m.row_seq[si.row]] + si.page_begin;
+        return seg == seg_begin ? tbl0 : m.tables + si.tbl;
+    };
+    auto page_ptr = [&](const SegInfo& si, uint32_t page) -> const unsigned char* {
+        return pool + (size_t(layer0 + si.layer) * n_pages + page) * (kPage * kRow * 2);
     };
     // L2 is the point of coherence, so pulling cache lines towards it ahead of the wait is safe even for the page
     // that the append of this layer-step is still writing: the first tiles' loads then find their pages in L2.
     if (warp == N_QK + N_PV + 1 && lane == 0 && seg_begin < seg_end) {
         for (uint32_t jj = 0; jj < min(2u, seg0.n_tiles); jj++) {
             const uint32_t pgid = tbl0[min(PAGES * jj + rank, seg0.n_pages - 1)];
-            if (pgid < n_pages) bulk_prefetch_l2(pool_layer + size_t(pgid) * (kPage * kRow * 2), kPage * kRow * 2);
+            if (pgid < n_pages) bulk_prefetch_l2(page_ptr(seg0, pgid), kPage * kRow * 2);
         }
     }
     grid_dependency_wait();          // queries, new cache rows and the state records belong to earlier kernels until here
@@ -231,12 +229,12 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
             bool ok = true;
             for (uint32_t seg = seg_begin; seg < seg_end && ok; seg++) {
                 const SegInfo s = seg_info(seg);
-                if (s.n_tiles == 0) continue;
+                if (s.n_tiles == 0 || s.heads <= hpair) continue;
                 const uint32_t* tbl = seg_table(seg, s);
                 ok = mbar_wait<kSleep>(bar(B_QEMPTY), (nseg & 1) ^ 1, abort_flag, status);
                 if (!ok) break;
                 if (rank == 0) mbar_expect_tx(bar(B_QFULL), 2 * Q_BYTES);
-                tma_load_3d_pair(sQ, &map_q, leader_qfull, 0, int(s.row * H + h0), 0);      // all 9 sub-tiles at once
+                tma_load_3d_pair(sQ, &map_q, leader_qfull, 0, int(s.q_row * H + h0), 0);      // all 9 sub-tiles at once
                 for (uint32_t j = 0; j < s.n_tiles && ok; j++, t++) {
                     uint32_t page = page_of(tbl, s, j, rank);
                     if (page >= n_pages) {
@@ -254,7 +252,7 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
 #pragma unroll 1
                         for (int c = N_QK * rd; c < min(N_QK * (rd + 1), NSUB); c++) {
                             if (rank == 0) mbar_expect_tx(bar(B_KFULL + c), 2 * SUB_BYTES);
-                            tma_load_3d_pair(sK + c * SUB_BYTES, &map_sub, leader_kfull + 8 * c, 64 * c, slot0, int(layer));
+                            tma_load_3d_pair(sK + c * SUB_BYTES, &map_sub, leader_kfull + 8 * c, 64 * c, slot0, int(layer0 + s.layer));
                         }
                     }
                 }
@@ -269,17 +267,17 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
             bool ok = true;
             for (uint32_t seg = seg_begin; seg < seg_end && ok; seg++) {
                 const SegInfo s = seg_info(seg);
-                if (s.n_tiles == 0) continue;
+                if (s.n_tiles == 0 || s.heads <= hpair) continue;
                 const uint32_t* tbl = seg_table(seg, s);
                 // tile 0 is demand-loaded right now; tiles 1 .. prefetch_tiles-1 have no earlier tile to ride on
                 for (uint32_t jj = 1; jj < min(prefetch_tiles, s.n_tiles); jj++) {
                     const uint32_t pgid = page_of(tbl, s, jj, rank);
-                    if (pgid < n_pages) bulk_prefetch_l2(pool_layer + size_t(pgid) * (kPage * kRow * 2), kPage * kRow * 2);
+                    if (pgid < n_pages) bulk_prefetch_l2(page_ptr(s, pgid), kPage * kRow * 2);
                 }
                 for (uint32_t j = 0; j < s.n_tiles && ok; j++, t++) {
                     if (prefetch_tiles > 0 && j + prefetch_tiles < s.n_tiles) {
                         const uint32_t pgid = page_of(tbl, s, j + prefetch_tiles, rank);
-                        if (pgid < n_pages) bulk_prefetch_l2(pool_layer + size_t(pgid) * (kPage * kRow * 2), kPage * kRow * 2);
+                        if (pgid < n_pages) bulk_prefetch_l2(page_ptr(s, pgid), kPage * kRow * 2);
                     }
 #pragma unroll 1
                     for (uint32_t pg = 0; pg < uint32_t(PAGES) && ok; pg++) {     // both chunk issuers release a page together
@@ -293,7 +291,7 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                             if (rank == 0) mbar_expect_tx(bar(B_VFULL + v), 2 * VBUF_BYTES);
                             // all 64 tokens of the page, this block's 128 dims of chunk ch = sub-tiles 4*ch + 2r, +1
                             tma_load_4d_pair(sV + v * VBUF_BYTES, &map_kv64, leader_vfull + 8 * v, 0, int(page * kPage),
-                                             4 * int(ch) + 2 * int(rank), int(layer));
+                                             4 * int(ch) + 2 * int(rank), int(layer0 + s.layer));
                         }
                     }
                 }
@@ -323,7 +321,7 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
             bool ok = true;
             for (uint32_t seg = seg_begin; seg < seg_end && ok; seg++) {
                 const SegInfo s = seg_info(seg);
-                if (s.n_tiles == 0) continue;
+                if (s.n_tiles == 0 || s.heads <= hpair) continue;
                 if (is_qk) ok = mbar_wait<kSleepCluster>(bar(B_QFULL), nseg & 1, abort_flag, status);
                 for (uint32_t j = 0; j < s.n_tiles && ok; j++, t++) {
                     if (is_qk) {
@@ -421,11 +419,12 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
         bool stop = false;
         for (uint32_t seg = seg_begin; seg < seg_end && !stop; seg++) {
             const SegInfo s = seg_info(seg);
+            if (s.heads <= hpair) continue;                   // a smaller group than the plan's largest: none of its rows here
             if (s.n_tiles == 0) {
                 // nothing to attend: each block writes its 256 dims of every head, and (m, l) of its own heads
                 for (uint32_t h = 0; h < 2 * HG; h++) {
-                    if (hpair + h >= H) break;
-                    float* rc = recs + (size_t(seg) * H + hpair + h) * kPart;
+                    if (hpair + h >= s.heads) break;
+                    float* rc = recs + (size_t(seg) * m.rec_stride + hpair + h) * kPart;
                     const uint32_t dim = (st_id / 128) * 256 + rank * 128 + (st_id % 128);
                     rc[2 + dim] = 0.0f;
                     if (st_id == 0 && h / HG == rank) { rc[0] = -INFINITY; rc[1] = 0.0f; }
@@ -434,6 +433,7 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
             }
             m_used = -INFINITY;
             l_part = 0.0f;
+            const int lim = seg_visible(s, h0 + hl, H);
             for (uint32_t j = 0; j < s.n_tiles; j++, t++) {
                 const uint32_t par = t & 1;
                 wait_w(bar(B_SFULL), t & 1);
@@ -468,11 +468,11 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                 }
                 // Scores stay unscaled in registers: the scale rides in the FMA in front of each exponential, and
                 // the mask pass runs only on a segment's last, partly filled tile.
-                const uint32_t valid = min(uint32_t(TILE), s.n_tok - j * TILE);
-                if (valid < uint32_t(TILE)) {
+                const int valid = lim - int(j * TILE);
+                if (valid < TILE) {
 #pragma unroll
                     for (int i = 0; i < 32; i++)
-                        if (tq * 32 + uint32_t(i) >= valid) sv[i] = __float_as_uint(-INFINITY);
+                        if (int(tq * 32) + i >= valid) sv[i] = __float_as_uint(-INFINITY);
                 }
                 float mx = -INFINITY;
 #pragma unroll
@@ -502,14 +502,16 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                         mbar_arrive_cluster_relaxed(r_synca[par]);
                     }
                 }
+                // a row that has seen no token yet (a segment that only later rows of its group reach): p = 0
+                float m_eff = m_used == -INFINITY ? 0.0f : m_used;
                 // optimistic: exponentials against the current maximum while the cluster round is in
                 // flight; they stand unless some head of the pair raised the flag
                 float sum = 0.0f;
                 uint32_t pk[16];
 #pragma unroll
                 for (int i = 0; i < 32; i += 2) {
-                    const float p0 = fast_ex2(fmaf(__uint_as_float(sv[i]), scale_log2, -m_used));
-                    const float p1 = fast_ex2(fmaf(__uint_as_float(sv[i + 1]), scale_log2, -m_used));
+                    const float p0 = fast_ex2(fmaf(__uint_as_float(sv[i]), scale_log2, -m_eff));
+                    const float p1 = fast_ex2(fmaf(__uint_as_float(sv[i + 1]), scale_log2, -m_eff));
                     sum += p0 + p1;
                     pk[i / 2] = Elem<T>::pack2(p0, p1);
                 }
@@ -541,11 +543,12 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                     wait_x(bar(B_SYNCB0 + par), nb[par] & 1);
                     nb[par]++;
                     l_part *= alpha;
+                    m_eff = m_used == -INFINITY ? 0.0f : m_used;
                     sum = 0.0f;
 #pragma unroll
                     for (int i = 0; i < 32; i += 2) {
-                        const float p0 = fast_ex2(fmaf(__uint_as_float(sv[i]), scale_log2, -m_used));
-                        const float p1 = fast_ex2(fmaf(__uint_as_float(sv[i + 1]), scale_log2, -m_used));
+                        const float p0 = fast_ex2(fmaf(__uint_as_float(sv[i]), scale_log2, -m_eff));
+                        const float p1 = fast_ex2(fmaf(__uint_as_float(sv[i + 1]), scale_log2, -m_eff));
                         sum += p0 + p1;
                         pk[i / 2] = Elem<T>::pack2(p0, p1);
                     }
@@ -606,11 +609,11 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                 const uint32_t hb = hpair + c * 32;
 #pragma unroll
                 for (int i = 0; i < 32; i++) {
-                    if (hb + i < H) recs[(size_t(seg) * H + hb + i) * kPart + 2 + dim] = __uint_as_float(o[i]);
+                    if (hb + i < s.heads) recs[(size_t(seg) * m.rec_stride + hb + i) * kPart + 2 + dim] = __uint_as_float(o[i]);
                 }
             }
-            if (tq == 0 && h0 + hl < H) {
-                float* rc = recs + (size_t(seg) * H + h0 + hl) * kPart;
+            if (tq == 0 && h0 + hl < s.heads) {
+                float* rc = recs + (size_t(seg) * m.rec_stride + h0 + hl) * kPart;
                 rc[0] = m_used;
                 rc[1] = l_part + l_other[hl] + l_other[HG + hl] + l_other[2 * HG + hl];
             }
@@ -649,21 +652,21 @@ int decode_tc5_pair128_configure()
 }
 
 // tmaps: the context's tensor-map array (kMapPoolSub = one K sub-tile, kMapPoolV = V boxes, kMapQueries = Q').
-// layer_pool: the layer's slice of the cache pool (linear L2 prefetch).
-int launch_decode_tc5_pair128(int dtype, const void* tmaps, const void* layer_pool, uint32_t layer, uint32_t n_pages,
+// pool: the whole cache pool (linear L2 prefetch).
+int launch_decode_tc5_pair128(int dtype, const void* tmaps, const void* pool, uint32_t layer0, uint32_t n_pages,
                               const StepMeta& m, float* recs, uint32_t H, uint32_t prefetch_tiles, const void* next_weights,
                               uint32_t next_weights_bytes, uint32_t* status, cudaStream_t st)
 {
     if (m.ctas == 0) return 0;
     const CUtensorMap* maps = static_cast<const CUtensorMap*>(tmaps);
     const float scale_log2 = 1.4426950408889634f / sqrtf(float(kQDim));
-    dim3 grid(2 * m.ctas, (H + 2 * HG - 1) / (2 * HG));          // clusters of 2 along x
+    dim3 grid(2 * m.ctas, (m.rec_stride + 2 * HG - 1) / (2 * HG));          // clusters of 2 along x
     if (dtype == 0)
         return int(launch_pdl(decode_tc5_pair128_kernel<__half>, grid, dim3(NUM_THREADS), SMEM_BYTES, st, maps[kMapPoolSub], maps[kMapPoolV], maps[kMapQueries],
-                              static_cast<const unsigned char*>(layer_pool), layer, n_pages, m, recs, H, scale_log2, prefetch_tiles,
+                              static_cast<const unsigned char*>(pool), layer0, n_pages, m, recs, H, scale_log2, prefetch_tiles,
                               static_cast<const unsigned char*>(next_weights), next_weights_bytes, status));
     return int(launch_pdl(decode_tc5_pair128_kernel<__nv_bfloat16>, grid, dim3(NUM_THREADS), SMEM_BYTES, st, maps[kMapPoolSub], maps[kMapPoolV],
-                          maps[kMapQueries], static_cast<const unsigned char*>(layer_pool), layer, n_pages, m, recs, H, scale_log2, prefetch_tiles,
+                          maps[kMapQueries], static_cast<const unsigned char*>(pool), layer0, n_pages, m, recs, H, scale_log2, prefetch_tiles,
                               static_cast<const unsigned char*>(next_weights), next_weights_bytes, status));
 }
 

@@ -80,18 +80,13 @@ static_assert(N_QK == 4 && N_PV == 2, "the split of a page over the issuers belo
 static_assert(B_COUNT * 8 <= M_TMEM, "barriers overflow their area");
 
 
-struct SegInfo {
-    uint32_t row, page_begin, n_tiles, n_tok;
+struct SegInfo : SegDesc {
+    uint32_t n_tiles;
 };
 
 __device__ __forceinline__ SegInfo load_seg(const StepMeta& m, uint32_t seg) {
     SegInfo s;
-    s.row = m.seg_row[seg];
-    s.page_begin = m.seg_page_begin[seg];
-    const uint32_t pe = m.seg_page_end[seg];
-    const uint32_t len = m.row_len[s.row];
-    const uint32_t tb = s.page_begin * kPage, te = min(len, pe * kPage);
-    s.n_tok = te > tb ? te - tb : 0;
+    static_cast<SegDesc&>(s) = load_seg_desc(m.seg + seg);
     s.n_tiles = (s.n_tok + TILE - 1) / TILE;
     return s;
 }
@@ -100,7 +95,7 @@ template <typename T>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 decode_tc5_t16_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid_constant__ CUtensorMap map_sub,
                       const __grid_constant__ CUtensorMap map_q,
-                  uint32_t layer, uint32_t n_pages, StepMeta m, float* __restrict__ recs, uint32_t H,
+                  uint32_t layer0, uint32_t n_pages, StepMeta m, float* __restrict__ recs, uint32_t H,
                   float scale_log2, uint32_t* __restrict__ status)
 {
     extern __shared__ unsigned char smem_raw[];
@@ -156,15 +151,15 @@ decode_tc5_t16_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid
             bool ok = true;
             for (uint32_t seg = seg_begin; seg < seg_end && ok; seg++) {
                 const SegInfo s = load_seg(m, seg);
-                if (s.n_tiles == 0) continue;
+                if (s.n_tiles == 0 || s.heads <= h0) continue;
                 // Q' of this row's head group: 9 sub-tiles of [16 heads][64 dims] in one box
                 ok = mbar_wait(bar(B_QEMPTY), (nseg & 1) ^ 1, abort_flag, status);
                 if (!ok) break;
                 mbar_expect_tx(bar(B_QFULL), Q_BYTES);
-                tma_load_3d(sQ, &map_q, bar(B_QFULL), 0, int(s.row * H + h0), 0);          // all 9 sub-tiles in one box
-                const uint32_t* tbl = m.tables + m.seq_tbl_off[m.row_seq[s.row]];
+                tma_load_3d(sQ, &map_q, bar(B_QFULL), 0, int(s.q_row * H + h0), 0);          // all 9 sub-tiles in one box
+                const uint32_t* tbl = m.tables + s.tbl;
                 for (uint32_t j = 0; j < s.n_tiles && ok; j++, t++) {
-                    uint32_t page = tbl[s.page_begin + j];
+                    uint32_t page = tbl[j];
                     if (page >= n_pages) {
                         atomicOr(status, ST_BAD_PAGE);
                         page = 0;
@@ -175,14 +170,14 @@ decode_tc5_t16_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid
                         ok = mbar_wait(bar(B_KE + slot), ((u / N_PAIR_SLOTS) & 1) ^ 1, abort_flag, status);
                         if (!ok) break;
                         mbar_expect_tx(bar(B_KF + slot), PAIR_BYTES);
-                        tma_load_4d(sPairs + slot * PAIR_BYTES, &map_pair, bar(B_KF + slot), 0, int(page * kPage), int(2 * i), int(layer));
+                        tma_load_4d(sPairs + slot * PAIR_BYTES, &map_pair, bar(B_KF + slot), 0, int(page * kPage), int(2 * i), int(layer0 + s.layer));
                     }
                     if (!ok) break;
                     const uint32_t rs = t % N_ROPE_SLOTS;
                     ok = mbar_wait(bar(B_RE + rs), ((t / N_ROPE_SLOTS) & 1) ^ 1, abort_flag, status);
                     if (!ok) break;
                     mbar_expect_tx(bar(B_RF + rs), SUB_BYTES);
-                    tma_load_3d(sRope + rs * SUB_BYTES, &map_sub, bar(B_RF + rs), kRank, int(page * kPage), int(layer));
+                    tma_load_3d(sRope + rs * SUB_BYTES, &map_sub, bar(B_RF + rs), kRank, int(page * kPage), int(layer0 + s.layer));
                 }
                 nseg++;
             }
@@ -207,7 +202,7 @@ decode_tc5_t16_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid
         bool ok = true;
         for (uint32_t seg = seg_begin; seg < seg_end && ok; seg++) {
             const SegInfo s = load_seg(m, seg);
-            if (s.n_tiles == 0) continue;
+            if (s.n_tiles == 0 || s.heads <= h0) continue;
             if (is_qk) ok = mbar_wait(bar(B_QFULL), nseg & 1, abort_flag, status);
             for (uint32_t j = 0; j < s.n_tiles && ok; j++, t++) {
                 if (is_qk) {
@@ -276,6 +271,7 @@ decode_tc5_t16_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid
         const uint32_t qd = lane & 3, tr = lane >> 2;         // head quad, token row within the warp's 16 (and + 8)
         auto head_of = [&](int j) { return uint32_t(8 * (j >> 1) + 2 * qd + (j & 1)); };   // this thread's four heads
         float m_ref[4], psum[4];
+        int lim[4];                                           // tokens of the segment that each of the four heads may see
         uint32_t t = 0, nseg = 0;
         bool fail = false;
         auto wait_w = [&](uint32_t b, uint32_t parity) {      // warp-uniform bounded wait
@@ -305,19 +301,24 @@ decode_tc5_t16_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid
         bool stop = false;
         for (uint32_t seg = seg_begin; seg < seg_end && !stop; seg++) {
             const SegInfo s = load_seg(m, seg);
+            if (s.heads <= h0) continue;                      // a smaller group than the plan's largest: none of its rows here
             if (s.n_tiles == 0) {
                 // nothing to attend: the state of an empty range
                 const uint32_t st = tid - (NUM_THREADS - SOFTMAX_THREADS);
                 for (uint32_t h = 0; h < HG; h++) {
-                    if (h0 + h >= H) break;
-                    float* rc = recs + (size_t(seg) * H + h0 + h) * kPart;
+                    if (h0 + h >= s.heads) break;
+                    float* rc = recs + (size_t(seg) * m.rec_stride + h0 + h) * kPart;
                     for (uint32_t d = st; d < kRank; d += SOFTMAX_THREADS) rc[2 + d] = 0.0f;
                     if (st == 0) { rc[0] = -INFINITY; rc[1] = 0.0f; }
                 }
                 continue;
             }
 #pragma unroll
-            for (int j = 0; j < 4; j++) { m_ref[j] = -INFINITY; psum[j] = 0.0f; }
+            for (int j = 0; j < 4; j++) {
+                m_ref[j] = -INFINITY;
+                psum[j] = 0.0f;
+                lim[j] = seg_visible(s, h0 + head_of(j), H);
+            }
             for (uint32_t j = 0; j < s.n_tiles; j++, t++) {
                 wait_w(bar(B_SFULL0), t & 1);
                 float sv[8];
@@ -339,15 +340,14 @@ decode_tc5_t16_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid
                     for (int i = 0; i < 8; i++) sv[i] = 0.0f;
                 }
                 // registers: i = 4k + 2e' + e -> head 8k + 2qd + e, token 16 q4 + tr + 8 e'
-                const uint32_t valid = min(uint32_t(TILE), s.n_tok - j * TILE);
                 const uint32_t tok_a = 16 * q4 + tr, tok_b = tok_a + 8;
-                const bool in_a = tok_a < valid, in_b = tok_b < valid;
                 float mx[4];
 #pragma unroll
                 for (int jj = 0; jj < 4; jj++) {
                     const int k = jj >> 1, e = jj & 1;
-                    const float va = in_a ? sv[4 * k + e] * scale_log2 : -INFINITY;
-                    const float vb = in_b ? sv[4 * k + 2 + e] * scale_log2 : -INFINITY;
+                    const int valid = lim[jj] - int(j * TILE);
+                    const float va = int(tok_a) < valid ? sv[4 * k + e] * scale_log2 : -INFINITY;
+                    const float vb = int(tok_b) < valid ? sv[4 * k + 2 + e] * scale_log2 : -INFINITY;
                     sv[4 * k + e] = va;
                     sv[4 * k + 2 + e] = vb;
                     mx[jj] = rows_max(fmaxf(va, vb));
@@ -437,15 +437,15 @@ decode_tc5_t16_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid
                 const uint32_t dim = c * 128 + q4 * 32 + lane;
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
-                    if (h0 + i < H) recs[(size_t(seg) * H + h0 + i) * kPart + 2 + dim] = __uint_as_float(o[i]);
+                    if (h0 + i < s.heads) recs[(size_t(seg) * m.rec_stride + h0 + i) * kPart + 2 + dim] = __uint_as_float(o[i]);
                 }
             }
             if (q4 == 0 && tr == 0) {
 #pragma unroll
                 for (int jj = 0; jj < 4; jj++) {
                     const uint32_t h = head_of(jj);
-                    if (h0 + h < H) {
-                        float* rc = recs + (size_t(seg) * H + h0 + h) * kPart;
+                    if (h0 + h < s.heads) {
+                        float* rc = recs + (size_t(seg) * m.rec_stride + h0 + h) * kPart;
                         rc[0] = m_ref[jj];
                         rc[1] = (lsum_s[h] + lsum_s[16 + h]) + (lsum_s[32 + h] + lsum_s[48 + h]);
                     }
@@ -478,18 +478,18 @@ int decode_tc5_t16_configure()
     return int(e);
 }
 
-int launch_decode_tc5_t16(int dtype, const void* tmaps, uint32_t layer, uint32_t n_pages, const StepMeta& m, float* recs,
+int launch_decode_tc5_t16(int dtype, const void* tmaps, uint32_t layer0, uint32_t n_pages, const StepMeta& m, float* recs,
                       uint32_t H, uint32_t* status, cudaStream_t st)
 {
     if (m.ctas == 0) return 0;
     const CUtensorMap* maps = static_cast<const CUtensorMap*>(tmaps);
     const float scale_log2 = 1.4426950408889634f / sqrtf(float(kQDim));
-    dim3 grid(m.ctas, (H + HG - 1) / HG);
+    dim3 grid(m.ctas, (m.rec_stride + HG - 1) / HG);
     if (dtype == 0)
         return int(launch_pdl(decode_tc5_t16_kernel<__half>, grid, dim3(NUM_THREADS), SMEM_BYTES, st, maps[kMapPoolV], maps[kMapPoolSub],
-                              maps[kMapQueries16], layer, n_pages, m, recs, H, scale_log2, status));
+                              maps[kMapQueries16], layer0, n_pages, m, recs, H, scale_log2, status));
     return int(launch_pdl(decode_tc5_t16_kernel<__nv_bfloat16>, grid, dim3(NUM_THREADS), SMEM_BYTES, st, maps[kMapPoolV],
-                          maps[kMapPoolSub], maps[kMapQueries16], layer, n_pages, m, recs, H, scale_log2, status));
+                          maps[kMapPoolSub], maps[kMapQueries16], layer0, n_pages, m, recs, H, scale_log2, status));
 }
 
 }  // namespace mla

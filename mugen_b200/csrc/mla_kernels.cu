@@ -1,5 +1,4 @@
-// Small kernels around the attention core: latent-row append, q absorption, partial merge +
-// W_UV projection, bulk row copy.  sm_100a.
+// Small kernels around the attention core: latent-row append, partial merge + W_UV projection, bulk row copy.  sm_100a.
 #include "mla_launch.h"
 
 namespace mla {
@@ -119,12 +118,6 @@ void launch_write_rows(const void* src, void* layer_pool, uint64_t pool_slots, c
                                                     table, row_begin, n, status);
 }
 
-// ------------------------------------------------------------------------------------------
-// q absorption (reference: transformer.cpp:2563-2573):
-//   q_abs[r][h][d] = sum_{i<128} q[r][h][i] * W_UK[h*128+i][d],   d < 512
-// and q_rope copied behind it, so that a query row has the layout of a cache row
-// (512 latent dims, then 64 rope dims) and the score is one 576-long dot product.
-// ------------------------------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1);
 template <>
@@ -140,93 +133,12 @@ __device__ __forceinline__ void mma16816<__nv_bfloat16>(float (&c)[4], const uin
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// Block = (head, quarter of the 512 output columns, group of up to 8 row tiles of 16 query rows);
-// C[16 x 128] = q_nope[16 x 128] . W_UK_h[128 x 128 cols] per row tile on the warp-level tensor path
-// (m16n8k16, f32 accumulate).  The weight is read from its transposed copy W_UK^T[h][d][i] (made
-// once at registration), so B fragments are 16-byte loads with the contraction index contiguous;
-// a warp loads the fragments of its 32 output columns ONCE and reuses them for every row tile of
-// the block, so W_UK crosses L2 once per 128 query rows.
-// 16-byte operand loads: within each block of 32 contraction indices, thread t4 takes indices
-// 8*t4 .. 8*t4+7 of its row, for A and for B alike.  The pairs (0,1),(2,3) feed one MMA as
-// (k, k+8) and (4,5),(6,7) the next: a fixed permutation of the contraction index applied to both
-// operands, which leaves the product unchanged.
-constexpr int kAbsorbTilesPerBlock = 8;
-template <typename T>
-__global__ void __launch_bounds__(128)
-absorb_kernel(const T* __restrict__ q, const T* __restrict__ w_uk_t, T* __restrict__ q_abs,
-              uint32_t rows, uint32_t H)
-{
-    const uint32_t h = blockIdx.x, nq = blockIdx.z, tid = threadIdx.x;
-    const uint32_t warp = tid / 32, lane = tid % 32, g = lane / 4, t4 = lane % 4;
-    const uint32_t rt_begin = blockIdx.y * kAbsorbTilesPerBlock;
-    const uint32_t rt_end = min(rt_begin + kAbsorbTilesPerBlock, (rows + 15) / 16);
-    const int col0 = nq * 128 + warp * 32;                     // this warp's 32 output columns
-    uint4 b[4][kNope / 32];
-#pragma unroll
-    for (int nt = 0; nt < 4; nt++) {
-        const T* wrow = w_uk_t + (size_t(h) * kRank + col0 + nt * 8 + g) * kNope + t4 * 8;
-#pragma unroll
-        for (int kb = 0; kb < kNope / 32; kb++) b[nt][kb] = *reinterpret_cast<const uint4*>(wrow + kb * 32);
-    }
-    for (uint32_t rt = rt_begin; rt < rt_end; rt++) {
-        const uint32_t r0 = rt * 16;
-        if (nq == 0) {
-            for (int idx = tid; idx < 16 * (kRope / 2); idx += 128) {        // rope part: straight copy
-                const uint32_t rr = idx / (kRope / 2), k = idx % (kRope / 2), r = r0 + rr;
-                if (r < rows)
-                    reinterpret_cast<uint32_t*>(q_abs + (size_t(r) * H + h) * kRow + kRank)[k] =
-                        reinterpret_cast<const uint32_t*>(q + (size_t(r) * H + h) * kQDim + kNope)[k];
-            }
-        }
-        uint4 a0[kNope / 32], a1[kNope / 32];
-        const bool v0 = r0 + g < rows, v1 = r0 + g + 8 < rows;
-        const T* q0 = q + (size_t(r0 + g) * H + h) * kQDim + t4 * 8;
-        const T* q1 = q + (size_t(r0 + g + 8) * H + h) * kQDim + t4 * 8;
-#pragma unroll
-        for (int kb = 0; kb < kNope / 32; kb++) {
-            a0[kb] = v0 ? *reinterpret_cast<const uint4*>(q0 + kb * 32) : make_uint4(0, 0, 0, 0);
-            a1[kb] = v1 ? *reinterpret_cast<const uint4*>(q1 + kb * 32) : make_uint4(0, 0, 0, 0);
-        }
-#pragma unroll
-        for (int nt = 0; nt < 4; nt++) {
-            float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-            for (int kb = 0; kb < kNope / 32; kb++) {
-                const uint32_t f0[4] = {a0[kb].x, a1[kb].x, a0[kb].y, a1[kb].y};
-                const uint32_t f1[4] = {a0[kb].z, a1[kb].z, a0[kb].w, a1[kb].w};
-                mma16816<T>(c, f0, b[nt][kb].x, b[nt][kb].y);
-                mma16816<T>(c, f1, b[nt][kb].z, b[nt][kb].w);
-            }
-            const int col = col0 + nt * 8 + t4 * 2;
-            if (v0) *reinterpret_cast<uint32_t*>(q_abs + (size_t(r0 + g) * H + h) * kRow + col) = Elem<T>::pack2(c[0], c[1]);
-            if (v1) *reinterpret_cast<uint32_t*>(q_abs + (size_t(r0 + g + 8) * H + h) * kRow + col) = Elem<T>::pack2(c[2], c[3]);
-        }
-    }
-}
-
-void launch_absorb(int dtype, const void* q, const void* w_uk_t, void* q_abs, uint32_t rows,
-                   uint32_t H, cudaStream_t st)
-{
-    if (rows == 0) return;
-    const uint32_t row_tiles = (rows + 15) / 16;
-    dim3 grid(H, (row_tiles + kAbsorbTilesPerBlock - 1) / kAbsorbTilesPerBlock, 4);
-    if (dtype == 0)
-        absorb_kernel<__half><<<grid, 128, 0, st>>>(static_cast<const __half*>(q), static_cast<const __half*>(w_uk_t),
-                                                    static_cast<__half*>(q_abs), rows, H);
-    else
-        absorb_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>(
-            static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(w_uk_t),
-            static_cast<__nv_bfloat16*>(q_abs), rows, H);
-}
-
 // ------------------------------------------------------------------------------------------
 // Merge of partial softmax states + W_UV projection (reference: transformer.cpp:2610-2620).
 // A partial record is 514 floats per (part, head): m (log2 domain), l, acc[512].
 //   M = max m_p ;  w_p = 2^(m_p - M) ;  o_c = sum w_p*acc_p / sum w_p*l_p
 //   out[r][h][j] = T( sum_d o_c[d] * W_UV[h*128+j][d] )
-// Parts of row r are either the row's split-KV segments (records seg*H + h, segments
-// row_seg_begin[r] .. row_seg_begin[r+1]) or the shards of a KV-range-sharded sequence (records
-// (p*rows + r)*H + h, p < n_parts).
+// Parts of row r are the row's split-KV segments, as its RowParts says.
 // ------------------------------------------------------------------------------------------
 
 // The merged, still un-normalised state of every (row, head) written out (the per-GPU partial of a KV-range-sharded
@@ -234,17 +146,14 @@ void launch_absorb(int dtype, const void* q, const void* w_uk_t, void* q_abs, ui
 // 64*k + 2*lane (+1), k = 0..7, so a warp load covers whole lines of a record), their sums meet in shared memory and
 // warp 0 folds them.  One sequence cut into 74 segments costs two round trips to memory.
 __global__ void __launch_bounds__(512)
-export_partial_kernel(const float* __restrict__ recs, const uint32_t* __restrict__ row_seg_begin, uint32_t n_parts,
-                      float* __restrict__ exported, uint32_t rows, uint32_t H)
+export_partial_kernel(const float* __restrict__ recs, const RowParts* __restrict__ parts, uint32_t rec_stride,
+                      float* __restrict__ exported, uint32_t H)
 {
     __shared__ float scratch[16][32][18];
     const uint32_t h = blockIdx.x, r = blockIdx.y, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    uint32_t pb = 0, pe = n_parts;
-    if (row_seg_begin) { pb = row_seg_begin[r]; pe = row_seg_begin[r + 1]; }
-    auto rec_of = [&](uint32_t p) -> const float* {
-        const size_t idx = row_seg_begin ? (size_t(p) * H + h) : ((size_t(p) * rows + r) * H + h);
-        return recs + idx * kPart;
-    };
+    const RowParts rp = parts[r];
+    uint32_t pb = rp.begin, pe = rp.end;
+    auto rec_of = [&](uint32_t p) -> const float* { return recs + (size_t(p) * rec_stride + rp.rec_off + h) * kPart; };
     const uint32_t chunk = (pe - pb + 15) / 16;
     pb = min(pe, pb + warp * chunk);
     pe = min(pe, pb + chunk);
@@ -322,9 +231,8 @@ constexpr int kMergePitch = kRank + 8;               // elements; keeps ldmatrix
 constexpr size_t kMergeSmem = size_t(kVDim + 32) * kMergePitch * 2 + 16 * 4 * 4;
 template <typename T>
 __global__ void __launch_bounds__(512)
-merge_outproj_mma_kernel(const float* __restrict__ recs, const uint32_t* __restrict__ row_seg_begin,
-                         uint32_t n_parts, const T* __restrict__ w_uv, T* __restrict__ out, uint32_t rows,
-                         uint32_t H, const uint32_t* __restrict__ att_row)
+merge_outproj_mma_kernel(const float* __restrict__ recs, const RowParts* __restrict__ parts, uint32_t rec_stride,
+                         const T* __restrict__ w_uv, T* __restrict__ out, uint32_t rows, uint32_t H)
 {
     constexpr int PITCH = kMergePitch;
     extern __shared__ __align__(16) unsigned char merge_smem[];
@@ -340,8 +248,7 @@ merge_outproj_mma_kernel(const float* __restrict__ recs, const uint32_t* __restr
     const uint32_t rt_begin = blockIdx.y * kMergeTilesPerBlock;
     const uint32_t rt_end = min(rt_begin + kMergeTilesPerBlock, (rows + 15) / 16);
     auto rec_of = [&](uint32_t r, uint32_t p) -> const float* {
-        const size_t idx = row_seg_begin ? (size_t(p) * H + h) : ((size_t(p) * rows + r) * H + h);
-        return recs + idx * kPart;
+        return recs + (size_t(p) * rec_stride + parts[r].rec_off + h) * kPart;
     };
     {   // stage W_UV_h: 128 rows x 64 chunks of 16 bytes, 16 chunks per thread, all in flight at once
         const uint4* src = reinterpret_cast<const uint4*>(w_uv + size_t(h) * kVDim * kRank);
@@ -364,10 +271,7 @@ merge_outproj_mma_kernel(const float* __restrict__ recs, const uint32_t* __restr
         {
             const uint32_t r = r0 + warp;                // warp <-> row
             uint32_t pb = 0, pe = 0;
-            if (r < rows) {
-                if (row_seg_begin) { pb = row_seg_begin[r]; pe = row_seg_begin[r + 1]; }
-                else               { pb = 0; pe = n_parts; }
-            }
+            if (r < rows) { pb = parts[r].begin; pe = parts[r].end; }
             float M = -INFINITY;
             for (uint32_t p = pb + lane; p < pe; p += 32) M = fmaxf(M, rec_of(r, p)[0]);
 #pragma unroll
@@ -435,9 +339,9 @@ merge_outproj_mma_kernel(const float* __restrict__ recs, const uint32_t* __restr
         }
         const int col = warp * 8 + t4 * 2;
         if (r0 + g < rows)
-            *reinterpret_cast<uint32_t*>(out + (size_t(att_row ? att_row[r0 + g] : r0 + g) * H + h) * kVDim + col) = Elem<T>::pack2(c[0], c[1]);
+            *reinterpret_cast<uint32_t*>(out + (size_t(r0 + g) * H + h) * kVDim + col) = Elem<T>::pack2(c[0], c[1]);
         if (r0 + g + 8 < rows)
-            *reinterpret_cast<uint32_t*>(out + (size_t(att_row ? att_row[r0 + g + 8] : r0 + g + 8) * H + h) * kVDim + col) = Elem<T>::pack2(c[2], c[3]);
+            *reinterpret_cast<uint32_t*>(out + (size_t(r0 + g + 8) * H + h) * kVDim + col) = Elem<T>::pack2(c[2], c[3]);
         __syncthreads();                                 // a_hi / a_lo / row_* are rewritten by the next tile
     }
 }
@@ -451,24 +355,24 @@ int merge_mma_configure()
     return int(e);
 }
 
-void launch_merge(int dtype, const float* recs, const uint32_t* row_seg_begin, uint32_t n_parts,
-                  const void* w_uv, void* out, float* exported, uint32_t rows, uint32_t H,
-                  cudaStream_t st, const uint32_t* att_row)
+void launch_merge(int dtype, const float* recs, const StepMeta& m, const void* w_uv, void* out, uint32_t H, cudaStream_t st)
 {
+    const uint32_t rows = m.rows * m.layers;
     if (rows == 0) return;
-    if (!exported) {
-        const uint32_t row_tiles = (rows + 15) / 16;
-        dim3 grid16(H, (row_tiles + kMergeTilesPerBlock - 1) / kMergeTilesPerBlock);
-        if (dtype == 0)
-            merge_outproj_mma_kernel<__half><<<grid16, 512, kMergeSmem, st>>>(
-                recs, row_seg_begin, n_parts, static_cast<const __half*>(w_uv), static_cast<__half*>(out), rows, H, att_row);
-        else
-            merge_outproj_mma_kernel<__nv_bfloat16><<<grid16, 512, kMergeSmem, st>>>(
-                recs, row_seg_begin, n_parts, static_cast<const __nv_bfloat16*>(w_uv),
-                static_cast<__nv_bfloat16*>(out), rows, H, att_row);
-        return;
-    }
-    export_partial_kernel<<<dim3(H, rows), 512, 0, st>>>(recs, row_seg_begin, n_parts, exported, rows, H);
+    const uint32_t row_tiles = (rows + 15) / 16;
+    dim3 grid16(H, (row_tiles + kMergeTilesPerBlock - 1) / kMergeTilesPerBlock);
+    if (dtype == 0)
+        merge_outproj_mma_kernel<__half><<<grid16, 512, kMergeSmem, st>>>(
+            recs, m.parts, m.rec_stride, static_cast<const __half*>(w_uv), static_cast<__half*>(out), rows, H);
+    else
+        merge_outproj_mma_kernel<__nv_bfloat16><<<grid16, 512, kMergeSmem, st>>>(
+            recs, m.parts, m.rec_stride, static_cast<const __nv_bfloat16*>(w_uv), static_cast<__nv_bfloat16*>(out), rows, H);
+}
+
+void launch_export_partial(const float* recs, const StepMeta& m, float* exported, uint32_t H, cudaStream_t st)
+{
+    if (m.rows == 0) return;
+    export_partial_kernel<<<dim3(H, m.rows), 512, 0, st>>>(recs, m.parts, m.rec_stride, exported, H);
 }
 
 }  // namespace mla

@@ -13,10 +13,6 @@ void launch_append(int dtype, const void* kv_a, void* layer_pool, uint64_t pool_
 void launch_write_rows(const void* src, void* layer_pool, uint64_t pool_slots, const uint32_t* table,
                        uint32_t row_begin, uint32_t n, uint32_t* status, cudaStream_t st);
 
-// w_uk_t: W_UK transposed per head, [H][512][128].
-void launch_absorb(int dtype, const void* q, const void* w_uk_t, void* q_abs, uint32_t rows,
-                   uint32_t H, cudaStream_t st);
-
 // Split-KV attention, legacy tensor path (mma.sync m16n8k16): grid (segments, ceil(H/16)).
 // Returns a cudaError_t-compatible code from the launch configuration.
 int launch_decode_mma(int dtype, const void* q_abs, const void* layer_pool, uint32_t n_pages,
@@ -26,13 +22,13 @@ int decode_mma_configure();   // the *_configure() functions set kernel attribut
 // Split-KV attention on the 5th-generation tensor cores (tcgen05.mma, accumulators in TMEM,
 // cache tiles staged by TMA): grid (persistent blocks, ceil(H/64)).  tmaps points at the context's
 // host CUtensorMap array (kMap* below); this kernel uses kMapPoolPage and kMapQueries.
-int launch_decode_tc5(int dtype, const void* tmaps, uint32_t layer, uint32_t n_pages, const StepMeta& m,
+int launch_decode_tc5(int dtype, const void* tmaps, uint32_t layer0, uint32_t n_pages, const StepMeta& m,
                       float* recs, uint32_t H, uint32_t* status, cudaStream_t st);
 int decode_tc5_configure();   // sets the kernel's attributes on the current device
 
 // The transposed form for narrow head counts (mla_decode_tc5_t16.cu): tokens are the M rows, groups of 16 heads the N
 // columns; grid (persistent blocks, ceil(H/16)).  Uses kMapPoolV, kMapPoolSub and kMapQueries16.
-int launch_decode_tc5_t16(int dtype, const void* tmaps, uint32_t layer, uint32_t n_pages, const StepMeta& m, float* recs,
+int launch_decode_tc5_t16(int dtype, const void* tmaps, uint32_t layer0, uint32_t n_pages, const StepMeta& m, float* recs,
                           uint32_t H, uint32_t* status, cudaStream_t st);
 int decode_tc5_t16_configure();
 
@@ -48,31 +44,32 @@ enum : int {
 
 // The same on a pair of SMs (cluster of 2, tcgen05.mma.cta_group::2), 128-token tiles (two pages per score
 // MMA series): grid (2 x persistent pairs, ceil(H/128)).  Uses kMapPoolSub, kMapPoolV, kMapQueries and the
-// layer's pool slice.
-int launch_decode_tc5_pair128(int dtype, const void* tmaps, const void* layer_pool, uint32_t layer, uint32_t n_pages,
+// whole pool.
+int launch_decode_tc5_pair128(int dtype, const void* tmaps, const void* pool, uint32_t layer0, uint32_t n_pages,
                               const StepMeta& m, float* recs, uint32_t H, uint32_t prefetch_tiles, const void* next_weights,
                               uint32_t next_weights_bytes, uint32_t* status, cudaStream_t st);
 int decode_tc5_pair128_configure();
 
-void launch_merge(int dtype, const float* recs, const uint32_t* row_seg_begin, uint32_t n_parts,
-                  const void* w_uv, void* out, float* exported, uint32_t rows, uint32_t H,
-                  cudaStream_t st, const uint32_t* att_row = nullptr);
+// Merge of the partial states + W_UV on the warp-level tensor path (the no-allocation entry point), and the merged,
+// un-normalised state of every row written out (the per-GPU partial of a KV-range-sharded sequence).
+void launch_merge(int dtype, const float* recs, const StepMeta& m, const void* w_uv, void* out, uint32_t H, cudaStream_t st);
+void launch_export_partial(const float* recs, const StepMeta& m, float* exported, uint32_t H, cudaStream_t st);
 int merge_mma_configure();
 
-// Absorb on tcgen05 (one block per head and 64 rows); w_map: host CUtensorMap over the layer's W_UK^T,
-// [H*512 d][128 i], box 64 i x 256 d, 128-byte swizzle.  With kv_a != nullptr the same launch appends the step's
+// Absorb on tcgen05 (one block per layer, head and 64 rows); w_map: host CUtensorMap over W_UK^T of all layers,
+// [layers*H*512 d][128 i], box 64 i x 256 d, 128-byte swizzle.  With kv_a != nullptr the same launch appends the step's
 // new rows (launch_append's arguments) in extra blocks.  rotate_q: q arrives before its RoPE; the kernel rotates
 // the last 64 dims of every head with the row's position (m.row_pos) and the cos/sin table.  append_waits: kv_a may
 // have been written by the kernel launched just before this one (the append blocks then wait for it before reading).
-int launch_absorb_tc5(int dtype, const void* q, const void* w_map, void* q_abs, uint32_t rows, uint32_t H, const void* kv_a,
+int launch_absorb_tc5(int dtype, const void* q, const void* w_map, void* q_abs, uint32_t H, uint32_t layer0, const void* kv_a,
                       void* layer_pool, uint64_t pool_slots, const void* norm_w, const float* cos_sin, uint32_t cs_rows,
                       float eps, const StepMeta& m, bool rotate_q, bool append_waits, uint32_t* status, cudaStream_t st);
 int absorb_tc5_configure();
 
-// The same merge + projection on tcgen05 (one block per head and 64 rows); w_map: host CUtensorMap over the
-// layer's W_UV, [H*128 outputs][512 dims], box 64 dims x 128 outputs, 128-byte swizzle.
-int launch_merge_tc5(int dtype, const float* recs, const uint32_t* row_seg_begin, uint32_t n_parts, const void* w_map,
-                     void* out, uint32_t rows, uint32_t H, const uint32_t* att_row, uint32_t* status, cudaStream_t st);
+// The same merge + projection on tcgen05 (one block per layer, head and 64 or 16 rows); w_map: host CUtensorMap over W_UV of
+// all layers, [layers*H*128 outputs][512 dims], box 64 dims x 128 outputs, 128-byte swizzle.
+int launch_merge_tc5(int dtype, const float* recs, const StepMeta& m, uint32_t n_parts, const void* w_map, void* out, uint32_t H,
+                     uint32_t layer0, uint32_t* status, cudaStream_t st);
 int merge_tc5_configure();
 
 // Dense projection C = A . W^T on tcgen05 (mla_gemm_tc5.cu).  A [M][K] pitch lda, W [N][K] pitch ldw (the reference's

@@ -46,8 +46,9 @@ constexpr uint32_t TMEM_COLS = 128;
 template <typename T, bool kSmall>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const float* __restrict__ recs,
-                         const uint32_t* __restrict__ row_seg_begin, uint32_t n_parts, T* __restrict__ out,
-                         uint32_t rows, uint32_t H, const uint32_t* __restrict__ att_row, uint32_t* __restrict__ status)
+                         const RowParts* __restrict__ parts, uint32_t rec_stride, uint32_t n_parts, T* __restrict__ out,
+                         uint32_t rows, uint32_t H, uint32_t layer0, const uint32_t* __restrict__ att_row,
+                         uint32_t* __restrict__ status)
 {
     extern __shared__ unsigned char merge_tc5_smem[];
     const uint32_t raw = smem_u32(merge_tc5_smem);
@@ -59,11 +60,19 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const float*
     volatile int* fail_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + M_FAIL);
 
     const uint32_t h = blockIdx.x, tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-    const uint32_t r0 = blockIdx.y * (kSmall ? 16u : uint32_t(MT));    // small form: 16 rows per block, one per warp
-    auto rec_of = [&](uint32_t r, uint32_t p) -> const float* {
-        const size_t idx = row_seg_begin ? (size_t(p) * H + h) : ((size_t(p) * rows + r) * H + h);
-        return recs + idx * kPart;
+    // blockIdx.y = (layer, row tile); small form: 16 rows per tile, one per warp
+    const uint32_t row_tiles = (rows + (kSmall ? 16u : uint32_t(MT)) - 1) / (kSmall ? 16u : uint32_t(MT));
+    const uint32_t li = blockIdx.y / row_tiles, r0 = (blockIdx.y % row_tiles) * (kSmall ? 16u : uint32_t(MT));
+    out += size_t(li) * rows * H * kVDim;
+    if (parts) parts += size_t(li) * rows;
+    // a row's part p: a segment of the plan (its RowParts say which, and where in the segment's records the row is), or
+    // shard p of a KV-range-sharded sequence (parts == nullptr)
+    auto row_parts = [&](uint32_t r) -> RowParts {
+        if (!parts) return RowParts{0, n_parts, r * H, 0};
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(parts + r));
+        return RowParts{v.x, v.y, v.z, 0};
     };
+    auto rec_of = [&](uint32_t off, uint32_t p) -> const float* { return recs + (size_t(p) * rec_stride + off + h) * kPart; };
 
     grid_launch_dependents();
     if (tid == 0) {
@@ -86,7 +95,7 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const float*
     if (tid == 0) {                                       // W_UV_h: eight boxes of 64 dims x 128 outputs
         mbar_expect_tx(bar_w, W_BYTES);
 #pragma unroll 1
-        for (int s = 0; s < kRank / 64; s++) tma_load_2d(sW + s * W_SUB, &map_w, bar_w, 64 * s, int(h) * kVDim);
+        for (int s = 0; s < kRank / 64; s++) tma_load_2d(sW + s * W_SUB, &map_w, bar_w, 64 * s, int((layer0 + li) * H + h) * kVDim);
     }
 
     // Reduction of the partial states, one warp per four rows (16 apart), two rows at a time.  A lane owns dims
@@ -100,15 +109,12 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const float*
     // A warp's four rows are warp, warp+16, warp+32, warp+48 of the block's 64: with a small batch (8 sequences
     // per GPU when the batch is sharded over 8) every row then has a warp of its own instead of two warps
     // walking all of them; a row of such a batch is cut into ~10 parts, three round trips to memory each half.
-    uint32_t pb4[4], pe4[4];                              // part ranges of this warp's four rows
+    RowParts rp4[4];                                      // parts of this warp's four rows
 #pragma unroll
     for (int x = 0; x < 4; x++) {
         const uint32_t rw = r0 + warp + 16 * x;
-        pb4[x] = pe4[x] = 0;
-        if (rw < rows) {
-            if (row_seg_begin) { pb4[x] = row_seg_begin[rw]; pe4[x] = row_seg_begin[rw + 1]; }
-            else               { pb4[x] = 0; pe4[x] = n_parts; }
-        }
+        rp4[x] = RowParts{0, 0, 0, 0};
+        if (!kSmall && rw < rows) rp4[x] = row_parts(rw);
     }
     // Small batches (at most 16 rows in this block, e.g. 8 sequences per GPU): a warp has one row and sweeps its parts
     // ONCE for all 512 dims (a lane owns dims 64*k + 2*lane (+1), k = 0..7), so a row of ~10 parts costs three round
@@ -123,17 +129,17 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const float*
         // shorter sweep saves: 56.5 against 55.9 us per layer-step)
         const uint32_t nrows = min(rows - r0, 16u);
         uint32_t max_parts = n_parts;
-        if (row_seg_begin) {
-            max_parts = 0;
-            for (uint32_t i = 0; i < nrows; i++) max_parts = max(max_parts, row_seg_begin[r0 + i + 1] - row_seg_begin[r0 + i]);
+        if (parts) {
+            const RowParts rp = row_parts(r0 + min(lane, nrows - 1));
+            max_parts = __reduce_max_sync(0xffffffffu, rp.end - rp.begin);
         }
         uint32_t G = 1;
         while (2 * G * nrows <= 16u && max_parts >= 12u * G) G *= 2;     // at least six parts per warp
         const uint32_t myrow = warp / G, g = warp % G, rw = r0 + myrow;
-        uint32_t pb = 0, pe = 0;
+        uint32_t pb = 0, pe = 0, off = 0;
         if (myrow < nrows) {
-            if (row_seg_begin) { pb = row_seg_begin[rw]; pe = row_seg_begin[rw + 1]; }
-            else               { pe = n_parts; }
+            const RowParts rp = row_parts(rw);
+            pb = rp.begin; pe = rp.end; off = rp.rec_off;
             const uint32_t chunk = (pe - pb + G - 1) / G;
             pb = min(pe, pb + g * chunk);
             pe = min(pe, pb + chunk);
@@ -146,7 +152,7 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const float*
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const bool on = p + i < pe;
-                const float* rc = rec_of(rw, on ? p + i : pb);
+                const float* rc = rec_of(off, on ? p + i : pb);
                 ml[i] = on ? *reinterpret_cast<const float2*>(rc) : make_float2(-INFINITY, 0.0f);
 #pragma unroll
                 for (int k = 0; k < 8; k++)
@@ -218,13 +224,13 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const float*
         }
 #pragma unroll 1
         for (int pr = 0; pr < 2 && !small; pr++) {
-            uint32_t p[2], pe[2], rw[2];
+            uint32_t p[2], pe[2], off[2];
             float M[2], L[2], acc[2][8];
 #pragma unroll
             for (int x = 0; x < 2; x++) {
-                rw[x] = r0 + warp + 16 * (2 * pr + x);
-                p[x] = pr == 0 ? pb4[x] : pb4[2 + x];
-                pe[x] = pr == 0 ? pe4[x] : pe4[2 + x];
+                p[x] = pr == 0 ? rp4[x].begin : rp4[2 + x].begin;
+                pe[x] = pr == 0 ? rp4[x].end : rp4[2 + x].end;
+                off[x] = pr == 0 ? rp4[x].rec_off : rp4[2 + x].rec_off;
                 M[x] = -INFINITY;
                 L[x] = 0.0f;
 #pragma unroll
@@ -237,7 +243,7 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const float*
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
                         const bool on = p[x] + i < pe[x];
-                        const float* rc = rec_of(rw[x], on ? p[x] + i : 0);
+                        const float* rc = rec_of(off[x], on ? p[x] + i : 0);
                         ml[x][i] = on ? *reinterpret_cast<const float2*>(rc) : make_float2(-INFINITY, 0.0f);
 #pragma unroll
                         for (int k = 0; k < 4; k++)
@@ -277,13 +283,13 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const float*
             for (int x = 0; x < 2; x++) {
                 const float inv = L[x] > 0.0f ? 1.0f / L[x] : 0.0f;
                 const uint32_t rr = warp + 16 * (2 * pr + x);
-                const uint32_t off = rr * 128 + (((lane / 4) ^ (rr & 7)) << 4) + (lane % 4) * 4;
+                const uint32_t so = rr * 128 + (((lane / 4) ^ (rr & 7)) << 4) + (lane % 4) * 4;
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
                     const float o0 = acc[x][2 * k] * inv, o1 = acc[x][2 * k + 1] * inv;
                     const T h0 = Elem<T>::from_f32(o0), h1 = Elem<T>::from_f32(o1);
-                    *reinterpret_cast<uint32_t*>(sm + OFF_AHI + k * A_SUB + off) = Elem<T>::pack2(o0, o1);
-                    *reinterpret_cast<uint32_t*>(sm + OFF_ALO + k * A_SUB + off) =
+                    *reinterpret_cast<uint32_t*>(sm + OFF_AHI + k * A_SUB + so) = Elem<T>::pack2(o0, o1);
+                    *reinterpret_cast<uint32_t*>(sm + OFF_ALO + k * A_SUB + so) =
                         Elem<T>::pack2(o0 - Elem<T>::to_f32(h0), o1 - Elem<T>::to_f32(h1));
                 }
             }
@@ -367,19 +373,23 @@ int merge_tc5_configure()
     return int(e);
 }
 
-// w_map: host CUtensorMap over this layer's W_UV ([H*128 outputs][512 dims], box 64 dims x 128 outputs, 128-byte swizzle)
-int launch_merge_tc5(int dtype, const float* recs, const uint32_t* row_seg_begin, uint32_t n_parts, const void* w_map,
-                     void* out, uint32_t rows, uint32_t H, const uint32_t* att_row, uint32_t* status, cudaStream_t st)
+// w_map: host CUtensorMap over W_UV of all layers ([layers*H*128 outputs][512 dims], box 64 dims x 128 outputs, 128-byte
+// swizzle).  m.layers consecutive layers from layer0; out holds them one after the other.  n_parts > 0: the records are
+// [n_parts][m.rows][H] instead of the plan's segments.
+int launch_merge_tc5(int dtype, const float* recs, const StepMeta& m, uint32_t n_parts, const void* w_map, void* out, uint32_t H,
+                     uint32_t layer0, uint32_t* status, cudaStream_t st)
 {
+    const uint32_t rows = m.rows;
     if (rows == 0) return 0;
     const CUtensorMap* map = static_cast<const CUtensorMap*>(w_map);
     // The small form (16 rows per block, a warp per row, one sweep over a row's parts for all 512 dims) serves steps of at
     // most 16 rows and head counts so small that tiles of 64 rows would leave most SMs idle (16 heads x 32 rows: 16 blocks
     // of 64 rows against 32 of 16), as long as its blocks still fit one wave.
-    const bool small = rows <= 16 || H * ((rows + 15) / 16) <= 128;
-    dim3 grid(H, small ? (rows + 15) / 16 : (rows + MT - 1) / MT);
+    const bool small = rows <= 16 || m.layers * H * ((rows + 15) / 16) <= 128;
+    dim3 grid(H, m.layers * (small ? (rows + 15) / 16 : (rows + MT - 1) / MT));
     auto go = [&](auto kernel, auto* o) {
-        return int(launch_pdl(kernel, grid, dim3(NUM_THREADS), SMEM_BYTES, st, *map, recs, row_seg_begin, n_parts, o, rows, H, att_row, status));
+        return int(launch_pdl(kernel, grid, dim3(NUM_THREADS), SMEM_BYTES, st, *map, recs, n_parts ? nullptr : m.parts,
+                              n_parts ? rows * H : m.rec_stride, n_parts, o, rows, H, layer0, n_parts ? nullptr : m.att_row, status));
     };
     if (dtype == 0)
         return small ? go(merge_outproj_tc5_kernel<__half, true>, static_cast<__half*>(out))

@@ -36,8 +36,8 @@ static_assert(kScratchBytes == 8577024, "the size quoted in the public header");
 
 // The call's bookkeeping at the start of the scratch array, in the form the attention kernels read.
 struct Meta {
-    uint32_t row_seq, row_len, tbl_off, row_seg_begin[2];
-    uint32_t seg_row[kMaxSegs], seg_pb[kMaxSegs], seg_pe[kMaxSegs];
+    mla::SegDesc seg[kMaxSegs];
+    mla::RowParts parts;
     uint32_t table[kMaxSeqLen / mla::kPage];
 };
 static_assert(sizeof(Meta) <= kMetaBytes - 4, "metadata region too small (its last word is the status word)");
@@ -80,22 +80,18 @@ absorb_one_row_kernel(const T* __restrict__ q, const T* __restrict__ w_uk, T* __
 // status word, written by the device itself: the host passes two integers, so a call copies nothing from
 // host memory.
 __global__ void __launch_bounds__(256)
-noalloc_plan_kernel(unsigned char* scratch, uint32_t seq_len, uint32_t pages, uint32_t segs)
+noalloc_plan_kernel(unsigned char* scratch, uint32_t seq_len, uint32_t pages, uint32_t segs, uint32_t n_heads)
 {
     Meta* mt = reinterpret_cast<Meta*>(scratch);
     const uint32_t tid = threadIdx.x;
     if (tid == 0) {
-        mt->row_seq = 0;
-        mt->row_len = seq_len;
-        mt->tbl_off = 0;
-        mt->row_seg_begin[0] = 0;
-        mt->row_seg_begin[1] = segs;
+        mt->parts = mla::RowParts{0, segs, 0, 0};
         *reinterpret_cast<uint32_t*>(scratch + kMetaBytes - 4) = 0;
     }
     if (tid < segs) {
-        mt->seg_row[tid] = 0;
-        mt->seg_pb[tid] = uint32_t(uint64_t(pages) * tid / segs);
-        mt->seg_pe[tid] = uint32_t(uint64_t(pages) * (tid + 1) / segs);
+        const uint32_t pb = uint32_t(uint64_t(pages) * tid / segs), pe = uint32_t(uint64_t(pages) * (tid + 1) / segs);
+        const uint32_t n_tok = min(seq_len, pe * mla::kPage) - min(seq_len, pb * mla::kPage);
+        mt->seg[tid] = mla::SegDesc{0, pb, n_tok, 0, int32_t(n_tok), n_heads, {0, 0}};
     }
     for (uint32_t p = tid; p < pages; p += blockDim.x) mt->table[p] = p;
 }
@@ -148,26 +144,17 @@ int mla_attention_noalloc(uint32_t dtype, uint32_t n_heads, uint32_t seq_len, co
     // ---- segment plan, identity block table and status word: written on the device
     const uint32_t pages = (seq_len + mla::kPage - 1) / mla::kPage;
     const uint32_t segs = pages == 0 ? 1 : (pages < kMaxSegs ? pages : kMaxSegs);
-    noalloc_plan_kernel<<<1, 256, 0, st>>>(scratch, seq_len, pages, segs);
+    noalloc_plan_kernel<<<1, 256, 0, st>>>(scratch, seq_len, pages, segs, n_heads);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(MLA_ERR_CUDA, std::string("plan launch: ") + cudaGetErrorString(e));
 
     mla::StepMeta m{};
-    auto at = [&](size_t off) { return reinterpret_cast<const uint32_t*>(scratch + off); };
-    m.row_seq = at(offsetof(Meta, row_seq));
-    m.row_len = at(offsetof(Meta, row_len));
-    m.row_pos = nullptr;
-    m.row_slot = nullptr;
-    m.seq_tbl_off = at(offsetof(Meta, tbl_off));
-    m.tables = at(offsetof(Meta, table));
-    m.seg_row = at(offsetof(Meta, seg_row));
-    m.seg_page_begin = at(offsetof(Meta, seg_pb));
-    m.seg_page_end = at(offsetof(Meta, seg_pe));
-    m.row_seg_begin = at(offsetof(Meta, row_seg_begin));
-    m.cta_seg_begin = nullptr;
-    m.rows = 1;
-    m.segs = segs;
-    m.ctas = segs;
+    m.seg = reinterpret_cast<const mla::SegDesc*>(scratch + offsetof(Meta, seg));
+    m.parts = reinterpret_cast<const mla::RowParts*>(scratch + offsetof(Meta, parts));
+    m.tables = reinterpret_cast<const uint32_t*>(scratch + offsetof(Meta, table));
+    m.rows = m.layers = 1;
+    m.segs = m.ctas = segs;
+    m.rec_stride = n_heads;
 
     void* q_abs = scratch + kOffQAbs;
     float* recs = reinterpret_cast<float*>(scratch + kOffRecs);
@@ -183,7 +170,7 @@ int mla_attention_noalloc(uint32_t dtype, uint32_t n_heads, uint32_t seq_len, co
     // the cache is addressed as pages of 64 rows with the identity table
     if (int rc = mla::launch_decode_mma(int(dtype), q_abs, cache, pages ? pages : 1, m, recs, n_heads, status, st))
         return fail(MLA_ERR_CUDA, std::string("attention launch: ") + cudaGetErrorString(cudaError_t(rc)));
-    mla::launch_merge(int(dtype), recs, m.row_seg_begin, 0, w_uv, out, nullptr, 1, n_heads, st);
+    mla::launch_merge(int(dtype), recs, m, w_uv, out, n_heads, st);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(MLA_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     return MLA_OK;

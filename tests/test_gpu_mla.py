@@ -668,3 +668,50 @@ def test_block_tables_are_permuted_pages(torch):
     assert len(pages) == 40 and len(set(pages.tolist())) == 40
     assert not np.array_equal(pages, np.sort(pages))
     ctx.close()
+
+
+@pytest.mark.parametrize("H,dt,L,lens", [
+    (16, synth.DT_F16, 5, [200]),                                   # one row per layer: all layers in one group
+    (40, synth.DT_BF16, 3, [1, 64, 65, 700, 0]),                    # tile edges and an empty sequence
+    (128, synth.DT_BF16, 7, [(37 * i) % 190 for i in range(100)]),  # 700 rows: groups of 3 layers and a tail of one
+])
+def test_step_layers_in_groups_of_layers(torch, H, dt, L, lens):
+    """step_layers plans groups of layers as one launch series; its cuts may differ from the per-layer calls', so outputs
+    agree within the attention tolerance and appended rows bit for bit."""
+    from mugen_b200.mla import MlaContext
+    B = len(lens)
+    case = synth.make_layer_case(900 + H, H, [n + 1 for n in lens], dt)
+    rng = np.random.default_rng(5)
+    kv = _dev(torch, synth.to_bits(rng.standard_normal((L, B, 576), np.float32), dt))
+    q = _dev(torch, synth.to_bits(rng.standard_normal((L, B, H, 192), np.float32) * np.float32(0.9), dt))
+    outs, rows = [], []
+    for grouped in (False, True):
+        ctx = MlaContext(n_layers=L, n_heads=H, dtype=dt, n_pages=sum(n // 64 + 1 for n in lens), max_seqs=B, max_seq_len=1024, **YARN)
+        ctx.shuffle_free_pages(9)
+        for l in range(L):          # every layer its own weights: scaled by an exact power of two
+            scale = 2.0 ** -(l % 3)
+            ctx.set_layer_weights(l, synth.to_bits(case.w_uk_f32 * scale, dt), synth.to_bits(case.w_uv_f32, dt), case.w_type, case.norm_w)
+        seqs = []
+        for b, n in enumerate(lens):
+            s_ = ctx.seq_create()
+            for l in range(L):
+                if n:
+                    ctx.write_rows(l, s_, 0, _dev(torch, np.roll(case.caches[b][:n], l, axis=0)))
+            ctx.advance_seq_len(s_, n)
+            seqs.append(s_)
+        out = torch.zeros((L, B, H, 128), dtype=torch.int16, device="cuda")
+        ctx.step_begin(seqs)
+        if grouped:
+            ctx.step_layers(0, L, kv, q, out)
+        else:
+            for l in range(L):
+                ctx.step_append(l, kv[l])
+                ctx.step_attend(l, q[l], out[l])
+        ctx.step_end()
+        outs.append(_host(out).copy())
+        rows.append(np.stack([ctx.read_rows(l, seqs[b], lens[b], 1) for l in range(L) for b in range(B)]))
+        assert ctx.status() == 0
+        ctx.close()
+    assert np.array_equal(rows[0], rows[1])
+    for l in range(L):
+        check_close(outs[1][l], outs[0][l], dt, f"layer {l}")
