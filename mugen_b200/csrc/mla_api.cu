@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <memory>
 #include <string>
 #include <vector>
@@ -47,6 +48,7 @@ enum { kPlanStep = 0, kPlanRest, kPlanStack, kPlanStackTail, kPlanRegions };
 struct BlockW {
     uint32_t embed = 0, q_lora = 0;
     void *attn_norm = nullptr, *q_a = nullptr, *q_a_norm = nullptr, *q_b = nullptr, *q = nullptr, *kv_a = nullptr, *wo = nullptr;
+    alignas(64) CUtensorMap q_a_map, q_b_map, q_map, kv_a_map, wo_map;
     bool set = false;
 };
 
@@ -74,13 +76,13 @@ struct mla_ctx {
     char* w_uv = nullptr;            // [layers][H*128][512]
     char* norm = nullptr;            // [layers][512]
     std::vector<char> layer_set;     // weights registered
-    alignas(64) CUtensorMap w_uk_map, w_uv_map;
+    alignas(64) CUtensorMap w_uk_map, w_uk_rows_map, w_uv_map;
     std::vector<BlockW> blocks;
-    // workspaces of the block projections, grown on demand: normalised hidden state, q_a, float K-slice partials,
+    // workspaces of the block projections, grown on demand: normalised hidden state, q_a,
     // and the block's q / kv_a / attention output when the library owns them (mla_step_block)
     void *blk_hidden2 = nullptr, *blk_qa = nullptr, *blk_q = nullptr, *blk_kv = nullptr, *blk_out = nullptr;
-    float* blk_partial = nullptr;
-    size_t blk_hidden2_cap = 0, blk_qa_cap = 0, blk_q_cap = 0, blk_kv_cap = 0, blk_out_cap = 0, blk_partial_cap = 0;
+    size_t blk_hidden2_cap = 0, blk_qa_cap = 0, blk_q_cap = 0, blk_kv_cap = 0, blk_out_cap = 0;
+    mla::GemmWorkspace gemm_ws{};    // partial tiles and counters of the projections
     float* cos_sin = nullptr;       // device [max positions][64]
     uint32_t cs_rows = 0;           // positions filled so far
     uint32_t cs_cap = 0;
@@ -107,12 +109,16 @@ struct mla_ctx {
     Plan plan, plan_rest, stack, stack_tail;
     bool has_chunks = false;
     std::vector<RowSpec> rows;       // of the open step
-    struct Chunk { uint32_t tbl_off, q_row0, n_new, start, base_pos; };   // tbl_off: of its block table in the upload
+    struct Chunk { uint32_t seq_index, q_row0, n_new, start, base_pos; };
     std::vector<Chunk> chunks;
+    // Chunks whose expanded keys and values share the workspace and the launches: `rows` expanded rows (every sequence padded
+    // to 128), their pages and query tiles in the upload of plan_rest
+    struct ChunkGroup { uint32_t rows, n_tiles; const uint32_t* pages; const mla::PrefillTile* tiles; };
+    std::vector<ChunkGroup> chunk_groups;
     uint32_t step_rows = 0;          // rows of the step in the caller's q / kv_a / out tensors
-    // prefill workspaces, grown on demand: gathered latent rows, expanded keys and values, rotated chunk queries
-    void *pf_latent = nullptr, *pf_kx = nullptr, *pf_vx = nullptr, *pf_q = nullptr;
-    size_t pf_latent_cap = 0, pf_kx_cap = 0, pf_vx_cap = 0, pf_q_cap = 0;
+    // prefill workspaces, grown on demand: expanded keys and values
+    void *pf_kx = nullptr, *pf_vx = nullptr;
+    size_t pf_kx_cap = 0, pf_vx_cap = 0;
 
     // pages of the last planned step per persistent worker (mla_step_balance)
     uint32_t plan_workers = 0, plan_min_pages = 0, plan_max_pages = 0;
@@ -171,6 +177,8 @@ size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 constexpr uint32_t kPrefillMin = 64;
 // Most query rows and bytes of absorbed queries of a group of layers (step_layers_grouped).
 constexpr uint64_t kGroupRows = 1024, kGroupBytes = 48ull << 20;
+// Expanded keys and values of the chunks that share a launch (a chunk that needs more has one of its own).
+constexpr uint64_t kExpandBytes = 1ull << 30;
 
 inline float half_bits_to_f32(uint16_t h) { return __half2float(__ushort_as_half(h)); }
 inline uint16_t f32_to_half_bits(float f) { return __half_as_ushort(__float2half_rn(f)); }
@@ -269,8 +277,18 @@ size_t meta_capacity(const mla_ctx* c)
     const size_t max_pages_per_seq = (size_t(c->cfg.max_seq_len) + mla::kPage - 1) / mla::kPage;
     const size_t tbl_entries = std::min<size_t>(size_t(c->cfg.max_seqs) * max_pages_per_seq, c->cfg.n_pages) + 4;
     return align16(R * 8) + 3 * align16(R * 4) + align16(tbl_entries * 4) + align16((W + V) * sizeof(mla::SegDesc)) +
-           align16(V * sizeof(mla::RowParts)) + align16((W + 1) * 4) + 256;
+           align16(V * sizeof(mla::RowParts)) + align16((W + 1) * 4) +
+           align16((tbl_entries + 2 * size_t(c->cfg.max_seqs)) * 4) +                                        // chunks: pages padded to 128 rows,
+           align16((R / 128 + c->cfg.max_seqs + 1) * sizeof(mla::PrefillTile)) + 256;                        // and query tiles
 }
+
+// what the prefill kernels of a step read (rest_plan)
+struct ChunkMeta {
+    std::vector<uint32_t> pages;             // page of every 64 expanded rows
+    std::vector<mla::PrefillTile> tiles;
+    struct Group { uint32_t rows, page0, tile0, n_tiles; };
+    std::vector<Group> groups;
+};
 
 // Plans `layers` identical layers of query rows over the persistent attention workers, packs the metadata of the launch
 // series (new rows to append, query rows, block tables, segments) and uploads it through the page-locked ring into region
@@ -279,7 +297,8 @@ size_t meta_capacity(const mla_ctx* c)
 //   query    the query rows; nullptr: app.  att_row: their rows in the caller's tensors (with query only)
 //   layers   0: no attention (append or row copy only)
 int build_plan(mla_ctx* c, Plan& plan, int region, const std::vector<uint32_t>& seq_ids, const std::vector<RowSpec>& app,
-               const std::vector<RowSpec>* query, const std::vector<uint32_t>* att_row, uint32_t layers, cudaStream_t st)
+               const std::vector<RowSpec>* query, const std::vector<uint32_t>* att_row, uint32_t layers, cudaStream_t st,
+               const ChunkMeta* chunks = nullptr)
 {
     const std::vector<RowSpec>& rows = query ? *query : app;
     const uint32_t A = uint32_t(app.size()), R = layers ? uint32_t(rows.size()) : 0, S = uint32_t(seq_ids.size()), H = c->cfg.n_heads;
@@ -329,7 +348,8 @@ int build_plan(mla_ctx* c, Plan& plan, int region, const std::vector<uint32_t>& 
     const size_t o_slot = take(size_t(A) * 8), o_apos = take(size_t(A) * 4), o_tbl = take(tbl_total * 4),
                  o_pos = query ? take(size_t(R) * 4) : o_apos, o_att = take(att_row ? size_t(R) * 4 : 0),
                  o_seg = take(size_t(G) * sizeof(mla::SegDesc)), o_parts = take(size_t(R) * layers * sizeof(mla::RowParts)),
-                 o_csb = take(size_t(W + 1) * 4);
+                 o_csb = take(size_t(W + 1) * 4), o_cpg = take(chunks ? chunks->pages.size() * 4 : 0),
+                 o_ctl = take(chunks ? chunks->tiles.size() * sizeof(mla::PrefillTile) : 0);
     if (off > c->meta_cap)
         return fail(c, MLA_ERR_CAPACITY, "step metadata (" + std::to_string(off) + " B) exceeds the buffer (" +
                                              std::to_string(c->meta_cap) + " B)");
@@ -364,6 +384,14 @@ int build_plan(mla_ctx* c, Plan& plan, int region, const std::vector<uint32_t>& 
     for (uint32_t v = 0; v < R * layers; v++) p_parts[v] = mla::RowParts{row_seg_begin[v], row_seg_begin[v + 1], 0, 0};
     std::memcpy(h + o_csb, cta_seg_begin.data(), size_t(W + 1) * 4);
     char* d = c->meta_dev + size_t(region) * c->meta_cap;
+    if (chunks) {
+        std::memcpy(h + o_cpg, chunks->pages.data(), chunks->pages.size() * 4);
+        std::memcpy(h + o_ctl, chunks->tiles.data(), chunks->tiles.size() * sizeof(mla::PrefillTile));
+        c->chunk_groups.clear();
+        for (const auto& g : chunks->groups)
+            c->chunk_groups.push_back({g.rows, g.n_tiles, reinterpret_cast<const uint32_t*>(d + o_cpg) + g.page0,
+                                       reinterpret_cast<const mla::PrefillTile*>(d + o_ctl) + g.tile0});
+    }
     CU_TRY(c, cudaMemcpyAsync(d, h, off, cudaMemcpyHostToDevice, st));
     CU_TRY(c, cudaEventRecord(mb.done, st));
     mb.in_flight = true;
@@ -406,7 +434,25 @@ int rest_plan(mla_ctx* c, cudaStream_t st)
             for (uint32_t t = 0; t < cnt; t++) { rest.push_back(c->rows[r + t]); att_row.push_back(r + t); }
         r += cnt;
     }
-    return build_plan(c, c->plan_rest, kPlanRest, c->step_seqs, c->rows, &rest, &att_row, 1, st);
+    // the chunks' expanded rows and query tiles, as many chunks per group as the workspace bound allows
+    ChunkMeta cm;
+    const uint64_t row_bytes = uint64_t(c->cfg.n_heads) * (mla::kNope + mla::kVDim) * 2;
+    for (const auto& ch : c->chunks) {
+        const uint32_t total = ch.start + ch.n_new, padded = (total + 127) / 128 * 128;
+        if (cm.groups.empty() || (cm.groups.back().rows + padded) * row_bytes > kExpandBytes) cm.groups.push_back({0, uint32_t(cm.pages.size()), uint32_t(cm.tiles.size()), 0});
+        auto& g = cm.groups.back();
+        const auto& pg = c->pt->seq(c->step_seqs[ch.seq_index])->pages;
+        const uint32_t n_pages = (total + mla::kPage - 1) / mla::kPage;
+        for (uint32_t i = 0; i < padded / mla::kPage; i++) cm.pages.push_back(pg[std::min(i, n_pages - 1)]);   // padding: the last page again
+        for (uint32_t t = 0; t < ch.n_new; t += 128)
+            cm.tiles.push_back({ch.q_row0 + t, std::min(128u, ch.n_new - t), ch.start + t, total, g.rows, ch.base_pos + ch.start + t, {0, 0}});
+        g.rows += padded;
+        g.n_tiles = uint32_t(cm.tiles.size()) - g.tile0;
+    }
+    for (auto& g : cm.groups)           // the tiles that see the most keys first
+        std::stable_sort(cm.tiles.begin() + g.tile0, cm.tiles.begin() + g.tile0 + g.n_tiles,
+                         [](const mla::PrefillTile& a, const mla::PrefillTile& b) { return a.pos > b.pos; });
+    return build_plan(c, c->plan_rest, kPlanRest, c->step_seqs, c->rows, &rest, &att_row, 1, st, &cm);
 }
 
 char* layer_pool(mla_ctx* c, uint32_t layer)
@@ -428,10 +474,10 @@ char* layer_norm(mla_ctx* c, uint32_t layer) { return c->norm + size_t(layer) * 
 
 int run_append(mla_ctx* c, uint32_t layer, const void* kv_a, const mla::StepMeta& m, cudaStream_t st)
 {
-    mla::launch_append(int(c->cfg.dtype), kv_a, layer_pool(c, layer), c->pool_slots, layer_norm(c, layer),
-                       c->cos_sin, c->cs_rows, c->cfg.rms_norm_eps, m, c->status_dev, st);
+    const int e = mla::launch_append(int(c->cfg.dtype), kv_a, layer_pool(c, layer), c->pool_slots, layer_norm(c, layer),
+                                     c->cos_sin, c->cs_rows, c->cfg.rms_norm_eps, m, c->status_dev, st);
+    if (e != 0) return fail(c, MLA_ERR_CUDA, std::string("append launch: ") + cudaGetErrorString(cudaError_t(e)));
     c->launches += m.app_rows ? 1 : 0;
-    CU_TRY(c, cudaGetLastError());
     return MLA_OK;
 }
 
@@ -467,13 +513,12 @@ int run_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, float* expo
     if (e != 0) return fail(c, MLA_ERR_CUDA, std::string("attention launch: ") + cudaGetErrorString(cudaError_t(e)));
     if (timed) CU_TRY(c, cudaEventRecord(c->prof_events[c->prof_used++].second, st));
     if (exported) {
-        mla::launch_export_partial(c->recs, m, exported, H, st);
+        e = mla::launch_export_partial(c->recs, m, exported, H, st);
     } else {
         e = mla::launch_merge_tc5(dt, c->recs, m, 0, &c->w_uv_map, out, H, layer, c->status_dev, st);
-        if (e != 0) return fail(c, MLA_ERR_CUDA, std::string("merge launch: ") + cudaGetErrorString(cudaError_t(e)));
     }
+    if (e != 0) return fail(c, MLA_ERR_CUDA, std::string("merge launch: ") + cudaGetErrorString(cudaError_t(e)));
     c->launches += 3;
-    CU_TRY(c, cudaGetLastError());
     return MLA_OK;
 }
 
@@ -489,47 +534,44 @@ int grow_buf(mla_ctx* c, void** p, size_t* cap, size_t bytes)
     return MLA_OK;
 }
 
-// The chunks of the open step, one after the other: gather the sequence's latent rows (the chunk's own rows were
-// appended by the launch before), expand them into per-head keys and values with W_UK / W_UV, run causal flash
-// attention of the chunk's queries over them.  Reference semantics: src/core/model/transformer.cpp:1263-1337.
+// The chunks of the open step: expand each sequence's latent rows (the chunk's own were appended by the launch before) into
+// per-head keys and values with W_UK / W_UV, straight from the cache pages, and run causal flash attention of the chunks'
+// queries over them.  Reference semantics: src/core/model/transformer.cpp:1263-1337.
 int run_chunks(mla_ctx* c, uint32_t layer, const void* q, void* out, cudaStream_t st)
 {
     const uint32_t H = c->cfg.n_heads;
     const int dt = int(c->cfg.dtype);
-    const char *w_uk = c->w_uk_rows + layer * weight_bytes(c), *w_uv = c->w_uv + layer * weight_bytes(c);
-    for (const auto& ch : c->chunks) {
-        const uint32_t total = ch.start + ch.n_new;
-        if (int e = grow_buf(c, &c->pf_latent, &c->pf_latent_cap, size_t(total) * mla::kRow * 2)) return e;
-        if (int e = grow_buf(c, &c->pf_kx, &c->pf_kx_cap, size_t(total) * H * mla::kNope * 2)) return e;
-        if (int e = grow_buf(c, &c->pf_vx, &c->pf_vx_cap, size_t(total) * H * mla::kVDim * 2)) return e;
-        const uint32_t* table = c->plan_rest.m.tables + ch.tbl_off;
-        int rc = mla::launch_gather_rows(layer_pool(c, layer), c->pool_slots, table, total, c->pf_latent, c->status_dev, st);
-        if (rc) return fail(c, MLA_ERR_CUDA, std::string("gather launch: ") + cudaGetErrorString(cudaError_t(rc)));
-        rc = mla::launch_gemm_tc5(dt, c->pf_latent, mla::kRow, w_uk, mla::kRank, total, H * mla::kNope, mla::kRank, c->pf_kx,
-                                  nullptr, 1, c->status_dev, st);
-        if (rc == 0)
-            rc = mla::launch_gemm_tc5(dt, c->pf_latent, mla::kRow, w_uv, mla::kRank, total, H * mla::kVDim, mla::kRank, c->pf_vx,
-                                      nullptr, 1, c->status_dev, st);
+    for (const auto& g : c->chunk_groups) {
+        if (int e = grow_buf(c, &c->pf_kx, &c->pf_kx_cap, size_t(g.rows) * H * mla::kNope * 2)) return e;
+        if (int e = grow_buf(c, &c->pf_vx, &c->pf_vx_cap, size_t(g.rows) * H * mla::kVDim * 2)) return e;
+        mla::GemmCall gc;
+        gc.paged_map = &c->tmaps[mla::kMapPoolSub];
+        gc.table = g.pages;
+        gc.layer = layer;
+        gc.n_pages = c->cfg.n_pages;
+        gc.M = g.rows;
+        gc.K = mla::kRank;
+        gc.n_weights = 2;
+        gc.w[0] = mla::GemmWeight{&c->w_uk_rows_map, layer * H * mla::kNope, H * mla::kNope, c->pf_kx};
+        gc.w[1] = mla::GemmWeight{&c->w_uv_map, layer * H * mla::kVDim, H * mla::kVDim, c->pf_vx};
+        int rc = mla::launch_gemm_tc5(dt, gc, c->gemm_ws, c->status_dev, st);
         if (rc) return fail(c, rc == -1 ? MLA_ERR_INVALID : MLA_ERR_CUDA, "key / value expansion launch failed");
-        const void* qp = q;
-        uint32_t q_rows_total = c->step_rows, q_row0 = ch.q_row0;
-        if (c->q_rope_in_kernel) {           // the chunk's queries arrive before their RoPE: rotate a copy
-            if (int e = grow_buf(c, &c->pf_q, &c->pf_q_cap, size_t(ch.n_new) * H * mla::kQDim * 2)) return e;
-            rc = mla::launch_rotate_q_rows(dt, static_cast<const char*>(q) + size_t(ch.q_row0) * H * mla::kQDim * 2, c->pf_q, ch.n_new, H,
-                                           ch.base_pos + ch.start, c->cos_sin, c->cs_rows, c->status_dev, st);
-            if (rc) return fail(c, MLA_ERR_CUDA, std::string("query rotation launch: ") + cudaGetErrorString(cudaError_t(rc)));
-            c->launches++;
-            qp = c->pf_q;
-            q_rows_total = ch.n_new;
-            q_row0 = 0;
-        }
-        // out rows are addressed from the chunk's first row in either case
-        rc = mla::launch_prefill_tc5(dt, qp, q_rows_total, q_row0, ch.n_new, ch.start, c->pf_kx, c->pf_vx, c->pf_latent,
-                                     static_cast<char*>(out) + (size_t(ch.q_row0) - q_row0) * H * mla::kVDim * 2, H, c->status_dev, st);
+        mla::PrefillCall p;
+        p.q = q; p.out = out; p.kx = c->pf_kx; p.vx = c->pf_vx;
+        p.pool_map = &c->tmaps[mla::kMapPoolSub];
+        p.pages = g.pages;
+        p.tiles = g.tiles;
+        p.n_tiles = g.n_tiles;
+        p.rows = g.rows;
+        p.H = H;
+        p.layer = layer;
+        p.n_pages = c->cfg.n_pages;
+        p.cos_sin = c->q_rope_in_kernel ? c->cos_sin : nullptr;
+        p.cs_rows = c->cs_rows;
+        rc = mla::launch_prefill_tc5(dt, p, c->status_dev, st);
         if (rc) return fail(c, rc == -1 ? MLA_ERR_INVALID : MLA_ERR_CUDA, "prefill attention launch failed");
-        c->launches += 4;
+        c->launches += 2;
     }
-    CU_TRY(c, cudaGetLastError());
     return MLA_OK;
 }
 
@@ -595,6 +637,7 @@ int make_tensor_maps(mla_ctx* c)
         };
         const cuuint64_t heads = cuuint64_t(c->cfg.n_layers) * c->cfg.n_heads;
         if (int e = weights(&c->w_uv_map, "W_UV", c->w_uv, mla::kRank, heads * mla::kVDim, mla::kVDim)) return e;
+        if (int e = weights(&c->w_uk_rows_map, "W_UK rows", c->w_uk_rows, mla::kRank, heads * mla::kNope, mla::kNope)) return e;
         if (int e = weights(&c->w_uk_map, "W_UK", c->w_uk, mla::kNope, heads * mla::kRank, 256)) return e;
     }
     {   // cache pool: 576 values innermost, then the token slots of a layer, then layers;
@@ -703,6 +746,11 @@ int mla_create(const mla_config* cfg, mla_ctx** out)
     CR_TRY(cudaMalloc(&c->recs, c->rec_cap * mla::kPart * sizeof(float)));
     CR_TRY(cudaMalloc(&c->status_dev, sizeof(uint32_t)));
     CR_TRY(cudaMemset(c->status_dev, 0, sizeof(uint32_t)));
+    c->gemm_ws.blocks = uint32_t(c->sm_count);
+    c->gemm_ws.max_tiles = 16 * c->gemm_ws.blocks;
+    CR_TRY(cudaMalloc(&c->gemm_ws.partial, mla::gemm_tc5_partial_bytes(c->gemm_ws.blocks)));
+    CR_TRY(cudaMalloc(&c->gemm_ws.counters, c->gemm_ws.max_tiles * 4));
+    CR_TRY(cudaMemset(c->gemm_ws.counters, 0, c->gemm_ws.max_tiles * 4));
     c->meta_cap = meta_capacity(cp);
     CR_TRY(cudaMalloc(&c->meta_dev, kPlanRegions * c->meta_cap));
     CR_TRY(cudaMallocHost(&c->meta_host, kMetaRing * c->meta_cap));
@@ -760,7 +808,7 @@ void mla_destroy(mla_ctx* c)
     cudaDeviceSynchronize();
     cudaFree(c->pool);
     cudaFree(c->w_uk); cudaFree(c->w_uk_rows); cudaFree(c->w_uv); cudaFree(c->norm);
-    cudaFree(c->pf_latent); cudaFree(c->pf_kx); cudaFree(c->pf_vx); cudaFree(c->pf_q);
+    cudaFree(c->pf_kx); cudaFree(c->pf_vx);
     cudaFree(c->cos_sin);
     cudaFree(c->q_abs);
     cudaFree(c->recs);
@@ -775,7 +823,7 @@ void mla_destroy(mla_ctx* c)
     if (c->h_out) cudaFreeHost(c->h_out);
     cudaFree(c->d_kv); cudaFree(c->d_q); cudaFree(c->d_out);
     for (auto& b : c->blocks) { cudaFree(b.attn_norm); cudaFree(b.q_a); cudaFree(b.q_a_norm); cudaFree(b.q_b); cudaFree(b.q); cudaFree(b.kv_a); cudaFree(b.wo); }
-    cudaFree(c->blk_hidden2); cudaFree(c->blk_qa); cudaFree(c->blk_q); cudaFree(c->blk_kv); cudaFree(c->blk_out); cudaFree(c->blk_partial);
+    cudaFree(c->blk_hidden2); cudaFree(c->blk_qa); cudaFree(c->blk_q); cudaFree(c->blk_kv); cudaFree(c->blk_out); cudaFree(c->gemm_ws.partial); cudaFree(c->gemm_ws.counters);
     for (auto& ev : c->host_ev) { cudaEventDestroy(ev.in); cudaEventDestroy(ev.compute); cudaEventDestroy(ev.out); }
     if (c->copy_in) cudaStreamDestroy(c->copy_in);
     if (c->copy_out) cudaStreamDestroy(c->copy_out);
@@ -792,7 +840,11 @@ int mla_status(mla_ctx* c, void* stream, uint32_t* device_status)
     uint32_t v = 0;
     CU_TRY(c, cudaMemcpyAsync(&v, c->status_dev, 4, cudaMemcpyDeviceToHost, st));
     CU_TRY(c, cudaStreamSynchronize(st));
-    if (v) CU_TRY(c, cudaMemsetAsync(c->status_dev, 0, 4, st));
+    if (v) {
+        CU_TRY(c, cudaMemsetAsync(c->status_dev, 0, 4, st));
+        // a projection that gave up in the middle may have left tile counters behind
+        CU_TRY(c, cudaMemsetAsync(c->gemm_ws.counters, 0, c->gemm_ws.max_tiles * 4, st));
+    }
     *device_status = v;
     if (v) return fail(c, MLA_ERR_DEVICE, "device status word = " + std::to_string(v));
     return MLA_OK;
@@ -985,7 +1037,6 @@ int mla_step_begin(mla_ctx* c, uint32_t n_seq, const uint32_t* seq_ids, const ui
     c->chunks.clear();
     c->has_chunks = false;
     c->step_new_rows = 0;
-    uint32_t tbl_off = 0;
     for (uint32_t i = 0; i < n_seq; i++) {
         const auto* s = c->pt->seq(seqs[i]);
         if (nn[i] == 0) {                                              // query-only row
@@ -995,7 +1046,7 @@ int mla_step_begin(mla_ctx* c, uint32_t n_seq, const uint32_t* seq_ids, const ui
             rows.push_back({i, s->len, 0, ~uint64_t(0)});
         }
         if (nn[i] >= kPrefillMin && c->kernel != MLA_KERNEL_MMA) {
-            c->chunks.push_back({tbl_off, uint32_t(rows.size()), nn[i], s->len, s->base_pos});
+            c->chunks.push_back({i, uint32_t(rows.size()), nn[i], s->len, s->base_pos});
             c->has_chunks = true;
         }
         for (uint32_t t = 0; t < nn[i]; t++) {
@@ -1003,7 +1054,6 @@ int mla_step_begin(mla_ctx* c, uint32_t n_seq, const uint32_t* seq_ids, const ui
             rows.push_back({i, local + 1, s->base_pos + local, c->pt->slot(seqs[i], local)});
         }
         c->step_new_rows += nn[i];
-        tbl_off += uint32_t(s->pages.size());
     }
     c->step_rows = uint32_t(rows.size());
     c->plan.ready = c->plan_rest.ready = c->stack.ready = c->stack_tail.ready = false;
@@ -1373,24 +1423,27 @@ int grow(mla_ctx* c, void** p, size_t* cap, size_t bytes)
     return MLA_OK;
 }
 
-// out[rows][N] = act[rows][K] . W[N][K]^T, rounded to the storage type, then `mode` (0 store, 1 RMSNorm(w), 2 += res)
-int project(mla_ctx* c, const void* act, const void* W, uint32_t rows, uint32_t N, uint32_t K, int mode, const void* w,
-            const void* res, void* out, cudaStream_t st)
+// out_i[rows][N_i] = act[rows][K] . W_i[N_i][K]^T, rounded to the storage type; residual: added to what out holds
+int project(mla_ctx* c, const void* act, uint32_t rows, uint32_t K, std::initializer_list<mla::GemmWeight> weights, bool residual, cudaStream_t st)
 {
-    uint32_t splits = mla::gemm_tc5_splits(rows, N, K, uint32_t(c->sm_count));
-    const bool direct = splits == 1 && mode == 0;
-    if (!direct)
-        if (int e = grow(c, reinterpret_cast<void**>(&c->blk_partial), &c->blk_partial_cap, size_t(splits) * rows * N * sizeof(float))) return e;
-    int rc = mla::launch_gemm_tc5(int(c->cfg.dtype), act, K, W, K, rows, N, K, direct ? out : nullptr,
-                                  direct ? nullptr : c->blk_partial, splits, c->status_dev, st);
+    mla::GemmCall g;
+    g.A = act;
+    g.M = rows;
+    g.K = K;
+    for (const auto& w : weights) g.w[g.n_weights++] = w;
+    g.residual = residual;
+    const int rc = mla::launch_gemm_tc5(int(c->cfg.dtype), g, c->gemm_ws, c->status_dev, st);
     if (rc == -1) return fail(c, MLA_ERR_INVALID, "projection operands must be 16-byte aligned with row lengths that are multiples of 8");
     if (rc != 0) return fail(c, MLA_ERR_CUDA, std::string("projection launch: ") + cudaGetErrorString(cudaError_t(rc)));
     c->launches++;
-    if (!direct) {
-        rc = mla::launch_gemm_finalize(int(c->cfg.dtype), c->blk_partial, splits, rows, N, mode, w, c->cfg.rms_norm_eps, res, out, st);
-        if (rc != 0) return fail(c, MLA_ERR_CUDA, std::string("projection finalize launch: ") + cudaGetErrorString(cudaError_t(rc)));
-        c->launches++;
-    }
+    return MLA_OK;
+}
+
+int rmsnorm(mla_ctx* c, const void* x, const void* w, void* y, uint32_t rows, uint32_t N, cudaStream_t st)
+{
+    if (int rc = mla::launch_rmsnorm_rows(int(c->cfg.dtype), x, w, y, rows, N, c->cfg.rms_norm_eps, st))
+        return fail(c, MLA_ERR_CUDA, std::string("rmsnorm launch: ") + cudaGetErrorString(cudaError_t(rc)));
+    c->launches++;
     return MLA_OK;
 }
 
@@ -1406,17 +1459,13 @@ int project_in(mla_ctx* c, const BlockW& b, uint32_t rows, const void* hidden, v
 {
     const uint32_t E = b.embed, H = c->cfg.n_heads, QD = H * uint32_t(mla::kQDim);
     if (int e = grow(c, &c->blk_hidden2, &c->blk_hidden2_cap, size_t(rows) * E * 2)) return e;
-    if (int rc = mla::launch_rmsnorm_rows(int(c->cfg.dtype), hidden, b.attn_norm, c->blk_hidden2, rows, E, c->cfg.rms_norm_eps, st))
-        return fail(c, MLA_ERR_CUDA, std::string("rmsnorm launch: ") + cudaGetErrorString(cudaError_t(rc)));
-    c->launches++;
-    if (b.q_lora) {
-        if (int e = grow(c, &c->blk_qa, &c->blk_qa_cap, size_t(rows) * b.q_lora * 2)) return e;
-        if (int e = project(c, c->blk_hidden2, b.q_a, rows, b.q_lora, E, 1, b.q_a_norm, nullptr, c->blk_qa, st)) return e;
-        if (int e = project(c, c->blk_qa, b.q_b, rows, QD, b.q_lora, 0, nullptr, nullptr, q, st)) return e;
-    } else {
-        if (int e = project(c, c->blk_hidden2, b.q, rows, QD, E, 0, nullptr, nullptr, q, st)) return e;
-    }
-    return project(c, c->blk_hidden2, b.kv_a, rows, uint32_t(mla::kRow), E, 0, nullptr, nullptr, kv_a, st);
+    if (int e = rmsnorm(c, hidden, b.attn_norm, c->blk_hidden2, rows, E, st)) return e;
+    const mla::GemmWeight kv{&b.kv_a_map, 0, uint32_t(mla::kRow), kv_a};
+    if (!b.q_lora) return project(c, c->blk_hidden2, rows, E, {{&b.q_map, 0, QD, q}, kv}, false, st);
+    if (int e = grow(c, &c->blk_qa, &c->blk_qa_cap, size_t(rows) * b.q_lora * 2)) return e;
+    if (int e = project(c, c->blk_hidden2, rows, E, {{&b.q_a_map, 0, b.q_lora, c->blk_qa}, kv}, false, st)) return e;
+    if (int e = rmsnorm(c, c->blk_qa, b.q_a_norm, c->blk_qa, rows, b.q_lora, st)) return e;
+    return project(c, c->blk_qa, rows, b.q_lora, {{&b.q_b_map, 0, QD, q}}, false, st);
 }
 
 }  // namespace
@@ -1448,6 +1497,13 @@ int mla_set_block_weights(mla_ctx* c, uint32_t layer, const mla_block_weights* w
     if (int e = put(&b.q, R ? nullptr : w->q, size_t(H) * mla::kQDim * E)) return e;
     if (int e = put(&b.kv_a, w->kv_a_mqa, size_t(mla::kRow) * E)) return e;
     if (int e = put(&b.wo, w->wo, size_t(E) * H * mla::kVDim)) return e;
+    const int dt = int(c->cfg.dtype);
+    const uint32_t QD = H * uint32_t(mla::kQDim);
+    if (!(R ? mla::gemm_tc5_weight_map(&b.q_a_map, dt, b.q_a, R, E) && mla::gemm_tc5_weight_map(&b.q_b_map, dt, b.q_b, QD, R)
+            : mla::gemm_tc5_weight_map(&b.q_map, dt, b.q, QD, E)) ||
+        !mla::gemm_tc5_weight_map(&b.kv_a_map, dt, b.kv_a, uint64_t(mla::kRow), E) ||
+        !mla::gemm_tc5_weight_map(&b.wo_map, dt, b.wo, E, uint64_t(H) * mla::kVDim))
+        return fail(c, MLA_ERR_CUDA, "cuTensorMapEncodeTiled(projection weights) failed");
     b.embed = E;
     b.q_lora = R;
     b.set = true;
@@ -1471,8 +1527,8 @@ int mla_block_project_out(mla_ctx* c, uint32_t layer, uint32_t rows, const void*
     const BlockW* b = nullptr;
     if (int e = block_of(c, layer, &b)) return e;
     if (rows == 0) return MLA_OK;
-    // hidden = hidden + W_o . attn_out: the residual is read and the sum written by the finalize kernel
-    return project(c, attn_out, b->wo, rows, b->embed, c->cfg.n_heads * uint32_t(mla::kVDim), 2, nullptr, hidden, hidden,
+    // hidden = hidden + W_o . attn_out
+    return project(c, attn_out, rows, c->cfg.n_heads * uint32_t(mla::kVDim), {{&b->wo_map, 0, b->embed, hidden}}, true,
                    static_cast<cudaStream_t>(stream));
 }
 
@@ -1494,7 +1550,7 @@ int mla_step_block(mla_ctx* c, uint32_t layer, void* hidden, void* stream)
     if (int e = grow(c, &c->blk_out, &c->blk_out_cap, size_t(rows) * H * mla::kVDim * 2)) return e;
     if (int e = project_in(c, *b, rows, hidden, c->blk_q, c->blk_kv, st)) return e;
     if (int e = run_layer(c, layer, c->blk_kv, c->blk_q, c->blk_out, st)) return e;
-    return project(c, c->blk_out, b->wo, rows, b->embed, H * uint32_t(mla::kVDim), 2, nullptr, hidden, hidden, st);
+    return project(c, c->blk_out, rows, H * uint32_t(mla::kVDim), {{&b->wo_map, 0, b->embed, hidden}}, true, st);
 }
 
 }  // extern "C"

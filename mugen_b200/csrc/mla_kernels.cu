@@ -1,91 +1,31 @@
 // Small kernels around the attention core: latent-row append, partial merge + W_UV projection, bulk row copy.  sm_100a.
+#include "mla_append.cuh"
 #include "mla_launch.h"
 
 namespace mla {
 
 // ------------------------------------------------------------------------------------------
-// Append: RMSNorm(c_kv)*w, NeoX RoPE(k_rope) and the scatter of the 576-value row into its
-// page slot.  Follows the reference's statements one by one so that the stored bits equal the
-// CPU path's (src/core/model/transformer.cpp:3935-3948 and :3964-3975):
-//   ss = sum_i x_i*x_i            sequential, float, multiply and add rounded separately
-//   r  = 1 / sqrt(ss/512 + eps)
-//   c_kv[i] = T( (x_i*r) * w_i )  two multiplies, one final rounding
-//   k[i]    = T( x0*cos - x1*sin ),  k[i+32] = T( x1*cos + x0*sin )   from the original x0, x1
-// cos/sin come from a host-built table (the host evaluates them with the same libm calls as
-// the CPU path; device cosf/sinf are not bit-identical to glibc's).
-// One block per row; the squares are formed in parallel, thread 0 adds them in order.
+// Append on its own (mla_append.cuh): eight rows per block, one warp each.
 // ------------------------------------------------------------------------------------------
+constexpr int kAppendWarps = 8;
 template <typename T>
-__global__ void __launch_bounds__(128)
-append_kernel(const T* __restrict__ kv_a, T* __restrict__ pool, uint64_t pool_slots,
-              const T* __restrict__ norm_w, const float* __restrict__ cos_sin, uint32_t cs_rows,
-              float eps, const uint32_t* __restrict__ row_pos,
-              const uint64_t* __restrict__ row_slot, uint32_t* __restrict__ status)
+__global__ void __launch_bounds__(32 * kAppendWarps)
+append_kernel(const AppendArgs a, uint32_t* __restrict__ status)
 {
-    __shared__ __align__(16) T xin[kRow];
-    __shared__ __align__(16) T xout[kRow];
-    __shared__ float sq[kRank];
-    __shared__ float rinv_s;
-    const uint32_t r = blockIdx.x, tid = threadIdx.x;
-    const uint64_t slot = row_slot[r];
-    const uint32_t pos = row_pos[r];
-    if (slot == ~uint64_t(0)) return;          // a query-only row: nothing to append
-    if (slot >= pool_slots || pos >= cs_rows) {
-        if (tid == 0) atomicOr(status, ST_BAD_SLOT);
-        return;
-    }
-    constexpr int kChunks = kRow * 2 / 16;   // 72 x 16 bytes
-    if (tid < kChunks)
-        reinterpret_cast<uint4*>(xin)[tid] =
-            reinterpret_cast<const uint4*>(kv_a + size_t(r) * kRow)[tid];
-    __syncthreads();
-    // squares in parallel (each product is rounded on its own, as in the reference), then ONE
-    // thread adds them in index order: the sum's rounding sequence is the reference's
-    for (int i = tid; i < kRank; i += 128) {
-        const float v = Elem<T>::to_f32(xin[i]);
-        sq[i] = __fmul_rn(v, v);
-    }
-    if (tid >= 32 && tid < 64) {
-        const int i = tid - 32;
-        const float c = cos_sin[size_t(pos) * kRope + i];
-        const float s = cos_sin[size_t(pos) * kRope + 32 + i];
-        const float x0 = Elem<T>::to_f32(xin[kRank + i]);
-        const float x1 = Elem<T>::to_f32(xin[kRank + 32 + i]);
-        xout[kRank + i]      = Elem<T>::from_f32(__fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s)));
-        xout[kRank + 32 + i] = Elem<T>::from_f32(__fadd_rn(__fmul_rn(x1, c), __fmul_rn(x0, s)));
-    }
-    __syncthreads();
-    if (tid == 0) {
-        float ss = 0.0f;
-#pragma unroll 16
-        for (int i = 0; i < kRank; i++) ss = __fadd_rn(ss, sq[i]);
-        rinv_s = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, float(kRank)), eps)));
-    }
-    __syncthreads();
-    const float rinv = rinv_s;
-    for (int i = tid; i < kRank; i += 128) {
-        const float v = __fmul_rn(Elem<T>::to_f32(xin[i]), rinv);
-        xout[i] = Elem<T>::from_f32(__fmul_rn(v, Elem<T>::to_f32(norm_w[i])));
-    }
-    __syncthreads();
-    if (tid < kChunks)
-        reinterpret_cast<uint4*>(pool + slot * kRow)[tid] = reinterpret_cast<const uint4*>(xout)[tid];
+    __shared__ __align__(16) unsigned char smem[kAppendWarps * kAppendRowSmem];
+    grid_launch_dependents();
+    grid_dependency_wait();              // kv_a comes from an earlier kernel of the stream
+    append_row<T>(a, 0, blockIdx.x * kAppendWarps + threadIdx.x / 32, smem + (threadIdx.x / 32) * kAppendRowSmem, status);
 }
 
-void launch_append(int dtype, const void* kv_a, void* layer_pool, uint64_t pool_slots,
-                   const void* norm_w, const float* cos_sin, uint32_t cs_rows, float eps,
-                   const StepMeta& m, uint32_t* status, cudaStream_t st)
+int launch_append(int dtype, const void* kv_a, void* layer_pool, uint64_t pool_slots, const void* norm_w, const float* cos_sin,
+                  uint32_t cs_rows, float eps, const StepMeta& m, uint32_t* status, cudaStream_t st)
 {
-    if (m.app_rows == 0) return;
-    if (dtype == 0)
-        append_kernel<__half><<<m.app_rows, 128, 0, st>>>(
-            static_cast<const __half*>(kv_a), static_cast<__half*>(layer_pool), pool_slots,
-            static_cast<const __half*>(norm_w), cos_sin, cs_rows, eps, m.app_pos, m.app_slot, status);
-    else
-        append_kernel<__nv_bfloat16><<<m.app_rows, 128, 0, st>>>(
-            static_cast<const __nv_bfloat16*>(kv_a), static_cast<__nv_bfloat16*>(layer_pool),
-            pool_slots, static_cast<const __nv_bfloat16*>(norm_w), cos_sin, cs_rows, eps, m.app_pos,
-            m.app_slot, status);
+    if (m.app_rows == 0) return 0;
+    const AppendArgs a{kv_a, layer_pool, pool_slots, norm_w, cos_sin, cs_rows, eps, m.app_pos, m.app_slot, m.app_rows, 1};
+    const dim3 grid((m.app_rows + kAppendWarps - 1) / kAppendWarps), block(32 * kAppendWarps);
+    return dtype == 0 ? int(launch_pdl(append_kernel<__half>, grid, block, 0, st, a, status))
+                      : int(launch_pdl(append_kernel<__nv_bfloat16>, grid, block, 0, st, a, status));
 }
 
 // ------------------------------------------------------------------------------------------
@@ -150,6 +90,8 @@ export_partial_kernel(const float* __restrict__ recs, const RowParts* __restrict
                       float* __restrict__ exported, uint32_t H)
 {
     __shared__ float scratch[16][32][18];
+    grid_launch_dependents();
+    grid_dependency_wait();
     const uint32_t h = blockIdx.x, r = blockIdx.y, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const RowParts rp = parts[r];
     uint32_t pb = rp.begin, pe = rp.end;
@@ -369,10 +311,10 @@ void launch_merge(int dtype, const float* recs, const StepMeta& m, const void* w
             recs, m.parts, m.rec_stride, static_cast<const __nv_bfloat16*>(w_uv), static_cast<__nv_bfloat16*>(out), rows, H);
 }
 
-void launch_export_partial(const float* recs, const StepMeta& m, float* exported, uint32_t H, cudaStream_t st)
+int launch_export_partial(const float* recs, const StepMeta& m, float* exported, uint32_t H, cudaStream_t st)
 {
-    if (m.rows == 0) return;
-    export_partial_kernel<<<dim3(H, m.rows), 512, 0, st>>>(recs, m.parts, m.rec_stride, exported, H);
+    if (m.rows == 0) return 0;
+    return int(launch_pdl(export_partial_kernel, dim3(H, m.rows), dim3(512), 0, st, recs, m.parts, m.rec_stride, exported, H));
 }
 
 }  // namespace mla

@@ -2,11 +2,13 @@
 // include/mugen_mla.h).
 #pragma once
 
+#include <cuda.h>
+
 #include "mla_common.cuh"
 
 namespace mla {
 
-void launch_append(int dtype, const void* kv_a, void* layer_pool, uint64_t pool_slots,
+int launch_append(int dtype, const void* kv_a, void* layer_pool, uint64_t pool_slots,
                    const void* norm_w, const float* cos_sin, uint32_t cs_rows, float eps,
                    const StepMeta& m, uint32_t* status, cudaStream_t st);
 
@@ -53,7 +55,7 @@ int decode_tc5_pair128_configure();
 // Merge of the partial states + W_UV on the warp-level tensor path (the no-allocation entry point), and the merged,
 // un-normalised state of every row written out (the per-GPU partial of a KV-range-sharded sequence).
 void launch_merge(int dtype, const float* recs, const StepMeta& m, const void* w_uv, void* out, uint32_t H, cudaStream_t st);
-void launch_export_partial(const float* recs, const StepMeta& m, float* exported, uint32_t H, cudaStream_t st);
+int launch_export_partial(const float* recs, const StepMeta& m, float* exported, uint32_t H, cudaStream_t st);
 int merge_mma_configure();
 
 // Absorb on tcgen05 (one block per layer, head and 64 rows); w_map: host CUtensorMap over W_UK^T of all layers,
@@ -72,26 +74,55 @@ int launch_merge_tc5(int dtype, const float* recs, const StepMeta& m, uint32_t n
                      uint32_t layer0, uint32_t* status, cudaStream_t st);
 int merge_tc5_configure();
 
-// Dense projection C = A . W^T on tcgen05 (mla_gemm_tc5.cu).  A [M][K] pitch lda, W [N][K] pitch ldw (the reference's
-// matvec weight layout), 16-bit DEVICE operands.  partial == nullptr: C in the storage type to `out`; else float
-// partials [splits][M][N] to be finished by launch_gemm_finalize (mode 0 store, 1 RMSNorm with w / eps, 2 residual
-// add of res).  Return: cudaError_t value, or -1 when a tensor map cannot be built.
-int launch_gemm_tc5(int dtype, const void* A, uint32_t lda, const void* W, uint32_t ldw, uint32_t M, uint32_t N, uint32_t K,
-                    void* out, float* partial, uint32_t splits, uint32_t* status, cudaStream_t st);
-int launch_gemm_finalize(int dtype, const float* partial, uint32_t splits, uint32_t M, uint32_t N, int mode, const void* w,
-                         float eps, const void* res, void* out, cudaStream_t st);
+// Dense projections C = A . W^T on tcgen05 (mla_gemm_tc5.cu), up to two weights over the same activations in one launch.
+struct GemmWeight {
+    const CUtensorMap* map;    // gemm_tc5_weight_map: W [rows][K], box of 64 values x 128 rows
+    uint32_t row0, N;          // first row of the weight inside the map, outputs (a multiple of 8)
+    void* out;                 // DEVICE [M][N] in the storage type
+};
+struct GemmCall {
+    const void* A = nullptr;                   // DEVICE [M][K], 16-byte aligned, or:
+    const CUtensorMap* paged_map = nullptr;    // the cache pool (kMapPoolSub): A = the first M rows of a sequence, K <= 576
+    const uint32_t* table = nullptr;           //   its block table (DEVICE)
+    uint32_t layer = 0, n_pages = 0;
+    uint32_t M = 0, K = 0;
+    int n_weights = 0;
+    GemmWeight w[2];
+    bool residual = false;                     // out = T(float(out) + float(T(x)))
+};
+struct GemmWorkspace {
+    float* partial;            // gemm_tc5_partial_bytes(blocks)
+    uint32_t* counters;        // [max_tiles], zero before the first launch
+    uint32_t blocks, max_tiles;
+};
+int launch_gemm_tc5(int dtype, const GemmCall& g, const GemmWorkspace& ws, uint32_t* status, cudaStream_t st);
+size_t gemm_tc5_partial_bytes(uint32_t blocks);
+bool gemm_tc5_weight_map(CUtensorMap* map, int dtype, const void* W, uint64_t rows, uint64_t K);
 int launch_rmsnorm_rows(int dtype, const void* x, const void* w, void* y, uint32_t rows, uint32_t N, float eps, cudaStream_t st);
-uint32_t gemm_tc5_splits(uint32_t M, uint32_t N, uint32_t K, uint32_t sm_count);   // K slices that fill the SMs once
 int gemm_tc5_configure();
 
-// Chunked prefill (mla_prefill_tc5.cu): gather of a sequence's latent rows into a contiguous buffer, rotation of a
-// chunk's query rows, and causal flash attention of one chunk over expanded keys / values (see the file's header).
-int launch_gather_rows(const void* layer_pool, uint64_t pool_slots, const uint32_t* table, uint32_t n, void* dst, uint32_t* status,
-                       cudaStream_t st);
-int launch_rotate_q_rows(int dtype, const void* q_in, void* q_out, uint32_t rows, uint32_t H, uint32_t pos0, const float* cos_sin,
-                         uint32_t cs_rows, uint32_t* status, cudaStream_t st);
-int launch_prefill_tc5(int dtype, const void* q, uint32_t q_rows_total, uint32_t q_row0, uint32_t n_new, uint32_t start,
-                       const void* kx, const void* vx, const void* latent, void* out, uint32_t H, uint32_t* status, cudaStream_t st);
+// Chunked prefill (mla_prefill_tc5.cu): causal flash attention of the new tokens of several sequences over expanded keys /
+// values (see the file's header).
+struct alignas(16) PrefillTile {       // 128 query tokens of one chunk
+    uint32_t q_row;            // first row of the tile in the caller's q / out
+    uint32_t n_q;              // live query tokens (1..128)
+    uint32_t pos;              // cache row of the tile's first query token in its sequence (causal limit)
+    uint32_t total;            // cache rows of the sequence, the chunk included
+    uint32_t row0;             // first row of the sequence in the expanded keys / values (a multiple of 128)
+    uint32_t rope_pos;         // global position of the first query token
+    uint32_t pad[2];
+};
+struct PrefillCall {
+    const void *q = nullptr, *kx = nullptr, *vx = nullptr;      // q [..][H][192]; kx / vx [rows][H][128]
+    void* out = nullptr;                                        // [..][H][128]
+    const CUtensorMap* pool_map = nullptr;                      // kMapPoolSub: the shared rope keys come from the cache pages
+    const uint32_t* pages = nullptr;                            // page of every 64 expanded rows (DEVICE)
+    const PrefillTile* tiles = nullptr;                         // (DEVICE)
+    uint32_t n_tiles = 0, rows = 0, H = 0, layer = 0, n_pages = 0;
+    const float* cos_sin = nullptr;                             // not null: q arrives before its RoPE
+    uint32_t cs_rows = 0;
+};
+int launch_prefill_tc5(int dtype, const PrefillCall& p, uint32_t* status, cudaStream_t st);
 int prefill_tc5_configure();
 
 // One block that waits `limit_cycles` on a barrier nothing completes, raises ST_WAIT_TIMEOUT in *status, frees its

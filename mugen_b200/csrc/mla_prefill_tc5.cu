@@ -13,8 +13,8 @@
 // One block per (tile of 128 query tokens, head); the whole tile state lives in tensor memory:
 //   Q        [128 queries][192 dims] written once into tensor memory by the softmax threads (row = lane, two dims per
 //            column) and used as the A operand of every score MMA: no shared-memory reads for it
-//   TMA      per step of KT = 128 keys K [128][192] (two boxes of expanded nope dims + one box of rope dims straight from
-//            the gathered latent rows) and V [128][128], rings of two each; a K buffer is free as soon as the score MMAs
+//   TMA      per step of KT = 128 keys K [128][192] (two boxes of expanded nope dims + the rope dims straight from the two
+//            cache pages) and V [128][128], rings of two each; a K buffer is free as soon as the score MMAs
 //            that read it complete, a V buffer one softmax later
 //   QK       S[128 queries x 128 keys] = Q . K^T         12 x tcgen05.mma M128 N128 K16 (A in tensor memory), two score
 //            tiles in flight (steps of 64 keys with rings of four and three score tiles measure 13 % slower: the fixed
@@ -74,18 +74,12 @@ enum { B_QFULL = 0, B_KFULL, B_KEMPTY = B_KFULL + K_STAGES, B_VFULL = B_KEMPTY +
 static_assert(B_COUNT * 8 <= M_HMAX && B_COUNT <= 32, "barriers overflow their area");
 static_assert(SMEM_BYTES <= 232448, "over the shared memory of one block");
 
-struct ChunkArgs {
-    uint32_t q_row0;        // first query row of the chunk in the q / out tensors
-    uint32_t n_new;         // query tokens in the chunk
-    uint32_t start;         // cache rows of the sequence before the chunk
-    uint32_t H;
-};
-
 template <typename T>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                   const __grid_constant__ CUtensorMap map_r, ChunkArgs a, T* __restrict__ out, float scale_log2,
-                   uint32_t* __restrict__ status)
+                   const __grid_constant__ CUtensorMap map_r, const PrefillTile* __restrict__ tiles, const uint32_t* __restrict__ pages,
+                   uint32_t H, uint32_t layer, uint32_t n_pages, const float* __restrict__ cos_sin, uint32_t cs_rows, T* __restrict__ out,
+                   float scale_log2, uint32_t* __restrict__ status)
 {
     extern __shared__ unsigned char prefill_smem[];
     const uint32_t raw = smem_u32(prefill_smem);
@@ -99,11 +93,15 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + M_ABORT);
 
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-    // long tiles first: the last query tile of a chunk sees the most keys
-    const uint32_t n_qt = (a.n_new + QT - 1) / QT, qt = n_qt - 1 - blockIdx.x, h = blockIdx.y;
-    const uint32_t q0 = qt * QT;                                   // first query token of this tile within the chunk
-    const uint32_t total = a.start + a.n_new;
-    const uint32_t kv_end = min(total, a.start + q0 + QT);         // keys any query of this tile may see
+    // the list is sorted, tiles that see the most keys first; the step's metadata was uploaded before its first kernel
+    PrefillTile a;
+    {
+        const uint4* p = reinterpret_cast<const uint4*>(tiles + blockIdx.x);
+        const uint4 x = __ldg(p), y = __ldg(p + 1);
+        a.q_row = x.x; a.n_q = x.y; a.pos = x.z; a.total = x.w; a.row0 = y.x; a.rope_pos = y.y;
+    }
+    const uint32_t h = blockIdx.y, total = a.total;
+    const uint32_t kv_end = min(total, a.pos + QT);                // keys any query of this tile may see
     const uint32_t n_kv = (kv_end + KT - 1) / KT;
 
     grid_launch_dependents();
@@ -123,21 +121,35 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
     if (warp == 0) {
         if (lane == 0) {
             bool ok = true;
+            constexpr int PG = KT / kPage;
+            const uint32_t* pg_list = pages + a.row0 / kPage;
+            uint32_t page[PG], next[PG];                             // page ids are requested a step ahead of their use
+#pragma unroll
+            for (int i = 0; i < PG; i++) next[i] = __ldg(pg_list + i);
             for (uint32_t t = 0; t < n_kv && ok; t++) {
+#pragma unroll
+                for (int i = 0; i < PG; i++) {
+                    page[i] = next[i];
+                    if (page[i] >= n_pages) { atomicOr(status, ST_BAD_PAGE); page[i] = 0; }
+                    next[i] = __ldg(pg_list + min(t + 1, n_kv - 1) * PG + i);
+                }
                 const int ks = int(t % K_STAGES), vs = int(t % V_STAGES);
                 ok = mbar_wait(bar(B_KEMPTY + ks), ((t / K_STAGES) & 1) ^ 1, abort_flag, status);
                 if (!ok) break;
                 const uint32_t kd = sK + ks * K_STAGE;
                 mbar_expect_tx(bar(B_KFULL + ks), K_STAGE);
-                tma_load_2d(kd, &map_k, bar(B_KFULL + ks), int(h * kNope), int(t * KT));
-                tma_load_2d(kd + K_SUB, &map_k, bar(B_KFULL + ks), int(h * kNope + 64), int(t * KT));
-                tma_load_2d(kd + 2 * K_SUB, &map_r, bar(B_KFULL + ks), kRank, int(t * KT));
+                const int row = int(a.row0 + t * KT);
+                tma_load_2d(kd, &map_k, bar(B_KFULL + ks), int(h * kNope), row);
+                tma_load_2d(kd + K_SUB, &map_k, bar(B_KFULL + ks), int(h * kNope + 64), row);
+#pragma unroll
+                for (int i = 0; i < PG; i++)                         // the rope keys of each page
+                    tma_load_3d(kd + 2 * K_SUB + i * kPage * 128, &map_r, bar(B_KFULL + ks), kRank, int(page[i] * kPage), int(layer));
                 ok = mbar_wait(bar(B_VEMPTY + vs), ((t / V_STAGES) & 1) ^ 1, abort_flag, status);
                 if (!ok) break;
                 const uint32_t vd = sV + vs * V_STAGE;
                 mbar_expect_tx(bar(B_VFULL + vs), V_STAGE);
-                tma_load_2d(vd, &map_v, bar(B_VFULL + vs), int(h * kVDim), int(t * KT));
-                tma_load_2d(vd + K_SUB, &map_v, bar(B_VFULL + vs), int(h * kVDim + 64), int(t * KT));
+                tma_load_2d(vd, &map_v, bar(B_VFULL + vs), int(h * kVDim), row);
+                tma_load_2d(vd + K_SUB, &map_v, bar(B_VFULL + vs), int(h * kVDim + 64), row);
             }
         }
     } else if (warp == 1) {
@@ -192,22 +204,40 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
         static_assert(NS == 1 || NS == 2 || NS == 4, "the part sizes below");
         const uint32_t q4 = warp % 4, part = (warp - FIRST_SOFTMAX_WARP) / 4, r = q4 * 32 + lane;
         const uint32_t lane_base = (q4 * 32u) << 16;
-        const uint32_t qi = q0 + r;                                      // query token within the chunk
-        const bool live = qi < a.n_new;
-        const uint32_t my_pos = a.start + qi;                            // last key this query may see
+        const bool live = r < a.n_q;
+        const uint32_t my_pos = a.pos + r;                               // last key this query may see
         {   // this thread's part of the query row: QP dims = QP / 2 columns, in three stores
             constexpr int W = QP / 6;
-            const uint4* src = reinterpret_cast<const uint4*>(q + (size_t(a.q_row0 + qi) * a.H + h) * kQDim + part * QP);
+            static_assert(NS == 2, "part 1 holds dims 96..191, all of the rope dims among them");
+            const uint4* src = reinterpret_cast<const uint4*>(q + (size_t(a.q_row + r) * H + h) * kQDim + part * QP);
+            uint32_t w[3][W];
 #pragma unroll
-            for (int c = 0; c < 3; c++) {
-                uint32_t w[W];
+            for (int c = 0; c < 3; c++)
 #pragma unroll
                 for (int j = 0; j < W / 4; j++) {
                     const uint4 v = live ? __ldg(src + c * (W / 4) + j) : make_uint4(0u, 0u, 0u, 0u);
-                    w[4 * j] = v.x; w[4 * j + 1] = v.y; w[4 * j + 2] = v.z; w[4 * j + 3] = v.w;
+                    w[c][4 * j] = v.x; w[c][4 * j + 1] = v.y; w[c][4 * j + 2] = v.z; w[c][4 * j + 3] = v.w;
                 }
-                tc_stn(tmem + lane_base + COL_Q + part * (QP / 2) + c * W, w);
+            if (cos_sin != nullptr && part == 1 && live) {
+                // q-side RoPE (NeoX pairs, the append's table and rounding: reference transformer.cpp:1204-1240): w[1] holds dims
+                // 128..159, w[2] their partners 160..191
+                const uint32_t pos = a.rope_pos + r;
+                if (pos >= cs_rows) {
+                    atomicOr(status, ST_BAD_SLOT);
+                } else {
+                    const float2* cp = reinterpret_cast<const float2*>(cos_sin + size_t(pos) * kRope);
+#pragma unroll
+                    for (int j = 0; j < W; j++) {
+                        const float2 cs = __ldg(cp + j), sn = __ldg(cp + 16 + j);
+                        const T *x0 = reinterpret_cast<const T*>(&w[1][j]), *x1 = reinterpret_cast<const T*>(&w[2][j]);
+                        const float a0 = Elem<T>::to_f32(x0[0]), a1 = Elem<T>::to_f32(x0[1]), b0 = Elem<T>::to_f32(x1[0]), b1 = Elem<T>::to_f32(x1[1]);
+                        w[1][j] = Elem<T>::pack2(__fsub_rn(__fmul_rn(a0, cs.x), __fmul_rn(b0, sn.x)), __fsub_rn(__fmul_rn(a1, cs.y), __fmul_rn(b1, sn.y)));
+                        w[2][j] = Elem<T>::pack2(__fadd_rn(__fmul_rn(b0, cs.x), __fmul_rn(a0, sn.x)), __fadd_rn(__fmul_rn(b1, cs.y), __fmul_rn(a1, sn.y)));
+                    }
+                }
             }
+#pragma unroll
+            for (int c = 0; c < 3; c++) tc_stn(tmem + lane_base + COL_Q + part * (QP / 2) + c * W, w[c]);
             tc_wait_st();
             tc_fence_before();
             mbar_arrive(bar(B_QFULL));
@@ -305,7 +335,7 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
 #pragma unroll
             for (int p = 0; p < NS; p++) l += lsum_s[p * QT + r];
             const float linv = l > 0.0f ? 1.0f / l : 0.0f;
-            uint4* dst = reinterpret_cast<uint4*>(out + (size_t(a.q_row0 + qi) * a.H + h) * kVDim + part * VP);
+            uint4* dst = reinterpret_cast<uint4*>(out + (size_t(a.q_row + r) * H + h) * kVDim + part * VP);
 #pragma unroll 1
             for (uint32_t c = 0; c < VP / 32; c++) {
                 uint32_t o[32];
@@ -328,45 +358,6 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
         tc_fence_after();
         tc_dealloc<TMEM_COLS>(tmem);
     }
-}
-
-// rows [0, n) of a sequence, page by page, into a contiguous [n][576] buffer
-__global__ void __launch_bounds__(128)
-gather_rows_kernel(const uint4* __restrict__ pool, uint64_t pool_slots, const uint32_t* __restrict__ table, uint32_t n,
-                   uint4* __restrict__ dst, uint32_t* __restrict__ status)
-{
-    grid_launch_dependents();
-    grid_dependency_wait();
-    constexpr int kChunks = kRow * 2 / 16;
-    const uint32_t r = blockIdx.x * 4 + threadIdx.x / 32;
-    if (r >= n) return;
-    const uint64_t slot = uint64_t(table[r / kPage]) * kPage + r % kPage;
-    if (slot >= pool_slots) {
-        if ((threadIdx.x & 31) == 0) atomicOr(status, ST_BAD_SLOT);
-        return;
-    }
-    for (int c = threadIdx.x & 31; c < kChunks; c += 32) dst[size_t(r) * kChunks + c] = pool[slot * kChunks + c];
-}
-
-// the last 64 dims of every head of `rows` query rows rotated with their positions (NeoX pairs, the append's table and
-// rounding: reference transformer.cpp:1204-1240), everything else copied: q_out = rotated copy of q_in
-template <typename T>
-__global__ void __launch_bounds__(192)
-rotate_q_rows_kernel(const T* __restrict__ q_in, T* __restrict__ q_out, uint32_t H, uint32_t pos0, const float* __restrict__ cos_sin,
-                     uint32_t cs_rows, uint32_t* __restrict__ status)
-{
-    grid_launch_dependents();
-    grid_dependency_wait();
-    const uint32_t row = blockIdx.x, h = blockIdx.y, i = threadIdx.x, pos = pos0 + row;
-    const T* src = q_in + (size_t(row) * H + h) * kQDim;
-    T* dst = q_out + (size_t(row) * H + h) * kQDim;
-    if (i < kNope) { dst[i] = src[i]; return; }
-    if (pos >= cs_rows) { if (i == kNope) atomicOr(status, ST_BAD_SLOT); return; }
-    const uint32_t j = (i - kNope) % 32;
-    const float cs = cos_sin[size_t(pos) * kRope + j], sn = cos_sin[size_t(pos) * kRope + 32 + j];
-    const float x0 = Elem<T>::to_f32(src[kNope + j]), x1 = Elem<T>::to_f32(src[kNope + 32 + j]);
-    dst[i] = i < kNope + 32 ? Elem<T>::from_f32(__fsub_rn(__fmul_rn(x0, cs), __fmul_rn(x1, sn)))
-                            : Elem<T>::from_f32(__fadd_rn(__fmul_rn(x1, cs), __fmul_rn(x0, sn)));
 }
 
 using TensorMapEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -402,48 +393,23 @@ int prefill_tc5_configure()
     return int(e);
 }
 
-int launch_gather_rows(const void* layer_pool, uint64_t pool_slots, const uint32_t* table, uint32_t n, void* dst, uint32_t* status,
-                       cudaStream_t st)
+// Returns a cudaError_t value, or -1 when a tensor map cannot be built.
+int launch_prefill_tc5(int dtype, const PrefillCall& p, uint32_t* status, cudaStream_t st)
 {
-    if (n == 0) return 0;
-    return int(launch_pdl(gather_rows_kernel, dim3((n + 3) / 4), dim3(128), 0, st, static_cast<const uint4*>(layer_pool), pool_slots,
-                          table, n, static_cast<uint4*>(dst), status));
-}
-
-int launch_rotate_q_rows(int dtype, const void* q_in, void* q_out, uint32_t rows, uint32_t H, uint32_t pos0, const float* cos_sin,
-                         uint32_t cs_rows, uint32_t* status, cudaStream_t st)
-{
-    if (rows == 0) return 0;
-    if (dtype == 0)
-        return int(launch_pdl(rotate_q_rows_kernel<__half>, dim3(rows, H), dim3(192), 0, st, static_cast<const __half*>(q_in),
-                              static_cast<__half*>(q_out), H, pos0, cos_sin, cs_rows, status));
-    return int(launch_pdl(rotate_q_rows_kernel<__nv_bfloat16>, dim3(rows, H), dim3(192), 0, st, static_cast<const __nv_bfloat16*>(q_in),
-                          static_cast<__nv_bfloat16*>(q_out), H, pos0, cos_sin, cs_rows, status));
-}
-
-// One chunk of one sequence.  q: [q_rows_total][H][192] post-RoPE (DEVICE), chunk rows start at q_row0; kx / vx: expanded keys
-// (nope dims) and values [total][H][128]; latent: the gathered rows [total][576] (their last 64 dims are the shared rope
-// keys); out: [q_rows_total][H][128].  Returns a cudaError_t value, or -1 when a tensor map cannot be built.
-int launch_prefill_tc5(int dtype, const void* q, uint32_t q_rows_total, uint32_t q_row0, uint32_t n_new, uint32_t start,
-                       const void* kx, const void* vx, const void* latent, void* out, uint32_t H, uint32_t* status, cudaStream_t st)
-{
-    if (n_new == 0) return 0;
-    const uint32_t total = start + n_new;
-    if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15u) return int(cudaErrorMisalignedAddress);
-    (void)q_rows_total;
-    alignas(64) CUtensorMap mk, mv, mr;
-    if (!make_map(&mk, dtype, kx, total, uint64_t(H) * kNope, uint64_t(H) * kNope, KT) ||
-        !make_map(&mv, dtype, vx, total, uint64_t(H) * kVDim, uint64_t(H) * kVDim, KT) ||
-        !make_map(&mr, dtype, latent, total, kRow, kRow, KT))
+    if (p.n_tiles == 0) return 0;
+    if ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.out)) & 15u) return int(cudaErrorMisalignedAddress);
+    alignas(64) CUtensorMap mk, mv;
+    if (!make_map(&mk, dtype, p.kx, p.rows, uint64_t(p.H) * kNope, uint64_t(p.H) * kNope, KT) ||
+        !make_map(&mv, dtype, p.vx, p.rows, uint64_t(p.H) * kVDim, uint64_t(p.H) * kVDim, KT))
         return -1;
-    const ChunkArgs a{q_row0, n_new, start, H};
     const float scale_log2 = 1.4426950408889634f / sqrtf(float(kQDim));
-    dim3 grid((n_new + QT - 1) / QT, H);
-    if (dtype == 0)
-        return int(launch_pdl(prefill_tc5_kernel<__half>, grid, dim3(NUM_THREADS), SMEM_BYTES, st, static_cast<const __half*>(q),
-                              mk, mv, mr, a, static_cast<__half*>(out), scale_log2, status));
-    return int(launch_pdl(prefill_tc5_kernel<__nv_bfloat16>, grid, dim3(NUM_THREADS), SMEM_BYTES, st,
-                          static_cast<const __nv_bfloat16*>(q), mk, mv, mr, a, static_cast<__nv_bfloat16*>(out), scale_log2, status));
+    dim3 grid(p.n_tiles, p.H);
+    auto go = [&](auto kernel, auto* q, auto* out) {
+        return int(launch_pdl(kernel, grid, dim3(NUM_THREADS), SMEM_BYTES, st, q, mk, mv, *p.pool_map, p.tiles, p.pages, p.H, p.layer, p.n_pages,
+                              p.cos_sin, p.cs_rows, out, scale_log2, status));
+    };
+    return dtype == 0 ? go(prefill_tc5_kernel<__half>, static_cast<const __half*>(p.q), static_cast<__half*>(p.out))
+                      : go(prefill_tc5_kernel<__nv_bfloat16>, static_cast<const __nv_bfloat16*>(p.q), static_cast<__nv_bfloat16*>(p.out));
 }
 
 }  // namespace mla
