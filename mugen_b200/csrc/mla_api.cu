@@ -48,7 +48,7 @@ enum { kPlanStep = 0, kPlanRest, kPlanStack, kPlanStackTail, kPlanRegions };
 struct BlockW {
     uint32_t embed = 0, q_lora = 0;
     void *attn_norm = nullptr, *q_a = nullptr, *q_a_norm = nullptr, *q_b = nullptr, *q = nullptr, *kv_a = nullptr, *wo = nullptr;
-    alignas(64) CUtensorMap q_a_map, q_b_map, q_map, kv_a_map, wo_map;
+    mla::GemmWeightMaps q_a_map, q_b_map, q_map, kv_a_map, wo_map;
     bool set = false;
 };
 
@@ -76,7 +76,8 @@ struct mla_ctx {
     char* w_uv = nullptr;            // [layers][H*128][512]
     char* norm = nullptr;            // [layers][512]
     std::vector<char> layer_set;     // weights registered
-    alignas(64) CUtensorMap w_uk_map, w_uk_rows_map, w_uv_map;
+    alignas(64) CUtensorMap w_uk_map, w_uv_map;
+    mla::GemmWeightMaps w_uk_rows_maps, w_uv_maps;       // the same weights for the prefill expansion
     std::vector<BlockW> blocks;
     // workspaces of the block projections, grown on demand: normalised hidden state, q_a,
     // and the block's q / kv_a / attention output when the library owns them (mla_step_block)
@@ -534,6 +535,11 @@ int grow_buf(mla_ctx* c, void** p, size_t* cap, size_t bytes)
     return MLA_OK;
 }
 
+mla::GemmWeight gemm_weight(const mla::GemmWeightMaps& maps, uint32_t n_outputs, void* out, uint32_t row0 = 0)
+{
+    return mla::GemmWeight{&maps.box128, &maps.box64, row0, n_outputs, out};
+}
+
 // The chunks of the open step: expand each sequence's latent rows (the chunk's own were appended by the launch before) into
 // per-head keys and values with W_UK / W_UV, straight from the cache pages, and run causal flash attention of the chunks'
 // queries over them.  Reference semantics: src/core/model/transformer.cpp:1263-1337.
@@ -552,8 +558,8 @@ int run_chunks(mla_ctx* c, uint32_t layer, const void* q, void* out, cudaStream_
         gc.M = g.rows;
         gc.K = mla::kRank;
         gc.n_weights = 2;
-        gc.w[0] = mla::GemmWeight{&c->w_uk_rows_map, layer * H * mla::kNope, H * mla::kNope, c->pf_kx};
-        gc.w[1] = mla::GemmWeight{&c->w_uv_map, layer * H * mla::kVDim, H * mla::kVDim, c->pf_vx};
+        gc.w[0] = gemm_weight(c->w_uk_rows_maps, H * mla::kNope, c->pf_kx, layer * H * mla::kNope);
+        gc.w[1] = gemm_weight(c->w_uv_maps, H * mla::kVDim, c->pf_vx, layer * H * mla::kVDim);
         int rc = mla::launch_gemm_tc5(dt, gc, c->gemm_ws, c->status_dev, st);
         if (rc) return fail(c, rc == -1 ? MLA_ERR_INVALID : MLA_ERR_CUDA, "key / value expansion launch failed");
         mla::PrefillCall p;
@@ -637,7 +643,9 @@ int make_tensor_maps(mla_ctx* c)
         };
         const cuuint64_t heads = cuuint64_t(c->cfg.n_layers) * c->cfg.n_heads;
         if (int e = weights(&c->w_uv_map, "W_UV", c->w_uv, mla::kRank, heads * mla::kVDim, mla::kVDim)) return e;
-        if (int e = weights(&c->w_uk_rows_map, "W_UK rows", c->w_uk_rows, mla::kRank, heads * mla::kNope, mla::kNope)) return e;
+        if (!mla::gemm_tc5_weight_maps(&c->w_uk_rows_maps, int(c->cfg.dtype), c->w_uk_rows, heads * mla::kNope, mla::kRank) ||
+            !mla::gemm_tc5_weight_maps(&c->w_uv_maps, int(c->cfg.dtype), c->w_uv, heads * mla::kVDim, mla::kRank))
+            return fail(c, MLA_ERR_CUDA, "cuTensorMapEncodeTiled(expansion weights) failed");
         if (int e = weights(&c->w_uk_map, "W_UK", c->w_uk, mla::kNope, heads * mla::kRank, 256)) return e;
     }
     {   // cache pool: 576 values innermost, then the token slots of a layer, then layers;
@@ -1460,12 +1468,12 @@ int project_in(mla_ctx* c, const BlockW& b, uint32_t rows, const void* hidden, v
     const uint32_t E = b.embed, H = c->cfg.n_heads, QD = H * uint32_t(mla::kQDim);
     if (int e = grow(c, &c->blk_hidden2, &c->blk_hidden2_cap, size_t(rows) * E * 2)) return e;
     if (int e = rmsnorm(c, hidden, b.attn_norm, c->blk_hidden2, rows, E, st)) return e;
-    const mla::GemmWeight kv{&b.kv_a_map, 0, uint32_t(mla::kRow), kv_a};
-    if (!b.q_lora) return project(c, c->blk_hidden2, rows, E, {{&b.q_map, 0, QD, q}, kv}, false, st);
+    const mla::GemmWeight kv = gemm_weight(b.kv_a_map, uint32_t(mla::kRow), kv_a);
+    if (!b.q_lora) return project(c, c->blk_hidden2, rows, E, {gemm_weight(b.q_map, QD, q), kv}, false, st);
     if (int e = grow(c, &c->blk_qa, &c->blk_qa_cap, size_t(rows) * b.q_lora * 2)) return e;
-    if (int e = project(c, c->blk_hidden2, rows, E, {{&b.q_a_map, 0, b.q_lora, c->blk_qa}, kv}, false, st)) return e;
+    if (int e = project(c, c->blk_hidden2, rows, E, {gemm_weight(b.q_a_map, b.q_lora, c->blk_qa), kv}, false, st)) return e;
     if (int e = rmsnorm(c, c->blk_qa, b.q_a_norm, c->blk_qa, rows, b.q_lora, st)) return e;
-    return project(c, c->blk_qa, rows, b.q_lora, {{&b.q_b_map, 0, QD, q}}, false, st);
+    return project(c, c->blk_qa, rows, b.q_lora, {gemm_weight(b.q_b_map, QD, q)}, false, st);
 }
 
 }  // namespace
@@ -1499,10 +1507,10 @@ int mla_set_block_weights(mla_ctx* c, uint32_t layer, const mla_block_weights* w
     if (int e = put(&b.wo, w->wo, size_t(E) * H * mla::kVDim)) return e;
     const int dt = int(c->cfg.dtype);
     const uint32_t QD = H * uint32_t(mla::kQDim);
-    if (!(R ? mla::gemm_tc5_weight_map(&b.q_a_map, dt, b.q_a, R, E) && mla::gemm_tc5_weight_map(&b.q_b_map, dt, b.q_b, QD, R)
-            : mla::gemm_tc5_weight_map(&b.q_map, dt, b.q, QD, E)) ||
-        !mla::gemm_tc5_weight_map(&b.kv_a_map, dt, b.kv_a, uint64_t(mla::kRow), E) ||
-        !mla::gemm_tc5_weight_map(&b.wo_map, dt, b.wo, E, uint64_t(H) * mla::kVDim))
+    if (!(R ? mla::gemm_tc5_weight_maps(&b.q_a_map, dt, b.q_a, R, E) && mla::gemm_tc5_weight_maps(&b.q_b_map, dt, b.q_b, QD, R)
+            : mla::gemm_tc5_weight_maps(&b.q_map, dt, b.q, QD, E)) ||
+        !mla::gemm_tc5_weight_maps(&b.kv_a_map, dt, b.kv_a, uint64_t(mla::kRow), E) ||
+        !mla::gemm_tc5_weight_maps(&b.wo_map, dt, b.wo, E, uint64_t(H) * mla::kVDim))
         return fail(c, MLA_ERR_CUDA, "cuTensorMapEncodeTiled(projection weights) failed");
     b.embed = E;
     b.q_lora = R;
@@ -1528,7 +1536,7 @@ int mla_block_project_out(mla_ctx* c, uint32_t layer, uint32_t rows, const void*
     if (int e = block_of(c, layer, &b)) return e;
     if (rows == 0) return MLA_OK;
     // hidden = hidden + W_o . attn_out
-    return project(c, attn_out, rows, c->cfg.n_heads * uint32_t(mla::kVDim), {{&b->wo_map, 0, b->embed, hidden}}, true,
+    return project(c, attn_out, rows, c->cfg.n_heads * uint32_t(mla::kVDim), {gemm_weight(b->wo_map, b->embed, hidden)}, true,
                    static_cast<cudaStream_t>(stream));
 }
 
@@ -1550,7 +1558,7 @@ int mla_step_block(mla_ctx* c, uint32_t layer, void* hidden, void* stream)
     if (int e = grow(c, &c->blk_out, &c->blk_out_cap, size_t(rows) * H * mla::kVDim * 2)) return e;
     if (int e = project_in(c, *b, rows, hidden, c->blk_q, c->blk_kv, st)) return e;
     if (int e = run_layer(c, layer, c->blk_kv, c->blk_q, c->blk_out, st)) return e;
-    return project(c, c->blk_out, rows, H * uint32_t(mla::kVDim), {{&b->wo_map, 0, b->embed, hidden}}, true, st);
+    return project(c, c->blk_out, rows, H * uint32_t(mla::kVDim), {gemm_weight(b->wo_map, b->embed, hidden)}, true, st);
 }
 
 }  // extern "C"

@@ -10,16 +10,19 @@
 // prefill path (M = tokens, K = 512).  Up to two weight matrices over the same activations share a launch (q and kv_a;
 // W_UK and W_UV).
 //
-// Work = (output tile, k-block of 64) units in one line; every SM gets an equal run of them (one persistent block per SM),
-// so a launch is balanced whatever its tile count.  A tile cut by a run boundary is finished by the block that arrives
-// last at the tile's counter: every contributor leaves its float partial in global memory (L2), the last one adds them in
-// the order of the runs (bit-reproducible) and stores.  Where there are many tiles per SM, runs end on tile boundaries.
-// Two orientations of one kernel:
-//   kSwap   up to 128 rows: 128 weight rows are the M side of the MMA, the rows of A its N side (16, 32, 64 or 128
-//           columns): the bytes in flight are weight bytes, and a step of 4 rows does not pay for 128.
-//   !kSwap  more rows: 128 rows of A x 256 outputs per tile; tiles of the storage type leave through shared memory and TMA.
-// Warps: 0 TMA producer (the first stages' weight tiles are constant and requested before the grid dependency is
-// waited for), 1 MMA issuer (tcgen05.mma M128 N=NT K16), 2-5 epilogue, two accumulators in turn.
+// Work = (output tile, k-block of 64) units in one line; every worker (a block, or a pair of blocks) gets an equal run of
+// them, so a launch is balanced whatever its tile count.  A tile cut by a run boundary is finished by the worker that
+// arrives last at the tile's counter: every contributor leaves its float partial in global memory (L2), the last one adds
+// them in the order of the runs (bit-reproducible) and stores.  Where that costs more than it saves, runs end on tile
+// boundaries (pick_shape).
+//   up to 128 rows   gemm_rows_kernel, one block per SM: 128 weight rows are the M side of the MMA, the rows of A its N side
+//                    (16, 32, 64 or 128 columns): the bytes in flight are weight bytes, and a step of 4 rows does not pay
+//                    for 128.  HBM-bound.
+//   more rows        gemm_pair_kernel on SM pairs (tcgen05.mma.cta_group::2): 256 rows of A x 256 or 128 outputs per tile, each
+//                    block holding 128 rows of A and half of the outputs' weight rows.  What bounds it is the L2 -> shared
+//                    memory feed (measured with one block per 128 x 256 tile: 48 KB per 4.2 MFLOP k-block, 930 TFLOP/s =
+//                    10.7 TB/s): the pair needs 32 KB for the same work.  Finished tiles leave through shared memory and TMA.
+// The first stages' weight tiles are constant and requested before the grid dependency is waited for.
 #include <cuda.h>
 
 #include <algorithm>
@@ -33,31 +36,45 @@ namespace {
 
 using namespace tc5;
 
-constexpr int BM = 128, BK = 64;                         // M side of the MMA, k-block
+constexpr int BM = 128, BK = 64;                         // M side of one block's MMA, k-block
 constexpr int A_BYTES = BM * BK * 2;                     // 16,384
 constexpr int STORE_BYTES = BM * 128;                    // one box of 64 outputs x 128 rows on its way out
 constexpr int NUM_THREADS = 32 * 6;
-constexpr int stage_bytes(int nt) { return A_BYTES + nt * BK * 2; }
-constexpr int n_stages(int nt) { return nt == 256 ? 4 : nt == 128 ? 6 : nt == 64 ? 8 : nt == 32 ? 10 : 11; }
-constexpr int off_store(int nt) { return n_stages(nt) * stage_bytes(nt); }
-constexpr int off_misc(int nt) { return off_store(nt) + (nt == 256 ? 2 * STORE_BYTES : 0); }
 constexpr int MISC_BYTES = 256;
-constexpr int smem_bytes(int nt) { return off_misc(nt) + MISC_BYTES + 1024; }      // + slack for 1 KB alignment
-static_assert(smem_bytes(256) <= 232448 && smem_bytes(16) <= 232448 && smem_bytes(128) <= 232448, "shared memory of one block");
+// gemm_rows_kernel: [128 weight rows][NT rows of A] per stage
+constexpr int rows_stage(int nt) { return A_BYTES + nt * BK * 2; }
+constexpr int rows_stages(int nt) { return nt == 128 ? 6 : nt == 64 ? 8 : nt == 32 ? 10 : 11; }
+constexpr int rows_smem(int nt) { return rows_stages(nt) * rows_stage(nt) + MISC_BYTES + 1024; }      // + slack for 1 KB alignment
+// gemm_pair_kernel: [128 rows of A][NT / 2 weight rows] per block and stage
+constexpr int pair_stage(int nt) { return A_BYTES + nt / 2 * BK * 2; }
+constexpr int pair_stages(int nt) { return nt == 256 ? 6 : 8; }
+constexpr int pair_off_store(int nt) { return pair_stages(nt) * pair_stage(nt); }
+constexpr int pair_smem(int nt) { return pair_off_store(nt) + 2 * STORE_BYTES + MISC_BYTES + 1024; }
+static_assert(rows_smem(16) <= 232448 && rows_smem(128) <= 232448 && pair_smem(256) <= 232448 && pair_smem(128) <= 232448, "shared memory of one block");
 
 struct GemmArgs {
     uint32_t M, kb;                     // rows of A, k-blocks
     uint32_t m_tiles, n_tiles[2];       // tiles along the rows of A, and along the outputs of each weight
     uint32_t N[2], w_row0[2];           // outputs of each weight; first row of the weight inside its map
-    uint32_t whole_tiles;               // runs end on tile boundaries
+    uint32_t units, run;                // tiles x k-blocks, and how many of them a worker takes
     uint32_t residual;                  // out = T(float(out) + float(T(x))) instead of T(x)
-    uint32_t tile_store;                // !kSwap: outputs leave by TMA
+    uint32_t tile_store;                // pairs: outputs leave by TMA
     uint32_t vec_io;                    // outputs start on a 16-byte boundary
-    const uint32_t* table;              // paged A: block table of the sequence (64 rows per page), else nullptr
+    const uint32_t* table;              // paged A: page of every 64 rows, else nullptr
     uint32_t layer, n_pages;
     float* partial;                     // [2 x blocks][NT/4][128] float4
-    uint32_t* counters;                 // [tiles], zero between launches
+    uint32_t* counters;                 // [tiles], pairs: [tiles][2]; zero between launches
 };
+
+struct Tile { uint32_t w, m, n; };      // which weight, tile along A's rows, tile along its outputs
+__device__ __forceinline__ Tile tile_of(const GemmArgs& a, uint32_t t) {
+    Tile r;
+    const uint32_t nt = t / a.m_tiles;
+    r.m = t % a.m_tiles;
+    r.w = nt >= a.n_tiles[0] ? 1u : 0u;
+    r.n = nt - (r.w ? a.n_tiles[0] : 0u);
+    return r;
+}
 
 // eight 16-bit values at any alignment of the type
 template <typename T>
@@ -78,50 +95,100 @@ __device__ __forceinline__ void store8(T* p, const uint4& v, bool vec) {
     for (int j = 0; j < 4; j++) { h[2 * j] = uint16_t(w[j]); h[2 * j + 1] = uint16_t(w[j] >> 16); }
 }
 
-template <typename T, int NT, bool kSwap, bool kPaged>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
-gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
-                const __grid_constant__ CUtensorMap map_c0, const __grid_constant__ CUtensorMap map_c1, T* __restrict__ out0, T* __restrict__ out1,
-                const GemmArgs a, uint32_t* __restrict__ status)
+template <int CH>
+__device__ __forceinline__ void load_acc(uint32_t addr, float (&v)[CH]) {
+    uint32_t x[CH];
+    tc_ldn(addr, x);
+    tc_wait_ld();
+#pragma unroll
+    for (int i = 0; i < CH; i++) v[i] = __uint_as_float(x[i]);
+}
+__device__ __forceinline__ void epilogue_sync() { asm volatile("barrier.cta.sync 1, 128;\n" ::: "memory"); }
+
+// The 128 epilogue threads hand a cut tile's accumulator (row r of it, NT columns, at tensor-memory address acc) over:
+// partial to global memory, then the tile's counter.  Returns true in the worker that arrived last; `sum(c, v)` then gives
+// columns c*CH.. of the whole tile.  Worker w's slots are 2w (the tile its run begins in) and 2w + 1 (the one it ends in).
+template <int NT, int CH, typename Release>
+__device__ __forceinline__ bool hand_over(const GemmArgs& a, uint32_t worker, uint32_t blocks_per_worker, uint32_t rank, uint32_t tile, uint32_t acc,
+                                          uint32_t r, bool ok, volatile uint32_t* last_slot, Release release)
 {
-    constexpr int STAGES = n_stages(NT), STAGE = stage_bytes(NT);
-    constexpr uint32_t TMEM_COLS = 2 * NT < 32 ? 32 : 2 * NT;
+    const uint32_t t0 = tile * a.kb;
+    float4* slot = reinterpret_cast<float4*>(a.partial) + size_t(2 * (worker * blocks_per_worker + rank) + (worker * a.run >= t0 ? 0 : 1)) * (NT / 4) * 128;
+#pragma unroll 1
+    for (int c = 0; c < NT / CH; c++) {
+        float v[CH];
+        load_acc(acc + c * CH, v);
+        if (c + 1 == NT / CH) release();
+#pragma unroll
+        for (int i = 0; i < CH / 4; i++) __stcg(slot + (c * (CH / 4) + i) * 128 + r, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
+    }
+    epilogue_sync();
+    if (r == 0) {
+        const uint32_t n = (t0 + a.kb - 1) / a.run - t0 / a.run + 1;      // workers whose runs meet the tile
+        uint32_t* counter = a.counters + tile * blocks_per_worker + rank;
+        __threadfence();
+        const uint32_t is_last = ok && atomicAdd(counter, 1u) == n - 1 ? 1u : 0u;
+        if (is_last) *counter = 0;                                       // as the next launch expects it
+        __threadfence();
+        *last_slot = is_last;
+    }
+    epilogue_sync();
+    const bool last = *last_slot != 0;
+    epilogue_sync();                                                     // read by everyone before the next cut tile writes it
+    return last;
+}
+template <int NT, int CH>
+__device__ __forceinline__ void sum_partials(const GemmArgs& a, uint32_t blocks_per_worker, uint32_t rank, uint32_t tile, uint32_t r, int c, float (&v)[CH])
+{
+    const uint32_t t0 = tile * a.kb, w0 = t0 / a.run, w1 = (t0 + a.kb - 1) / a.run;
+    constexpr int Q = CH / 4, BATCH = 32 / Q;                             // 32 loads of 16 bytes in flight per thread
+    const float4* base = reinterpret_cast<const float4*>(a.partial) + c * Q * 128 + r;
+#pragma unroll
+    for (int i = 0; i < CH; i++) v[i] = 0.0f;
+    for (uint32_t w = w0; w <= w1; w += BATCH) {
+        float4 p[BATCH][Q];
+#pragma unroll
+        for (int b = 0; b < BATCH; b++) {
+            const uint32_t ww = min(w + b, w1);
+            const float4* sl = base + size_t(2 * (ww * blocks_per_worker + rank) + (ww * a.run >= t0 ? 0 : 1)) * (NT / 4) * 128;
+#pragma unroll
+            for (int i = 0; i < Q; i++) p[b][i] = w + b <= w1 ? __ldcg(sl + i * 128) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int b = 0; b < BATCH; b++)
+#pragma unroll
+            for (int i = 0; i < Q; i++) { v[4 * i] += p[b][i].x; v[4 * i + 1] += p[b][i].y; v[4 * i + 2] += p[b][i].z; v[4 * i + 3] += p[b][i].w; }
+    }
+}
+
+template <typename T, int NT>
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
+                 T* __restrict__ out0, T* __restrict__ out1, const GemmArgs a, uint32_t* __restrict__ status)
+{
+    constexpr int STAGES = rows_stages(NT), STAGE = rows_stage(NT), OFF_MISC = STAGES * STAGE;
+    constexpr uint32_t TMEM_COLS = 2 * NT;
     extern __shared__ unsigned char gemm_smem[];
     const uint32_t raw = smem_u32(gemm_smem);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char* sm = gemm_smem + (base - raw);
-    const uint32_t bar0 = base + off_misc(NT);                   // full[STAGES], empty[STAGES], acc_full[2], acc_empty[2]
+    const uint32_t bar0 = base + OFF_MISC;                       // full[STAGES], empty[STAGES], acc_full[2], acc_empty[2]
     auto full = [&](int s) { return bar0 + 8u * uint32_t(s); };
     auto empty = [&](int s) { return bar0 + 8u * uint32_t(STAGES + s); };
-    auto acc_full = [&](int b) { return bar0 + 8u * uint32_t(2 * STAGES + b); };
-    auto acc_empty = [&](int b) { return bar0 + 8u * uint32_t(2 * STAGES + 2 + b); };
+    auto acc_full = [&](uint32_t b) { return bar0 + 8u * (2 * STAGES + b); };
+    auto acc_empty = [&](uint32_t b) { return bar0 + 8u * (2 * STAGES + 2 + b); };
     static_assert((2 * STAGES + 4) * 8 <= 224, "barriers overflow their area");
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + off_misc(NT) + 224);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + off_misc(NT) + 228);
-    volatile uint32_t* last_slot = reinterpret_cast<volatile uint32_t*>(sm + off_misc(NT) + 232);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + OFF_MISC + 224);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + 228);
+    volatile uint32_t* last_slot = reinterpret_cast<volatile uint32_t*>(sm + OFF_MISC + 232);
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-
-    // this block's run of units
-    const uint32_t tiles = a.m_tiles * (a.n_tiles[0] + a.n_tiles[1]), blocks = gridDim.x;
-    auto run_begin = [&](uint32_t b) -> uint32_t {
-        return a.whole_tiles ? uint32_t(uint64_t(tiles) * b / blocks) * a.kb : uint32_t(uint64_t(tiles) * a.kb * b / blocks);
-    };
-    const uint32_t u0 = run_begin(blockIdx.x), u1 = run_begin(blockIdx.x + 1);
-    struct Tile { uint32_t w, m, n; };                            // which weight, tile along A's rows, tile along its outputs
-    auto tile_of = [&](uint32_t t) -> Tile {
-        Tile r;
-        const uint32_t nt = t / a.m_tiles;
-        r.m = t % a.m_tiles;
-        r.w = nt >= a.n_tiles[0] ? 1u : 0u;
-        r.n = nt - (r.w ? a.n_tiles[0] : 0u);
-        return r;
-    };
+    const uint32_t u0 = blockIdx.x * a.run, u1 = min(a.units, u0 + a.run);       // this block's run of units
 
     grid_launch_dependents();
     if (tid == 0) {
         *abort_flag = 0;
         for (int s = 0; s < STAGES; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
-        for (int b = 0; b < 2; b++) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 128); }
+        for (uint32_t b = 0; b < 2; b++) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 128); }
         mbar_init_fence();
     }
     if (warp == 1) tc_alloc<TMEM_COLS>(tmem_slot);
@@ -132,40 +199,13 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 
     if (warp == 0) {
         if (lane == 0) {
-            // operand addresses of a stage: [M side 128 rows][N side NT rows]; the weight is the M side when kSwap
             auto load_w = [&](uint32_t u, int s) {
-                const Tile t = tile_of(u / a.kb);
-                const int k = int(u % a.kb) * BK;
-                const CUtensorMap* mw = t.w ? &map_w1 : &map_w0;
-                const uint32_t dst = base + s * STAGE + (kSwap ? 0 : A_BYTES);
-                const int row = int(a.w_row0[t.w] + t.n * (kSwap ? BM : NT));
-                tma_load_2d(dst, mw, full(s), k, row);
-                if (!kSwap) tma_load_2d(dst + A_BYTES, mw, full(s), k, row + BM);       // boxes of 128 weight rows
+                const Tile t = tile_of(a, u / a.kb);
+                tma_load_2d(base + s * STAGE, t.w ? &map_w1 : &map_w0, full(s), int(u % a.kb) * BK, int(a.w_row0[t.w] + t.n * BM));
             };
-            uint32_t cur_m = ~0u, next_m = ~0u, page[2] = {0, 0}, next_page[2] = {0, 0};
-            auto page_of = [&](uint32_t i) { return __ldg(a.table + min(i, (a.M + kPage - 1) / kPage - 1)); };   // past the end: the last page again
             auto load_a = [&](uint32_t u, int s) {
-                const Tile t = tile_of(u / a.kb);
-                const int k = int(u % a.kb) * BK;
-                const uint32_t dst = base + s * STAGE + (kSwap ? A_BYTES : 0);
-                if constexpr (kPaged) {
-                    if (t.m != cur_m) {                            // the page ids of the next tile are requested a tile ahead
-                        if (t.m == next_m) { page[0] = next_page[0]; page[1] = next_page[1]; }
-                        else { page[0] = page_of(2 * t.m); page[1] = page_of(2 * t.m + 1); }
-                        cur_m = t.m;
-                        next_m = t.m + 1 < a.m_tiles ? t.m + 1 : 0;
-                        next_page[0] = page_of(2 * next_m);
-                        next_page[1] = page_of(2 * next_m + 1);
-                    }
-#pragma unroll
-                    for (uint32_t h = 0; h < 2; h++) {             // two pages of 64 rows
-                        uint32_t pg = page[h];
-                        if (pg >= a.n_pages) { atomicOr(status, ST_BAD_PAGE); pg = 0; }
-                        tma_load_3d(dst + h * (A_BYTES / 2), &map_a, full(s), k, int(pg * kPage), int(a.layer));
-                    }
-                } else {
-                    tma_load_2d(dst, &map_a, full(s), k, int(t.m * (kSwap ? NT : BM)));
-                }
+                const Tile t = tile_of(a, u / a.kb);
+                tma_load_2d(base + s * STAGE + A_BYTES, &map_a, full(s), int(u % a.kb) * BK, int(t.m * NT));
             };
             const uint32_t n = u1 - u0, ahead = min(n, uint32_t(STAGES));
             for (uint32_t i = 0; i < ahead; i++) {
@@ -185,13 +225,13 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             }
         }
     } else if (warp == 1) {
-        grid_dependency_wait();
         constexpr uint32_t IDESC = instr_desc(Fmt<T>::v, BM, NT);
+        grid_dependency_wait();
         bool ok = true;
         uint32_t nt = 0;
         for (uint32_t u = u0, i = 0; u < u1 && ok; nt++) {
             const uint32_t end = min(u1, (u / a.kb + 1) * a.kb);
-            ok = mbar_wait(acc_empty(int(nt & 1)), ((nt >> 1) & 1) ^ 1, abort_flag, status);
+            ok = mbar_wait(acc_empty(nt & 1), ((nt >> 1) & 1) ^ 1, abort_flag, status);
             if (!ok) break;
             const uint32_t d = tmem + (nt & 1) * NT;
             for (bool first = true; u < end && ok; u++, i++, first = false) {
@@ -205,168 +245,291 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                     for (int k = 0; k < BK / 16; k++)
                         tc_mma(d, da + ((k * 32) >> 4), desc_hi(1024), db + ((k * 32) >> 4), desc_hi(1024), IDESC, (first && k == 0) ? 0u : 1u);
                     tc_commit(empty(s));
-                    if (u + 1 == end) tc_commit(acc_full(int(nt & 1)));
+                    if (u + 1 == end) tc_commit(acc_full(nt & 1));
                 }
                 __syncwarp();
             }
         }
     } else {
-        // epilogue: warp w reads TMEM lanes 32*(w%4) .. +31; thread = one row of the tile's M side
+        // epilogue: warp w reads TMEM lanes 32*(w%4) .. +31; thread = one weight row (output), columns = rows of A
         grid_dependency_wait();
         const uint32_t q4 = warp % 4, r = q4 * 32 + lane;
-        auto group_sync = [&]() { asm volatile("barrier.cta.sync 1, 128;\n" ::: "memory"); };
+        constexpr int CH = NT < 32 ? NT : 32;                     // columns per step
         bool ok = true;
-        uint32_t nt = 0, boxes = 0;
+        uint32_t nt = 0;
         for (uint32_t u = u0; u < u1; nt++) {
             const uint32_t tile = u / a.kb, t_end = (tile + 1) * a.kb, end = min(u1, t_end);
-            const bool split = u != tile * a.kb || end != t_end;
-            ok = ok && mbar_wait(acc_full(int(nt & 1)), (nt >> 1) & 1, abort_flag, status);
+            const bool cut = u != tile * a.kb || end != t_end;
+            const Tile tl = tile_of(a, tile);
+            const uint32_t N = a.N[tl.w], o = tl.n * BM + r;
+            T* out = tl.w ? out1 : out0;
+            ok = ok && mbar_wait(acc_full(nt & 1), (nt >> 1) & 1, abort_flag, status);
             ok = __all_sync(0xffffffffu, ok);
             tc_fence_after();
             const uint32_t acc = tmem + ((q4 * 32u) << 16) + (nt & 1) * NT;
-            constexpr int CH = NT < 32 ? NT : 32;                 // columns per step
-            auto load_acc = [&](int c, float (&v)[CH]) {
-                uint32_t x[CH];
-                if constexpr (CH == 16) tc_ld16(acc + c * CH, x);
-                else tc_ld32(acc + c * CH, x);
-                tc_wait_ld();
-#pragma unroll
-                for (int i = 0; i < CH; i++) v[i] = __uint_as_float(x[i]);
-            };
-            const Tile tl = tile_of(tile);
-            const uint32_t N = a.N[tl.w];
-            T* out = tl.w ? out1 : out0;
+            auto release = [&]() { tc_fence_before(); mbar_arrive(acc_empty(nt & 1)); };
             // columns c*CH.. of the tile, complete: round and store
             auto finish = [&](int c, const float (&v)[CH]) {
-                if constexpr (kSwap) {
-                    const uint32_t o = tl.n * BM + r;
-                    if (o >= N) return;
-                    const uint32_t m0 = tl.m * NT + c * CH, live = min(uint32_t(CH), a.M > m0 ? a.M - m0 : 0u);
-                    T* p = out + size_t(m0) * N + o;
-                    T res[CH];                                     // all of them on their way before the first store
-                    if (a.residual) {
+                if (o >= N || !ok) return;
+                const uint32_t m0 = tl.m * NT + c * CH, live = min(uint32_t(CH), a.M > m0 ? a.M - m0 : 0u);
+                T* p = out + size_t(m0) * N + o;
+                T res[CH];                                         // all of them on their way before the first store
+                if (a.residual) {
 #pragma unroll
-                        for (int i = 0; i < CH; i++) if (uint32_t(i) < live) res[i] = p[size_t(i) * N];
-                    }
+                    for (int i = 0; i < CH; i++) if (uint32_t(i) < live) res[i] = p[size_t(i) * N];
+                }
 #pragma unroll
-                    for (int i = 0; i < CH; i++) {
-                        if (uint32_t(i) >= live) continue;
-                        T x = Elem<T>::from_f32(v[i]);
-                        if (a.residual) x = Elem<T>::from_f32(Elem<T>::to_f32(res[i]) + Elem<T>::to_f32(x));
-                        p[size_t(i) * N] = x;
-                    }
-                } else {
-                    const uint32_t m = tl.m * BM + r, n0 = tl.n * NT + c * CH;
-                    T* p = out + size_t(m) * N + n0;
-                    uint32_t pk[16];
-#pragma unroll
-                    for (int i = 0; i < 16; i++) pk[i] = Elem<T>::pack2(v[2 * i], v[2 * i + 1]);
-                    if (a.residual && m < a.M) {
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            if (n0 + 8 * i >= N) break;
-                            const uint4 o4 = load8(p + 8 * i, a.vec_io);
-                            const uint32_t ow[4] = {o4.x, o4.y, o4.z, o4.w};
-#pragma unroll
-                            for (int j = 0; j < 4; j++) {
-                                const auto* xo = reinterpret_cast<const T*>(&ow[j]);
-                                const T* xn = reinterpret_cast<const T*>(&pk[4 * i + j]);
-                                pk[4 * i + j] = Elem<T>::pack2(Elem<T>::to_f32(xo[0]) + Elem<T>::to_f32(xn[0]), Elem<T>::to_f32(xo[1]) + Elem<T>::to_f32(xn[1]));
-                            }
-                        }
-                    }
-                    if (a.tile_store) {
-                        // 64 outputs x 128 rows go to shared memory in the 128-byte swizzle and TMA writes whole rows of the box; a
-                        // thread storing its own 64 bytes per row piece reaches a third of that rate on 400 MB of output.
-                        unsigned char* box = sm + off_store(NT) + (boxes & 1) * STORE_BYTES + r * 128;
-                        if (c % 2 == 0) {                          // the box that used this buffer before must have been read
-                            if (warp == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");
-                            group_sync();
-                        }
-#pragma unroll
-                        for (int i = 0; i < 4; i++)
-                            *reinterpret_cast<uint4*>(box + ((((c % 2) * 4 + i) ^ (r & 7)) << 4)) = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
-                        if (c % 2 == 1) {
-                            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                            group_sync();
-                            if (warp == 2 && lane == 0) {
-                                if (*abort_flag == 0 && tl.n * NT + (c - 1) * CH < N)
-                                    tma_store_2d(tl.w ? &map_c1 : &map_c0, base + off_store(NT) + (boxes & 1) * STORE_BYTES, int(tl.n * NT + (c - 1) * CH), int(tl.m * BM));
-                                asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
-                            }
-                            boxes++;
-                        }
-                        return;
-                    }
-                    if (m >= a.M) return;
-#pragma unroll
-                    for (int i = 0; i < 4; i++)
-                        if (n0 + 8 * i < N) store8(p + 8 * i, make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]), a.vec_io);
+                for (int i = 0; i < CH; i++) {
+                    if (uint32_t(i) >= live) continue;
+                    T x = Elem<T>::from_f32(v[i]);
+                    if (a.residual) x = Elem<T>::from_f32(Elem<T>::to_f32(res[i]) + Elem<T>::to_f32(x));
+                    p[size_t(i) * N] = x;
                 }
             };
-            if (!split) {
+            if (!cut) {
 #pragma unroll 1
                 for (int c = 0; c < NT / CH; c++) {
                     float v[CH];
-                    load_acc(c, v);
-                    if (c + 1 == NT / CH) { tc_fence_before(); mbar_arrive(acc_empty(int(nt & 1))); }
+                    load_acc(acc + c * CH, v);
+                    if (c + 1 == NT / CH) release();
                     finish(c, v);
                 }
-            } else {
-                // slot 0 of a block: the tile its run begins in, slot 1: the tile its run ends in
-                float4* slot = reinterpret_cast<float4*>(a.partial) + size_t(2 * blockIdx.x + (nt == 0 ? 0 : 1)) * (NT / 4) * 128;
+            } else if (hand_over<NT, CH>(a, blockIdx.x, 1, 0, tile, acc, r, ok, last_slot, release)) {
 #pragma unroll 1
                 for (int c = 0; c < NT / CH; c++) {
                     float v[CH];
-                    load_acc(c, v);
-                    if (c + 1 == NT / CH) { tc_fence_before(); mbar_arrive(acc_empty(int(nt & 1))); }
-#pragma unroll
-                    for (int i = 0; i < CH / 4; i++) __stcg(slot + (c * (CH / 4) + i) * 128 + r, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
+                    sum_partials<NT, CH>(a, 1, 0, tile, r, c, v);
+                    finish(c, v);
                 }
-                // contributors: the blocks whose runs meet [tile * kb, (tile + 1) * kb)
-                uint32_t b0 = blockIdx.x, b1 = blockIdx.x;
-                while (b0 > 0 && run_begin(b0) > tile * a.kb) b0--;
-                while (b1 + 1 < blocks && run_begin(b1 + 1) < t_end) b1++;
-                __threadfence();
-                group_sync();
-                if (warp == 2 && lane == 0) {
-                    const uint32_t before = ok ? atomicAdd(a.counters + tile, 1u) : 0u;
-                    const uint32_t is_last = ok && before == b1 - b0 ? 1u : 0u;
-                    if (is_last) a.counters[tile] = 0;             // as the next launch expects it
-                    *last_slot = is_last;
-                }
-                group_sync();
-                if (*last_slot) {
-                    __threadfence();
-#pragma unroll 1
-                    for (int c = 0; c < NT / CH; c++) {
-                        float v[CH];
-#pragma unroll
-                        for (int i = 0; i < CH; i++) v[i] = 0.0f;
-                        for (uint32_t b = b0; b <= b1; b++) {
-                            const float4* sl = reinterpret_cast<const float4*>(a.partial) +
-                                               size_t(2 * b + (run_begin(b) / a.kb == tile ? 0 : 1)) * (NT / 4) * 128;
-#pragma unroll
-                            for (int i = 0; i < CH / 4; i++) {
-                                const float4 p = __ldcg(sl + (c * (CH / 4) + i) * 128 + r);
-                                v[4 * i] += p.x; v[4 * i + 1] += p.y; v[4 * i + 2] += p.z; v[4 * i + 3] += p.w;
-                            }
-                        }
-                        finish(c, v);
-                    }
-                }
-                group_sync();                                      // last_slot is read by everyone before the next tile's writer
             }
             u = end;
         }
-        if constexpr (!kSwap)
-            if (a.tile_store && warp == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
         tc_dealloc<TMEM_COLS>(tmem);
+    }
+}
+
+template <typename T, int NT, bool kPaged>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
+                 const __grid_constant__ CUtensorMap map_c0, const __grid_constant__ CUtensorMap map_c1, T* __restrict__ out0, T* __restrict__ out1,
+                 const GemmArgs a, uint32_t* __restrict__ status)
+{
+    constexpr int STAGES = pair_stages(NT), STAGE = pair_stage(NT), OFF_STORE = pair_off_store(NT), OFF_MISC = OFF_STORE + 2 * STORE_BYTES;
+    constexpr uint32_t TMEM_COLS = 2 * NT;
+    extern __shared__ unsigned char gemm_smem[];
+    const uint32_t raw = smem_u32(gemm_smem);                     // both blocks of a pair see the same offset
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    unsigned char* sm = gemm_smem + (base - raw);
+    const uint32_t bar0 = base + OFF_MISC;                        // full[STAGES], empty[STAGES], acc_full[2], acc_empty[2]
+    auto full = [&](int s) { return bar0 + 8u * uint32_t(s); };
+    auto empty = [&](int s) { return bar0 + 8u * uint32_t(STAGES + s); };
+    auto acc_full = [&](uint32_t b) { return bar0 + 8u * (2 * STAGES + b); };
+    auto acc_empty = [&](uint32_t b) { return bar0 + 8u * (2 * STAGES + 2 + b); };
+    static_assert((2 * STAGES + 4) * 8 <= 224, "barriers overflow their area");
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + OFF_MISC + 224);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + 228);
+    volatile uint32_t* last_slot = reinterpret_cast<volatile uint32_t*>(sm + OFF_MISC + 232);
+    const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    const uint32_t rank = cluster_rank(), worker = blockIdx.x / 2;               // rank 0 issues the MMAs
+    const uint32_t u0 = worker * a.run, u1 = min(a.units, u0 + a.run);           // this pair's run of units
+
+    grid_launch_dependents();
+    if (tid == 0) {
+        *abort_flag = 0;
+        for (int s = 0; s < STAGES; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
+        for (uint32_t b = 0; b < 2; b++) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 8); }      // four epilogue warps of each block
+        mbar_init_fence();
+    }
+    if (warp == 1) tc_alloc_pair<TMEM_COLS>(tmem_slot);
+    tc_fence_before();
+    // both blocks' barriers must exist before either sends a remote arrive or a TMA completion
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            const uint32_t leader_full = map_to_rank(full(0), 0);
+            auto load_w = [&](uint32_t u, int s) {               // this block's half of the outputs, in boxes of up to 128 weight rows
+                const Tile t = tile_of(a, u / a.kb);
+                tma_load_2d_pair(base + s * STAGE + A_BYTES, t.w ? &map_w1 : &map_w0, leader_full + 8u * s, int(u % a.kb) * BK,
+                                 int(a.w_row0[t.w] + t.n * NT + rank * (NT / 2)));
+            };
+            uint32_t cur_m = ~0u, next_m = ~0u, page[2] = {0, 0}, next_page[2] = {0, 0};
+            auto page_of = [&](uint32_t i) { return __ldg(a.table + min(i, (a.M + kPage - 1) / kPage - 1)); };   // past the end: the last page again
+            auto load_a = [&](uint32_t u, int s) {
+                const Tile t = tile_of(a, u / a.kb);
+                const int k = int(u % a.kb) * BK;
+                const uint32_t dst = base + s * STAGE;
+                if constexpr (kPaged) {
+                    if (t.m != cur_m) {                            // the page ids of the next tile are requested a tile ahead
+                        if (t.m == next_m) { page[0] = next_page[0]; page[1] = next_page[1]; }
+                        else { page[0] = page_of(4 * t.m + 2 * rank); page[1] = page_of(4 * t.m + 2 * rank + 1); }
+                        cur_m = t.m;
+                        next_m = t.m + 1 < a.m_tiles ? t.m + 1 : 0;
+                        next_page[0] = page_of(4 * next_m + 2 * rank);
+                        next_page[1] = page_of(4 * next_m + 2 * rank + 1);
+                    }
+#pragma unroll
+                    for (uint32_t h = 0; h < 2; h++) {             // two pages of 64 rows
+                        uint32_t pg = page[h];
+                        if (pg >= a.n_pages) { atomicOr(status, ST_BAD_PAGE); pg = 0; }
+                        tma_load_3d_pair(dst + h * (A_BYTES / 2), &map_a, leader_full + 8u * s, k, int(pg * kPage), int(a.layer));
+                    }
+                } else {
+                    tma_load_2d_pair(dst, &map_a, leader_full + 8u * s, k, int(t.m * 2 * BM + rank * BM));
+                }
+            };
+            const uint32_t n = u1 - u0, ahead = min(n, uint32_t(STAGES));
+            for (uint32_t i = 0; i < ahead; i++) {
+                if (rank == 0) mbar_expect_tx(full(int(i)), 2 * STAGE);
+                load_w(u0 + i, int(i));
+            }
+            grid_dependency_wait();      // the activations come from an earlier kernel of the stream
+            for (uint32_t i = 0; i < ahead; i++) load_a(u0 + i, int(i));
+            bool ok = true;
+            for (uint32_t i = ahead; i < n && ok; i++) {
+                const int s = int(i % STAGES);
+                ok = mbar_wait(empty(s), ((i / STAGES) & 1) ^ 1, abort_flag, status);
+                if (!ok) break;
+                if (rank == 0) mbar_expect_tx(full(s), 2 * STAGE);
+                load_w(u0 + i, s);
+                load_a(u0 + i, s);
+            }
+        }
+    } else if (warp == 1) {
+        grid_dependency_wait();
+        if (rank == 0) {
+            constexpr uint32_t IDESC = instr_desc(Fmt<T>::v, 2 * BM, NT);
+            bool ok = true;
+            uint32_t nt = 0;
+            for (uint32_t u = u0, i = 0; u < u1 && ok; nt++) {
+                const uint32_t end = min(u1, (u / a.kb + 1) * a.kb);
+                ok = mbar_wait<kSleepCluster>(acc_empty(nt & 1), ((nt >> 1) & 1) ^ 1, abort_flag, status);
+                if (!ok) break;
+                const uint32_t d = tmem + (nt & 1) * NT;
+                for (bool first = true; u < end && ok; u++, i++, first = false) {
+                    const int s = int(i % STAGES);
+                    ok = mbar_wait<kSleepCluster>(full(s), (i / STAGES) & 1, abort_flag, status);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint32_t da = desc_lo(base + s * STAGE), db = desc_lo(base + s * STAGE + A_BYTES);
+#pragma unroll
+                        for (int k = 0; k < BK / 16; k++)
+                            tc_mma_pair(d, da + ((k * 32) >> 4), desc_hi(1024), db + ((k * 32) >> 4), desc_hi(1024), IDESC, (first && k == 0) ? 0u : 1u);
+                        tc_commit_pair(empty(s));
+                        if (u + 1 == end) tc_commit_pair(acc_full(nt & 1));
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+    } else {
+        // epilogue: warp w reads TMEM lanes 32*(w%4) .. +31; thread = one row of this block's 128, columns = outputs
+        grid_dependency_wait();
+        const uint32_t q4 = warp % 4, r = q4 * 32 + lane;
+        const uint32_t leader_empty = map_to_rank(acc_empty(0), 0);
+        constexpr int CH = 32;
+        bool ok = true;
+        uint32_t nt = 0, boxes = 0;
+        for (uint32_t u = u0; u < u1; nt++) {
+            const uint32_t tile = u / a.kb, t_end = (tile + 1) * a.kb, end = min(u1, t_end);
+            const bool cut = u != tile * a.kb || end != t_end;
+            const Tile tl = tile_of(a, tile);
+            const uint32_t N = a.N[tl.w], m0 = (2 * tl.m + rank) * BM, m = m0 + r;
+            T* out = tl.w ? out1 : out0;
+            ok = ok && mbar_wait(acc_full(nt & 1), (nt >> 1) & 1, abort_flag, status);
+            ok = __all_sync(0xffffffffu, ok);
+            tc_fence_after();
+            const uint32_t acc = tmem + ((q4 * 32u) << 16) + (nt & 1) * NT;
+            auto release = [&]() {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(leader_empty + 8u * (nt & 1));
+            };
+            // columns c*CH.. of the tile, complete: round and store.  All 128 threads pass its barriers.
+            auto finish = [&](int c, const float (&v)[CH]) {
+                const uint32_t n0 = tl.n * NT + c * CH;
+                T* p = out + size_t(m) * N + n0;
+                uint32_t pk[16];
+#pragma unroll
+                for (int i = 0; i < 16; i++) pk[i] = Elem<T>::pack2(v[2 * i], v[2 * i + 1]);
+                if (a.residual && m < a.M) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        if (n0 + 8 * i >= N) break;
+                        const uint4 o4 = load8(p + 8 * i, a.vec_io);
+                        const uint32_t ow[4] = {o4.x, o4.y, o4.z, o4.w};
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            const auto* xo = reinterpret_cast<const T*>(&ow[j]);
+                            const T* xn = reinterpret_cast<const T*>(&pk[4 * i + j]);
+                            pk[4 * i + j] = Elem<T>::pack2(Elem<T>::to_f32(xo[0]) + Elem<T>::to_f32(xn[0]), Elem<T>::to_f32(xo[1]) + Elem<T>::to_f32(xn[1]));
+                        }
+                    }
+                }
+                if (!a.tile_store) {
+                    if (m >= a.M || !ok) return;
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        if (n0 + 8 * i < N) store8(p + 8 * i, make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]), a.vec_io);
+                    return;
+                }
+                // 64 outputs x 128 rows go to shared memory in the 128-byte swizzle and TMA writes whole rows of the box; a thread
+                // storing its own 64 bytes per row piece reaches a third of that rate on 400 MB of output.
+                unsigned char* box = sm + OFF_STORE + (boxes & 1) * STORE_BYTES + r * 128;
+                if (c % 2 == 0) {                                  // the box that used this buffer before must have been read
+                    if (warp == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");
+                    epilogue_sync();
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    *reinterpret_cast<uint4*>(box + ((((c % 2) * 4 + i) ^ (r & 7)) << 4)) = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
+                if (c % 2 == 1) {
+                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                    epilogue_sync();
+                    if (warp == 2 && lane == 0) {
+                        if (*abort_flag == 0 && n0 - CH < N && m0 < a.M)
+                            tma_store_2d(tl.w ? &map_c1 : &map_c0, base + OFF_STORE + (boxes & 1) * STORE_BYTES, int(n0 - CH), int(m0));
+                        asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+                    }
+                    boxes++;
+                }
+            };
+            if (!cut) {
+#pragma unroll 1
+                for (int c = 0; c < NT / CH; c++) {
+                    float v[CH];
+                    load_acc(acc + c * CH, v);
+                    if (c + 1 == NT / CH) release();
+                    finish(c, v);
+                }
+            } else if (hand_over<NT, CH>(a, worker, 2, rank, tile, acc, r, ok, last_slot, release)) {
+#pragma unroll 1
+                for (int c = 0; c < NT / CH; c++) {
+                    float v[CH];
+                    sum_partials<NT, CH>(a, 2, rank, tile, r, c, v);
+                    finish(c, v);
+                }
+            }
+            u = end;
+        }
+        if (a.tile_store && warp == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+    }
+    // neither block may leave while its twin can still signal its barriers or feed a pair MMA from its shared memory
+    tc_fence_before();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    if (warp == 1) {
+        tc_fence_after();
+        tc_dealloc_pair<TMEM_COLS>(tmem);
     }
 }
 
@@ -457,37 +620,76 @@ template <typename T>
 cudaError_t configure_type()
 {
     auto set = [](auto kernel, int bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
-    cudaError_t e = set(gemm_tc5_kernel<T, 16, true, false>, smem_bytes(16));
-    if (e == cudaSuccess) e = set(gemm_tc5_kernel<T, 32, true, false>, smem_bytes(32));
-    if (e == cudaSuccess) e = set(gemm_tc5_kernel<T, 64, true, false>, smem_bytes(64));
-    if (e == cudaSuccess) e = set(gemm_tc5_kernel<T, 128, true, false>, smem_bytes(128));
-    if (e == cudaSuccess) e = set(gemm_tc5_kernel<T, 256, false, false>, smem_bytes(256));
-    if (e == cudaSuccess) e = set(gemm_tc5_kernel<T, 256, false, true>, smem_bytes(256));
+    cudaError_t e = set(gemm_rows_kernel<T, 16>, rows_smem(16));
+    if (e == cudaSuccess) e = set(gemm_rows_kernel<T, 32>, rows_smem(32));
+    if (e == cudaSuccess) e = set(gemm_rows_kernel<T, 64>, rows_smem(64));
+    if (e == cudaSuccess) e = set(gemm_rows_kernel<T, 128>, rows_smem(128));
+    if (e == cudaSuccess) e = set(gemm_pair_kernel<T, 128, false>, pair_smem(128));
+    if (e == cudaSuccess) e = set(gemm_pair_kernel<T, 256, false>, pair_smem(256));
+    if (e == cudaSuccess) e = set(gemm_pair_kernel<T, 128, true>, pair_smem(128));
+    if (e == cudaSuccess) e = set(gemm_pair_kernel<T, 256, true>, pair_smem(256));
     return e;
+}
+
+// Tile width and run length of a launch: the shortest estimate, in SM cycles, of whole tiles against equal runs with cut
+// tiles.  A k-block of a pair takes 820 (256 outputs) or 610 (128) cycles at the L2 feed rate, one of gemm_rows_kernel
+// about 400 at the HBM rate; cutting tiles adds the hand-over (about 4000 cycles: partial out, counter, partials in) and
+// about 50 cycles per column.
+struct Shape { uint32_t nt, m_tiles, n_tiles[2], run; };
+Shape pick_shape(const GemmCall& g, bool rows_kernel, uint32_t kb, const GemmWorkspace& ws)
+{
+    Shape best{};
+    uint64_t best_cost = ~0ull;
+    const uint32_t workers = rows_kernel ? ws.blocks : ws.blocks / 2;
+    auto consider = [&](uint32_t nt, uint32_t m_side, uint32_t n_side, uint64_t cyc) {
+        Shape s{nt, (g.M + m_side - 1) / m_side, {0, 0}, 0};
+        for (int i = 0; i < g.n_weights; i++) s.n_tiles[i] = (g.w[i].N + n_side - 1) / n_side;
+        const uint64_t tiles = uint64_t(s.m_tiles) * (s.n_tiles[0] + s.n_tiles[1]);
+        const uint64_t per = (tiles + workers - 1) / workers, whole = per * kb * cyc;
+        const uint64_t run = (tiles * kb + workers - 1) / workers, cut = run * cyc + 4000 + 50 * nt;
+        s.run = uint32_t(per * kb);
+        if (whole < best_cost) { best_cost = whole; best = s; }
+        s.run = uint32_t(std::max<uint64_t>(run, 2));
+        if (cut < best_cost && tiles * (rows_kernel ? 1 : 2) <= ws.max_tiles) { best_cost = cut; best = s; }
+    };
+    if (rows_kernel) {
+        const uint32_t nt = g.M <= 16 ? 16 : g.M <= 32 ? 32 : g.M <= 64 ? 64 : 128;
+        consider(nt, nt, BM, 400);
+    } else {
+        consider(256, 2 * BM, 256, 820);
+        consider(128, 2 * BM, 128, 610);
+    }
+    return best;
 }
 
 template <typename T>
 int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t* status, cudaStream_t st)
 {
-    const bool swap = !g.paged_map && g.M <= 128;
-    const uint32_t nt = !swap ? 256 : g.M <= 16 ? 16 : g.M <= 32 ? 32 : g.M <= 64 ? 64 : 128;
+    const bool rows_kernel = !g.paged_map && g.M <= 128;
     GemmArgs a{};
     a.M = g.M;
     a.kb = (g.K + BK - 1) / BK;
-    a.m_tiles = (g.M + (swap ? nt : BM) - 1) / (swap ? nt : BM);
+    const Shape sh = pick_shape(g, rows_kernel, a.kb, ws);
+    const uint32_t nt = sh.nt;
+    a.m_tiles = sh.m_tiles;
+    a.n_tiles[0] = sh.n_tiles[0];
+    a.n_tiles[1] = sh.n_tiles[1];
+    a.units = a.m_tiles * (a.n_tiles[0] + a.n_tiles[1]) * a.kb;
+    a.run = sh.run;
+    const uint32_t workers = (a.units + a.run - 1) / a.run;
     a.residual = g.residual ? 1u : 0u;
-    const uint32_t n_side = swap ? BM : nt;
+    a.tile_store = rows_kernel ? 0u : 1u;
+    a.vec_io = 1u;
+    a.partial = ws.partial;
+    a.counters = ws.counters;
     alignas(64) CUtensorMap ma, mc[2];
     T* out[2] = {nullptr, nullptr};
-    a.tile_store = swap ? 0u : 1u;
-    a.vec_io = 1u;
     for (int i = 0; i < g.n_weights; i++) {
         const GemmWeight& w = g.w[i];
+        if (w.N % 8) return -1;
         a.N[i] = w.N;
         a.w_row0[i] = w.row0;
-        a.n_tiles[i] = (w.N + n_side - 1) / n_side;
         out[i] = static_cast<T*>(w.out);
-        if (w.N % 8) return -1;
         if (reinterpret_cast<uintptr_t>(w.out) & 15u) a.vec_io = a.tile_store = 0u;
         // storage-type output with rows that TMA can address: the epilogue stores tiles (see the kernel)
         if (a.tile_store && !make_map(&mc[i], dtype, w.out, g.M, w.N, w.N, BM)) a.tile_store = 0u;
@@ -496,27 +698,23 @@ int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t*
         a.table = g.table;
         a.layer = g.layer;
         a.n_pages = g.n_pages;
-    } else if (!make_map(&ma, dtype, g.A, g.M, g.K, g.K, swap ? nt : BM)) return -1;
-    if (g.n_weights == 1 || !a.tile_store) mc[1] = a.tile_store ? mc[0] : *g.w[0].map;
-    if (!a.tile_store) mc[0] = *g.w[0].map;
-    const uint32_t tiles = a.m_tiles * (a.n_tiles[0] + a.n_tiles[1]);
-    // whole tiles where the imbalance of the last one is below a sixteenth, or where a cut tile would cost more than it
-    // saves (fewer than two k-blocks per block); otherwise equal runs of k-blocks
-    a.whole_tiles = tiles >= 16 * ws.blocks || uint64_t(tiles) * a.kb < 2ull * ws.blocks ? 1u : 0u;
-    const uint32_t blocks = std::min(ws.blocks, a.whole_tiles ? tiles : tiles * a.kb);
-    if (!a.whole_tiles && tiles > ws.max_tiles) a.whole_tiles = 1u;
-    a.partial = ws.partial;
-    a.counters = ws.counters;
-    const CUtensorMap& m0 = *g.w[0].map;
-    const CUtensorMap& m1 = g.n_weights > 1 ? *g.w[1].map : m0;
+    } else if (!make_map(&ma, dtype, g.A, g.M, g.K, g.K, rows_kernel ? nt : BM)) return -1;
+    const int last = g.n_weights - 1;
+    auto map_of = [&](int i) -> const CUtensorMap& { return rows_kernel || nt == 256 ? *g.w[i].map : *g.w[i].map64; };   // boxes of 128 or 64 weight rows
+    const CUtensorMap &m0 = map_of(0), &m1 = map_of(last), &pa = g.paged_map ? *g.paged_map : ma;
+    if (rows_kernel) {
+        auto go = [&](auto kernel) {
+            return int(launch_pdl(kernel, dim3(workers), dim3(NUM_THREADS), size_t(rows_smem(int(nt))), st, pa, m0, m1, out[0], out[1], a, status));
+        };
+        return nt == 16 ? go(gemm_rows_kernel<T, 16>) : nt == 32 ? go(gemm_rows_kernel<T, 32>)
+             : nt == 64 ? go(gemm_rows_kernel<T, 64>) : go(gemm_rows_kernel<T, 128>);
+    }
+    const CUtensorMap &c0 = a.tile_store ? mc[0] : m0, &c1 = a.tile_store ? mc[last] : m0;
     auto go = [&](auto kernel) {
-        return int(launch_pdl(kernel, dim3(blocks), dim3(NUM_THREADS), size_t(smem_bytes(int(nt))), st, g.paged_map ? *g.paged_map : ma, m0, m1,
-                              mc[0], mc[1], out[0], out[1], a, status));
+        return int(launch_pdl(kernel, dim3(2 * workers), dim3(NUM_THREADS), size_t(pair_smem(int(nt))), st, pa, m0, m1, c0, c1, out[0], out[1], a, status));
     };
-    if (g.paged_map) return go(gemm_tc5_kernel<T, 256, false, true>);
-    if (!swap) return go(gemm_tc5_kernel<T, 256, false, false>);
-    return nt == 16 ? go(gemm_tc5_kernel<T, 16, true, false>) : nt == 32 ? go(gemm_tc5_kernel<T, 32, true, false>)
-         : nt == 64 ? go(gemm_tc5_kernel<T, 64, true, false>) : go(gemm_tc5_kernel<T, 128, true, false>);
+    if (g.paged_map) return nt == 256 ? go(gemm_pair_kernel<T, 256, true>) : go(gemm_pair_kernel<T, 128, true>);
+    return nt == 256 ? go(gemm_pair_kernel<T, 256, false>) : go(gemm_pair_kernel<T, 128, false>);
 }
 
 }  // namespace
@@ -528,10 +726,13 @@ int gemm_tc5_configure()
     return int(e);
 }
 
-// two slots of 128 x 256 floats per block
+// two slots of 128 x 256 floats per block (a worker of a pair launch is two blocks)
 size_t gemm_tc5_partial_bytes(uint32_t blocks) { return size_t(2) * blocks * 128 * 256 * sizeof(float); }
 
-bool gemm_tc5_weight_map(CUtensorMap* map, int dtype, const void* W, uint64_t rows, uint64_t K) { return make_map(map, dtype, W, rows, K, K, BM); }
+bool gemm_tc5_weight_maps(GemmWeightMaps* maps, int dtype, const void* W, uint64_t rows, uint64_t K)
+{
+    return make_map(&maps->box128, dtype, W, rows, K, K, 128) && make_map(&maps->box64, dtype, W, rows, K, K, 64);
+}
 
 // Returns a cudaError_t value, or -1 when the operands cannot be addressed (pointers must be 16-byte aligned, row lengths
 // multiples of 8).

@@ -75,8 +75,11 @@ int launch_merge_tc5(int dtype, const float* recs, const StepMeta& m, uint32_t n
 int merge_tc5_configure();
 
 // Dense projections C = A . W^T on tcgen05 (mla_gemm_tc5.cu), up to two weights over the same activations in one launch.
+struct alignas(64) GemmWeightMaps {
+    CUtensorMap box128, box64;     // W [rows][K] in boxes of 64 values x 128 / 64 rows
+};
 struct GemmWeight {
-    const CUtensorMap* map;    // gemm_tc5_weight_map: W [rows][K], box of 64 values x 128 rows
+    const CUtensorMap *map, *map64;
     uint32_t row0, N;          // first row of the weight inside the map, outputs (a multiple of 8)
     void* out;                 // DEVICE [M][N] in the storage type
 };
@@ -97,7 +100,7 @@ struct GemmWorkspace {
 };
 int launch_gemm_tc5(int dtype, const GemmCall& g, const GemmWorkspace& ws, uint32_t* status, cudaStream_t st);
 size_t gemm_tc5_partial_bytes(uint32_t blocks);
-bool gemm_tc5_weight_map(CUtensorMap* map, int dtype, const void* W, uint64_t rows, uint64_t K);
+bool gemm_tc5_weight_maps(GemmWeightMaps* maps, int dtype, const void* W, uint64_t rows, uint64_t K);
 int launch_rmsnorm_rows(int dtype, const void* x, const void* w, void* y, uint32_t rows, uint32_t N, float eps, cudaStream_t st);
 int gemm_tc5_configure();
 
