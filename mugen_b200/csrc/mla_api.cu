@@ -261,15 +261,28 @@ uint32_t workers_of(const mla_ctx* c, uint32_t kernel, uint32_t heads)
     return std::max<uint32_t>(1, c->sm_count * 2 / ((heads + 15) / 16));
 }
 
-// The attention kernel for `heads` head rows over one stream of the cache.  128 rows go to the SM-pair kernel; up to 16
-// take the transposed tcgen05 form (tokens as rows, the heads as 16 columns); everything between fills (part of) the
-// 64-row tiles of the single-block kernel, which streams the cache once per 64 heads (measured at 32 heads, 64 sequences x
-// 8192 tokens: 128 us against 186 us for two passes of the 16-column form and 300 us for mma.sync).
+// The attention kernel for `heads` head rows over one stream of the cache.  More than 64 rows go to the SM-pair kernel,
+// which streams the cache once for 128 of them at the same rate whether all are live or not (a second pass of the 64-row
+// kernel costs more than the padding); up to 16 take the transposed tcgen05 form (tokens as rows, the heads as 16
+// columns); everything between fills (part of) the 64-row tiles of the single-block kernel (measured at 32 heads, 64
+// sequences x 8192 tokens: 128 us against 186 us for two passes of the 16-column form and 300 us for mma.sync).
 uint32_t kernel_for(const mla_ctx* c, uint32_t heads)
 {
     if (c->cfg.kernel != MLA_KERNEL_AUTO) return c->cfg.kernel;
-    return (heads % 128 == 0 && c->sm_count % 2 == 0) ? uint32_t(MLA_KERNEL_TCGEN05_PAIR128)
+    return (heads > 64 && c->sm_count % 2 == 0) ? uint32_t(MLA_KERNEL_TCGEN05_PAIR128)
          : heads > 16 ? uint32_t(MLA_KERNEL_TCGEN05) : uint32_t(MLA_KERNEL_TCGEN05_T16);
+}
+
+// Head rows that one stream of the cache can serve: what a query group may fill.
+uint32_t group_heads(const mla_ctx* c)
+{
+    switch (c->cfg.kernel) {
+    case MLA_KERNEL_AUTO: return c->sm_count % 2 == 0 ? 128 : 64;
+    case MLA_KERNEL_TCGEN05_PAIR128: return 128;
+    case MLA_KERNEL_TCGEN05: return 64;
+    case MLA_KERNEL_TCGEN05_T16: return 16;
+    default: return 1;
+    }
 }
 
 size_t meta_capacity(const mla_ctx* c)
@@ -315,21 +328,47 @@ int build_plan(mla_ctx* c, Plan& plan, int region, const std::vector<uint32_t>& 
         tbl_total += c->pt->seq(seq_ids[i])->pages.size();
     }
     std::vector<Segment> segs;
-    std::vector<uint32_t> row_seg_begin{0}, cta_seg_begin{0};
-    plan.kernel = kernel_for(c, H);
+    std::vector<uint32_t> grp_seg_begin{0}, cta_seg_begin{0};
+    // Query groups: the new tokens of a sequence are consecutive rows whose attend lengths grow by one, and with few heads
+    // several of them fit the head rows of one stream of the cache (5 rows of 16 heads: one pass instead of five).
+    struct Group { uint32_t row, n; };
+    std::vector<Group> groups;
+    uint32_t k = 1;                  // rows of the largest group
+    auto follows = [&](uint32_t r) {
+        return rows[r].seq_index == rows[r - 1].seq_index && rows[r].attend_len == rows[r - 1].attend_len + 1 && rows[r - 1].attend_len > 0;
+    };
     if (R) {
-        std::vector<uint32_t> lens(size_t(R) * layers);
-        for (uint32_t r = 0; r < R; r++) lens[r] = rows[r].attend_len;
-        for (uint32_t l = 1; l < layers; l++) std::copy(lens.begin(), lens.begin() + R, lens.begin() + size_t(l) * R);
-        const uint32_t workers = workers_of(c, plan.kernel, H);
-        if (plan.kernel == MLA_KERNEL_TCGEN05_PAIR128)
-            // a worker pays about five tiles' time per segment it starts (queries, pipeline fill, state drain: ~10 us)
-            mugen::mla::plan_min_makespan(lens, mla::kPage, workers, segs, row_seg_begin, cta_seg_begin, 2u, 5u);
-        else
-            mugen::mla::plan_balanced(lens, mla::kPage, workers, segs, row_seg_begin, cta_seg_begin, 1u);
-        if (segs.size() * H > c->rec_cap)
+        uint32_t longest = 1;
+        for (uint32_t r = 1, run = 1; r < R; r++) {
+            run = follows(r) ? run + 1 : 1;
+            longest = std::max(longest, run);
+        }
+        for (uint32_t cap = std::max(1u, std::min(group_heads(c) / H, longest));; cap = cap / 2) {
+            const uint32_t n_groups = (longest + cap - 1) / cap;
+            k = (longest + n_groups - 1) / n_groups;
+            groups.clear();
+            for (uint32_t r = 0; r < R; r++) {
+                if (r && follows(r) && groups.back().n < k) groups.back().n++;
+                else groups.push_back({r, 1});
+            }
+            const uint32_t NG = uint32_t(groups.size());
+            plan.kernel = kernel_for(c, k * H);
+            const uint32_t workers = workers_of(c, plan.kernel, k * H);
+            if ((size_t(workers) + size_t(NG) * layers) * k * H > c->rec_cap && k > 1) continue;     // many single rows beside a long run
+            std::vector<uint32_t> lens(size_t(NG) * layers);
+            for (uint32_t g = 0; g < NG; g++) lens[g] = rows[groups[g].row + groups[g].n - 1].attend_len;
+            for (uint32_t l = 1; l < layers; l++) std::copy(lens.begin(), lens.begin() + NG, lens.begin() + size_t(l) * NG);
+            if (plan.kernel == MLA_KERNEL_TCGEN05_PAIR128)
+                // a worker pays about five tiles' time per segment it starts (queries, pipeline fill, state drain: ~10 us)
+                mugen::mla::plan_min_makespan(lens, mla::kPage, workers, segs, grp_seg_begin, cta_seg_begin, 2u, 5u);
+            else
+                mugen::mla::plan_balanced(lens, mla::kPage, workers, segs, grp_seg_begin, cta_seg_begin, 1u);
+            break;
+        }
+        if (segs.size() * k * H > c->rec_cap)
             return fail(c, MLA_ERR_CAPACITY, "step needs " + std::to_string(segs.size()) + " KV segments, more than the workspace holds");
     }
+    const uint32_t NG = uint32_t(groups.size());
     const uint32_t G = uint32_t(segs.size()), W = uint32_t(cta_seg_begin.size()) - 1;
     if (R) {
         plan.min_pages = W ? ~0u : 0u;
@@ -376,13 +415,20 @@ int build_plan(mla_ctx* c, Plan& plan, int region, const std::vector<uint32_t>& 
     if (att_row) std::memcpy(h + o_att, att_row->data(), size_t(R) * 4);
     auto* p_seg = reinterpret_cast<mla::SegDesc*>(h + o_seg);
     for (uint32_t g = 0; g < G; g++) {
-        const RowSpec& rs = rows[segs[g].row % R];
-        const uint32_t tok0 = segs[g].page_begin * mla::kPage, tok1 = std::min(rs.attend_len, segs[g].page_end * uint32_t(mla::kPage));
+        const uint32_t l = segs[g].row / NG;
+        const Group& gr = groups[segs[g].row % NG];
+        const RowSpec &first = rows[gr.row], &last = rows[gr.row + gr.n - 1];
+        const uint32_t tok0 = segs[g].page_begin * mla::kPage, tok1 = std::min(last.attend_len, segs[g].page_end * uint32_t(mla::kPage));
         const uint32_t n_tok = tok1 > tok0 ? tok1 - tok0 : 0;
-        p_seg[g] = mla::SegDesc{segs[g].row, tbl_off[rs.seq_index] + segs[g].page_begin, n_tok, segs[g].row / R, int32_t(n_tok), H, {0, 0}};
+        p_seg[g] = mla::SegDesc{l * R + gr.row, tbl_off[first.seq_index] + segs[g].page_begin, n_tok, l,
+                                int32_t(first.attend_len) - int32_t(tok0), gr.n * H, {0, 0}};
     }
     auto* p_parts = reinterpret_cast<mla::RowParts*>(h + o_parts);
-    for (uint32_t v = 0; v < R * layers; v++) p_parts[v] = mla::RowParts{row_seg_begin[v], row_seg_begin[v + 1], 0, 0};
+    for (uint32_t l = 0; l < layers; l++)
+        for (uint32_t g = 0; g < NG; g++) {
+            const uint32_t v = l * NG + g;
+            for (uint32_t i = 0; i < groups[g].n; i++) p_parts[l * R + groups[g].row + i] = mla::RowParts{grp_seg_begin[v], grp_seg_begin[v + 1], i * H, 0};
+        }
     std::memcpy(h + o_csb, cta_seg_begin.data(), size_t(W + 1) * 4);
     char* d = c->meta_dev + size_t(region) * c->meta_cap;
     if (chunks) {
@@ -407,7 +453,7 @@ int build_plan(mla_ctx* c, Plan& plan, int region, const std::vector<uint32_t>& 
     m.layers = layers ? layers : 1;
     m.segs = G;
     m.ctas = W;
-    m.rec_stride = H;
+    m.rec_stride = k * H;
     m.app_rows = A;
     m.app_pos = reinterpret_cast<const uint32_t*>(d + o_apos);
     m.app_slot = reinterpret_cast<const uint64_t*>(d + o_slot);
@@ -749,8 +795,9 @@ int mla_create(const mla_config* cfg, mla_ctx** out)
     // 64 spare rows: the tcgen05 kernel fetches queries in boxes of 64 head rows
     CR_TRY(cudaMalloc(&c->q_abs, (size_t(c->ws_rows) * H + 64) * mla::kRow * 2));
     CR_TRY(cudaMemset(c->q_abs, 0, (size_t(c->ws_rows) * H + 64) * mla::kRow * 2));
-    // a plan has at most one segment per row more than it has workers
+    // a plan has at most one segment per query group more than it has workers, each of up to group_heads (or H) records
     c->rec_cap = (size_t(workers_of(cp, c->kernel, H)) + c->ws_rows) * H;
+    if (group_heads(cp) >= 2 * H) c->rec_cap += size_t(c->sm_count) * group_heads(cp) + size_t(c->ws_rows) * H;
     CR_TRY(cudaMalloc(&c->recs, c->rec_cap * mla::kPart * sizeof(float)));
     CR_TRY(cudaMalloc(&c->status_dev, sizeof(uint32_t)));
     CR_TRY(cudaMemset(c->status_dev, 0, sizeof(uint32_t)));

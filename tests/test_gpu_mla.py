@@ -715,3 +715,43 @@ def test_step_layers_in_groups_of_layers(torch, H, dt, L, lens):
     assert np.array_equal(rows[0], rows[1])
     for l in range(L):
         check_close(outs[1][l], outs[0][l], dt, f"layer {l}")
+
+
+@pytest.mark.parametrize("H,dt,spec", [
+    (16, synth.DT_F16, [(62, 5), (0, 5), (1000, 5)]),               # 80 head rows per stream; a page that only the later rows reach
+    (16, synth.DT_BF16, [(127, 2), (63, 2), (500, 1)]),             # 32 head rows, and a single row beside them
+    (16, synth.DT_F16, [(190, 4)]),                                 # 64: a full tile
+    (8, synth.DT_BF16, [(63, 2), (64, 1)]),                         # 16 columns of the transposed kernel
+    (5, synth.DT_F16, [(60, 7), (200, 3)]),                         # 35 head rows off every tile
+    (32, synth.DT_BF16, [(125, 7)]),                                # 7 rows in groups of 4 and 3
+    (16, synth.DT_F16, [(10, 1)] * 40 + [(300, 40)]),               # many single rows beside a long run
+    (100, synth.DT_BF16, [(130, 2), (64, 1)]),                      # no grouping; heads between 64 and 128
+])
+def test_rows_of_one_sequence_share_a_stream(torch, oracle, H, dt, spec):
+    """Several new tokens of a sequence in one step are attended over one stream of its pages; every row against the CPU
+    attention at its own length."""
+    from mugen_b200.mla import MlaContext
+    case = synth.make_layer_case(700 + H + len(spec), H, [a + b for a, b in spec], dt)
+    R = sum(b for _, b in spec)
+    ctx = MlaContext(n_layers=1, n_heads=H, dtype=dt, n_pages=sum((a + b) // 64 + 1 for a, b in spec), max_seqs=len(spec),
+                     max_seq_len=max(a + b for a, b in spec), max_rows=R, **YARN)
+    ctx.shuffle_free_pages(13)
+    ctx.set_layer_weights(0, case.w_uk, case.w_uv, case.w_type, case.norm_w)
+    seqs = fill(torch, ctx, case, upto=[a for a, _ in spec])
+    rng = np.random.default_rng(31)
+    kv = synth.to_bits(rng.standard_normal((R, 576), np.float32), dt)
+    q = synth.to_bits(rng.standard_normal((R, H, 192), np.float32) * np.float32(0.9), dt)
+    out = torch.zeros((R, H, 128), dtype=torch.int16, device="cuda")
+    ctx.step_begin(seqs, [b for _, b in spec])
+    ctx.step_layers(0, 1, _dev(torch, kv)[None], _dev(torch, q)[None], out[None])
+    ctx.step_end()
+    assert ctx.status() == 0
+    got, r = _host(out), 0
+    for i, (a, b) in enumerate(spec):
+        rows = oracle.append_rows(kv[r:r + b], list(range(a, a + b)), case.norm_w, YARN["rms_norm_eps"], 40.0, 4096, 10000.0, dt)
+        cache = np.concatenate([case.caches[i][:a], rows])
+        for t in range(b):
+            want = oracle.attention(q[r + t], cache, a + t + 1, case.w_uk, case.w_uv, case.w_type, H, dt)
+            check_close(got[r + t], want, dt, f"sequence {i} (start {a}), token {t}")
+        r += b
+    ctx.close()
