@@ -4,19 +4,20 @@
 //   q_abs[r][h][d] = sum_{i<128} q[r][h][i] * W_UK[h*128+i][d],  d < 512;  q_abs[r][h][512..575] = q_rope
 //   (reference: transformer.cpp:2563-2573; a query row gets the layout of a cache row)
 //
-// Absorb blocks: one per (head, group of 64 query rows).  W_UK_h^T ([512 d][128 i], contraction index
-// contiguous, made once at registration) arrives by TMA as two K-major sub-tiles [512 d][64 i]
-// (128 KB); the threads copy q_nope[64 rows][128] into swizzled operand rows; D[64 x 512] fills the
-// 512 TMEM columns with 16 tcgen05.mma M=64 N=256 K=16; 16 warps drain TMEM into whole 256-byte
-// row pieces of q_abs.
+// What bounds it is W_UK (131 KB per layer and head, read once), so the kernel is a weight stream: persistent blocks, one
+// per SM, each with an equal run of (layer, head) units.  W_UK_h^T ([512 d][128 i], contraction index contiguous, made
+// once at registration) arrives by TMA in pieces of 128 d x 64 i (16 KB) through a ring of eight or nine, across unit
+// boundaries, and is the M side of the MMA (tcgen05.mma M128 N=NT K16, four d-tiles of NT = 16, 32 or 64 columns, two
+// accumulator sets in turn); the query rows are its N side, so a step of one row does not pay for 64.  Four warps copy
+// q_nope into swizzled operand rows (two buffers) and q_rope behind the absorbed dims; four drain the accumulators.
+// Where there are fewer units than SMs (16 heads, one layer) a unit is a part of a head: one to four d-tiles, and a part of
+// the row tiles.  (One block per head with everything in sequence: 27 layers x 16 heads x 1 row took 24 us for 57 MB.)
 //
-// Append blocks (present when the caller fuses the two steps): sixteen new rows per block, one warp
-// each, the bit-exact RMSNorm + RoPE + scatter of append_kernel (mla_kernels.cu).  They share the
-// launch because the append is a chain of dependent float additions that takes as long as the absorb
-// itself and needs only a handful of SMs.
-//
-// One launch serves `layers` consecutive layers of a step whose inputs are all at hand: with one row
-// per layer (16 heads, 27 layers) a launch per layer is 16 blocks on 148 SMs.
+// Append (when the caller fuses the two steps): one new row per warp, the bit-exact RMSNorm + RoPE + scatter of
+// mla_append.cuh.  It shares the launch because it is a chain of dependent float additions that takes as long as the absorb
+// itself: four further warps of every block take up to two rows each, blocks behind the absorb blocks what is left.
+#include <algorithm>
+
 #include "mla_append.cuh"
 #include "mla_launch.h"
 #include "mla_tc5.cuh"
@@ -27,210 +28,311 @@ namespace {
 
 using namespace tc5;
 
-constexpr int MT = 64;                          // query rows per absorb block
-constexpr int W_SUB = kRank * 128;              // 65,536: [512 d][64 i]
-constexpr int W_BYTES = 2 * W_SUB;              // 131,072
-constexpr int A_SUB = MT * 128;                 // 8,192: [64 rows][64 i]
-constexpr int OFF_W = 0;
-constexpr int OFF_A = OFF_W + W_BYTES;
-constexpr int OFF_MISC = OFF_A + 2 * A_SUB;     // 147,456
-constexpr int M_BAR = 0;                        // [0] W landed, [1] MMAs complete
-constexpr int M_TMEM = 16;
-constexpr int M_FAIL = 20;
-constexpr int MISC_BYTES = 64;
-constexpr int SMEM_BYTES = OFF_MISC + MISC_BYTES + 1024;   // + slack to round the base up to 1 KB
-constexpr int NUM_THREADS = 512;
-constexpr int APPEND_ROWS = NUM_THREADS / 32;   // rows per append block
-constexpr uint32_t TMEM_COLS = 512;
+constexpr int PIECE = 128 * 128;                // 16,384: [128 d][64 i]
+constexpr int APPEND_WARPS = 4, FIRST_APPEND = 10;
+constexpr int NUM_WARPS = FIRST_APPEND + APPEND_WARPS, NUM_THREADS = 32 * NUM_WARPS;   // W producer, MMA issuer, 4 epilogue, 4 query, 4 append warps
+constexpr uint32_t APPEND_PER_WARP = 2;         // rows an absorb block's append warp takes at most
+constexpr int a_bytes(int nt) { return nt * 256; }                              // q_nope of a row tile: two sub-tiles [NT][64 i]
+constexpr int stages(int nt) { return nt == 64 ? 10 : 12; }
+constexpr int off_a(int nt) { return stages(nt) * PIECE; }
+constexpr int off_append(int nt) { return off_a(nt) + 2 * a_bytes(nt); }
+constexpr int off_misc(int nt) { return off_append(nt) + APPEND_WARPS * kAppendRowSmem; }
+constexpr int MISC_BYTES = 320;
+constexpr int smem_bytes(int nt) { return off_misc(nt) + MISC_BYTES + 1024; }   // + slack to round the base up to 1 KB
+static_assert(smem_bytes(16) <= 232448 && smem_bytes(32) <= 232448 && smem_bytes(64) <= 232448, "shared memory of one block");
+static_assert(NUM_WARPS * kAppendRowSmem <= smem_bytes(16), "the append blocks live in the absorb blocks' shared memory");
 
+struct AbsorbArgs {
+    uint32_t rows, H, layer0;
+    uint32_t d_parts, r_parts;          // a head's d-tiles (4 / d_parts per unit) and row tiles are cut into so many units
+    uint32_t units, run, blocks;        // all layers' units; units per block; absorb blocks of the grid
+    const float* cos_sin;               // not null: rotate the last 64 dims of every head with the row's position
+    const uint32_t *q_pos, *att_row;
+    uint32_t cs_rows, app_layers;
+};
 
-static_assert(APPEND_ROWS * kAppendRowSmem <= SMEM_BYTES, "the append blocks live in the absorb blocks' shared memory");
-
-template <typename T>
+template <typename T, int NT>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict__ q, T* __restrict__ q_abs, uint32_t rows,
-                  uint32_t H, uint32_t layer0, uint32_t absorb_blocks, const AppendArgs app, const float* __restrict__ q_cos_sin,
-                  const uint32_t* __restrict__ q_pos, const uint32_t* __restrict__ att_row, uint32_t cs_rows,
-                  uint32_t* __restrict__ status)
+absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict__ q, T* __restrict__ q_abs, const AbsorbArgs a,
+                  const AppendArgs app, uint32_t* __restrict__ status)
 {
+    constexpr int STAGES = stages(NT), OFF_A = off_a(NT), OFF_MISC = off_misc(NT);
+    constexpr uint32_t TMEM_COLS = 8 * NT;                      // two sets of four d-tiles x NT columns
     extern __shared__ unsigned char absorb_tc5_smem[];
     grid_launch_dependents();
-    if (blockIdx.x >= absorb_blocks) {
-        // Apart from kv_a the append touches nothing that an earlier kernel of the stream still reads or writes:
-        // constant tables, the step metadata (uploaded before the step's first kernel), and slots of this layer's
-        // pool, last read by this layer's attention in the PREVIOUS step.  Where the host knows that kv_a was complete
-        // before the kernel ahead of this one started (the later layers of a multi-layer call, whose kv_a the caller
-        // handed over with the first layer's), the append works first and waits last; the wait then only keeps "this
-        // kernel completes after its predecessors", which the kernels behind it rely on.
-        if (app.wait_first) grid_dependency_wait();
-        const uint32_t per_layer = (app.rows + APPEND_ROWS - 1) / APPEND_ROWS, b = blockIdx.x - absorb_blocks;
-        append_row<T>(app, b / per_layer, (b % per_layer) * APPEND_ROWS + threadIdx.x / 32, absorb_tc5_smem + (threadIdx.x / 32) * kAppendRowSmem, status);
-        if (!app.wait_first) grid_dependency_wait();
+    const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    // Apart from kv_a the append touches nothing that an earlier kernel of the stream still reads or writes: constant
+    // tables, the step metadata (uploaded before the step's first kernel), and slots of this layer's pool, last read by
+    // this layer's attention in the PREVIOUS step.  Where the host knows that kv_a was complete before the kernel ahead of
+    // this one started (the later layers of a multi-layer call, whose kv_a the caller handed over with the first layer's),
+    // the append works first and waits last; the wait then only keeps "this kernel completes after its predecessors", which
+    // the kernels behind it rely on.
+    const uint32_t app_total = app.rows * a.app_layers, app_inside = min(app_total, a.blocks * APPEND_WARPS * APPEND_PER_WARP);
+    auto append = [&](uint32_t i0, uint32_t step, uint32_t end, unsigned char* smem) {
+        bool waited = !app.wait_first;
+        for (uint32_t i = i0; i < end; i += step) {
+            AppendRow<T> row;
+            row.prepare(app, i / app.rows, i % app.rows, status);
+            if (!waited) { grid_dependency_wait(); waited = true; }
+            row.run(app, smem);
+        }
+        if (!app.wait_first || !waited) grid_dependency_wait();
+    };
+    if (blockIdx.x >= a.blocks) {
+        append(app_inside + (blockIdx.x - a.blocks) * NUM_WARPS + warp, ~0u / 2, app_total, absorb_tc5_smem + warp * kAppendRowSmem);
         return;
     }
     const uint32_t raw = smem_u32(absorb_tc5_smem);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char* sm = absorb_tc5_smem + (base - raw);
-    const uint32_t sW = base + OFF_W, sA = base + OFF_A;
-    const uint32_t bar_w = base + OFF_MISC + M_BAR, bar_mma = bar_w + 8;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + OFF_MISC + M_TMEM);
-    volatile int* fail_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + M_FAIL);
-    const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-    // head fastest, then row tile, then layer; virtual row layer * rows + r indexes q_abs (and q, unless att_row renames it)
-    const uint32_t row_tiles = (rows + MT - 1) / MT, rest = blockIdx.x / H;
-    const uint32_t h = blockIdx.x % H, r0 = (rest % row_tiles) * MT, li = rest / row_tiles;
-    q += size_t(li) * rows * H * kQDim;
-    q_abs += size_t(li) * rows * H * kRow;
+    const uint32_t bar0 = base + OFF_MISC;        // full[STAGES], empty[STAGES], a_full[2], a_empty[2], acc_full[2], acc_empty[2]
+    auto full = [&](uint32_t s) { return bar0 + 8u * s; };
+    auto empty = [&](uint32_t s) { return bar0 + 8u * (STAGES + s); };
+    auto a_full = [&](uint32_t b) { return bar0 + 8u * (2 * STAGES + b); };
+    auto a_empty = [&](uint32_t b) { return bar0 + 8u * (2 * STAGES + 2 + b); };
+    auto acc_full = [&](uint32_t b) { return bar0 + 8u * (2 * STAGES + 4 + b); };
+    auto acc_empty = [&](uint32_t b) { return bar0 + 8u * (2 * STAGES + 6 + b); };
+    static_assert((2 * STAGES + 8) * 8 <= 304, "barriers overflow their area");
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + OFF_MISC + 304);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + 308);
+
+    const uint32_t row_tiles = (a.rows + NT - 1) / NT, n_d = 4 / a.d_parts;
+    const uint32_t u0 = blockIdx.x * a.run, u1 = min(a.units, u0 + a.run);
+    struct Unit { uint32_t li, h, d0, rt0, rt1; };
+    auto unit_of = [&](uint32_t u) -> Unit {
+        Unit x;
+        const uint32_t parts = a.d_parts * a.r_parts, hu = u / parts, p = u % parts, rp = p % a.r_parts;
+        x.h = hu % a.H;
+        x.li = hu / a.H;
+        x.d0 = (p / a.r_parts) * n_d;
+        x.rt0 = row_tiles * rp / a.r_parts;
+        x.rt1 = row_tiles * (rp + 1) / a.r_parts;
+        return x;
+    };
 
     if (tid == 0) {
-        *fail_flag = 0;
-        mbar_init(bar_w, 1);
-        mbar_init(bar_mma, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        mbar_expect_tx(bar_w, W_BYTES);                      // W_UK_h^T: four boxes of 64 i x 256 d
-#pragma unroll 1
-        for (int bx = 0; bx < 4; bx++)
-            tma_load_2d(sW + (bx / 2) * W_SUB + (bx % 2) * (W_SUB / 2), &map_w, bar_w, 64 * (bx / 2), int((layer0 + li) * H + h) * kRank + 256 * (bx % 2));
+        *abort_flag = 0;
+        for (uint32_t s = 0; s < STAGES; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
+        for (uint32_t b = 0; b < 2; b++) { mbar_init(a_full(b), 128); mbar_init(a_empty(b), 1); mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 128); }
+        mbar_init_fence();
     }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
-                     ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    }
-    // the weights are constant; everything below reads or writes what earlier kernels of the stream touch
-    grid_dependency_wait();
-    // q_nope tile -> two swizzled K-major sub-tiles; q_rope -> behind the absorbed dims
-    for (uint32_t c = tid; c < MT * 16; c += NUM_THREADS) {                 // 16 chunks of 16 bytes per row
-        const uint32_t rr = c / 16, ch = c % 16, r = r0 + rr;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (r < rows) v = reinterpret_cast<const uint4*>(q + (size_t(att_row ? att_row[r] : r) * H + h) * kQDim)[ch];
-        *reinterpret_cast<uint4*>(sm + OFF_A + (ch / 8) * A_SUB + rr * 128 + (((ch % 8) ^ (rr & 7)) << 4)) = v;
-    }
-    if (q_cos_sin == nullptr) {
-        for (uint32_t c = tid; c < MT * 8; c += NUM_THREADS) {              // rope part, already rotated: 8 chunks per row
-            const uint32_t rr = c / 8, ch = c % 8, r = r0 + rr;
-            if (r < rows)
-                reinterpret_cast<uint4*>(q_abs + (size_t(r) * H + h) * kRow + kRank)[ch] =
-                    reinterpret_cast<const uint4*>(q + (size_t(att_row ? att_row[r] : r) * H + h) * kQDim + kNope)[ch];
-        }
-    } else {
-        // q-side RoPE (reference: transformer.cpp:3882-3921, NeoX pairs (i, i+32), YaRN frequencies): the same
-        // table and the same separately rounded products as the k_rope rotation of the append
-        for (uint32_t c = tid; c < MT * (kRope / 2); c += NUM_THREADS) {
-            const uint32_t rr = c / (kRope / 2), i = c % (kRope / 2), r = r0 + rr;
-            if (r >= rows) continue;
-            const uint32_t pos = q_pos[r];
-            if (pos >= cs_rows) {
-                if (i == 0) atomicOr(status, ST_BAD_SLOT);
-                continue;
-            }
-            const T* src = q + (size_t(att_row ? att_row[r] : r) * H + h) * kQDim + kNope;
-            T* dst = q_abs + (size_t(r) * H + h) * kRow + kRank;
-            const float cs = q_cos_sin[size_t(pos) * kRope + i], sn = q_cos_sin[size_t(pos) * kRope + 32 + i];
-            const float x0 = Elem<T>::to_f32(src[i]), x1 = Elem<T>::to_f32(src[32 + i]);
-            dst[i]      = Elem<T>::from_f32(__fsub_rn(__fmul_rn(x0, cs), __fmul_rn(x1, sn)));
-            dst[32 + i] = Elem<T>::from_f32(__fadd_rn(__fmul_rn(x1, cs), __fmul_rn(x0, sn)));
-        }
-    }
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    if (warp == 1) tc_alloc<TMEM_COLS>(tmem_slot);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    bool ok = true;
     if (warp == 0) {
-        ok = mbar_wait(bar_w, 0, fail_flag, status);
-        tc_fence_after();
-        if (ok && elect_one()) {
-            constexpr uint32_t IDESC = instr_desc(Fmt<T>::v, MT, 256);
-#pragma unroll
-            for (int half = 0; half < 2; half++) {
-#pragma unroll
-                for (int s = 0; s < 2; s++) {
-#pragma unroll
-                    for (int k = 0; k < 4; k++)
-                        tc_mma(tmem + half * 256, desc_lo(sA + s * A_SUB + k * 32), desc_hi(1024),
-                               desc_lo(sW + s * W_SUB + half * (W_SUB / 2) + k * 32), desc_hi(1024), IDESC, (s == 0 && k == 0) ? 0u : 1u);
+        // ---- the weights are constant: their loads do not wait for earlier kernels
+        if (lane == 0) {
+            bool ok = true;
+            uint32_t i = 0;
+            for (uint32_t u = u0; u < u1 && ok; u++) {
+                const Unit x = unit_of(u);
+                const int row = int(((a.layer0 + x.li) * a.H + x.h) * kRank);
+                for (uint32_t p = 0; p < 2 * n_d && ok; p++, i++) {
+                    const uint32_t s = i % STAGES;
+                    ok = mbar_wait(empty(s), ((i / STAGES) & 1) ^ 1, abort_flag, status);
+                    if (!ok) break;
+                    mbar_expect_tx(full(s), PIECE);
+                    tma_load_2d(base + s * PIECE, &map_w, full(s), 64 * int(p & 1), row + 128 * int(x.d0 + p / 2));
                 }
             }
-            tc_commit(bar_mma);
+            grid_dependency_wait();
         }
-        __syncwarp();
-    }
-    // D (M=64): rows 16*q .. 16*q+15 sit in lanes 0-15 of TMEM sub-partition q; warp w drains the
-    // 128 columns 128*(w/4) .. of sub-partition w%4
-    ok = mbar_wait(bar_mma, 0, fail_flag, status) && ok;
-    ok = __all_sync(0xffffffffu, ok);
-    if (ok) {
-        tc_fence_after();
-        const uint32_t qp = warp % 4, cg = warp / 4;
-        const uint32_t row = r0 + 16 * qp + lane;
+    } else if (warp == 1) {
+        constexpr uint32_t IDESC = instr_desc(Fmt<T>::v, 128, NT), HI = desc_hi(1024);
+        bool ok = true;
+        uint32_t i = 0, n = 0;                     // weight pieces and row tiles so far
+        for (uint32_t u = u0; u < u1 && ok; u++) {
+            const Unit x = unit_of(u);
+            for (uint32_t rt = x.rt0; rt < x.rt1 && ok; rt++, n++) {
+                const uint32_t b = n & 1, par = (n >> 1) & 1;
+                ok = mbar_wait(a_full(b), par, abort_flag, status) && mbar_wait(acc_empty(b), par ^ 1, abort_flag, status);
+                for (uint32_t p = 0; p < 2 * n_d && ok; p++) {
+                    const uint32_t s = (i + p) % STAGES;
+                    ok = mbar_wait(full(s), ((i + p) / STAGES) & 1, abort_flag, status);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint32_t da = desc_lo(base + s * PIECE), db = desc_lo(base + OFF_A + b * a_bytes(NT) + (p & 1) * (NT * 128));
+#pragma unroll
+                        for (int k = 0; k < 4; k++)
+                            tc_mma(tmem + b * 4 * NT + (p / 2) * NT, da + ((k * 32) >> 4), HI, db + ((k * 32) >> 4), HI, IDESC, ((p & 1) == 0 && k == 0) ? 0u : 1u);
+                        if (rt + 1 == x.rt1) tc_commit(empty(s));          // the unit's last row tile frees the weights
+                        if (p + 1 == 2 * n_d) { tc_commit(a_empty(b)); tc_commit(acc_full(b)); }
+                    }
+                    __syncwarp();
+                }
+            }
+            i += 2 * n_d;
+        }
+    } else if (warp < 6) {
+        // ---- epilogue: lane = d, columns = query rows
+        grid_dependency_wait();                    // q_abs is still read by the attention kernel before
+        const uint32_t q4 = warp % 4;
+        bool ok = true;
+        uint32_t n = 0;
+        for (uint32_t u = u0; u < u1; u++) {
+            const Unit x = unit_of(u);
+            for (uint32_t rt = x.rt0; rt < x.rt1; rt++, n++) {
+                const uint32_t b = n & 1;
+                ok = ok && mbar_wait(acc_full(b), (n >> 1) & 1, abort_flag, status);
+                ok = __all_sync(0xffffffffu, ok);
+                tc_fence_after();
+                constexpr int CH = NT < 32 ? 16 : 32;
+                const uint32_t live = min(uint32_t(NT), a.rows - rt * NT);
 #pragma unroll 1
-        for (int c = 0; c < 4; c++) {
-            uint32_t o[32];
-            tc_ld32(tmem + ((qp * 32u) << 16) + cg * 128 + c * 32, o);
-            tc_wait_ld();
-            if (lane < 16 && row < rows) {
-                uint4* dst = reinterpret_cast<uint4*>(q_abs + (size_t(row) * H + h) * kRow + cg * 128 + c * 32);
+                for (uint32_t d = 0; d < n_d; d++) {
+                    T* dst = q_abs + ((size_t(x.li) * a.rows + rt * NT) * a.H + x.h) * kRow + (x.d0 + d) * 128 + q4 * 32 + lane;
+#pragma unroll 1
+                    for (uint32_t c = 0; c < NT; c += CH) {
+                        if (c >= live) break;
+                        uint32_t o[CH];
+                        tc_ldn(tmem + ((q4 * 32u) << 16) + b * 4 * NT + d * NT + c, o);
+                        tc_wait_ld();
 #pragma unroll
-                for (int x = 0; x < 4; x++) {
-                    uint32_t pk[4];
+                        for (int k = 0; k < CH; k++)
+                            if (ok && c + k < live) dst[size_t(c + k) * a.H * kRow] = Elem<T>::from_f32(__uint_as_float(o[k]));
+                    }
+                }
+                tc_fence_before();
+                mbar_arrive(acc_empty(b));
+            }
+        }
+    } else if (warp >= FIRST_APPEND) {
+        append(blockIdx.x * APPEND_WARPS + warp - FIRST_APPEND, a.blocks * APPEND_WARPS, app_inside, sm + off_append(NT) + (warp - FIRST_APPEND) * kAppendRowSmem);
+    } else {
+        // ---- query rows: q_nope -> operand rows, q_rope -> behind the absorbed dims (by the unit that has d-tile 0)
+        grid_dependency_wait();
+        const uint32_t t = tid - 6 * 32;
+        bool ok = true;
+        uint32_t n = 0;
+        for (uint32_t u = u0; u < u1; u++) {
+            const Unit x = unit_of(u);
+            const T* ql = q + size_t(x.li) * a.rows * a.H * kQDim;
+            for (uint32_t rt = x.rt0; rt < x.rt1; rt++, n++) {
+                const uint32_t b = n & 1, r0 = rt * NT;
+                ok = ok && mbar_wait(a_empty(b), ((n >> 1) & 1) ^ 1, abort_flag, status);
+                unsigned char* dst = sm + OFF_A + b * a_bytes(NT);
+                auto q_row = [&](uint32_t r) -> const T* { return ql + (size_t(a.att_row ? a.att_row[r] : r) * a.H + x.h) * kQDim; };
+                uint4 v[NT / 8];                                          // 16 chunks of 16 bytes per row
 #pragma unroll
-                    for (int i = 0; i < 4; i++)
-                        pk[i] = Elem<T>::pack2(__uint_as_float(o[8 * x + 2 * i]), __uint_as_float(o[8 * x + 2 * i + 1]));
-                    dst[x] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                for (int k = 0; k < NT / 8; k++) {
+                    const uint32_t c = t + 128 * k, rr = c / 16;
+                    v[k] = r0 + rr < a.rows ? reinterpret_cast<const uint4*>(q_row(r0 + rr))[c % 16] : make_uint4(0, 0, 0, 0);
+                }
+#pragma unroll
+                for (int k = 0; k < NT / 8; k++) {
+                    const uint32_t c = t + 128 * k, rr = c / 16, ch = c % 16;
+                    *reinterpret_cast<uint4*>(dst + (ch / 8) * (NT * 128) + rr * 128 + (((ch % 8) ^ (rr & 7)) << 4)) = v[k];
+                }
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                mbar_arrive(a_full(b));
+                if (x.d0 != 0) continue;
+                T* qa = q_abs + (size_t(x.li) * a.rows * a.H + x.h) * kRow + kRank;
+                if (a.cos_sin == nullptr) {
+                    for (uint32_t c = t; c < NT * 8; c += 128) {          // already rotated: 8 chunks per row
+                        const uint32_t r = r0 + c / 8;
+                        if (r < a.rows)
+                            reinterpret_cast<uint4*>(qa + size_t(r) * a.H * kRow)[c % 8] = reinterpret_cast<const uint4*>(q_row(r) + kNope)[c % 8];
+                    }
+                } else {
+                    // q-side RoPE (reference: transformer.cpp:3882-3921, NeoX pairs (i, i+32), YaRN frequencies): the same
+                    // table and the same separately rounded products as the k_rope rotation of the append; eight pairs at a time
+                    for (uint32_t c = t; c < NT * 4; c += 128) {
+                        const uint32_t r = r0 + c / 4, i = (c % 4) * 8;
+                        if (r >= a.rows) continue;
+                        const uint32_t pos = a.q_pos[r];
+                        const uint4* src = reinterpret_cast<const uint4*>(q_row(r) + kNope + i);
+                        const uint4 v0 = src[0], v1 = src[4];
+                        if (pos >= a.cs_rows) {
+                            if (i == 0) atomicOr(status, ST_BAD_SLOT);
+                            continue;
+                        }
+                        const float4* tb = reinterpret_cast<const float4*>(a.cos_sin + size_t(pos) * kRope + i);
+                        const float4 c0 = __ldg(tb), c1 = __ldg(tb + 1), s0 = __ldg(tb + 8), s1 = __ldg(tb + 9);
+                        const float cs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w}, sn[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+                        const T *x0 = reinterpret_cast<const T*>(&v0), *x1 = reinterpret_cast<const T*>(&v1);
+                        float y0[8], y1[8];
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            const float f0 = Elem<T>::to_f32(x0[j]), f1 = Elem<T>::to_f32(x1[j]);
+                            y0[j] = __fsub_rn(__fmul_rn(f0, cs[j]), __fmul_rn(f1, sn[j]));
+                            y1[j] = __fadd_rn(__fmul_rn(f1, cs[j]), __fmul_rn(f0, sn[j]));
+                        }
+                        uint4* o = reinterpret_cast<uint4*>(qa + size_t(r) * a.H * kRow + i);
+                        o[0] = make_uint4(Elem<T>::pack2(y0[0], y0[1]), Elem<T>::pack2(y0[2], y0[3]), Elem<T>::pack2(y0[4], y0[5]), Elem<T>::pack2(y0[6], y0[7]));
+                        o[4] = make_uint4(Elem<T>::pack2(y1[0], y1[1]), Elem<T>::pack2(y1[2], y1[3]), Elem<T>::pack2(y1[4], y1[5]), Elem<T>::pack2(y1[6], y1[7]));
+                    }
                 }
             }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) {
+    if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+        tc_dealloc<TMEM_COLS>(tmem);
     }
+}
+
+template <typename T>
+cudaError_t configure_type()
+{
+    auto set = [](auto kernel, int bytes) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        // every kernel of a layer-step asks for the same (maximal) shared-memory carve-out, so the SMs are not
+        // re-partitioned between consecutive launches
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    };
+    cudaError_t e = set(absorb_tc5_kernel<T, 16>, smem_bytes(16));
+    if (e == cudaSuccess) e = set(absorb_tc5_kernel<T, 32>, smem_bytes(32));
+    if (e == cudaSuccess) e = set(absorb_tc5_kernel<T, 64>, smem_bytes(64));
+    return e;
 }
 
 }  // namespace
 
 int absorb_tc5_configure()
 {
-    cudaError_t e = cudaFuncSetAttribute(absorb_tc5_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return int(e);
-    e = cudaFuncSetAttribute(absorb_tc5_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return int(e);
-    // every kernel of a layer-step asks for the same (maximal) shared-memory carve-out, so the SMs are not
-    // re-partitioned between consecutive launches
-    e = cudaFuncSetAttribute(absorb_tc5_kernel<__half>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return int(e);
-    e = cudaFuncSetAttribute(absorb_tc5_kernel<__nv_bfloat16>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    return int(e);
+    const cudaError_t e = configure_type<__half>();
+    return int(e != cudaSuccess ? e : configure_type<__nv_bfloat16>());
 }
 
-// w_map: host CUtensorMap over W_UK^T of all layers ([layers*H*512 d][128 i], box 64 i x 256 d, 128-byte swizzle).  q, q_abs
+// w_map: host CUtensorMap over W_UK^T of all layers ([layers*H*512 d][128 i], box 64 i x 128 d, 128-byte swizzle).  q, q_abs
 // and (with kv_a != nullptr: the launch also appends) kv_a hold m.layers consecutive layers from layer0; layer_pool and
 // norm_w point at layer0's slices.  With rotate_q the last 64 dims of every query head are rotated with the row's
 // position (m.row_pos) before they are stored.
 int launch_absorb_tc5(int dtype, const void* q, const void* w_map, void* q_abs, uint32_t H, uint32_t layer0, const void* kv_a,
                       void* layer_pool, uint64_t pool_slots, const void* norm_w, const float* cos_sin, uint32_t cs_rows,
-                      float eps, const StepMeta& m, bool rotate_q, bool append_waits, uint32_t* status, cudaStream_t st)
+                      float eps, const StepMeta& m, bool rotate_q, bool append_waits, uint32_t sm_count, uint32_t* status, cudaStream_t st)
 {
     if (m.rows == 0) return 0;
     const CUtensorMap* map = static_cast<const CUtensorMap*>(w_map);
     AppendArgs app{};
     if (kv_a) app = AppendArgs{kv_a, layer_pool, pool_slots, norm_w, cos_sin, cs_rows, eps, m.app_pos, m.app_slot, m.app_rows, append_waits ? 1u : 0u};
-    const uint32_t absorb_blocks = m.layers * H * ((m.rows + MT - 1) / MT);
-    const uint32_t append_blocks = m.layers * ((app.rows + APPEND_ROWS - 1) / APPEND_ROWS);
-    // append blocks carry the trailing indices
-    dim3 grid(absorb_blocks + append_blocks);
+    const uint32_t nt = m.rows <= 16 ? 16 : m.rows <= 32 ? 32 : 64, row_tiles = (m.rows + nt - 1) / nt, heads = m.layers * H;
+    AbsorbArgs a{m.rows, H, layer0, 1, 1, 0, 0, 0, rotate_q ? cos_sin : nullptr, m.row_pos, m.att_row, cs_rows, m.layers};
+    // a head is cut while its parts still leave SMs idle: along d first (the weights are then still read once)
+    while (a.d_parts < 4 && heads * a.d_parts * 2 <= sm_count) a.d_parts *= 2;
+    a.r_parts = std::max(1u, std::min(row_tiles, sm_count / (heads * a.d_parts)));
+    a.units = heads * a.d_parts * a.r_parts;
+    a.run = (a.units + sm_count - 1) / sm_count;
+    a.blocks = (a.units + a.run - 1) / a.run;
+    const uint32_t app_total = app.rows * m.layers, app_inside = std::min(app_total, a.blocks * APPEND_WARPS * APPEND_PER_WARP);
+    dim3 grid(a.blocks + (app_total - app_inside + NUM_WARPS - 1) / NUM_WARPS);        // append blocks carry the trailing indices
     auto go = [&](auto kernel, auto* qp, auto* qa) {
-        return int(launch_pdl(kernel, grid, dim3(NUM_THREADS), SMEM_BYTES, st, *map, qp, qa, m.rows, H, layer0, absorb_blocks, app,
-                              rotate_q ? cos_sin : nullptr, m.row_pos, m.att_row, cs_rows, status));
+        return int(launch_pdl(kernel, grid, dim3(NUM_THREADS), size_t(smem_bytes(int(nt))), st, *map, qp, qa, a, app, status));
     };
-    if (dtype == 0) return go(absorb_tc5_kernel<__half>, static_cast<const __half*>(q), static_cast<__half*>(q_abs));
-    return go(absorb_tc5_kernel<__nv_bfloat16>, static_cast<const __nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(q_abs));
+    if (dtype == 0) {
+        const auto* qp = static_cast<const __half*>(q);
+        auto* qa = static_cast<__half*>(q_abs);
+        return nt == 16 ? go(absorb_tc5_kernel<__half, 16>, qp, qa) : nt == 32 ? go(absorb_tc5_kernel<__half, 32>, qp, qa) : go(absorb_tc5_kernel<__half, 64>, qp, qa);
+    }
+    const auto* qp = static_cast<const __nv_bfloat16*>(q);
+    auto* qa = static_cast<__nv_bfloat16*>(q_abs);
+    return nt == 16 ? go(absorb_tc5_kernel<__nv_bfloat16, 16>, qp, qa) : nt == 32 ? go(absorb_tc5_kernel<__nv_bfloat16, 32>, qp, qa) : go(absorb_tc5_kernel<__nv_bfloat16, 64>, qp, qa);
 }
 
 }  // namespace mla

@@ -359,10 +359,10 @@ int build_plan(mla_ctx* c, Plan& plan, int region, const std::vector<uint32_t>& 
             for (uint32_t g = 0; g < NG; g++) lens[g] = rows[groups[g].row + groups[g].n - 1].attend_len;
             for (uint32_t l = 1; l < layers; l++) std::copy(lens.begin(), lens.begin() + NG, lens.begin() + size_t(l) * NG);
             if (plan.kernel == MLA_KERNEL_TCGEN05_PAIR128)
-                // a worker pays about five tiles' time per segment it starts (queries, pipeline fill, state drain: ~10 us)
-                mugen::mla::plan_min_makespan(lens, mla::kPage, workers, segs, grp_seg_begin, cta_seg_begin, 2u, 5u);
+                // a worker pays a few tiles' time per segment it starts (queries, pipeline fill, state drain)
+                mugen::mla::plan_min_makespan(lens, mla::kPage, workers, segs, grp_seg_begin, cta_seg_begin, 2u, 3u);
             else
-                mugen::mla::plan_balanced(lens, mla::kPage, workers, segs, grp_seg_begin, cta_seg_begin, 1u);
+                mugen::mla::plan_min_makespan(lens, mla::kPage, workers, segs, grp_seg_begin, cta_seg_begin, 1u, 2u);
             break;
         }
         if (segs.size() * k * H > c->rec_cap)
@@ -539,7 +539,7 @@ int run_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, float* expo
     const int dt = int(c->cfg.dtype);
     const int ae = mla::launch_absorb_tc5(dt, q, &c->w_uk_map, c->q_abs, H, layer, fused_kv_a, layer_pool(c, layer), c->pool_slots,
                                           layer_norm(c, layer), c->cos_sin, c->cs_rows, c->cfg.rms_norm_eps, m, c->q_rope_in_kernel,
-                                          !kv_a_settled, c->status_dev, st);
+                                          !kv_a_settled, uint32_t(c->sm_count), c->status_dev, st);
     if (ae != 0) return fail(c, MLA_ERR_CUDA, std::string("absorb launch: ") + cudaGetErrorString(cudaError_t(ae)));
     int e;
     const bool timed = c->profiling && c->prof_used < c->prof_events.size() && (c->prof_seq++ % c->prof_stride) == 0;
@@ -562,7 +562,7 @@ int run_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, float* expo
     if (exported) {
         e = mla::launch_export_partial(c->recs, m, exported, H, st);
     } else {
-        e = mla::launch_merge_tc5(dt, c->recs, m, 0, &c->w_uv_map, out, H, layer, c->status_dev, st);
+        e = mla::launch_merge_tc5(dt, c->recs, m, 0, &c->w_uv_map, out, H, layer, uint32_t(c->sm_count), c->status_dev, st);
     }
     if (e != 0) return fail(c, MLA_ERR_CUDA, std::string("merge launch: ") + cudaGetErrorString(cudaError_t(e)));
     c->launches += 3;
@@ -677,7 +677,7 @@ int make_tensor_maps(mla_ctx* c)
         return MLA_OK;
     };
     {   // W_UV of all layers as [layers*H*128 outputs][512 dims], boxes of 64 dims x 128 outputs (merge), and W_UK^T as
-        // [layers*H*512 d][128 i], boxes of 64 i x 256 d (absorb)
+        // [layers*H*512 d][128 i], boxes of 64 i x 128 d (absorb)
         auto weights = [&](CUtensorMap* map, const char* what, void* basep, cuuint64_t inner, cuuint64_t outer, cuuint32_t box_rows) -> int {
             const cuuint64_t dims[2] = {inner, outer}, strides[1] = {inner * 2};
             const cuuint32_t box[2] = {64, box_rows};
@@ -692,7 +692,7 @@ int make_tensor_maps(mla_ctx* c)
         if (!mla::gemm_tc5_weight_maps(&c->w_uk_rows_maps, int(c->cfg.dtype), c->w_uk_rows, heads * mla::kNope, mla::kRank) ||
             !mla::gemm_tc5_weight_maps(&c->w_uv_maps, int(c->cfg.dtype), c->w_uv, heads * mla::kVDim, mla::kRank))
             return fail(c, MLA_ERR_CUDA, "cuTensorMapEncodeTiled(expansion weights) failed");
-        if (int e = weights(&c->w_uk_map, "W_UK", c->w_uk, mla::kNope, heads * mla::kRank, 256)) return e;
+        if (int e = weights(&c->w_uk_map, "W_UK", c->w_uk, mla::kNope, heads * mla::kRank, 128)) return e;
     }
     {   // cache pool: 576 values innermost, then the token slots of a layer, then layers;
         // box = 64 values (128 B, one swizzle row) x 64 tokens (one page)
@@ -1215,7 +1215,7 @@ int mla_merge_partials(mla_ctx* c, uint32_t layer, uint32_t n_parts, uint32_t ro
     mla::StepMeta m{};
     m.rows = rows;
     m.layers = 1;
-    const int e = mla::launch_merge_tc5(int(c->cfg.dtype), partials, m, n_parts, &c->w_uv_map, out, c->cfg.n_heads, layer, c->status_dev,
+    const int e = mla::launch_merge_tc5(int(c->cfg.dtype), partials, m, n_parts, &c->w_uv_map, out, c->cfg.n_heads, layer, uint32_t(c->sm_count), c->status_dev,
                                         static_cast<cudaStream_t>(stream));
     if (e != 0) return fail(c, MLA_ERR_CUDA, std::string("merge launch: ") + cudaGetErrorString(cudaError_t(e)));
     c->launches += rows ? 1 : 0;
@@ -1486,6 +1486,7 @@ int project(mla_ctx* c, const void* act, uint32_t rows, uint32_t K, std::initial
     g.M = rows;
     g.K = K;
     for (const auto& w : weights) g.w[g.n_weights++] = w;
+    g.packed = true;
     g.residual = residual;
     const int rc = mla::launch_gemm_tc5(int(c->cfg.dtype), g, c->gemm_ws, c->status_dev, st);
     if (rc == -1) return fail(c, MLA_ERR_INVALID, "projection operands must be 16-byte aligned with row lengths that are multiples of 8");
@@ -1537,6 +1538,7 @@ int mla_set_block_weights(mla_ctx* c, uint32_t layer, const mla_block_weights* w
     if (!w->attn_norm || !w->kv_a_mqa || !w->wo || (R ? (!w->q_a || !w->q_a_norm || !w->q_b) : !w->q))
         return fail(c, MLA_ERR_INVALID, "missing projection weight for this q_lora_rank");
     BlockW& b = c->blocks[layer];
+    const uint32_t QD = H * uint32_t(mla::kQDim), VD = H * uint32_t(mla::kVDim);
     auto put = [&](void** dst, const void* src, size_t n) -> int {
         if (*dst) { cudaFree(*dst); *dst = nullptr; }
         if (!src) return MLA_OK;
@@ -1544,21 +1546,31 @@ int mla_set_block_weights(mla_ctx* c, uint32_t layer, const mla_block_weights* w
         CU_TRY(c, cudaMemcpy(*dst, src, n * 2, cudaMemcpyHostToDevice));
         return MLA_OK;
     };
+    // matrices are staged row-major and repacked into tiles on the device
+    void* stage = nullptr;
+    const size_t stage_values = std::max({size_t(R) * E, R ? size_t(QD) * R : size_t(QD) * E, size_t(mla::kRow) * E, size_t(E) * VD});
+    CU_TRY(c, cudaMalloc(&stage, stage_values * 2));
+    auto put_matrix = [&](void** dst, mla::GemmWeightMaps* maps, const void* src, uint32_t N, uint32_t K) -> int {
+        if (*dst) { cudaFree(*dst); *dst = nullptr; }
+        if (!src) return MLA_OK;
+        CU_TRY(c, cudaMalloc(dst, mla::gemm_tc5_packed_values(N, K) * 2));
+        CU_TRY(c, cudaMemcpy(stage, src, size_t(N) * K * 2, cudaMemcpyHostToDevice));
+        if (int rc = mla::launch_gemm_pack(stage, *dst, N, K, nullptr)) return fail(c, MLA_ERR_CUDA, std::string("weight packing: ") + cudaGetErrorString(cudaError_t(rc)));
+        if (!mla::gemm_tc5_packed_maps(maps, int(c->cfg.dtype), *dst, N, K)) return fail(c, MLA_ERR_CUDA, "cuTensorMapEncodeTiled(projection weights) failed");
+        return MLA_OK;
+    };
     b.set = false;
-    if (int e = put(&b.attn_norm, w->attn_norm, E)) return e;
-    if (int e = put(&b.q_a, R ? w->q_a : nullptr, size_t(R) * E)) return e;
-    if (int e = put(&b.q_a_norm, R ? w->q_a_norm : nullptr, R)) return e;
-    if (int e = put(&b.q_b, R ? w->q_b : nullptr, size_t(H) * mla::kQDim * R)) return e;
-    if (int e = put(&b.q, R ? nullptr : w->q, size_t(H) * mla::kQDim * E)) return e;
-    if (int e = put(&b.kv_a, w->kv_a_mqa, size_t(mla::kRow) * E)) return e;
-    if (int e = put(&b.wo, w->wo, size_t(E) * H * mla::kVDim)) return e;
-    const int dt = int(c->cfg.dtype);
-    const uint32_t QD = H * uint32_t(mla::kQDim);
-    if (!(R ? mla::gemm_tc5_weight_maps(&b.q_a_map, dt, b.q_a, R, E) && mla::gemm_tc5_weight_maps(&b.q_b_map, dt, b.q_b, QD, R)
-            : mla::gemm_tc5_weight_maps(&b.q_map, dt, b.q, QD, E)) ||
-        !mla::gemm_tc5_weight_maps(&b.kv_a_map, dt, b.kv_a, uint64_t(mla::kRow), E) ||
-        !mla::gemm_tc5_weight_maps(&b.wo_map, dt, b.wo, E, uint64_t(H) * mla::kVDim))
-        return fail(c, MLA_ERR_CUDA, "cuTensorMapEncodeTiled(projection weights) failed");
+    int e = put(&b.attn_norm, w->attn_norm, E);
+    if (!e) e = put(&b.q_a_norm, R ? w->q_a_norm : nullptr, R);
+    if (!e) e = put_matrix(&b.q_a, &b.q_a_map, R ? w->q_a : nullptr, R, E);
+    if (!e) e = put_matrix(&b.q_b, &b.q_b_map, R ? w->q_b : nullptr, QD, R);
+    if (!e) e = put_matrix(&b.q, &b.q_map, R ? nullptr : w->q, QD, E);
+    if (!e) e = put_matrix(&b.kv_a, &b.kv_a_map, w->kv_a_mqa, uint32_t(mla::kRow), E);
+    if (!e) e = put_matrix(&b.wo, &b.wo_map, w->wo, E, VD);
+    const cudaError_t done = cudaDeviceSynchronize();            // the packing runs on the default stream, the projections need not
+    cudaFree(stage);
+    if (e) return e;
+    CU_TRY(c, done);
     b.embed = E;
     b.q_lora = R;
     b.set = true;

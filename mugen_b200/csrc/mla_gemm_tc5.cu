@@ -22,7 +22,10 @@
 //                    block holding 128 rows of A and half of the outputs' weight rows.  What bounds it is the L2 -> shared
 //                    memory feed (measured with one block per 128 x 256 tile: 48 KB per 4.2 MFLOP k-block, 930 TFLOP/s =
 //                    10.7 TB/s): the pair needs 32 KB for the same work.  Finished tiles leave through shared memory and TMA.
-// The first stages' weight tiles are constant and requested before the grid dependency is waited for.
+// The first stages' weight tiles are constant and requested before the grid dependency is waited for.  Projection weights are
+// kept packed (gemm_tc5_pack): tiles of 128 outputs x 64 inputs as 16 KB runs, k-block after k-block, so that a block's
+// stream of tiles is one stream of consecutive bytes; in the row-major matrix a tile is 128 pieces of 128 bytes that lie
+// 2 K bytes apart.
 #include <cuda.h>
 
 #include <algorithm>
@@ -57,6 +60,7 @@ struct GemmArgs {
     uint32_t m_tiles, n_tiles[2];       // tiles along the rows of A, and along the outputs of each weight
     uint32_t N[2], w_row0[2];           // outputs of each weight; first row of the weight inside its map
     uint32_t units, run;                // tiles x k-blocks, and how many of them a worker takes
+    uint32_t packed;                    // weights in the layout of gemm_tc5_pack
     uint32_t residual;                  // out = T(float(out) + float(T(x))) instead of T(x)
     uint32_t tile_store;                // pairs: outputs leave by TMA
     uint32_t vec_io;                    // outputs start on a 16-byte boundary
@@ -201,7 +205,9 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         if (lane == 0) {
             auto load_w = [&](uint32_t u, int s) {
                 const Tile t = tile_of(a, u / a.kb);
-                tma_load_2d(base + s * STAGE, t.w ? &map_w1 : &map_w0, full(s), int(u % a.kb) * BK, int(a.w_row0[t.w] + t.n * BM));
+                const uint32_t k = u % a.kb;
+                tma_load_2d(base + s * STAGE, t.w ? &map_w1 : &map_w0, full(s), a.packed ? 0 : int(k * BK),
+                            a.packed ? int((t.n * a.kb + k) * BM) : int(a.w_row0[t.w] + t.n * BM));
             };
             auto load_a = [&](uint32_t u, int s) {
                 const Tile t = tile_of(a, u / a.kb);
@@ -358,8 +364,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             const uint32_t leader_full = map_to_rank(full(0), 0);
             auto load_w = [&](uint32_t u, int s) {               // this block's half of the outputs, in boxes of up to 128 weight rows
                 const Tile t = tile_of(a, u / a.kb);
-                tma_load_2d_pair(base + s * STAGE + A_BYTES, t.w ? &map_w1 : &map_w0, leader_full + 8u * s, int(u % a.kb) * BK,
-                                 int(a.w_row0[t.w] + t.n * NT + rank * (NT / 2)));
+                const uint32_t k = u % a.kb, o = t.n * NT + rank * (NT / 2);           // first of this block's outputs
+                tma_load_2d_pair(base + s * STAGE + A_BYTES, t.w ? &map_w1 : &map_w0, leader_full + 8u * s, a.packed ? 0 : int(k * BK),
+                                 a.packed ? int(((o / BM) * a.kb + k) * BM + o % BM) : int(a.w_row0[t.w] + o));
             };
             uint32_t cur_m = ~0u, next_m = ~0u, page[2] = {0, 0}, next_page[2] = {0, 0};
             auto page_of = [&](uint32_t i) { return __ldg(a.table + min(i, (a.M + kPage - 1) / kPage - 1)); };   // past the end: the last page again
@@ -680,6 +687,7 @@ int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t*
     a.residual = g.residual ? 1u : 0u;
     a.tile_store = rows_kernel ? 0u : 1u;
     a.vec_io = 1u;
+    a.packed = g.packed ? 1u : 0u;
     a.partial = ws.partial;
     a.counters = ws.counters;
     alignas(64) CUtensorMap ma, mc[2];
@@ -728,6 +736,32 @@ int gemm_tc5_configure()
 
 // two slots of 128 x 256 floats per block (a worker of a pair launch is two blocks)
 size_t gemm_tc5_partial_bytes(uint32_t blocks) { return size_t(2) * blocks * 128 * 256 * sizeof(float); }
+
+// src [N][K] row-major -> dst [ceil(N / 128)][ceil(K / 64)][128][64], zero-filled: one warp per 128-byte piece row
+static __global__ void __launch_bounds__(256)
+gemm_pack_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, uint32_t N, uint32_t K)
+{
+    const uint32_t kb = (K + BK - 1) / BK, tile = blockIdx.y, k = blockIdx.x;
+    for (uint32_t i = threadIdx.x; i < BM * 8; i += 256) {
+        const uint32_t row = tile * BM + i / 8, col = k * BK + (i % 8) * 8;
+        dst[(size_t(tile) * kb + k) * (BM * 8) + i] = row < N && col < K ? src[(size_t(row) * K + col) / 8] : make_uint4(0, 0, 0, 0);
+    }
+}
+
+size_t gemm_tc5_packed_values(uint64_t N, uint64_t K) { return (N + BM - 1) / BM * BM * ((K + BK - 1) / BK) * BK; }
+
+bool gemm_tc5_packed_maps(GemmWeightMaps* maps, int dtype, const void* packed, uint64_t N, uint64_t K)
+{
+    const uint64_t rows = gemm_tc5_packed_values(N, K) / BK;
+    return make_map(&maps->box128, dtype, packed, rows, BK, BK, 128) && make_map(&maps->box64, dtype, packed, rows, BK, BK, 64);
+}
+
+// K a multiple of 8; both DEVICE
+int launch_gemm_pack(const void* src, void* dst, uint32_t N, uint32_t K, cudaStream_t st)
+{
+    gemm_pack_kernel<<<dim3((K + BK - 1) / BK, (N + BM - 1) / BM), 256, 0, st>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst), N, K);
+    return int(cudaGetLastError());
+}
 
 bool gemm_tc5_weight_maps(GemmWeightMaps* maps, int dtype, const void* W, uint64_t rows, uint64_t K)
 {

@@ -14,8 +14,10 @@ append_kernel(const AppendArgs a, uint32_t* __restrict__ status)
 {
     __shared__ __align__(16) unsigned char smem[kAppendWarps * kAppendRowSmem];
     grid_launch_dependents();
+    AppendRow<T> row;
+    row.prepare(a, 0, blockIdx.x * kAppendWarps + threadIdx.x / 32, status);
     grid_dependency_wait();              // kv_a comes from an earlier kernel of the stream
-    append_row<T>(a, 0, blockIdx.x * kAppendWarps + threadIdx.x / 32, smem + (threadIdx.x / 32) * kAppendRowSmem, status);
+    row.run(a, smem + (threadIdx.x / 32) * kAppendRowSmem);
 }
 
 int launch_append(int dtype, const void* kv_a, void* layer_pool, uint64_t pool_slots, const void* norm_w, const float* cos_sin,
@@ -84,14 +86,13 @@ __device__ __forceinline__ void mma16816<__nv_bfloat16>(float (&c)[4], const uin
 // The merged, still un-normalised state of every (row, head) written out (the per-GPU partial of a KV-range-sharded
 // sequence): one block per (head, row); the 16 warps take a slice of the row's parts each (a lane owns dims
 // 64*k + 2*lane (+1), k = 0..7, so a warp load covers whole lines of a record), their sums meet in shared memory and
-// warp 0 folds them.  One sequence cut into 74 segments costs two round trips to memory.
+// every thread folds one dim.  One sequence cut into 74 segments costs two round trips to memory.
 __global__ void __launch_bounds__(512)
 export_partial_kernel(const float* __restrict__ recs, const RowParts* __restrict__ parts, uint32_t rec_stride,
                       float* __restrict__ exported, uint32_t H)
 {
-    __shared__ float scratch[16][32][18];
+    __shared__ __align__(8) float scratch[16][kRank], ml_s[16][2];
     grid_launch_dependents();
-    grid_dependency_wait();
     const uint32_t h = blockIdx.x, r = blockIdx.y, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const RowParts rp = parts[r];
     uint32_t pb = rp.begin, pe = rp.end;
@@ -102,6 +103,7 @@ export_partial_kernel(const float* __restrict__ recs, const RowParts* __restrict
     float M = -INFINITY, L = 0.0f, acc[16];
 #pragma unroll
     for (int k = 0; k < 16; k++) acc[k] = 0.0f;
+    grid_dependency_wait();              // the states belong to the attention kernel; the plan was there before
     for (uint32_t p = pb; p < pe; p += 4) {
         float2 ml[4], v[4][8];
 #pragma unroll
@@ -132,31 +134,24 @@ export_partial_kernel(const float* __restrict__ recs, const RowParts* __restrict
             M = Mn;
         }
     }
-    float* mine = scratch[warp][lane];
-    mine[0] = M;
-    mine[1] = L;
+    // thread t folds dim t over the sixteen slices
 #pragma unroll
-    for (int k = 0; k < 16; k++) mine[2 + k] = acc[k];
+    for (int k = 0; k < 8; k++) *reinterpret_cast<float2*>(scratch[warp] + 64 * k + 2 * lane) = make_float2(acc[2 * k], acc[2 * k + 1]);
+    if (lane == 0) { ml_s[warp][0] = M; ml_s[warp][1] = L; }
     __syncthreads();
-    if (warp != 0) return;
-    M = -INFINITY;
-    L = 0.0f;
+    float big = -INFINITY;
 #pragma unroll
-    for (int k = 0; k < 16; k++) acc[k] = 0.0f;
+    for (int j = 0; j < 16; j++) big = fmaxf(big, ml_s[j][0]);
+    float sum = 0.0f, lsum = 0.0f;
+#pragma unroll
     for (int j = 0; j < 16; j++) {
-        const float* o = scratch[j][lane];
-        const float Mj = o[0];
-        if (Mj == -INFINITY) continue;
-        const float Mn = fmaxf(M, Mj), sc = exp2f(M - Mn), w = exp2f(Mj - Mn);
-        L = fmaf(w, o[1], L * sc);
-#pragma unroll
-        for (int k = 0; k < 16; k++) acc[k] = fmaf(w, o[2 + k], acc[k] * sc);
-        M = Mn;
+        const float w = big == -INFINITY ? 0.0f : exp2f(ml_s[j][0] - big);
+        sum = fmaf(w, scratch[j][threadIdx.x], sum);
+        lsum = fmaf(w, ml_s[j][1], lsum);
     }
     float* ex = exported + (size_t(r) * H + h) * kPart;
-    if (lane == 0) { ex[0] = M; ex[1] = L; }
-#pragma unroll
-    for (int k = 0; k < 8; k++) *reinterpret_cast<float2*>(ex + 2 + 64 * k + 2 * lane) = make_float2(acc[2 * k], acc[2 * k + 1]);
+    ex[2 + threadIdx.x] = sum;
+    if (threadIdx.x == 0) { ex[0] = big; ex[1] = lsum; }
 }
 
 // Same merge, projection on the warp-level tensor path.  Block = (head, group of up to 4 row tiles

@@ -58,25 +58,25 @@ void launch_merge(int dtype, const float* recs, const StepMeta& m, const void* w
 int launch_export_partial(const float* recs, const StepMeta& m, float* exported, uint32_t H, cudaStream_t st);
 int merge_mma_configure();
 
-// Absorb on tcgen05 (one block per layer, head and 64 rows); w_map: host CUtensorMap over W_UK^T of all layers,
-// [layers*H*512 d][128 i], box 64 i x 256 d, 128-byte swizzle.  With kv_a != nullptr the same launch appends the step's
+// Absorb on tcgen05; w_map: host CUtensorMap over W_UK^T of all layers,
+// [layers*H*512 d][128 i], box 64 i x 128 d, 128-byte swizzle.  With kv_a != nullptr the same launch appends the step's
 // new rows (launch_append's arguments) in extra blocks.  rotate_q: q arrives before its RoPE; the kernel rotates
 // the last 64 dims of every head with the row's position (m.row_pos) and the cos/sin table.  append_waits: kv_a may
 // have been written by the kernel launched just before this one (the append blocks then wait for it before reading).
 int launch_absorb_tc5(int dtype, const void* q, const void* w_map, void* q_abs, uint32_t H, uint32_t layer0, const void* kv_a,
                       void* layer_pool, uint64_t pool_slots, const void* norm_w, const float* cos_sin, uint32_t cs_rows,
-                      float eps, const StepMeta& m, bool rotate_q, bool append_waits, uint32_t* status, cudaStream_t st);
+                      float eps, const StepMeta& m, bool rotate_q, bool append_waits, uint32_t sm_count, uint32_t* status, cudaStream_t st);
 int absorb_tc5_configure();
 
-// The same merge + projection on tcgen05 (one block per layer, head and 64 or 16 rows); w_map: host CUtensorMap over W_UV of
+// The same merge + projection on tcgen05; w_map: host CUtensorMap over W_UV of
 // all layers, [layers*H*128 outputs][512 dims], box 64 dims x 128 outputs, 128-byte swizzle.
 int launch_merge_tc5(int dtype, const float* recs, const StepMeta& m, uint32_t n_parts, const void* w_map, void* out, uint32_t H,
-                     uint32_t layer0, uint32_t* status, cudaStream_t st);
+                     uint32_t layer0, uint32_t sm_count, uint32_t* status, cudaStream_t st);
 int merge_tc5_configure();
 
 // Dense projections C = A . W^T on tcgen05 (mla_gemm_tc5.cu), up to two weights over the same activations in one launch.
 struct alignas(64) GemmWeightMaps {
-    CUtensorMap box128, box64;     // W [rows][K] in boxes of 64 values x 128 / 64 rows
+    CUtensorMap box128, box64;     // W [rows][K] (or its packed form) in boxes of 64 values x 128 / 64 rows
 };
 struct GemmWeight {
     const CUtensorMap *map, *map64;
@@ -91,6 +91,7 @@ struct GemmCall {
     uint32_t M = 0, K = 0;
     int n_weights = 0;
     GemmWeight w[2];
+    bool packed = false;                       // weights in the layout of launch_gemm_pack (row0 = 0)
     bool residual = false;                     // out = T(float(out) + float(T(x)))
 };
 struct GemmWorkspace {
@@ -100,6 +101,10 @@ struct GemmWorkspace {
 };
 int launch_gemm_tc5(int dtype, const GemmCall& g, const GemmWorkspace& ws, uint32_t* status, cudaStream_t st);
 size_t gemm_tc5_partial_bytes(uint32_t blocks);
+// Projection weights repacked into tiles (see the kernel file): values of the packed form, the packing itself, its maps.
+size_t gemm_tc5_packed_values(uint64_t N, uint64_t K);
+int launch_gemm_pack(const void* src, void* dst, uint32_t N, uint32_t K, cudaStream_t st);
+bool gemm_tc5_packed_maps(GemmWeightMaps* maps, int dtype, const void* packed, uint64_t N, uint64_t K);
 bool gemm_tc5_weight_maps(GemmWeightMaps* maps, int dtype, const void* W, uint64_t rows, uint64_t K);
 int launch_rmsnorm_rows(int dtype, const void* x, const void* w, void* y, uint32_t rows, uint32_t N, float eps, cudaStream_t st);
 int gemm_tc5_configure();
