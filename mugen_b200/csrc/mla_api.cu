@@ -179,7 +179,7 @@ constexpr uint32_t kPrefillMin = 64;
 // Most query rows and bytes of absorbed queries of a group of layers (step_layers_grouped).
 constexpr uint64_t kGroupRows = 1024, kGroupBytes = 48ull << 20;
 // Expanded keys and values of the chunks that share a launch (a chunk that needs more has one of its own).
-constexpr uint64_t kExpandBytes = 1ull << 30;
+constexpr uint64_t kExpandBytes = 256ull << 20;
 
 inline float half_bits_to_f32(uint16_t h) { return __half2float(__ushort_as_half(h)); }
 inline uint16_t f32_to_half_bits(float f) { return __half_as_ushort(__float2half_rn(f)); }

@@ -10,27 +10,30 @@
 // over 192-dim keys and 128-dim values: 2 x (192 + 128) flops per (query, key, head) pair instead of the absorbed
 // form's 2 x (576 + 512), and each staged key/value tile serves 128 query tokens instead of one.
 //
-// One block per (tile of 128 query tokens, head); the whole tile state lives in tensor memory:
-//   Q        [128 queries][192 dims] written once into tensor memory by the softmax threads (row = lane, two dims per
-//            column) and used as the A operand of every score MMA: no shared-memory reads for it
+// One block per (tile of 128 query tokens, head); scores, probabilities and the output accumulate in tensor memory:
+//   Q        [128 queries][192 dims] rotated and written once into shared memory by the softmax threads
 //   TMA      per step of KT = 128 keys K [128][192] (two boxes of expanded nope dims + the rope dims straight from the two
-//            cache pages) and V [128][128], rings of two each; a K buffer is free as soon as the score MMAs
-//            that read it complete, a V buffer one softmax later
-//   QK       S[128 queries x 128 keys] = Q . K^T         12 x tcgen05.mma M128 N128 K16 (A in tensor memory), two score
-//            tiles in flight (steps of 64 keys with rings of four and three score tiles measure 13 % slower: the fixed
-//            cost of a step - waits, the exchange of the maxima, the hand-over to the PV issuer - is paid per step)
-//   softmax  NS = 2 threads per query row, 64 keys each (the parts of a row exchange their maxima through shared memory;
-//            1, 2 and 4 threads per row measure the same within 2 %, 4 slightly slower): causal mask, log2-domain online
-//            softmax with lazy rescaling (threshold 2^8); P in the storage type goes back into the tensor-memory columns
-//            its scores came from
+//            cache pages) and V [128][128], rings of two each, every ring with a thread of its own (one thread for both starts
+//            K of step t + 1 only after the PV of step t - 2 has freed V's buffer: 2,300 instead of 1,850 cycles per step);
+//            a K buffer is free as soon as the score MMAs that read it complete, a V buffer one softmax later
+//   QK       S[128 queries x 128 keys] = Q . K^T         12 x tcgen05.mma M128 N128 K16, two score tiles in flight; a tile is
+//            free for the step after next as soon as its group has loaded it into registers (P has columns of its own: with Q
+//            in tensor memory there is no room for them, P overwrites its scores and QK of step t + 2 waits for PV of step t)
+//   softmax  two groups of four warps take the key steps in turn (group g: steps g, g + 2, ..), one thread per query row and
+//            all 128 keys of it, so that one group's exponentials run while the other waits for its scores or stores P.
+//            Causal mask, log2-domain online softmax with lazy rescaling (threshold 2^8).  What a step needs from the one
+//            before is the row's reference maximum alone (one float through shared memory, warp to warp); every group sums
+//            its own steps' probabilities and the epilogue adds the two.  P goes back to tensor memory in the storage type
 //   PV       O[128 queries x 128 value dims] += P . V    8 x tcgen05.mma M128 N128 K16, A = P in tensor memory, B = the
 //            staged V tile read MN-major (no transpose)
-//   rescale  a row whose maximum moved rescales its own O row (its own lane) after the previous PV completes; no
-//            block-wide agreement is needed
+//   rescale  a row whose maximum moved rescales its own O row (its own lane) after the previous PV completes; nothing else
+//            waits for that PV, and no block-wide agreement is needed
 //   epilogue O / l -> out[query][head][128], rounded once to the storage type
-// The tensor core reads only K and V from shared memory (6 KB per MMA step would be 2 + 4 KB with Q and P there too).
-// Warps: 0 TMA producer, 1 score-MMA issuer, 2 PV-MMA issuer (two issuers keep the tensor pipe fed while one of them
-// waits), 3.. softmax / correction / epilogue.  All waits are bounded.
+// What bounds it is the softmax: 16,384 exponentials per step take the special-function units 1,200 cycles (measured 9.5
+// cycles per warp instruction), the float and conversion instructions around them about 4.7 issue slots per value, against
+// 1,300 cycles of MMAs.  A quarter of the exponentials therefore run as polynomials on the float pipe (poly_ex2).
+// Warps: 0 K producer, 1 score-MMA issuer, 2 PV-MMA issuer (two issuers keep the tensor pipe fed while one of them
+// waits), 3 V producer, 4.. softmax / correction / epilogue.  All waits are bounded.
 #include <cuda.h>
 
 #include <algorithm>
@@ -44,35 +47,66 @@ namespace {
 
 using namespace tc5;
 
-#ifndef MLA_PREFILL_KT
-#define MLA_PREFILL_KT 128
-#endif
-constexpr int QT = 128, KT = MLA_PREFILL_KT;           // queries per block, keys per step (64 or 128)
-constexpr int K_SUB = KT * 128;                        // [KT keys][64 dims]
-constexpr int K_STAGE = 3 * K_SUB, V_STAGE = 2 * K_SUB;        // K: 192 dims, V: 128 dims of KT keys
-constexpr int K_STAGES = KT == 64 ? 4 : 2, V_STAGES = KT == 64 ? 4 : 2;
-constexpr int OFF_K = 0, OFF_V = OFF_K + K_STAGES * K_STAGE, OFF_MISC = OFF_V + V_STAGES * V_STAGE;
-#ifndef MLA_PREFILL_NS
-#define MLA_PREFILL_NS 2
-#endif
-constexpr int NS = MLA_PREFILL_NS;                     // softmax threads per query row (1, 2 or 4)
-constexpr int KP = KT / NS, QP = kQDim / NS, VP = kVDim / NS;   // keys, query dims, value dims per thread of a row
-// hmax: [2 step parities][NS parts][128 rows]; lsum: [NS parts][128 rows]
-constexpr int M_HMAX = 256, M_LSUM = M_HMAX + 2 * NS * QT * 4, M_TMEM = M_LSUM + NS * QT * 4, M_ABORT = M_TMEM + 4, MISC_BYTES = M_TMEM + 64;
+constexpr int QT = 128, KT = 128;                      // queries per block, keys per step
+constexpr int SUB = KT * 128;                          // [128 queries or keys][64 dims]
+constexpr int Q_BYTES = 3 * SUB;                       // 192 dims
+constexpr int STAGES = 2, K_STAGE = 3 * SUB, V_STAGE = 2 * SUB;        // K: 192 dims, V: 128 dims of KT keys
+constexpr int OFF_Q = 0, OFF_K = OFF_Q + Q_BYTES, OFF_V = OFF_K + STAGES * K_STAGE, OFF_MISC = OFF_V + STAGES * V_STAGE;
+constexpr int QP = kQDim / 2, VP = kVDim / 2;          // query dims, value dims that a thread of a group loads / stores of its row
+// reference maximum of each row after step t: [2 step parities][128 rows]; row sums and maxima of the groups: [2][128] each
+constexpr int M_MREF = 320, M_LSUM = M_MREF + 2 * QT * 4, M_MLAST = M_LSUM + 2 * QT * 4, M_TMEM = M_MLAST + 2 * QT * 4, M_ABORT = M_TMEM + 4,
+              MISC_BYTES = M_TMEM + 64;
 constexpr int SMEM_BYTES = OFF_MISC + MISC_BYTES + 1024;       // + slack for 1 KB alignment
-constexpr int NUM_SOFTMAX = NS * QT;
-constexpr int FIRST_SOFTMAX_WARP = 3;
+constexpr int NUM_SOFTMAX = 2 * QT;
+constexpr int FIRST_SOFTMAX_WARP = 4;
 constexpr int NUM_THREADS = 32 * FIRST_SOFTMAX_WARP + NUM_SOFTMAX;
-// tensor memory columns: Q as 16-bit pairs (96), S_BUFS score tiles (P of a step overwrites the head of each part of its
-// scores), O
-constexpr int S_BUFS = KT == 64 ? 3 : 2;                              // score tiles in flight: QK of step t + 1 never waits for softmax t
-constexpr uint32_t TMEM_COLS = 512, COL_Q = 0, COL_S = 128, COL_O = COL_S + S_BUFS * KT;
+// tensor memory columns: a score tile and a tile of P (16-bit pairs) per softmax group, O
+constexpr int S_BUFS = 2;
+constexpr uint32_t TMEM_COLS = 512, COL_S = 0, COL_P = COL_S + S_BUFS * KT, COL_O = COL_P + S_BUFS * KT / 2;
 static_assert(COL_O + kVDim <= TMEM_COLS, "tensor memory columns");
 constexpr float RESCALE_THRESHOLD = 8.0f;
-enum { B_QFULL = 0, B_KFULL, B_KEMPTY = B_KFULL + K_STAGES, B_VFULL = B_KEMPTY + K_STAGES, B_VEMPTY = B_VFULL + V_STAGES,
-       B_SFULL = B_VEMPTY + V_STAGES, B_PFULL = B_SFULL + S_BUFS, B_PVDONE, B_OFULL = B_PVDONE + S_BUFS, B_COUNT };
-static_assert(B_COUNT * 8 <= M_HMAX && B_COUNT <= 32, "barriers overflow their area");
+enum { B_QFULL = 0, B_KFULL, B_KEMPTY = B_KFULL + STAGES, B_VFULL = B_KEMPTY + STAGES, B_VEMPTY = B_VFULL + STAGES,
+       B_SFULL = B_VEMPTY + STAGES, B_SEMPTY = B_SFULL + S_BUFS, B_PFULL = B_SEMPTY + S_BUFS, B_PVDONE = B_PFULL + S_BUFS,
+       B_OFULL = B_PVDONE + S_BUFS, B_MREF, B_COUNT = B_MREF + 8 };       // B_MREF: [2 step parities][4 warps of a group]
+static_assert(B_COUNT * 8 <= M_MREF && B_COUNT <= 32, "barriers overflow their area");
 static_assert(SMEM_BYTES <= 232448, "over the shared memory of one block");
+
+// Two floats at a time (sm_100 has packed f32 arithmetic; every half rounds as the scalar instruction does)
+struct F2 {
+    uint64_t v;
+    __device__ __forceinline__ F2(float lo, float hi) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi)); }
+    __device__ __forceinline__ void get(float& lo, float& hi) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+};
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(a.v) : "l"(b.v), "l"(c.v)); return a; }
+__device__ __forceinline__ F2 fma2_ftz(F2 a, F2 b, F2 c) { asm("fma.rn.ftz.f32x2 %0, %0, %1, %2;" : "+l"(a.v) : "l"(b.v), "l"(c.v)); return a; }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a.v) : "l"(b.v)); return a; }
+__device__ __forceinline__ float max_nan(float a, float b) { float r; asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b)); return r; }
+
+// 2^x without the special-function unit: x = n + f with n the nearest integer (adding 1.5 * 2^23 leaves n in the low bits),
+// 2^f on [-0.5, 0.5] by a polynomial of degree 6 (weighted least squares brought to equal relative error: 1.9e-9, evaluated
+// in float 7.9e-8), n added to its exponent.  x is clamped where the result leaves the normal range below; the last
+// operation flushes what is below it to zero and carries a NaN on, as the unit's instruction does.  x must not exceed 127.
+__device__ __forceinline__ void poly_ex2(F2 x, float& y0, float& y1)
+{
+    float a, b;
+    x.get(a, b);
+    const F2 xc(max_nan(a, -126.5f), max_nan(b, -126.5f));
+    const F2 t = add2(xc, F2(12582912.0f, 12582912.0f));
+    const F2 f = add2(xc, fma2(t, F2(-1.0f, -1.0f), F2(12582912.0f, 12582912.0f)));
+    F2 p(1.5345811e-4f, 1.5345811e-4f);
+    p = fma2(p, f, F2(1.33999309e-3f, 1.33999309e-3f));
+    p = fma2(p, f, F2(9.61848907e-3f, 9.61848907e-3f));
+    p = fma2(p, f, F2(5.55032864e-2f, 5.55032864e-2f));
+    p = fma2(p, f, F2(0.240226462f, 0.240226462f));
+    p = fma2(p, f, F2(0.693147182f, 0.693147182f));
+    p = fma2(p, f, F2(1.0f, 1.0f));
+    float t0, t1, p0, p1;
+    t.get(t0, t1);
+    p.get(p0, p1);
+    p0 = __uint_as_float(__float_as_uint(p0) + (__float_as_uint(t0) << 23));
+    p1 = __uint_as_float(__float_as_uint(p1) + (__float_as_uint(t1) << 23));
+    fma2_ftz(xc, F2(0.0f, 0.0f), F2(p0, p1)).get(y0, y1);
+}
 
 template <typename T>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -85,10 +119,11 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
     const uint32_t raw = smem_u32(prefill_smem);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char* sm = prefill_smem + (base - raw);
-    const uint32_t sK = base + OFF_K, sV = base + OFF_V, sBar = base + OFF_MISC;
+    const uint32_t sQ = base + OFF_Q, sK = base + OFF_K, sV = base + OFF_V, sBar = base + OFF_MISC;
     auto bar = [&](int i) { return sBar + 8u * uint32_t(i); };
-    float* hmax_s = reinterpret_cast<float*>(sm + OFF_MISC + M_HMAX);
+    float* mref_s = reinterpret_cast<float*>(sm + OFF_MISC + M_MREF);
     float* lsum_s = reinterpret_cast<float*>(sm + OFF_MISC + M_LSUM);
+    float* mlast_s = reinterpret_cast<float*>(sm + OFF_MISC + M_MLAST);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + OFF_MISC + M_TMEM);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + M_ABORT);
 
@@ -104,10 +139,14 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
     const uint32_t kv_end = min(total, a.pos + QT);                // keys any query of this tile may see
     const uint32_t n_kv = (kv_end + KT - 1) / KT;
 
+    auto arrive = [&](int i) {      // one arrival per warp
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(i));
+    };
     grid_launch_dependents();
     if (warp == 0 && lane < B_COUNT) {
         const int i = int(lane);
-        mbar_init(bar(i), i == B_QFULL || i == B_PFULL ? uint32_t(NUM_SOFTMAX) : 1u);
+        mbar_init(bar(i), i == B_QFULL ? 8u : i >= B_SEMPTY && i < B_PFULL + S_BUFS ? 4u : 1u);
     }
     if (warp == 0) mbar_init_fence();
     if (tid == 0) *abort_flag = 0;
@@ -133,66 +172,69 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
                     if (page[i] >= n_pages) { atomicOr(status, ST_BAD_PAGE); page[i] = 0; }
                     next[i] = __ldg(pg_list + min(t + 1, n_kv - 1) * PG + i);
                 }
-                const int ks = int(t % K_STAGES), vs = int(t % V_STAGES);
-                ok = mbar_wait(bar(B_KEMPTY + ks), ((t / K_STAGES) & 1) ^ 1, abort_flag, status);
+                const int st = int(t % STAGES), row = int(a.row0 + t * KT);
+                ok = mbar_wait(bar(B_KEMPTY + st), ((t / STAGES) & 1) ^ 1, abort_flag, status);
                 if (!ok) break;
-                const uint32_t kd = sK + ks * K_STAGE;
-                mbar_expect_tx(bar(B_KFULL + ks), K_STAGE);
-                const int row = int(a.row0 + t * KT);
-                tma_load_2d(kd, &map_k, bar(B_KFULL + ks), int(h * kNope), row);
-                tma_load_2d(kd + K_SUB, &map_k, bar(B_KFULL + ks), int(h * kNope + 64), row);
+                const uint32_t kd = sK + st * K_STAGE;
+                mbar_expect_tx(bar(B_KFULL + st), K_STAGE);
+                tma_load_2d(kd, &map_k, bar(B_KFULL + st), int(h * kNope), row);
+                tma_load_2d(kd + SUB, &map_k, bar(B_KFULL + st), int(h * kNope + 64), row);
 #pragma unroll
                 for (int i = 0; i < PG; i++)                         // the rope keys of each page
-                    tma_load_3d(kd + 2 * K_SUB + i * kPage * 128, &map_r, bar(B_KFULL + ks), kRank, int(page[i] * kPage), int(layer));
-                ok = mbar_wait(bar(B_VEMPTY + vs), ((t / V_STAGES) & 1) ^ 1, abort_flag, status);
+                    tma_load_3d(kd + 2 * SUB + i * kPage * 128, &map_r, bar(B_KFULL + st), kRank, int(page[i] * kPage), int(layer));
+            }
+        }
+    } else if (warp == 3) {
+        if (lane == 0) {
+            bool ok = true;
+            for (uint32_t t = 0; t < n_kv && ok; t++) {
+                const int st = int(t % STAGES), row = int(a.row0 + t * KT);
+                ok = mbar_wait(bar(B_VEMPTY + st), ((t / STAGES) & 1) ^ 1, abort_flag, status);
                 if (!ok) break;
-                const uint32_t vd = sV + vs * V_STAGE;
-                mbar_expect_tx(bar(B_VFULL + vs), V_STAGE);
-                tma_load_2d(vd, &map_v, bar(B_VFULL + vs), int(h * kVDim), row);
-                tma_load_2d(vd + K_SUB, &map_v, bar(B_VFULL + vs), int(h * kVDim + 64), row);
+                const uint32_t vd = sV + st * V_STAGE;
+                mbar_expect_tx(bar(B_VFULL + st), V_STAGE);
+                tma_load_2d(vd, &map_v, bar(B_VFULL + st), int(h * kVDim), row);
+                tma_load_2d(vd + SUB, &map_v, bar(B_VFULL + st), int(h * kVDim + 64), row);
             }
         }
     } else if (warp == 1) {
-        // ---- score MMAs.  The score buffer of step t held P(t - S_BUFS): wait for the PV MMAs that read it.
-        constexpr uint32_t IDESC_QK = instr_desc(Fmt<T>::v, QT, KT, 0, 0);
-        constexpr uint32_t HI = desc_hi(1024);
+        // ---- score MMAs: a score tile is free again as soon as its group has loaded it into registers
+        constexpr uint32_t IDESC_QK = instr_desc(Fmt<T>::v, QT, KT, 0, 0), HI = desc_hi(1024);
         bool ok = mbar_wait(bar(B_QFULL), 0, abort_flag, status);
         for (uint32_t t = 0; t < n_kv && ok; t++) {
-            const int ks = int(t % K_STAGES), b = int(t % S_BUFS);
-            ok = mbar_wait(bar(B_KFULL + ks), (t / K_STAGES) & 1, abort_flag, status) &&
-                 (t < S_BUFS || mbar_wait(bar(B_PVDONE + b), (t / S_BUFS - 1) & 1, abort_flag, status));
+            const int ks = int(t % STAGES), b = int(t % S_BUFS);
+            ok = mbar_wait(bar(B_KFULL + ks), (t / STAGES) & 1, abort_flag, status) &&
+                 mbar_wait(bar(B_SEMPTY + b), ((t / S_BUFS) & 1) ^ 1, abort_flag, status);
             if (!ok) break;
             tc_fence_after();
             if (elect_one()) {
-                const uint32_t kb = desc_lo(sK + ks * K_STAGE);
+                const uint32_t qa = desc_lo(sQ), kb = desc_lo(sK + ks * K_STAGE);
 #pragma unroll
                 for (int c = 0; c < 3; c++)
 #pragma unroll
                     for (int k = 0; k < 4; k++)
-                        tc_mma_ts(tmem + COL_S + b * KT, tmem + COL_Q + (c * 4 + k) * 8, kb + ((c * K_SUB + k * 32) >> 4), HI,
-                                  IDESC_QK, (c == 0 && k == 0) ? 0u : 1u);
+                        tc_mma(tmem + COL_S + b * KT, qa + ((c * SUB + k * 32) >> 4), HI, kb + ((c * SUB + k * 32) >> 4), HI, IDESC_QK,
+                               (c == 0 && k == 0) ? 0u : 1u);
                 tc_commit(bar(B_SFULL + b));
                 tc_commit(bar(B_KEMPTY + ks));
             }
             __syncwarp();
         }
     } else if (warp == 2) {
-        // ---- O += P(t) . V(t); P(t) sits where the scores of step t were
-        constexpr uint32_t IDESC_PV = instr_desc(Fmt<T>::v, QT, kVDim, 0, 1);
-        constexpr uint32_t HI = desc_hi(1024);
+        // ---- O += P(t) . V(t)
+        constexpr uint32_t IDESC_PV = instr_desc(Fmt<T>::v, QT, kVDim, 0, 1), HI = desc_hi(1024);
         bool ok = true;
         for (uint32_t t = 0; t < n_kv && ok; t++) {
-            const int vs = int(t % V_STAGES);
-            ok = mbar_wait(bar(B_VFULL + vs), (t / V_STAGES) & 1, abort_flag, status) &&
-                 mbar_wait(bar(B_PFULL), t & 1, abort_flag, status);
+            const int vs = int(t % STAGES);
+            ok = mbar_wait(bar(B_VFULL + vs), (t / STAGES) & 1, abort_flag, status) &&
+                 mbar_wait(bar(B_PFULL + t % S_BUFS), (t / S_BUFS) & 1, abort_flag, status);
             if (!ok) break;
             tc_fence_after();
             if (elect_one()) {
-                const uint32_t vb = desc_lo(sV + vs * V_STAGE, K_SUB), pa = tmem + COL_S + (t % S_BUFS) * KT;
+                const uint32_t vb = desc_lo(sV + vs * V_STAGE, SUB), pa = tmem + COL_P + (t % S_BUFS) * (KT / 2);
 #pragma unroll
-                for (int k = 0; k < KT / 16; k++)    // keys 16k..: 8 columns at the head of the score columns of their part
-                    tc_mma_ts(tmem + COL_O, pa + (16 * k / KP) * KP + (16 * k % KP) / 2, vb + ((k * 2048) >> 4), HI, IDESC_PV,
-                              (t == 0 && k == 0) ? 0u : 1u);
+                for (int k = 0; k < KT / 16; k++)    // keys 16k..: 8 columns
+                    tc_mma_ts(tmem + COL_O, pa + 8 * k, vb + ((k * 2048) >> 4), HI, IDESC_PV, (t == 0 && k == 0) ? 0u : 1u);
                 tc_commit(bar(B_VEMPTY + vs));
                 tc_commit(bar(B_PVDONE + (t % S_BUFS)));
                 if (t + 1 == n_kv) tc_commit(bar(B_OFULL));
@@ -200,15 +242,13 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
             __syncwarp();
         }
     } else {
-        // ===== softmax / correction / epilogue: NS threads per query row; the row is this thread's tensor-memory lane =====
-        static_assert(NS == 1 || NS == 2 || NS == 4, "the part sizes below");
+        // ===== softmax / correction / epilogue: the query row is this thread's tensor-memory lane; `part` is its group =====
         const uint32_t q4 = warp % 4, part = (warp - FIRST_SOFTMAX_WARP) / 4, r = q4 * 32 + lane;
         const uint32_t lane_base = (q4 * 32u) << 16;
         const bool live = r < a.n_q;
         const uint32_t my_pos = a.pos + r;                               // last key this query may see
-        {   // this thread's part of the query row: QP dims = QP / 2 columns, in three stores
-            constexpr int W = QP / 6;
-            static_assert(NS == 2, "part 1 holds dims 96..191, all of the rope dims among them");
+        {   // this thread's half of the query row into the operand tiles
+            constexpr int W = QP / 6;            // part 1 holds dims 96..191, all of the rope dims among them
             const uint4* src = reinterpret_cast<const uint4*>(q + (size_t(a.q_row + r) * H + h) * kQDim + part * QP);
             uint32_t w[3][W];
 #pragma unroll
@@ -237,12 +277,17 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
                 }
             }
 #pragma unroll
-            for (int c = 0; c < 3; c++) tc_stn(tmem + lane_base + COL_Q + part * (QP / 2) + c * W, w[c]);
-            tc_wait_st();
-            tc_fence_before();
-            mbar_arrive(bar(B_QFULL));
+            for (int c = 0; c < 3; c++)
+#pragma unroll
+                for (int j = 0; j < W / 4; j++) {
+                    const uint32_t ch = part * (QP / 8) + c * (W / 4) + j;                // 16-byte piece of the row
+                    *reinterpret_cast<uint4*>(sm + OFF_Q + (ch / 8) * SUB + r * 128 + (((ch % 8) ^ (r & 7)) << 4)) =
+                        make_uint4(w[c][4 * j], w[c][4 * j + 1], w[c][4 * j + 2], w[c][4 * j + 3]);
+                }
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            arrive(B_QFULL);
         }
-        float m_run = -INFINITY, l_run = 0.0f;                           // l_run: this part's share of the row sum
+        float m_run = -INFINITY, l_run = 0.0f;       // the row's reference maximum, and the sum of this group's steps relative to it
         bool fail = false;
         auto wait_w = [&](uint32_t b, uint32_t parity) {
             if (!fail) fail = !mbar_wait(b, parity, abort_flag, status);
@@ -258,82 +303,106 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
                 : "=r"(rr) : "r"(uint32_t(pred)), "n"(NUM_SOFTMAX) : "memory");
             return rr != 0;
         };
-        auto group_sync = [&]() { asm volatile("barrier.cta.sync 2, %0;\n" :: "n"(NUM_SOFTMAX) : "memory"); };
-        for (uint32_t t = 0; t < n_kv; t++) {
-            const uint32_t b = t % S_BUFS;
-            const uint32_t s_addr = tmem + lane_base + COL_S + b * KT + part * KP;
-            wait_w(bar(B_SFULL + b), (t / S_BUFS) & 1);
-            uint32_t sv[KP];
-            if (!fail) {
-                tc_fence_after();
-                tc_ldn(s_addr, sv);
-                tc_wait_ld();
-            } else {
+        for (uint32_t t = part; t < n_kv; t += 2) {
+            const uint32_t b = part;                                     // = t % S_BUFS
+            const uint32_t s_addr = tmem + lane_base + COL_S + b * KT, p_addr = tmem + lane_base + COL_P + b * (KT / 2);
+            wait_w(bar(B_SFULL + b), (t / 2) & 1);
+            if (fail) break;
+            tc_fence_after();
+            float sv[KT];
 #pragma unroll
-                for (int i = 0; i < KP; i++) sv[i] = 0u;
-            }
-            const uint32_t k0 = t * KT + part * KP;
-            if (k0 + KP > my_pos + 1 || k0 + KP > total) {               // causal / end mask (only near the diagonal)
+            for (int c = 0; c < KT / 32; c++) tc_ld32(s_addr + 32 * c, reinterpret_cast<uint32_t (&)[32]>(sv[32 * c]));
+            tc_wait_ld();
+            tc_fence_before();
+            arrive(B_SEMPTY + int(b));
+            const uint32_t k0 = t * KT;
+            if (k0 + KT > my_pos + 1 || k0 + KT > total) {               // causal / end mask (only near the diagonal)
+                const uint32_t end = min(my_pos + 1, total);
 #pragma unroll
-                for (int i = 0; i < KP; i++)
-                    if (k0 + uint32_t(i) > my_pos || k0 + uint32_t(i) >= total) sv[i] = __float_as_uint(-INFINITY);
+                for (int i = 0; i < KT; i++) if (k0 + uint32_t(i) >= end) sv[i] = -INFINITY;
             }
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-            for (int i = 0; i < KP; i++) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(sv[i]));
-            float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            // Two buffers by step parity: another part of a row may already be one step ahead when this one reads.
-            if constexpr (NS > 1) {
-                float* hm = hmax_s + (t & 1) * NS * QT;
-                hm[part * QT + r] = mx;
-                group_sync();
+            for (int i = 0; i < KT; i += 8)
 #pragma unroll
-                for (int p = 0; p < NS; p++) mx = fmaxf(mx, hm[p * QT + r]);
+                for (int j = 0; j < 4; j++) mx4[j] = fmaxf(fmaxf(mx4[j], sv[i + j]), sv[i + 4 + j]);
+            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
+            float m_prev = -INFINITY;                                    // the row's reference after step t - 1
+            if (t > 0) {
+                wait_w(bar(B_MREF + ((t - 1) & 1) * 4 + q4), ((t - 1) / 2) & 1);
+                if (fail) break;
+                m_prev = mref_s[((t - 1) & 1) * QT + r];
             }
-            mx *= scale_log2;                                            // the same in all parts of a row
-            float alpha = 1.0f;
-            bool need = false;
-            if (m_run == -INFINITY) { m_run = mx; }                     // nothing accumulated for this row yet
-            else if (mx > m_run + RESCALE_THRESHOLD) { alpha = fast_ex2(m_run - mx); m_run = mx; need = true; }
-            float sum2[2] = {0.0f, 0.0f};
-            uint32_t pk[KP / 2];
+            const bool need = m_prev != -INFINITY && mx > m_prev + RESCALE_THRESHOLD;
+            const float m_new = m_prev == -INFINITY || need ? mx : m_prev;
+            // the other group has read what this slot held (it could not have posted step t - 1 otherwise)
+            mref_s[(t & 1) * QT + r] = m_new;
+            arrive(B_MREF + int((t & 1) * 4 + q4));
+            if (m_new != m_run) {                                        // this group's sum follows (-infinity: nothing summed yet)
+                l_run = m_run == -INFINITY ? 0.0f : l_run * fast_ex2(m_run - m_new);
+                m_run = m_new;
+            }
             const float mref = m_run == -INFINITY ? 0.0f : m_run;         // a row whose keys so far are all masked: p = 0
-#pragma unroll
-            for (int i = 0; i < KP; i += 2) {
-                const float p0 = fast_ex2(fmaf(__uint_as_float(sv[i]), scale_log2, -mref));
-                const float p1 = fast_ex2(fmaf(__uint_as_float(sv[i + 1]), scale_log2, -mref));
-                sum2[(i >> 1) & 1] += p0 + p1;
-                pk[i / 2] = Elem<T>::pack2(p0, p1);
+            if (t >= S_BUFS) {                                           // P(t - 2) has been read
+                wait_w(bar(B_PVDONE + b), (t / S_BUFS - 1) & 1);
+                if (fail) break;
+                tc_fence_after();
             }
-            l_run = l_run * alpha + (sum2[0] + sum2[1]);
-            if (t > 0) wait_w(bar(B_PVDONE + ((t - 1) % S_BUFS)), ((t - 1) / S_BUFS) & 1);   // PV of the previous step complete: this row of O is stable
-            if (fail) continue;
-            tc_fence_after();
+            const F2 scale2(scale_log2, scale_log2), mref2(-mref, -mref);
+            F2 sum2[2] = {F2(0.0f, 0.0f), F2(0.0f, 0.0f)};
+#pragma unroll
+            for (int c = 0; c < KT / 32; c++) {
+                uint32_t pk[16];
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const F2 x = fma2(F2(sv[32 * c + 2 * i], sv[32 * c + 2 * i + 1]), scale2, mref2);       // at most the threshold
+                    float p0, p1;
+                    if (i % 4 == 3) {
+                        poly_ex2(x, p0, p1);
+                    } else {
+                        x.get(p0, p1);
+                        p0 = fast_ex2(p0);
+                        p1 = fast_ex2(p1);
+                    }
+                    sum2[i & 1] = add2(sum2[i & 1], F2(p0, p1));
+                    pk[i] = Elem<T>::pack2(p0, p1);
+                }
+                tc_st16(p_addr + 16 * c, pk);
+            }
+            float s0, s1, s2, s3;
+            sum2[0].get(s0, s1);
+            sum2[1].get(s2, s3);
+            l_run += (s0 + s1) + (s2 + s3);
             // tcgen05.ld / .st are warp-wide: the warp rescales when any of its rows needs it (the others multiply by 1)
-            if (t > 0 && __any_sync(0xffffffffu, need)) {    // O[this row][this part's VP value dims] *= alpha
+            if (__any_sync(0xffffffffu, need)) {
+                wait_w(bar(B_PVDONE + ((t - 1) & 1)), ((t - 1) / 2) & 1);        // PV of the previous step complete: this row of O is stable
+                if (fail) break;
+                tc_fence_after();
+                const float alpha = need ? fast_ex2(m_prev - m_new) : 1.0f;
 #pragma unroll 1
-                for (uint32_t c = 0; c < VP / 32; c++) {
+                for (uint32_t c = 0; c < kVDim / 32; c++) {
                     uint32_t o[32];
-                    tc_ld32(tmem + lane_base + COL_O + part * VP + c * 32, o);
+                    tc_ld32(tmem + lane_base + COL_O + c * 32, o);
                     tc_wait_ld();
 #pragma unroll
                     for (int i = 0; i < 32; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                    tc_st32(tmem + lane_base + COL_O + part * VP + c * 32, o);
+                    tc_st32(tmem + lane_base + COL_O + c * 32, o);
                 }
             }
-            tc_stn(s_addr, pk);              // P over the first half of this thread's own score columns
             tc_wait_st();
             tc_fence_before();
-            mbar_arrive(bar(B_PFULL));
+            arrive(B_PFULL + int(b));
         }
         wait_w(bar(B_OFULL), 0);
         lsum_s[part * QT + r] = l_run;
+        mlast_s[part * QT + r] = m_run;
         const bool bad = group_or(fail);
         if (!bad) {
             tc_fence_after();
+            const float ma = mlast_s[r], mb = mlast_s[QT + r], m_end = fmaxf(ma, mb);     // O stands relative to the later one, the larger
             float l = 0.0f;
-#pragma unroll
-            for (int p = 0; p < NS; p++) l += lsum_s[p * QT + r];
+            if (ma != -INFINITY) l += lsum_s[r] * fast_ex2(ma - m_end);
+            if (mb != -INFINITY) l += lsum_s[QT + r] * fast_ex2(mb - m_end);
             const float linv = l > 0.0f ? 1.0f / l : 0.0f;
             uint4* dst = reinterpret_cast<uint4*>(out + (size_t(a.q_row + r) * H + h) * kVDim + part * VP);
 #pragma unroll 1

@@ -467,6 +467,47 @@ def test_prefill_chunks_take_the_expanded_path(torch, oracle, H, dt, spec, q_rop
     ctx.close()
 
 
+@pytest.mark.parametrize("start,n_new", [(0, 64), (1, 127), (0, 129), (120, 137), (300, 212), (0, 1025)])
+def test_prefill_maxima_that_move_at_every_step(torch, start, n_new):
+    """1 to 9 steps of 128 keys whose rows grow along the sequence, so that the maxima move (and the output is rescaled) in
+    steps of both softmax groups, with the sums spread over them; sharp queries, so that most exponents lie far below zero.
+    Against float64 from the rows the cache holds.  Expanded keys are rounded to fp16 (2^-12 of each value): scores of
+    standard deviation ~8 carry an error of ~1e-3, within the usual 5e-3 / 2e-2."""
+    H, dt = 8, synth.DT_F16
+    total = start + n_new
+    case = synth.make_layer_case(5100 + n_new, H, [total], dt)
+    from mugen_b200.mla import MlaContext
+    ctx = MlaContext(n_layers=1, n_heads=H, dtype=dt, n_pages=total // 64 + 3, max_seqs=1, max_seq_len=total + 64, max_rows=n_new, **YARN)
+    ctx.shuffle_free_pages(2)
+    ctx.set_layer_weights(0, case.w_uk, case.w_uv, case.w_type, case.norm_w)
+    s = ctx.seq_create()
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n_new)
+    grow = torch.linspace(0.5, 2.0, total, device="cuda")[:, None]
+    rows = (torch.randn((total, 576), device="cuda", generator=gen) * grow).half()
+    if start:
+        ctx.write_rows(0, s, 0, rows[:start].view(torch.int16))
+        ctx.advance_seq_len(s, start)
+    kv = rows[start:].contiguous()
+    kv[:, 512:] *= 4                                       # the append normalises the latent part: the rope part keeps growing
+    q = (torch.randn((n_new, H, 192), device="cuda", generator=gen) * 3).half()
+    out = torch.zeros((n_new, H, 128), dtype=torch.float16, device="cuda")
+    ctx.step_begin([s], [n_new])
+    ctx.step_layers(0, 1, kv[None], q[None], out[None])
+    ctx.step_end()
+    assert ctx.status() == 0
+    held = torch.from_numpy(ctx.read_rows(0, s, 0, total).view(np.int16)).cuda().view(torch.float16).double()
+    uk, uv = (torch.from_numpy(w.view(np.int16)).cuda().view(torch.float16).double().view(H, 128, 512) for w in (case.w_uk, case.w_uv))
+    qd = q.double()
+    sc = torch.einsum("nhi,hid,td->hnt", qd[..., :128], uk, held[:, :512]) + torch.einsum("nhi,ti->hnt", qd[..., 128:], held[:, 512:])
+    pos = torch.arange(total, device="cuda")
+    sc = (sc / 192 ** 0.5).masked_fill(pos[None, None] > pos[None, start:, None], -torch.inf)
+    want = torch.einsum("hnt,td,hid->nhi", torch.softmax(sc, -1), held[:, :512], uv)
+    err = (out.double() - want).abs()
+    assert err.max() <= 2e-2 * max(1.0, want.abs().max().item()) and err.norm() <= 5e-3 * want.norm(), (err.max(), err.norm() / want.norm())
+    ctx.close()
+
+
 @pytest.mark.parametrize("fused", [False, True])
 @pytest.mark.parametrize("kernel", KERNELS)
 def test_kv_range_shards_merge(torch, oracle, kernel, fused):
