@@ -31,7 +31,9 @@
 //   epilogue O / l -> out[query][head][128], rounded once to the storage type
 // What bounds it is the softmax: 16,384 exponentials per step take the special-function units 1,200 cycles (measured 9.5
 // cycles per warp instruction), the float and conversion instructions around them about 4.7 issue slots per value, against
-// 1,300 cycles of MMAs.  A quarter of the exponentials therefore run as polynomials on the float pipe (poly_ex2).
+// 1,300 cycles of MMAs; a step takes 1,800.  (An eighth or a quarter of the exponentials as polynomials on the float pipe is
+// 5 % slower; a pair of blocks sharing K and V by cta_group::2 halves the L2 feed and is 15 % slower, its barriers are a
+// cluster hop away.)  128 heads, chunks of 4096 tokens at 8192: 3.47 -> 3.05 ms, 990 -> 1,130 TFLOP/s.
 // Warps: 0 K producer, 1 score-MMA issuer, 2 PV-MMA issuer (two issuers keep the tensor pipe fed while one of them
 // waits), 3 V producer, 4.. softmax / correction / epilogue.  All waits are bounded.
 #include <cuda.h>
@@ -78,35 +80,7 @@ struct F2 {
     __device__ __forceinline__ void get(float& lo, float& hi) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
 };
 __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(a.v) : "l"(b.v), "l"(c.v)); return a; }
-__device__ __forceinline__ F2 fma2_ftz(F2 a, F2 b, F2 c) { asm("fma.rn.ftz.f32x2 %0, %0, %1, %2;" : "+l"(a.v) : "l"(b.v), "l"(c.v)); return a; }
 __device__ __forceinline__ F2 add2(F2 a, F2 b) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a.v) : "l"(b.v)); return a; }
-__device__ __forceinline__ float max_nan(float a, float b) { float r; asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b)); return r; }
-
-// 2^x without the special-function unit: x = n + f with n the nearest integer (adding 1.5 * 2^23 leaves n in the low bits),
-// 2^f on [-0.5, 0.5] by a polynomial of degree 6 (weighted least squares brought to equal relative error: 1.9e-9, evaluated
-// in float 7.9e-8), n added to its exponent.  x is clamped where the result leaves the normal range below; the last
-// operation flushes what is below it to zero and carries a NaN on, as the unit's instruction does.  x must not exceed 127.
-__device__ __forceinline__ void poly_ex2(F2 x, float& y0, float& y1)
-{
-    float a, b;
-    x.get(a, b);
-    const F2 xc(max_nan(a, -126.5f), max_nan(b, -126.5f));
-    const F2 t = add2(xc, F2(12582912.0f, 12582912.0f));
-    const F2 f = add2(xc, fma2(t, F2(-1.0f, -1.0f), F2(12582912.0f, 12582912.0f)));
-    F2 p(1.5345811e-4f, 1.5345811e-4f);
-    p = fma2(p, f, F2(1.33999309e-3f, 1.33999309e-3f));
-    p = fma2(p, f, F2(9.61848907e-3f, 9.61848907e-3f));
-    p = fma2(p, f, F2(5.55032864e-2f, 5.55032864e-2f));
-    p = fma2(p, f, F2(0.240226462f, 0.240226462f));
-    p = fma2(p, f, F2(0.693147182f, 0.693147182f));
-    p = fma2(p, f, F2(1.0f, 1.0f));
-    float t0, t1, p0, p1;
-    t.get(t0, t1);
-    p.get(p0, p1);
-    p0 = __uint_as_float(__float_as_uint(p0) + (__float_as_uint(t0) << 23));
-    p1 = __uint_as_float(__float_as_uint(p1) + (__float_as_uint(t1) << 23));
-    fma2_ftz(xc, F2(0.0f, 0.0f), F2(p0, p1)).get(y0, y1);
-}
 
 template <typename T>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -355,15 +329,11 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
                 uint32_t pk[16];
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
-                    const F2 x = fma2(F2(sv[32 * c + 2 * i], sv[32 * c + 2 * i + 1]), scale2, mref2);       // at most the threshold
+                    const F2 x = fma2(F2(sv[32 * c + 2 * i], sv[32 * c + 2 * i + 1]), scale2, mref2);
                     float p0, p1;
-                    if (i % 4 == 3) {
-                        poly_ex2(x, p0, p1);
-                    } else {
-                        x.get(p0, p1);
-                        p0 = fast_ex2(p0);
-                        p1 = fast_ex2(p1);
-                    }
+                    x.get(p0, p1);
+                    p0 = fast_ex2(p0);
+                    p1 = fast_ex2(p1);
                     sum2[i & 1] = add2(sum2[i & 1], F2(p0, p1));
                     pk[i] = Elem<T>::pack2(p0, p1);
                 }
