@@ -552,9 +552,9 @@ int run_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, float* expo
         e = mla::launch_decode_tc5_pair128(dt, c->tmaps, c->pool, layer, c->cfg.n_pages, m, c->recs, H, p.max_pages <= 64 ? 1u : 0u,
                                            next_w, next_w ? uint32_t(weight_bytes(c)) : 0u, c->status_dev, st);
     else if (p.kernel == MLA_KERNEL_TCGEN05)
-        e = mla::launch_decode_tc5(dt, c->tmaps, layer, c->cfg.n_pages, m, c->recs, H, c->status_dev, st);
+        e = mla::launch_decode_tc5(dt, c->tmaps, c->pool, layer, c->cfg.n_pages, m, c->recs, H, c->status_dev, st);
     else if (p.kernel == MLA_KERNEL_TCGEN05_T16)
-        e = mla::launch_decode_tc5_t16(dt, c->tmaps, layer, c->cfg.n_pages, m, c->recs, H, c->status_dev, st);
+        e = mla::launch_decode_tc5_t16(dt, c->tmaps, c->pool, layer, c->cfg.n_pages, m, c->recs, H, c->status_dev, st);
     else
         e = mla::launch_decode_mma(dt, c->q_abs, layer_pool(c, layer), c->cfg.n_pages, m, c->recs, H, c->status_dev, st);
     if (e != 0) return fail(c, MLA_ERR_CUDA, std::string("attention launch: ") + cudaGetErrorString(cudaError_t(e)));

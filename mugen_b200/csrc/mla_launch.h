@@ -23,14 +23,14 @@ int decode_mma_configure();   // the *_configure() functions set kernel attribut
 
 // Split-KV attention on the 5th-generation tensor cores (tcgen05.mma, accumulators in TMEM,
 // cache tiles staged by TMA): grid (persistent blocks, ceil(H/64)).  tmaps points at the context's
-// host CUtensorMap array (kMap* below); this kernel uses kMapPoolPage and kMapQueries.
-int launch_decode_tc5(int dtype, const void* tmaps, uint32_t layer0, uint32_t n_pages, const StepMeta& m,
+// host CUtensorMap array (kMap* below), pool at the whole cache pool; this kernel uses kMapPoolPage and kMapQueries.
+int launch_decode_tc5(int dtype, const void* tmaps, const void* pool, uint32_t layer0, uint32_t n_pages, const StepMeta& m,
                       float* recs, uint32_t H, uint32_t* status, cudaStream_t st);
 int decode_tc5_configure();   // sets the kernel's attributes on the current device
 
 // The transposed form for narrow head counts (mla_decode_tc5_t16.cu): tokens are the M rows, groups of 16 heads the N
 // columns; grid (persistent blocks, ceil(H/16)).  Uses kMapPoolV, kMapPoolSub and kMapQueries16.
-int launch_decode_tc5_t16(int dtype, const void* tmaps, uint32_t layer0, uint32_t n_pages, const StepMeta& m, float* recs,
+int launch_decode_tc5_t16(int dtype, const void* tmaps, const void* pool, uint32_t layer0, uint32_t n_pages, const StepMeta& m, float* recs,
                           uint32_t H, uint32_t* status, cudaStream_t st);
 int decode_tc5_t16_configure();
 

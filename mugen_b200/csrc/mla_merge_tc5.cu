@@ -11,8 +11,8 @@
 // (together ~16 mantissa bits for bf16, ~22 for fp16, so the float state is not rounded to the storage type before the
 // projection), two buffers in turn: sixteen warps reduce the next tile's partial states while the tensor core works on
 // this one's.
-// Reduction: G = 8, 4, 2 or 1 warps per row for steps of up to 2, 4, 8 or more rows, each with its share of the 512 dims, so
-// that 16 loads of 8 bytes are in flight per lane whatever the mix of rows and parts; weights come from one pass over
+// Reduction: G = 16, 8, 4, 2 or 1 warps per row for steps of up to 1, 2, 4, 8 or more rows, each with its share of the 512 dims,
+// so that 128 bytes of loads are in flight per lane whatever the mix of rows and parts; weights come from one pass over
 // (m, l), 32 parts at a time, and no exchange between warps is needed.
 // (One block per head and 16 or 64 rows with load, reduction and MMAs in sequence: 27 layers x 16 heads x 1 row took 24 us
 // for 57 MB.)
@@ -49,11 +49,11 @@ struct MergeArgs {
     const uint32_t* att_row;
 };
 
-// One row's merged state by one warp: dims dim0 + 64*k + 2*lane (+1), k < DL/2.  acc comes back normalised.
+// One row's merged state by one warp: dims dim0 + 64*k + 2*lane (+1), k < DL/2 (DL = 1: dim0 + lane).  acc comes back normalised.
 template <int DL>
 __device__ __forceinline__ void reduce_row(const MergeArgs& a, const RowParts& rp, uint32_t h, uint32_t dim0, uint32_t lane, float (&acc)[DL])
 {
-    constexpr int Q = DL / 2, PB = 16 / Q;                     // loads per part, parts per batch: 16 loads in flight
+    constexpr int W = DL == 1 ? 1 : 2, Q = DL / W, PB = 32 / DL;      // floats per load, loads per part, parts per batch
     float M = -INFINITY, L = 0.0f;
 #pragma unroll
     for (int k = 0; k < DL; k++) acc[k] = 0.0f;
@@ -62,14 +62,23 @@ __device__ __forceinline__ void reduce_row(const MergeArgs& a, const RowParts& r
     for (uint32_t c0 = rp.begin; c0 < rp.end; c0 += 32) {
         const uint32_t n = min(32u, rp.end - c0);
         const float* rec = rec0 + size_t(c0) * stride;
-        const float* src = rec + 2 + dim0 + 2 * lane;
-        float2 v[PB][Q];
+        const float* src = rec + 2 + dim0 + W * lane;
+        float v[PB][Q][W];
         auto load = [&](uint32_t p0) {
 #pragma unroll
             for (int i = 0; i < PB; i++)
 #pragma unroll
                 for (int k = 0; k < Q; k++)
-                    if (p0 + i < n) v[i][k] = *reinterpret_cast<const float2*>(src + (p0 + i) * stride + 64 * k);
+                    if (p0 + i < n) {
+                        const float* at = src + (p0 + i) * stride + 64 * k;
+                        if constexpr (W == 1) {
+                            v[i][k][0] = *at;
+                        } else {
+                            const float2 f = *reinterpret_cast<const float2*>(at);
+                            v[i][k][0] = f.x;
+                            v[i][k][1] = f.y;
+                        }
+                    }
         };
         float2 ml = lane < n ? *reinterpret_cast<const float2*>(rec + lane * stride) : make_float2(-INFINITY, 0.0f);
         load(0);
@@ -93,10 +102,7 @@ __device__ __forceinline__ void reduce_row(const MergeArgs& a, const RowParts& r
                 const float wi = __shfl_sync(0xffffffffu, w, int((p0 + i) & 31));
                 if (p0 + i >= n) continue;
 #pragma unroll
-                for (int k = 0; k < Q; k++) {
-                    acc[2 * k] = fmaf(wi, v[i][k].x, acc[2 * k]);
-                    acc[2 * k + 1] = fmaf(wi, v[i][k].y, acc[2 * k + 1]);
-                }
+                for (int k = 0; k < DL; k++) acc[k] = fmaf(wi, v[i][k / W][k % W], acc[k]);
             }
         }
     }
@@ -253,6 +259,12 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
                 if (rr < live) reduce_row<16 / G>(a, rp, x.h, dim0, lane, acc);
                 ok = ok && mbar_wait(a_empty(b), ((n >> 1) & 1) ^ 1, abort_flag, status);      // the MMAs of two tiles ago have read this buffer
                 if (rr < live) {
+                    if constexpr (G == 16) {                       // row 0 (of one): 32 dims, half a row of a sub-tile
+                        unsigned char* p = hi + (dim0 / 64) * A_SUB + (dim0 % 64 + lane) * 2;
+                        const T h0 = Elem<T>::from_f32(acc[0]);
+                        *reinterpret_cast<T*>(p) = h0;
+                        *reinterpret_cast<T*>(p + A_HALF) = Elem<T>::from_f32(acc[0] - Elem<T>::to_f32(h0));
+                    }
                     const uint32_t so = rr * 128 + (((lane / 4) ^ (rr & 7)) << 4) + (lane % 4) * 4;
 #pragma unroll
                     for (int k = 0; k < 8 / G; k++) {
@@ -290,10 +302,12 @@ int merge_tc5_configure()
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__half, 2>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__half, 4>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__half, 8>);
+    if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__half, 16>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__nv_bfloat16, 1>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__nv_bfloat16, 2>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__nv_bfloat16, 4>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__nv_bfloat16, 8>);
+    if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__nv_bfloat16, 16>);
     return int(e);
 }
 
@@ -314,11 +328,11 @@ int launch_merge_tc5(int dtype, const float* recs, const StepMeta& m, uint32_t n
     a.run = (a.units + sm_count - 1) / sm_count;
     dim3 grid((a.units + a.run - 1) / a.run);
     auto go = [&](auto kernel, auto* o) { return int(launch_pdl(kernel, grid, dim3(NUM_THREADS), SMEM_BYTES, st, *map, o, a, status)); };
-    auto pick = [&](auto k1, auto k2, auto k4, auto k8, auto* o) { return m.rows <= 2 ? go(k8, o) : m.rows <= 4 ? go(k4, o) : m.rows <= 8 ? go(k2, o) : go(k1, o); };
+    auto pick = [&](auto k1, auto k2, auto k4, auto k8, auto k16, auto* o) { return m.rows <= 1 ? go(k16, o) : m.rows <= 2 ? go(k8, o) : m.rows <= 4 ? go(k4, o) : m.rows <= 8 ? go(k2, o) : go(k1, o); };
     return dtype == 0 ? pick(merge_outproj_tc5_kernel<__half, 1>, merge_outproj_tc5_kernel<__half, 2>, merge_outproj_tc5_kernel<__half, 4>,
-                             merge_outproj_tc5_kernel<__half, 8>, static_cast<__half*>(out))
+                             merge_outproj_tc5_kernel<__half, 8>, merge_outproj_tc5_kernel<__half, 16>, static_cast<__half*>(out))
                       : pick(merge_outproj_tc5_kernel<__nv_bfloat16, 1>, merge_outproj_tc5_kernel<__nv_bfloat16, 2>, merge_outproj_tc5_kernel<__nv_bfloat16, 4>,
-                             merge_outproj_tc5_kernel<__nv_bfloat16, 8>, static_cast<__nv_bfloat16*>(out));
+                             merge_outproj_tc5_kernel<__nv_bfloat16, 8>, merge_outproj_tc5_kernel<__nv_bfloat16, 16>, static_cast<__nv_bfloat16*>(out));
 }
 
 }  // namespace mla

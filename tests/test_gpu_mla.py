@@ -796,3 +796,27 @@ def test_rows_of_one_sequence_share_a_stream(torch, oracle, H, dt, spec):
             check_close(got[r + t], want, dt, f"sequence {i} (start {a}), token {t}")
         r += b
     ctx.close()
+
+
+@pytest.mark.parametrize("H,dt,lens", [
+    (5, synth.DT_F16, [6000]),                             # one row in 94 parts: sixteen warps share its dims
+    (32, synth.DT_BF16, [2100]),
+    (70, synth.DT_F16, [65]),                              # few parts
+    (16, synth.DT_BF16, [4100, 40]),                       # two rows: eight warps each
+])
+def test_merge_of_few_rows_in_many_parts(torch, oracle, H, dt, lens):
+    """The merge's warps per row for the smallest steps (mla_merge_tc5.cu), every head against the CPU."""
+    case = synth.make_layer_case(6100 + H, H, [n + 1 for n in lens], dt)
+    ctx = make_ctx(case, capi.KERNEL_AUTO, shuffle=5, max_rows=len(lens), max_seqs=len(lens))
+    seqs = fill(torch, ctx, case, upto=lens)
+    out = torch.zeros((len(lens), H, 128), dtype=torch.int16, device="cuda")
+    ctx.step_begin(seqs)
+    ctx.step_layers(0, 1, _dev(torch, case.kv_a)[None], _dev(torch, case.q)[None], out[None])
+    ctx.step_end()
+    assert ctx.status() == 0
+    got = _host(out)
+    rows = oracle.append_rows(case.kv_a, lens, case.norm_w, YARN["rms_norm_eps"], 40.0, 4096, 10000.0, dt)
+    for b, n in enumerate(lens):
+        cache = np.concatenate([case.caches[b][:n], rows[b:b + 1]])
+        check_close(got[b], oracle.attention(case.q[b], cache, n + 1, case.w_uk, case.w_uv, case.w_type, H, dt), dt, f"row {b}")
+    ctx.close()
