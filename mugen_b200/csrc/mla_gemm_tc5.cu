@@ -452,6 +452,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             const Tile tl = tile_of(a, tile);
             const uint32_t N = a.N[tl.w], m0 = (2 * tl.m + rank) * BM, m = m0 + r;
             T* out = tl.w ? out1 : out0;
+            // what the outputs are added to is requested two steps of 32 columns ahead, the first two while the tile is
+            // computed: a thread's pieces lie a row apart, and each step would wait for its own round trip to memory (27 blocks
+            // over a prompt of 777 tokens: 2067 -> 2025 us; the same in gemm_rows_kernel, where it is one trip, costs 1.5 %).
+            // A worker of a cut tile asks before it hands its part over, so nobody has stored yet.
+            auto residual = [&](int c, uint4 (&rs)[4]) {
+                const uint32_t n0 = tl.n * NT + c * CH;
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (a.residual && m < a.M && c < NT / CH && n0 + 8 * i < N) rs[i] = load8(out + size_t(m) * N + n0 + 8 * i, a.vec_io);
+            };
+            uint4 rs0[4], rs1[4];
+            residual(0, rs0);
+            residual(1, rs1);
             ok = ok && mbar_wait(acc_full(nt & 1), (nt >> 1) & 1, abort_flag, status);
             ok = __all_sync(0xffffffffu, ok);
             tc_fence_after();
@@ -462,7 +475,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 if (lane == 0) mbar_arrive_cluster(leader_empty + 8u * (nt & 1));
             };
             // columns c*CH.. of the tile, complete: round and store.  All 128 threads pass its barriers.
-            auto finish = [&](int c, const float (&v)[CH]) {
+            auto finish = [&](int c, const float (&v)[CH], uint4 (&rs)[4]) {
                 const uint32_t n0 = tl.n * NT + c * CH;
                 T* p = out + size_t(m) * N + n0;
                 uint32_t pk[16];
@@ -472,8 +485,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
                         if (n0 + 8 * i >= N) break;
-                        const uint4 o4 = load8(p + 8 * i, a.vec_io);
-                        const uint32_t ow[4] = {o4.x, o4.y, o4.z, o4.w};
+                        const uint32_t ow[4] = {rs[i].x, rs[i].y, rs[i].z, rs[i].w};
 #pragma unroll
                         for (int j = 0; j < 4; j++) {
                             const auto* xo = reinterpret_cast<const T*>(&ow[j]);
@@ -482,6 +494,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                         }
                     }
                 }
+                residual(c + 2, rs);
                 if (!a.tile_store) {
                     if (m >= a.M || !ok) return;
 #pragma unroll
@@ -512,18 +525,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             };
             if (!cut) {
 #pragma unroll 1
-                for (int c = 0; c < NT / CH; c++) {
+                for (int c = 0; c < NT / CH; c += 2) {
                     float v[CH];
                     load_acc(acc + c * CH, v);
-                    if (c + 1 == NT / CH) release();
-                    finish(c, v);
+                    finish(c, v, rs0);
+                    load_acc(acc + (c + 1) * CH, v);
+                    if (c + 2 == NT / CH) release();
+                    finish(c + 1, v, rs1);
                 }
             } else if (hand_over<NT, CH>(a, worker, 2, rank, tile, acc, r, ok, last_slot, release)) {
 #pragma unroll 1
-                for (int c = 0; c < NT / CH; c++) {
+                for (int c = 0; c < NT / CH; c += 2) {
                     float v[CH];
                     sum_partials<NT, CH>(a, 2, rank, tile, r, c, v);
-                    finish(c, v);
+                    finish(c, v, rs0);
+                    sum_partials<NT, CH>(a, 2, rank, tile, r, c + 1, v);
+                    finish(c + 1, v, rs1);
                 }
             }
             u = end;
