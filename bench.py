@@ -701,7 +701,7 @@ def sub_prefill(torch, peak):
                                  "chunk_tokens_per_s_61_layers_scaled": R / (ms * 1e-3) / 61,
                                  "tflops_expanded_form": (pairs * H * 2.0 * (192 + 128) + expand) / (ms * 1e-3) / 1e12,
                                  "tflops_if_counted_in_absorbed_form": pairs * H * 2.0 * (576 + 512) / (ms * 1e-3) / 1e12,
-                                 "path": "append + gather + key/value expansion (tcgen05 GEMM) + causal flash attention (tcgen05), per chunk"}
+                                 "path": "append + key/value expansion (tcgen05 GEMM) + causal flash attention (tcgen05), per chunk"}
         ctx.close()
         del q, kv, out
         torch.cuda.empty_cache()
