@@ -33,7 +33,7 @@
 // cycles per warp instruction), the float and conversion instructions around them about 4.7 issue slots per value, against
 // 1,300 cycles of MMAs; a step takes 1,800.  (An eighth or a quarter of the exponentials as polynomials on the float pipe is
 // 5 % slower; a pair of blocks sharing K and V by cta_group::2 halves the L2 feed and is 15 % slower, its barriers are a
-// cluster hop away.)  128 heads, chunks of 4096 tokens at 8192: 3.47 -> 3.05 ms, 990 -> 1,130 TFLOP/s.
+// cluster hop away.)  128 heads, chunks of 4096 tokens at 8192: 3.47 -> 2.83 ms, 990 -> 1,214 TFLOP/s.
 // Warps: 0 K producer, 1 score-MMA issuer, 2 PV-MMA issuer (two issuers keep the tensor pipe fed while one of them
 // waits), 3 V producer, 4.. softmax / correction / epilogue.  All waits are bounded.
 #include <cuda.h>
