@@ -29,8 +29,11 @@ namespace {
 using namespace tc5;
 
 constexpr int PIECE = 128 * 128;                // 16,384: [128 d][64 i]
-constexpr int APPEND_WARPS = 4, FIRST_APPEND = 10;
-constexpr int NUM_WARPS = FIRST_APPEND + APPEND_WARPS, NUM_THREADS = 32 * NUM_WARPS;   // W producer, MMA issuer, 4 epilogue, 4 query, 4 append warps
+// A tcgen05.mma costs its issuing warp about a hundred cycles whatever its size and a head takes 32 of them per row tile: an
+// issuer per d-tile (with the merge's issuers: 8 layers x 128 heads x 8 sequences, layer by layer, 514.6 -> 508.4 us).
+constexpr int ISSUERS = 4, FIRST_EPI = 1 + ISSUERS, FIRST_QUERY = FIRST_EPI + 4;
+constexpr int APPEND_WARPS = 4, FIRST_APPEND = FIRST_QUERY + 4;
+constexpr int NUM_WARPS = FIRST_APPEND + APPEND_WARPS, NUM_THREADS = 32 * NUM_WARPS;   // W producer, MMA issuers, 4 epilogue, 4 query, 4 append warps
 constexpr uint32_t APPEND_PER_WARP = 2;         // rows an absorb block's append warp takes at most
 constexpr int a_bytes(int nt) { return nt * 256; }                              // q_nope of a row tile: two sub-tiles [NT][64 i]
 constexpr int stages(int nt) { return nt == 64 ? 10 : 12; }
@@ -113,7 +116,7 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
     if (tid == 0) {
         *abort_flag = 0;
         for (uint32_t s = 0; s < STAGES; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
-        for (uint32_t b = 0; b < 2; b++) { mbar_init(a_full(b), 128); mbar_init(a_empty(b), 1); mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 128); }
+        for (uint32_t b = 0; b < 2; b++) { mbar_init(a_full(b), 128); mbar_init(a_empty(b), ISSUERS); mbar_init(acc_full(b), ISSUERS); mbar_init(acc_empty(b), 128); }
         mbar_init_fence();
     }
     if (warp == 1) tc_alloc<TMEM_COLS>(tmem_slot);
@@ -140,7 +143,8 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
             }
             grid_dependency_wait();
         }
-    } else if (warp == 1) {
+    } else if (warp < FIRST_EPI) {
+        const uint32_t d = warp - 1;               // this issuer's d-tile of every unit
         constexpr uint32_t IDESC = instr_desc(Fmt<T>::v, 128, NT), HI = desc_hi(1024);
         bool ok = true;
         uint32_t i = 0, n = 0;                     // weight pieces and row tiles so far
@@ -149,25 +153,30 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
             for (uint32_t rt = x.rt0; rt < x.rt1 && ok; rt++, n++) {
                 const uint32_t b = n & 1, par = (n >> 1) & 1;
                 ok = mbar_wait(a_full(b), par, abort_flag, status) && mbar_wait(acc_empty(b), par ^ 1, abort_flag, status);
-                for (uint32_t p = 0; p < 2 * n_d && ok; p++) {
-                    const uint32_t s = (i + p) % STAGES;
+                if (d >= n_d) {                    // a part of a head has fewer
+                    if (ok && lane == 0) { mbar_arrive(a_empty(b)); mbar_arrive(acc_full(b)); }
+                    __syncwarp();
+                    continue;
+                }
+                for (uint32_t half = 0; half < 2 && ok; half++) {
+                    const uint32_t p = 2 * d + half, s = (i + p) % STAGES;
                     ok = mbar_wait(full(s), ((i + p) / STAGES) & 1, abort_flag, status);
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
-                        const uint32_t da = desc_lo(base + s * PIECE), db = desc_lo(base + OFF_A + b * a_bytes(NT) + (p & 1) * (NT * 128));
+                        const uint32_t da = desc_lo(base + s * PIECE), db = desc_lo(base + OFF_A + b * a_bytes(NT) + half * (NT * 128));
 #pragma unroll
                         for (int k = 0; k < 4; k++)
-                            tc_mma(tmem + b * 4 * NT + (p / 2) * NT, da + ((k * 32) >> 4), HI, db + ((k * 32) >> 4), HI, IDESC, ((p & 1) == 0 && k == 0) ? 0u : 1u);
+                            tc_mma(tmem + b * 4 * NT + d * NT, da + ((k * 32) >> 4), HI, db + ((k * 32) >> 4), HI, IDESC, (half == 0 && k == 0) ? 0u : 1u);
                         if (rt + 1 == x.rt1) tc_commit(empty(s));          // the unit's last row tile frees the weights
-                        if (p + 1 == 2 * n_d) { tc_commit(a_empty(b)); tc_commit(acc_full(b)); }
+                        if (half) { tc_commit(a_empty(b)); tc_commit(acc_full(b)); }
                     }
                     __syncwarp();
                 }
             }
             i += 2 * n_d;
         }
-    } else if (warp < 6) {
+    } else if (warp < FIRST_QUERY) {
         // ---- epilogue: lane = d, columns = query rows
         grid_dependency_wait();                    // q_abs is still read by the attention kernel before
         const uint32_t q4 = warp % 4;
@@ -205,7 +214,7 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
     } else {
         // ---- query rows: q_nope -> operand rows, q_rope -> behind the absorbed dims (by the unit that has d-tile 0)
         grid_dependency_wait();
-        const uint32_t t = tid - 6 * 32;
+        const uint32_t t = tid - FIRST_QUERY * 32;
         bool ok = true;
         uint32_t n = 0;
         for (uint32_t u = u0; u < u1; u++) {

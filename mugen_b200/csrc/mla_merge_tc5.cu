@@ -36,9 +36,17 @@ constexpr int OFF_A = NSUB * W_SUB;            // two buffers of hi + lo
 constexpr int OFF_MISC = OFF_A + 2 * 2 * A_HALF;
 constexpr int MISC_BYTES = 256;
 constexpr int SMEM_BYTES = OFF_MISC + MISC_BYTES + 1024;   // + slack to round the base up to 1 KB
-constexpr int RED_WARPS = 16, FIRST_RED = 6;    // W producer, MMA issuer, 4 epilogue warps, then the reduction
-constexpr int NUM_THREADS = 32 * (FIRST_RED + RED_WARPS);
-constexpr uint32_t TMEM_COLS = 32;
+constexpr int RED_WARPS = 16;
+// A tcgen05.mma costs its issuing warp about a hundred cycles whatever its size, and a tile takes 64 of them (hi and lo).  With
+// few rows that is longer than the tile's loads: four issuers take two sub-tiles each into accumulators of their own, which the
+// epilogue adds in a fixed order (27 blocks of 16 heads x 4 rows: 996 -> 970 us with the absorb's issuers).  With more than 8
+// rows (G = 1) the reduction is what takes long and needs the registers: one issuer there (four: 80 rows x 16 heads x 27 layers
+// 385 -> 392 us).
+template <int G>
+struct Roles {        // warps: W producer, MMA issuers, 4 epilogue, then the reduction
+    static constexpr int ISSUERS = G == 1 ? 1 : 4, FIRST_EPI = 1 + ISSUERS, FIRST_RED = FIRST_EPI + 4, THREADS = 32 * (FIRST_RED + RED_WARPS);
+    static constexpr uint32_t TMEM_COLS = 2 * ISSUERS * MT;
+};
 
 struct MergeArgs {
     const float* recs;
@@ -112,9 +120,11 @@ __device__ __forceinline__ void reduce_row(const MergeArgs& a, const RowParts& r
 }
 
 template <typename T, int G>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(Roles<G>::THREADS, 1)
 merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restrict__ out, const MergeArgs a, uint32_t* __restrict__ status)
 {
+    constexpr int ISSUERS = Roles<G>::ISSUERS, FIRST_EPI = Roles<G>::FIRST_EPI, FIRST_RED = Roles<G>::FIRST_RED;
+    constexpr uint32_t TMEM_COLS = Roles<G>::TMEM_COLS;
     extern __shared__ unsigned char merge_tc5_smem[];
     const uint32_t raw = smem_u32(merge_tc5_smem);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -143,7 +153,7 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
     if (tid == 0) {
         *abort_flag = 0;
         for (uint32_t s = 0; s < NSUB; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
-        for (uint32_t b = 0; b < 2; b++) { mbar_init(a_full(b), 32 * RED_WARPS); mbar_init(a_empty(b), 1); mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 128); }
+        for (uint32_t b = 0; b < 2; b++) { mbar_init(a_full(b), 32 * RED_WARPS); mbar_init(a_empty(b), ISSUERS); mbar_init(acc_full(b), ISSUERS); mbar_init(acc_empty(b), 128); }
         mbar_init_fence();
     }
     if (warp == 1) tc_alloc<TMEM_COLS>(tmem_slot);
@@ -168,7 +178,8 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
             }
             grid_dependency_wait();
         }
-    } else if (warp == 1) {
+    } else if (warp < FIRST_EPI) {
+        const uint32_t part = warp - 1;
         constexpr uint32_t IDESC = instr_desc(Fmt<T>::v, kVDim, MT), HI = desc_hi(1024);
         bool ok = true;
         uint32_t n = 0, un = 0;                    // row tiles and units so far
@@ -177,7 +188,8 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
             for (uint32_t rt = x.rt0; rt < x.rt1 && ok; rt++, n++) {
                 const uint32_t b = n & 1, par = (n >> 1) & 1;
                 ok = mbar_wait(a_full(b), par, abort_flag, status) && mbar_wait(acc_empty(b), par ^ 1, abort_flag, status);
-                for (uint32_t s = 0; s < NSUB && ok; s++) {
+                for (uint32_t i = 0; i < NSUB / ISSUERS && ok; i++) {
+                    const uint32_t s = part * (NSUB / ISSUERS) + i, d = tmem + (b * ISSUERS + part) * MT;
                     ok = mbar_wait(full(s), un & 1, abort_flag, status);
                     if (!ok) break;
                     tc_fence_after();
@@ -185,11 +197,11 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
                         const uint32_t da = desc_lo(base + s * W_SUB), db = desc_lo(base + OFF_A + b * 2 * A_HALF + s * A_SUB);
 #pragma unroll
                         for (int k = 0; k < 4; k++) {
-                            tc_mma(tmem + b * MT, da + ((k * 32) >> 4), HI, db + ((k * 32) >> 4), HI, IDESC, (s == 0 && k == 0) ? 0u : 1u);
-                            tc_mma(tmem + b * MT, da + ((k * 32) >> 4), HI, db + ((A_HALF + k * 32) >> 4), HI, IDESC, 1u);
+                            tc_mma(d, da + ((k * 32) >> 4), HI, db + ((k * 32) >> 4), HI, IDESC, (i == 0 && k == 0) ? 0u : 1u);
+                            tc_mma(d, da + ((k * 32) >> 4), HI, db + ((A_HALF + k * 32) >> 4), HI, IDESC, 1u);
                         }
                         if (rt + 1 == x.rt1) tc_commit(empty(s));          // the unit's last row tile frees the weights
-                        if (s + 1 == NSUB) { tc_commit(a_empty(b)); tc_commit(acc_full(b)); }
+                        if (i + 1 == NSUB / ISSUERS) { tc_commit(a_empty(b)); tc_commit(acc_full(b)); }
                     }
                     __syncwarp();
                 }
@@ -206,23 +218,39 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
             for (uint32_t rt = x.rt0; rt < x.rt1; rt++, n++) {
                 const uint32_t b = n & 1, live = min(uint32_t(MT), a.rows - rt * MT);
                 T* dst = out + (size_t(x.li) * a.rows * a.H + x.h) * kVDim + q4 * 32 + lane;
-                size_t at[MT];
-#pragma unroll
-                for (int k = 0; k < MT; k++) {
-                    const uint32_t r = rt * MT + min(uint32_t(k), live - 1);
-                    at[k] = size_t(a.att_row ? a.att_row[r] : r) * a.H * kVDim;
-                }
+                // the caller's row of column `lane`, read ahead of the wait
+                const uint32_t my_row = rt * MT + min(lane, live - 1), my_at = a.att_row ? a.att_row[my_row] : my_row;
                 ok = ok && mbar_wait(acc_full(b), (n >> 1) & 1, abort_flag, status);
                 ok = __all_sync(0xffffffffu, ok);
                 tc_fence_after();
-                uint32_t o[MT];
-                tc_ld16(tmem + ((q4 * 32u) << 16) + b * MT, o);
-                tc_wait_ld();
+                float v[MT];
+                {
+                    const uint32_t acc = tmem + ((q4 * 32u) << 16) + b * ISSUERS * MT;
+                    uint32_t o0[MT], o1[MT];
+                    tc_ld16(acc, o0);
+                    if constexpr (ISSUERS == 4) {
+                        tc_ld16(acc + MT, o1);
+                        tc_wait_ld();
+#pragma unroll
+                        for (int k = 0; k < MT; k++) v[k] = __uint_as_float(o0[k]) + __uint_as_float(o1[k]);
+                        tc_ld16(acc + 2 * MT, o0);
+                        tc_ld16(acc + 3 * MT, o1);
+                        tc_wait_ld();
+#pragma unroll
+                        for (int k = 0; k < MT; k++) v[k] += __uint_as_float(o0[k]) + __uint_as_float(o1[k]);
+                    } else {
+                        tc_wait_ld();
+#pragma unroll
+                        for (int k = 0; k < MT; k++) v[k] = __uint_as_float(o0[k]);
+                    }
+                }
                 tc_fence_before();
                 mbar_arrive(acc_empty(b));
 #pragma unroll
-                for (int k = 0; k < MT; k++)
-                    if (ok && uint32_t(k) < live) dst[at[k]] = Elem<T>::from_f32(__uint_as_float(o[k]));
+                for (int k = 0; k < MT; k++) {
+                    const uint32_t at = __shfl_sync(0xffffffffu, my_at, k);
+                    if (ok && uint32_t(k) < live) dst[size_t(at) * a.H * kVDim] = Elem<T>::from_f32(v[k]);
+                }
             }
         }
     } else {
@@ -327,7 +355,8 @@ int launch_merge_tc5(int dtype, const float* recs, const StepMeta& m, uint32_t n
     a.units = heads * a.r_parts;
     a.run = (a.units + sm_count - 1) / sm_count;
     dim3 grid((a.units + a.run - 1) / a.run);
-    auto go = [&](auto kernel, auto* o) { return int(launch_pdl(kernel, grid, dim3(NUM_THREADS), SMEM_BYTES, st, *map, o, a, status)); };
+    constexpr uint32_t T1 = Roles<1>::THREADS, TN = Roles<2>::THREADS;
+    auto go = [&](auto kernel, auto* o) { return int(launch_pdl(kernel, grid, dim3(m.rows <= 8 ? TN : T1), SMEM_BYTES, st, *map, o, a, status)); };
     auto pick = [&](auto k1, auto k2, auto k4, auto k8, auto k16, auto* o) { return m.rows <= 1 ? go(k16, o) : m.rows <= 2 ? go(k8, o) : m.rows <= 4 ? go(k4, o) : m.rows <= 8 ? go(k2, o) : go(k1, o); };
     return dtype == 0 ? pick(merge_outproj_tc5_kernel<__half, 1>, merge_outproj_tc5_kernel<__half, 2>, merge_outproj_tc5_kernel<__half, 4>,
                              merge_outproj_tc5_kernel<__half, 8>, merge_outproj_tc5_kernel<__half, 16>, static_cast<__half*>(out))
