@@ -139,3 +139,53 @@ def test_projection_shapes_against_numpy_restatement(torch, dt, rows, H, E, R):
     _close(_bits(hid), want_h, dt, "Wo + residual")
     assert ctx.status() == 0
     ctx.close()
+
+
+@pytest.mark.parametrize("rows,H,E,R,shift", [
+    (1, 5, 72, 0, 0),               # a k-block of 8 values behind a whole one; outputs off every tile
+    (16, 16, 2048, 0, 0), (17, 16, 2048, 0, 4),       # the widths of gemm_rows_kernel and one row more; outputs off 16 bytes
+    (33, 5, 1000, 200, 0), (65, 16, 520, 64, 0), (128, 3, 2048, 0, 1),
+    (129, 16, 2048, 0, 0),          # SM pairs: a second tile of one row ...
+    (256, 5, 72, 0, 4), (257, 128, 1000, 136, 0), (700, 16, 2048, 0, 0),
+])
+def test_projections_at_the_edges_of_their_tiles(torch, rows, H, E, R, shift):
+    """Both projection kernels against float64 of the same rounded operands: norms and q_a are rounded to fp16 as the reference
+    rounds them, so what remains is one rounding per output (2^-11 at most, 2.9e-4 in the mean square), a few last places
+    of the normalised rows that fall the other way, and in the residual a second rounding: rel-L2 1e-3."""
+    from mugen_b200.mla import MlaContext
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(rows * 7 + E)
+    rn = lambda *shape, scale=1.0: (torch.randn(shape, device="cuda", generator=gen) * scale).half()
+    bits = lambda t: t.view(torch.int16).cpu().numpy().view(np.uint16)
+    eps, QD, VD = 1e-6, H * 192, H * 128
+    ctx = MlaContext(n_layers=1, n_heads=H, dtype=synth.DT_F16, n_pages=2, max_seqs=1, max_seq_len=64, rope_theta=1e4,
+                     rope_scaling_factor=1.0, rope_original_ctx=4096, rms_norm_eps=eps)
+    w = dict(attn_norm=1 + rn(E, scale=0.1), kv_a_mqa=rn(576, E, scale=E ** -0.5), wo=rn(E, VD, scale=VD ** -0.5))
+    w.update(dict(q_a=rn(R, E, scale=E ** -0.5), q_a_norm=1 + rn(R, scale=0.1), q_b=rn(QD, R, scale=R ** -0.5)) if R
+             else dict(q=rn(QD, E, scale=E ** -0.5)))
+    ctx.set_block_weights(0, **{k: bits(v) for k, v in w.items()})
+
+    def at(n_cols):                 # an output that starts `shift` values behind a 16-byte boundary
+        return torch.zeros(rows * n_cols + 8, dtype=torch.float16, device="cuda")[shift:shift + rows * n_cols].view(rows, n_cols)
+
+    def norm(x, g):
+        return (x.double() * torch.rsqrt((x.double() ** 2).mean(-1, keepdim=True) + eps) * g.double()).half()
+
+    def close(got, want, what):
+        e = (got.double() - want).norm() / want.norm()
+        assert e <= 1e-3, f"{what}: rel-L2 {e:.2e}"
+
+    hidden, q, kv = rn(rows, E), at(QD), at(576)
+    ctx.block_project_in(0, hidden, q, kv)
+    x = norm(hidden, w["attn_norm"])
+    a = x
+    if R:
+        a = norm((x.double() @ w["q_a"].double().T).half(), w["q_a_norm"])
+    close(q, a.double() @ (w["q_b"] if R else w["q"]).double().T, "q")
+    close(kv, x.double() @ w["kv_a_mqa"].double().T, "kv_a")
+    att, out = rn(rows, VD), at(E)
+    out.copy_(hidden)
+    ctx.block_project_out(0, att, out)
+    close(out, hidden.double() + (att.double() @ w["wo"].double().T).half().double(), "hidden")
+    assert ctx.status() == 0
+    ctx.close()
