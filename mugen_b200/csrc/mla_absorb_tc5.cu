@@ -6,7 +6,7 @@
 //
 // What bounds it is W_UK (131 KB per layer and head, read once), so the kernel is a weight stream: persistent blocks, one
 // per SM, each with an equal run of (layer, head) units.  W_UK_h^T ([512 d][128 i], contraction index contiguous, made
-// once at registration) arrives by TMA in pieces of 128 d x 64 i (16 KB) through a ring of eight or nine, across unit
+// once at registration) arrives by TMA in pieces of 128 d x 64 i (16 KB) through a ring of twelve or eight, across unit
 // boundaries, and is the M side of the MMA (tcgen05.mma M128 N=NT K16, four d-tiles of NT = 16, 32 or 64 columns, two
 // accumulator sets in turn); the query rows are its N side, so a step of one row does not pay for 64.  Four warps copy
 // q_nope into swizzled operand rows (two buffers) and q_rope behind the absorbed dims; four drain the accumulators.
@@ -18,6 +18,7 @@
 // itself: four further warps of every block take up to two rows each, blocks behind the absorb blocks what is left.
 #include <algorithm>
 
+#include "mla_absorb_ring.h"
 #include "mla_append.cuh"
 #include "mla_launch.h"
 #include "mla_tc5.cuh"
@@ -36,7 +37,7 @@ constexpr int APPEND_WARPS = 4, FIRST_APPEND = FIRST_QUERY + 4;
 constexpr int NUM_WARPS = FIRST_APPEND + APPEND_WARPS, NUM_THREADS = 32 * NUM_WARPS;   // W producer, MMA issuers, 4 epilogue, 4 query, 4 append warps
 constexpr uint32_t APPEND_PER_WARP = 2;         // rows an absorb block's append warp takes at most
 constexpr int a_bytes(int nt) { return nt * 256; }                              // q_nope of a row tile: two sub-tiles [NT][64 i]
-constexpr int stages(int nt) { return nt == 64 ? 10 : 12; }
+constexpr int stages(int nt) { return ISSUERS * (nt == 64 ? 2 : 3); }             // as many per issuer as fit (mla_absorb_ring.h)
 constexpr int off_a(int nt) { return stages(nt) * PIECE; }
 constexpr int off_append(int nt) { return off_a(nt) + 2 * a_bytes(nt); }
 constexpr int off_misc(int nt) { return off_append(nt) + APPEND_WARPS * kAppendRowSmem; }
@@ -60,6 +61,7 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
                   const AppendArgs app, uint32_t* __restrict__ status)
 {
     constexpr int STAGES = stages(NT), OFF_A = off_a(NT), OFF_MISC = off_misc(NT);
+    constexpr AbsorbRing RING{STAGES / ISSUERS};
     constexpr uint32_t TMEM_COLS = 8 * NT;                      // two sets of four d-tiles x NT columns
     extern __shared__ unsigned char absorb_tc5_smem[];
     grid_launch_dependents();
@@ -129,13 +131,12 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
         // ---- the weights are constant: their loads do not wait for earlier kernels
         if (lane == 0) {
             bool ok = true;
-            uint32_t i = 0;
             for (uint32_t u = u0; u < u1 && ok; u++) {
                 const Unit x = unit_of(u);
                 const int row = int(((a.layer0 + x.li) * a.H + x.h) * kRank);
-                for (uint32_t p = 0; p < 2 * n_d && ok; p++, i++) {
-                    const uint32_t s = i % STAGES;
-                    ok = mbar_wait(empty(s), ((i / STAGES) & 1) ^ 1, abort_flag, status);
+                for (uint32_t p = 0; p < 2 * n_d && ok; p++) {
+                    const uint32_t s = RING.stage(p / 2, u - u0, p & 1);
+                    ok = mbar_wait(empty(s), RING.parity(u - u0, p & 1) ^ 1, abort_flag, status);
                     if (!ok) break;
                     mbar_expect_tx(full(s), PIECE);
                     tma_load_2d(base + s * PIECE, &map_w, full(s), 64 * int(p & 1), row + 128 * int(x.d0 + p / 2));
@@ -147,7 +148,7 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
         const uint32_t d = warp - 1;               // this issuer's d-tile of every unit
         constexpr uint32_t IDESC = instr_desc(Fmt<T>::v, 128, NT), HI = desc_hi(1024);
         bool ok = true;
-        uint32_t i = 0, n = 0;                     // weight pieces and row tiles so far
+        uint32_t n = 0;                            // row tiles so far
         for (uint32_t u = u0; u < u1 && ok; u++) {
             const Unit x = unit_of(u);
             for (uint32_t rt = x.rt0; rt < x.rt1 && ok; rt++, n++) {
@@ -159,8 +160,8 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
                     continue;
                 }
                 for (uint32_t half = 0; half < 2 && ok; half++) {
-                    const uint32_t p = 2 * d + half, s = (i + p) % STAGES;
-                    ok = mbar_wait(full(s), ((i + p) / STAGES) & 1, abort_flag, status);
+                    const uint32_t s = RING.stage(d, u - u0, half);
+                    ok = mbar_wait(full(s), RING.parity(u - u0, half), abort_flag, status);
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
@@ -174,7 +175,6 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
                     __syncwarp();
                 }
             }
-            i += 2 * n_d;
         }
     } else if (warp < FIRST_QUERY) {
         // ---- epilogue: lane = d, columns = query rows

@@ -9,6 +9,7 @@
 #include <fstream>
 #include <numeric>
 
+#include "../../mugen_b200/csrc/mla_absorb_ring.h"
 #include "../../mugen_b200/host/mla_host.hpp"
 #include "../../mugen_b200/host/page_table.hpp"
 #include "../../mugen_b200/host/rope_table.hpp"
@@ -173,6 +174,81 @@ static void test_planner()
     }
 }
 
+// The absorb kernel's weight ring with its barriers as the hardware tests them: one bit of the phase number.  Copies in flight
+// land in any order, an issuer may run one row tile ahead of the slowest (two query buffers), and a stage's release may lag.
+// Random schedules; returns false where an issuer reads a piece that has not landed, a piece is requested into a stage that
+// is still read, or nothing can move any more.
+template <typename Stage, typename Parity>
+static bool ring_holds(uint32_t n_d, uint32_t n_stages, uint32_t units, uint32_t seed, Stage stage, Parity parity)
+{
+    const auto passes = [](uint32_t completed, uint32_t bit) { return (completed & 1) != bit; };       // mbarrier.try_wait.parity
+    std::vector<uint32_t> full(n_stages, 0), empty(n_stages, 0);          // completed phases
+    std::vector<int> in(n_stages, -1);                                    // landed and not yet released piece of a stage
+    std::vector<uint32_t> flying, released, at(n_d, 0), done(units, 0);   // at: an issuer's next piece; done: issuers past a unit
+    const uint32_t pieces = units * 2 * n_d;
+    uint32_t requested = 0, finished = 0;
+    const auto where = [&](uint32_t p) { return stage((p / 2) % n_d, p / (2 * n_d), p % 2); };
+    const auto bit = [&](uint32_t p) { return parity((p / 2) % n_d, p / (2 * n_d), p % 2); };
+    while (finished < n_d || !released.empty()) {
+        bool moved = false;
+        for (uint32_t tries = 0; tries < 64 && !moved; tries++) {
+            seed = seed * 1664525u + 1013904223u;
+            const uint32_t pick = seed >> 16, act = pick % (n_d + 3);
+            if (act == 0 && requested < pieces && passes(empty[where(requested)], bit(requested) ^ 1)) {
+                const uint32_t s = where(requested);
+                for (uint32_t f : flying) if (where(f) == s) return false;
+                if (in[s] >= 0) return false;
+                flying.push_back(requested++);
+                moved = true;
+            } else if (act == 1 && !flying.empty()) {
+                const uint32_t k = (pick >> 4) % flying.size(), p = flying[k];
+                flying.erase(flying.begin() + k);
+                in[where(p)] = int(p);
+                full[where(p)]++;
+                moved = true;
+            } else if (act == 2 && !released.empty()) {
+                const uint32_t k = (pick >> 4) % released.size(), s = released[k];
+                released.erase(released.begin() + k);
+                in[s] = -1;
+                empty[s]++;
+                moved = true;
+            } else if (act >= 3) {
+                const uint32_t d = act - 3, unit = at[d] / 2;
+                if (unit >= units || (unit >= 2 && done[unit - 2] < n_d)) continue;
+                const uint32_t p = (unit * n_d + d) * 2 + at[d] % 2, s = where(p);
+                if (!passes(full[s], bit(p))) continue;
+                if (in[s] != int(p)) return false;
+                released.push_back(s);
+                at[d]++;
+                if (at[d] % 2 == 0) done[unit]++;
+                if (at[d] == 2 * units) finished++;
+                moved = true;
+            }
+        }
+        if (!moved) return false;
+    }
+    return true;
+}
+
+static void test_absorb_ring()
+{
+    for (uint32_t n_d : {1u, 2u, 4u})
+        for (uint32_t per : {2u, 3u})
+            for (uint32_t seed = 1; seed <= 300; seed++) {
+                const mla::AbsorbRing ring{per};
+                CHECK(ring_holds(n_d, 4 * per, 12, seed, [&](uint32_t d, uint32_t u, uint32_t h) { return ring.stage(d, u, h); },
+                                 [&](uint32_t, uint32_t u, uint32_t h) { return ring.parity(u, h); }));
+            }
+    // a ring that all issuers share does not hold: the model finds the read ahead of the copy
+    for (uint32_t stages : {10u, 12u}) {
+        uint32_t broken = 0;
+        for (uint32_t seed = 1; seed <= 300; seed++)
+            broken += !ring_holds(4, stages, 12, seed, [&](uint32_t d, uint32_t u, uint32_t h) { return (8 * u + 2 * d + h) % stages; },
+                                  [&](uint32_t d, uint32_t u, uint32_t h) { return ((8 * u + 2 * d + h) / stages) & 1; });
+        CHECK(broken > 0);
+    }
+}
+
 static void test_wrapper_without_gpu()
 {
     LatentKVCacheConfig cfg;
@@ -235,6 +311,7 @@ int main(int argc, char** argv)
     if (argc >= 2 && !std::strcmp(argv[1], "units")) {
         test_page_table();
         test_planner();
+        test_absorb_ring();
         test_wrapper_without_gpu();
         std::puts("host units ok");
         return 0;

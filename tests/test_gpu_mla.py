@@ -820,3 +820,49 @@ def test_merge_of_few_rows_in_many_parts(torch, oracle, H, dt, lens):
         cache = np.concatenate([case.caches[b][:n], rows[b:b + 1]])
         check_close(got[b], oracle.attention(case.q[b], cache, n + 1, case.w_uk, case.w_uv, case.w_type, H, dt), dt, f"row {b}")
     ctx.close()
+
+
+@pytest.mark.parametrize("rows,L", [(8, 6), (24, 6), (48, 6), (70, 3)])
+def test_absorb_streams_the_weights_of_many_units_per_block(torch, rows, L):
+    """128 heads x L layers in one launch: every block of the absorb walks several (layer, head) units through its ring, with
+    query tiles of 16, 32 and 64 rows.  Every layer has weights of its own; all rows and heads against float64."""
+    from mugen_b200.mla import MlaContext
+    H, dt = 128, synth.DT_BF16
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(rows)
+    rn = lambda *shape, scale=1.0: (torch.randn(shape, device="cuda", generator=gen) * scale).bfloat16()
+    bits = lambda t: t.view(torch.int16).cpu().numpy().view(np.uint16)
+    lens = [5 + 7 * i % 61 for i in range(rows)]
+    ctx = MlaContext(n_layers=L, n_heads=H, dtype=dt, n_pages=2 * rows, max_seqs=rows, max_seq_len=128, **YARN)
+    ctx.shuffle_free_pages(3)
+    w_uk, w_uv = rn(L, H, 128, 512, scale=0.02), rn(L, H, 128, 512, scale=0.02)
+    for l in range(L):
+        ctx.set_layer_weights(l, bits(w_uk[l]), bits(w_uv[l]), synth.W_BF16, bits(1 + rn(512, scale=0.1)))
+    seqs = [ctx.seq_create() for _ in lens]
+    for l in range(L):
+        for s, n in zip(seqs, lens):
+            ctx.write_rows(l, s, 0, rn(n, 576).view(torch.int16))
+    for s, n in zip(seqs, lens):
+        ctx.advance_seq_len(s, n)
+    kv, q = rn(L, rows, 576), rn(L, rows, H, 192, scale=0.9)
+    out = torch.zeros((L, rows, H, 128), device="cuda", dtype=torch.bfloat16)
+    for rep in range(20):                     # the copies of a launch land in another order every time
+        out.zero_()
+        ctx.step_begin(seqs)
+        ctx.step_layers(0, L, kv, q, out)
+        ctx.step_end()
+        if rep < 19:
+            ctx.rollback(seqs, lens)
+        assert ctx.status() == 0
+        first = out.clone() if rep == 0 else first
+        assert torch.equal(out, first)
+    for l in range(L):
+        for r, (s, n) in enumerate(zip(seqs, lens)):
+            c = torch.from_numpy(ctx.read_rows(l, s, 0, n + 1).view(np.int16)).cuda().view(torch.bfloat16).double()
+            qa = torch.einsum("hi,hid->hd", q[l, r, :, :128].double(), w_uk[l].double())
+            p = torch.softmax((qa @ c[:, :512].T + q[l, r, :, 128:].double() @ c[:, 512:].T) / 192 ** 0.5, -1)
+            want = torch.einsum("hd,hjd->hj", p @ c[:, :512], w_uv[l].double())
+            e = ((out[l, r].double() - want).norm(dim=-1) / want.norm(dim=-1)).max().item()      # per head
+            # absorbed queries, probabilities and outputs are rounded to 8 bits once each (2^-9 at most); REL_L2 holds over all heads
+            assert e <= 4 * REL_L2, f"layer {l}, row {r}: rel-L2 of the worst head {e:.2e}"
+    ctx.close()
