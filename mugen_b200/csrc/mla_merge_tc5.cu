@@ -17,6 +17,7 @@
 // (One block per head and 16 or 64 rows with load, reduction and MMAs in sequence: 27 layers x 16 heads x 1 row took 24 us
 // for 57 MB.)
 #include <algorithm>
+#include <type_traits>
 
 #include "mla_launch.h"
 #include "mla_tc5.cuh"
@@ -58,14 +59,15 @@ struct MergeArgs {
 };
 
 // One row's merged state by one warp: dims dim0 + 64*k + 2*lane (+1), k < DL/2 (DL = 1: dim0 + lane).  acc comes back normalised.
-template <int DL>
+// Index: of a float within 32 parts, 64 bits where a caller's partials need them (launch_merge_tc5).
+template <int DL, typename Index>
 __device__ __forceinline__ void reduce_row(const MergeArgs& a, const RowParts& rp, uint32_t h, uint32_t dim0, uint32_t lane, float (&acc)[DL])
 {
     constexpr int W = DL == 1 ? 1 : 2, Q = DL / W, PB = 32 / DL;      // floats per load, loads per part, parts per batch
     float M = -INFINITY, L = 0.0f;
 #pragma unroll
     for (int k = 0; k < DL; k++) acc[k] = 0.0f;
-    const uint32_t stride = a.rec_stride * kPart;             // floats (a workspace holds fewer than 2^32)
+    const Index stride = Index(a.rec_stride) * kPart;
     const float* rec0 = a.recs + size_t(rp.rec_off + h) * kPart;
     for (uint32_t c0 = rp.begin; c0 < rp.end; c0 += 32) {
         const uint32_t n = min(32u, rp.end - c0);
@@ -119,7 +121,7 @@ __device__ __forceinline__ void reduce_row(const MergeArgs& a, const RowParts& r
     for (int k = 0; k < DL; k++) acc[k] *= inv;
 }
 
-template <typename T, int G>
+template <typename T, int G, typename Index = uint32_t>
 __global__ void __launch_bounds__(Roles<G>::THREADS, 1)
 merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restrict__ out, const MergeArgs a, uint32_t* __restrict__ status)
 {
@@ -284,7 +286,7 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
                 const RowParts rp = next;
                 fetch(u, rt + 1);
                 float acc[16 / G];
-                if (rr < live) reduce_row<16 / G>(a, rp, x.h, dim0, lane, acc);
+                if (rr < live) reduce_row<16 / G, Index>(a, rp, x.h, dim0, lane, acc);
                 ok = ok && mbar_wait(a_empty(b), ((n >> 1) & 1) ^ 1, abort_flag, status);      // the MMAs of two tiles ago have read this buffer
                 if (rr < live) {
                     if constexpr (G == 16) {                       // row 0 (of one): 32 dims, half a row of a sub-tile
@@ -326,11 +328,13 @@ int merge_tc5_configure()
         // re-partitioned between consecutive launches
         return e != cudaSuccess ? e : cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     };
-    cudaError_t e = set(merge_outproj_tc5_kernel<__half, 1>);
+    cudaError_t e = set(merge_outproj_tc5_kernel<__half, 1, uint64_t>);
+    if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__half, 1>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__half, 2>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__half, 4>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__half, 8>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__half, 16>);
+    if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__nv_bfloat16, 1, uint64_t>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__nv_bfloat16, 1>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__nv_bfloat16, 2>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__nv_bfloat16, 4>);
@@ -355,13 +359,21 @@ int launch_merge_tc5(int dtype, const float* recs, const StepMeta& m, uint32_t n
     a.units = heads * a.r_parts;
     a.run = (a.units + sm_count - 1) / sm_count;
     dim3 grid((a.units + a.run - 1) / a.run);
-    constexpr uint32_t T1 = Roles<1>::THREADS, TN = Roles<2>::THREADS;
-    auto go = [&](auto kernel, auto* o) { return int(launch_pdl(kernel, grid, dim3(m.rows <= 8 ? TN : T1), SMEM_BYTES, st, *map, o, a, status)); };
-    auto pick = [&](auto k1, auto k2, auto k4, auto k8, auto k16, auto* o) { return m.rows <= 1 ? go(k16, o) : m.rows <= 2 ? go(k8, o) : m.rows <= 4 ? go(k4, o) : m.rows <= 8 ? go(k2, o) : go(k1, o); };
-    return dtype == 0 ? pick(merge_outproj_tc5_kernel<__half, 1>, merge_outproj_tc5_kernel<__half, 2>, merge_outproj_tc5_kernel<__half, 4>,
-                             merge_outproj_tc5_kernel<__half, 8>, merge_outproj_tc5_kernel<__half, 16>, static_cast<__half*>(out))
-                      : pick(merge_outproj_tc5_kernel<__nv_bfloat16, 1>, merge_outproj_tc5_kernel<__nv_bfloat16, 2>, merge_outproj_tc5_kernel<__nv_bfloat16, 4>,
-                             merge_outproj_tc5_kernel<__nv_bfloat16, 8>, merge_outproj_tc5_kernel<__nv_bfloat16, 16>, static_cast<__nv_bfloat16*>(out));
+    // 32 parts of a plan's records are far below 2^32 floats; of a caller's partials they may be more (128 heads: from 2,040
+    // rows on).  64-bit indices everywhere cost 1 % (128 heads x 8 sequences, layer by layer: 510 -> 517 us).
+    const bool wide = uint64_t(32) * a.rec_stride * kPart > ~0u;
+    auto launch = [&](auto k1, auto k2, auto k4, auto k8, auto k16, auto k_wide, auto* o) {
+        auto go = [&](auto kernel, uint32_t threads) { return int(launch_pdl(kernel, grid, dim3(threads), SMEM_BYTES, st, *map, o, a, status)); };
+        constexpr uint32_t T1 = Roles<1>::THREADS, TN = Roles<2>::THREADS;
+        if (wide) return go(k_wide, T1);
+        return m.rows <= 1 ? go(k16, TN) : m.rows <= 2 ? go(k8, TN) : m.rows <= 4 ? go(k4, TN) : m.rows <= 8 ? go(k2, TN) : go(k1, T1);
+    };
+    auto pick = [&](auto* o) {
+        using T = std::remove_pointer_t<decltype(o)>;
+        return launch(merge_outproj_tc5_kernel<T, 1>, merge_outproj_tc5_kernel<T, 2>, merge_outproj_tc5_kernel<T, 4>, merge_outproj_tc5_kernel<T, 8>,
+                      merge_outproj_tc5_kernel<T, 16>, merge_outproj_tc5_kernel<T, 1, uint64_t>, o);
+    };
+    return dtype == 0 ? pick(static_cast<__half*>(out)) : pick(static_cast<__nv_bfloat16*>(out));
 }
 
 }  // namespace mla

@@ -866,3 +866,32 @@ def test_absorb_streams_the_weights_of_many_units_per_block(torch, rows, L):
             # absorbed queries, probabilities and outputs are rounded to 8 bits once each (2^-9 at most); REL_L2 holds over all heads
             assert e <= 4 * REL_L2, f"layer {l}, row {r}: rel-L2 of the worst head {e:.2e}"
     ctx.close()
+
+
+def test_merge_of_partials_beyond_4g_floats(torch):
+    """mla_merge_partials over a caller's buffer of more than 2^32 floats (17 GB): what the parts behind that line hold must reach
+    the outputs.  All states are empty (l = 0) but a few in the last two parts, so every other output is exactly 0."""
+    from mugen_b200.mla import MlaContext
+    H, rows, parts = 128, 2107, 33
+    assert (parts - 2) * rows * H * 514 > 1 << 32
+    if torch.cuda.mem_get_info()[0] < 20 << 30:
+        pytest.skip("needs 20 GB of device memory")
+    ctx = MlaContext(n_layers=1, n_heads=H, dtype=synth.DT_F16, n_pages=2, max_seqs=1, max_seq_len=64, **YARN)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(1)
+    w_uv = (torch.randn(H, 128, 512, device="cuda", generator=gen) * 0.05).half()
+    bits = w_uv.view(torch.int16).cpu().numpy().view(np.uint16)
+    ctx.set_layer_weights(0, bits, bits, synth.W_F16, np.full(512, 0x3C00, np.uint16))
+    p = torch.zeros((parts, rows, H, 514), device="cuda")
+    want = torch.zeros((rows, H, 128), device="cuda", dtype=torch.float64)
+    for part, row, head in [(31, 0, 0), (31, 1000, 64), (31, rows - 1, H - 1), (32, 17, 5), (32, rows - 1, 0)]:
+        acc = torch.randn(512, device="cuda", generator=gen)
+        p[part, row, head, 1] = 1.0
+        p[part, row, head, 2:] = acc
+        want[row, head] = w_uv[head].double() @ acc.double()
+    out = torch.full((rows, H, 128), 7.0, device="cuda", dtype=torch.float16)
+    ctx.merge_partials(0, parts, rows, p, out)
+    assert ctx.status() == 0
+    # the state goes to the product in two halves of 11 bits each: what is left is the rounding of the output
+    assert (out.double() - want).abs().max().item() <= 2.0 ** -11 * want.abs().max().item() * 1.1
+    ctx.close()
