@@ -136,7 +136,7 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
                 const int row = int(((a.layer0 + x.li) * a.H + x.h) * kRank);
                 for (uint32_t p = 0; p < 2 * n_d && ok; p++) {
                     const uint32_t s = RING.stage(p / 2, u - u0, p & 1);
-                    ok = mbar_wait(empty(s), RING.parity(u - u0, p & 1) ^ 1, abort_flag, status);
+                    ok = mbar_wait<kPoll, true>(empty(s), RING.parity(u - u0, p & 1) ^ 1, abort_flag, status);
                     if (!ok) break;
                     mbar_expect_tx(full(s), PIECE);
                     tma_load_2d(base + s * PIECE, &map_w, full(s), 64 * int(p & 1), row + 128 * int(x.d0 + p / 2));
@@ -153,7 +153,7 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
             const Unit x = unit_of(u);
             for (uint32_t rt = x.rt0; rt < x.rt1 && ok; rt++, n++) {
                 const uint32_t b = n & 1, par = (n >> 1) & 1;
-                ok = mbar_wait(a_full(b), par, abort_flag, status) && mbar_wait(acc_empty(b), par ^ 1, abort_flag, status);
+                ok = mbar_wait<kPoll, true>(a_full(b), par, abort_flag, status) && mbar_wait(acc_empty(b), par ^ 1, abort_flag, status);
                 if (d >= n_d) {                    // a part of a head has fewer
                     if (ok && lane == 0) { mbar_arrive(a_empty(b)); mbar_arrive(acc_full(b)); }
                     __syncwarp();

@@ -172,7 +172,7 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
             for (uint32_t u = u0; u < u1 && ok; u++, n++) {
                 const Unit x = unit_of(u);
                 for (uint32_t s = 0; s < NSUB && ok; s++) {
-                    ok = mbar_wait(empty(s), (n & 1) ^ 1, abort_flag, status);
+                    ok = mbar_wait<kPoll, true>(empty(s), (n & 1) ^ 1, abort_flag, status);
                     if (!ok) break;
                     mbar_expect_tx(full(s), W_SUB);
                     tma_load_2d(base + s * W_SUB, &map_w, full(s), 64 * int(s), int(((a.layer0 + x.li) * a.H + x.h) * kVDim));
@@ -189,7 +189,7 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
             const Unit x = unit_of(u);
             for (uint32_t rt = x.rt0; rt < x.rt1 && ok; rt++, n++) {
                 const uint32_t b = n & 1, par = (n >> 1) & 1;
-                ok = mbar_wait(a_full(b), par, abort_flag, status) && mbar_wait(acc_empty(b), par ^ 1, abort_flag, status);
+                ok = mbar_wait<kPoll, true>(a_full(b), par, abort_flag, status) && mbar_wait(acc_empty(b), par ^ 1, abort_flag, status);
                 for (uint32_t i = 0; i < NSUB / ISSUERS && ok; i++) {
                     const uint32_t s = part * (NSUB / ISSUERS) + i, d = tmem + (b * ISSUERS + part) * MT;
                     ok = mbar_wait(full(s), un & 1, abort_flag, status);

@@ -6,6 +6,7 @@ caches).  Every test runs once per attention kernel family the library offers.
 """
 import base64
 import os
+import time
 
 import numpy as np
 import pytest
@@ -894,4 +895,40 @@ def test_merge_of_partials_beyond_4g_floats(torch):
     assert ctx.status() == 0
     # the state goes to the product in two halves of 11 bits each: what is left is the rounding of the output
     assert (out.double() - want).abs().max().item() <= 2.0 ** -11 * want.abs().max().item() * 1.1
+    ctx.close()
+
+
+def test_bounded_waits_do_not_run_while_an_earlier_kernel_does(torch, oracle):
+    """A kernel ahead of the absorb and the merge that lets them start early and then runs for longer than the limit of their
+    barrier waits (about two seconds): the limits must start when it ends, and the results must stand."""
+    spin = torch.cuda._compile_kernel('extern "C" __global__ void spin(int mcycles) {'
+                                      ' asm volatile("griddepcontrol.launch_dependents;");'
+                                      ' const long long t0 = clock64(); while (clock64() - t0 < mcycles * 1000000LL) __nanosleep(1000); }', "spin")
+    H, dt, lens = 128, synth.DT_BF16, [100, 300]
+    case = synth.make_layer_case(77, H, [n + 1 for n in lens], dt)
+    ctx = make_ctx(case, capi.KERNEL_AUTO, max_rows=len(lens))
+    seqs = fill(torch, ctx, case, upto=lens)
+    q, kv = _dev(torch, case.q), _dev(torch, case.kv_a)
+    out, again = (torch.zeros((len(lens), H, 128), dtype=torch.int16, device="cuda") for _ in range(2))
+    partial = torch.zeros((len(lens), H, 514), device="cuda")
+    long = 4_800                                         # 2.4 s at the highest clock; the limit is 4e9 cycles
+    ctx.step_begin(seqs)
+    ctx.step_append(0, kv)
+    ctx.step_attend_partial(0, q, partial)               # also: the step's plan is on the device
+    torch.cuda.synchronize()
+    t0 = time.perf_counter()
+    spin((1, 1, 1), (1, 1, 1), (long,))
+    ctx.step_attend(0, q, out)
+    torch.cuda.synchronize()
+    assert time.perf_counter() - t0 > 2.1
+    spin((1, 1, 1), (1, 1, 1), (long,))
+    ctx.merge_partials(0, 1, len(lens), partial, again)
+    torch.cuda.synchronize()
+    ctx.step_end()
+    assert ctx.status() == 0
+    rows = oracle.append_rows(case.kv_a, lens, case.norm_w, YARN["rms_norm_eps"], 40.0, 4096, 10000.0, dt)
+    for b, n in enumerate(lens):
+        want = oracle.attention(case.q[b], np.concatenate([case.caches[b][:n], rows[b:b + 1]]), n + 1, case.w_uk, case.w_uv, case.w_type, H, dt)
+        check_close(_host(out)[b], want, dt, f"row {b}")
+        check_close(_host(again)[b], want, dt, f"row {b}, merged partial")
     ctx.close()
