@@ -159,8 +159,8 @@ int mla_attend_rows(mla_ctx* ctx, uint32_t layer, uint32_t n, const uint32_t* se
  * >1: a prefill chunk, causal; 0: the sequence takes no token here but still answers the step's
  * query with one row attending its seq_len rows — a KV-range shard that does not own the tail;
  * its kv_a row is ignored) at positions seq_len .. seq_len+n_new-1.  step_begin reserves
- * pages, balances the KV ranges over the SMs and uploads the step's metadata once; the
- * per-layer calls then take only data pointers.  Ordering contract of the reference driver
+ * pages, balances the KV ranges over the SMs and uploads the step's metadata once, on `stream`; the
+ * per-layer calls then take only data pointers, on any stream ordered behind it, and can be captured.  Ordering contract of the reference driver
  * (transformer.cpp:3702, 3980-3996, 4401-4403): per layer append THEN attend over
  * seq_len + (row's offset) + 1 rows; counters advance once, after all layers (step_end). */
 int mla_step_begin(mla_ctx* ctx, uint32_t n_seq, const uint32_t* seq_ids, const uint32_t* n_new,
@@ -184,7 +184,7 @@ int mla_step_layers(mla_ctx* ctx, uint32_t layer_begin, uint32_t n_layers, const
 int mla_step_layer_host(mla_ctx* ctx, uint32_t layer, const void* kv_a_host, const void* q_host,
                         void* out_host, void* stream);
 int mla_step_end(mla_ctx* ctx);
-/* Rows in the current step and the number of KV segments they were split into. */
+/* Rows in the current step and the number of KV segments that one layer of them was split into. */
 int mla_step_info(const mla_ctx* ctx, uint32_t* rows, uint32_t* segments);
 
 /* How the planner spread the last planned step over the persistent attention workers (SM pairs or SMs): their

@@ -102,11 +102,12 @@ struct mla_ctx {
     size_t meta_cap = 0;
     char* meta_dev = nullptr;       // [kPlanRegions][meta_cap]
     char* meta_host = nullptr;      // [kMetaRing][meta_cap], page-locked
-    // Plans of the open step, made and uploaded by the first call that needs them.  `plan`: every new token is a decode-style
-    // query row, one layer at a time.  A step that holds prefill chunks (sequences taking >= kPrefillMin new tokens) also
-    // has `plan_rest`: its query rows are the step's OTHER rows, the chunks go through the expanded-form prefill kernels
-    // (run_layer); the explicit per-layer calls (mla_step_append / _attend / _attend_partial) keep using the first.
-    // `stack` / `stack_tail`: groups of layers of one mla_step_layers call.
+    // Plans of the open step.  `plan`: every new token is a decode-style query row, one layer at a time.  A step that holds
+    // prefill chunks (sequences taking >= kPrefillMin new tokens) also has `plan_rest`: its query rows are the step's OTHER
+    // rows, the chunks go through the expanded-form prefill kernels (run_layer); the explicit per-layer calls
+    // (mla_step_append / _attend / _attend_partial) keep using the first.  mla_step_begin makes and uploads these two on its
+    // own stream, so that the calls behind it only launch: on any stream ordered behind it, and under capture.
+    // `stack` / `stack_tail`: groups of layers of one mla_step_layers call, made and uploaded by the call that needs them.
     Plan plan, plan_rest, stack, stack_tail;
     bool has_chunks = false;
     std::vector<RowSpec> rows;       // of the open step
@@ -370,17 +371,19 @@ int build_plan(mla_ctx* c, Plan& plan, int region, const std::vector<uint32_t>& 
     }
     const uint32_t NG = uint32_t(groups.size());
     const uint32_t G = uint32_t(segs.size()), W = uint32_t(cta_seg_begin.size()) - 1;
-    if (R) {
-        plan.min_pages = W ? ~0u : 0u;
+    if (layers) {
+        plan.min_pages = R && W ? ~0u : 0u;
         for (uint32_t w = 0; w < W; w++) {
             uint32_t pages = 0;
             for (uint32_t g = cta_seg_begin[w]; g < cta_seg_begin[w + 1]; g++) pages += segs[g].page_end - segs[g].page_begin;
             plan.min_pages = std::min(plan.min_pages, pages);
             plan.max_pages = std::max(plan.max_pages, pages);
         }
-        c->plan_workers = W;
-        c->plan_min_pages = plan.min_pages;
-        c->plan_max_pages = plan.max_pages;
+        if (region == kPlanStep || region == kPlanRest) {      // what mla_step_balance reports: one layer of the step
+            c->plan_workers = std::max(W, 1u);
+            c->plan_min_pages = plan.min_pages;
+            c->plan_max_pages = plan.max_pages;
+        }
     }
     // layout
     size_t off = 0;
@@ -462,16 +465,9 @@ int build_plan(mla_ctx* c, Plan& plan, int region, const std::vector<uint32_t>& 
     return MLA_OK;
 }
 
-// the open step's plan for one layer at a time
-int step_plan(mla_ctx* c, cudaStream_t st)
-{
-    return c->plan.ready ? int(MLA_OK) : build_plan(c, c->plan, kPlanStep, c->step_seqs, c->rows, nullptr, nullptr, 1, st);
-}
-
 // the plan of a step with prefill chunks: its decode-style rows are the query rows, all its rows are appended
 int rest_plan(mla_ctx* c, cudaStream_t st)
 {
-    if (c->plan_rest.ready) return MLA_OK;
     std::vector<RowSpec> rest;
     std::vector<uint32_t> att_row;
     uint32_t r = 0;
@@ -633,7 +629,6 @@ int run_layer(mla_ctx* c, uint32_t layer, const void* kv_a, const void* q, void*
 {
     if (c->has_chunks) {
         // decode-style rows through their own plan (their append covers ALL new rows of the step), then the chunks
-        if (int e = rest_plan(c, st)) return e;
         if (c->plan_rest.m.rows) {
             if (int e = run_attend(c, layer, q, out, nullptr, c->plan_rest, st, kv_a, kv_a_settled)) return e;
         } else {
@@ -641,7 +636,6 @@ int run_layer(mla_ctx* c, uint32_t layer, const void* kv_a, const void* q, void*
         }
         return run_chunks(c, layer, q, out, st);
     }
-    if (int e = step_plan(c, st)) return e;
     return run_attend(c, layer, q, out, nullptr, c->plan, st, kv_a, kv_a_settled);
 }
 
@@ -1111,9 +1105,12 @@ int mla_step_begin(mla_ctx* c, uint32_t n_seq, const uint32_t* seq_ids, const ui
         c->step_new_rows += nn[i];
     }
     c->step_rows = uint32_t(rows.size());
-    c->plan.ready = c->plan_rest.ready = c->stack.ready = c->stack_tail.ready = false;
+    c->stack.ready = c->stack_tail.ready = false;
     c->step_seqs = std::move(seqs);
     c->step_nnew = std::move(nn);
+    if (int e = build_plan(c, c->plan, kPlanStep, c->step_seqs, rows, nullptr, nullptr, 1, st)) return e;
+    if (c->has_chunks)
+        if (int e = rest_plan(c, st)) return e;
     c->in_step = true;
     return MLA_OK;
 }
@@ -1124,9 +1121,7 @@ int mla_step_append(mla_ctx* c, uint32_t layer, const void* kv_a, void* stream)
     USE_DEVICE(c);
     if (!c->in_step) return fail(c, MLA_ERR_STATE, "step_append outside step_begin/step_end");
     if (int e = check_layer(c, layer, true)) return e;
-    auto st = static_cast<cudaStream_t>(stream);
-    if (int e = step_plan(c, st)) return e;
-    return run_append(c, layer, kv_a, c->plan.m, st);
+    return run_append(c, layer, kv_a, c->plan.m, static_cast<cudaStream_t>(stream));
 }
 
 int mla_step_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, void* stream)
@@ -1135,9 +1130,17 @@ int mla_step_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, void* 
     USE_DEVICE(c);
     if (!c->in_step) return fail(c, MLA_ERR_STATE, "step_attend outside step_begin/step_end");
     if (int e = check_layer(c, layer, true)) return e;
-    auto st = static_cast<cudaStream_t>(stream);
-    if (int e = step_plan(c, st)) return e;
-    return run_attend(c, layer, q, out, nullptr, c->plan, st);
+    return run_attend(c, layer, q, out, nullptr, c->plan, static_cast<cudaStream_t>(stream));
+}
+
+static bool capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return status != cudaStreamCaptureStatusNone;
 }
 
 int mla_step_layers(mla_ctx* c, uint32_t layer_begin, uint32_t n_layers, const void* kv_a, const void* q, void* out,
@@ -1156,6 +1159,9 @@ int mla_step_layers(mla_ctx* c, uint32_t layer_begin, uint32_t n_layers, const v
     // attention and one merge launch, planned together, so that a step of few rows fills the machine.
     uint32_t group = 1;
     if (!c->has_chunks && rows && c->kernel != MLA_KERNEL_MMA) group = uint32_t(std::min<uint64_t>(n_layers, c->ws_rows / rows));
+    // The group's plan is uploaded by this call: not into a captured graph, whose replays would copy from the upload ring again
+    // long after it went on.  A captured call goes layer by layer with the plan of mla_step_begin.
+    if (group > 1 && capturing(st)) group = 1;
     if (group > 1) {
         const uint32_t n_groups = (n_layers + group - 1) / group;
         group = (n_layers + n_groups - 1) / n_groups;
@@ -1187,9 +1193,7 @@ int mla_step_attend_partial(mla_ctx* c, uint32_t layer, const void* q, float* pa
     USE_DEVICE(c);
     if (!c->in_step) return fail(c, MLA_ERR_STATE, "step_attend_partial outside step_begin/step_end");
     if (int e = check_layer(c, layer, true)) return e;
-    auto st = static_cast<cudaStream_t>(stream);
-    if (int e = step_plan(c, st)) return e;
-    return run_attend(c, layer, q, nullptr, partial, c->plan, st);
+    return run_attend(c, layer, q, nullptr, partial, c->plan, static_cast<cudaStream_t>(stream));
 }
 
 int mla_step_layer_partial(mla_ctx* c, uint32_t layer, const void* kv_a, const void* q, float* partial, void* stream)
@@ -1202,7 +1206,6 @@ int mla_step_layer_partial(mla_ctx* c, uint32_t layer, const void* kv_a, const v
     if (c->step_new_rows && !kv_a) return fail(c, MLA_ERR_INVALID, "the step appends rows on this GPU: kv_a is needed");
     auto st = static_cast<cudaStream_t>(stream);
     if (!c->step_new_rows) kv_a = nullptr;           // query-only rows: nothing to append, kv_a is never read
-    if (int e = step_plan(c, st)) return e;
     return run_attend(c, layer, q, nullptr, partial, c->plan, st, kv_a);
 }
 
@@ -1326,8 +1329,8 @@ int mla_step_info(const mla_ctx* c, uint32_t* rows, uint32_t* segments)
 {
     if (!c) return MLA_ERR_INVALID;
     if (rows) *rows = c->step_rows;
-    // the segments of the step's (or the last explicit call's) one-layer plan, which exists once a layer has been launched
-    if (segments) *segments = c->plan.ready ? c->plan.m.segs : c->plan_rest.ready ? c->plan_rest.m.segs : c->stack.m.segs;
+    // of one layer of the step (or of the last explicit call), whatever groups of layers mla_step_layers launches
+    if (segments) *segments = c->plan.m.segs;
     return MLA_OK;
 }
 

@@ -932,3 +932,136 @@ def test_bounded_waits_do_not_run_while_an_earlier_kernel_does(torch, oracle):
         check_close(_host(out)[b], want, dt, f"row {b}")
         check_close(_host(again)[b], want, dt, f"row {b}, merged partial")
     ctx.close()
+
+
+def _step_ctx(torch, H=16, dt=synth.DT_F16, L=3, lens=(100, 700, 64, 5)):
+    """L layers over sequences of `lens` cached tokens, with one new token each: context, sequences, kv_a and q of all layers."""
+    from mugen_b200.mla import MlaContext
+    case = synth.make_layer_case(4400 + H, H, [n + 1 for n in lens], dt)
+    ctx = MlaContext(n_layers=L, n_heads=H, dtype=dt, n_pages=sum(n // 64 + 3 for n in lens) + 8, max_seqs=len(lens) + 1, max_seq_len=2048,
+                     max_rows=256, **YARN)
+    for l in range(L):
+        ctx.set_layer_weights(l, case.w_uk, case.w_uv, case.w_type, case.norm_w)
+    seqs = []
+    for b, n in enumerate(lens):
+        s = ctx.seq_create()
+        for l in range(L):
+            ctx.write_rows(l, s, 0, _dev(torch, np.roll(case.caches[b][:n], l, axis=0)))
+        ctx.advance_seq_len(s, n)
+        seqs.append(s)
+    rng = np.random.default_rng(8)
+    kv = _dev(torch, synth.to_bits(rng.standard_normal((L, len(lens), 576), np.float32), dt))
+    q = _dev(torch, synth.to_bits(rng.standard_normal((L, len(lens), H, 192), np.float32) * np.float32(0.9), dt))
+    return ctx, seqs, list(lens), kv, q
+
+
+def test_step_info_and_balance_describe_the_open_step(torch):
+    """From step_begin on, whichever calls follow: rows, segments and balance of ONE layer of the step that is open."""
+    ctx, seqs, lens, kv, q = _step_ctx(torch)
+    L, B = kv.shape[:2]
+    out = torch.zeros((L, B, 16, 128), dtype=torch.int16, device="cuda")
+    pages = [(n + 1 + 63) // 64 for n in lens]
+    seen = []
+    for part in (seqs, seqs[:1], seqs):
+        n, k = len(part), sum(pages[:len(part)])
+        ctx.step_begin(part)
+        first = (ctx.step_info(), ctx.step_balance())
+        assert first[0][0] == n and n <= first[0][1] <= k and first[1][0] <= k and 1 <= first[1][1] <= first[1][2] <= k
+        ctx.step_layers(0, L, kv[:, :n].contiguous(), q[:, :n].contiguous(), out[:, :n].contiguous())       # one group of three layers
+        assert (ctx.step_info(), ctx.step_balance()) == first
+        ctx.step_append(0, kv[0, :n].contiguous())
+        ctx.step_attend(0, q[0, :n].contiguous(), out[0, :n].contiguous())
+        assert (ctx.step_info(), ctx.step_balance()) == first
+        ctx.step_end()
+        ctx.rollback(seqs, lens)
+        seen.append(first)
+    assert seen[0] == seen[2] != seen[1]
+    ctx.step_begin(seqs[:1], [130])               # a prompt chunk alone: no row is left to the decode kernels
+    assert ctx.step_info()[0] == 130 and ctx.step_balance() == (1, 0, 0)
+    ctx.step_end()
+    assert ctx.status() == 0
+    ctx.close()
+
+
+def test_calls_of_a_step_on_streams_of_their_own(torch):
+    """The step's metadata is on the device when step_begin's stream says so: appends of two layers (which share no workspace) on
+    two streams, both ordered behind that stream and not behind each other.  The first is held back by a busy stream."""
+    ctx, seqs, lens, kv, q = _step_ctx(torch)
+    L = kv.shape[0]
+    ctx.step_begin(seqs)
+    for l in range(L):
+        ctx.step_append(l, kv[l])
+    ctx.step_end()
+    want = [[ctx.read_rows(l, s, n, 1).copy() for s, n in zip(seqs, lens)] for l in range(L)]
+    ctx.rollback(seqs, lens)
+    other = ctx.seq_create()                       # a step of other rows in between: what a stale upload would hold
+    ctx.step_begin([other])
+    ctx.step_append(0, kv[0, :1].contiguous())
+    ctx.step_end()
+    for s, n in zip(seqs, lens):
+        for l in range(L):
+            ctx.write_rows(l, s, n, torch.zeros((1, 576), dtype=torch.int16, device="cuda"))
+    torch.cuda.synchronize()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    ctx.step_begin(seqs)
+    a.wait_stream(torch.cuda.current_stream())
+    b.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(a):
+        torch.cuda._sleep(100_000_000)             # about 50 ms
+        ctx.step_append(0, kv[0])
+    with torch.cuda.stream(b):
+        ctx.step_append(1, kv[1])
+    b.synchronize()
+    assert not a.query()                           # layer 1 did not wait for layer 0's stream
+    a.synchronize()
+    ctx.step_append(2, kv[2])
+    ctx.step_end()
+    assert ctx.status() == 0
+    for l in range(L):
+        for i, (s, n) in enumerate(zip(seqs, lens)):
+            assert np.array_equal(ctx.read_rows(l, s, n, 1), want[l][i]), (l, i)
+    ctx.close()
+
+
+@pytest.mark.parametrize("how", ["layers", "calls"])
+def test_the_calls_of_an_open_step_can_be_captured(torch, how):
+    """step_begin uploads; the calls behind it are launches alone, also inside a stream capture.  The graph is replayed over other
+    inputs and after later steps have used the upload ring, and must give what the direct calls give."""
+    ctx, seqs, lens, kv, q = _step_ctx(torch, H=128, dt=synth.DT_BF16, lens=(100, 700, 64))
+    L, B = kv.shape[:2]
+    out, want = (torch.zeros((L, B, 128, 128), dtype=torch.int16, device="cuda") for _ in range(2))
+
+    def calls(o):
+        if how == "layers":
+            ctx.step_layers(0, L, kv, q, o)
+        for l in range(L if how == "calls" else 0):
+            ctx.step_append(l, kv[l])
+            ctx.step_attend(l, q[l], o[l])
+
+    for _ in range(20):                            # the ring goes round; kernels are loaded
+        ctx.step_begin(seqs)
+        calls(want)
+        ctx.step_end()
+        ctx.rollback(seqs, lens)
+    torch.cuda.synchronize()
+    ctx.step_begin(seqs)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        calls(out)
+    q.copy_(torch.flip(q, (1,)))
+    g.replay()
+    calls(want)
+    torch.cuda.synchronize()
+    for l in range(L):
+        check_close(_host(out[l]), _host(want[l]), synth.DT_BF16, f"layer {l}")
+    ctx.step_end()
+    ctx.rollback(seqs, lens)
+    for _ in range(10):
+        ctx.step_begin(seqs)
+        calls(want)
+        ctx.step_end()
+        ctx.rollback(seqs, lens)
+    assert ctx.status() == 0
+    del g
+    ctx.close()
