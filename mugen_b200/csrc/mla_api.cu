@@ -577,6 +577,24 @@ int grow_buf(mla_ctx* c, void** p, size_t* cap, size_t bytes)
     return MLA_OK;
 }
 
+// partial tiles and counters of the projections: contexts that register no block and take no prompt chunk have none
+int ensure_gemm_workspace(mla_ctx* c)
+{
+    mla::GemmWorkspace& w = c->gemm_ws;
+    if (w.counters) return MLA_OK;
+    w.blocks = uint32_t(c->sm_count);
+    w.max_tiles = 16 * w.blocks;
+    if (!w.partial) CU_TRY(c, cudaMalloc(&w.partial, mla::gemm_tc5_partial_bytes(w.blocks)));
+    uint32_t* counters = nullptr;
+    CU_TRY(c, cudaMalloc(&counters, w.max_tiles * 4));
+    cudaError_t e = cudaMemset(counters, 0, w.max_tiles * 4);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();       // the launches that count on zeros are on other streams
+    if (e != cudaSuccess) cudaFree(counters);
+    CU_TRY(c, e);
+    w.counters = counters;
+    return MLA_OK;
+}
+
 mla::GemmWeight gemm_weight(const mla::GemmWeightMaps& maps, uint32_t n_outputs, void* out, uint32_t row0 = 0)
 {
     return mla::GemmWeight{&maps.box128, &maps.box64, row0, n_outputs, out};
@@ -589,6 +607,7 @@ int run_chunks(mla_ctx* c, uint32_t layer, const void* q, void* out, cudaStream_
 {
     const uint32_t H = c->cfg.n_heads;
     const int dt = int(c->cfg.dtype);
+    if (int e = ensure_gemm_workspace(c)) return e;
     for (const auto& g : c->chunk_groups) {
         if (int e = grow_buf(c, &c->pf_kx, &c->pf_kx_cap, size_t(g.rows) * H * mla::kNope * 2)) return e;
         if (int e = grow_buf(c, &c->pf_vx, &c->pf_vx_cap, size_t(g.rows) * H * mla::kVDim * 2)) return e;
@@ -786,20 +805,8 @@ int mla_create(const mla_config* cfg, mla_ctx** out)
     const uint64_t row_bytes = uint64_t(H) * mla::kRow * 2;
     c->ws_rows = std::max<uint32_t>(c->cfg.max_rows, uint32_t(std::min<uint64_t>({uint64_t(c->cfg.max_rows) * cfg->n_layers, kGroupRows,
                                                                                   std::max<uint64_t>(1, kGroupBytes / row_bytes)})));
-    // 64 spare rows: the tcgen05 kernel fetches queries in boxes of 64 head rows
-    CR_TRY(cudaMalloc(&c->q_abs, (size_t(c->ws_rows) * H + 64) * mla::kRow * 2));
-    CR_TRY(cudaMemset(c->q_abs, 0, (size_t(c->ws_rows) * H + 64) * mla::kRow * 2));
-    // a plan has at most one segment per query group more than it has workers, each of up to group_heads (or H) records
-    c->rec_cap = (size_t(workers_of(cp, c->kernel, H)) + c->ws_rows) * H;
-    if (group_heads(cp) >= 2 * H) c->rec_cap += size_t(c->sm_count) * group_heads(cp) + size_t(c->ws_rows) * H;
-    CR_TRY(cudaMalloc(&c->recs, c->rec_cap * mla::kPart * sizeof(float)));
     CR_TRY(cudaMalloc(&c->status_dev, sizeof(uint32_t)));
     CR_TRY(cudaMemset(c->status_dev, 0, sizeof(uint32_t)));
-    c->gemm_ws.blocks = uint32_t(c->sm_count);
-    c->gemm_ws.max_tiles = 16 * c->gemm_ws.blocks;
-    CR_TRY(cudaMalloc(&c->gemm_ws.partial, mla::gemm_tc5_partial_bytes(c->gemm_ws.blocks)));
-    CR_TRY(cudaMalloc(&c->gemm_ws.counters, c->gemm_ws.max_tiles * 4));
-    CR_TRY(cudaMemset(c->gemm_ws.counters, 0, c->gemm_ws.max_tiles * 4));
     c->meta_cap = meta_capacity(cp);
     CR_TRY(cudaMalloc(&c->meta_dev, kPlanRegions * c->meta_cap));
     CR_TRY(cudaMallocHost(&c->meta_host, kMetaRing * c->meta_cap));
@@ -832,6 +839,24 @@ int mla_create(const mla_config* cfg, mla_ctx** out)
         cp->err = std::string("tcgen05 merge kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));
         return bail(MLA_ERR_CUDA);
     }
+    // The last allocations.  Where the device is too full for groups of layers and of rows, one layer of max_rows rows must do:
+    // steps then go layer by layer, and rows of one sequence share a stream of its pages as far as the records hold them.
+    auto workspace = [&](uint32_t rows, bool groups) -> cudaError_t {
+        c->ws_rows = rows;
+        // a plan has at most one segment per query group more than it has workers, each of up to group_heads (or H) records
+        c->rec_cap = (size_t(workers_of(cp, c->kernel, H)) + rows) * H;
+        if (groups && group_heads(cp) >= 2 * H) c->rec_cap += size_t(c->sm_count) * group_heads(cp) + size_t(rows) * H;
+        // 64 spare rows: the tcgen05 kernels fetch queries in boxes of 64 head rows
+        const size_t q_bytes = (size_t(rows) * H + 64) * mla::kRow * 2;
+        cudaError_t e = cudaMalloc(&c->q_abs, q_bytes);
+        if (e == cudaSuccess) e = cudaMalloc(&c->recs, c->rec_cap * mla::kPart * sizeof(float));
+        if (e == cudaSuccess) return cudaMemset(c->q_abs, 0, q_bytes);
+        cudaGetLastError();
+        cudaFree(c->q_abs);
+        c->q_abs = nullptr;
+        return e;
+    };
+    if (workspace(c->ws_rows, true) == cudaErrorMemoryAllocation) CR_TRY(workspace(c->cfg.max_rows, false));
     if (int rc = make_tensor_maps(cp)) return bail(rc);
     if (int ce = mla::decode_tc5_pair128_configure()) {
         cp->err = std::string("tcgen05 pair128 kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));
@@ -892,7 +917,7 @@ int mla_status(mla_ctx* c, void* stream, uint32_t* device_status)
     if (v) {
         CU_TRY(c, cudaMemsetAsync(c->status_dev, 0, 4, st));
         // a projection that gave up in the middle may have left tile counters behind
-        CU_TRY(c, cudaMemsetAsync(c->gemm_ws.counters, 0, c->gemm_ws.max_tiles * 4, st));
+        if (c->gemm_ws.counters) CU_TRY(c, cudaMemsetAsync(c->gemm_ws.counters, 0, c->gemm_ws.max_tiles * 4, st));
     }
     *device_status = v;
     if (v) return fail(c, MLA_ERR_DEVICE, "device status word = " + std::to_string(v));
@@ -1549,16 +1574,24 @@ int mla_set_block_weights(mla_ctx* c, uint32_t layer, const mla_block_weights* w
         CU_TRY(c, cudaMemcpy(*dst, src, n * 2, cudaMemcpyHostToDevice));
         return MLA_OK;
     };
-    // matrices are staged row-major and repacked into tiles on the device
+    if (int e = ensure_gemm_workspace(c)) return e;
+    // matrices are staged row-major, a run of 128-row tiles at a time, and repacked on the device
     void* stage = nullptr;
-    const size_t stage_values = std::max({size_t(R) * E, R ? size_t(QD) * R : size_t(QD) * E, size_t(mla::kRow) * E, size_t(E) * VD});
-    CU_TRY(c, cudaMalloc(&stage, stage_values * 2));
+    constexpr size_t kStageBytes = 32ull << 20;
+    auto stage_rows = [&](uint32_t K) { return uint32_t(std::max<size_t>(1, kStageBytes / (size_t(K) * 2 * 128)) * 128); };
+    auto stage_bytes = [&](uint32_t N, uint32_t K) { return size_t(std::min(N, stage_rows(K))) * K * 2; };
+    CU_TRY(c, cudaMalloc(&stage, std::max({R ? stage_bytes(R, E) : 0, R ? stage_bytes(QD, R) : stage_bytes(QD, E), stage_bytes(uint32_t(mla::kRow), E),
+                                           stage_bytes(E, VD)})));
     auto put_matrix = [&](void** dst, mla::GemmWeightMaps* maps, const void* src, uint32_t N, uint32_t K) -> int {
         if (*dst) { cudaFree(*dst); *dst = nullptr; }
         if (!src) return MLA_OK;
         CU_TRY(c, cudaMalloc(dst, mla::gemm_tc5_packed_values(N, K) * 2));
-        CU_TRY(c, cudaMemcpy(stage, src, size_t(N) * K * 2, cudaMemcpyHostToDevice));
-        if (int rc = mla::launch_gemm_pack(stage, *dst, N, K, nullptr)) return fail(c, MLA_ERR_CUDA, std::string("weight packing: ") + cudaGetErrorString(cudaError_t(rc)));
+        for (uint32_t r0 = 0, n; r0 < N; r0 += n) {
+            n = std::min(N - r0, stage_rows(K));
+            CU_TRY(c, cudaMemcpy(stage, static_cast<const char*>(src) + size_t(r0) * K * 2, size_t(n) * K * 2, cudaMemcpyHostToDevice));
+            if (int rc = mla::launch_gemm_pack(stage, static_cast<char*>(*dst) + mla::gemm_tc5_packed_values(r0, K) * 2, n, K, nullptr))
+                return fail(c, MLA_ERR_CUDA, std::string("weight packing: ") + cudaGetErrorString(cudaError_t(rc)));
+        }
         if (!mla::gemm_tc5_packed_maps(maps, int(c->cfg.dtype), *dst, N, K)) return fail(c, MLA_ERR_CUDA, "cuTensorMapEncodeTiled(projection weights) failed");
         return MLA_OK;
     };

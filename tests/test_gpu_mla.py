@@ -1065,3 +1065,53 @@ def test_the_calls_of_an_open_step_can_be_captured(torch, how):
     assert ctx.status() == 0
     del g
     ctx.close()
+
+
+def test_a_context_on_a_device_with_little_room_left(torch, oracle):
+    """The workspace for groups of layers is a matter of speed: where it does not fit any more the context is created without it,
+    and its steps give the same."""
+    from mugen_b200.mla import MlaContext
+    H, dt, L, lens = 16, synth.DT_F16, 27, [200, 65]
+    case = synth.make_layer_case(31, H, [n + 1 for n in lens], dt)
+    make = lambda: MlaContext(n_layers=L, n_heads=H, dtype=dt, n_pages=16, max_seqs=2, max_seq_len=256, max_rows=10, **YARN)
+    make().close()                                         # what the process itself allocates is there
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free0 = torch.cuda.mem_get_info()[0]
+    ctx = make()
+    need = free0 - torch.cuda.mem_get_info()[0]
+    ctx.close()
+    # records: 148 workers x 128 head rows more than one layer's rows need, and 27 x 10 rows instead of 10; half of it is missing
+    extra = 148 * 128 * 514 * 4
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - need + extra // 2, dtype=torch.uint8, device="cuda")
+    try:
+        ctx = make()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    for l in range(L):
+        ctx.set_layer_weights(l, case.w_uk, case.w_uv, case.w_type, case.norm_w)
+    seqs = []
+    for b, n in enumerate(lens):
+        s = ctx.seq_create()
+        for l in range(L):
+            ctx.write_rows(l, s, 0, _dev(torch, case.caches[b][:n]))
+        ctx.advance_seq_len(s, n)
+        seqs.append(s)
+    rng = np.random.default_rng(2)
+    kv = synth.to_bits(rng.standard_normal((L, 10, 576), np.float32), dt)          # five new tokens each
+    q = synth.to_bits(rng.standard_normal((L, 10, H, 192), np.float32) * np.float32(0.9), dt)
+    out = torch.zeros((L, 10, H, 128), dtype=torch.int16, device="cuda")
+    before = ctx.launch_count()
+    ctx.step_begin(seqs, [5, 5])
+    ctx.step_layers(0, L, _dev(torch, kv), _dev(torch, q), out)
+    ctx.step_end()
+    assert ctx.status() == 0 and ctx.launch_count() - before == 3 * L          # layer by layer
+    for l in (0, L - 1):
+        for b, n in enumerate(lens):
+            rows = oracle.append_rows(kv[l, 5 * b:5 * b + 5], list(range(n, n + 5)), case.norm_w, YARN["rms_norm_eps"], 40.0, 4096, 10000.0, dt)
+            cache = np.concatenate([case.caches[b][:n], rows])
+            for t in range(5):
+                want = oracle.attention(q[l, 5 * b + t], cache, n + t + 1, case.w_uk, case.w_uv, case.w_type, H, dt)
+                check_close(_host(out[l, 5 * b + t]), want, dt, f"layer {l}, sequence {b}, token {t}")
+    ctx.close()
