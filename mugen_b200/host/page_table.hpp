@@ -278,7 +278,12 @@ inline void plan_min_makespan(const std::vector<uint32_t>& attend_lens, uint32_t
         }
         return used;
     };
-    uint64_t lo = 1, hi = total + uint64_t(seg_overhead) * (rows + workers) + 1;
+    // Every row costs at least one segment; and a worker closes at T - seg_overhead or above, there are at most rows + workers
+    // segments, so `hi` holds everything.  (Bounds this close matter for a step of thousands of rows: 20 pours are 4.)
+    uint64_t live = 0;
+    for (uint32_t u : units) live += u > 0;
+    uint64_t lo = std::max<uint64_t>(1, (total + seg_overhead * live + workers - 1) / workers);
+    uint64_t hi = (total + seg_overhead * (live + workers) + workers - 1) / workers + seg_overhead + 1;
     while (lo < hi) {
         const uint64_t mid = (lo + hi) / 2;
         if (pour(mid, false) <= workers) hi = mid; else lo = mid + 1;

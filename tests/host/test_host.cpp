@@ -166,6 +166,28 @@ static void test_planner()
             CHECK(cost_of(s2, w2, 4) <= cost_of(s1, w1, 4));
         }
     }
+    // the bounds of the search hold the answer: never more workers than there are, and one unit less would need more
+    uint32_t rnd = 7;
+    auto next_rnd = [&](uint32_t n) { rnd = rnd * 1664525u + 1013904223u; return (rnd >> 8) % n; };
+    for (int rep = 0; rep < 2000; rep++) {
+        std::vector<uint32_t> ls(1 + next_rnd(60));
+        const uint32_t top = 1u << (1 + next_rnd(17)), workers = 1 + next_rnd(200), granule = 1 + next_rnd(2), price = next_rnd(5);
+        for (auto& l : ls) l = next_rnd(4) ? next_rnd(top) : top;
+        std::vector<Segment> s2;
+        std::vector<uint32_t> r2, w2;
+        plan_min_makespan(ls, 64, workers, s2, r2, w2, granule, price);
+        CHECK(w2.size() <= workers + 1u);
+        uint64_t worst = 0, work = 0;
+        for (size_t w = 0; w + 1 < w2.size(); w++) {
+            uint64_t load = 0;
+            for (uint32_t g = w2[w]; g < w2[w + 1]; g++)
+                if (const uint32_t n = s2[g].page_end - s2[g].page_begin) load += price + (n + granule - 1) / granule;
+            worst = std::max(worst, load);
+            work += load;
+        }
+        CHECK(worst * std::min<uint64_t>(workers, std::max<uint64_t>(work, 1)) >= work);
+        CHECK(worst <= (work + (workers - 1)) / workers + 2 * price + 2);                // greedy: every worker but the last is full
+    }
     {   // 8 rows of 128 tiles over 74 workers: nobody gets two segments for the price of one
         std::vector<Segment> s2;
         std::vector<uint32_t> r2, w2;
