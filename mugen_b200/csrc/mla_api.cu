@@ -1190,11 +1190,14 @@ int mla_step_layers(mla_ctx* c, uint32_t layer_begin, uint32_t n_layers, const v
     if (group > 1) {
         const uint32_t n_groups = (n_layers + group - 1) / group;
         group = (n_layers + n_groups - 1) / n_groups;
+        // both plans go up ahead of the first launch: a copy between two launches ends their overlap
+        auto plan_of = [&](uint32_t n) -> Plan& { return n == group ? c->stack : c->stack_tail; };
+        for (uint32_t n : {group, n_layers % group})
+            if (Plan& p = plan_of(n); n && (!p.ready || p.m.layers != n))
+                if (int e = build_plan(c, p, n == group ? kPlanStack : kPlanStackTail, c->step_seqs, c->rows, nullptr, nullptr, n, st)) return e;
         for (uint32_t i = 0; i < n_layers; i += group) {
             const uint32_t n = std::min(group, n_layers - i);
-            Plan& p = n == group ? c->stack : c->stack_tail;
-            if (!p.ready || p.m.layers != n)
-                if (int e = build_plan(c, p, n == group ? kPlanStack : kPlanStackTail, c->step_seqs, c->rows, nullptr, nullptr, n, st)) return e;
+            Plan& p = plan_of(n);
             if (int e = run_attend(c, layer_begin + i, static_cast<const char*>(q) + i * q_b, static_cast<char*>(out) + i * o_b, nullptr, p, st,
                                    static_cast<const char*>(kv_a) + i * kv_b, i > 0))
                 return e;

@@ -657,8 +657,10 @@ cudaError_t configure_type()
 
 // Tile width and run length of a launch: the shortest estimate, in SM cycles, of whole tiles against equal runs with cut
 // tiles.  A k-block of a pair takes 820 (256 outputs) or 610 (128) cycles at the L2 feed rate, one of gemm_rows_kernel
-// about 400 at the HBM rate; cutting tiles adds the hand-over (about 4000 cycles: partial out, counter, partials in) and
-// about 50 cycles per column.
+// about 400 at the HBM rate.  Cutting tiles adds the hand-over (partial out, counter, partials in): in gemm_rows_kernel about
+// 4000 cycles and 50 per column; in a pair 190 per column, 13 and 26 us, fitted to whole and cut runs of both widths over 8
+// weights x 9 row counts (N = K = 2048, 129 to 512 rows: whole tiles 15 us, cut 22 to 25; N = 2048, K = 8192, 400 rows: cut
+// 128-wide tiles 34, whole 46, cut 256-wide 43).
 struct Shape { uint32_t nt, m_tiles, n_tiles[2], run; };
 Shape pick_shape(const GemmCall& g, bool rows_kernel, uint32_t kb, const GemmWorkspace& ws)
 {
@@ -670,7 +672,7 @@ Shape pick_shape(const GemmCall& g, bool rows_kernel, uint32_t kb, const GemmWor
         for (int i = 0; i < g.n_weights; i++) s.n_tiles[i] = (g.w[i].N + n_side - 1) / n_side;
         const uint64_t tiles = uint64_t(s.m_tiles) * (s.n_tiles[0] + s.n_tiles[1]);
         const uint64_t per = (tiles + workers - 1) / workers, whole = per * kb * cyc;
-        const uint64_t run = (tiles * kb + workers - 1) / workers, cut = run * cyc + 4000 + 50 * nt;
+        const uint64_t run = (tiles * kb + workers - 1) / workers, cut = run * cyc + (rows_kernel ? 4000 + 50 * nt : 190 * nt);
         s.run = uint32_t(per * kb);
         if (whole < best_cost) { best_cost = whole; best = s; }
         s.run = uint32_t(std::max<uint64_t>(run, 2));
