@@ -41,11 +41,11 @@ constexpr int RED_WARPS = 16;
 // A tcgen05.mma costs its issuing warp about a hundred cycles whatever its size, and a tile takes 64 of them (hi and lo).  With
 // few rows that is longer than the tile's loads: four issuers take two sub-tiles each into accumulators of their own, which the
 // epilogue adds in a fixed order (27 blocks of 16 heads x 4 rows: 996 -> 970 us with the absorb's issuers).  With more than 8
-// rows (G = 1) the reduction is what takes long and needs the registers: one issuer there (four: 80 rows x 16 heads x 27 layers
-// 385 -> 392 us).
+// rows (G = 1) the reduction takes longer and needs the registers: two issuers there (3 layers x 128 heads x 128 sequences of 64
+// tokens: one 218 us, two 205, four 244 with 160 bytes of spills; 2 layers x 128 heads x 128 verify rows: 305, 297, 324).
 template <int G>
 struct Roles {        // warps: W producer, MMA issuers, 4 epilogue, then the reduction
-    static constexpr int ISSUERS = G == 1 ? 1 : 4, FIRST_EPI = 1 + ISSUERS, FIRST_RED = FIRST_EPI + 4, THREADS = 32 * (FIRST_RED + RED_WARPS);
+    static constexpr int ISSUERS = G == 1 ? 2 : 4, FIRST_EPI = 1 + ISSUERS, FIRST_RED = FIRST_EPI + 4, THREADS = 32 * (FIRST_RED + RED_WARPS);
     static constexpr uint32_t TMEM_COLS = 2 * ISSUERS * MT;
 };
 
@@ -241,9 +241,10 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
 #pragma unroll
                         for (int k = 0; k < MT; k++) v[k] += __uint_as_float(o0[k]) + __uint_as_float(o1[k]);
                     } else {
+                        tc_ld16(acc + MT, o1);
                         tc_wait_ld();
 #pragma unroll
-                        for (int k = 0; k < MT; k++) v[k] = __uint_as_float(o0[k]);
+                        for (int k = 0; k < MT; k++) v[k] = __uint_as_float(o0[k]) + __uint_as_float(o1[k]);
                     }
                 }
                 tc_fence_before();
