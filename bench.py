@@ -1,11 +1,11 @@
 #!/usr/bin/env python
 """Benchmark of the MLA absorbed-attention decode path on B200.
 
-Workload (BASELINE.json configs[2], the one the headline target is quoted on): DeepSeek-V3-shaped
+Workload (the one the headline target is quoted on): DeepSeek-V3-shaped
 MLA decode — 61 layers, 128 heads, batch 64, context 16384 per sequence, bf16 paged latent cache
 (64-token pages, shuffled block tables), one token appended per sequence per step.  One "step" is
 one decode step of the whole attention stack: for every layer append(new c_kv/k_rope rows) and
-absorbed attention (q absorb -> split-KV attention -> merge -> W_UV), three kernel launches per layer
+absorbed attention (q absorb -> split-KV attention -> merge -> W_UV), three kernel launches per group of up to five layers
 through mla_step_layers (the append runs in spare blocks of the absorb launch).  Inputs are seeded synthetic
 tensors of the model's shapes; with N GPUs the batch of 64 is sharded by sequence (no collective on
 the data path), so total work is fixed ("strong" scaling).
@@ -41,13 +41,14 @@ if ROOT not in sys.path:
 from mugen_b200 import synth  # noqa: E402
 
 METRIC, UNIT = "mla_decode_tokens_per_s", "tokens/s"
-# dram__bytes_read.sum + dram__bytes_write.sum of one attention launch at the default workload, from an ncu capture.
+# dram__bytes_read.sum + dram__bytes_write.sum of ONE layer's attention at the default workload, from an ncu capture.
 # The figure belongs to one version of the kernel's source: it is reported only while that file still hashes to the
 # value below (otherwise `traffic` is null until the capture is repeated).
 NCU_TRAFFIC = {"kernel": "tcgen05-pair128", "source": "mugen_b200/csrc/mla_decode_tc5_pair2.cu",
-               "source_sha256_16": "b8d4546c35b93d5f", "bytes_per_launch": 1.2647e9}
+               "source_sha256_16": "b8d4546c35b93d5f", "bytes_per_layer": 1.2647e9}
 # The attention kernel is timed live by CUDA events inside the library on every 7th launch of the timed region
-# (7 is coprime to 61 layers, so every layer gets sampled over the steps): an event between two kernels stops
+# (61 layers are 13 launches of five layers each and a last of one; 7 is coprime to 13, so every group gets sampled over
+# the steps): an event between two kernels stops
 # the next one from becoming resident while the previous drains, and bracketing every launch would slow the
 # step that `value` reports by about 3 %.
 KERNEL_EVENT_STRIDE = 7
@@ -75,16 +76,16 @@ def parse_args():
 def workload_name(a) -> str:
     shape = (a.layers, a.heads, a.batch, a.ctx, a.dtype)
     if shape == (61, 128, 64, 16384, "bf16"):
-        tag = "deepseek-v3-shaped MLA decode (configs[2])"
+        tag = "deepseek-v3-shaped MLA decode"
     elif shape == (27, 16, 32, 8192, "f16"):
-        tag = "deepseek-v2-lite-shaped MLA decode (configs[1])"
+        tag = "deepseek-v2-lite-shaped MLA decode"
     else:
-        tag = "MLA decode (not one of BASELINE.json's configs)"
+        tag = "MLA decode (not one of the named shapes)"
     return (f"{tag}: {a.layers} layers, {a.heads} heads, batch {a.batch}, "
             f"ctx {a.ctx}, {a.dtype} paged latent cache, page 64")
 
 
-def ncu_traffic(kernel_name: str, a, seqs_on_this_gpu: int):
+def ncu_traffic(kernel_name: str, a, seqs_on_this_gpu: int, layers_per_launch: float):
     """Per-launch DRAM traffic of the attention kernel from the committed ncu capture, scaled by the sequences this
     GPU streams; None when the capture does not describe the kernel source or the workload that just ran."""
     import hashlib
@@ -95,7 +96,7 @@ def ncu_traffic(kernel_name: str, a, seqs_on_this_gpu: int):
         return None
     if h != NCU_TRAFFIC["source_sha256_16"] or kernel_name != NCU_TRAFFIC["kernel"] or (a.heads, a.ctx) != (128, 16384):
         return None
-    return NCU_TRAFFIC["bytes_per_launch"] * seqs_on_this_gpu / 64.0
+    return NCU_TRAFFIC["bytes_per_layer"] * layers_per_launch * seqs_on_this_gpu / 64.0
 
 
 def algo_bytes_layer_step(lens, H: int, n_new_rows: int | None = None) -> float:
@@ -343,7 +344,7 @@ def run_ours(a):
     ms = ev0.elapsed_time(ev1)
     ctx.profile_enable(False)
     n_attn, attn_ms = ctx.profile_read()
-    launches = ctx.launch_count() - launches0
+    launches = own_launches = ctx.launch_count() - launches0
     clk = clocks.stop() if clocks else None
     assert ctx.status() == 0, "a kernel flagged a fault during the timed region"
 
@@ -359,14 +360,16 @@ def run_ours(a):
 
     # ---- roofline of the dominant kernel (split-KV attention), this rank's launches
     peak, peak_src = measured_peak_gbs()
-    rows_per_launch = lens_sum / max(1, a.steps)                      # cache rows streamed per launch
-    algo_bytes = rows_per_launch * 576 * 2 + B * H * 576 * 2 + (rows_per_launch / 64) * 4
+    # step_layers launches groups of layers, three kernels per group: a timed launch holds so many layers in the mean
+    layers_per_launch = L * a.steps / max(1, own_launches / 3)
+    rows_per_launch = lens_sum / max(1, a.steps) * layers_per_launch  # cache rows streamed per launch
+    algo_bytes = rows_per_launch * 576 * 2 + layers_per_launch * B * H * 576 * 2 + (rows_per_launch / 64) * 4
     per_launch_s = (attn_ms * 1e-3) / max(1, n_attn)
     achieved = algo_bytes / per_launch_s / 1e9 if per_launch_s > 0 else 0.0
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": ncu_traffic(ctx.kernel_name(), a, B), "kernel": f"split-KV attention ({ctx.kernel_name()})",
+                "traffic": ncu_traffic(ctx.kernel_name(), a, B, layers_per_launch), "kernel": f"split-KV attention ({ctx.kernel_name()})",
                 "peak_source": peak_src, "algorithmic_bytes_per_launch": algo_bytes,
-                "avg_launch_us": per_launch_s * 1e6, "launches_timed": n_attn}
+                "avg_launch_us": per_launch_s * 1e6, "layers_per_launch": layers_per_launch, "launches_timed": n_attn}
     # The same launch seen from the tensor side: 2 * (576 + 512) flops per head and cached row. At 128 heads that is
     # 242 flops per cache byte, the machine's own ratio of measured matmul rate to measured copy rate, so the kernel
     # sits at the corner of the roofline and both fractions are reported.
@@ -518,42 +521,42 @@ def _decode_numbers(torch, ctx, seqs, q, kv, out, lens, H, L, peak, warmup=3, st
     B = len(lens)
     step_bytes = algo_bytes_layer_step(cur, H)
     attn_bytes = sum(cur) * 1152.0 + B * H * 576 * 2 + sum((n + 63) // 64 for n in cur) * 4.0
-    attn_us = attn_ms * 1e3 / max(1, n_attn)
+    attn_us = attn_ms * 1e3 / L                                      # of one layer: a launch holds L / n_attn of them
     w, lo, hi = ctx.step_balance()
     return {"layers": L, "ms_per_step": ms, "us_per_layer_step": ms * 1e3 / L,
             "tokens_per_s_this_many_layers": B / (ms * 1e-3),
             "layer_step_algorithmic_bytes": step_bytes, "whole_step_frac_of_measured_peak": step_bytes * L / (ms * 1e-3) / 1e9 / peak,
-            "attention_kernel": ctx.kernel_name(), "attention_kernel_us": attn_us,
+            "attention_kernel": ctx.kernel_name(), "attention_kernel_us": attn_us, "attention_layers_per_launch": L / max(1, n_attn),
             "attention_kernel_frac_of_measured_peak": attn_bytes / (attn_us * 1e-6) / 1e9 / peak if attn_us > 0 else None,
             "planner": {"workers": w, "min_pages": lo, "max_pages": hi}}
 
 
 def sub_ragged(torch, peak):
-    """BASELINE.json configs[4], decode part: 128 sequences with log-uniform lengths 256..32768 in one step."""
+    """Ragged decode rows: 128 sequences with log-uniform lengths 256..32768 in one step."""
     lens = synth.ragged_lengths(42, 128, 256, 32768)
     H, L = 128, 4
     ctx, seqs, q, kv, out = _decode_case(torch, lens, H, L, synth.DT_BF16, torch.bfloat16, 4242)
     r = _decode_numbers(torch, ctx, seqs, q, kv, out, lens, H, L, peak)
     ctx.close()
-    r.update({"workload": "configs[4] decode rows: 128 sequences, lengths log-uniform 256..32768 (seed 42), 128 heads, bf16",
+    r.update({"workload": "ragged decode rows: 128 sequences, lengths log-uniform 256..32768 (seed 42), 128 heads, bf16",
               "tokens_cached": int(sum(lens)), "tokens_per_s_61_layers_scaled": 128 / (r["us_per_layer_step"] * 61e-6)})
     return r
 
 
 def sub_v2lite(torch, peak):
-    """16 heads, 27 layers, batch 32, ctx 8192, fp16."""
+    """The V2-Lite shape: 16 heads, 27 layers, batch 32, ctx 8192, fp16."""
     H, L, B, S = 16, 27, 32, 8192
     lens = [S - 9] * B
     ctx, seqs, q, kv, out = _decode_case(torch, lens, H, L, synth.DT_F16, torch.float16, 1717)
     r = _decode_numbers(torch, ctx, seqs, q, kv, out, lens, H, L, peak)
     ctx.close()
-    r.update({"workload": "deepseek-v2-lite-shaped MLA decode (configs[1]): 27 layers, 16 heads, batch 32, ctx 8192, f16 paged latent cache",
+    r.update({"workload": "deepseek-v2-lite-shaped MLA decode: 27 layers, 16 heads, batch 32, ctx 8192, f16 paged latent cache",
               "tokens_per_s": r.pop("tokens_per_s_this_many_layers")})
     return r
 
 
 def sub_kv_range(torch, dist, world, rank, local, peak):
-    """BASELINE.json configs[3]: ONE sequence of 131072 tokens, 128 heads, bf16, cut into `world` contiguous
+    """ONE sequence of 131072 tokens, 128 heads, bf16, cut into `world` contiguous
     page-aligned KV ranges (world = 1: the control).  Per layer every rank computes the partial softmax state
     (m, l, acc[512]) of its range for the replicated query, ONE all-gather moves the states, every rank merges
     them and applies W_UV.  The tail rank appends the step's new row."""
@@ -655,7 +658,7 @@ def sub_kv_range(torch, dist, world, rank, local, peak):
     ctx.close()
     us_layer = ms * 1e3 / L
     per_gpu_bytes = (S / world) * 1152.0
-    return {"workload": f"configs[3]: one sequence, ctx {S}, 128 heads, bf16, KV range split over {world} GPU(s), {L} layers timed",
+    return {"workload": f"one sequence, ctx {S}, 128 heads, bf16, KV range split over {world} GPU(s), {L} layers timed",
             "us_per_layer_step": us_layer, "all_gather_us": ag_us,
             "all_gather_bytes_per_gpu": H * sharding.PART * 4,
             "latent_kv_gbs_per_gpu": per_gpu_bytes / (us_layer * 1e-6) / 1e9,
@@ -665,11 +668,11 @@ def sub_kv_range(torch, dist, world, rank, local, peak):
 
 
 def sub_prefill(torch, peak):
-    """BASELINE.json configs[4], chunk part: 4 sequences, each appending one 4096-token chunk in ONE step, causal
+    """Prompt chunks: 4 sequences, each appending one 4096-token chunk in ONE step, causal
     (token t attends [0, start+t+1)), at start_position 0 and 8192; 128 heads, bf16, one layer timed."""
     from mugen_b200.mla import MlaContext
     H, N, C, dt, tdt = 128, 4096, 4, synth.DT_BF16, torch.bfloat16
-    res = {"workload": "configs[4] chunks: 4 sequences x one 4096-token chunk in one step, causal, 128 heads, bf16, 1 layer"}
+    res = {"workload": "prompt chunks: 4 sequences x one 4096-token chunk in one step, causal, 128 heads, bf16, 1 layer"}
     for start in (0, 8192):
         R = N * C
         ctx = MlaContext(n_layers=1, n_heads=H, dtype=dt, n_pages=C * ((start + N) // 64 + 2) + 8, max_seqs=C,
