@@ -189,3 +189,55 @@ def test_projections_at_the_edges_of_their_tiles(torch, rows, H, E, R, shift):
     close(out, hidden.double() + (att.double() @ w["wo"].double().T).half().double(), "hidden")
     assert ctx.status() == 0
     ctx.close()
+
+
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+@pytest.mark.parametrize("rows,H,E,R,shift", [
+    (1, 5, 72, 0, 0), (16, 16, 2048, 0, 0), (17, 16, 520, 64, 4), (33, 5, 1000, 200, 0), (65, 3, 520, 0, 1), (128, 3, 2048, 0, 8),
+    (129, 16, 2048, 0, 0), (256, 5, 72, 0, 4), (257, 64, 1000, 136, 0), (700, 16, 2048, 0, 8),
+])
+def test_every_output_of_the_projections_and_nothing_beside_them(torch, rows, H, E, R, shift, dt):
+    """Element by element against float64, and the values in front of and behind each output untouched.  An output is one rounding
+    of a float sum (u = 2^-11 or 2^-8 of it) over operands that were rounded to the storage type: a normalised value or a q_a
+    that falls the other way (u of ITS magnitude, independent) moves an output by about u * |x| * |w|, here with |w| = 1 / sqrt(K)
+    and |x| near 1 by u in the mean square; six of those beside one rounding (two in the residual) hold every element."""
+    from mugen_b200.mla import MlaContext
+    tdt, code, u = (torch.float16, synth.DT_F16, 2.0 ** -11) if dt == "f16" else (torch.bfloat16, synth.DT_BF16, 2.0 ** -8)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(rows * 11 + E)
+    rn = lambda *shape, scale=1.0: (torch.randn(shape, device="cuda", generator=gen) * scale).to(tdt)
+    bits = lambda t: t.view(torch.int16).cpu().numpy().view(np.uint16)
+    eps, QD, VD, pad, mark = 1e-6, H * 192, H * 128, 256, 0x7BAD
+    ctx = MlaContext(n_layers=1, n_heads=H, dtype=code, n_pages=2, max_seqs=1, max_seq_len=64, rope_theta=1e4,
+                     rope_scaling_factor=1.0, rope_original_ctx=4096, rms_norm_eps=eps)
+    w = dict(attn_norm=1 + rn(E, scale=0.1), kv_a_mqa=rn(576, E, scale=E ** -0.5), wo=rn(E, VD, scale=VD ** -0.5))
+    w.update(dict(q_a=rn(R, E, scale=E ** -0.5), q_a_norm=1 + rn(R, scale=0.1), q_b=rn(QD, R, scale=R ** -0.5)) if R
+             else dict(q=rn(QD, E, scale=E ** -0.5)))
+    ctx.set_block_weights(0, **{k: bits(v) for k, v in w.items()})
+    whole = {}
+
+    def at(what, n_cols):
+        whole[what] = torch.full((pad + shift + rows * n_cols + pad,), mark, dtype=torch.int16, device="cuda")
+        return whole[what].view(tdt)[pad + shift:pad + shift + rows * n_cols].view(rows, n_cols)
+
+    def norm(x, g):
+        return (x.double() * torch.rsqrt((x.double() ** 2).mean(-1, keepdim=True) + eps) * g.double()).to(tdt)
+
+    def close(got, want, what, roundings=1):
+        bad = (got.double() - want).abs() > u * (roundings * want.abs() + 6)
+        assert not bad.any(), f"{what}: {int(bad.sum())} elements, the first at {bad.nonzero()[0].tolist()}"
+        buf = whole[what]
+        assert (buf[:pad + shift] == mark).all() and (buf[pad + shift + got.numel():] == mark).all(), f"{what}: written beside the output"
+
+    hidden, q, kv = rn(rows, E), at("q", QD), at("kv_a", 576)
+    ctx.block_project_in(0, hidden, q, kv)
+    x = norm(hidden, w["attn_norm"])
+    a = norm((x.double() @ w["q_a"].double().T).to(tdt), w["q_a_norm"]) if R else x
+    close(q, a.double() @ (w["q_b"] if R else w["q"]).double().T, "q")
+    close(kv, x.double() @ w["kv_a_mqa"].double().T, "kv_a")
+    att, out = rn(rows, VD), at("hidden", E)
+    out.copy_(hidden)
+    ctx.block_project_out(0, att, out)
+    close(out, hidden.double() + (att.double() @ w["wo"].double().T).to(tdt).double(), "hidden", 2)
+    assert ctx.status() == 0
+    ctx.close()
