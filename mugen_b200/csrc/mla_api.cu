@@ -565,15 +565,17 @@ int run_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, float* expo
     return MLA_OK;
 }
 
-int grow_buf(mla_ctx* c, void** p, size_t* cap, size_t bytes)
+// slack: a quarter more, for a buffer whose need grows from step to step
+int grow(mla_ctx* c, void** p, size_t* cap, size_t bytes, bool slack = false)
 {
     if (bytes <= *cap) return MLA_OK;
+    if (slack) bytes += bytes / 4;
     CU_TRY(c, cudaDeviceSynchronize());          // an earlier launch may still use the smaller buffer
     if (*p) cudaFree(*p);
     *p = nullptr;
     *cap = 0;
-    CU_TRY(c, cudaMalloc(p, bytes + bytes / 4));
-    *cap = bytes + bytes / 4;
+    CU_TRY(c, cudaMalloc(p, bytes));
+    *cap = bytes;
     return MLA_OK;
 }
 
@@ -609,8 +611,8 @@ int run_chunks(mla_ctx* c, uint32_t layer, const void* q, void* out, cudaStream_
     const int dt = int(c->cfg.dtype);
     if (int e = ensure_gemm_workspace(c)) return e;
     for (const auto& g : c->chunk_groups) {
-        if (int e = grow_buf(c, &c->pf_kx, &c->pf_kx_cap, size_t(g.rows) * H * mla::kNope * 2)) return e;
-        if (int e = grow_buf(c, &c->pf_vx, &c->pf_vx_cap, size_t(g.rows) * H * mla::kVDim * 2)) return e;
+        if (int e = grow(c, &c->pf_kx, &c->pf_kx_cap, size_t(g.rows) * H * mla::kNope * 2, true)) return e;
+        if (int e = grow(c, &c->pf_vx, &c->pf_vx_cap, size_t(g.rows) * H * mla::kVDim * 2, true)) return e;
         mla::GemmCall gc;
         gc.paged_map = &c->tmaps[mla::kMapPoolSub];
         gc.table = g.pages;
@@ -658,24 +660,9 @@ int run_layer(mla_ctx* c, uint32_t layer, const void* kv_a, const void* q, void*
     return run_attend(c, layer, q, out, nullptr, c->plan, st, kv_a, kv_a_settled);
 }
 
-using TensorMapEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                       const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                       CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// cuTensorMapEncodeTiled through the runtime's driver entry point: no link-time libcuda.
-TensorMapEncodeFn tensor_map_encoder()
-{
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess ||
-        qres != cudaDriverEntryPointSuccess)
-        return nullptr;
-    return reinterpret_cast<TensorMapEncodeFn>(fn);
-}
-
 int make_tensor_maps(mla_ctx* c)
 {
-    TensorMapEncodeFn enc = tensor_map_encoder();
+    const mla::TensorMapEncodeFn enc = mla::tensor_map_encoder();
     if (!enc) return fail(c, MLA_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
     const CUtensorMapDataType dt = c->cfg.dtype == MLA_DTYPE_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                                                  : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -691,21 +678,13 @@ int make_tensor_maps(mla_ctx* c)
     };
     {   // W_UV of all layers as [layers*H*128 outputs][512 dims], boxes of 64 dims x 128 outputs (merge), and W_UK^T as
         // [layers*H*512 d][128 i], boxes of 64 i x 128 d (absorb)
-        auto weights = [&](CUtensorMap* map, const char* what, void* basep, cuuint64_t inner, cuuint64_t outer, cuuint32_t box_rows) -> int {
-            const cuuint64_t dims[2] = {inner, outer}, strides[1] = {inner * 2};
-            const cuuint32_t box[2] = {64, box_rows};
-            const CUresult r = enc(map, dt, 2, basep, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (r != CUDA_SUCCESS)
-                return fail(c, MLA_ERR_CUDA, std::string("cuTensorMapEncodeTiled(") + what + ") failed with code " + std::to_string(int(r)));
-            return MLA_OK;
-        };
-        const cuuint64_t heads = cuuint64_t(c->cfg.n_layers) * c->cfg.n_heads;
-        if (int e = weights(&c->w_uv_map, "W_UV", c->w_uv, mla::kRank, heads * mla::kVDim, mla::kVDim)) return e;
-        if (!mla::gemm_tc5_weight_maps(&c->w_uk_rows_maps, int(c->cfg.dtype), c->w_uk_rows, heads * mla::kNope, mla::kRank) ||
-            !mla::gemm_tc5_weight_maps(&c->w_uv_maps, int(c->cfg.dtype), c->w_uv, heads * mla::kVDim, mla::kRank))
-            return fail(c, MLA_ERR_CUDA, "cuTensorMapEncodeTiled(expansion weights) failed");
-        if (int e = weights(&c->w_uk_map, "W_UK", c->w_uk, mla::kNope, heads * mla::kRank, 128)) return e;
+        const uint64_t heads = uint64_t(c->cfg.n_layers) * c->cfg.n_heads;
+        const int type = int(c->cfg.dtype);
+        if (!mla::make_matrix_map(&c->w_uv_map, type, c->w_uv, heads * mla::kVDim, mla::kRank, mla::kVDim) ||
+            !mla::make_matrix_map(&c->w_uk_map, type, c->w_uk, heads * mla::kRank, mla::kNope, 128) ||
+            !mla::gemm_tc5_weight_maps(&c->w_uk_rows_maps, type, c->w_uk_rows, heads * mla::kNope, mla::kRank) ||
+            !mla::gemm_tc5_weight_maps(&c->w_uv_maps, type, c->w_uv, heads * mla::kVDim, mla::kRank))
+            return fail(c, MLA_ERR_CUDA, "cuTensorMapEncodeTiled(W_UK, W_UV) failed");
     }
     {   // cache pool: 576 values innermost, then the token slots of a layer, then layers;
         // box = 64 values (128 B, one swizzle row) x 64 tokens (one page)
@@ -1496,18 +1475,6 @@ int mla_write_rows(mla_ctx* c, uint32_t layer, uint32_t id, uint32_t row_begin, 
 
 // ---- attention block: the projections around the op -----------------------------------------------------------
 namespace {
-
-int grow(mla_ctx* c, void** p, size_t* cap, size_t bytes)
-{
-    if (bytes <= *cap) return MLA_OK;
-    CU_TRY(c, cudaDeviceSynchronize());          // an earlier launch may still use the smaller buffer
-    if (*p) cudaFree(*p);
-    *p = nullptr;
-    *cap = 0;
-    CU_TRY(c, cudaMalloc(p, bytes));
-    *cap = bytes;
-    return MLA_OK;
-}
 
 // out_i[rows][N_i] = act[rows][K] . W_i[N_i][K]^T, rounded to the storage type; residual: added to what out holds
 int project(mla_ctx* c, const void* act, uint32_t rows, uint32_t K, std::initializer_list<mla::GemmWeight> weights, bool residual, cudaStream_t st)

@@ -53,6 +53,7 @@ constexpr int pair_stage(int nt) { return A_BYTES + nt / 2 * BK * 2; }
 constexpr int pair_stages(int nt) { return nt == 256 ? 6 : 8; }
 constexpr int pair_off_store(int nt) { return pair_stages(nt) * pair_stage(nt); }
 constexpr int pair_smem(int nt) { return pair_off_store(nt) + 2 * STORE_BYTES + MISC_BYTES + 1024; }
+static_assert(BK == 64, "the box width of make_matrix_map");
 static_assert(rows_smem(16) <= 232448 && rows_smem(128) <= 232448 && pair_smem(256) <= 232448 && pair_smem(128) <= 232448, "shared memory of one block");
 
 struct GemmArgs {
@@ -609,37 +610,6 @@ rmsnorm_rows_kernel(const T* x, const T* __restrict__ w, T* y, uint32_t N, float
         store8(yr + 8 * p, scale8(load8(xr + 8 * p, vec), load8(w + 8 * p, true)), true);
 }
 
-using TensorMapEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                       const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                       CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-TensorMapEncodeFn encoder()
-{
-    static TensorMapEncodeFn fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<TensorMapEncodeFn>(p);
-    }();
-    return fn;
-}
-
-// rows x K matrix of 16-bit values, K contiguous, row pitch ld elements: box 64 values x box_rows rows, 128-byte swizzle
-bool make_map(CUtensorMap* map, int dtype, const void* ptr, uint64_t rows, uint64_t K, uint64_t ld, uint32_t box_rows)
-{
-    TensorMapEncodeFn enc = encoder();
-    if (!enc) return false;
-    const cuuint64_t dims[2] = {K, rows};
-    const cuuint64_t strides[1] = {ld * 2};
-    const cuuint32_t box[2] = {BK, box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    return enc(map, dtype == 0 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr),
-               dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 template <typename T>
 cudaError_t configure_type()
 {
@@ -719,13 +689,13 @@ int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t*
         out[i] = static_cast<T*>(w.out);
         if (reinterpret_cast<uintptr_t>(w.out) & 15u) a.vec_io = a.tile_store = 0u;
         // storage-type output with rows that TMA can address: the epilogue stores tiles (see the kernel)
-        if (a.tile_store && !make_map(&mc[i], dtype, w.out, g.M, w.N, w.N, BM)) a.tile_store = 0u;
+        if (a.tile_store && !make_matrix_map(&mc[i], dtype, w.out, g.M, w.N, BM)) a.tile_store = 0u;
     }
     if (g.paged_map) {
         a.table = g.table;
         a.layer = g.layer;
         a.n_pages = g.n_pages;
-    } else if (!make_map(&ma, dtype, g.A, g.M, g.K, g.K, rows_kernel ? nt : BM)) return -1;
+    } else if (!make_matrix_map(&ma, dtype, g.A, g.M, g.K, rows_kernel ? nt : BM)) return -1;
     const int last = g.n_weights - 1;
     auto map_of = [&](int i) -> const CUtensorMap& { return rows_kernel || nt == 256 ? *g.w[i].map : *g.w[i].map64; };   // boxes of 128 or 64 weight rows
     const CUtensorMap &m0 = map_of(0), &m1 = map_of(last), &pa = g.paged_map ? *g.paged_map : ma;
@@ -772,7 +742,7 @@ size_t gemm_tc5_packed_values(uint64_t N, uint64_t K) { return (N + BM - 1) / BM
 bool gemm_tc5_packed_maps(GemmWeightMaps* maps, int dtype, const void* packed, uint64_t N, uint64_t K)
 {
     const uint64_t rows = gemm_tc5_packed_values(N, K) / BK;
-    return make_map(&maps->box128, dtype, packed, rows, BK, BK, 128) && make_map(&maps->box64, dtype, packed, rows, BK, BK, 64);
+    return make_matrix_map(&maps->box128, dtype, packed, rows, BK, 128) && make_matrix_map(&maps->box64, dtype, packed, rows, BK, 64);
 }
 
 // K a multiple of 8; both DEVICE
@@ -784,7 +754,7 @@ int launch_gemm_pack(const void* src, void* dst, uint32_t N, uint32_t K, cudaStr
 
 bool gemm_tc5_weight_maps(GemmWeightMaps* maps, int dtype, const void* W, uint64_t rows, uint64_t K)
 {
-    return make_map(&maps->box128, dtype, W, rows, K, K, 128) && make_map(&maps->box64, dtype, W, rows, K, K, 64);
+    return make_matrix_map(&maps->box128, dtype, W, rows, K, 128) && make_matrix_map(&maps->box64, dtype, W, rows, K, 64);
 }
 
 // Returns a cudaError_t value, or -1 when the operands cannot be addressed (pointers must be 16-byte aligned, row lengths

@@ -8,6 +8,34 @@
 
 namespace mla {
 
+// cuTensorMapEncodeTiled through the runtime's driver entry point (no link-time libcuda); nullptr where the driver has none
+using TensorMapEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                       const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                       CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+inline TensorMapEncodeFn tensor_map_encoder()
+{
+    static const TensorMapEncodeFn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return reinterpret_cast<TensorMapEncodeFn>(p);
+    }();
+    return fn;
+}
+
+// rows x cols matrix of 16-bit values (0: half, 1: bfloat16), row after row: boxes of 64 values x box_rows rows, 128-byte swizzle
+inline bool make_matrix_map(CUtensorMap* map, int dtype, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows)
+{
+    const TensorMapEncodeFn enc = tensor_map_encoder();
+    if (!enc) return false;
+    const cuuint64_t dims[2] = {cols, rows}, strides[1] = {cols * 2};
+    const cuuint32_t box[2] = {64, box_rows}, estr[2] = {1, 1};
+    return enc(map, dtype == 0 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box,
+               estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int launch_append(int dtype, const void* kv_a, void* layer_pool, uint64_t pool_slots,
                    const void* norm_w, const float* cos_sin, uint32_t cs_rows, float eps,
                    const StepMeta& m, uint32_t* status, cudaStream_t st);

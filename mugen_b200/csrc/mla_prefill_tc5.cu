@@ -399,30 +399,6 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
     }
 }
 
-using TensorMapEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                       const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                       CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-bool make_map(CUtensorMap* map, int dtype, const void* ptr, uint64_t rows, uint64_t cols, uint64_t pitch, uint32_t box_rows)
-{
-    static TensorMapEncodeFn enc = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<TensorMapEncodeFn>(p);
-    }();
-    if (!enc) return false;
-    const cuuint64_t dims[2] = {cols, rows};
-    const cuuint64_t strides[1] = {pitch * 2};
-    const cuuint32_t box[2] = {64, box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    return enc(map, dtype == 0 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr),
-               dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 }  // namespace
 
 int prefill_tc5_configure()
@@ -438,8 +414,8 @@ int launch_prefill_tc5(int dtype, const PrefillCall& p, uint32_t* status, cudaSt
     if (p.n_tiles == 0) return 0;
     if ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.out)) & 15u) return int(cudaErrorMisalignedAddress);
     alignas(64) CUtensorMap mk, mv;
-    if (!make_map(&mk, dtype, p.kx, p.rows, uint64_t(p.H) * kNope, uint64_t(p.H) * kNope, KT) ||
-        !make_map(&mv, dtype, p.vx, p.rows, uint64_t(p.H) * kVDim, uint64_t(p.H) * kVDim, KT))
+    if (!make_matrix_map(&mk, dtype, p.kx, p.rows, uint64_t(p.H) * kNope, KT) ||
+        !make_matrix_map(&mv, dtype, p.vx, p.rows, uint64_t(p.H) * kVDim, KT))
         return -1;
     const float scale_log2 = 1.4426950408889634f / sqrtf(float(kQDim));
     dim3 grid(p.n_tiles, p.H);

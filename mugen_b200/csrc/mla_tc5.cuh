@@ -248,12 +248,6 @@ __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16])
           "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
 }
-// 32 lanes x 32 bits, repeated along 8 columns: thread i writes lane i, columns 0..7
-__device__ __forceinline__ void tc_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
-}
 // 32 lanes x 32 bits, repeated along 16 columns: thread i receives lane i, columns 0..15
 __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
@@ -301,13 +295,6 @@ __device__ __forceinline__ void tc_ld16x256_x8(uint32_t taddr, uint32_t (&r)[32]
 // the same by array size
 __device__ __forceinline__ void tc_ldn(uint32_t taddr, uint32_t (&r)[16]) { tc_ld16(taddr, r); }
 __device__ __forceinline__ void tc_ldn(uint32_t taddr, uint32_t (&r)[32]) { tc_ld32(taddr, r); }
-__device__ __forceinline__ void tc_ldn(uint32_t taddr, uint32_t (&r)[64]) {
-    tc_ld32(taddr, reinterpret_cast<uint32_t (&)[32]>(r[0]));
-    tc_ld32(taddr + 32, reinterpret_cast<uint32_t (&)[32]>(r[32]));
-}
-__device__ __forceinline__ void tc_stn(uint32_t taddr, const uint32_t (&r)[8]) { tc_st8(taddr, r); }
-__device__ __forceinline__ void tc_stn(uint32_t taddr, const uint32_t (&r)[16]) { tc_st16(taddr, r); }
-__device__ __forceinline__ void tc_stn(uint32_t taddr, const uint32_t (&r)[32]) { tc_st32(taddr, r); }
 // the same shape, two blocks (16 columns): registers 4k..4k+3 as above for k = 0, 1
 __device__ __forceinline__ void tc_ld16x256_x2(uint32_t taddr, uint32_t (&r)[8]) {
     asm volatile(
