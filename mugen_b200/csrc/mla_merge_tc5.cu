@@ -54,7 +54,7 @@ struct MergeArgs {
     const RowParts* parts;              // nullptr: n_parts records per row, [part][row][head]
     uint32_t rec_stride, n_parts;
     uint32_t rows, H, layer0;
-    uint32_t r_parts, units, run;       // a head's row tiles are cut into r_parts units; units of all layers; units per block
+    uint32_t r_parts, units, run;       // a head's rows are cut into r_parts units; units of all layers; units per block
     const uint32_t* att_row;
 };
 
@@ -143,12 +143,11 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + 228);
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
 
-    const uint32_t row_tiles = (a.rows + MT - 1) / MT;
     const uint32_t u0 = blockIdx.x * a.run, u1 = min(a.units, u0 + a.run);
-    struct Unit { uint32_t li, h, rt0, rt1; };
+    struct Unit { uint32_t li, h, r0, r1; };                // rows r0 .. r1 - 1 in tiles of MT from r0
     auto unit_of = [&](uint32_t u) -> Unit {
         const uint32_t hu = u / a.r_parts, rp = u % a.r_parts;
-        return Unit{hu / a.H, hu % a.H, row_tiles * rp / a.r_parts, row_tiles * (rp + 1) / a.r_parts};
+        return Unit{hu / a.H, hu % a.H, a.rows * rp / a.r_parts, a.rows * (rp + 1) / a.r_parts};
     };
 
     grid_launch_dependents();
@@ -187,7 +186,7 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
         uint32_t n = 0, un = 0;                    // row tiles and units so far
         for (uint32_t u = u0; u < u1 && ok; u++, un++) {
             const Unit x = unit_of(u);
-            for (uint32_t rt = x.rt0; rt < x.rt1 && ok; rt++, n++) {
+            for (uint32_t r0 = x.r0; r0 < x.r1 && ok; r0 += MT, n++) {
                 const uint32_t b = n & 1, par = (n >> 1) & 1;
                 ok = mbar_wait<kPoll, true>(a_full(b), par, abort_flag, status) && mbar_wait(acc_empty(b), par ^ 1, abort_flag, status);
                 for (uint32_t i = 0; i < NSUB / ISSUERS && ok; i++) {
@@ -202,7 +201,7 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
                             tc_mma(d, da + ((k * 32) >> 4), HI, db + ((k * 32) >> 4), HI, IDESC, (i == 0 && k == 0) ? 0u : 1u);
                             tc_mma(d, da + ((k * 32) >> 4), HI, db + ((A_HALF + k * 32) >> 4), HI, IDESC, 1u);
                         }
-                        if (rt + 1 == x.rt1) tc_commit(empty(s));          // the unit's last row tile frees the weights
+                        if (r0 + MT >= x.r1) tc_commit(empty(s));          // the unit's last row tile frees the weights
                         if (i + 1 == NSUB / ISSUERS) { tc_commit(a_empty(b)); tc_commit(acc_full(b)); }
                     }
                     __syncwarp();
@@ -217,11 +216,11 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
         uint32_t n = 0;
         for (uint32_t u = u0; u < u1; u++) {
             const Unit x = unit_of(u);
-            for (uint32_t rt = x.rt0; rt < x.rt1; rt++, n++) {
-                const uint32_t b = n & 1, live = min(uint32_t(MT), a.rows - rt * MT);
+            for (uint32_t r0 = x.r0; r0 < x.r1; r0 += MT, n++) {
+                const uint32_t b = n & 1, live = min(uint32_t(MT), x.r1 - r0);
                 T* dst = out + (size_t(x.li) * a.rows * a.H + x.h) * kVDim + q4 * 32 + lane;
                 // the caller's row of column `lane`, read ahead of the wait
-                const uint32_t my_row = rt * MT + min(lane, live - 1), my_at = a.att_row ? a.att_row[my_row] : my_row;
+                const uint32_t my_row = r0 + min(lane, live - 1), my_at = a.att_row ? a.att_row[my_row] : my_row;
                 ok = ok && mbar_wait(acc_full(b), (n >> 1) & 1, abort_flag, status);
                 ok = __all_sync(0xffffffffu, ok);
                 tc_fence_after();
@@ -267,12 +266,11 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
             return RowParts{v.x, v.y, v.z, 0};
         };
         RowParts next{0, 0, 0, 0};                                 // of this warp's row in the next tile
-        auto fetch = [&](uint32_t u, uint32_t rt) {
+        auto fetch = [&](uint32_t u, uint32_t r0) {
             Unit x = unit_of(u);
-            if (rt == ~0u) rt = x.rt0;
-            else if (rt == x.rt1) { if (++u == u1) return; x = unit_of(u); rt = x.rt0; }
-            const uint32_t r = rt * MT + rw / G;
-            if (r < a.rows) next = row_parts(x.li, r);
+            if (r0 == ~0u) r0 = x.r0;
+            else if (r0 >= x.r1) { if (++u == u1) return; x = unit_of(u); r0 = x.r0; }
+            if (r0 + rw / G < x.r1) next = row_parts(x.li, r0 + rw / G);
         };
         if (u0 < u1) fetch(u0, ~0u);
         grid_dependency_wait();          // the states belong to the attention kernel
@@ -280,12 +278,12 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
         uint32_t n = 0;
         for (uint32_t u = u0; u < u1; u++) {
             const Unit x = unit_of(u);
-            for (uint32_t rt = x.rt0; rt < x.rt1; rt++, n++) {
-                const uint32_t b = n & 1, live = min(uint32_t(MT), a.rows - rt * MT);
+            for (uint32_t r0 = x.r0; r0 < x.r1; r0 += MT, n++) {
+                const uint32_t b = n & 1, live = min(uint32_t(MT), x.r1 - r0);
                 unsigned char* hi = sm + OFF_A + b * 2 * A_HALF;
                 const uint32_t rr = rw / G, dim0 = (rw % G) * (kRank / G);      // G warps x (16 / G) rows: one pass per tile
                 const RowParts rp = next;
-                fetch(u, rt + 1);
+                fetch(u, r0 + MT);
                 float acc[16 / G];
                 if (rr < live) reduce_row<16 / G, Index>(a, rp, x.h, dim0, lane, acc);
                 ok = ok && mbar_wait(a_empty(b), ((n >> 1) & 1) ^ 1, abort_flag, status);      // the MMAs of two tiles ago have read this buffer
@@ -352,11 +350,13 @@ int launch_merge_tc5(int dtype, const float* recs, const StepMeta& m, uint32_t n
 {
     if (m.rows == 0) return 0;
     const CUtensorMap* map = static_cast<const CUtensorMap*>(w_map);
-    const uint32_t heads = m.layers * H, row_tiles = (m.rows + MT - 1) / MT;
+    const uint32_t heads = m.layers * H;
     MergeArgs a{recs, n_parts ? nullptr : m.parts, n_parts ? m.rows * H : m.rec_stride, n_parts, m.rows, H, layer0, 1, 0, 0,
                 n_parts ? nullptr : m.att_row};
-    // a head's row tiles are cut while that still leaves SMs idle (the parts then read the head's weights through L2)
-    a.r_parts = std::max(1u, std::min(row_tiles, sm_count / heads));
+    // A head's rows are cut while that still leaves SMs idle (the parts then read the head's weights through L2): the reduction of
+    // the partial states is what takes the time, and a row's is the same whoever else is in its block.
+    a.r_parts = std::max(1u, std::min(m.rows, sm_count / heads));
+    const uint32_t unit_rows = (m.rows + a.r_parts - 1) / a.r_parts;
     a.units = heads * a.r_parts;
     a.run = (a.units + sm_count - 1) / sm_count;
     dim3 grid((a.units + a.run - 1) / a.run);
@@ -367,7 +367,7 @@ int launch_merge_tc5(int dtype, const float* recs, const StepMeta& m, uint32_t n
         auto go = [&](auto kernel, uint32_t threads) { return int(launch_pdl(kernel, grid, dim3(threads), SMEM_BYTES, st, *map, o, a, status)); };
         constexpr uint32_t T1 = Roles<1>::THREADS, TN = Roles<2>::THREADS;
         if (wide) return go(k_wide, T1);
-        return m.rows <= 1 ? go(k16, TN) : m.rows <= 2 ? go(k8, TN) : m.rows <= 4 ? go(k4, TN) : m.rows <= 8 ? go(k2, TN) : go(k1, T1);
+        return unit_rows <= 1 ? go(k16, TN) : unit_rows <= 2 ? go(k8, TN) : unit_rows <= 4 ? go(k4, TN) : unit_rows <= 8 ? go(k2, TN) : go(k1, T1);
     };
     auto pick = [&](auto* o) {
         using T = std::remove_pointer_t<decltype(o)>;
