@@ -586,6 +586,7 @@ int ensure_gemm_workspace(mla_ctx* c)
     if (w.counters) return MLA_OK;
     w.blocks = uint32_t(c->sm_count);
     w.max_tiles = 16 * w.blocks;
+    CU_TRY(c, cudaError_t(mla::gemm_few_tc5_clusters(w.clusters)));
     if (!w.partial) CU_TRY(c, cudaMalloc(&w.partial, mla::gemm_tc5_partial_bytes(w.blocks)));
     uint32_t* counters = nullptr;
     CU_TRY(c, cudaMalloc(&counters, w.max_tiles * 4));
@@ -1477,7 +1478,9 @@ int mla_write_rows(mla_ctx* c, uint32_t layer, uint32_t id, uint32_t row_begin, 
 namespace {
 
 // out_i[rows][N_i] = act[rows][K] . W_i[N_i][K]^T, rounded to the storage type; residual: added to what out holds
-int project(mla_ctx* c, const void* act, uint32_t rows, uint32_t K, std::initializer_list<mla::GemmWeight> weights, bool residual, cudaStream_t st)
+// norm_w: act's rows go through the RMSNorm first, by way of norm_out where the projection does not do it itself
+int project(mla_ctx* c, const void* act, uint32_t rows, uint32_t K, std::initializer_list<mla::GemmWeight> weights, bool residual, cudaStream_t st,
+            const void* norm_w = nullptr, void* norm_out = nullptr)
 {
     mla::GemmCall g;
     g.A = act;
@@ -1486,18 +1489,12 @@ int project(mla_ctx* c, const void* act, uint32_t rows, uint32_t K, std::initial
     for (const auto& w : weights) g.w[g.n_weights++] = w;
     g.packed = true;
     g.residual = residual;
-    const int rc = mla::launch_gemm_tc5(int(c->cfg.dtype), g, c->gemm_ws, c->status_dev, st);
+    g.norm_w = norm_w;
+    g.norm_out = norm_out;
+    g.eps = c->cfg.rms_norm_eps;
+    const int rc = mla::launch_gemm_tc5(int(c->cfg.dtype), g, c->gemm_ws, c->status_dev, st, &c->launches);
     if (rc == -1) return fail(c, MLA_ERR_INVALID, "projection operands must be 16-byte aligned with row lengths that are multiples of 8");
     if (rc != 0) return fail(c, MLA_ERR_CUDA, std::string("projection launch: ") + cudaGetErrorString(cudaError_t(rc)));
-    c->launches++;
-    return MLA_OK;
-}
-
-int rmsnorm(mla_ctx* c, const void* x, const void* w, void* y, uint32_t rows, uint32_t N, cudaStream_t st)
-{
-    if (int rc = mla::launch_rmsnorm_rows(int(c->cfg.dtype), x, w, y, rows, N, c->cfg.rms_norm_eps, st))
-        return fail(c, MLA_ERR_CUDA, std::string("rmsnorm launch: ") + cudaGetErrorString(cudaError_t(rc)));
-    c->launches++;
     return MLA_OK;
 }
 
@@ -1513,13 +1510,11 @@ int project_in(mla_ctx* c, const BlockW& b, uint32_t rows, const void* hidden, v
 {
     const uint32_t E = b.embed, H = c->cfg.n_heads, QD = H * uint32_t(mla::kQDim);
     if (int e = grow(c, &c->blk_hidden2, &c->blk_hidden2_cap, size_t(rows) * E * 2)) return e;
-    if (int e = rmsnorm(c, hidden, b.attn_norm, c->blk_hidden2, rows, E, st)) return e;
     const mla::GemmWeight kv = gemm_weight(b.kv_a_map, uint32_t(mla::kRow), kv_a);
-    if (!b.q_lora) return project(c, c->blk_hidden2, rows, E, {gemm_weight(b.q_map, QD, q), kv}, false, st);
+    if (!b.q_lora) return project(c, hidden, rows, E, {gemm_weight(b.q_map, QD, q), kv}, false, st, b.attn_norm, c->blk_hidden2);
     if (int e = grow(c, &c->blk_qa, &c->blk_qa_cap, size_t(rows) * b.q_lora * 2)) return e;
-    if (int e = project(c, c->blk_hidden2, rows, E, {gemm_weight(b.q_a_map, b.q_lora, c->blk_qa), kv}, false, st)) return e;
-    if (int e = rmsnorm(c, c->blk_qa, b.q_a_norm, c->blk_qa, rows, b.q_lora, st)) return e;
-    return project(c, c->blk_qa, rows, b.q_lora, {gemm_weight(b.q_b_map, QD, q)}, false, st);
+    if (int e = project(c, hidden, rows, E, {gemm_weight(b.q_a_map, b.q_lora, c->blk_qa), kv}, false, st, b.attn_norm, c->blk_hidden2)) return e;
+    return project(c, c->blk_qa, rows, b.q_lora, {gemm_weight(b.q_b_map, QD, q)}, false, st, b.q_a_norm, c->blk_qa);
 }
 
 }  // namespace

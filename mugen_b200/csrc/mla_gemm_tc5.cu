@@ -22,6 +22,7 @@
 //                    block holding 128 rows of A and half of the outputs' weight rows.  What bounds it is the L2 -> shared
 //                    memory feed (measured with one block per 128 x 256 tile: 48 KB per 4.2 MFLOP k-block, 930 TFLOP/s =
 //                    10.7 TB/s): the pair needs 32 KB for the same work.  Finished tiles leave through shared memory and TMA.
+// Calls of up to 32 rows whose tiles are few go to a kernel of their own (mla_gemm_few_tc5.cu).
 // The first stages' weight tiles are constant and requested before the grid dependency is waited for.  Projection weights are
 // kept packed (gemm_tc5_pack): tiles of 128 outputs x 64 inputs as 16 KB runs, k-block after k-block, so that a block's
 // stream of tiles is one stream of consecutive bytes; in the row-major matrix a tile is 128 pieces of 128 bytes that lie
@@ -718,6 +719,7 @@ int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t*
 
 int gemm_tc5_configure()
 {
+    if (const int e = gemm_few_tc5_configure()) return e;
     cudaError_t e = configure_type<__half>();
     if (e == cudaSuccess) e = configure_type<__nv_bfloat16>();
     return int(e);
@@ -759,9 +761,31 @@ bool gemm_tc5_weight_maps(GemmWeightMaps* maps, int dtype, const void* W, uint64
 
 // Returns a cudaError_t value, or -1 when the operands cannot be addressed (pointers must be 16-byte aligned, row lengths
 // multiples of 8).
-int launch_gemm_tc5(int dtype, const GemmCall& g, const GemmWorkspace& ws, uint32_t* status, cudaStream_t st)
+int launch_gemm_tc5(int dtype, const GemmCall& call, const GemmWorkspace& ws, uint32_t* status, cudaStream_t st, uint64_t* launched)
 {
-    if (g.M == 0 || g.n_weights == 0) return 0;
+    if (call.M == 0 || call.n_weights == 0) return 0;
+    uint64_t unused;
+    uint64_t& n = launched ? *launched : unused;
+    GemmCall g = call;
+    const bool aligned = (reinterpret_cast<uintptr_t>(g.A) & 15u) == 0;
+    // an output over the rows themselves: the kernel that normalises on the way would read what its other blocks wrote
+    bool apart = true;
+    for (int i = 0; i < g.n_weights; i++) {
+        const char *o = static_cast<const char*>(g.w[i].out), *x = static_cast<const char*>(g.A);
+        if (g.A && o < x + size_t(g.M) * g.K * 2 && x < o + size_t(g.M) * g.w[i].N * 2) apart = false;
+        if (g.w[i].N % 8) return -1;
+    }
+    if (g.A && g.K % 8 == 0 && aligned && apart)
+        if (const uint32_t cs = gemm_few_tc5_cluster(g, ws.clusters)) {
+            n++;
+            return launch_gemm_few_tc5(dtype, g, cs, status, st);
+        }
+    if (g.norm_w) {
+        if (const int e = launch_rmsnorm_rows(dtype, g.A, g.norm_w, g.norm_out, g.M, g.K, g.eps, st)) return e;
+        n++;
+        g.A = g.norm_out;
+    }
+    n++;
     return dtype == 0 ? launch_type<__half>(g, ws, dtype, status, st) : launch_type<__nv_bfloat16>(g, ws, dtype, status, st);
 }
 

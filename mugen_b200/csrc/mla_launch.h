@@ -121,13 +121,23 @@ struct GemmCall {
     GemmWeight w[2];
     bool packed = false;                       // weights in the layout of launch_gemm_pack (row0 = 0)
     bool residual = false;                     // out = T(float(out) + float(T(x)))
+    const void* norm_w = nullptr;              // not null: A's rows go through the RMSNorm with this weight first, ...
+    float eps = 0.0f;
+    void* norm_out = nullptr;                  // ... rounded to the storage type here [M][K] where the kernel does not do it itself
 };
 struct GemmWorkspace {
     float* partial;            // gemm_tc5_partial_bytes(blocks)
     uint32_t* counters;        // [max_tiles], zero before the first launch
     uint32_t blocks, max_tiles;
+    uint32_t clusters[4];      // gemm_few_tc5_clusters
 };
-int launch_gemm_tc5(int dtype, const GemmCall& g, const GemmWorkspace& ws, uint32_t* status, cudaStream_t st);
+// launched: kernels launched are added to it
+int launch_gemm_tc5(int dtype, const GemmCall& g, const GemmWorkspace& ws, uint32_t* status, cudaStream_t st, uint64_t* launched = nullptr);
+// The same for few rows and weights that fit the SMs in one go, the norm included (mla_gemm_few_tc5.cu); launch_gemm_tc5 picks.
+uint32_t gemm_few_tc5_cluster(const GemmCall& g, const uint32_t (&resident)[4]);
+int launch_gemm_few_tc5(int dtype, const GemmCall& g, uint32_t cs, uint32_t* status, cudaStream_t st);
+int gemm_few_tc5_clusters(uint32_t (&n)[4]);
+int gemm_few_tc5_configure();
 size_t gemm_tc5_partial_bytes(uint32_t blocks);
 // Projection weights repacked into tiles (see the kernel file): values of the packed form, the packing itself, its maps.
 size_t gemm_tc5_packed_values(uint64_t N, uint64_t K);

@@ -241,3 +241,51 @@ def test_every_output_of_the_projections_and_nothing_beside_them(torch, rows, H,
     close(out, hidden.double() + (att.double() @ w["wo"].double().T).to(tdt).double(), "hidden", 2)
     assert ctx.status() == 0
     ctx.close()
+
+
+@pytest.mark.parametrize("rows,H,E,R", [
+    (1, 1, 64, 0), (2, 2, 1024, 0), (3, 2, 1032, 8), (4, 5, 2048, 0), (5, 16, 4096, 512), (8, 5, 72, 64), (9, 16, 2048, 0), (16, 4, 7168, 1536),
+    (17, 2, 1024, 0), (24, 5, 520, 200), (31, 2, 4096, 136), (32, 16, 2048, 0),
+])
+def test_projections_of_few_rows_in_every_cluster_size(torch, rows, H, E, R):
+    """Clusters of 1, 2, 4 and 8 blocks per tile, shared and whole rows per warp, k-blocks that end early.  The operands of one row
+    go to no other: the rows of a call equal, bit for bit, the same rows of a call with other rows beside them, where both calls
+    have rows of the same number per warp; and every output is within the bounds of the test above."""
+    from mugen_b200.mla import MlaContext
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(rows * 13 + E)
+    rn = lambda *shape, scale=1.0: (torch.randn(shape, device="cuda", generator=gen) * scale).half()
+    bits = lambda t: t.view(torch.int16).cpu().numpy().view(np.uint16)
+    eps, u, QD, VD = 1e-6, 2.0 ** -11, H * 192, H * 128
+    ctx = MlaContext(n_layers=1, n_heads=H, dtype=synth.DT_F16, n_pages=2, max_seqs=1, max_seq_len=64, rope_theta=1e4,
+                     rope_scaling_factor=1.0, rope_original_ctx=4096, rms_norm_eps=eps)
+    w = dict(attn_norm=1 + rn(E, scale=0.1), kv_a_mqa=rn(576, E, scale=E ** -0.5), wo=rn(E, VD, scale=VD ** -0.5))
+    w.update(dict(q_a=rn(R, E, scale=E ** -0.5), q_a_norm=1 + rn(R, scale=0.1), q_b=rn(QD, R, scale=R ** -0.5)) if R
+             else dict(q=rn(QD, E, scale=E ** -0.5)))
+    ctx.set_block_weights(0, **{k: bits(v) for k, v in w.items()})
+    norm = lambda x, g: (x.double() * torch.rsqrt((x.double() ** 2).mean(-1, keepdim=True) + eps) * g.double()).half()
+
+    def run(hidden, att):
+        q, kv, out = torch.zeros((len(hidden), QD), device="cuda").half(), torch.zeros((len(hidden), 576), device="cuda").half(), hidden.clone()
+        ctx.block_project_in(0, hidden, q, kv)
+        ctx.block_project_out(0, att, out)
+        return q, kv, out
+
+    hidden, att = rn(rows, E), rn(rows, VD)
+    q, kv, out = run(hidden, att)
+    x = norm(hidden, w["attn_norm"])
+    a = norm((x.double() @ w["q_a"].double().T).half(), w["q_a_norm"]) if R else x
+    for got, want, n in ((q, a.double() @ (w["q_b"] if R else w["q"]).double().T, 1), (kv, x.double() @ w["kv_a_mqa"].double().T, 1),
+                         (out, hidden.double() + (att.double() @ w["wo"].double().T).half().double(), 2)):
+        assert not ((got.double() - want).abs() > u * (n * want.abs() + 6)).any()
+    other_hidden, other_att = rn(rows, E, scale=30.0), rn(rows, VD, scale=30.0)
+    other_hidden[rows // 2], other_att[rows // 2] = hidden[rows // 2], att[rows // 2]
+    for got, want in zip(run(other_hidden, other_att), (q, kv, out)):
+        assert torch.equal(got[rows // 2], want[rows // 2])
+    # an output over the rows themselves: they are read before it is written
+    if not R and QD <= E:
+        buf = hidden.clone()
+        ctx.block_project_in(0, buf, buf.view(-1)[:rows * QD], kv)
+        assert not ((buf.view(-1)[:rows * QD].view(rows, QD).double() - a.double() @ w["q"].double().T).abs() > u * ((a.double() @ w["q"].double().T).abs() + 6)).any()
+    assert ctx.status() == 0
+    ctx.close()
