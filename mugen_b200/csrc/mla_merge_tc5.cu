@@ -5,9 +5,12 @@
 //
 // What bounds it is W_UV (131 KB per layer and head, read once) and the partial states, so the kernel streams both:
 // persistent blocks, one per SM, each with an equal run of (layer, head) units.  W_UV_h (128 outputs x 512 dims) arrives by
-// TMA as eight sub-tiles [128 outputs][64 dims] in a ring of eight and is the M side of the MMA (tcgen05.mma M128 N16
-// K16): it stays in shared memory for all row tiles of its unit and its buffers are re-loaded for the next unit as the
-// last tile's MMAs release them.  The N side is a tile of 16 rows of o_c, split into hi = T(o) and lo = T(o - hi)
+// TMA as eight sub-tiles [128 outputs][64 dims] in a ring of eight and is the M side of the MMA (tcgen05.mma M128 N32 or
+// N16, K16): it stays in shared memory for all row tiles of its unit and its buffers are re-loaded for the next unit as the
+// last tile's MMAs release them.  The N side is a tile of 16 or 8 rows of o_c, split into hi = T(o) and lo = T(o - hi)
+// that stand side by side, so that W passes through the tensor core once for both (two MMAs per step, hi then lo, took 1.7 us
+// of a tile of 8 rows against 0.9; 27 blocks of 16 heads x 4 rows 796 -> 775 us with what follows from it, 8 layers of 128 heads x
+// 8 sequences by calls 1.5 % faster, one sequence of 131,072 tokens 1.8 %)
 // (together ~16 mantissa bits for bf16, ~22 for fp16, so the float state is not rounded to the storage type before the
 // projection), two buffers in turn: sixteen warps reduce the next tile's partial states while the tensor core works on
 // this one's.
@@ -28,25 +31,24 @@ namespace {
 
 using namespace tc5;
 
-constexpr int MT = 16;                         // rows per tile: the N side
 constexpr int W_SUB = kVDim * 128;             // 16,384: [128 outputs][64 dims]
 constexpr int NSUB = kRank / 64;               // 8
-constexpr int A_SUB = MT * 128;                // 2,048: [16 rows][64 dims]
-constexpr int A_HALF = NSUB * A_SUB;           // 16,384: hi or lo of a tile
-constexpr int OFF_A = NSUB * W_SUB;            // two buffers of hi + lo
-constexpr int OFF_MISC = OFF_A + 2 * 2 * A_HALF;
+constexpr int OFF_A = NSUB * W_SUB;            // two buffers of operand tiles: [sub-tile][hi rows, lo rows][64 dims]
+constexpr int OFF_MISC = OFF_A + 2 * NSUB * 32 * 128;
 constexpr int MISC_BYTES = 256;
 constexpr int SMEM_BYTES = OFF_MISC + MISC_BYTES + 1024;   // + slack to round the base up to 1 KB
 constexpr int RED_WARPS = 16;
-// A tcgen05.mma costs its issuing warp about a hundred cycles whatever its size, and a tile takes 64 of them (hi and lo).  With
+// A tcgen05.mma costs its issuing warp about a hundred cycles whatever its size, and a tile takes 32 of them.  With
 // few rows that is longer than the tile's loads: four issuers take two sub-tiles each into accumulators of their own, which the
 // epilogue adds in a fixed order (27 blocks of 16 heads x 4 rows: 996 -> 970 us with the absorb's issuers).  With more than 8
 // rows (G = 1) the reduction takes longer and needs the registers: two issuers there (3 layers x 128 heads x 128 sequences of 64
 // tokens: one 218 us, two 205, four 244 with 160 bytes of spills; 2 layers x 128 heads x 128 verify rows: 305, 297, 324).
 template <int G>
 struct Roles {        // warps: W producer, MMA issuers, 4 epilogue, then the reduction
+    // rows per tile; hi and lo of them side by side are the N side, so that a sub-tile of W goes through the tensor core once
+    static constexpr int MT = G == 1 ? 16 : 8, NB = 2 * MT, A_SUB = NB * 128, A_BUF = NSUB * A_SUB;
     static constexpr int ISSUERS = G == 1 ? 2 : 4, FIRST_EPI = 1 + ISSUERS, FIRST_RED = FIRST_EPI + 4, THREADS = 32 * (FIRST_RED + RED_WARPS);
-    static constexpr uint32_t TMEM_COLS = 2 * ISSUERS * MT;
+    static constexpr uint32_t TMEM_COLS = 2 * ISSUERS * NB;
 };
 
 struct MergeArgs {
@@ -125,6 +127,7 @@ template <typename T, int G, typename Index = uint32_t>
 __global__ void __launch_bounds__(Roles<G>::THREADS, 1)
 merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restrict__ out, const MergeArgs a, uint32_t* __restrict__ status)
 {
+    constexpr int MT = Roles<G>::MT, NB = Roles<G>::NB, A_SUB = Roles<G>::A_SUB, A_BUF = Roles<G>::A_BUF;
     constexpr int ISSUERS = Roles<G>::ISSUERS, FIRST_EPI = Roles<G>::FIRST_EPI, FIRST_RED = Roles<G>::FIRST_RED;
     constexpr uint32_t TMEM_COLS = Roles<G>::TMEM_COLS;
     extern __shared__ unsigned char merge_tc5_smem[];
@@ -181,7 +184,7 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
         }
     } else if (warp < FIRST_EPI) {
         const uint32_t part = warp - 1;
-        constexpr uint32_t IDESC = instr_desc(Fmt<T>::v, kVDim, MT), HI = desc_hi(1024);
+        constexpr uint32_t IDESC = instr_desc(Fmt<T>::v, kVDim, NB), HI = desc_hi(1024);
         bool ok = true;
         uint32_t n = 0, un = 0;                    // row tiles and units so far
         for (uint32_t u = u0; u < u1 && ok; u++, un++) {
@@ -190,17 +193,14 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
                 const uint32_t b = n & 1, par = (n >> 1) & 1;
                 ok = mbar_wait<kPoll, true>(a_full(b), par, abort_flag, status) && mbar_wait(acc_empty(b), par ^ 1, abort_flag, status);
                 for (uint32_t i = 0; i < NSUB / ISSUERS && ok; i++) {
-                    const uint32_t s = part * (NSUB / ISSUERS) + i, d = tmem + (b * ISSUERS + part) * MT;
+                    const uint32_t s = part * (NSUB / ISSUERS) + i, d = tmem + (b * ISSUERS + part) * NB;
                     ok = mbar_wait(full(s), un & 1, abort_flag, status);
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
-                        const uint32_t da = desc_lo(base + s * W_SUB), db = desc_lo(base + OFF_A + b * 2 * A_HALF + s * A_SUB);
+                        const uint32_t da = desc_lo(base + s * W_SUB), db = desc_lo(base + OFF_A + b * A_BUF + s * A_SUB);
 #pragma unroll
-                        for (int k = 0; k < 4; k++) {
-                            tc_mma(d, da + ((k * 32) >> 4), HI, db + ((k * 32) >> 4), HI, IDESC, (i == 0 && k == 0) ? 0u : 1u);
-                            tc_mma(d, da + ((k * 32) >> 4), HI, db + ((A_HALF + k * 32) >> 4), HI, IDESC, 1u);
-                        }
+                        for (int k = 0; k < 4; k++) tc_mma(d, da + ((k * 32) >> 4), HI, db + ((k * 32) >> 4), HI, IDESC, (i == 0 && k == 0) ? 0u : 1u);
                         if (r0 + MT >= x.r1) tc_commit(empty(s));          // the unit's last row tile frees the weights
                         if (i + 1 == NSUB / ISSUERS) { tc_commit(a_empty(b)); tc_commit(acc_full(b)); }
                     }
@@ -225,25 +225,16 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
                 ok = __all_sync(0xffffffffu, ok);
                 tc_fence_after();
                 float v[MT];
-                {
-                    const uint32_t acc = tmem + ((q4 * 32u) << 16) + b * ISSUERS * MT;
-                    uint32_t o0[MT], o1[MT];
-                    tc_ld16(acc, o0);
-                    if constexpr (ISSUERS == 4) {
-                        tc_ld16(acc + MT, o1);
+                {   // the issuers' sums over hi and lo, always in this order
+#pragma unroll
+                    for (int k = 0; k < MT; k++) v[k] = 0.0f;
+#pragma unroll 1
+                    for (int p = 0; p < ISSUERS; p++) {
+                        uint32_t o[NB];
+                        tc_ldn(tmem + ((q4 * 32u) << 16) + (b * ISSUERS + p) * NB, o);
                         tc_wait_ld();
 #pragma unroll
-                        for (int k = 0; k < MT; k++) v[k] = __uint_as_float(o0[k]) + __uint_as_float(o1[k]);
-                        tc_ld16(acc + 2 * MT, o0);
-                        tc_ld16(acc + 3 * MT, o1);
-                        tc_wait_ld();
-#pragma unroll
-                        for (int k = 0; k < MT; k++) v[k] += __uint_as_float(o0[k]) + __uint_as_float(o1[k]);
-                    } else {
-                        tc_ld16(acc + MT, o1);
-                        tc_wait_ld();
-#pragma unroll
-                        for (int k = 0; k < MT; k++) v[k] = __uint_as_float(o0[k]) + __uint_as_float(o1[k]);
+                        for (int k = 0; k < MT; k++) v[k] += __uint_as_float(o[k]) + __uint_as_float(o[MT + k]);
                     }
                 }
                 tc_fence_before();
@@ -265,34 +256,31 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
             const uint4 v = __ldg(reinterpret_cast<const uint4*>(a.parts + size_t(li) * a.rows + r));
             return RowParts{v.x, v.y, v.z, 0};
         };
-        RowParts next{0, 0, 0, 0};                                 // of this warp's row in the next tile
-        auto fetch = [&](uint32_t u, uint32_t r0) {
-            Unit x = unit_of(u);
-            if (r0 == ~0u) r0 = x.r0;
-            else if (r0 >= x.r1) { if (++u == u1) return; x = unit_of(u); r0 = x.r0; }
-            if (r0 + rw / G < x.r1) next = row_parts(x.li, r0 + rw / G);
-        };
-        if (u0 < u1) fetch(u0, ~0u);
+        // Unit, tile and parts of this warp's row come ahead of their use: the divisions of unit_of and the load would each stand
+        // between the wait and the first state.
+        const uint32_t rr = rw / G, dim0 = (rw % G) * (kRank / G);      // G warps x (16 / G) rows: one pass per tile
+        Unit x{};
+        RowParts rp{0, 0, 0, 0};
+        auto fetch = [&](const Unit& at, uint32_t r0) { if (r0 + rr < at.r1) rp = row_parts(at.li, r0 + rr); };
+        if (u0 < u1) { x = unit_of(u0); fetch(x, x.r0); }
         grid_dependency_wait();          // the states belong to the attention kernel
         bool ok = true;
         uint32_t n = 0;
         for (uint32_t u = u0; u < u1; u++) {
-            const Unit x = unit_of(u);
             for (uint32_t r0 = x.r0; r0 < x.r1; r0 += MT, n++) {
                 const uint32_t b = n & 1, live = min(uint32_t(MT), x.r1 - r0);
-                unsigned char* hi = sm + OFF_A + b * 2 * A_HALF;
-                const uint32_t rr = rw / G, dim0 = (rw % G) * (kRank / G);      // G warps x (16 / G) rows: one pass per tile
-                const RowParts rp = next;
-                fetch(u, r0 + MT);
+                unsigned char* hi = sm + OFF_A + b * A_BUF;
                 float acc[16 / G];
                 if (rr < live) reduce_row<16 / G, Index>(a, rp, x.h, dim0, lane, acc);
+                if (r0 + MT < x.r1) fetch(x, r0 + MT);
+                else if (u + 1 < u1) { const Unit y = unit_of(u + 1); fetch(y, y.r0); }
                 ok = ok && mbar_wait(a_empty(b), ((n >> 1) & 1) ^ 1, abort_flag, status);      // the MMAs of two tiles ago have read this buffer
                 if (rr < live) {
                     if constexpr (G == 16) {                       // row 0 (of one): 32 dims, half a row of a sub-tile
                         unsigned char* p = hi + (dim0 / 64) * A_SUB + (dim0 % 64 + lane) * 2;
                         const T h0 = Elem<T>::from_f32(acc[0]);
                         *reinterpret_cast<T*>(p) = h0;
-                        *reinterpret_cast<T*>(p + A_HALF) = Elem<T>::from_f32(acc[0] - Elem<T>::to_f32(h0));
+                        *reinterpret_cast<T*>(p + MT * 128) = Elem<T>::from_f32(acc[0] - Elem<T>::to_f32(h0));
                     }
                     const uint32_t so = rr * 128 + (((lane / 4) ^ (rr & 7)) << 4) + (lane % 4) * 4;
 #pragma unroll
@@ -301,12 +289,13 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
                         const T h0 = Elem<T>::from_f32(o0), h1 = Elem<T>::from_f32(o1);
                         unsigned char* p = hi + (dim0 / 64 + k) * A_SUB + so;
                         *reinterpret_cast<uint32_t*>(p) = Elem<T>::pack2(o0, o1);
-                        *reinterpret_cast<uint32_t*>(p + A_HALF) = Elem<T>::pack2(o0 - Elem<T>::to_f32(h0), o1 - Elem<T>::to_f32(h1));
+                        *reinterpret_cast<uint32_t*>(p + MT * 128) = Elem<T>::pack2(o0 - Elem<T>::to_f32(h0), o1 - Elem<T>::to_f32(h1));
                     }
                 }
                 asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                 mbar_arrive(a_full(b));
             }
+            if (u + 1 < u1) x = unit_of(u + 1);
         }
     }
     tc_fence_before();
