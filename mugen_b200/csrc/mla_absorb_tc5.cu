@@ -213,12 +213,12 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
         append(blockIdx.x * APPEND_WARPS + warp - FIRST_APPEND, a.blocks * APPEND_WARPS, app_inside, sm + off_append(NT) + (warp - FIRST_APPEND) * kAppendRowSmem);
     } else {
         // ---- query rows: q_nope -> operand rows, q_rope -> behind the absorbed dims (by the unit that has d-tile 0)
+        Unit x = unit_of(u0);                      // the divisions not behind the wait
         grid_dependency_wait();
         const uint32_t t = tid - FIRST_QUERY * 32;
         bool ok = true;
         uint32_t n = 0;
-        for (uint32_t u = u0; u < u1; u++) {
-            const Unit x = unit_of(u);
+        for (uint32_t u = u0; u < u1; u++, x = unit_of(u)) {
             const T* ql = q + size_t(x.li) * a.rows * a.H * kQDim;
             for (uint32_t rt = x.rt0; rt < x.rt1; rt++, n++) {
                 const uint32_t b = n & 1, r0 = rt * NT;

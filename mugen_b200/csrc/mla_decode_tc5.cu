@@ -128,8 +128,12 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_const
     // The first pages of the block's first segment towards L2 while the absorb launch ends (two pages fit the stages): L2 is the point of
     // coherence, so this is safe even for the page that the append is still writing.  8 layers of 64 heads x 16
     // sequences, one launch series each: 375 -> 365 us.
+    // The first segment's descriptor is read here too, not behind the wait (the step's metadata was uploaded ahead of its first kernel).
+    SegInfo seg0{};
+    if (seg_begin < seg_end) seg0 = load_seg(m, seg_begin);
+    auto seg_info = [&](uint32_t seg) -> SegInfo { return seg == seg_begin ? seg0 : load_seg(m, seg); };
     if (warp == 0 && lane == 0 && seg_begin < seg_end) {
-        const SegInfo s = load_seg(m, seg_begin);
+        const SegInfo& s = seg0;
         for (uint32_t j = 0; j < min(2u, s.n_tiles); j++) {
             const uint32_t page = m.tables[s.tbl + j];
             if (page < n_pages) bulk_prefetch_l2(pool + (size_t(layer0 + s.layer) * n_pages + page) * (kPage * kRow * 2), kPage * kRow * 2);
@@ -145,7 +149,7 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_const
             uint32_t t = 0, nseg = 0;
             bool ok = true;
             for (uint32_t seg = seg_begin; seg < seg_end && ok; seg++) {
-                const SegInfo s = load_seg(m, seg);
+                const SegInfo s = seg_info(seg);
                 if (s.n_tiles == 0 || s.heads <= h0) continue;
                 // Q' of this row's head group: 9 boxes of [64 heads][64 dims]
                 ok = mbar_wait(bar(B_QEMPTY), (nseg & 1) ^ 1, abort_flag, status);
@@ -192,7 +196,7 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_const
         uint32_t t = 0, nseg = 0;
         bool ok = true;
         for (uint32_t seg = seg_begin; seg < seg_end && ok; seg++) {
-            const SegInfo s = load_seg(m, seg);
+            const SegInfo s = seg_info(seg);
             if (s.n_tiles == 0 || s.heads <= h0) continue;
             if (is_qk) ok = mbar_wait(bar(B_QFULL), nseg & 1, abort_flag, status);
             for (uint32_t j = 0; j < s.n_tiles && ok; j++, t++) {
@@ -282,7 +286,7 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_const
         };
         bool stop = false;
         for (uint32_t seg = seg_begin; seg < seg_end && !stop; seg++) {
-            const SegInfo s = load_seg(m, seg);
+            const SegInfo s = seg_info(seg);
             if (s.heads <= h0) continue;                      // a smaller group than the plan's largest: none of its rows here
             if (s.n_tiles == 0) {
                 // nothing to attend: the state of an empty range
