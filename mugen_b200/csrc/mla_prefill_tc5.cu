@@ -54,7 +54,7 @@ constexpr int SUB = KT * 128;                          // [128 queries or keys][
 constexpr int Q_BYTES = 3 * SUB;                       // 192 dims
 constexpr int STAGES = 2, K_STAGE = 3 * SUB, V_STAGE = 2 * SUB;        // K: 192 dims, V: 128 dims of KT keys
 constexpr int OFF_Q = 0, OFF_K = OFF_Q + Q_BYTES, OFF_V = OFF_K + STAGES * K_STAGE, OFF_MISC = OFF_V + STAGES * V_STAGE;
-constexpr int QP = kQDim / 2, VP = kVDim / 2;          // query dims, value dims that a thread of a group loads / stores of its row
+constexpr int VP = kVDim / 2;                          // value dims that a thread of a group normalises of its row
 // reference maximum of each row after step t: [2 step parities][128 rows]; row sums and maxima of the groups: [2][128] each
 constexpr int M_MREF = 320, M_LSUM = M_MREF + 2 * QT * 4, M_MLAST = M_LSUM + 2 * QT * 4, M_TMEM = M_MLAST + 2 * QT * 4, M_ABORT = M_TMEM + 4,
               MISC_BYTES = M_TMEM + 64;
@@ -219,45 +219,58 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
         // ===== softmax / correction / epilogue: the query row is this thread's tensor-memory lane; `part` is its group =====
         const uint32_t q4 = warp % 4, part = (warp - FIRST_SOFTMAX_WARP) / 4, r = q4 * 32 + lane;
         const uint32_t lane_base = (q4 * 32u) << 16;
-        const bool live = r < a.n_q;
         const uint32_t my_pos = a.pos + r;                               // last key this query may see
-        {   // this thread's half of the query row into the operand tiles
-            constexpr int W = QP / 6;            // part 1 holds dims 96..191, all of the rope dims among them
-            const uint4* src = reinterpret_cast<const uint4*>(q + (size_t(a.q_row + r) * H + h) * kQDim + part * QP);
-            uint32_t w[3][W];
+        {   // The query rows into the operand tiles: neighbouring lanes take neighbouring 16-byte pieces of a row.  (A thread per half row
+            // makes every load of a warp 32 cache lines of 16 bytes used, and the 32 loads of cosines and sines more of them: 6.7 us
+            // from the wait to the last query of a block, 2.4 now; with the stores at the end 27 blocks over a 777-token prompt 2020 ->
+            // 1900 us.)
+            const uint32_t st = tid - 32 * FIRST_SOFTMAX_WARP;
+            const size_t pitch = size_t(H) * kQDim;
+            const T* q0 = q + (size_t(a.q_row) * H + h) * kQDim;
+            auto put = [&](uint32_t row, uint32_t ch, const uint4& v) {          // ch: 16-byte piece of the row
+                *reinterpret_cast<uint4*>(sm + OFF_Q + (ch / 8) * SUB + row * 128 + (((ch % 8) ^ (row & 7)) << 4)) = v;
+            };
+            constexpr uint32_t NP = kNope / 8, RP = kRope / 16;                  // pieces of the plain dims, pairs of pieces of the rope dims
+            uint4 v[QT * NP / NUM_SOFTMAX], x0[QT * RP / NUM_SOFTMAX], x1[QT * RP / NUM_SOFTMAX];
 #pragma unroll
-            for (int c = 0; c < 3; c++)
-#pragma unroll
-                for (int j = 0; j < W / 4; j++) {
-                    const uint4 v = live ? __ldg(src + c * (W / 4) + j) : make_uint4(0u, 0u, 0u, 0u);
-                    w[c][4 * j] = v.x; w[c][4 * j + 1] = v.y; w[c][4 * j + 2] = v.z; w[c][4 * j + 3] = v.w;
-                }
-            if (cos_sin != nullptr && part == 1 && live) {
-                // q-side RoPE (NeoX pairs, the append's table and rounding: reference transformer.cpp:1204-1240): w[1] holds dims
-                // 128..159, w[2] their partners 160..191
-                const uint32_t pos = a.rope_pos + r;
-                if (pos >= cs_rows) {
-                    atomicOr(status, ST_BAD_SLOT);
-                } else {
-                    const float2* cp = reinterpret_cast<const float2*>(cos_sin + size_t(pos) * kRope);
-#pragma unroll
-                    for (int j = 0; j < W; j++) {
-                        const float2 cs = __ldg(cp + j), sn = __ldg(cp + 16 + j);
-                        const T *x0 = reinterpret_cast<const T*>(&w[1][j]), *x1 = reinterpret_cast<const T*>(&w[2][j]);
-                        const float a0 = Elem<T>::to_f32(x0[0]), a1 = Elem<T>::to_f32(x0[1]), b0 = Elem<T>::to_f32(x1[0]), b1 = Elem<T>::to_f32(x1[1]);
-                        w[1][j] = Elem<T>::pack2(__fsub_rn(__fmul_rn(a0, cs.x), __fmul_rn(b0, sn.x)), __fsub_rn(__fmul_rn(a1, cs.y), __fmul_rn(b1, sn.y)));
-                        w[2][j] = Elem<T>::pack2(__fadd_rn(__fmul_rn(b0, cs.x), __fmul_rn(a0, sn.x)), __fadd_rn(__fmul_rn(b1, cs.y), __fmul_rn(a1, sn.y)));
-                    }
-                }
+            for (int k = 0; k < int(QT * NP / NUM_SOFTMAX); k++) {
+                const uint32_t row = (st + k * NUM_SOFTMAX) / NP, ch = st % NP;
+                v[k] = row < a.n_q ? __ldg(reinterpret_cast<const uint4*>(q0 + row * pitch) + ch) : make_uint4(0u, 0u, 0u, 0u);
             }
 #pragma unroll
-            for (int c = 0; c < 3; c++)
+            for (int k = 0; k < int(QT * RP / NUM_SOFTMAX); k++) {
+                const uint32_t row = (st + k * NUM_SOFTMAX) / RP, ch = NP + st % RP;
+                x0[k] = row < a.n_q ? __ldg(reinterpret_cast<const uint4*>(q0 + row * pitch) + ch) : make_uint4(0u, 0u, 0u, 0u);
+                x1[k] = row < a.n_q ? __ldg(reinterpret_cast<const uint4*>(q0 + row * pitch) + ch + RP) : make_uint4(0u, 0u, 0u, 0u);
+            }
 #pragma unroll
-                for (int j = 0; j < W / 4; j++) {
-                    const uint32_t ch = part * (QP / 8) + c * (W / 4) + j;                // 16-byte piece of the row
-                    *reinterpret_cast<uint4*>(sm + OFF_Q + (ch / 8) * SUB + r * 128 + (((ch % 8) ^ (r & 7)) << 4)) =
-                        make_uint4(w[c][4 * j], w[c][4 * j + 1], w[c][4 * j + 2], w[c][4 * j + 3]);
+            for (int k = 0; k < int(QT * NP / NUM_SOFTMAX); k++) put((st + k * NUM_SOFTMAX) / NP, st % NP, v[k]);
+#pragma unroll
+            for (int k = 0; k < int(QT * RP / NUM_SOFTMAX); k++) {
+                const uint32_t row = (st + k * NUM_SOFTMAX) / RP, i = (st % RP) * 8, pos = a.rope_pos + row;
+                if (cos_sin != nullptr && row < a.n_q) {
+                    // q-side RoPE (NeoX pairs (i, i + 32), the append's table and rounding: reference transformer.cpp:1204-1240)
+                    if (pos >= cs_rows) {
+                        atomicOr(status, ST_BAD_SLOT);
+                    } else {
+                        const float4* tb = reinterpret_cast<const float4*>(cos_sin + size_t(pos) * kRope + i);
+                        const float4 c0 = __ldg(tb), c1 = __ldg(tb + 1), s0 = __ldg(tb + 8), s1 = __ldg(tb + 9);
+                        const float cs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w}, sn[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+                        const T *f0 = reinterpret_cast<const T*>(&x0[k]), *f1 = reinterpret_cast<const T*>(&x1[k]);
+                        uint32_t y0[4], y1[4];
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            const float a0 = Elem<T>::to_f32(f0[2 * j]), a1 = Elem<T>::to_f32(f0[2 * j + 1]), b0 = Elem<T>::to_f32(f1[2 * j]), b1 = Elem<T>::to_f32(f1[2 * j + 1]);
+                            y0[j] = Elem<T>::pack2(__fsub_rn(__fmul_rn(a0, cs[2 * j]), __fmul_rn(b0, sn[2 * j])), __fsub_rn(__fmul_rn(a1, cs[2 * j + 1]), __fmul_rn(b1, sn[2 * j + 1])));
+                            y1[j] = Elem<T>::pack2(__fadd_rn(__fmul_rn(b0, cs[2 * j]), __fmul_rn(a0, sn[2 * j])), __fadd_rn(__fmul_rn(b1, cs[2 * j + 1]), __fmul_rn(a1, sn[2 * j + 1])));
+                        }
+                        x0[k] = make_uint4(y0[0], y0[1], y0[2], y0[3]);
+                        x1[k] = make_uint4(y1[0], y1[1], y1[2], y1[3]);
+                    }
                 }
+                put(row, NP + st % RP, x0[k]);
+                put(row, NP + RP + st % RP, x1[k]);
+            }
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
             arrive(B_QFULL);
         }
@@ -374,19 +387,35 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
             if (ma != -INFINITY) l += lsum_s[r] * fast_ex2(ma - m_end);
             if (mb != -INFINITY) l += lsum_s[QT + r] * fast_ex2(mb - m_end);
             const float linv = l > 0.0f ? 1.0f / l : 0.0f;
-            uint4* dst = reinterpret_cast<uint4*>(out + (size_t(a.q_row + r) * H + h) * kVDim + part * VP);
+            // by way of the query tile's shared memory (its MMAs are done), so that the lanes of a warp store whole rows
+            unsigned char* box = sm + OFF_Q + r * (kVDim * 2);
 #pragma unroll 1
             for (uint32_t c = 0; c < VP / 32; c++) {
                 uint32_t o[32];
                 tc_ld32(tmem + lane_base + COL_O + part * VP + c * 32, o);
                 tc_wait_ld();
-                uint32_t w[16];
 #pragma unroll
-                for (int i = 0; i < 16; i++)
-                    w[i] = Elem<T>::pack2(__uint_as_float(o[2 * i]) * linv, __uint_as_float(o[2 * i + 1]) * linv);
+                for (int j = 0; j < 4; j++) {
+                    uint32_t w[4];
 #pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (live) dst[c * 4 + j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+                    for (int i = 0; i < 4; i++)
+                        w[i] = Elem<T>::pack2(__uint_as_float(o[8 * j + 2 * i]) * linv, __uint_as_float(o[8 * j + 2 * i + 1]) * linv);
+                    *reinterpret_cast<uint4*>(box + (((part * (VP / 8) + c * 4 + j) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+                }
+            }
+            asm volatile("barrier.cta.sync 1, %0;\n" ::"n"(NUM_SOFTMAX) : "memory");
+            constexpr uint32_t OP = kVDim / 8;                           // 16-byte pieces of an output row
+            // read again: the loop above has no registers to carry these
+            uint32_t st, q_row, n_q;
+            asm volatile("mov.u32 %0, %%tid.x;\n" : "=r"(st));
+            asm volatile("ld.global.v2.u32 {%0, %1}, [%2];\n" : "=r"(q_row), "=r"(n_q) : "l"(tiles + blockIdx.x) : "memory");
+            st -= 32 * FIRST_SOFTMAX_WARP;
+            T* dst = out + (size_t(q_row) * H + blockIdx.y) * kVDim;
+#pragma unroll
+            for (int k = 0; k < int(QT * OP / NUM_SOFTMAX); k++) {
+                const uint32_t row = (st + k * NUM_SOFTMAX) / OP, ch = st % OP;
+                if (row < n_q)
+                    reinterpret_cast<uint4*>(dst + row * size_t(H) * kVDim)[ch] = *reinterpret_cast<const uint4*>(sm + OFF_Q + row * (kVDim * 2) + ((ch ^ (row & 7)) << 4));
             }
         }
         tc_fence_before();
