@@ -140,7 +140,7 @@ __device__ __forceinline__ void epilogue_sync() { asm volatile("barrier.cta.sync
 // The epilogue threads hand a cut tile's accumulator (row r of it, NT columns, at tensor-memory address acc; a thread's share are
 // columns c0*CH .. c1*CH - 1) over: partial to global memory, then the tile's counter.  Returns true in the worker that arrived
 // last; sum_partials then gives columns c*CH.. of the whole tile.  Worker w's slots are 2w (the tile its run begins in) and
-// 2w + 1 (the one it ends in).
+// 2w + 1 (the one it ends in).  last_slot: not the one of the cut tile before.
 template <int NT, int CH, int THREADS, typename Release>
 __device__ __forceinline__ bool hand_over(const GemmArgs& a, uint32_t worker, uint32_t blocks_per_worker, uint32_t rank, uint32_t tile, uint32_t acc,
                                           uint32_t r, int c0, int c1, bool first_thread, bool ok, volatile uint32_t* last_slot, Release release)
@@ -159,16 +159,15 @@ __device__ __forceinline__ bool hand_over(const GemmArgs& a, uint32_t worker, ui
     if (first_thread) {
         const uint32_t n = (t0 + a.kb - 1) / a.run - t0 / a.run + 1;      // workers whose runs meet the tile
         uint32_t* counter = a.counters + tile * blocks_per_worker + rank;
-        __threadfence();
-        const uint32_t is_last = ok && atomicAdd(counter, 1u) == n - 1 ? 1u : 0u;
+        // releases the partials that the barrier above put behind this thread, acquires those of the workers before
+        uint32_t before = 0;
+        if (ok) asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;\n" : "=r"(before) : "l"(counter) : "memory");
+        const uint32_t is_last = ok && before == n - 1 ? 1u : 0u;
         if (is_last) *counter = 0;                                       // as the next launch expects it
-        __threadfence();
         *last_slot = is_last;
     }
     epilogue_sync<THREADS>();
-    const bool last = *last_slot != 0;
-    epilogue_sync<THREADS>();                                            // read by everyone before the next cut tile writes it
-    return last;
+    return *last_slot != 0;
 }
 template <int NT, int CH>
 __device__ __forceinline__ void sum_partials(const GemmArgs& a, uint32_t blocks_per_worker, uint32_t rank, uint32_t tile, uint32_t r, int c, float (&v)[CH])
@@ -213,7 +212,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     static_assert((2 * STAGES + 4) * 8 <= 224, "barriers overflow their area");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + OFF_MISC + 224);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + 228);
-    volatile uint32_t* last_slot = reinterpret_cast<volatile uint32_t*>(sm + OFF_MISC + 232);
+    volatile uint32_t* last_slot = reinterpret_cast<volatile uint32_t*>(sm + OFF_MISC + 232);      // two, in turn
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const uint32_t u0 = blockIdx.x * a.run, u1 = min(a.units, u0 + a.run);       // this block's run of units
 
@@ -329,7 +328,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     if (c + 1 == NT / CH) release();
                     finish(c, v);
                 }
-            } else if (hand_over<NT, CH, 128>(a, blockIdx.x, 1, 0, tile, acc, r, 0, NT / CH, r == 0, ok, last_slot, release)) {
+            } else if (hand_over<NT, CH, 128>(a, blockIdx.x, 1, 0, tile, acc, r, 0, NT / CH, r == 0, ok, last_slot + (nt & 1), release)) {
 #pragma unroll 1
                 for (int c = 0; c < NT / CH; c++) {
                     float v[CH];
@@ -368,7 +367,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     static_assert((2 * STAGES + 4) * 8 <= 224, "barriers overflow their area");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + OFF_MISC + 224);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + 228);
-    volatile uint32_t* last_slot = reinterpret_cast<volatile uint32_t*>(sm + OFF_MISC + 232);
+    volatile uint32_t* last_slot = reinterpret_cast<volatile uint32_t*>(sm + OFF_MISC + 232);      // two, in turn
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const uint32_t rank = cluster_rank(), worker = blockIdx.x / 2;               // rank 0 issues the MMAs
     // this pair's run of units; with whole tiles (stride) the units of its own tiles, counted from 0
@@ -572,7 +571,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     if (c + 2 == c_first + CHUNKS) release();
                     finish(c + 1, v, rs1);
                 }
-            } else if (hand_over<NT, CH, 32 * EPI_WARPS>(a, worker, 2, rank, tile, acc, r, c_first, c_first + CHUNKS, tid == 64, ok, last_slot, release)) {
+            } else if (hand_over<NT, CH, 32 * EPI_WARPS>(a, worker, 2, rank, tile, acc, r, c_first, c_first + CHUNKS, tid == 64, ok, last_slot + (nt & 1), release)) {
 #pragma unroll 1
                 for (int c = c_first; c < c_first + CHUNKS; c += 2) {
                     float v[CH];
