@@ -18,6 +18,7 @@
 
 #include <algorithm>
 
+#include "mla_few_ring.h"
 #include "mla_launch.h"
 #include "mla_tc5.cuh"
 
@@ -29,8 +30,8 @@ using namespace tc5;
 
 constexpr int BM = 128, BK = 64;
 constexpr int W_BYTES = BM * BK * 2;                        // 16,384: one packed tile of 128 outputs x 64 inputs
-constexpr int STAGES = 9;
-constexpr int ISSUERS = 4, ROW_WARPS = 8;                   // the row warps load and normalise the rows, and finish the tile
+constexpr int STAGES = FewRing::stages, ISSUERS = FewRing::issuers;
+constexpr int ROW_WARPS = 8;                                // the row warps load and normalise the rows, and finish the tile
 constexpr int FIRST_ROW_WARP = 1 + ISSUERS, NUM_THREADS = 32 * (FIRST_ROW_WARP + ROW_WARPS);
 constexpr int MAX_CLUSTER = 8;
 constexpr int A_BYTES = 32768;                              // operand tiles [k-block][NT rows][64 inputs]
@@ -108,8 +109,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constan
             const CUtensorMap* map = second ? &map_w1 : &map_w0;
             const int row0 = int((tn * a.kb + kb0) * BM);
             for (uint32_t i = 0; i < kbs; i++) {
-                const uint32_t s = i % STAGES;
-                ok = mbar_wait<kPoll, true>(empty(s), ((i / STAGES) & 1) ^ 1, abort_flag, status);
+                const uint32_t s = FewRing::stage(i);
+                ok = mbar_wait<kPoll, true>(empty(s), FewRing::parity(i) ^ 1, abort_flag, status);
                 if (!ok) break;
                 mbar_expect_tx(full(s), W_BYTES);
                 tma_load_2d(base + s * W_BYTES, map, full(s), 0, row0 + int(i * BM));
@@ -117,13 +118,14 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constan
             grid_dependency_wait();
         }
     } else if (warp < FIRST_ROW_WARP) {
-        // ---- issuer p takes k-blocks p, p + 4, ..
+        // ---- issuer p takes the k-blocks of its own stages (mla_few_ring.h), in order
         constexpr uint32_t IDESC = instr_desc(Fmt<T>::v, BM, NT), HI = desc_hi(1024);
         const uint32_t p = warp - 1;
         bool ok = p < kbs && mbar_wait<kPoll, true>(a_full, 0, abort_flag, status);
-        for (uint32_t i = p; i < kbs && ok; i += ISSUERS) {
-            const uint32_t s = i % STAGES;
-            ok = mbar_wait(full(s), (i / STAGES) & 1, abort_flag, status);
+        for (uint32_t i = p, next; i < kbs && ok; i = next) {
+            const uint32_t s = FewRing::stage(i);
+            next = FewRing::next(i);
+            ok = mbar_wait(full(s), FewRing::parity(i), abort_flag, status);
             if (!ok) break;
             tc_fence_after();
             if (elect_one()) {
@@ -132,7 +134,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constan
                 for (int k = 0; k < BK / 16; k++)
                     tc_mma(tmem + p * NT, da + ((k * 32) >> 4), HI, db + ((k * 32) >> 4), HI, IDESC, (i == p && k == 0) ? 0u : 1u);
                 tc_commit(empty(s));
-                if (i + ISSUERS >= kbs) tc_commit(acc_full);
+                if (next >= kbs) tc_commit(acc_full);
             }
             __syncwarp();
         }

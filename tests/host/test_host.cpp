@@ -10,6 +10,7 @@
 #include <numeric>
 
 #include "../../mugen_b200/csrc/mla_absorb_ring.h"
+#include "../../mugen_b200/csrc/mla_few_ring.h"
 #include "../../mugen_b200/host/mla_host.hpp"
 #include "../../mugen_b200/host/page_table.hpp"
 #include "../../mugen_b200/host/rope_table.hpp"
@@ -271,6 +272,69 @@ static void test_absorb_ring()
     }
 }
 
+// The same for the few-row projection kernel: one block of kbs k-blocks, requested in order, landing in any; an issuer walks
+// k-blocks p, next(p), .. on its own, and nothing holds it back but the stages' barriers.
+template <typename Next>
+static bool few_ring_holds(uint32_t kbs, uint32_t seed, Next next)
+{
+    using R = mla::FewRing;
+    const auto passes = [](uint32_t completed, uint32_t bit) { return (completed & 1) != bit; };
+    std::vector<uint32_t> full(R::stages, 0), empty(R::stages, 0), flying, released, at(R::issuers), seen(kbs, 0);
+    std::vector<int> in(R::stages, -1);
+    for (uint32_t p = 0; p < R::issuers; p++) at[p] = p;
+    uint32_t requested = 0, left = kbs;
+    while (left || !released.empty()) {
+        bool moved = false;
+        for (uint32_t tries = 0; tries < 128 && !moved; tries++) {
+            seed = seed * 1664525u + 1013904223u;
+            const uint32_t pick = seed >> 16, act = pick % (R::issuers + 3);
+            if (act == 0 && requested < kbs && passes(empty[R::stage(requested)], R::parity(requested) ^ 1)) {
+                const uint32_t s = R::stage(requested);
+                for (uint32_t f : flying) if (R::stage(f) == s) return false;
+                if (in[s] >= 0) return false;
+                flying.push_back(requested++);
+                moved = true;
+            } else if (act == 1 && !flying.empty()) {
+                const uint32_t k = (pick >> 4) % flying.size(), i = flying[k];
+                flying.erase(flying.begin() + k);
+                in[R::stage(i)] = int(i);
+                full[R::stage(i)]++;
+                moved = true;
+            } else if (act == 2 && !released.empty()) {
+                const uint32_t k = (pick >> 4) % released.size(), s = released[k];
+                released.erase(released.begin() + k);
+                in[s] = -1;
+                empty[s]++;
+                moved = true;
+            } else if (act >= 3) {
+                const uint32_t p = act - 3, i = at[p], s = R::stage(i);
+                if (i >= kbs || !passes(full[s], R::parity(i))) continue;
+                if (in[s] != int(i) || seen[i]++) return false;
+                released.push_back(s);
+                at[p] = next(i);
+                left--;
+                moved = true;
+            }
+        }
+        if (!moved) return false;
+    }
+    return flying.empty();
+}
+
+static void test_few_ring()
+{
+    using R = mla::FewRing;
+    for (uint32_t kbs = 1; kbs <= 32; kbs++)
+        for (uint32_t seed = 1; seed <= 200; seed++) CHECK(few_ring_holds(kbs, seed, R::next));
+    for (uint32_t i = 0; i < 64; i++) CHECK(R::issuer(R::next(i)) == R::issuer(i) && (i >= R::issuers || R::issuer(i) == i));
+    // k-blocks dealt out in turn hold while no stage comes round again, and do not behind that
+    const auto in_turn = [](uint32_t i) { return i + R::issuers; };
+    uint32_t broken[17] = {};
+    for (uint32_t kbs = 1; kbs <= 16; kbs++)
+        for (uint32_t seed = 1; seed <= 3000; seed++) broken[kbs] += !few_ring_holds(kbs, seed, in_turn);
+    for (uint32_t kbs = 1; kbs <= 16; kbs++) CHECK((broken[kbs] > 0) == (kbs > R::stages));
+}
+
 static void test_wrapper_without_gpu()
 {
     LatentKVCacheConfig cfg;
@@ -334,6 +398,7 @@ int main(int argc, char** argv)
         test_page_table();
         test_planner();
         test_absorb_ring();
+        test_few_ring();
         test_wrapper_without_gpu();
         std::puts("host units ok");
         return 0;

@@ -289,3 +289,66 @@ def test_projections_of_few_rows_in_every_cluster_size(torch, rows, H, E, R):
         assert not ((buf.view(-1)[:rows * QD].view(rows, QD).double() - a.double() @ w["q"].double().T).abs() > u * ((a.double() @ w["q"].double().T).abs() + 6)).any()
     assert ctx.status() == 0
     ctx.close()
+
+
+@pytest.mark.parametrize("rows,H,E,R,dt", [
+    (4, 64, 2048, 0, "bf16"),            # Wo: 16 k-blocks per block in clusters of 8
+    (16, 32, 4096, 512, "f16"),          # Wo: 16 in clusters of 4
+    (9, 16, 7168, 1536, "bf16"),         # Wo: 16 in clusters of 2; q_a and kv_a: 14 where 17 clusters of 8 are resident
+    (16, 16, 7168, 1536, "f16"),
+])
+def test_projections_of_few_rows_whose_weight_ring_comes_round(torch, rows, H, E, R, dt):
+    """10 to 16 k-blocks per block: every stage of the weight ring is used again (which issuer may then wait for it is tested on the
+    CPU, tests/host).  Six layers, launched as close as launches can follow each other, must leave the bits that the same calls leave
+    with the device idle before each; and one call's outputs are those of float64."""
+    from mugen_b200.mla import MlaContext
+    tdt, code, u = (torch.float16, synth.DT_F16, 2.0 ** -11) if dt == "f16" else (torch.bfloat16, synth.DT_BF16, 2.0 ** -8)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(rows * 17 + E)
+    rn = lambda *shape, scale=1.0: (torch.randn(shape, device="cuda", generator=gen) * scale).to(tdt)
+    bits = lambda t: t.view(torch.int16).cpu().numpy().view(np.uint16)
+    L, QD, VD, eps = 6, H * 192, H * 128, 1e-6
+    ctx = MlaContext(n_layers=L, n_heads=H, dtype=code, n_pages=2, max_seqs=1, max_seq_len=64, rope_theta=1e4,
+                     rope_scaling_factor=1.0, rope_original_ctx=4096, rms_norm_eps=eps)
+    g, ga = 1 + rn(E, scale=0.1), 1 + rn(max(R, 8), scale=0.1)
+    kv_w = [rn(576, E, scale=E ** -0.5) for _ in range(L)]
+    wo = [rn(E, VD, scale=VD ** -0.5) for _ in range(L)]
+    q_w = rn(QD, R or E, scale=(R or E) ** -0.5)
+    for l in range(L):
+        more = dict(q_a=bits(rn(R, E, scale=E ** -0.5)), q_a_norm=bits(ga), q_b=bits(q_w)) if R else dict(q=bits(q_w))
+        ctx.set_block_weights(l, attn_norm=bits(g), kv_a_mqa=bits(kv_w[l]), wo=bits(wo[l]), **more)
+    hidden, att = rn(rows, E), rn(rows, VD)
+    q, kv, out = torch.zeros((L, rows, QD), device="cuda", dtype=tdt), torch.zeros((L, rows, 576), device="cuda", dtype=tdt), hidden.clone()
+
+    def calls(between):
+        for l in range(L):
+            ctx.block_project_in(l, hidden, q[l], kv[l])
+            between()
+        for l in range(L):
+            ctx.block_project_out(l, att, out)
+            between()
+
+    calls(torch.cuda.synchronize)
+    want = [t.clone() for t in (q, kv, out)]
+    x = (hidden.double() * torch.rsqrt((hidden.double() ** 2).mean(-1, keepdim=True) + eps) * g.double()).to(tdt)
+    for l in range(L):                       # the bounds of the element-by-element test above
+        ref = x.double() @ kv_w[l].double().T
+        assert not ((kv[l].double() - ref).abs() > u * (ref.abs() + 6)).any()
+    one = hidden.clone()
+    ctx.block_project_out(0, att, one)
+    ref = hidden.double() + (att.double() @ wo[0].double().T).to(tdt).double()
+    assert not ((one.double() - ref).abs() > u * (2 * ref.abs() + 6)).any()
+    graph, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=s):
+        calls(lambda: None)
+    for _ in range(50):
+        q.zero_(), kv.zero_(), out.copy_(hidden)
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        for got, w in zip((q, kv, out), want):
+            assert torch.equal(got, w)
+    assert ctx.status() == 0
+    del graph
+    ctx.close()
