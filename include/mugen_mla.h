@@ -307,7 +307,9 @@ int mla_gguf_register(mla_ctx* ctx, mla_gguf* g, uint32_t ctx_dtype);
  * raises the ST_WAIT_TIMEOUT bit (value 4) in the context's device status word, the block frees its tensor memory
  * and returns.  This is the mechanism every kernel here uses instead of hanging or trapping; a following
  * mla_status() returns MLA_ERR_DEVICE with device_status = 4 and clears the word, and the context stays usable.
- * waited_cycles (HOST pointer, may be NULL) receives how long the block waited.  Synchronises the stream. */
+ * A second launch, a cluster of two blocks one of which never gets its share of a sum together (limit: the smaller of
+ * limit_cycles and 1,000,000), checks that neither block takes the sum for complete; MLA_ERR_DEVICE where one does.
+ * waited_cycles (HOST pointer, may be NULL) receives how long the first launch waited.  Synchronises the stream. */
 int mla_selftest_wait_timeout(mla_ctx* ctx, uint64_t limit_cycles, void* stream, uint32_t* waited_cycles);
 
 /* ---- for callers that may not allocate ------------------------------------------------------ */

@@ -1374,17 +1374,19 @@ int mla_selftest_wait_timeout(mla_ctx* c, uint64_t limit_cycles, void* stream, u
         return fail(c, MLA_ERR_INVALID, "limit_cycles must be in 1 .. 2e9 (about a second)");
     auto st = static_cast<cudaStream_t>(stream);
     uint32_t* report = nullptr;
-    CU_TRY(c, cudaMalloc(&report, 8));
+    CU_TRY(c, cudaMalloc(&report, 16));
     mla::launch_wait_timeout_selftest(static_cast<long long>(limit_cycles), c->status_dev, report, st);
-    c->launches++;
-    uint32_t host[2] = {1, 0};
+    mla::launch_lost_share_selftest(static_cast<long long>(std::min<uint64_t>(limit_cycles, 1000000)), c->status_dev, report + 2, st);
+    c->launches += 2;
+    uint32_t host[4] = {1, 0, 1, 1};
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(host, report, 8, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(host, report, 16, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     cudaFree(report);
     if (e != cudaSuccess) return fail(c, MLA_ERR_CUDA, std::string("wait-timeout self-test: ") + cudaGetErrorString(e));
     if (waited_cycles) *waited_cycles = host[1];
     if (host[0] != 0) return fail(c, MLA_ERR_DEVICE, "the self-test's wait did not give up");
+    if (host[2] != 0 || host[3] != 0) return fail(c, MLA_ERR_DEVICE, "a block of the self-test took a share that never came for complete");
     return MLA_OK;
 }
 

@@ -266,7 +266,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constan
             }
         }
         __syncwarp();
-        if (lane < a.cs) mbar_arrive_cluster(map_to_rank(red_full, lane));
+        if (lane < a.cs) announce_share(map_to_rank(red_full, lane), ok);
         __syncwarp();
         cluster_arrive();
         const bool all = mbar_wait<kSleepCluster>(red_full, 0, abort_flag, status);

@@ -173,6 +173,8 @@ int prefill_tc5_configure();
 
 // One block that waits `limit_cycles` on a barrier nothing completes, raises ST_WAIT_TIMEOUT in *status, frees its
 // tensor memory and returns; report[0] = 0 when the wait gave up, report[1] = cycles waited.
+// stored[rank] = 1 where a block of two took the sum for complete although the other one's share never came
+void launch_lost_share_selftest(long long limit_cycles, uint32_t* status, uint32_t* stored, cudaStream_t st);
 void launch_wait_timeout_selftest(long long limit_cycles, uint32_t* status, uint32_t* report, cudaStream_t st);
 
 }  // namespace mla

@@ -1,10 +1,11 @@
-// Self-test of the bounded-wait path: a one-block kernel whose threads wait on an mbarrier that
+// Self-tests of the bounded-wait path.  First a one-block kernel whose threads wait on an mbarrier that
 // nothing will ever complete.  It exercises, on purpose and in isolation, what every tcgen05 kernel
 // of this library does when a wait runs out (a lost TMA completion, a twin block that never
 // signals): the waiter gives up after `limit_cycles`, raises ST_WAIT_TIMEOUT in the status word,
 // tells the rest of the block through the abort flag, the block frees the tensor memory it holds
 // and returns normally.  The context stays usable; the host sees the failure through mla_status.
-// The product kernels' own barriers are never starved to test this.
+// The product kernels' own barriers are never starved to test this.  Then the same across a cluster: one of two blocks never gets
+// its share of a sum together, so neither may store the sum.
 #include "../../include/mugen_mla.h"
 #include "mla_launch.h"
 #include "mla_tc5.cuh"
@@ -52,7 +53,38 @@ wait_timeout_selftest_kernel(long long limit_cycles, uint32_t* __restrict__ stat
     }
 }
 
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32)
+lost_share_selftest_kernel(long long limit_cycles, uint32_t* __restrict__ status, uint32_t* __restrict__ stored)
+{
+    __shared__ __align__(8) uint64_t bar_storage[2];
+    __shared__ int abort_flag;
+    const uint32_t never = smem_u32(bar_storage), shares = never + 8, lane = threadIdx.x, rank = cluster_rank();
+    if (lane == 0) {
+        abort_flag = 0;
+        mbar_init(never, 1);               // no arrival will come
+        mbar_init(shares, 2);              // one of each block
+        mbar_init_fence();
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    bool ok = rank == 0 || mbar_wait<kPoll>(never, 0, &abort_flag, status, limit_cycles);
+    ok = __all_sync(0xffffffffu, ok);
+    if (lane < 2) announce_share(map_to_rank(shares, lane), ok);
+    __syncwarp();
+    const bool all = mbar_wait<kSleepCluster>(shares, 0, &abort_flag, status, 4 * limit_cycles);      // long enough to see a late announcement
+    ok = __all_sync(0xffffffffu, all && ok);
+    if (lane == 0) stored[rank] = ok ? 1u : 0u;
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
 }  // namespace
+
+void launch_lost_share_selftest(long long limit_cycles, uint32_t* status, uint32_t* stored, cudaStream_t st)
+{
+    lost_share_selftest_kernel<<<2, 32, 0, st>>>(limit_cycles, status, stored);
+}
 
 void launch_wait_timeout_selftest(long long limit_cycles, uint32_t* status, uint32_t* report, cudaStream_t st)
 {

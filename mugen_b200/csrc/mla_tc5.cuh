@@ -51,6 +51,11 @@ __device__ __forceinline__ void mbar_arrive_local_release_cluster(uint32_t bar) 
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
 }
+// A share of a sum that the blocks of a cluster put together: announced where it has been sent.  ok = false: it was not (a wait ran
+// out).  Then there is no announcement, the block that counts on it gives up too, and stores nothing.
+__device__ __forceinline__ void announce_share(uint32_t cluster_addr, bool ok) {
+    if (ok) mbar_arrive_cluster(cluster_addr);
+}
 __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
 }

@@ -699,6 +699,19 @@ def test_a_wait_that_runs_out_raises_the_status_bit_and_leaves_the_context_usabl
     ctx.close()
 
 
+def test_a_share_that_never_comes_is_not_added(torch):
+    """The blocks of a cluster put a projection's sums together.  Where one of them gives up, the others must not take what their
+    shared memory holds for its share: the self-test's second launch reports any block that does (and raises here)."""
+    ctx = make_ctx(synth.make_layer_case(11, 2, [3], synth.DT_F16), capi.KERNEL_AUTO)
+    before = ctx.launch_count()
+    ctx.selftest_wait_timeout(200_000)
+    assert ctx.launch_count() - before == 2
+    with pytest.raises(capi.MlaError) as ei:
+        ctx.status()
+    assert "= 4" in str(ei.value) and ctx.status() == 0
+    ctx.close()
+
+
 def test_block_tables_are_permuted_pages(torch):
     from mugen_b200.mla import MlaContext
     ctx = MlaContext(n_layers=1, n_heads=2, dtype=synth.DT_F16, n_pages=64, max_seqs=2, max_seq_len=4096,
