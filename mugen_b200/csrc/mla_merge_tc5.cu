@@ -43,12 +43,15 @@ constexpr int RED_WARPS = 16;
 // epilogue adds in a fixed order (27 blocks of 16 heads x 4 rows: 996 -> 970 us with the absorb's issuers).  With more than 8
 // rows (G = 1) the reduction takes longer and needs the registers: two issuers there (3 layers x 128 heads x 128 sequences of 64
 // tokens: one 218 us, two 205, four 244 with 160 bytes of spills; 2 layers x 128 heads x 128 verify rows: 305, 297, 324).
+// An accumulator takes two sub-tiles whoever issues them: G follows from how many layers and heads share a launch, and a row's sums
+// must not.
+constexpr int ACCS = NSUB / 2;
 template <int G>
 struct Roles {        // warps: W producer, MMA issuers, 4 epilogue, then the reduction
     // rows per tile; hi and lo of them side by side are the N side, so that a sub-tile of W goes through the tensor core once
     static constexpr int MT = G == 1 ? 16 : 8, NB = 2 * MT, A_SUB = NB * 128, A_BUF = NSUB * A_SUB;
     static constexpr int ISSUERS = G == 1 ? 2 : 4, FIRST_EPI = 1 + ISSUERS, FIRST_RED = FIRST_EPI + 4, THREADS = 32 * (FIRST_RED + RED_WARPS);
-    static constexpr uint32_t TMEM_COLS = 2 * ISSUERS * NB;
+    static constexpr uint32_t TMEM_COLS = 2 * ACCS * NB;
 };
 
 struct MergeArgs {
@@ -193,14 +196,14 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
                 const uint32_t b = n & 1, par = (n >> 1) & 1;
                 ok = mbar_wait<kPoll, true>(a_full(b), par, abort_flag, status) && mbar_wait(acc_empty(b), par ^ 1, abort_flag, status);
                 for (uint32_t i = 0; i < NSUB / ISSUERS && ok; i++) {
-                    const uint32_t s = part * (NSUB / ISSUERS) + i, d = tmem + (b * ISSUERS + part) * NB;
+                    const uint32_t s = part * (NSUB / ISSUERS) + i, d = tmem + (b * ACCS + s / 2) * NB;
                     ok = mbar_wait(full(s), un & 1, abort_flag, status);
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
                         const uint32_t da = desc_lo(base + s * W_SUB), db = desc_lo(base + OFF_A + b * A_BUF + s * A_SUB);
 #pragma unroll
-                        for (int k = 0; k < 4; k++) tc_mma(d, da + ((k * 32) >> 4), HI, db + ((k * 32) >> 4), HI, IDESC, (i == 0 && k == 0) ? 0u : 1u);
+                        for (int k = 0; k < 4; k++) tc_mma(d, da + ((k * 32) >> 4), HI, db + ((k * 32) >> 4), HI, IDESC, (s % 2 == 0 && k == 0) ? 0u : 1u);
                         if (r0 + MT >= x.r1) tc_commit(empty(s));          // the unit's last row tile frees the weights
                         if (i + 1 == NSUB / ISSUERS) { tc_commit(a_empty(b)); tc_commit(acc_full(b)); }
                     }
@@ -225,13 +228,13 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
                 ok = __all_sync(0xffffffffu, ok);
                 tc_fence_after();
                 float v[MT];
-                {   // the issuers' sums over hi and lo, always in this order
+                {   // the accumulators' sums over hi and lo, always in this order
 #pragma unroll
                     for (int k = 0; k < MT; k++) v[k] = 0.0f;
 #pragma unroll 1
-                    for (int p = 0; p < ISSUERS; p++) {
+                    for (int p = 0; p < ACCS; p++) {
                         uint32_t o[NB];
-                        tc_ldn(tmem + ((q4 * 32u) << 16) + (b * ISSUERS + p) * NB, o);
+                        tc_ldn(tmem + ((q4 * 32u) << 16) + (b * ACCS + p) * NB, o);
                         tc_wait_ld();
 #pragma unroll
                         for (int k = 0; k < MT; k++) v[k] += __uint_as_float(o[k]) + __uint_as_float(o[MT + k]);

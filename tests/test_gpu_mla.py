@@ -836,6 +836,49 @@ def test_merge_of_few_rows_in_many_parts(torch, oracle, H, dt, lens):
     ctx.close()
 
 
+@pytest.mark.parametrize("H,dt,rows,L", [
+    (16, synth.DT_F16, 16, 5),       # alone a layer's heads are cut into nine parts of one or two rows, five layers take whole heads
+    (5, synth.DT_F16, 29, 7),        # parts of one row; four of seven and eight
+    (40, synth.DT_BF16, 11, 4),      # three of three and four; one
+    (24, synth.DT_BF16, 70, 3),      # six of eleven and twelve; two of 35
+])
+def test_a_rows_projection_is_the_same_whoever_shares_its_launch(torch, oracle, H, dt, rows, L):
+    """Contexts of one page are never cut, so a layer's outputs are the same bits alone and in a launch of several layers, whichever
+    kernel the merge takes for the rows that a block has; and they are the CPU's."""
+    lens = [(11 * i) % 60 for i in range(rows)]
+    case = synth.make_layer_case(7300 + H, H, [n + 1 for n in lens], dt)
+    kv, q = _dev(torch, case.kv_a), _dev(torch, case.q)
+    outs = []
+    for grouped in (False, True):
+        ctx = make_ctx(case, capi.KERNEL_AUTO, n_layers=L, shuffle=3, max_rows=rows, max_seqs=rows)
+        seqs = []
+        for b, n in enumerate(lens):
+            seqs.append(ctx.seq_create())
+            for l in range(L):
+                if n:
+                    ctx.write_rows(l, seqs[b], 0, _dev(torch, case.caches[b][:n]))
+            ctx.advance_seq_len(seqs[b], n)
+        out = torch.zeros((L, rows, H, 128), dtype=torch.int16, device="cuda")
+        ctx.step_begin(seqs)
+        if grouped:
+            before = ctx.launch_count()
+            ctx.step_layers(0, L, torch.stack([kv] * L), torch.stack([q] * L), out)
+            assert ctx.launch_count() - before == 3          # all layers in one absorb, one attention, one merge
+        else:
+            for l in range(L):
+                ctx.step_append(l, kv)
+                ctx.step_attend(l, q, out[l])
+        ctx.step_end()
+        outs.append(_host(out).copy())
+        assert ctx.status() == 0
+        ctx.close()
+    assert np.array_equal(outs[0], outs[1])
+    appended = oracle.append_rows(case.kv_a, lens, case.norm_w, YARN["rms_norm_eps"], 40.0, 4096, 10000.0, dt)
+    for b, n in enumerate(lens):
+        want = oracle.attention(case.q[b], np.concatenate([case.caches[b][:n], appended[b:b + 1]]), n + 1, case.w_uk, case.w_uv, case.w_type, H, dt)
+        check_close(outs[0][0][b], want, dt, f"row {b}")
+
+
 @pytest.mark.parametrize("rows,L", [(8, 6), (24, 6), (48, 6), (70, 3)])
 def test_absorb_streams_the_weights_of_many_units_per_block(torch, rows, L):
     """128 heads x L layers in one launch: every block of the absorb walks several (layer, head) units through its ring, with
