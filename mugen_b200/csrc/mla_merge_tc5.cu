@@ -14,7 +14,7 @@
 // (together ~16 mantissa bits for bf16, ~22 for fp16, so the float state is not rounded to the storage type before the
 // projection), two buffers in turn: sixteen warps reduce the next tile's partial states while the tensor core works on
 // this one's.
-// Reduction: G = 16, 8, 4, 2 or 1 warps per row for steps of up to 1, 2, 4, 8 or more rows, each with its share of the 512 dims,
+// Reduction: G = 8, 4, 2 or 1 warps per row for blocks of up to 2, 4, 8 or more rows, each with its share of the 512 dims,
 // so that 128 bytes of loads are in flight per lane whatever the mix of rows and parts; weights come from one pass over
 // (m, l), 32 parts at a time, and no exchange between warps is needed.
 // (One block per head and 16 or 64 rows with load, reduction and MMAs in sequence: 27 layers x 16 heads x 1 row took 24 us
@@ -63,12 +63,12 @@ struct MergeArgs {
     const uint32_t* att_row;
 };
 
-// One row's merged state by one warp: dims dim0 + 64*k + 2*lane (+1), k < DL/2 (DL = 1: dim0 + lane).  acc comes back normalised.
+// One row's merged state by one warp: dims dim0 + 64*k + 2*lane (+1), k < DL/2.  acc comes back normalised.
 // Index: of a float within 32 parts, 64 bits where a caller's partials need them (launch_merge_tc5).
 template <int DL, typename Index>
 __device__ __forceinline__ void reduce_row(const MergeArgs& a, const RowParts& rp, uint32_t h, uint32_t dim0, uint32_t lane, float (&acc)[DL])
 {
-    constexpr int W = DL == 1 ? 1 : 2, Q = DL / W, PB = 32 / DL;      // floats per load, loads per part, parts per batch
+    constexpr int Q = DL / 2, PB = 32 / DL;      // loads per part, parts per batch
     float M = -INFINITY, L = 0.0f;
 #pragma unroll
     for (int k = 0; k < DL; k++) acc[k] = 0.0f;
@@ -77,8 +77,8 @@ __device__ __forceinline__ void reduce_row(const MergeArgs& a, const RowParts& r
     for (uint32_t c0 = rp.begin; c0 < rp.end; c0 += 32) {
         const uint32_t n = min(32u, rp.end - c0);
         const float* rec = rec0 + size_t(c0) * stride;
-        const float* src = rec + 2 + dim0 + W * lane;
-        float v[PB][Q][W];
+        const float* src = rec + 2 + dim0 + 2 * lane;
+        float v[PB][Q][2];
         auto load = [&](uint32_t p0) {
 #pragma unroll
             for (int i = 0; i < PB; i++)
@@ -86,13 +86,9 @@ __device__ __forceinline__ void reduce_row(const MergeArgs& a, const RowParts& r
                 for (int k = 0; k < Q; k++)
                     if (p0 + i < n) {
                         const float* at = src + (p0 + i) * stride + 64 * k;
-                        if constexpr (W == 1) {
-                            v[i][k][0] = *at;
-                        } else {
-                            const float2 f = *reinterpret_cast<const float2*>(at);
-                            v[i][k][0] = f.x;
-                            v[i][k][1] = f.y;
-                        }
+                        const float2 f = *reinterpret_cast<const float2*>(at);
+                        v[i][k][0] = f.x;
+                        v[i][k][1] = f.y;
                     }
         };
         float2 ml = lane < n ? *reinterpret_cast<const float2*>(rec + lane * stride) : make_float2(-INFINITY, 0.0f);
@@ -117,7 +113,7 @@ __device__ __forceinline__ void reduce_row(const MergeArgs& a, const RowParts& r
                 const float wi = __shfl_sync(0xffffffffu, w, int((p0 + i) & 31));
                 if (p0 + i >= n) continue;
 #pragma unroll
-                for (int k = 0; k < DL; k++) acc[k] = fmaf(wi, v[i][k / W][k % W], acc[k]);
+                for (int k = 0; k < DL; k++) acc[k] = fmaf(wi, v[i][k / 2][k % 2], acc[k]);
             }
         }
     }
@@ -279,12 +275,6 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
                 else if (u + 1 < u1) { const Unit y = unit_of(u + 1); fetch(y, y.r0); }
                 ok = ok && mbar_wait(a_empty(b), ((n >> 1) & 1) ^ 1, abort_flag, status);      // the MMAs of two tiles ago have read this buffer
                 if (rr < live) {
-                    if constexpr (G == 16) {                       // row 0 (of one): 32 dims, half a row of a sub-tile
-                        unsigned char* p = hi + (dim0 / 64) * A_SUB + (dim0 % 64 + lane) * 2;
-                        const T h0 = Elem<T>::from_f32(acc[0]);
-                        *reinterpret_cast<T*>(p) = h0;
-                        *reinterpret_cast<T*>(p + MT * 128) = Elem<T>::from_f32(acc[0] - Elem<T>::to_f32(h0));
-                    }
                     const uint32_t so = rr * 128 + (((lane / 4) ^ (rr & 7)) << 4) + (lane % 4) * 4;
 #pragma unroll
                     for (int k = 0; k < 8 / G; k++) {
@@ -324,13 +314,11 @@ int merge_tc5_configure()
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__half, 2>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__half, 4>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__half, 8>);
-    if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__half, 16>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__nv_bfloat16, 1, uint64_t>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__nv_bfloat16, 1>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__nv_bfloat16, 2>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__nv_bfloat16, 4>);
     if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__nv_bfloat16, 8>);
-    if (e == cudaSuccess) e = set(merge_outproj_tc5_kernel<__nv_bfloat16, 16>);
     return int(e);
 }
 
@@ -355,16 +343,18 @@ int launch_merge_tc5(int dtype, const float* recs, const StepMeta& m, uint32_t n
     // 32 parts of a plan's records are far below 2^32 floats; of a caller's partials they may be more (128 heads: from 2,040
     // rows on).  64-bit indices everywhere cost 1 % (128 heads x 8 sequences, layer by layer: 510 -> 517 us).
     const bool wide = uint64_t(32) * a.rec_stride * kPart > ~0u;
-    auto launch = [&](auto k1, auto k2, auto k4, auto k8, auto k16, auto k_wide, auto* o) {
+    auto launch = [&](auto k1, auto k2, auto k4, auto k8, auto k_wide, auto* o) {
         auto go = [&](auto kernel, uint32_t threads) { return int(launch_pdl(kernel, grid, dim3(threads), SMEM_BYTES, st, *map, o, a, status)); };
         constexpr uint32_t T1 = Roles<1>::THREADS, TN = Roles<2>::THREADS;
         if (wide) return go(k_wide, T1);
-        return unit_rows <= 1 ? go(k16, TN) : unit_rows <= 2 ? go(k8, TN) : unit_rows <= 4 ? go(k4, TN) : unit_rows <= 8 ? go(k2, TN) : go(k1, T1);
+        // (Sixteen warps for a single row were slower however many parts it has: their loop over parts is 32 wide, and 4-byte loads.
+        // One layer, 16 heads x 8 rows in blocks of one row: 1 part 5.4 us, 4.5 with eight warps on it; 64 parts 7.7, 7.3.)
+        return unit_rows <= 2 ? go(k8, TN) : unit_rows <= 4 ? go(k4, TN) : unit_rows <= 8 ? go(k2, TN) : go(k1, T1);
     };
     auto pick = [&](auto* o) {
         using T = std::remove_pointer_t<decltype(o)>;
         return launch(merge_outproj_tc5_kernel<T, 1>, merge_outproj_tc5_kernel<T, 2>, merge_outproj_tc5_kernel<T, 4>, merge_outproj_tc5_kernel<T, 8>,
-                      merge_outproj_tc5_kernel<T, 16>, merge_outproj_tc5_kernel<T, 1, uint64_t>, o);
+                      merge_outproj_tc5_kernel<T, 1, uint64_t>, o);
     };
     return dtype == 0 ? pick(static_cast<__half*>(out)) : pick(static_cast<__nv_bfloat16*>(out));
 }
