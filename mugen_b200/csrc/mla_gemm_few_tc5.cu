@@ -376,12 +376,27 @@ int gemm_few_tc5_clusters(uint32_t (&n)[4])
     return 0;
 }
 
-// Blocks of a cluster for this call, 0: not a call for this kernel.  Its tiles must be resident at once: a second round of
-// clusters would cost as much as the first, and the general kernel's equal runs have none.  The most blocks that fit, also
-// where they leave fewer SMs to the launches before and behind (16 heads x 4 rows: clusters of 4 808 us, of 2 835).  Against the
-// general kernel and the norm's own launch, input projections from registered weights (us; heads, hidden, q_lora, rows):
-//   16, 2048, -, 8: 11.7 -> 8.8     16, 4096, 512, 16: 17.5 -> 13.9     16, 7168, 1536, 16: 24.1 -> 20.3
-//   64, 4096, 512, 8: 18.0 -> 13.8  128, 4096, 512, 32: 23.7 -> 20.9    64, 4096, 512, 32: 20.4 -> 20.8
+// Blocks of a cluster for this call, 0: not a call for this kernel, or one that the general kernel is faster at.  Its tiles must be
+// resident at once: a second round of clusters would cost as much as the first, and the general kernel's equal runs have none.  The
+// most blocks that fit, also where they leave fewer SMs to the launches before and behind (16 heads x 4 rows: clusters of 4 808 us,
+// of 2 835).
+// What a cluster gains over the general kernel are the k-blocks that a tile's block does not walk itself, and the hand-over of a cut
+// tile; what it loses is the way of the sums from block to block, more with more blocks and with more rows that each must finish.
+// One projection from packed weights in a chain of such launches, general kernel -> this one (us; - / +: the rule refuses / takes):
+//   k-blocks  tiles  cluster  blocks    4 rows         16 rows        32 rows
+//      4       16       4       64     2.9 -> 2.9     3.0 -> 3.3     3.7 -> 4.2     -
+//      8       32       4      128     3.8 -> 4.2     4.0 -> 4.5     4.7 -> 5.5     -
+//     10       16       4       64     4.1 -> 3.0     4.3 -> 3.5     5.0 -> 4.6     +
+//     10       24       4       96     4.3 -> 3.9     4.4 -> 4.3     5.2 -> 5.3     + up to 8 rows
+//     10       72       2      144     4.5 -> 5.1     4.7 -> 5.6     5.5 -> 6.8     -
+//     16       48       2       96     5.6 -> 4.7     5.8 -> 5.3     6.6 -> 6.5     +
+//     16       72       2      144     6.5 -> 6.3     6.6 -> 6.8     7.4 -> 8.0     + up to 16 rows
+//     16       96       1       96     7.3 -> 7.6     7.5 -> 8.6                    -
+//     32       24       4       96     7.2 -> 5.0     7.4 -> 5.4     9.7 -> 6.4     +
+//     32       56       2      112     9.8 -> 7.8     9.9 -> 8.6                    +
+// With the norm in front the general kernel has a launch more, and only single blocks with more than 8 rows lose: 64 heads, hidden
+// 4096, q_lora 512, all by the general kernel / both projections here / as the rule has it: 8 rows 14.7 / 12.9 / 12.9, 16 rows 14.7 /
+// 15.3 / 14.0, 32 rows 18.1 / 20.1 / 17.3.  16 heads x 4 rows: hidden 4096 13.0 -> 11.2, hidden 7168 with q_lora 1536 20.4 -> 17.3.
 uint32_t gemm_few_tc5_cluster(const GemmCall& g, const uint32_t (&resident)[4])
 {
     if (!g.packed || g.M > 32 || g.M == 0) return 0;
@@ -390,7 +405,12 @@ uint32_t gemm_few_tc5_cluster(const GemmCall& g, const uint32_t (&resident)[4])
     for (int i = 0; i < g.n_weights; i++) tiles += (g.w[i].N + BM - 1) / BM;
     for (int i = 3; i >= 0; i--) {              // the most blocks that fit
         const uint32_t cs = 1u << i;
-        if (cs <= kb && tiles <= resident[i]) return (kb + cs - 1) / cs <= kmax ? cs : 0;
+        if (cs > kb || tiles > resident[i]) continue;
+        const uint32_t kbs = (kb + cs - 1) / cs;
+        if (kbs > kmax) return 0;
+        if (g.norm_w) return cs > 1 || g.M <= 8 ? cs : 0;
+        const uint32_t blocks = tiles * cs, spared = g.M <= 8 && blocks <= 112 ? 5 : blocks <= 64 ? 6 : 8;
+        return cs > 1 && kb - kbs >= spared && (cs > 2 || g.M <= 16 || blocks <= 96) ? cs : 0;
     }
     return 0;
 }

@@ -292,7 +292,7 @@ def test_projections_of_few_rows_in_every_cluster_size(torch, rows, H, E, R):
 
 
 @pytest.mark.parametrize("rows,H,E,R,dt", [
-    (4, 64, 2048, 0, "bf16"),            # Wo: 16 k-blocks per block in clusters of 8
+    (4, 64, 1024, 0, "bf16"),            # Wo: 16 k-blocks per block in clusters of 8
     (16, 32, 4096, 512, "f16"),          # Wo: 16 in clusters of 4
     (9, 16, 7168, 1536, "bf16"),         # Wo: 16 in clusters of 2; q_a and kv_a: 14 where 17 clusters of 8 are resident
     (16, 16, 7168, 1536, "f16"),
@@ -351,4 +351,31 @@ def test_projections_of_few_rows_whose_weight_ring_comes_round(torch, rows, H, E
             assert torch.equal(got, w)
     assert ctx.status() == 0
     del graph
+    ctx.close()
+
+
+@pytest.mark.parametrize("rows,H,E,R,launches", [
+    (1, 16, 2048, 0, 1), (32, 16, 2048, 0, 1), (33, 16, 2048, 0, 2),
+    (32, 16, 4096, 512, 2),              # q_b in clusters of 4
+    (8, 64, 4096, 512, 2),               # q_b: 96 tiles, single blocks, up to 8 rows
+    (9, 64, 4096, 512, 3), (32, 64, 4096, 512, 3),
+    (32, 128, 7168, 1536, 4),            # more k-blocks than a block holds, more tiles than SMs
+])
+def test_which_input_projections_take_the_kernel_for_few_rows(torch, rows, H, E, R, launches):
+    """That kernel normalises the rows itself; the general one has the norm as a launch ahead of it."""
+    from mugen_b200.mla import MlaContext
+    ctx = MlaContext(n_layers=1, n_heads=H, dtype=synth.DT_F16, n_pages=2, max_seqs=1, max_seq_len=64)
+    one = lambda *shape: np.full(shape, 0x3C00 if len(shape) == 1 else 0x2000, np.uint16)
+    w = dict(attn_norm=one(E), kv_a_mqa=one(576, E), wo=one(E, H * 128))
+    w.update(dict(q_a=one(R, E), q_a_norm=one(R), q_b=one(H * 192, R)) if R else dict(q=one(H * 192, E)))
+    ctx.set_block_weights(0, **w)
+    q, kv = (torch.zeros((rows, n), device="cuda", dtype=torch.float16) for n in (H * 192, 576))
+    before = ctx.launch_count()
+    ctx.block_project_in(0, torch.ones((rows, E), device="cuda", dtype=torch.float16), q, kv)
+    assert ctx.launch_count() - before == launches
+    # all values equal: a row of ones is its own norm, and an output the sum of its weights (0x2000 = 2^-7), of twice the roundings
+    a = E * 2.0 ** -7
+    want = R * 2.0 ** -7 if R else a                       # q_a's rows are equal values again: the norm makes ones of them
+    assert (kv.double() - a).abs().max() <= a * 2.0 ** -10 and (q.double() - want).abs().max() <= want * 2.0 ** -9
+    assert ctx.status() == 0
     ctx.close()
