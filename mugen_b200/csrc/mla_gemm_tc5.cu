@@ -59,11 +59,27 @@ static_assert(BK == 64, "the box width of make_matrix_map");
 static_assert(rows_smem(16) <= 232448 && rows_smem(128) <= 232448 && pair_smem(256) <= 232448 && pair_smem(128) <= 232448, "shared memory of one block");
 
 // Pairs with whole tiles take them in turn, so that those which compute at one time stand side by side in the line of tiles and
-// ask for the same rows of A, or the same weights, at about the same time: such requests are merged on the way to L2.  Eight
-// tiles of A's rows beside each other; one where A's rows lie far apart (a piece of 128 bytes each) and are better read by
-// all.  Groups of 1 / 2 / 8 / 16, 2048 rows: K = 16384 389 / 404 / 423 / 424 us, K = 7168 and 1536 together 188 / 185 / 179 / 179;
-// the expansion of a chunk of 4096 at 8192 413 / 414 / 405 / 396.
-constexpr uint32_t GROUP_M = 8, FAR_ROWS = 16384;
+// ask for the same rows of A, or the same weights, at about the same time: such requests are merged on the way to L2.  How many
+// tiles along A's rows stand beside each other (the rest of the rows comes behind all outputs) decides which of the two they share.
+// Time over that of consecutive tiles per pair, all of A's rows side by side, in the kernel with four epilogue warps; groups of
+// 1 / 2 / 8 / 16 (all, up to 4096 rows); outputs x K; best of three processes, between which one call differs by up to a tenth:
+//                     512 rows               1100 rows              2048 rows              3000 rows              4096 rows
+//   7168 x 16384   0.86 .95 .95 .95       0.96 .95 .91 .91       0.90 .92 .96 .95       0.99 1.03 1.14 1.04    0.92 .87 1.10 1.05
+//   7168 x 12288   0.93 .92 .92 .92       0.94 .94 .90 .90       1.00 1.04 .94 .95      0.88 1.01 1.06 .98     0.94 .92 1.10 1.03
+//   7168 x  8192   0.91 .89 .89 .90       0.95 .94 .90 .90       0.99 .99 .94 .94       0.92 .91 .88 .88       0.91 .89 1.00 .95
+//   4096 x 16384   0.83 .91 .91 .90       1.09 .97 .93 .93       0.87 .86 .95 .96       0.92 .83 .92 .97       0.95 1.07 1.08 .98
+//   4096 x 12288   0.78 .78 .75 .77       1.02 .96 .92 .92       0.94 .94 .93 .93       0.95 .83 .89 .97       0.94 .98 1.06 .96
+//   4096 x  8192   0.78 .78 .78 .77       0.93 .94 .88 .88       0.94 .94 .92 .92       0.94 .94 .94 .94       0.95 .94 1.00 .94
+//   2048 x 16384   0.80 .83 .83 .78       0.94 .88 .92 .92       0.93 .93 .93 .93       0.88 .84 .82 .95       1.09 1.09 1.09 .95
+// All rows side by side are the safe order: 0.95 in the mean over 5000 to 8192 rows, where groups of 1 to 16 reach 1.15 to 1.27.
+// Up to K = 8192 nothing is steadily better.  Where A's rows are further apart and not many: one where the outputs are many, or A's
+// tiles very few; two in between.  (Expansion of a chunk of 4096 at 8192, groups of 1 / 8 / 16 / all: 357 / 366 / 363 / 361 us.)
+inline uint32_t group_of(uint32_t K, uint32_t outputs, uint32_t m_tiles) {
+    constexpr uint32_t FAR_K = 9216, MANY_OUTPUTS = 5632;          // between the sizes measured
+    if (K < FAR_K || m_tiles > 16) return m_tiles;
+    if (outputs >= MANY_OUTPUTS || m_tiles < 4) return 1;
+    return m_tiles < 14 ? 2 : m_tiles;
+}
 
 struct GemmArgs {
     uint32_t M, kb;                     // rows of A, k-blocks
@@ -711,7 +727,8 @@ int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t*
     a.units = a.m_tiles * (a.n_tiles[0] + a.n_tiles[1]) * a.kb;
     a.run = sh.run;
     const uint32_t whole_tiles = a.units / a.kb;
-    a.group_m = rows_kernel ? a.m_tiles : std::min(a.m_tiles, g.K >= FAR_ROWS ? 1u : GROUP_M);
+    const uint32_t outputs = g.w[0].N + (g.n_weights > 1 ? g.w[1].N : 0u);
+    a.group_m = rows_kernel ? a.m_tiles : group_of(g.K, outputs, a.m_tiles);
     a.stride = !rows_kernel && a.run % a.kb == 0 ? std::min(whole_tiles, ws.blocks / 2) : 0u;
     const uint32_t workers = a.stride ? a.stride : (a.units + a.run - 1) / a.run;
     a.residual = g.residual ? 1u : 0u;
