@@ -624,7 +624,7 @@ int run_chunks(mla_ctx* c, uint32_t layer, const void* q, void* out, cudaStream_
         gc.n_weights = 2;
         gc.w[0] = gemm_weight(c->w_uk_rows_maps, H * mla::kNope, c->pf_kx, layer * H * mla::kNope);
         gc.w[1] = gemm_weight(c->w_uv_maps, H * mla::kVDim, c->pf_vx, layer * H * mla::kVDim);
-        int rc = mla::launch_gemm_tc5(dt, gc, c->gemm_ws, c->status_dev, st);
+        int rc = mla::launch_gemm_tc5(dt, gc, c->gemm_ws, c->status_dev, st, c->launches);
         if (rc) return fail(c, rc == -1 ? MLA_ERR_INVALID : MLA_ERR_CUDA, "key / value expansion launch failed");
         mla::PrefillCall p;
         p.q = q; p.out = out; p.kx = c->pf_kx; p.vx = c->pf_vx;
@@ -640,7 +640,7 @@ int run_chunks(mla_ctx* c, uint32_t layer, const void* q, void* out, cudaStream_
         p.cs_rows = c->cs_rows;
         rc = mla::launch_prefill_tc5(dt, p, c->status_dev, st);
         if (rc) return fail(c, rc == -1 ? MLA_ERR_INVALID : MLA_ERR_CUDA, "prefill attention launch failed");
-        c->launches += 2;
+        c->launches++;
     }
     return MLA_OK;
 }
@@ -1494,7 +1494,7 @@ int project(mla_ctx* c, const void* act, uint32_t rows, uint32_t K, std::initial
     g.norm_w = norm_w;
     g.norm_out = norm_out;
     g.eps = c->cfg.rms_norm_eps;
-    const int rc = mla::launch_gemm_tc5(int(c->cfg.dtype), g, c->gemm_ws, c->status_dev, st, &c->launches);
+    const int rc = mla::launch_gemm_tc5(int(c->cfg.dtype), g, c->gemm_ws, c->status_dev, st, c->launches);
     if (rc == -1) return fail(c, MLA_ERR_INVALID, "projection operands must be 16-byte aligned with row lengths that are multiples of 8");
     if (rc != 0) return fail(c, MLA_ERR_CUDA, std::string("projection launch: ") + cudaGetErrorString(cudaError_t(rc)));
     return MLA_OK;

@@ -818,11 +818,9 @@ bool gemm_tc5_weight_maps(GemmWeightMaps* maps, int dtype, const void* W, uint64
 
 // Returns a cudaError_t value, or -1 when the operands cannot be addressed (pointers must be 16-byte aligned, row lengths
 // multiples of 8).
-int launch_gemm_tc5(int dtype, const GemmCall& call, const GemmWorkspace& ws, uint32_t* status, cudaStream_t st, uint64_t* launched)
+int launch_gemm_tc5(int dtype, const GemmCall& call, const GemmWorkspace& ws, uint32_t* status, cudaStream_t st, uint64_t& launched)
 {
     if (call.M == 0 || call.n_weights == 0) return 0;
-    uint64_t unused;
-    uint64_t& n = launched ? *launched : unused;
     GemmCall g = call;
     const bool aligned = (reinterpret_cast<uintptr_t>(g.A) & 15u) == 0;
     // an output over the rows themselves: the kernel that normalises on the way would read what its other blocks wrote
@@ -834,15 +832,15 @@ int launch_gemm_tc5(int dtype, const GemmCall& call, const GemmWorkspace& ws, ui
     }
     if (g.A && g.K % 8 == 0 && aligned && apart)
         if (const uint32_t cs = gemm_few_tc5_cluster(g, ws.clusters)) {
-            n++;
+            launched++;
             return launch_gemm_few_tc5(dtype, g, cs, status, st);
         }
     if (g.norm_w) {
         if (const int e = launch_rmsnorm_rows(dtype, g.A, g.norm_w, g.norm_out, g.M, g.K, g.eps, st)) return e;
-        n++;
+        launched++;
         g.A = g.norm_out;
     }
-    n++;
+    launched++;
     return dtype == 0 ? launch_type<__half>(g, ws, dtype, status, st) : launch_type<__nv_bfloat16>(g, ws, dtype, status, st);
 }
 

@@ -132,7 +132,7 @@ struct GemmWorkspace {
     uint32_t clusters[4];      // gemm_few_tc5_clusters
 };
 // launched: kernels launched are added to it
-int launch_gemm_tc5(int dtype, const GemmCall& g, const GemmWorkspace& ws, uint32_t* status, cudaStream_t st, uint64_t* launched = nullptr);
+int launch_gemm_tc5(int dtype, const GemmCall& g, const GemmWorkspace& ws, uint32_t* status, cudaStream_t st, uint64_t& launched);
 // The same for few rows and weights that fit the SMs in one go, the norm included (mla_gemm_few_tc5.cu); launch_gemm_tc5 picks.
 uint32_t gemm_few_tc5_cluster(const GemmCall& g, const uint32_t (&resident)[4]);
 int launch_gemm_few_tc5(int dtype, const GemmCall& g, uint32_t cs, uint32_t* status, cudaStream_t st);

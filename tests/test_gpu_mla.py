@@ -468,6 +468,23 @@ def test_prefill_chunks_take_the_expanded_path(torch, oracle, H, dt, spec, q_rop
     ctx.close()
 
 
+@pytest.mark.parametrize("decode_rows,launches", [(0, 3), (2, 5)])
+def test_launches_of_a_step_with_a_chunk_are_counted(torch, decode_rows, launches):
+    """The append or, with decode rows, absorb, attention and merge; then the expansion and the chunk's attention."""
+    n = 1 + decode_rows
+    case = synth.make_layer_case(4400, 4, [100] * n, synth.DT_F16)
+    ctx = make_ctx(case, capi.KERNEL_AUTO, max_rows=130)
+    seqs = fill(torch, ctx, case)
+    new = [100] + [1] * decode_rows
+    kv, q, out = (torch.zeros((1, sum(new)) + d, dtype=torch.int16, device="cuda") for d in ((576,), (4, 192), (4, 128)))
+    before = ctx.launch_count()
+    ctx.step_begin(seqs, new)
+    ctx.step_layers(0, 1, kv, q, out)
+    ctx.step_end()
+    assert ctx.launch_count() - before == launches and ctx.status() == 0
+    ctx.close()
+
+
 @pytest.mark.parametrize("start,n_new", [(0, 64), (1, 127), (0, 129), (120, 137), (300, 212), (0, 1025)])
 def test_prefill_maxima_that_move_at_every_step(torch, start, n_new):
     """1 to 9 steps of 128 keys whose rows grow along the sequence, so that the maxima move (and the output is rescaled) in
