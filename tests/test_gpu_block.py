@@ -195,6 +195,8 @@ def test_projections_at_the_edges_of_their_tiles(torch, rows, H, E, R, shift):
 @pytest.mark.parametrize("rows,H,E,R,shift", [
     (1, 5, 72, 0, 0), (16, 16, 2048, 0, 0), (17, 16, 520, 64, 4), (33, 5, 1000, 200, 0), (65, 3, 520, 0, 1), (128, 3, 2048, 0, 8),
     (129, 16, 2048, 0, 0), (256, 5, 72, 0, 4), (257, 64, 1000, 136, 0), (700, 16, 2048, 0, 8),
+    # the order of the tiles, Wo: two by two with one over; one by one; 9 tiles of rows side by side, the last one of 252 rows
+    (1100, 72, 520, 0, 0), (600, 80, 520, 0, 0), (2300, 3, 1032, 0, 0),
 ])
 def test_every_output_of_the_projections_and_nothing_beside_them(torch, rows, H, E, R, shift, dt):
     """Element by element against float64, and the values in front of and behind each output untouched.  An output is one rounding
@@ -243,40 +245,48 @@ def test_every_output_of_the_projections_and_nothing_beside_them(torch, rows, H,
     ctx.close()
 
 
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
 @pytest.mark.parametrize("rows,H,E,R", [
     (1, 1, 64, 0), (2, 2, 1024, 0), (3, 2, 1032, 8), (4, 5, 2048, 0), (5, 16, 4096, 512), (8, 5, 72, 64), (9, 16, 2048, 0), (16, 4, 7168, 1536),
     (17, 2, 1024, 0), (24, 5, 520, 200), (31, 2, 4096, 136), (32, 16, 2048, 0),
+    (8, 64, 4096, 512), (4, 64, 1024, 0),          # single blocks of 8 and of 16 k-blocks
+    (16, 4, 7168, 1024),                           # 14 k-blocks per block of a cluster of 8
 ])
-def test_projections_of_few_rows_in_every_cluster_size(torch, rows, H, E, R):
+def test_projections_of_few_rows_in_every_cluster_size(torch, rows, H, E, R, dt):
     """Clusters of 1, 2, 4 and 8 blocks per tile, shared and whole rows per warp, k-blocks that end early.  The operands of one row
     go to no other: the rows of a call equal, bit for bit, the same rows of a call with other rows beside them, where both calls
-    have rows of the same number per warp; and every output is within the bounds of the test above."""
+    have rows of the same number per warp; and every output is within the bounds of the test above.  That the input projections
+    ran in this kernel shows in the launches: the norm is not one of them."""
     from mugen_b200.mla import MlaContext
     gen = torch.Generator(device="cuda")
     gen.manual_seed(rows * 13 + E)
-    rn = lambda *shape, scale=1.0: (torch.randn(shape, device="cuda", generator=gen) * scale).half()
+    tdt, code, u = (torch.float16, synth.DT_F16, 2.0 ** -11) if dt == "f16" else (torch.bfloat16, synth.DT_BF16, 2.0 ** -8)
+    rn = lambda *shape, scale=1.0: (torch.randn(shape, device="cuda", generator=gen) * scale).to(tdt)
     bits = lambda t: t.view(torch.int16).cpu().numpy().view(np.uint16)
-    eps, u, QD, VD = 1e-6, 2.0 ** -11, H * 192, H * 128
-    ctx = MlaContext(n_layers=1, n_heads=H, dtype=synth.DT_F16, n_pages=2, max_seqs=1, max_seq_len=64, rope_theta=1e4,
+    eps, QD, VD = 1e-6, H * 192, H * 128
+    ctx = MlaContext(n_layers=1, n_heads=H, dtype=code, n_pages=2, max_seqs=1, max_seq_len=64, rope_theta=1e4,
                      rope_scaling_factor=1.0, rope_original_ctx=4096, rms_norm_eps=eps)
     w = dict(attn_norm=1 + rn(E, scale=0.1), kv_a_mqa=rn(576, E, scale=E ** -0.5), wo=rn(E, VD, scale=VD ** -0.5))
     w.update(dict(q_a=rn(R, E, scale=E ** -0.5), q_a_norm=1 + rn(R, scale=0.1), q_b=rn(QD, R, scale=R ** -0.5)) if R
              else dict(q=rn(QD, E, scale=E ** -0.5)))
     ctx.set_block_weights(0, **{k: bits(v) for k, v in w.items()})
-    norm = lambda x, g: (x.double() * torch.rsqrt((x.double() ** 2).mean(-1, keepdim=True) + eps) * g.double()).half()
+    norm = lambda x, g: (x.double() * torch.rsqrt((x.double() ** 2).mean(-1, keepdim=True) + eps) * g.double()).to(tdt)
 
     def run(hidden, att):
-        q, kv, out = torch.zeros((len(hidden), QD), device="cuda").half(), torch.zeros((len(hidden), 576), device="cuda").half(), hidden.clone()
+        q, kv, out = torch.zeros((len(hidden), QD), device="cuda").to(tdt), torch.zeros((len(hidden), 576), device="cuda").to(tdt), hidden.clone()
         ctx.block_project_in(0, hidden, q, kv)
         ctx.block_project_out(0, att, out)
         return q, kv, out
 
     hidden, att = rn(rows, E), rn(rows, VD)
+    before = ctx.launch_count()
     q, kv, out = run(hidden, att)
+    if (E, R) != (7168, 1536):               # 17 tiles of 112 k-blocks: a device holds 17 clusters of 8, or the call goes elsewhere
+        assert ctx.launch_count() - before == (3 if R else 2)
     x = norm(hidden, w["attn_norm"])
-    a = norm((x.double() @ w["q_a"].double().T).half(), w["q_a_norm"]) if R else x
+    a = norm((x.double() @ w["q_a"].double().T).to(tdt), w["q_a_norm"]) if R else x
     for got, want, n in ((q, a.double() @ (w["q_b"] if R else w["q"]).double().T, 1), (kv, x.double() @ w["kv_a_mqa"].double().T, 1),
-                         (out, hidden.double() + (att.double() @ w["wo"].double().T).half().double(), 2)):
+                         (out, hidden.double() + (att.double() @ w["wo"].double().T).to(tdt).double(), 2)):
         assert not ((got.double() - want).abs() > u * (n * want.abs() + 6)).any()
     other_hidden, other_att = rn(rows, E, scale=30.0), rn(rows, VD, scale=30.0)
     other_hidden[rows // 2], other_att[rows // 2] = hidden[rows // 2], att[rows // 2]
