@@ -19,9 +19,12 @@
 //                    (16, 32, 64 or 128 columns): the bytes in flight are weight bytes, and a step of 4 rows does not pay
 //                    for 128.  HBM-bound.
 //   more rows        gemm_pair_kernel on SM pairs (tcgen05.mma.cta_group::2): 256 rows of A x 256 or 128 outputs per tile, each
-//                    block holding 128 rows of A and half of the outputs' weight rows.  What bounds it is the L2 -> shared
-//                    memory feed (measured with one block per 128 x 256 tile: 48 KB per 4.2 MFLOP k-block, 930 TFLOP/s =
-//                    10.7 TB/s): the pair needs 32 KB for the same work.  Finished tiles leave through shared memory and TMA.
+//                    block holding 128 rows of A and half of the outputs' weight rows: 32 KB from L2 for a k-block of 4.2
+//                    MFLOP per block, where one block per 128 x 256 tile needs 48 (930 TFLOP/s = 10.7 TB/s from L2, which
+//                    bounds that form).  2048 rows x 7168 outputs, K = 16384, run at 1,404 TFLOP/s, what cuBLAS
+//                    sustains on the card.  With few k-blocks or tiles the start, the end and the last wave count: 777 rows x
+//                    2048 outputs, K = 2048, 420 TFLOP/s.
+//                    Finished tiles leave through shared memory and TMA.
 // Calls of up to 32 rows whose tiles are few go to a kernel of their own (mla_gemm_few_tc5.cu).
 // The first stages' weight tiles are constant and requested before the grid dependency is waited for.  Projection weights are
 // kept packed (gemm_tc5_pack): tiles of 128 outputs x 64 inputs as 16 KB runs, k-block after k-block, so that a block's
@@ -156,7 +159,9 @@ __device__ __forceinline__ void epilogue_sync() { asm volatile("barrier.cta.sync
 // The epilogue threads hand a cut tile's accumulator (row r of it, NT columns, at tensor-memory address acc; a thread's share are
 // columns c0*CH .. c1*CH - 1) over: partial to global memory, then the tile's counter.  Returns true in the worker that arrived
 // last; sum_partials then gives columns c*CH.. of the whole tile.  Worker w's slots are 2w (the tile its run begins in) and
-// 2w + 1 (the one it ends in).  last_slot: not the one of the cut tile before.
+// 2w + 1 (the one it ends in).  last_slot is one word: who writes it for the next cut tile has passed that tile's first barrier, and
+// everyone arrives there with this tile's value read.  (With two fences and a third barrier instead of the atomic that releases and
+// acquires: 32 heads, hidden 2048, 129 rows, output projection 21.9 us, 20.9 now; 96 heads 29.9, 29.1.)
 template <int NT, int CH, int THREADS, typename Release>
 __device__ __forceinline__ bool hand_over(const GemmArgs& a, uint32_t worker, uint32_t blocks_per_worker, uint32_t rank, uint32_t tile, uint32_t acc,
                                           uint32_t r, int c0, int c1, bool first_thread, bool ok, volatile uint32_t* last_slot, Release release)
@@ -228,7 +233,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     static_assert((2 * STAGES + 4) * 8 <= 224, "barriers overflow their area");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + OFF_MISC + 224);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + 228);
-    volatile uint32_t* last_slot = reinterpret_cast<volatile uint32_t*>(sm + OFF_MISC + 232);      // two, in turn
+    volatile uint32_t* last_slot = reinterpret_cast<volatile uint32_t*>(sm + OFF_MISC + 232);
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const uint32_t u0 = blockIdx.x * a.run, u1 = min(a.units, u0 + a.run);       // this block's run of units
 
@@ -344,7 +349,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     if (c + 1 == NT / CH) release();
                     finish(c, v);
                 }
-            } else if (hand_over<NT, CH, 128>(a, blockIdx.x, 1, 0, tile, acc, r, 0, NT / CH, r == 0, ok, last_slot + (nt & 1), release)) {
+            } else if (hand_over<NT, CH, 128>(a, blockIdx.x, 1, 0, tile, acc, r, 0, NT / CH, r == 0, ok, last_slot, release)) {
 #pragma unroll 1
                 for (int c = 0; c < NT / CH; c++) {
                     float v[CH];
@@ -383,7 +388,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     static_assert((2 * STAGES + 4) * 8 <= 224, "barriers overflow their area");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + OFF_MISC + 224);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + 228);
-    volatile uint32_t* last_slot = reinterpret_cast<volatile uint32_t*>(sm + OFF_MISC + 232);      // two, in turn
+    volatile uint32_t* last_slot = reinterpret_cast<volatile uint32_t*>(sm + OFF_MISC + 232);
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const uint32_t rank = cluster_rank(), worker = blockIdx.x / 2;               // rank 0 issues the MMAs
     // this pair's run of units; with whole tiles (stride) the units of its own tiles, counted from 0
@@ -587,7 +592,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     if (c + 2 == c_first + CHUNKS) release();
                     finish(c + 1, v, rs1);
                 }
-            } else if (hand_over<NT, CH, 32 * EPI_WARPS>(a, worker, 2, rank, tile, acc, r, c_first, c_first + CHUNKS, tid == 64, ok, last_slot + (nt & 1), release)) {
+            } else if (hand_over<NT, CH, 32 * EPI_WARPS>(a, worker, 2, rank, tile, acc, r, c_first, c_first + CHUNKS, tid == 64, ok, last_slot, release)) {
 #pragma unroll 1
                 for (int c = c_first; c < c_first + CHUNKS; c += 2) {
                     float v[CH];
@@ -680,11 +685,12 @@ cudaError_t configure_type()
 }
 
 // Tile width and run length of a launch: the shortest estimate, in SM cycles, of whole tiles against equal runs with cut
-// tiles.  A k-block of a pair takes 820 (256 outputs) or 610 (128) cycles at the L2 feed rate, one of gemm_rows_kernel
-// about 400 at the HBM rate.  Cutting tiles adds the hand-over (partial out, counter, partials in): in gemm_rows_kernel about
-// 4000 cycles and 50 per column; in a pair 190 per column, 13 and 26 us, fitted to whole and cut runs of both widths over 8
-// weights x 9 row counts (N = K = 2048, 129 to 512 rows: whole tiles 15 us, cut 22 to 25; N = 2048, K = 8192, 400 rows: cut
-// 128-wide tiles 34, whole 46, cut 256-wide 43).
+// tiles.  A k-block of a pair counts 820 (256 outputs) or 610 (128) cycles, one of gemm_rows_kernel about 400 (the HBM rate).  Cutting
+// tiles adds the hand-over (partial out, counter, partials in): in gemm_rows_kernel about 4000 cycles and 50 per column; in a pair
+// 190 per column, 13 and 26 us, fitted to whole and cut runs of both widths over 8 weights x 9 row counts.  The pair's figures are
+// those of the kernel whose loading thread divided for every k-block, with four epilogue warps and three barriers in the
+// hand-over; both kinds of run have become faster since (N = K = 2048, 129 to 512 rows, whole tiles: 15 us then, 12 now), the
+// balance between them has not been fitted again.
 struct Shape { uint32_t nt, m_tiles, n_tiles[2], run; };
 Shape pick_shape(const GemmCall& g, bool rows_kernel, uint32_t kb, const GemmWorkspace& ws)
 {
