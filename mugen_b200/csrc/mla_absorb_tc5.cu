@@ -315,7 +315,7 @@ int absorb_tc5_configure()
 // position (m.row_pos) before they are stored.
 int launch_absorb_tc5(int dtype, const void* q, const void* w_map, void* q_abs, uint32_t H, uint32_t layer0, const void* kv_a,
                       void* layer_pool, uint64_t pool_slots, const void* norm_w, const float* cos_sin, uint32_t cs_rows,
-                      float eps, const StepMeta& m, bool rotate_q, bool append_waits, uint32_t sm_count, uint32_t* status, cudaStream_t st)
+                      float eps, const StepMeta& m, bool rotate_q, bool append_waits, uint32_t sm_count, uint32_t* status, const LaunchStream& st)
 {
     if (m.rows == 0) return 0;
     const CUtensorMap* map = static_cast<const CUtensorMap*>(w_map);

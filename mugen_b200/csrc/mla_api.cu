@@ -102,6 +102,8 @@ struct mla_ctx {
     size_t meta_cap = 0;
     char* meta_dev = nullptr;       // [kPlanRegions][meta_cap]
     char* meta_host = nullptr;      // [kMetaRing][meta_cap], page-locked
+    bool fresh = false;             // the last upload went to fresh_stream and no kernel has followed it there yet (launch_stream)
+    cudaStream_t fresh_stream = nullptr;
     // Plans of the open step.  `plan`: every new token is a decode-style query row, one layer at a time.  A step that holds
     // prefill chunks (sequences taking >= kPrefillMin new tokens) also has `plan_rest`: its query rows are the step's OTHER
     // rows, the chunks go through the expanded-form prefill kernels (run_layer); the explicit per-layer calls
@@ -442,7 +444,9 @@ int build_plan(mla_ctx* c, Plan& plan, int region, const std::vector<uint32_t>& 
             c->chunk_groups.push_back({g.rows, g.n_tiles, reinterpret_cast<const uint32_t*>(d + o_cpg) + g.page0,
                                        reinterpret_cast<const mla::PrefillTile*>(d + o_ctl) + g.tile0});
     }
-    CU_TRY(c, cudaMemcpyAsync(d, h, off, cudaMemcpyHostToDevice, st));
+    CU_TRY(c, cudaError_t(mla::launch_fetch(h, d, uint32_t(off / 16), st)));
+    c->fresh = true;
+    c->fresh_stream = st;
     CU_TRY(c, cudaEventRecord(mb.done, st));
     mb.in_flight = true;
 
@@ -498,6 +502,21 @@ int rest_plan(mla_ctx* c, cudaStream_t st)
     return build_plan(c, c->plan_rest, kPlanRest, c->step_seqs, c->rows, &rest, &att_row, 1, st, &cm);
 }
 
+bool capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
+// the stream of a launch that may be the first behind an upload of metadata
+mla::LaunchStream launch_stream(const mla_ctx* c, cudaStream_t st) { return mla::LaunchStream(st, c->fresh && c->fresh_stream == st); }
+// ... and once it is in the stream (a captured launch is not)
+void launched(mla_ctx* c, cudaStream_t st) { if (c->fresh && c->fresh_stream == st && !capturing(st)) c->fresh = false; }
+
 char* layer_pool(mla_ctx* c, uint32_t layer)
 {
     return c->pool + size_t(layer) * c->pool_slots * mla::kRow * 2;
@@ -518,8 +537,9 @@ char* layer_norm(mla_ctx* c, uint32_t layer) { return c->norm + size_t(layer) * 
 int run_append(mla_ctx* c, uint32_t layer, const void* kv_a, const mla::StepMeta& m, cudaStream_t st)
 {
     const int e = mla::launch_append(int(c->cfg.dtype), kv_a, layer_pool(c, layer), c->pool_slots, layer_norm(c, layer),
-                                     c->cos_sin, c->cs_rows, c->cfg.rms_norm_eps, m, c->status_dev, st);
+                                     c->cos_sin, c->cs_rows, c->cfg.rms_norm_eps, m, c->status_dev, launch_stream(c, st));
     if (e != 0) return fail(c, MLA_ERR_CUDA, std::string("append launch: ") + cudaGetErrorString(cudaError_t(e)));
+    if (m.app_rows) launched(c, st);
     c->launches += m.app_rows ? 1 : 0;
     return MLA_OK;
 }
@@ -535,8 +555,9 @@ int run_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, float* expo
     const int dt = int(c->cfg.dtype);
     const int ae = mla::launch_absorb_tc5(dt, q, &c->w_uk_map, c->q_abs, H, layer, fused_kv_a, layer_pool(c, layer), c->pool_slots,
                                           layer_norm(c, layer), c->cos_sin, c->cs_rows, c->cfg.rms_norm_eps, m, c->q_rope_in_kernel,
-                                          !kv_a_settled, uint32_t(c->sm_count), c->status_dev, st);
+                                          !kv_a_settled, uint32_t(c->sm_count), c->status_dev, launch_stream(c, st));
     if (ae != 0) return fail(c, MLA_ERR_CUDA, std::string("absorb launch: ") + cudaGetErrorString(cudaError_t(ae)));
+    launched(c, st);
     int e;
     const bool timed = c->profiling && c->prof_used < c->prof_events.size() && (c->prof_seq++ % c->prof_stride) == 0;
     if (timed) CU_TRY(c, cudaEventRecord(c->prof_events[c->prof_used].first, st));
@@ -1138,16 +1159,6 @@ int mla_step_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, void* 
     return run_attend(c, layer, q, out, nullptr, c->plan, static_cast<cudaStream_t>(stream));
 }
 
-static bool capturing(cudaStream_t st)
-{
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return status != cudaStreamCaptureStatusNone;
-}
-
 int mla_step_layers(mla_ctx* c, uint32_t layer_begin, uint32_t n_layers, const void* kv_a, const void* q, void* out,
                     void* stream)
 {
@@ -1226,9 +1237,11 @@ int mla_merge_partials(mla_ctx* c, uint32_t layer, uint32_t n_parts, uint32_t ro
     mla::StepMeta m{};
     m.rows = rows;
     m.layers = 1;
+    auto st = static_cast<cudaStream_t>(stream);
     const int e = mla::launch_merge_tc5(int(c->cfg.dtype), partials, m, n_parts, &c->w_uv_map, out, c->cfg.n_heads, layer, uint32_t(c->sm_count), c->status_dev,
-                                        static_cast<cudaStream_t>(stream));
+                                        launch_stream(c, st));
     if (e != 0) return fail(c, MLA_ERR_CUDA, std::string("merge launch: ") + cudaGetErrorString(cudaError_t(e)));
+    if (rows) launched(c, st);
     c->launches += rows ? 1 : 0;
     CU_TRY(c, cudaGetLastError());
     return MLA_OK;
@@ -1494,9 +1507,10 @@ int project(mla_ctx* c, const void* act, uint32_t rows, uint32_t K, std::initial
     g.norm_w = norm_w;
     g.norm_out = norm_out;
     g.eps = c->cfg.rms_norm_eps;
-    const int rc = mla::launch_gemm_tc5(int(c->cfg.dtype), g, c->gemm_ws, c->status_dev, st, c->launches);
+    const int rc = mla::launch_gemm_tc5(int(c->cfg.dtype), g, c->gemm_ws, c->status_dev, launch_stream(c, st), c->launches);
     if (rc == -1) return fail(c, MLA_ERR_INVALID, "projection operands must be 16-byte aligned with row lengths that are multiples of 8");
     if (rc != 0) return fail(c, MLA_ERR_CUDA, std::string("projection launch: ") + cudaGetErrorString(cudaError_t(rc)));
+    if (rows) launched(c, st);
     return MLA_OK;
 }
 

@@ -35,17 +35,24 @@ enum : uint32_t {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
+// The first kernel behind an upload of step metadata is launched plain: it starts when the upload is done and flushed, and so does
+// every kernel behind it, all of which read the metadata ahead of their wait.
+struct LaunchStream {
+    cudaStream_t st;
+    bool plain;
+    LaunchStream(cudaStream_t s, bool is_plain = false) : st(s), plain(is_plain) {}
+};
 template <typename K, typename... Args>
-inline cudaError_t launch_pdl(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args)
+inline cudaError_t launch_pdl(K kernel, dim3 grid, dim3 block, size_t smem, const LaunchStream& st, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
+    cfg.stream = st.st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[0].val.programmaticStreamSerializationAllowed = st.plain ? 0 : 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, args...);

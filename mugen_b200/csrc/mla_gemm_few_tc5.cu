@@ -297,10 +297,10 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constan
     }
 }
 
-cudaLaunchConfig_t launch_config(cudaLaunchAttribute (&at)[2], uint32_t blocks, uint32_t cs, cudaStream_t st)
+cudaLaunchConfig_t launch_config(cudaLaunchAttribute (&at)[2], uint32_t blocks, uint32_t cs, const LaunchStream& st)
 {
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[0].val.programmaticStreamSerializationAllowed = st.plain ? 0 : 1;
     at[1].id = cudaLaunchAttributeClusterDimension;
     at[1].val.clusterDim.x = cs;
     at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
@@ -308,7 +308,7 @@ cudaLaunchConfig_t launch_config(cudaLaunchAttribute (&at)[2], uint32_t blocks, 
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(NUM_THREADS);
     cfg.dynamicSmemBytes = SMEM_BYTES;
-    cfg.stream = st;
+    cfg.stream = st.st;
     cfg.attrs = at;
     cfg.numAttrs = 2;
     return cfg;
@@ -326,7 +326,7 @@ cudaError_t configure_type()
 }
 
 template <typename T>
-int launch_type(const GemmCall& g, uint32_t cs, uint32_t* status, cudaStream_t st)
+int launch_type(const GemmCall& g, uint32_t cs, uint32_t* status, const LaunchStream& st)
 {
     FewArgs a{};
     a.M = g.M;
@@ -367,7 +367,7 @@ int gemm_few_tc5_clusters(uint32_t (&n)[4])
 {
     for (int i = 0; i < 4; i++) {
         cudaLaunchAttribute at[2];
-        const cudaLaunchConfig_t cfg = launch_config(at, 1u << i, 1u << i, nullptr);
+        const cudaLaunchConfig_t cfg = launch_config(at, 1u << i, 1u << i, cudaStream_t(nullptr));
         int c = 0;
         const cudaError_t e = cudaOccupancyMaxActiveClusters(&c, gemm_few_kernel<__half, 32>, &cfg);
         if (e != cudaSuccess) return int(e);
@@ -415,7 +415,7 @@ uint32_t gemm_few_tc5_cluster(const GemmCall& g, const uint32_t (&resident)[4])
     return 0;
 }
 
-int launch_gemm_few_tc5(int dtype, const GemmCall& g, uint32_t cs, uint32_t* status, cudaStream_t st)
+int launch_gemm_few_tc5(int dtype, const GemmCall& g, uint32_t cs, uint32_t* status, const LaunchStream& st)
 {
     return dtype == 0 ? launch_type<__half>(g, cs, status, st) : launch_type<__nv_bfloat16>(g, cs, status, st);
 }

@@ -719,7 +719,7 @@ Shape pick_shape(const GemmCall& g, bool rows_kernel, uint32_t kb, const GemmWor
 }
 
 template <typename T>
-int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t* status, cudaStream_t st)
+int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t* status, const LaunchStream& st)
 {
     const bool rows_kernel = !g.paged_map && g.M <= 128;
     GemmArgs a{};
@@ -824,7 +824,7 @@ bool gemm_tc5_weight_maps(GemmWeightMaps* maps, int dtype, const void* W, uint64
 
 // Returns a cudaError_t value, or -1 when the operands cannot be addressed (pointers must be 16-byte aligned, row lengths
 // multiples of 8).
-int launch_gemm_tc5(int dtype, const GemmCall& call, const GemmWorkspace& ws, uint32_t* status, cudaStream_t st, uint64_t& launched)
+int launch_gemm_tc5(int dtype, const GemmCall& call, const GemmWorkspace& ws, uint32_t* status, const LaunchStream& st, uint64_t& launched)
 {
     if (call.M == 0 || call.n_weights == 0) return 0;
     GemmCall g = call;
@@ -847,10 +847,11 @@ int launch_gemm_tc5(int dtype, const GemmCall& call, const GemmWorkspace& ws, ui
         g.A = g.norm_out;
     }
     launched++;
-    return dtype == 0 ? launch_type<__half>(g, ws, dtype, status, st) : launch_type<__nv_bfloat16>(g, ws, dtype, status, st);
+    const LaunchStream s(st.st, st.plain && !g.norm_w);          // the norm went first
+    return dtype == 0 ? launch_type<__half>(g, ws, dtype, status, s) : launch_type<__nv_bfloat16>(g, ws, dtype, status, s);
 }
 
-int launch_rmsnorm_rows(int dtype, const void* x, const void* w, void* y, uint32_t rows, uint32_t N, float eps, cudaStream_t st)
+int launch_rmsnorm_rows(int dtype, const void* x, const void* w, void* y, uint32_t rows, uint32_t N, float eps, const LaunchStream& st)
 {
     if (rows == 0) return 0;
     const bool vec = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;      // w and y are the library's own buffers

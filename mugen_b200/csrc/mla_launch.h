@@ -38,7 +38,11 @@ inline bool make_matrix_map(CUtensorMap* map, int dtype, const void* ptr, uint64
 
 int launch_append(int dtype, const void* kv_a, void* layer_pool, uint64_t pool_slots,
                    const void* norm_w, const float* cos_sin, uint32_t cs_rows, float eps,
-                   const StepMeta& m, uint32_t* status, cudaStream_t st);
+                   const StepMeta& m, uint32_t* status, const LaunchStream& st);
+
+// Page-locked host memory -> device memory in pieces of 16 bytes, both 16-byte aligned.  A kernel behind it that is not launched plain
+// (LaunchStream) starts before the copy is done.
+int launch_fetch(const void* host, void* device, uint32_t pieces, cudaStream_t st);
 
 void launch_write_rows(const void* src, void* layer_pool, uint64_t pool_slots, const uint32_t* table,
                        uint32_t row_begin, uint32_t n, uint32_t* status, cudaStream_t st);
@@ -93,13 +97,13 @@ int merge_mma_configure();
 // have been written by the kernel launched just before this one (the append blocks then wait for it before reading).
 int launch_absorb_tc5(int dtype, const void* q, const void* w_map, void* q_abs, uint32_t H, uint32_t layer0, const void* kv_a,
                       void* layer_pool, uint64_t pool_slots, const void* norm_w, const float* cos_sin, uint32_t cs_rows,
-                      float eps, const StepMeta& m, bool rotate_q, bool append_waits, uint32_t sm_count, uint32_t* status, cudaStream_t st);
+                      float eps, const StepMeta& m, bool rotate_q, bool append_waits, uint32_t sm_count, uint32_t* status, const LaunchStream& st);
 int absorb_tc5_configure();
 
 // The same merge + projection on tcgen05; w_map: host CUtensorMap over W_UV of
 // all layers, [layers*H*128 outputs][512 dims], box 64 dims x 128 outputs, 128-byte swizzle.
 int launch_merge_tc5(int dtype, const float* recs, const StepMeta& m, uint32_t n_parts, const void* w_map, void* out, uint32_t H,
-                     uint32_t layer0, uint32_t sm_count, uint32_t* status, cudaStream_t st);
+                     uint32_t layer0, uint32_t sm_count, uint32_t* status, const LaunchStream& st);
 int merge_tc5_configure();
 
 // Dense projections C = A . W^T on tcgen05 (mla_gemm_tc5.cu), up to two weights over the same activations in one launch.
@@ -132,10 +136,10 @@ struct GemmWorkspace {
     uint32_t clusters[4];      // gemm_few_tc5_clusters
 };
 // launched: kernels launched are added to it
-int launch_gemm_tc5(int dtype, const GemmCall& g, const GemmWorkspace& ws, uint32_t* status, cudaStream_t st, uint64_t& launched);
+int launch_gemm_tc5(int dtype, const GemmCall& g, const GemmWorkspace& ws, uint32_t* status, const LaunchStream& st, uint64_t& launched);
 // The same for few rows and weights that fit the SMs in one go, the norm included (mla_gemm_few_tc5.cu); launch_gemm_tc5 picks.
 uint32_t gemm_few_tc5_cluster(const GemmCall& g, const uint32_t (&resident)[4]);
-int launch_gemm_few_tc5(int dtype, const GemmCall& g, uint32_t cs, uint32_t* status, cudaStream_t st);
+int launch_gemm_few_tc5(int dtype, const GemmCall& g, uint32_t cs, uint32_t* status, const LaunchStream& st);
 int gemm_few_tc5_clusters(uint32_t (&n)[4]);
 int gemm_few_tc5_configure();
 size_t gemm_tc5_partial_bytes(uint32_t blocks);
@@ -144,7 +148,7 @@ size_t gemm_tc5_packed_values(uint64_t N, uint64_t K);
 int launch_gemm_pack(const void* src, void* dst, uint32_t N, uint32_t K, cudaStream_t st);
 bool gemm_tc5_packed_maps(GemmWeightMaps* maps, int dtype, const void* packed, uint64_t N, uint64_t K);
 bool gemm_tc5_weight_maps(GemmWeightMaps* maps, int dtype, const void* W, uint64_t rows, uint64_t K);
-int launch_rmsnorm_rows(int dtype, const void* x, const void* w, void* y, uint32_t rows, uint32_t N, float eps, cudaStream_t st);
+int launch_rmsnorm_rows(int dtype, const void* x, const void* w, void* y, uint32_t rows, uint32_t N, float eps, const LaunchStream& st);
 int gemm_tc5_configure();
 
 // Chunked prefill (mla_prefill_tc5.cu): causal flash attention of the new tokens of several sequences over expanded keys /

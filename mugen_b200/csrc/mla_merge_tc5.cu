@@ -326,7 +326,7 @@ int merge_tc5_configure()
 // swizzle).  m.layers consecutive layers from layer0; out holds them one after the other.  n_parts > 0: the records are
 // [n_parts][m.rows][H] instead of the plan's segments.
 int launch_merge_tc5(int dtype, const float* recs, const StepMeta& m, uint32_t n_parts, const void* w_map, void* out, uint32_t H,
-                     uint32_t layer0, uint32_t sm_count, uint32_t* status, cudaStream_t st)
+                     uint32_t layer0, uint32_t sm_count, uint32_t* status, const LaunchStream& st)
 {
     if (m.rows == 0) return 0;
     const CUtensorMap* map = static_cast<const CUtensorMap*>(w_map);

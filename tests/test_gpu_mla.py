@@ -1188,3 +1188,32 @@ def test_a_context_on_a_device_with_little_room_left(torch, oracle):
                 want = oracle.attention(q[l, 5 * b + t], cache, n + t + 1, case.w_uk, case.w_uv, case.w_type, H, dt)
                 check_close(_host(out[l, 5 * b + t]), want, dt, f"layer {l}, sequence {b}, token {t}")
     ctx.close()
+
+
+@pytest.mark.parametrize("n_seq, pages", [(1, 1), (85, 1), (86, 1), (300, 1), (40, 120)])
+def test_step_metadata_of_any_size_reaches_the_kernels(torch, n_seq, pages):
+    """The metadata goes up in pieces of 16 bytes, 1,024 to a block: a step of many rows, or of many pages, writes the same cache rows
+    as the same tokens one sequence to a step, whose metadata is a piece or two, and again when the steps follow each other at once."""
+    from mugen_b200.mla import MlaContext
+    rng = np.random.default_rng(n_seq)
+    norm = synth.to_bits(rng.standard_normal(512, np.float32), synth.DT_F16)
+    w = synth.to_bits(rng.standard_normal((16 * 128, 512), np.float32), synth.DT_F16)
+    kv = _dev(torch, synth.to_bits(rng.standard_normal((3, n_seq, 576), np.float32), synth.DT_F16))
+    rows = []
+    for together in (True, False):
+        ctx = MlaContext(n_layers=1, n_heads=16, dtype=synth.DT_F16, n_pages=n_seq * (pages + 1), max_seqs=n_seq, max_seq_len=64 * pages + 8, **YARN)
+        ctx.set_layer_weights(0, w, w, synth.W_F16, norm)
+        seqs = [ctx.seq_create() for _ in range(n_seq)]
+        start = torch.zeros((64 * pages - 1, 576), dtype=torch.int16, device="cuda")
+        for s in seqs:
+            ctx.write_rows(0, s, 0, start)
+            ctx.advance_seq_len(s, 64 * pages - 1)
+        for t in range(3):
+            for some in [slice(None)] if together else [slice(i, i + 1) for i in range(n_seq)]:
+                ctx.step_begin(seqs[some])
+                ctx.step_append(0, kv[t, some].contiguous())
+                ctx.step_end()
+        assert ctx.status() == 0
+        rows.append(np.stack([ctx.read_rows(0, s, 64 * pages - 1, 3) for s in seqs]))
+        ctx.close()
+    assert np.array_equal(rows[0], rows[1]) and rows[0].any(axis=(1, 2)).all()
