@@ -28,20 +28,23 @@ struct AppendArgs {          // rows == 0: no append blocks in this launch
     uint32_t wait_first;     // kv_a may be the output of the kernel just before this one in the stream
 };
 
-constexpr int kAppendRowSmem = kRow * 2 + kRank * 4;      // 3,200 bytes of shared memory per row (16-byte aligned)
+constexpr int kAppendRowSmem = kRank * 4;      // the row's squares: 2,048 bytes of shared memory per row (16-byte aligned)
 
 // One new cache row by one warp, in two steps.  `prepare` reads what the step's metadata and the constant tables hold (slot,
 // position, cos / sin, norm weights) and may run ahead of the grid dependency wait; `run` needs kv_a.  Left where they are
 // used these loads form a chain of dependent round trips to memory (~1 us each) in a kernel whose whole budget is a few
-// microseconds.  The row is normalised and rotated in place in shared memory: every element (pair) has one lane.  What
-// bounds it then is the sum of squares, a chain of 512 dependent additions (~1.1 us).
+// microseconds.  The row stays in registers, 16-byte pieces lane + 32 * k of it (pieces 64..71 are the rope dims, in lanes 0..7; the
+// pairs (i, i + 32) meet by a shuffle): only its squares go through shared memory, to the lane that adds them.
+// What bounds it is that sum, a chain of 512 dependent additions: 1.1 us, 1.3 to 2.5 measured.  (The whole row through shared memory in
+// 16-bit values, then its squares, a value at a time, and the sum without the loads ahead of it: 4.1 us for the sum, 5.5 in all; 27
+// blocks over a 777-token prompt 1806 -> 1725 us, 8 layers of 128 heads x 8 sequences by calls 456 -> 454.)
 template <typename T>
 struct AppendRow {
     bool live = false;
     uint64_t slot = 0;
     uint32_t layer = 0, row = 0;
-    float cs = 0.0f, sn = 0.0f;
-    T nw[kRank / 32];
+    uint4 nw[2];                       // norm weights of this lane's two pieces of c_kv
+    float4 cs[2], sn[2];               // lanes 0..7: cos / sin of pairs 8 * (lane % 4) .. + 7
 
     __device__ __forceinline__ void prepare(const AppendArgs& a, uint32_t layer_, uint32_t r, uint32_t* status) {
         const uint32_t lane = threadIdx.x % 32;
@@ -57,56 +60,85 @@ struct AppendRow {
             live = false;
             return;
         }
-        cs = a.cos_sin[size_t(pos) * kRope + lane];
-        sn = a.cos_sin[size_t(pos) * kRope + 32 + lane];
-        const T* norm_w = static_cast<const T*>(a.norm_w) + size_t(layer) * kRank;
+        const float4* tb = reinterpret_cast<const float4*>(a.cos_sin + size_t(pos) * kRope) + 2 * (lane % 4);
 #pragma unroll
-        for (int k = 0; k < kRank / 32; k++) nw[k] = norm_w[lane + 32 * k];
+        for (int k = 0; k < 2; k++) {
+            if (lane < 8) { cs[k] = tb[k]; sn[k] = tb[8 + k]; }
+            nw[k] = reinterpret_cast<const uint4*>(static_cast<const T*>(a.norm_w) + size_t(layer) * kRank)[lane + 32 * k];
+        }
     }
 
     __device__ __forceinline__ void run(const AppendArgs& a, unsigned char* smem) const {
         if (!live) return;
         const uint32_t lane = threadIdx.x % 32;
-        float* sq = reinterpret_cast<float*>(smem);
-        T* x = reinterpret_cast<T*>(smem + kRank * 4);
-        constexpr uint32_t kChunks = kRow * 2 / 16;   // 72 x 16 bytes
         const uint4* src = reinterpret_cast<const uint4*>(static_cast<const T*>(a.kv_a) + (size_t(layer) * a.rows + row) * kRow);
-        uint4 chunk[3];
+        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(a.pool) + (size_t(layer) * a.pool_slots + slot) * kRow);
+        uint4 x[2], rope = make_uint4(0, 0, 0, 0);
 #pragma unroll
-        for (uint32_t k = 0; k < 3; k++) if (lane + 32 * k < kChunks) chunk[k] = src[lane + 32 * k];
-        __syncwarp();                                  // the row before has left the buffer
+        for (int k = 0; k < 2; k++) x[k] = src[lane + 32 * k];
+        if (lane < 8) rope = src[64 + lane];
+        __syncwarp();                                  // the row before has been summed
+        float4* sq = reinterpret_cast<float4*>(smem);
 #pragma unroll
-        for (uint32_t k = 0; k < 3; k++) if (lane + 32 * k < kChunks) reinterpret_cast<uint4*>(x)[lane + 32 * k] = chunk[k];
-        __syncwarp();
-        float v[kRank / 32];
+        for (int k = 0; k < 2; k++) {
+            const T* e = reinterpret_cast<const T*>(&x[k]);
+            float s[8];
 #pragma unroll
-        for (int k = 0; k < kRank / 32; k++) {
-            v[k] = Elem<T>::to_f32(x[lane + 32 * k]);
-            sq[lane + 32 * k] = __fmul_rn(v[k], v[k]);
-        }
-        {
-            const float x0 = Elem<T>::to_f32(x[kRank + lane]), x1 = Elem<T>::to_f32(x[kRank + 32 + lane]);
-            x[kRank + lane]      = Elem<T>::from_f32(__fsub_rn(__fmul_rn(x0, cs), __fmul_rn(x1, sn)));
-            x[kRank + 32 + lane] = Elem<T>::from_f32(__fadd_rn(__fmul_rn(x1, cs), __fmul_rn(x0, sn)));
+            for (int j = 0; j < 8; j++) { const float f = Elem<T>::to_f32(e[j]); s[j] = __fmul_rn(f, f); }
+            sq[2 * (lane + 32 * k)] = make_float4(s[0], s[1], s[2], s[3]);
+            sq[2 * (lane + 32 * k) + 1] = make_float4(s[4], s[5], s[6], s[7]);
         }
         __syncwarp();
         float rinv = 0.0f;
         if (lane == 0) {
+            // the next eight pieces are on their way while these are added: the additions alone make the chain
+            constexpr int AHEAD = 8;
             float ss = 0.0f;
-#pragma unroll 16
-            for (int i = 0; i < kRank; i += 4) {
-                const float4 s4 = *reinterpret_cast<const float4*>(sq + i);
-                ss = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(ss, s4.x), s4.y), s4.z), s4.w);
+            float4 now[AHEAD], next[AHEAD];
+#pragma unroll
+            for (int j = 0; j < AHEAD; j++) now[j] = sq[j];
+#pragma unroll 2
+            for (int i = 0; i < kRank / 4; i += AHEAD) {
+#pragma unroll
+                for (int j = 0; j < AHEAD; j++) next[j] = sq[(i + AHEAD + j) % (kRank / 4)];
+#pragma unroll
+                for (int j = 0; j < AHEAD; j++) {
+                    ss = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(ss, now[j].x), now[j].y), now[j].z), now[j].w);
+                    now[j] = next[j];
+                }
             }
             rinv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, float(kRank)), a.eps)));
         }
+        {   // NeoX pairs (i, i + 32): piece 64 + j holds x0 of pairs 8 j .., piece 68 + j their x1
+            uint32_t mine[4] = {rope.x, rope.y, rope.z, rope.w}, other[4], y[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) other[j] = __shfl_xor_sync(0xffffffffu, mine[j], 4);
+            if (lane < 8) {
+                const float c[8] = {cs[0].x, cs[0].y, cs[0].z, cs[0].w, cs[1].x, cs[1].y, cs[1].z, cs[1].w};
+                const float s[8] = {sn[0].x, sn[0].y, sn[0].z, sn[0].w, sn[1].x, sn[1].y, sn[1].z, sn[1].w};
+                const T *em = reinterpret_cast<const T*>(mine), *eo = reinterpret_cast<const T*>(other);
+                float v[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const float fm = Elem<T>::to_f32(em[j]), fo = Elem<T>::to_f32(eo[j]);
+                    v[j] = lane < 4 ? __fsub_rn(__fmul_rn(fm, c[j]), __fmul_rn(fo, s[j])) : __fadd_rn(__fmul_rn(fm, c[j]), __fmul_rn(fo, s[j]));
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) y[j] = Elem<T>::pack2(v[2 * j], v[2 * j + 1]);
+                dst[64 + lane] = make_uint4(y[0], y[1], y[2], y[3]);
+            }
+        }
         rinv = __shfl_sync(0xffffffffu, rinv, 0);
 #pragma unroll
-        for (int k = 0; k < kRank / 32; k++) x[lane + 32 * k] = Elem<T>::from_f32(__fmul_rn(__fmul_rn(v[k], rinv), Elem<T>::to_f32(nw[k])));
-        __syncwarp();
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(a.pool) + (size_t(layer) * a.pool_slots + slot) * kRow);
+        for (int k = 0; k < 2; k++) {
+            const T *e = reinterpret_cast<const T*>(&x[k]), *w = reinterpret_cast<const T*>(&nw[k]);
+            uint32_t y[4];
 #pragma unroll
-        for (uint32_t k = 0; k < 3; k++) if (lane + 32 * k < kChunks) dst[lane + 32 * k] = reinterpret_cast<const uint4*>(x)[lane + 32 * k];
+            for (int j = 0; j < 4; j++)
+                y[j] = Elem<T>::pack2(__fmul_rn(__fmul_rn(Elem<T>::to_f32(e[2 * j]), rinv), Elem<T>::to_f32(w[2 * j])),
+                                      __fmul_rn(__fmul_rn(Elem<T>::to_f32(e[2 * j + 1]), rinv), Elem<T>::to_f32(w[2 * j + 1])));
+            dst[lane + 32 * k] = make_uint4(y[0], y[1], y[2], y[3]);
+        }
     }
 };
 
