@@ -33,6 +33,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "mla_launch.h"
 #include "mla_tc5.cuh"
@@ -101,7 +102,10 @@ struct GemmArgs {
     uint32_t* counters;                 // [tiles], pairs: [tiles][2]; zero between launches
 };
 
-struct Tile { uint32_t w, m, n; };      // which weight, tile along A's rows, tile along its outputs
+// Which weight, tile along A's rows, tile along its outputs.  What GemmArgs holds twice is chosen by a comparison: with an index that is
+// known at run time the arguments are copied to the stack first, by every thread, and each use is a load (27 blocks over a 777-token
+// prompt 1643 -> 1609 us, 32 rows of 7168 values 378 -> 377).
+struct Tile { uint32_t w, m, n; };
 __device__ __forceinline__ Tile tile_of(const GemmArgs& a, uint32_t t) {
     Tile r;
     const uint32_t per = a.group_m * (a.n_tiles[0] + a.n_tiles[1]), g = t / per, m0 = g * a.group_m, gm = m0 < a.m_tiles ? min(a.group_m, a.m_tiles - m0) : 1u, nt = (t - g * per) / gm;      // one past the end is asked for, not used
@@ -255,7 +259,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             auto same = [](uint32_t t) { return t; };
             auto load_w = [&](const Walk& x, int s) {
                 tma_load_2d(base + s * STAGE, x.t.w ? &map_w1 : &map_w0, full(s), a.packed ? 0 : int(x.k * BK),
-                            a.packed ? int((x.t.n * a.kb + x.k) * BM) : int(a.w_row0[x.t.w] + x.t.n * BM));
+                            a.packed ? int((x.t.n * a.kb + x.k) * BM) : int((x.t.w ? a.w_row0[1] : a.w_row0[0]) + x.t.n * BM));
             };
             auto load_a = [&](const Walk& x, int s) { tma_load_2d(base + s * STAGE + A_BYTES, &map_a, full(s), int(x.k * BK), int(x.t.m * NT)); };
             const uint32_t n = u1 - u0, ahead = min(n, uint32_t(STAGES));
@@ -316,7 +320,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             const uint32_t tile = u / a.kb, t_end = (tile + 1) * a.kb, end = min(u1, t_end);
             const bool cut = u != tile * a.kb || end != t_end;
             const Tile tl = tile_of(a, tile);
-            const uint32_t N = a.N[tl.w], o = tl.n * BM + r;
+            const uint32_t N = tl.w ? a.N[1] : a.N[0], o = tl.n * BM + r;
             T* out = tl.w ? out1 : out0;
             ok = ok && mbar_wait(acc_full(nt & 1), (nt >> 1) & 1, abort_flag, status);
             ok = __all_sync(0xffffffffu, ok);
@@ -417,7 +421,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             auto load_w = [&](const Walk& x, int s) {            // this block's half of the outputs, in boxes of up to 128 weight rows
                 const uint32_t o = x.t.n * NT + rank * (NT / 2);                       // first of this block's outputs
                 tma_load_2d_pair(base + s * STAGE + A_BYTES, x.t.w ? &map_w1 : &map_w0, leader_full + 8u * s, a.packed ? 0 : int(x.k * BK),
-                                 a.packed ? int(((o / BM) * a.kb + x.k) * BM + o % BM) : int(a.w_row0[x.t.w] + o));
+                                 a.packed ? int(((o / BM) * a.kb + x.k) * BM + o % BM) : int((x.t.w ? a.w_row0[1] : a.w_row0[0]) + o));
             };
             uint32_t cur_m = ~0u, next_m = ~0u, page[2] = {0, 0}, next_page[2] = {0, 0};
             auto page_of = [&](uint32_t i) { return __ldg(a.table + min(i, (a.M + kPage - 1) / kPage - 1)); };   // past the end: the last page again
@@ -511,7 +515,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             const uint32_t vt = u / a.kb, t_end = (vt + 1) * a.kb, end = min(u1, t_end), tile = tile_id(vt);
             const bool cut = u != vt * a.kb || end != t_end;
             const Tile tl = tile_of(a, tile);
-            const uint32_t N = a.N[tl.w], m0 = (2 * tl.m + rank) * BM + q4 * 32, m = m0 + lane;
+            const uint32_t N = tl.w ? a.N[1] : a.N[0], m0 = (2 * tl.m + rank) * BM + q4 * 32, m = m0 + lane;
             T* out = tl.w ? out1 : out0;
             // what the outputs are added to is requested two steps of 32 columns ahead, the first two while the tile is
             // computed: a thread's pieces lie a row apart, and each step would wait for its own round trip to memory (27 blocks
@@ -620,8 +624,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // y = T(float(x) * rsqrt(mean(x^2) + eps) * float(w)) per row (the reference's rms_norm kernel, src/metal/kernel_sources.h:
 // 264-312; step A of the driver, and q_a_norm from the ROUNDED projection).  Bound by one round trip to memory: a thread
 // keeps its values in registers between the two passes, in 16-byte pieces.  x and y may be the same buffer.
-constexpr int NORM_THREADS = 512, NORM_MAX = 4;                    // pieces of 8 values per thread held in registers
-template <typename T>
+// As many rows per SM at a time as there can be, because the next kernel's blocks start when the last row has: rows of 2,048 values in
+// blocks of 256 threads with a piece each are eight to an SM, with 512 threads and room for four pieces each they were two, 777 rows of a
+// prompt three waves, and the projection behind them began 3 us later (27 blocks, hidden 2048: 1725 -> 1656 us).
+// NORM_MAX: pieces of 8 values per thread held in registers.
+template <typename T, int NORM_THREADS, int NORM_MAX>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_rows_kernel(const T* x, const T* __restrict__ w, T* y, uint32_t N, float eps, bool vec)
 {
@@ -855,11 +862,12 @@ int launch_rmsnorm_rows(int dtype, const void* x, const void* w, void* y, uint32
 {
     if (rows == 0) return 0;
     const bool vec = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;      // w and y are the library's own buffers
-    if (dtype == 0)
-        return int(launch_pdl(rmsnorm_rows_kernel<__half>, dim3(rows), dim3(NORM_THREADS), 0, st, static_cast<const __half*>(x),
-                              static_cast<const __half*>(w), static_cast<__half*>(y), N, eps, vec));
-    return int(launch_pdl(rmsnorm_rows_kernel<__nv_bfloat16>, dim3(rows), dim3(NORM_THREADS), 0, st, static_cast<const __nv_bfloat16*>(x),
-                          static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y), N, eps, vec));
+    auto go = [&](auto* out) {
+        using T = std::remove_pointer_t<decltype(out)>;
+        const auto kernel = N <= 2048 ? rmsnorm_rows_kernel<T, 256, 1> : N <= 8192 ? rmsnorm_rows_kernel<T, 256, 4> : rmsnorm_rows_kernel<T, 512, 4>;
+        return int(launch_pdl(kernel, dim3(rows), dim3(N <= 8192 ? 256 : 512), 0, st, static_cast<const T*>(x), static_cast<const T*>(w), out, N, eps, vec));
+    };
+    return dtype == 0 ? go(static_cast<__half*>(y)) : go(static_cast<__nv_bfloat16*>(y));
 }
 
 }  // namespace mla

@@ -389,3 +389,34 @@ def test_which_input_projections_take_the_kernel_for_few_rows(torch, rows, H, E,
     assert (kv.double() - a).abs().max() <= a * 2.0 ** -10 and (q.double() - want).abs().max() <= want * 2.0 ** -9
     assert ctx.status() == 0
     ctx.close()
+
+
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+@pytest.mark.parametrize("rows,E", [(40, 2048), (777, 2048), (40, 2056), (1300, 4096), (40, 8192), (40, 8200), (33, 72)])
+def test_the_norm_ahead_of_a_projection_in_every_block_shape(torch, rows, E, dt):
+    """Blocks of 256 threads with one piece or four, of 512 with four and more: the kv_a rows are unit vectors, so that its outputs are
+    the normalised values themselves.  They are one rounding of a value whose float error (a sum of E squares, two products, a
+    reciprocal root of two units in the last place) is below 2^-17 of it."""
+    from mugen_b200.mla import MlaContext
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(rows + E)
+    tdt, code, u = (torch.float16, synth.DT_F16, 2.0 ** -11) if dt == "f16" else (torch.bfloat16, synth.DT_BF16, 2.0 ** -8)
+    bits = lambda t: t.view(torch.int16).cpu().numpy().view(np.uint16)
+    ctx = MlaContext(n_layers=1, n_heads=1, dtype=code, n_pages=2, max_seqs=1, max_seq_len=64, rope_theta=1e4, rope_scaling_factor=1.0,
+                     rope_original_ctx=4096, rms_norm_eps=1e-6)
+    at = torch.linspace(0, E - 1, 576).long() if E >= 576 else torch.arange(576) % E
+    unit = torch.zeros((576, E), dtype=tdt)
+    unit[torch.arange(576), at] = 1.0
+    zeros = torch.zeros((192, E), dtype=tdt)
+    g = (1.0 + 0.1 * torch.randn((E,), device="cuda", generator=gen)).to(tdt)
+    ctx.set_block_weights(0, attn_norm=bits(g), kv_a_mqa=bits(unit), wo=bits(torch.zeros((E, 128), dtype=tdt)), q=bits(zeros))
+    hidden = (torch.randn((rows, E), device="cuda", generator=gen) * torch.logspace(-2, 2, rows, device="cuda")[:, None]).to(tdt)
+    q, kv = torch.zeros((rows, 192), device="cuda").to(tdt), torch.zeros((rows, 576), device="cuda").to(tdt)
+    before = ctx.launch_count()
+    ctx.block_project_in(0, hidden, q, kv)
+    assert ctx.launch_count() - before == 2 and ctx.status() == 0
+    x = hidden.double()
+    want = (x * torch.rsqrt((x ** 2).mean(-1, keepdim=True) + 1e-6) * g.double())[:, at.cuda()]
+    tiny = 2.0 ** -25 if dt == "f16" else 0.0                  # half a unit of the subnormal numbers
+    assert not ((kv.double() - want).abs() > (u + 2.0 ** -17) * want.abs() + tiny).any()
+    ctx.close()
