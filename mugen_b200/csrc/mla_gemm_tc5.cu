@@ -400,7 +400,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const uint32_t u0 = a.stride ? 0u : worker * a.run, u1 = a.stride ? (tiles - worker + a.stride - 1) / a.stride * a.kb : min(a.units, u0 + a.run);
     auto tile_id = [&](uint32_t vt) -> uint32_t { return a.stride ? worker + vt * a.stride : vt; };
 
-    grid_launch_dependents();
+    if constexpr (!kPaged) grid_launch_dependents();
     if (tid == 0) {
         *abort_flag = 0;
         for (int s = 0; s < STAGES; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
@@ -471,6 +471,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
     } else if (warp == 1) {
         grid_dependency_wait();
+        // Behind the expansion comes the prefill attention, which reads its queries ahead of its own wait: it may start once the kernels
+        // before this one, and with them the queries, are done.
+        if constexpr (kPaged) grid_launch_dependents();
         if (rank == 0) {
             constexpr uint32_t IDESC = instr_desc(Fmt<T>::v, 2 * BM, NT);
             bool ok = true;

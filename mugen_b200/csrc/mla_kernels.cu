@@ -316,6 +316,7 @@ merge_outproj_mma_kernel(const float* __restrict__ recs, const RowParts* __restr
 // Once per device, with that device current (function attributes are per device).
 int merge_mma_configure()
 {
+
     cudaError_t e = cudaFuncSetAttribute(merge_outproj_mma_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMergeSmem));
     if (e != cudaSuccess) return int(e);
     e = cudaFuncSetAttribute(merge_outproj_mma_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMergeSmem));
