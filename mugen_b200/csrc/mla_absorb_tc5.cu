@@ -189,20 +189,30 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
                 ok = ok && mbar_wait(acc_full(b), (n >> 1) & 1, abort_flag, status);
                 ok = __all_sync(0xffffffffu, ok);
                 tc_fence_after();
+                // Two neighbouring lanes trade a value of every other column, so that a store carries two dims of a row: even lanes write
+                // column k, odd lanes column k + 1, 64 bytes of either per warp.  (A 16-bit store per value: 3.8 us for the 4 x 128 x 64
+                // values of a tile, 2.7 now.)
                 constexpr int CH = NT < 32 ? 16 : 32;
-                const uint32_t live = min(uint32_t(NT), a.rows - rt * NT);
+                const uint32_t live = min(uint32_t(NT), a.rows - rt * NT), odd = lane & 1;
+                const size_t pitch = size_t(a.H) * kRow;
+                T* dst0 = q_abs + ((size_t(x.li) * a.rows + rt * NT + odd) * a.H + x.h) * kRow + x.d0 * 128 + q4 * 32 + (lane - odd);
 #pragma unroll 1
                 for (uint32_t d = 0; d < n_d; d++) {
-                    T* dst = q_abs + ((size_t(x.li) * a.rows + rt * NT) * a.H + x.h) * kRow + (x.d0 + d) * 128 + q4 * 32 + lane;
 #pragma unroll 1
                     for (uint32_t c = 0; c < NT; c += CH) {
                         if (c >= live) break;
                         uint32_t o[CH];
                         tc_ldn(tmem + ((q4 * 32u) << 16) + b * 4 * NT + d * NT + c, o);
                         tc_wait_ld();
+                        T* dst = dst0 + d * 128 + c * pitch;
 #pragma unroll
-                        for (int k = 0; k < CH; k++)
-                            if (ok && c + k < live) dst[size_t(c + k) * a.H * kRow] = Elem<T>::from_f32(__uint_as_float(o[k]));
+                        for (int k = 0; k < CH; k += 2) {
+                            const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? o[k] : o[k + 1], 1);
+                            const uint32_t w = odd ? Elem<T>::pack2(__uint_as_float(got), __uint_as_float(o[k + 1]))
+                                                   : Elem<T>::pack2(__uint_as_float(o[k]), __uint_as_float(got));
+                            if (ok && c + k + odd < live) *reinterpret_cast<uint32_t*>(dst) = w;
+                            dst += 2 * pitch;
+                        }
                     }
                 }
                 tc_fence_before();
@@ -214,6 +224,21 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
     } else {
         // ---- query rows: q_nope -> operand rows, q_rope -> behind the absorbed dims (by the unit that has d-tile 0)
         Unit x = unit_of(u0);                      // the divisions not behind the wait
+        // Rows of many steps lie far apart and have not been touched for a pass over the cache: the first load of a tile took 5 us from the
+        // wait on, W_UK was there after 2 (16 sequences x 5 rows to verify, with the epilogue's wider stores 324.6 -> 320.2 us; 32
+        // sequences through three blocks of 128 heads 375 -> 372).  L2 is the point of coherence, so asking ahead of the wait is safe.  (Not with one tile of up to
+        // 16 rows, which the kernel before may just be writing: 27 blocks of 4 sequences 757 -> 761 us.)
+        if constexpr (NT > 16) {
+            for (uint32_t u = u0; u < u1; u++) {
+                const Unit y = unit_of(u);
+                const uint32_t ra = y.rt0 * NT, n = min(a.rows, y.rt1 * NT) - ra;
+                for (uint32_t i = tid - FIRST_QUERY * 32; i < 3 * n; i += 128) {
+                    const uint32_t r = ra + i / 3;
+                    const T* p = q + ((size_t(y.li) * a.rows + (a.att_row ? a.att_row[r] : r)) * a.H + y.h) * kQDim + (i % 3) * 64;
+                    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));
+                }
+            }
+        }
         grid_dependency_wait();
         const uint32_t t = tid - FIRST_QUERY * 32;
         bool ok = true;
