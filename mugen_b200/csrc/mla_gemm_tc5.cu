@@ -46,13 +46,22 @@ using namespace tc5;
 
 constexpr int BM = 128, BK = 64;                         // M side of one block's MMA, k-block
 constexpr int A_BYTES = BM * BK * 2;                     // 16,384
-constexpr int NUM_THREADS = 32 * 6;
+// gemm_rows_kernel: a tcgen05.mma costs its issuing warp about 130 cycles whatever its size, 510 per k-block.  HBM does not bring k-blocks
+// faster, but those that were requested ahead of the wait are all there behind it.  So with up to 32 rows three warps issue, into
+// accumulators of their own that the epilogue adds in their order (three blocks of 128 heads x 32 rows, hidden 7168, with fewer
+// stages 374 -> 367 us; input projections of 4 to 32 rows 1 to 5 % shorter, output projections between 2 % shorter and 1.5 % longer).
+// With more rows reading three accumulators costs more than that (33 to 128 rows, seven shapes: 3 to 10 % slower); a fourth issuer
+// would be the ninth warp of the block and leave a thread 168 registers, of which the sums of cut tiles spill hundreds.
+constexpr int rows_issuers(int nt) { return nt <= 32 ? 3 : 1; }
+constexpr int rows_threads(int nt) { return 32 * (1 + rows_issuers(nt) + 4); }
 constexpr int EPI_WARPS = 8, PAIR_THREADS = 32 * (2 + EPI_WARPS);        // gemm_pair_kernel: two epilogue warps per 32 rows
 constexpr int STORE_BYTES = 32 * 128;                    // a warp's box of 64 outputs x 32 rows on its way out
 constexpr int MISC_BYTES = 256;
 // gemm_rows_kernel: [128 weight rows][NT rows of A] per stage
 constexpr int rows_stage(int nt) { return A_BYTES + nt * BK * 2; }
-constexpr int rows_stages(int nt) { return nt == 128 ? 6 : nt == 64 ? 8 : nt == 32 ? 10 : 11; }
+// (More stages are not faster: with what fits, 12 / 11 / 9 / 7, three blocks of 128 heads x 32 rows take 371 us, 367 with these, and
+// projections of 33 to 128 rows up to a tenth more.)
+constexpr int rows_stages(int nt) { return nt == 128 ? 6 : nt == 64 ? 8 : nt == 32 ? 8 : 9; }
 constexpr int rows_smem(int nt) { return rows_stages(nt) * rows_stage(nt) + MISC_BYTES + 1024; }      // + slack for 1 KB alignment
 // gemm_pair_kernel: [128 rows of A][NT / 2 weight rows] per block and stage
 constexpr int pair_stage(int nt) { return A_BYTES + nt / 2 * BK * 2; }
@@ -60,7 +69,7 @@ constexpr int pair_stages(int nt) { return nt == 256 ? 6 : 8; }
 constexpr int pair_off_store(int nt) { return pair_stages(nt) * pair_stage(nt); }
 constexpr int pair_smem(int nt) { return pair_off_store(nt) + EPI_WARPS * STORE_BYTES + MISC_BYTES + 1024; }
 static_assert(BK == 64, "the box width of make_matrix_map");
-static_assert(rows_smem(16) <= 232448 && rows_smem(128) <= 232448 && pair_smem(256) <= 232448 && pair_smem(128) <= 232448, "shared memory of one block");
+static_assert(rows_smem(16) <= 232448 && rows_smem(32) <= 232448 && rows_smem(64) <= 232448 && rows_smem(128) <= 232448 && pair_smem(256) <= 232448 && pair_smem(128) <= 232448, "shared memory of one block");
 
 // Pairs with whole tiles take them in turn, so that those which compute at one time stand side by side in the line of tiles and
 // ask for the same rows of A, or the same weights, at about the same time: such requests are merged on the way to L2.  How many
@@ -160,14 +169,14 @@ __device__ __forceinline__ void load_acc(uint32_t addr, float (&v)[CH]) {
 template <int THREADS>
 __device__ __forceinline__ void epilogue_sync() { asm volatile("barrier.cta.sync 1, %0;\n" ::"n"(THREADS) : "memory"); }
 
-// The epilogue threads hand a cut tile's accumulator (row r of it, NT columns, at tensor-memory address acc; a thread's share are
-// columns c0*CH .. c1*CH - 1) over: partial to global memory, then the tile's counter.  Returns true in the worker that arrived
+// The epilogue threads hand a cut tile's accumulator (row r of it, NT columns, load(c, v) brings CH of them from column c*CH; a thread's
+// share are columns c0*CH .. c1*CH - 1) over: partial to global memory, then the tile's counter.  Returns true in the worker that arrived
 // last; sum_partials then gives columns c*CH.. of the whole tile.  Worker w's slots are 2w (the tile its run begins in) and
 // 2w + 1 (the one it ends in).  last_slot is one word: who writes it for the next cut tile has passed that tile's first barrier, and
 // everyone arrives there with this tile's value read.  (With two fences and a third barrier instead of the atomic that releases and
 // acquires: 32 heads, hidden 2048, 129 rows, output projection 21.9 us, 20.9 now; 96 heads 29.9, 29.1.)
-template <int NT, int CH, int THREADS, typename Release>
-__device__ __forceinline__ bool hand_over(const GemmArgs& a, uint32_t worker, uint32_t blocks_per_worker, uint32_t rank, uint32_t tile, uint32_t acc,
+template <int NT, int CH, int THREADS, typename Load, typename Release>
+__device__ __forceinline__ bool hand_over(const GemmArgs& a, uint32_t worker, uint32_t blocks_per_worker, uint32_t rank, uint32_t tile, Load load,
                                           uint32_t r, int c0, int c1, bool first_thread, bool ok, volatile uint32_t* last_slot, Release release)
 {
     const uint32_t t0 = tile * a.kb;
@@ -175,7 +184,7 @@ __device__ __forceinline__ bool hand_over(const GemmArgs& a, uint32_t worker, ui
 #pragma unroll 1
     for (int c = c0; c < c1; c++) {
         float v[CH];
-        load_acc(acc + c * CH, v);
+        load(c, v);
         if (c + 1 == c1) release();
 #pragma unroll
         for (int i = 0; i < CH / 4; i++) __stcg(slot + (c * (CH / 4) + i) * 128 + r, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
@@ -219,12 +228,14 @@ __device__ __forceinline__ void sum_partials(const GemmArgs& a, uint32_t blocks_
 }
 
 template <typename T, int NT>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(rows_threads(NT), 1)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
                  T* __restrict__ out0, T* __restrict__ out1, const GemmArgs a, uint32_t* __restrict__ status)
 {
     constexpr int STAGES = rows_stages(NT), STAGE = rows_stage(NT), OFF_MISC = STAGES * STAGE;
-    constexpr uint32_t TMEM_COLS = 2 * NT;
+    constexpr int ISSUERS = rows_issuers(NT), FIRST_EPI = 1 + ISSUERS;
+    constexpr uint32_t TMEM_COLS = ISSUERS == 1 ? 2 * NT : 8 * NT;          // a power of two
+    static_assert(TMEM_COLS <= 512 && TMEM_COLS >= 2 * ISSUERS * NT && ISSUERS <= STAGES);
     extern __shared__ unsigned char gemm_smem[];
     const uint32_t raw = smem_u32(gemm_smem);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -245,7 +256,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     if (tid == 0) {
         *abort_flag = 0;
         for (int s = 0; s < STAGES; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
-        for (uint32_t b = 0; b < 2; b++) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 128); }
+        for (uint32_t b = 0; b < 2; b++) { mbar_init(acc_full(b), ISSUERS); mbar_init(acc_empty(b), 128); }
         mbar_init_fence();
     }
     if (warp == 1) tc_alloc<TMEM_COLS>(tmem_slot);
@@ -282,20 +293,26 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 if (++s == STAGES) { s = 0; par ^= 1; }
             }
         }
-    } else if (warp == 1) {
+    } else if (warp < FIRST_EPI) {
+        // ---- issuer p takes the k-blocks of stages p, p + ISSUERS, .. : a stage belongs to one issuer (mla_few_ring.h has the reason)
         constexpr uint32_t IDESC = instr_desc(Fmt<T>::v, BM, NT);
         grid_dependency_wait();
+        const uint32_t p = warp - 1, n = u1 - u0;
         bool ok = true;
-        uint32_t nt = 0, par = 0;
-        int s = 0;
-        for (uint32_t u = u0; u < u1 && ok; nt++) {
-            const uint32_t end = min(u1, (u / a.kb + 1) * a.kb);
+        uint32_t nt = 0, i = p, par = 0;              // tiles so far, this issuer's k-block, its phase
+        int s = int(p);                               // and stage
+        for (uint32_t u = 0; u < n && ok; nt++) {
+            const uint32_t end = min(n, ((u0 + u) / a.kb + 1) * a.kb - u0), d = tmem + ((nt & 1) * ISSUERS + p) * NT;
             ok = mbar_wait(acc_empty(nt & 1), ((nt >> 1) & 1) ^ 1, abort_flag, status);
             if (!ok) break;
-            const uint32_t d = tmem + (nt & 1) * NT;
-            for (bool first = true; u < end && ok; u++, first = false) {
+            if (i >= end && lane == 0) mbar_arrive(acc_full(nt & 1));          // none of this tile's
+            __syncwarp();
+            for (bool first = true; i < end; first = false) {
                 ok = mbar_wait(full(s), par, abort_flag, status);
                 if (!ok) break;
+                uint32_t next = i + ISSUERS;
+                int s2 = s + ISSUERS;
+                if (s2 >= STAGES) { next = i + STAGES - s + p; s2 = int(p); }
                 tc_fence_after();
                 if (elect_one()) {
                     const uint32_t da = desc_lo(base + s * STAGE), db = desc_lo(base + s * STAGE + A_BYTES);
@@ -303,11 +320,14 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     for (int k = 0; k < BK / 16; k++)
                         tc_mma(d, da + ((k * 32) >> 4), desc_hi(1024), db + ((k * 32) >> 4), desc_hi(1024), IDESC, (first && k == 0) ? 0u : 1u);
                     tc_commit(empty(s));
-                    if (u + 1 == end) tc_commit(acc_full(nt & 1));
+                    if (next >= end) tc_commit(acc_full(nt & 1));
                 }
                 __syncwarp();
-                if (++s == STAGES) { s = 0; par ^= 1; }
+                if (s2 <= s) par ^= 1;
+                s = s2;
+                i = next;
             }
+            u = end;
         }
     } else {
         // epilogue: warp w reads TMEM lanes 32*(w%4) .. +31; thread = one weight row (output), columns = rows of A
@@ -322,24 +342,42 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             const Tile tl = tile_of(a, tile);
             const uint32_t N = tl.w ? a.N[1] : a.N[0], o = tl.n * BM + r;
             T* out = tl.w ? out1 : out0;
+            uint32_t live = (1u << ISSUERS) - 1;              // issuers that have a k-block of this tile
+            if (ISSUERS > 1 && end - u < uint32_t(STAGES)) {
+                live = 0;
+                for (uint32_t i = u - u0; i < end - u0; i++) live |= 1u << (i % STAGES % ISSUERS);
+            }
             ok = ok && mbar_wait(acc_full(nt & 1), (nt >> 1) & 1, abort_flag, status);
             ok = __all_sync(0xffffffffu, ok);
             tc_fence_after();
-            const uint32_t acc = tmem + ((q4 * 32u) << 16) + (nt & 1) * NT;
+            const uint32_t acc = tmem + ((q4 * 32u) << 16) + (nt & 1) * ISSUERS * NT;
+            auto load = [&](int c, float (&v)[CH]) {
+                if constexpr (ISSUERS == 1) { load_acc(acc + c * CH, v); return; }
+#pragma unroll
+                for (int i = 0; i < CH; i++) v[i] = 0.0f;
+#pragma unroll
+                for (int p = 0; p < ISSUERS; p++) {
+                    if (!(live >> p & 1)) continue;
+                    float x[CH];
+                    load_acc(acc + p * NT + c * CH, x);
+#pragma unroll
+                    for (int i = 0; i < CH; i++) v[i] += x[i];
+                }
+            };
             auto release = [&]() { tc_fence_before(); mbar_arrive(acc_empty(nt & 1)); };
-            // columns c*CH.. of the tile, complete: round and store
+            // columns from c*C on of the tile, complete: round and store
             auto finish = [&](int c, const float (&v)[CH]) {
                 if (o >= N || !ok) return;
-                const uint32_t m0 = tl.m * NT + c * CH, live = min(uint32_t(CH), a.M > m0 ? a.M - m0 : 0u);
+                const uint32_t m0 = tl.m * NT + c * CH, rows = min(uint32_t(CH), a.M > m0 ? a.M - m0 : 0u);
                 T* p = out + size_t(m0) * N + o;
                 T res[CH];                                         // all of them on their way before the first store
                 if (a.residual) {
 #pragma unroll
-                    for (int i = 0; i < CH; i++) if (uint32_t(i) < live) res[i] = p[size_t(i) * N];
+                    for (int i = 0; i < CH; i++) if (uint32_t(i) < rows) res[i] = p[size_t(i) * N];
                 }
 #pragma unroll
                 for (int i = 0; i < CH; i++) {
-                    if (uint32_t(i) >= live) continue;
+                    if (uint32_t(i) >= rows) continue;
                     T x = Elem<T>::from_f32(v[i]);
                     if (a.residual) x = Elem<T>::from_f32(Elem<T>::to_f32(res[i]) + Elem<T>::to_f32(x));
                     p[size_t(i) * N] = x;
@@ -349,11 +387,11 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll 1
                 for (int c = 0; c < NT / CH; c++) {
                     float v[CH];
-                    load_acc(acc + c * CH, v);
+                    load(c, v);
                     if (c + 1 == NT / CH) release();
                     finish(c, v);
                 }
-            } else if (hand_over<NT, CH, 128>(a, blockIdx.x, 1, 0, tile, acc, r, 0, NT / CH, r == 0, ok, last_slot, release)) {
+            } else if (hand_over<NT, CH, 128>(a, blockIdx.x, 1, 0, tile, load, r, 0, NT / CH, r == 0, ok, last_slot, release)) {
 #pragma unroll 1
                 for (int c = 0; c < NT / CH; c++) {
                     float v[CH];
@@ -599,7 +637,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     if (c + 2 == c_first + CHUNKS) release();
                     finish(c + 1, v, rs1);
                 }
-            } else if (hand_over<NT, CH, 32 * EPI_WARPS>(a, worker, 2, rank, tile, acc, r, c_first, c_first + CHUNKS, tid == 64, ok, last_slot, release)) {
+            } else if (hand_over<NT, CH, 32 * EPI_WARPS>(a, worker, 2, rank, tile, [&](int c, float (&v)[CH]) { load_acc(acc + c * CH, v); }, r, c_first, c_first + CHUNKS, tid == 64, ok, last_slot, release)) {
 #pragma unroll 1
                 for (int c = c_first; c < c_first + CHUNKS; c += 2) {
                     float v[CH];
@@ -775,7 +813,7 @@ int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t*
     const CUtensorMap &m0 = map_of(0), &m1 = map_of(last), &pa = g.paged_map ? *g.paged_map : ma;
     if (rows_kernel) {
         auto go = [&](auto kernel) {
-            return int(launch_pdl(kernel, dim3(workers), dim3(NUM_THREADS), size_t(rows_smem(int(nt))), st, pa, m0, m1, out[0], out[1], a, status));
+            return int(launch_pdl(kernel, dim3(workers), dim3(rows_threads(int(nt))), size_t(rows_smem(int(nt))), st, pa, m0, m1, out[0], out[1], a, status));
         };
         return nt == 16 ? go(gemm_rows_kernel<T, 16>) : nt == 32 ? go(gemm_rows_kernel<T, 32>)
              : nt == 64 ? go(gemm_rows_kernel<T, 64>) : go(gemm_rows_kernel<T, 128>);

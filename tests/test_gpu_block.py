@@ -420,3 +420,40 @@ def test_the_norm_ahead_of_a_projection_in_every_block_shape(torch, rows, E, dt)
     tiny = 2.0 ** -25 if dt == "f16" else 0.0                  # half a unit of the subnormal numbers
     assert not ((kv.double() - want).abs() > (u + 2.0 ** -17) * want.abs() + tiny).any()
     ctx.close()
+
+
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+@pytest.mark.parametrize("rows", [1, 16, 17, 32, 33, 128])
+@pytest.mark.parametrize("E", [64, 136, 200, 320, 704])
+def test_projections_whose_tiles_have_fewer_k_blocks_than_issuers(torch, E, rows, dt):
+    """The general kernel of up to 128 rows (155 tiles are more than the device has SMs, which the one for few rows does not take) with
+    up to 32 rows deals a block's k-blocks out to three issuers with accumulators of their own: whole tiles of 1 to 11 k-blocks, and in
+    the output projection tiles of 200 k-blocks cut into runs of a few, so that an issuer has none, one or several of a tile."""
+    from mugen_b200.mla import MlaContext
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(rows * 17 + E)
+    tdt, code, u = (torch.float16, synth.DT_F16, 2.0 ** -11) if dt == "f16" else (torch.bfloat16, synth.DT_BF16, 2.0 ** -8)
+    H, QD, VD = 100, 19200, 12800
+    rn = lambda *shape, scale=1.0: (torch.randn(shape, device="cuda", generator=gen) * scale).to(tdt)
+    bits = lambda t: t.view(torch.int16).cpu().numpy().view(np.uint16)
+    ctx = MlaContext(n_layers=1, n_heads=H, dtype=code, n_pages=2, max_seqs=1, max_seq_len=64, rope_theta=1e4, rope_scaling_factor=1.0,
+                     rope_original_ctx=4096, rms_norm_eps=1e-6)
+    w = dict(attn_norm=1 + rn(E, scale=0.1), kv_a_mqa=rn(576, E, scale=E ** -0.5), wo=rn(E, VD, scale=VD ** -0.5), q=rn(QD, E, scale=E ** -0.5))
+    ctx.set_block_weights(0, **{k: bits(v) for k, v in w.items()})
+    hidden, att = rn(rows, E), rn(rows, VD)
+    q, kv, out = torch.zeros((rows, QD), device="cuda").to(tdt), torch.zeros((rows, 576), device="cuda").to(tdt), hidden.clone()
+    before = ctx.launch_count()
+    ctx.block_project_in(0, hidden, q, kv)
+    ctx.block_project_out(0, att, out)
+    assert ctx.status() == 0 and ctx.launch_count() - before == 3
+    x = (hidden.double() * torch.rsqrt((hidden.double() ** 2).mean(-1, keepdim=True) + 1e-6) * w["attn_norm"].double()).to(tdt).double()
+    # one rounding of the output (two with the residual), and as the bound beside it six units of the storage type on sums of order one:
+    # where the normalised rows round the other way than here
+    for got, want, n in ((q, x @ w["q"].double().T, 1), (kv, x @ w["kv_a_mqa"].double().T, 1),
+                         (out, hidden.double() + (att.double() @ w["wo"].double().T).to(tdt).double(), 2)):
+        assert not ((got.double() - want).abs() > u * (n * want.abs() + 6)).any()
+    q2, out2 = torch.zeros_like(q), hidden.clone()
+    ctx.block_project_in(0, hidden, q2, kv)
+    ctx.block_project_out(0, att, out2)
+    assert torch.equal(q, q2) and torch.equal(out, out2)
+    ctx.close()
