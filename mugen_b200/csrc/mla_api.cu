@@ -179,8 +179,16 @@ size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
 // Sequences that take at least this many new tokens in a step go through the prefill kernels.
 constexpr uint32_t kPrefillMin = 64;
-// Most query rows and bytes of absorbed queries of a group of layers (step_layers_grouped).
-constexpr uint64_t kGroupRows = 1024, kGroupBytes = 48ull << 20;
+// Most query rows and bytes of absorbed queries of a group of layers (mla_step_layers).  Queries and partial states of a group this
+// large do not stay in L2 between its launches, and that costs less than the start, the drain and the uneven last segments of more
+// launches: 1024 rows and 48 MB against these, 27 layers of 16 heads, 16 sequences x 5 rows 321 -> 305 us, 64 x 8 rows 1312 -> 969,
+// 40 single rows 201 -> 176, 128 of 2000 tokens 1470 -> 1415; 6 layers of 64 heads x 120 ragged sequences 334 -> 287; 3 layers of 128
+// heads x 128 837 -> 830; slower in one of 27 shapes (4 layers of 128 heads, 30 sequences x 4 rows: 466 -> 468).  160 MB give no more.
+constexpr uint64_t kGroupRows = 4096, kGroupBytes = 96ull << 20;
+// The smaller ones where less of the device is free when a context is made: what it or its caller allocates later (expanded keys of a
+// long prompt, weights) has the room that it had.
+constexpr uint64_t kSmallGroupRows = 1024, kSmallGroupBytes = 48ull << 20;
+constexpr size_t kRoomForGroups = 16ull << 30;
 // Expanded keys and values of the chunks that share a launch (a chunk that needs more has one of its own).
 constexpr uint64_t kExpandBytes = 256ull << 20;
 
@@ -801,11 +809,15 @@ int mla_create(const mla_config* cfg, mla_ctx** out)
     // rotary table: one row per position a sequence can reach
     c->cs_cap = std::max(cfg->max_seq_len, cfg->max_position);
     CR_TRY(cudaMalloc(&c->cos_sin, size_t(c->cs_cap) * mla::kRope * sizeof(float)));
-    // Workspace for the rows of one step, or of a group of layers when a step has few rows (step_layers_grouped): the
-    // absorbed queries of a group stay within kGroupBytes, so that they and the partial states stay in L2 between launches.
+    // Workspace for the rows of one step, or of a group of layers when a step has few rows (mla_step_layers).
     const uint64_t row_bytes = uint64_t(H) * mla::kRow * 2;
-    c->ws_rows = std::max<uint32_t>(c->cfg.max_rows, uint32_t(std::min<uint64_t>({uint64_t(c->cfg.max_rows) * cfg->n_layers, kGroupRows,
-                                                                                  std::max<uint64_t>(1, kGroupBytes / row_bytes)})));
+    auto group_rows = [&](uint64_t rows, uint64_t bytes) {
+        return std::max<uint32_t>(c->cfg.max_rows, uint32_t(std::min<uint64_t>({uint64_t(c->cfg.max_rows) * cfg->n_layers, rows,
+                                                                                std::max<uint64_t>(1, bytes / row_bytes)})));
+    };
+    size_t free_bytes = 0, total_bytes = 0;
+    CR_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+    c->ws_rows = free_bytes >= kRoomForGroups ? group_rows(kGroupRows, kGroupBytes) : group_rows(kSmallGroupRows, kSmallGroupBytes);
     CR_TRY(cudaMalloc(&c->status_dev, sizeof(uint32_t)));
     CR_TRY(cudaMemset(c->status_dev, 0, sizeof(uint32_t)));
     c->meta_cap = meta_capacity(cp);

@@ -1217,3 +1217,13 @@ def test_step_metadata_of_any_size_reaches_the_kernels(torch, n_seq, pages):
         rows.append(np.stack([ctx.read_rows(0, s, 64 * pages - 1, 3) for s in seqs]))
         ctx.close()
     assert np.array_equal(rows[0], rows[1]) and rows[0].any(axis=(1, 2)).all()
+
+
+@pytest.mark.parametrize("H,dt,L,rows", [
+    (5, synth.DT_F16, 27, 60),         # 1,620 rows: one group
+    (16, synth.DT_BF16, 27, 101),      # 2,727 of the 2,730 that 96 MB of queries hold
+    (16, synth.DT_F16, 9, 304),        # 2,736: five layers and four
+    (5, synth.DT_BF16, 9, 456),        # 4,104 of 4,096: five and four
+])
+def test_groups_of_layers_of_thousands_of_rows(torch, H, dt, L, rows):
+    test_step_layers_in_groups_of_layers(torch, H, dt, L, [(29 * i) % 150 for i in range(rows)])
