@@ -145,6 +145,7 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
         return;
     }
 
+    if (tid == 64) { prefetch_map(&map_q); prefetch_map(&map_sub); prefetch_map(&map_kv64); }
     // one barrier per thread of warp 0 (31 of them): initialised in one step instead of 31 by a single thread
     if (warp == 0) {
         if (lane == 0) {

@@ -116,6 +116,7 @@ decode_tc5_t16_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid
     const uint32_t seg_begin = m.cta_seg_begin[cta], seg_end = m.cta_seg_begin[cta + 1];
 
     grid_launch_dependents();
+    if (tid == 64) { prefetch_map(&map_q); prefetch_map(&map_pair); prefetch_map(&map_sub); }
     if (tid == 0) {
         *abort_flag = 0;
         mbar_init(bar(B_QFULL), 1);

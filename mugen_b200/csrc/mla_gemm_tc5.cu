@@ -253,6 +253,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const uint32_t u0 = blockIdx.x * a.run, u1 = min(a.units, u0 + a.run);       // this block's run of units
 
     grid_launch_dependents();
+    if (tid == 64) prefetch_map(&map_a);
     if (tid == 0) {
         *abort_flag = 0;
         for (int s = 0; s < STAGES; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
@@ -439,6 +440,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     auto tile_id = [&](uint32_t vt) -> uint32_t { return a.stride ? worker + vt * a.stride : vt; };
 
     if constexpr (!kPaged) grid_launch_dependents();
+    if (tid == 64) { prefetch_map(&map_a); prefetch_map(&map_c0); prefetch_map(&map_c1); }
     if (tid == 0) {
         *abort_flag = 0;
         for (int s = 0; s < STAGES; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }

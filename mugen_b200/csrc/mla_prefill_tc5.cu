@@ -118,6 +118,7 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
         if (lane == 0) mbar_arrive(bar(i));
     };
     grid_launch_dependents();
+    if (tid == 64) { prefetch_map(&map_k); prefetch_map(&map_v); prefetch_map(&map_r); }
     if (warp == 0 && lane < B_COUNT) {
         const int i = int(lane);
         mbar_init(bar(i), i == B_QFULL ? 8u : i >= B_SEMPTY && i < B_PFULL + S_BUFS ? 4u : 1u);
