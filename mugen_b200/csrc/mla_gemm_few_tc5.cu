@@ -10,10 +10,12 @@
 //   * a cluster of 1, 2, 4 or 8 blocks takes one tile of 128 outputs, every block an equal share of K: the sums meet in the
 //     blocks' shared memory (each block finishes the rows c = rank, rank + cluster size, ..), in the order of the ranks;
 //   * four warps issue the MMAs, into accumulators of their own that the epilogue adds in a fixed order;
-//   * the rows come by ordinary loads, so that their normalisation needs no pass of its own: a block sums the squares of its
-//     share of K, the cluster exchanges the sums, and the rounded values go to the operand tile.
-// 27 blocks of 16 heads x 4 rows: 937 -> 808 us per step.  The parts of its seven microseconds there: rows loaded 1.0, sums exchanged
-// 0.8, normalised 1.0, MMAs 1.0, sums to their blocks 0.9, stored and left 0.8.
+//   * the rows come by ordinary loads, so that their normalisation needs no pass of its own: every warp sums the squares of its rows,
+//     or, where they are long, those of its block's share of K, and the cluster exchanges the sums; the rounded values go to the
+//     operand tile.
+// 27 blocks of 16 heads x 4 rows: 937 -> 808 us per step, 752 -> 701 with whole rows summed by their warp (the exchange had taken 1.25 of
+// a projection's seven microseconds) and with kernels of less code.  The parts of what is left: rows loaded 0.6, squares 0.4, normalised
+// 0.8, MMAs 1.1, sums to their blocks 0.9, stored and left 0.6.
 #include <cuda.h>
 
 #include <algorithm>
@@ -57,17 +59,51 @@ struct FewArgs {
     uint32_t cs, cs_log2;               // blocks of a cluster
     uint32_t split, split_log2;         // row warps that share a row (up to four rows)
     uint32_t n_tiles0, N[2];            // tiles of the first weight; outputs of each
-    uint32_t residual;
+    uint32_t residual, whole;
     float eps;
 };
 
-template <typename T, int NT>
+// Sums of squares of a warp's rows (pitch 8 rows) in pieces of 8 values, in every lane; eight loads of a lane in flight.
+template <typename T, int ROWS>
+__device__ __forceinline__ void row_squares(const T* row0, size_t pitch, uint32_t rows, uint32_t pieces, uint32_t lane, float (&sum)[ROWS]) {
+    constexpr int PER = 8 / ROWS;
+    float s[ROWS][4] = {};
+    for (uint32_t c0 = lane; c0 < pieces; c0 += 32 * PER) {
+        uint4 v[ROWS][PER];
+#pragma unroll
+        for (int r = 0; r < ROWS; r++)
+#pragma unroll
+            for (int i = 0; i < PER; i++)
+                v[r][i] = uint32_t(r) < rows && c0 + 32 * i < pieces ? load_here(row0 + r * pitch + size_t(c0 + 32 * i) * 8) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int r = 0; r < ROWS; r++)
+#pragma unroll
+            for (int i = 0; i < PER; i++) {
+                const T* f = reinterpret_cast<const T*>(&v[r][i]);
+#pragma unroll
+                for (int j = 0; j < 8; j++) { const float y = Elem<T>::to_f32(f[j]); s[r][j % 4] += y * y; }
+            }
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) {
+        float t = (s[r][0] + s[r][1]) + (s[r][2] + s[r][3]);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+        sum[r] = t;
+    }
+}
+// ROWS: rows of a row warp, at most.  Norm: none, the cluster's blocks exchange their shares of a row's squares, every warp sums its whole
+// rows itself, or any of them.  A kernel of its own for each is the faster one, by what it does not have to fetch of its own code: all
+// of them and all numbers of rows in one, 16 heads x 9 to 32 rows, hidden 2048, 5 to 20 % slower.  With up to 8 rows, where that is least,
+// one kernel for both projections of a block is the better choice yet (27 blocks of 4 sequences 709 us with two, 699 with one).
+enum NormKind { kNoNorm = 0, kExchange = 1, kWhole = 2, kAny = 3 };
+template <typename T, int NT, int ROWS, int Norm>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_few_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1, const T* x,
                 const T* norm_w, T* out0, T* out1, const FewArgs a, uint32_t* __restrict__ status)
 {
     constexpr uint32_t TMEM_COLS = ISSUERS * NT;
-    constexpr int ROWS = NT / ROW_WARPS, PER = max_kblocks(NT) * 8 / 32;      // rows of a row warp, pieces of 8 values per lane and row, at most
+    constexpr int PER = max_kblocks(NT) * 8 / 32;      // pieces of 8 values per lane and row, at most
     extern __shared__ unsigned char few_smem[];
     const uint32_t raw = smem_u32(few_smem);                    // every block of a cluster sees the same offset
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -148,7 +184,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constan
         auto row_of = [&](int r) -> uint32_t { return (e >> a.split_log2) + ROW_WARPS * r; };
         auto piece = [&](int k) -> uint32_t { return lane + 32 * (part + a.split * k); };
         uint4 g[PER];
-        if (norm_w) {
+        if (Norm != kNoNorm && (Norm != kAny || norm_w)) {
 #pragma unroll
             for (int k = 0; k < PER; k++) {
                 const uint32_t c = piece(k);
@@ -179,7 +215,28 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constan
                 if (c < pieces && p0 + c < n_pieces) v[r][k] = load_here(x + size_t(row) * a.K + size_t(p0 + c) * 8);
             }
         }
-        if (norm_w && my_rows) {
+        // row r of this warp as the projection takes it
+        auto normalise = [&](int r, float inv) {
+#pragma unroll
+            for (int k = 0; k < PER; k++) {
+                if (32 * a.split * k >= pieces) break;
+                const T *f = reinterpret_cast<const T*>(&v[r][k]), *w = reinterpret_cast<const T*>(&g[k]);
+                uint32_t y[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    y[j] = Elem<T>::pack2(Elem<T>::to_f32(f[2 * j]) * inv * Elem<T>::to_f32(w[2 * j]), Elem<T>::to_f32(f[2 * j + 1]) * inv * Elem<T>::to_f32(w[2 * j + 1]));
+                v[r][k] = make_uint4(y[0], y[1], y[2], y[3]);
+            }
+        };
+        if (Norm == kWhole || (Norm == kAny && a.whole)) {
+            if (my_rows) {
+                float sum[ROWS];
+                row_squares<T, ROWS>(x + size_t(row_of(0)) * a.K, size_t(ROW_WARPS) * a.K, my_rows, n_pieces, lane, sum);
+#pragma unroll
+                for (int r = 0; r < ROWS; r++)
+                    if (uint32_t(r) < my_rows) normalise(r, rsqrtf(sum[r] / float(a.K) + a.eps));
+            }
+        } else if ((Norm == kExchange || (Norm == kAny && norm_w)) && my_rows) {
             float* ss = reinterpret_cast<float*>(sm + OFF_SS);
             float sq[ROWS];
 #pragma unroll
@@ -214,17 +271,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constan
                 for (uint32_t s = 0; s < a.cs; s++)
 #pragma unroll
                     for (uint32_t p = 0; p < ROW_WARPS; p++) if (p < a.split) tot += ss[s * 32 + at + p];
-                const float inv = rsqrtf(tot / float(a.K) + a.eps);
-#pragma unroll
-                for (int k = 0; k < PER; k++) {
-                    if (32 * a.split * k >= pieces) break;
-                    const T *f = reinterpret_cast<const T*>(&v[r][k]), *w = reinterpret_cast<const T*>(&g[k]);
-                    uint32_t y[4];
-#pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        y[j] = Elem<T>::pack2(Elem<T>::to_f32(f[2 * j]) * inv * Elem<T>::to_f32(w[2 * j]), Elem<T>::to_f32(f[2 * j + 1]) * inv * Elem<T>::to_f32(w[2 * j + 1]));
-                    v[r][k] = make_uint4(y[0], y[1], y[2], y[3]);
-                }
+                normalise(r, rsqrtf(tot / float(a.K) + a.eps));
             }
         }
         // rows behind the last one keep what the memory held: a row reaches no column but its own
@@ -314,6 +361,14 @@ cudaLaunchConfig_t launch_config(cudaLaunchAttribute (&at)[2], uint32_t blocks, 
     return cfg;
 }
 
+template <typename T, typename F>
+void for_each_kernel(F f)
+{
+    f(gemm_few_kernel<T, 16, 1, kAny>);
+    f(gemm_few_kernel<T, 16, 2, kNoNorm>); f(gemm_few_kernel<T, 16, 2, kExchange>); f(gemm_few_kernel<T, 16, 2, kWhole>);
+    f(gemm_few_kernel<T, 32, 4, kNoNorm>); f(gemm_few_kernel<T, 32, 4, kExchange>); f(gemm_few_kernel<T, 32, 4, kWhole>);
+}
+
 template <typename T>
 cudaError_t configure_type()
 {
@@ -321,8 +376,9 @@ cudaError_t configure_type()
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
         return e != cudaSuccess ? e : cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     };
-    const cudaError_t e = set(gemm_few_kernel<T, 16>);
-    return e != cudaSuccess ? e : set(gemm_few_kernel<T, 32>);
+    cudaError_t e = cudaSuccess;
+    for_each_kernel<T>([&](auto kernel) { if (e == cudaSuccess) e = set(kernel); });
+    return e;
 }
 
 template <typename T>
@@ -351,7 +407,17 @@ int launch_type(const GemmCall& g, uint32_t cs, uint32_t* status, const LaunchSt
         return int(cudaLaunchKernelEx(&cfg, kernel, *g.w[0].map, *g.w[last].map, static_cast<const T*>(g.A), static_cast<const T*>(g.norm_w),
                                       static_cast<T*>(g.w[0].out), static_cast<T*>(g.w[last].out), a, status));
     };
-    return g.M <= 16 ? go(gemm_few_kernel<T, 16>) : go(gemm_few_kernel<T, 32>);
+    // A warp's whole rows are a trip to L2 for every 256 pieces of 8 values of them, the exchange is one trip and one through the cluster:
+    // (16 heads, hidden 2048, input projections of 1 / 8 / 16 / 32 rows: 7.0 / 7.1 / 7.9 / 9.9 us by exchange, 5.7 / 5.8 / 7.0 / 8.6
+    // whole.)  Short rows of more than 8, where it matters least, use the exchange because the kernel for it has just run for the
+    // longer rows of q_a (16 blocks of 32 heads x 20 rows, hidden 4096, q_lora 512: 848 us whole, 840).
+    const bool whole = g.M <= 8 ? g.K <= 4096 : g.K >= 1024 && g.K <= 2048;
+    const int norm = !g.norm_w ? kNoNorm : whole ? kWhole : kExchange;
+    a.whole = norm == kWhole;
+    auto pick = [&](auto none, auto exchange, auto whole) { return norm == kNoNorm ? go(none) : norm == kWhole ? go(whole) : go(exchange); };
+    if (g.M <= 8) return go(gemm_few_kernel<T, 16, 1, kAny>);
+    if (g.M <= 16) return pick(gemm_few_kernel<T, 16, 2, kNoNorm>, gemm_few_kernel<T, 16, 2, kExchange>, gemm_few_kernel<T, 16, 2, kWhole>);
+    return pick(gemm_few_kernel<T, 32, 4, kNoNorm>, gemm_few_kernel<T, 32, 4, kExchange>, gemm_few_kernel<T, 32, 4, kWhole>);
 }
 
 }  // namespace
@@ -369,7 +435,7 @@ int gemm_few_tc5_clusters(uint32_t (&n)[4])
         cudaLaunchAttribute at[2];
         const cudaLaunchConfig_t cfg = launch_config(at, 1u << i, 1u << i, cudaStream_t(nullptr));
         int c = 0;
-        const cudaError_t e = cudaOccupancyMaxActiveClusters(&c, gemm_few_kernel<__half, 32>, &cfg);
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&c, gemm_few_kernel<__half, 32, 4, kExchange>, &cfg);
         if (e != cudaSuccess) return int(e);
         n[i] = uint32_t(c);
     }
