@@ -411,7 +411,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
 }
 
-template <typename T, int NT, bool kPaged>
+// kCut: runs may end inside a tile; kResidual: outputs are added to what is there
+template <typename T, int NT, bool kPaged, bool kCut, bool kResidual>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
                  const __grid_constant__ CUtensorMap map_c0, const __grid_constant__ CUtensorMap map_c1, T* __restrict__ out0, T* __restrict__ out1,
@@ -556,7 +557,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         uint32_t nt = 0;
         for (uint32_t u = u0; u < u1; nt++) {
             const uint32_t vt = u / a.kb, t_end = (vt + 1) * a.kb, end = min(u1, t_end), tile = tile_id(vt);
-            const bool cut = u != vt * a.kb || end != t_end;
+            const bool cut = kCut && (u != vt * a.kb || end != t_end);
             const Tile tl = tile_of(a, tile);
             const uint32_t N = tl.w ? a.N[1] : a.N[0], m0 = (2 * tl.m + rank) * BM + q4 * 32, m = m0 + lane;
             T* out = tl.w ? out1 : out0;
@@ -568,7 +569,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 const uint32_t n0 = tl.n * NT + c * CH;
 #pragma unroll
                 for (int i = 0; i < 4; i++)
-                    if (a.residual && m < a.M && c < c_first + CHUNKS && n0 + 8 * i < N) rs[i] = load8(out + size_t(m) * N + n0 + 8 * i, a.vec_io);
+                    if (kResidual && m < a.M && c < c_first + CHUNKS && n0 + 8 * i < N) rs[i] = load8(out + size_t(m) * N + n0 + 8 * i, a.vec_io);
             };
             uint4 rs0[4], rs1[4];
             residual(c_first, rs0);
@@ -589,7 +590,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 uint32_t pk[16];
 #pragma unroll
                 for (int i = 0; i < 16; i++) pk[i] = Elem<T>::pack2(v[2 * i], v[2 * i + 1]);
-                if (a.residual && m < a.M) {
+                if (kResidual && m < a.M) {
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
                         if (n0 + 8 * i >= N) break;
@@ -629,7 +630,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 }
             };
             static_assert(CHUNKS % 2 == 0, "boxes of two chunks");
-            if (!cut) {
+            if (!kCut || !cut) {
 #pragma unroll 1
                 for (int c = c_first; c < c_first + CHUNKS; c += 2) {
                     float v[CH];
@@ -639,7 +640,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     if (c + 2 == c_first + CHUNKS) release();
                     finish(c + 1, v, rs1);
                 }
-            } else if (hand_over<NT, CH, 32 * EPI_WARPS>(a, worker, 2, rank, tile, [&](int c, float (&v)[CH]) { load_acc(acc + c * CH, v); }, r, c_first, c_first + CHUNKS, tid == 64, ok, last_slot, release)) {
+            }
+            if constexpr (kCut) if (cut && hand_over<NT, CH, 32 * EPI_WARPS>(a, worker, 2, rank, tile, [&](int c, float (&v)[CH]) { load_acc(acc + c * CH, v); }, r, c_first, c_first + CHUNKS, tid == 64, ok, last_slot, release)) {
 #pragma unroll 1
                 for (int c = c_first; c < c_first + CHUNKS; c += 2) {
                     float v[CH];
@@ -727,10 +729,16 @@ cudaError_t configure_type()
     if (e == cudaSuccess) e = set(gemm_rows_kernel<T, 32>, rows_smem(32));
     if (e == cudaSuccess) e = set(gemm_rows_kernel<T, 64>, rows_smem(64));
     if (e == cudaSuccess) e = set(gemm_rows_kernel<T, 128>, rows_smem(128));
-    if (e == cudaSuccess) e = set(gemm_pair_kernel<T, 128, false>, pair_smem(128));
-    if (e == cudaSuccess) e = set(gemm_pair_kernel<T, 256, false>, pair_smem(256));
-    if (e == cudaSuccess) e = set(gemm_pair_kernel<T, 128, true>, pair_smem(128));
-    if (e == cudaSuccess) e = set(gemm_pair_kernel<T, 256, true>, pair_smem(256));
+    auto pair = [&]<bool kPaged, bool kCut, bool kResidual>() {
+        if (e == cudaSuccess) e = set(gemm_pair_kernel<T, 128, kPaged, kCut, kResidual>, pair_smem(128));
+        if (e == cudaSuccess) e = set(gemm_pair_kernel<T, 256, kPaged, kCut, kResidual>, pair_smem(256));
+    };
+    pair.template operator()<false, false, false>();
+    pair.template operator()<false, false, true>();
+    pair.template operator()<false, true, false>();
+    pair.template operator()<false, true, true>();
+    pair.template operator()<true, false, false>();
+    pair.template operator()<true, true, false>();
     return e;
 }
 
@@ -824,8 +832,13 @@ int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t*
     auto go = [&](auto kernel) {
         return int(launch_pdl(kernel, dim3(2 * workers), dim3(PAIR_THREADS), size_t(pair_smem(int(nt))), st, pa, m0, m1, c0, c1, out[0], out[1], a, status));
     };
-    if (g.paged_map) return nt == 256 ? go(gemm_pair_kernel<T, 256, true>) : go(gemm_pair_kernel<T, 128, true>);
-    return nt == 256 ? go(gemm_pair_kernel<T, 256, false>) : go(gemm_pair_kernel<T, 128, false>);
+    auto width = [&]<bool kPaged, bool kCut, bool kResidual>() {
+        return nt == 256 ? go(gemm_pair_kernel<T, 256, kPaged, kCut, kResidual>) : go(gemm_pair_kernel<T, 128, kPaged, kCut, kResidual>);
+    };
+    const bool cut = !a.stride;
+    if (g.paged_map) return cut ? width.template operator()<true, true, false>() : width.template operator()<true, false, false>();
+    if (g.residual) return cut ? width.template operator()<false, true, true>() : width.template operator()<false, false, true>();
+    return cut ? width.template operator()<false, true, false>() : width.template operator()<false, false, false>();
 }
 
 }  // namespace
