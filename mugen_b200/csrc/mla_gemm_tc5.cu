@@ -411,8 +411,10 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
 }
 
-// kCut: runs may end inside a tile; kResidual: outputs are added to what is there
-template <typename T, int NT, bool kPaged, bool kCut, bool kResidual>
+// kCut: runs may end inside a tile; kResidual: outputs are added to what is there; kTma: outputs leave by TMA.  A launch fetches only
+// the instructions that its outputs need.  Without kTma (outputs off a 16-byte boundary: rare) the two others are true and the
+// arguments say: 27 layers of a 777-token prompt at 16 heads 1,548 -> 1,539 us, eight layers of 2,300 tokens 889 -> 878.
+template <typename T, int NT, bool kPaged, bool kCut, bool kResidual, bool kTma>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
                  const __grid_constant__ CUtensorMap map_c0, const __grid_constant__ CUtensorMap map_c1, T* __restrict__ out0, T* __restrict__ out1,
@@ -569,7 +571,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 const uint32_t n0 = tl.n * NT + c * CH;
 #pragma unroll
                 for (int i = 0; i < 4; i++)
-                    if (kResidual && m < a.M && c < c_first + CHUNKS && n0 + 8 * i < N) rs[i] = load8(out + size_t(m) * N + n0 + 8 * i, a.vec_io);
+                    if (kResidual && (kTma || a.residual) && m < a.M && c < c_first + CHUNKS && n0 + 8 * i < N) rs[i] = load8(out + size_t(m) * N + n0 + 8 * i, kTma || a.vec_io);
             };
             uint4 rs0[4], rs1[4];
             residual(c_first, rs0);
@@ -590,7 +592,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 uint32_t pk[16];
 #pragma unroll
                 for (int i = 0; i < 16; i++) pk[i] = Elem<T>::pack2(v[2 * i], v[2 * i + 1]);
-                if (kResidual && m < a.M) {
+                if (kResidual && (kTma || a.residual) && m < a.M) {
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
                         if (n0 + 8 * i >= N) break;
@@ -604,7 +606,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     }
                 }
                 residual(c + 2, rs);
-                if (!a.tile_store) {
+                if constexpr (!kTma) {
                     if (m >= a.M || !ok) return;
 #pragma unroll
                     for (int i = 0; i < 4; i++)
@@ -653,7 +655,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             }
             u = end;
         }
-        if (a.tile_store && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+        if (kTma && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
         __syncwarp();
     }
     // neither block may leave while its twin can still signal its barriers or feed a pair MMA from its shared memory
@@ -729,16 +731,17 @@ cudaError_t configure_type()
     if (e == cudaSuccess) e = set(gemm_rows_kernel<T, 32>, rows_smem(32));
     if (e == cudaSuccess) e = set(gemm_rows_kernel<T, 64>, rows_smem(64));
     if (e == cudaSuccess) e = set(gemm_rows_kernel<T, 128>, rows_smem(128));
-    auto pair = [&]<bool kPaged, bool kCut, bool kResidual>() {
-        if (e == cudaSuccess) e = set(gemm_pair_kernel<T, 128, kPaged, kCut, kResidual>, pair_smem(128));
-        if (e == cudaSuccess) e = set(gemm_pair_kernel<T, 256, kPaged, kCut, kResidual>, pair_smem(256));
+    auto pair = [&]<bool kPaged, bool kCut, bool kResidual, bool kTma>() {
+        if (e == cudaSuccess) e = set(gemm_pair_kernel<T, 128, kPaged, kCut, kResidual, kTma>, pair_smem(128));
+        if (e == cudaSuccess) e = set(gemm_pair_kernel<T, 256, kPaged, kCut, kResidual, kTma>, pair_smem(256));
     };
-    pair.template operator()<false, false, false>();
-    pair.template operator()<false, false, true>();
-    pair.template operator()<false, true, false>();
-    pair.template operator()<false, true, true>();
-    pair.template operator()<true, false, false>();
-    pair.template operator()<true, true, false>();
+    pair.template operator()<false, false, false, true>();
+    pair.template operator()<false, false, true, true>();
+    pair.template operator()<false, true, false, true>();
+    pair.template operator()<false, true, true, true>();
+    pair.template operator()<false, true, true, false>();
+    pair.template operator()<true, false, false, true>();
+    pair.template operator()<true, true, false, true>();
     return e;
 }
 
@@ -832,13 +835,17 @@ int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t*
     auto go = [&](auto kernel) {
         return int(launch_pdl(kernel, dim3(2 * workers), dim3(PAIR_THREADS), size_t(pair_smem(int(nt))), st, pa, m0, m1, c0, c1, out[0], out[1], a, status));
     };
-    auto width = [&]<bool kPaged, bool kCut, bool kResidual>() {
-        return nt == 256 ? go(gemm_pair_kernel<T, 256, kPaged, kCut, kResidual>) : go(gemm_pair_kernel<T, 128, kPaged, kCut, kResidual>);
+    auto width = [&]<bool kPaged, bool kCut, bool kResidual, bool kTma>() {
+        return nt == 256 ? go(gemm_pair_kernel<T, 256, kPaged, kCut, kResidual, kTma>) : go(gemm_pair_kernel<T, 128, kPaged, kCut, kResidual, kTma>);
     };
     const bool cut = !a.stride;
-    if (g.paged_map) return cut ? width.template operator()<true, true, false>() : width.template operator()<true, false, false>();
-    if (g.residual) return cut ? width.template operator()<false, true, true>() : width.template operator()<false, false, true>();
-    return cut ? width.template operator()<false, true, false>() : width.template operator()<false, false, false>();
+    if (g.paged_map) {                                   // outputs in the library's own buffers
+        if (!a.tile_store) return -1;
+        return cut ? width.template operator()<true, true, false, true>() : width.template operator()<true, false, false, true>();
+    }
+    if (!a.tile_store) return width.template operator()<false, true, true, false>();
+    if (g.residual) return cut ? width.template operator()<false, true, true, true>() : width.template operator()<false, false, true, true>();
+    return cut ? width.template operator()<false, true, false, true>() : width.template operator()<false, false, false, true>();
 }
 
 }  // namespace

@@ -197,6 +197,8 @@ def test_projections_at_the_edges_of_their_tiles(torch, rows, H, E, R, shift):
     (129, 16, 2048, 0, 0), (256, 5, 72, 0, 4), (257, 64, 1000, 136, 0), (700, 16, 2048, 0, 8),
     # the order of the tiles, Wo: two by two with one over; one by one; 9 tiles of rows side by side, the last one of 252 rows
     (1100, 72, 520, 0, 0), (600, 80, 520, 0, 0), (2300, 3, 1032, 0, 0),
+    # outputs off a 16-byte boundary in both widths of tile, in whole runs and cut ones
+    (1100, 72, 520, 0, 4), (777, 16, 2048, 0, 1),
 ])
 def test_every_output_of_the_projections_and_nothing_beside_them(torch, rows, H, E, R, shift, dt):
     """Element by element against float64, and the values in front of and behind each output untouched.  An output is one rounding
