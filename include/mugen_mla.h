@@ -221,7 +221,7 @@ int mla_merge_partials(mla_ctx* ctx, uint32_t layer, uint32_t n_parts, uint32_t 
 int mla_set_q_rope(mla_ctx* ctx, int in_kernel);
 
 /* ---- introspection used by benchmarks --------------------------------------------------- */
-/* Kernel launches issued by this context since creation. */
+/* Kernel launches issued by this context since creation (those that upload step metadata are not counted). */
 int mla_launch_count(const mla_ctx* ctx, uint64_t* n);
 /* Device timing of the split-KV attention kernel alone: while enabled, launches of that kernel
  * are bracketed by CUDA events on the launching stream (up to 8192 launches are kept).  on = 1

@@ -80,9 +80,9 @@ struct mla_ctx {
     mla::GemmWeightMaps w_uk_rows_maps, w_uv_maps;       // the same weights for the prefill expansion
     std::vector<BlockW> blocks;
     // workspaces of the block projections, grown on demand: normalised hidden state, q_a,
-    // and the block's q / kv_a / attention output when the library owns them (mla_step_block)
-    void *blk_hidden2 = nullptr, *blk_qa = nullptr, *blk_q = nullptr, *blk_kv = nullptr, *blk_out = nullptr;
-    size_t blk_hidden2_cap = 0, blk_qa_cap = 0, blk_q_cap = 0, blk_kv_cap = 0, blk_out_cap = 0;
+    // and the block's q, kv_a and attention output when the library owns them (mla_step_block: one allocation)
+    void *blk_hidden2 = nullptr, *blk_qa = nullptr, *blk_rows = nullptr;
+    size_t blk_hidden2_cap = 0, blk_qa_cap = 0, blk_rows_cap = 0;
     mla::GemmWorkspace gemm_ws{};    // partial tiles and counters of the projections
     float* cos_sin = nullptr;       // device [max positions][64]
     uint32_t cs_rows = 0;           // positions filled so far
@@ -120,9 +120,9 @@ struct mla_ctx {
     struct ChunkGroup { uint32_t rows, n_tiles; const uint32_t* pages; const mla::PrefillTile* tiles; };
     std::vector<ChunkGroup> chunk_groups;
     uint32_t step_rows = 0;          // rows of the step in the caller's q / kv_a / out tensors
-    // prefill workspaces, grown on demand: expanded keys and values
-    void *pf_kx = nullptr, *pf_vx = nullptr;
-    size_t pf_kx_cap = 0, pf_vx_cap = 0;
+    // prefill workspace, grown on demand: expanded keys, then values
+    void* pf_kv = nullptr;
+    size_t pf_kv_cap = 0;
 
     // pages of the last planned step per persistent worker (mla_step_balance)
     uint32_t plan_workers = 0, plan_min_pages = 0, plan_max_pages = 0;
@@ -641,8 +641,9 @@ int run_chunks(mla_ctx* c, uint32_t layer, const void* q, void* out, cudaStream_
     const int dt = int(c->cfg.dtype);
     if (int e = ensure_gemm_workspace(c)) return e;
     for (const auto& g : c->chunk_groups) {
-        if (int e = grow(c, &c->pf_kx, &c->pf_kx_cap, size_t(g.rows) * H * mla::kNope * 2, true)) return e;
-        if (int e = grow(c, &c->pf_vx, &c->pf_vx_cap, size_t(g.rows) * H * mla::kVDim * 2, true)) return e;
+        const size_t k_bytes = size_t(g.rows) * H * mla::kNope * 2, v_bytes = size_t(g.rows) * H * mla::kVDim * 2;
+        if (int e = grow(c, &c->pf_kv, &c->pf_kv_cap, k_bytes + v_bytes, true)) return e;
+        void *kx = c->pf_kv, *vx = static_cast<char*>(c->pf_kv) + k_bytes;               // rows of 256 bytes
         mla::GemmCall gc;
         gc.paged_map = &c->tmaps[mla::kMapPoolSub];
         gc.table = g.pages;
@@ -651,12 +652,12 @@ int run_chunks(mla_ctx* c, uint32_t layer, const void* q, void* out, cudaStream_
         gc.M = g.rows;
         gc.K = mla::kRank;
         gc.n_weights = 2;
-        gc.w[0] = gemm_weight(c->w_uk_rows_maps, H * mla::kNope, c->pf_kx, layer * H * mla::kNope);
-        gc.w[1] = gemm_weight(c->w_uv_maps, H * mla::kVDim, c->pf_vx, layer * H * mla::kVDim);
+        gc.w[0] = gemm_weight(c->w_uk_rows_maps, H * mla::kNope, kx, layer * H * mla::kNope);
+        gc.w[1] = gemm_weight(c->w_uv_maps, H * mla::kVDim, vx, layer * H * mla::kVDim);
         int rc = mla::launch_gemm_tc5(dt, gc, c->gemm_ws, c->status_dev, st, c->launches);
         if (rc) return fail(c, rc == -1 ? MLA_ERR_INVALID : MLA_ERR_CUDA, "key / value expansion launch failed");
         mla::PrefillCall p;
-        p.q = q; p.out = out; p.kx = c->pf_kx; p.vx = c->pf_vx;
+        p.q = q; p.out = out; p.kx = kx; p.vx = vx;
         p.pool_map = &c->tmaps[mla::kMapPoolSub];
         p.pages = g.pages;
         p.tiles = g.tiles;
@@ -895,7 +896,7 @@ void mla_destroy(mla_ctx* c)
     cudaDeviceSynchronize();
     cudaFree(c->pool);
     cudaFree(c->w_uk); cudaFree(c->w_uk_rows); cudaFree(c->w_uv); cudaFree(c->norm);
-    cudaFree(c->pf_kx); cudaFree(c->pf_vx);
+    cudaFree(c->pf_kv);
     cudaFree(c->cos_sin);
     cudaFree(c->q_abs);
     cudaFree(c->recs);
@@ -910,7 +911,7 @@ void mla_destroy(mla_ctx* c)
     if (c->h_out) cudaFreeHost(c->h_out);
     cudaFree(c->d_kv); cudaFree(c->d_q); cudaFree(c->d_out);
     for (auto& b : c->blocks) { cudaFree(b.attn_norm); cudaFree(b.q_a); cudaFree(b.q_a_norm); cudaFree(b.q_b); cudaFree(b.q); cudaFree(b.kv_a); cudaFree(b.wo); }
-    cudaFree(c->blk_hidden2); cudaFree(c->blk_qa); cudaFree(c->blk_q); cudaFree(c->blk_kv); cudaFree(c->blk_out); cudaFree(c->gemm_ws.partial); cudaFree(c->gemm_ws.counters);
+    cudaFree(c->blk_hidden2); cudaFree(c->blk_qa); cudaFree(c->blk_rows); cudaFree(c->gemm_ws.partial); cudaFree(c->gemm_ws.counters);
     for (auto& ev : c->host_ev) { cudaEventDestroy(ev.in); cudaEventDestroy(ev.compute); cudaEventDestroy(ev.out); }
     if (c->copy_in) cudaStreamDestroy(c->copy_in);
     if (c->copy_out) cudaStreamDestroy(c->copy_out);
@@ -1187,13 +1188,13 @@ int mla_step_layers(mla_ctx* c, uint32_t layer_begin, uint32_t n_layers, const v
     // attention and one merge launch, planned together, so that a step of few rows fills the machine.
     uint32_t group = 1;
     if (!c->has_chunks && rows && c->kernel != MLA_KERNEL_MMA) group = uint32_t(std::min<uint64_t>(n_layers, c->ws_rows / rows));
-    // The group's plan is uploaded by this call: not into a captured graph, whose replays would copy from the upload ring again
+    // The group's plan is uploaded by this call: not into a captured graph, whose replays would read the upload ring again
     // long after it went on.  A captured call goes layer by layer with the plan of mla_step_begin.
     if (group > 1 && capturing(st)) group = 1;
     if (group > 1) {
         const uint32_t n_groups = (n_layers + group - 1) / group;
         group = (n_layers + n_groups - 1) / n_groups;
-        // both plans go up ahead of the first launch: a copy between two launches ends their overlap
+        // both plans go up ahead of the first launch: an upload between two launches ends their overlap
         auto plan_of = [&](uint32_t n) -> Plan& { return n == group ? c->stack : c->stack_tail; };
         for (uint32_t n : {group, n_layers % group})
             if (Plan& p = plan_of(n); n && (!p.ready || p.m.layers != n))
@@ -1641,12 +1642,12 @@ int mla_step_block(mla_ctx* c, uint32_t layer, void* hidden, void* stream)
     auto st = static_cast<cudaStream_t>(stream);
     const uint32_t rows = c->step_rows, H = c->cfg.n_heads;
     if (rows == 0) return MLA_OK;
-    if (int e = grow(c, &c->blk_q, &c->blk_q_cap, size_t(rows) * H * mla::kQDim * 2)) return e;
-    if (int e = grow(c, &c->blk_kv, &c->blk_kv_cap, size_t(rows) * mla::kRow * 2)) return e;
-    if (int e = grow(c, &c->blk_out, &c->blk_out_cap, size_t(rows) * H * mla::kVDim * 2)) return e;
-    if (int e = project_in(c, *b, rows, hidden, c->blk_q, c->blk_kv, st)) return e;
-    if (int e = run_layer(c, layer, c->blk_kv, c->blk_q, c->blk_out, st)) return e;
-    return project(c, c->blk_out, rows, H * uint32_t(mla::kVDim), {gemm_weight(b->wo_map, b->embed, hidden)}, true, st);
+    const size_t q_bytes = size_t(rows) * H * mla::kQDim * 2, kv_bytes = size_t(rows) * mla::kRow * 2, out_bytes = size_t(rows) * H * mla::kVDim * 2;
+    if (int e = grow(c, &c->blk_rows, &c->blk_rows_cap, q_bytes + kv_bytes + out_bytes)) return e;
+    char *q = static_cast<char*>(c->blk_rows), *kv = q + q_bytes, *out = kv + kv_bytes;          // rows are multiples of 128 bytes
+    if (int e = project_in(c, *b, rows, hidden, q, kv, st)) return e;
+    if (int e = run_layer(c, layer, kv, q, out, st)) return e;
+    return project(c, out, rows, H * uint32_t(mla::kVDim), {gemm_weight(b->wo_map, b->embed, hidden)}, true, st);
 }
 
 }  // extern "C"
