@@ -13,8 +13,8 @@
 // Work = (output tile, k-block of 64) units in one line; every worker (a block, or a pair of blocks) gets an equal run of
 // them, so a launch is balanced whatever its tile count.  A tile cut by a run boundary is finished by the worker that
 // arrives last at the tile's counter: every contributor leaves its float partial in global memory (L2), the last one adds
-// them in the order of the runs (bit-reproducible) and stores.  Where that costs more than it saves, runs end on tile
-// boundaries (pick_shape).
+// them in the order of the runs (bit-reproducible) and stores.  Where that costs more than it saves, pairs take whole tiles, or cut
+// only what does not fill a round of all pairs (pick_shape).
 //   up to 128 rows   gemm_rows_kernel, one block per SM: 128 weight rows are the M side of the MMA, the rows of A its N side
 //                    (16, 32, 64 or 128 columns): the bytes in flight are weight bytes, and a step of 4 rows does not pay
 //                    for 128.  HBM-bound.
@@ -99,7 +99,8 @@ struct GemmArgs {
     uint32_t m_tiles, n_tiles[2];       // tiles along the rows of A, and along the outputs of each weight
     uint32_t N[2], w_row0[2];           // outputs of each weight; first row of the weight inside its map
     uint32_t units, run;                // tiles x k-blocks, and how many of them a worker takes
-    uint32_t stride;                    // pairs, whole tiles: worker w takes tiles w, w + stride, ..; 0: equal runs
+    uint32_t cut_tiles, stride;         // pairs: the first tiles of the line are cut into equal runs; of the others, whole ones, worker w
+                                        // takes the tiles w, w + stride, ..
     uint32_t group_m;                   // tiles along A's rows that stand side by side in the line of tiles
     uint32_t packed;                    // weights in the layout of gemm_tc5_pack
     uint32_t residual;                  // out = T(float(out) + float(T(x))) instead of T(x)
@@ -128,14 +129,18 @@ __device__ __forceinline__ Tile tile_of(const GemmArgs& a, uint32_t t) {
 // one loading thread of a block, not the memory behind it, set the pace of the main loop (300 rows, 4096 x 8192: 51.9 us, 41.8
 // without; 777 rows, 7168 and 1536 inputs together: 119.6, 104.8; 27 blocks over a 777-token prompt, the output projection: 16.0,
 // 14.4).
+template <bool kJump>
 struct Walk {
     uint32_t vt, k;                     // tile of this worker's line (tile_id makes it a tile of the launch), k-block of it
     Tile t;
+    uint32_t left;                      // kJump: units of this worker's run of cut tiles; its whole tiles come behind them
     template <typename TileId>
-    __device__ __forceinline__ Walk(const GemmArgs& a, uint32_t u, TileId tile_id) : vt(u / a.kb), k(u % a.kb), t(tile_of(a, tile_id(vt))) {}
+    __device__ __forceinline__ Walk(const GemmArgs& a, uint32_t u, TileId tile_id, uint32_t run = 0)
+        : vt(u / a.kb), k(u % a.kb), t(tile_of(a, tile_id(vt))), left(run) {}
     template <typename TileId>
     __device__ __forceinline__ void next(const GemmArgs& a, TileId tile_id) {
-        if (++k == a.kb) { k = 0; t = tile_of(a, tile_id(++vt)); }
+        if (kJump && left != 0 && --left == 0) { vt = a.cut_tiles; k = 0; t = tile_of(a, tile_id(vt)); }
+        else if (++k == a.kb) { k = 0; t = tile_of(a, tile_id(++vt)); }
     }
 };
 
@@ -269,13 +274,13 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     if (warp == 0) {
         if (lane == 0) {
             auto same = [](uint32_t t) { return t; };
-            auto load_w = [&](const Walk& x, int s) {
+            auto load_w = [&](const Walk<false>& x, int s) {
                 tma_load_2d(base + s * STAGE, x.t.w ? &map_w1 : &map_w0, full(s), a.packed ? 0 : int(x.k * BK),
                             a.packed ? int((x.t.n * a.kb + x.k) * BM) : int((x.t.w ? a.w_row0[1] : a.w_row0[0]) + x.t.n * BM));
             };
-            auto load_a = [&](const Walk& x, int s) { tma_load_2d(base + s * STAGE + A_BYTES, &map_a, full(s), int(x.k * BK), int(x.t.m * NT)); };
+            auto load_a = [&](const Walk<false>& x, int s) { tma_load_2d(base + s * STAGE + A_BYTES, &map_a, full(s), int(x.k * BK), int(x.t.m * NT)); };
             const uint32_t n = u1 - u0, ahead = min(n, uint32_t(STAGES));
-            Walk x(a, u0, same), y = x;
+            Walk<false> x(a, u0, same), y = x;
             for (uint32_t i = 0; i < ahead; i++, x.next(a, same)) {
                 mbar_expect_tx(full(int(i)), STAGE);
                 load_w(x, int(i));
@@ -437,10 +442,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     volatile uint32_t* last_slot = reinterpret_cast<volatile uint32_t*>(sm + OFF_MISC + 232);
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const uint32_t rank = cluster_rank(), worker = blockIdx.x / 2;               // rank 0 issues the MMAs
-    // this pair's run of units; with whole tiles (stride) the units of its own tiles, counted from 0
-    const uint32_t tiles = a.units / a.kb;
-    const uint32_t u0 = a.stride ? 0u : worker * a.run, u1 = a.stride ? (tiles - worker + a.stride - 1) / a.stride * a.kb : min(a.units, u0 + a.run);
-    auto tile_id = [&](uint32_t vt) -> uint32_t { return a.stride ? worker + vt * a.stride : vt; };
+    // this pair's units: its run [c0, c1) of the cut tiles, then, counted from their end, those of its whole tiles
+    const uint32_t tiles = a.units / a.kb, cut_tiles = kCut ? a.cut_tiles : 0u, cut_end = cut_tiles * a.kb;
+    const uint32_t c0 = kCut ? min(worker * a.run, cut_end) : 0u, c1 = kCut ? min(c0 + a.run, cut_end) : 0u;
+    const uint32_t whole = tiles - cut_tiles > worker ? (tiles - cut_tiles - worker + a.stride - 1) / a.stride : 0u;
+    const uint32_t u0 = c0 < c1 ? c0 : cut_end, u1 = cut_end + whole * a.kb;
+    auto tile_id = [&](uint32_t vt) -> uint32_t { return kCut && vt < cut_tiles ? vt : cut_tiles + worker + (vt - cut_tiles) * a.stride; };
 
     if constexpr (!kPaged) grid_launch_dependents();
     if (tid == 64) { prefetch_map(&map_a); prefetch_map(&map_c0); prefetch_map(&map_c1); }
@@ -461,14 +468,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     if (warp == 0) {
         if (lane == 0) {
             const uint32_t leader_full = map_to_rank(full(0), 0);
-            auto load_w = [&](const Walk& x, int s) {            // this block's half of the outputs, in boxes of up to 128 weight rows
+            auto load_w = [&](const Walk<kCut>& x, int s) {            // this block's half of the outputs, in boxes of up to 128 weight rows
                 const uint32_t o = x.t.n * NT + rank * (NT / 2);                       // first of this block's outputs
                 tma_load_2d_pair(base + s * STAGE + A_BYTES, x.t.w ? &map_w1 : &map_w0, leader_full + 8u * s, a.packed ? 0 : int(x.k * BK),
                                  a.packed ? int(((o / BM) * a.kb + x.k) * BM + o % BM) : int((x.t.w ? a.w_row0[1] : a.w_row0[0]) + o));
             };
             uint32_t cur_m = ~0u, next_m = ~0u, page[2] = {0, 0}, next_page[2] = {0, 0};
             auto page_of = [&](uint32_t i) { return __ldg(a.table + min(i, (a.M + kPage - 1) / kPage - 1)); };   // past the end: the last page again
-            auto load_a = [&](const Walk& x, int s) {
+            auto load_a = [&](const Walk<kCut>& x, int s) {
                 const Tile& t = x.t;
                 const int k = int(x.k * BK);
                 const uint32_t dst = base + s * STAGE;
@@ -492,8 +499,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     tma_load_2d_pair(dst, &map_a, leader_full + 8u * s, k, int(t.m * 2 * BM + rank * BM));
                 }
             };
-            const uint32_t n = u1 - u0, ahead = min(n, uint32_t(STAGES));
-            Walk x(a, u0, tile_id), y = x;
+            const uint32_t n = (c1 - c0) + whole * a.kb, ahead = min(n, uint32_t(STAGES));
+            Walk<kCut> x(a, u0, tile_id, c1 - c0), y = x;
             for (uint32_t i = 0; i < ahead; i++, x.next(a, tile_id)) {
                 if (rank == 0) mbar_expect_tx(full(int(i)), 2 * STAGE);
                 load_w(x, int(i));
@@ -523,7 +530,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             uint32_t nt = 0, par = 0;
             int s = 0;
             for (uint32_t u = u0; u < u1 && ok; nt++) {
-                const uint32_t end = min(u1, (u / a.kb + 1) * a.kb);
+                const uint32_t end = min(kCut && u < c1 ? c1 : u1, (u / a.kb + 1) * a.kb);
                 ok = mbar_wait<kSleepCluster>(acc_empty(nt & 1), ((nt >> 1) & 1) ^ 1, abort_flag, status);
                 if (!ok) break;
                 const uint32_t d = tmem + (nt & 1) * NT;
@@ -542,6 +549,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     __syncwarp();
                     if (++s == STAGES) { s = 0; par ^= 1; }
                 }
+                if (kCut && u == c1) u = cut_end;
             }
         }
     } else {
@@ -558,7 +566,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         bool ok = true;
         uint32_t nt = 0;
         for (uint32_t u = u0; u < u1; nt++) {
-            const uint32_t vt = u / a.kb, t_end = (vt + 1) * a.kb, end = min(u1, t_end), tile = tile_id(vt);
+            const uint32_t vt = u / a.kb, t_end = (vt + 1) * a.kb, end = min(kCut && u < c1 ? c1 : u1, t_end), tile = tile_id(vt);
             const bool cut = kCut && (u != vt * a.kb || end != t_end);
             const Tile tl = tile_of(a, tile);
             const uint32_t N = tl.w ? a.N[1] : a.N[0], m0 = (2 * tl.m + rank) * BM + q4 * 32, m = m0 + lane;
@@ -653,7 +661,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     finish(c + 1, v, rs1);
                 }
             }
-            u = end;
+            u = kCut && end == c1 ? cut_end : end;
         }
         if (kTma && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
         __syncwarp();
@@ -745,36 +753,58 @@ cudaError_t configure_type()
     return e;
 }
 
-// Tile width and run length of a launch: the shortest estimate, in SM cycles, of whole tiles against equal runs with cut
-// tiles.  A k-block of a pair counts 820 (256 outputs) or 610 (128) cycles, one of gemm_rows_kernel about 400 (the HBM rate).  Cutting
-// tiles adds the hand-over (partial out, counter, partials in): in gemm_rows_kernel about 4000 cycles and 50 per column; in a pair
-// 190 per column, 13 and 26 us, fitted to whole and cut runs of both widths over 8 weights x 9 row counts.  The pair's figures are
-// those of the kernel whose loading thread divided for every k-block, with four epilogue warps and three barriers in the
-// hand-over; both kinds of run have become faster since (N = K = 2048, 129 to 512 rows, whole tiles: 15 us then, 12 now), the
-// balance between them has not been fitted again.
-struct Shape { uint32_t nt, m_tiles, n_tiles[2], run; };
+// Tile width, cut tiles and run length of a launch: the shortest estimate of
+//   whole tiles         a round of full tiles of all pairs costs 400 ns per k-block with 256 outputs, 275 with 128; the last round, with
+//                       fewer pairs at work, 273 to 399, or 207 to 289;
+//   all tiles cut       equal runs of k-blocks, and the hand-over (partial out, counter, partials in): 15 and 9 us more.  A k-block costs 417
+//                       or 272 ns, and more with many rows of A: the pairs stand at different places along K, so that what they ask of
+//                       L2 is not merged (7168 x 16384, 2300 rows: 0.63 us per k-block, 0.40 with whole tiles; a tenth of that where
+//                       every pair has one tile or less);
+//   the rest cut        the tiles beyond full rounds (or those and one round's) are cut and come first, whole tiles follow.
+// Fitted to whole and cut runs of both widths over 20 weights x 9 row counts, 160 to 4096 (whole tiles: within 3.5 % standard deviation).
+// Against one cost per k-block for both, and no rest, us:  7168 x 16384, 1300 / 2600 / 3500 rows 339 / 730 / 918 -> 262 / 526 / 647;
+// 6144 x 8192, 900: 103 -> 78; 25152 x 7168, 600 / 1300: 228 / 484 -> 192 / 378; 1536 x 12288, 3500: 120 -> 102; 198 shapes of 129 to
+// 3500 rows 0.97 in the mean.  gemm_rows_kernel: cycles, about 400 per k-block (the HBM rate), hand-over about 4000 and 50 per column.
+struct Shape { uint32_t nt, m_tiles, n_tiles[2], run, cut_tiles; };
 Shape pick_shape(const GemmCall& g, bool rows_kernel, uint32_t kb, const GemmWorkspace& ws)
 {
     Shape best{};
     uint64_t best_cost = ~0ull;
     const uint32_t workers = rows_kernel ? ws.blocks : ws.blocks / 2;
-    auto consider = [&](uint32_t nt, uint32_t m_side, uint32_t n_side, uint64_t cyc) {
-        Shape s{nt, (g.M + m_side - 1) / m_side, {0, 0}, 0};
+    auto consider = [&](uint32_t nt, uint32_t m_side, uint32_t n_side, auto whole_cost, auto cut_cost) {
+        Shape s{nt, (g.M + m_side - 1) / m_side, {0, 0}, 0, 0};
         for (int i = 0; i < g.n_weights; i++) s.n_tiles[i] = (g.w[i].N + n_side - 1) / n_side;
-        const uint64_t tiles = uint64_t(s.m_tiles) * (s.n_tiles[0] + s.n_tiles[1]);
-        const uint64_t per = (tiles + workers - 1) / workers, whole = per * kb * cyc;
-        const uint64_t run = (tiles * kb + workers - 1) / workers, cut = run * cyc + (rows_kernel ? 4000 + 50 * nt : 190 * nt);
-        s.run = uint32_t(per * kb);
-        if (whole < best_cost) { best_cost = whole; best = s; }
-        s.run = uint32_t(std::max<uint64_t>(run, 2));
-        if (cut < best_cost && tiles * (rows_kernel ? 1 : 2) <= ws.max_tiles) { best_cost = cut; best = s; }
+        const uint32_t tiles = s.m_tiles * (s.n_tiles[0] + s.n_tiles[1]), rounds = tiles / workers, rest = tiles % workers;
+        auto take = [&](uint64_t cost, uint64_t run, uint32_t cut_tiles) {
+            if (cost >= best_cost) return;
+            best_cost = cost;
+            best = s;
+            best.run = uint32_t(run);
+            best.cut_tiles = cut_tiles;
+        };
+        take(whole_cost(rounds, double(rest) / workers), uint64_t(rounds + (rest > 0)) * kb, 0);
+        for (uint32_t whole = 0; whole <= rounds; whole++) {             // rounds of whole tiles behind the cut ones
+            if (whole && (rows_kernel || whole + 1 < rounds)) continue;
+            const uint32_t cut = tiles - whole * workers;
+            const uint64_t run = std::max<uint64_t>({(uint64_t(cut) * kb + workers - 1) / workers, 2, whole ? kb / 4 : 0});
+            if (cut && cut * (rows_kernel ? 1 : 2) <= ws.max_tiles) take(cut_cost(run, whole, s.m_tiles), run, cut);
+        }
     };
-    if (rows_kernel) {
+    if (rows_kernel) {                                       // cycles
         const uint32_t nt = g.M <= 16 ? 16 : g.M <= 32 ? 32 : g.M <= 64 ? 64 : 128;
-        consider(nt, nt, BM, 400);
-    } else {
-        consider(256, 2 * BM, 256, 820);
-        consider(128, 2 * BM, 128, 610);
+        consider(nt, nt, BM, [&](uint64_t rounds, double rest) { return (rounds + (rest > 0)) * kb * 400; },
+                 [&](uint64_t run, uint64_t, uint64_t) { return run * 400 + 4000 + 50 * nt; });
+    } else {                                                 // nanoseconds
+        auto pairs = [&](uint32_t nt, double start, double tile, double full, double few, double more, double cut_start, double cut, double far) {
+            consider(nt, 2 * BM, nt,
+                     [=](uint64_t rounds, double rest) { return uint64_t(start + (rounds + (rest > 0)) * tile + kb * (rounds * full + (rest > 0 ? few + more * rest : 0))); },
+                     [=](uint64_t run, uint64_t rounds, uint64_t m_tiles) {
+                         const double rows = std::clamp<double>(double(m_tiles) * kb, 400, 2500) - 400;
+                         return uint64_t(cut_start + rounds * (tile + kb * full) + run * (cut + (run > kb ? 1.0 : 0.1) * far * rows));
+                     });
+        };
+        pairs(256, 6000, 0, 400, 273, 126, 20700, 417, 0.0716);
+        pairs(128, 4500, 420, 275, 207, 82, 13600, 272, 0.033);
     }
     return best;
 }
@@ -796,8 +826,9 @@ int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t*
     const uint32_t whole_tiles = a.units / a.kb;
     const uint32_t outputs = g.w[0].N + (g.n_weights > 1 ? g.w[1].N : 0u);
     a.group_m = rows_kernel ? a.m_tiles : group_of(g.K, outputs, a.m_tiles);
-    a.stride = !rows_kernel && a.run % a.kb == 0 ? std::min(whole_tiles, ws.blocks / 2) : 0u;
-    const uint32_t workers = a.stride ? a.stride : (a.units + a.run - 1) / a.run;
+    a.cut_tiles = sh.cut_tiles;
+    a.stride = std::max(1u, std::min(whole_tiles - sh.cut_tiles, ws.blocks / 2));          // all pairs where tiles are cut and others are whole
+    const uint32_t workers = rows_kernel || sh.cut_tiles == whole_tiles ? (a.units + a.run - 1) / a.run : a.stride;
     a.residual = g.residual ? 1u : 0u;
     a.tile_store = rows_kernel ? 0u : 1u;
     a.vec_io = 1u;
@@ -838,7 +869,7 @@ int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t*
     auto width = [&]<bool kPaged, bool kCut, bool kResidual, bool kTma>() {
         return nt == 256 ? go(gemm_pair_kernel<T, 256, kPaged, kCut, kResidual, kTma>) : go(gemm_pair_kernel<T, 128, kPaged, kCut, kResidual, kTma>);
     };
-    const bool cut = !a.stride;
+    const bool cut = sh.cut_tiles != 0;
     if (g.paged_map) {                                   // outputs in the library's own buffers
         if (!a.tile_store) return -1;
         return cut ? width.template operator()<true, true, false, true>() : width.template operator()<true, false, false, true>();

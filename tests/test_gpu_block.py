@@ -199,6 +199,8 @@ def test_projections_at_the_edges_of_their_tiles(torch, rows, H, E, R, shift):
     (1100, 72, 520, 0, 0), (600, 80, 520, 0, 0), (2300, 3, 1032, 0, 0),
     # outputs off a 16-byte boundary in both widths of tile, in whole runs and cut ones
     (1100, 72, 520, 0, 4), (777, 16, 2048, 0, 1),
+    # cut tiles ahead of a round of whole ones: the input projections, with TMA and without; the output projection
+    (1300, 16, 5120, 0, 0), (1500, 16, 5120, 0, 4), (2000, 48, 3072, 0, 0),
 ])
 def test_every_output_of_the_projections_and_nothing_beside_them(torch, rows, H, E, R, shift, dt):
     """Element by element against float64, and the values in front of and behind each output untouched.  An output is one rounding
