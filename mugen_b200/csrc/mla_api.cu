@@ -615,7 +615,7 @@ int ensure_gemm_workspace(mla_ctx* c)
     if (w.counters) return MLA_OK;
     w.blocks = uint32_t(c->sm_count);
     w.max_tiles = 16 * w.blocks;
-    CU_TRY(c, cudaError_t(mla::gemm_few_tc5_clusters(w.clusters)));
+    CU_TRY(c, cudaError_t(mla::gemm_few_tc5_clusters(int(c->cfg.dtype), w.clusters)));
     if (!w.partial) CU_TRY(c, cudaMalloc(&w.partial, mla::gemm_tc5_partial_bytes(w.blocks)));
     uint32_t* counters = nullptr;
     CU_TRY(c, cudaMalloc(&counters, w.max_tiles * 4));
@@ -841,7 +841,7 @@ int mla_create(const mla_config* cfg, mla_ctx** out)
         cp->err = std::string("tcgen05 prefill kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));
         return bail(MLA_ERR_CUDA);
     }
-    if (int ce = mla::gemm_tc5_configure()) {
+    if (int ce = mla::gemm_tc5_configure(int(cfg->dtype))) {
         cp->err = std::string("tcgen05 projection kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));
         return bail(MLA_ERR_CUDA);
     }

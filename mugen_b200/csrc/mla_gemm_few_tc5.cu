@@ -422,20 +422,17 @@ int launch_type(const GemmCall& g, uint32_t cs, uint32_t* status, const LaunchSt
 
 }  // namespace
 
-int gemm_few_tc5_configure()
-{
-    const cudaError_t e = configure_type<__half>();
-    return int(e != cudaSuccess ? e : configure_type<__nv_bfloat16>());
-}
+int gemm_few_tc5_configure(int dtype) { return int(dtype == 0 ? configure_type<__half>() : configure_type<__nv_bfloat16>()); }
 
 // clusters of 1, 2, 4 and 8 blocks that the current device holds at a time
-int gemm_few_tc5_clusters(uint32_t (&n)[4])
+int gemm_few_tc5_clusters(int dtype, uint32_t (&n)[4])
 {
     for (int i = 0; i < 4; i++) {
         cudaLaunchAttribute at[2];
         const cudaLaunchConfig_t cfg = launch_config(at, 1u << i, 1u << i, cudaStream_t(nullptr));
         int c = 0;
-        const cudaError_t e = cudaOccupancyMaxActiveClusters(&c, gemm_few_kernel<__half, 32, 4, kExchange>, &cfg);
+        const cudaError_t e = dtype == 0 ? cudaOccupancyMaxActiveClusters(&c, gemm_few_kernel<__half, 32, 4, kExchange>, &cfg)
+                                         : cudaOccupancyMaxActiveClusters(&c, gemm_few_kernel<__nv_bfloat16, 32, 4, kExchange>, &cfg);
         if (e != cudaSuccess) return int(e);
         n[i] = uint32_t(c);
     }

@@ -140,8 +140,8 @@ int launch_gemm_tc5(int dtype, const GemmCall& g, const GemmWorkspace& ws, uint3
 // The same for few rows and weights that fit the SMs in one go, the norm included (mla_gemm_few_tc5.cu); launch_gemm_tc5 picks.
 uint32_t gemm_few_tc5_cluster(const GemmCall& g, const uint32_t (&resident)[4]);
 int launch_gemm_few_tc5(int dtype, const GemmCall& g, uint32_t cs, uint32_t* status, const LaunchStream& st);
-int gemm_few_tc5_clusters(uint32_t (&n)[4]);
-int gemm_few_tc5_configure();
+int gemm_few_tc5_clusters(int dtype, uint32_t (&n)[4]);
+int gemm_few_tc5_configure(int dtype);
 size_t gemm_tc5_partial_bytes(uint32_t blocks);
 // Projection weights repacked into tiles (see the kernel file): values of the packed form, the packing itself, its maps.
 size_t gemm_tc5_packed_values(uint64_t N, uint64_t K);
@@ -149,7 +149,7 @@ int launch_gemm_pack(const void* src, void* dst, uint32_t N, uint32_t K, cudaStr
 bool gemm_tc5_packed_maps(GemmWeightMaps* maps, int dtype, const void* packed, uint64_t N, uint64_t K);
 bool gemm_tc5_weight_maps(GemmWeightMaps* maps, int dtype, const void* W, uint64_t rows, uint64_t K);
 int launch_rmsnorm_rows(int dtype, const void* x, const void* w, void* y, uint32_t rows, uint32_t N, float eps, const LaunchStream& st);
-int gemm_tc5_configure();
+int gemm_tc5_configure(int dtype);
 
 // Chunked prefill (mla_prefill_tc5.cu): causal flash attention of the new tokens of several sequences over expanded keys /
 // values (see the file's header).
