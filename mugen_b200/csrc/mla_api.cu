@@ -15,6 +15,7 @@
 
 #include "../host/page_table.hpp"
 #include "../host/rope_table.hpp"
+#include "../host/upload_order.hpp"
 #include "mla_launch.h"
 
 using mugen::mla::PageTable;
@@ -102,8 +103,7 @@ struct mla_ctx {
     size_t meta_cap = 0;
     char* meta_dev = nullptr;       // [kPlanRegions][meta_cap]
     char* meta_host = nullptr;      // [kMetaRing][meta_cap], page-locked
-    bool fresh = false;             // the last upload went to fresh_stream and no kernel has followed it there yet (launch_stream)
-    cudaStream_t fresh_stream = nullptr;
+    mugen::mla::UploadOrder<kPlanRegions> uploads;       // those that no kernel has followed yet (launch_stream)
     // Plans of the open step.  `plan`: every new token is a decode-style query row, one layer at a time.  A step that holds
     // prefill chunks (sequences taking >= kPrefillMin new tokens) also has `plan_rest`: its query rows are the step's OTHER
     // rows, the chunks go through the expanded-form prefill kernels (run_layer); the explicit per-layer calls
@@ -173,6 +173,15 @@ int pt_code(mla_ctx* c, int e)
     if (e == mugen::mla::PT_OK) return MLA_OK;
     c->err = c->pt->error();
     return e;   // PT_* values equal the MLA_ERR_* values they stand for
+}
+
+// Names a stream whatever handle it goes by: the default stream has two handles, the per-thread one is another stream in every
+// thread.  (cudaStreamGetId would tell them apart too, but a call of it ends a capture.)
+uint64_t stream_key(cudaStream_t st)
+{
+    static thread_local char this_thread;
+    if (st == cudaStreamPerThread) return uint64_t(reinterpret_cast<uintptr_t>(&this_thread));
+    return st == cudaStreamLegacy ? 0 : uint64_t(reinterpret_cast<uintptr_t>(st));
 }
 
 size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
@@ -453,8 +462,7 @@ int build_plan(mla_ctx* c, Plan& plan, int region, const std::vector<uint32_t>& 
                                        reinterpret_cast<const mla::PrefillTile*>(d + o_ctl) + g.tile0});
     }
     CU_TRY(c, cudaError_t(mla::launch_fetch(h, d, uint32_t(off / 16), st)));
-    c->fresh = true;
-    c->fresh_stream = st;
+    c->uploads.uploaded(size_t(region), stream_key(st));
     CU_TRY(c, cudaEventRecord(mb.done, st));
     mb.in_flight = true;
 
@@ -521,9 +529,9 @@ bool capturing(cudaStream_t st)
 }
 
 // the stream of a launch that may be the first behind an upload of metadata
-mla::LaunchStream launch_stream(const mla_ctx* c, cudaStream_t st) { return mla::LaunchStream(st, c->fresh && c->fresh_stream == st); }
+mla::LaunchStream launch_stream(const mla_ctx* c, cudaStream_t st) { return mla::LaunchStream(st, c->uploads.open(stream_key(st))); }
 // ... and once it is in the stream (a captured launch is not)
-void launched(mla_ctx* c, cudaStream_t st) { if (c->fresh && c->fresh_stream == st && !capturing(st)) c->fresh = false; }
+void launched(mla_ctx* c, cudaStream_t st) { if (c->uploads.open(stream_key(st)) && !capturing(st)) c->uploads.followed(stream_key(st)); }
 
 char* layer_pool(mla_ctx* c, uint32_t layer)
 {

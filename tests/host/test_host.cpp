@@ -14,6 +14,7 @@
 #include "../../mugen_b200/host/mla_host.hpp"
 #include "../../mugen_b200/host/page_table.hpp"
 #include "../../mugen_b200/host/rope_table.hpp"
+#include "../../mugen_b200/host/upload_order.hpp"
 
 #define CHECK(cond)                                                              \
     do {                                                                         \
@@ -335,6 +336,62 @@ static void test_few_ring()
     for (uint32_t kbs = 1; kbs <= 16; kbs++) CHECK((broken[kbs] > 0) == (kbs > R::stages));
 }
 
+// Uploads and launches in any order on three streams.  A launch must wait for an upload that stands between it and the kernel before
+// it on its stream, unless the region has been written anew since; no other launch needs to.  Returns (launches that did not wait and had to,
+// launches that waited for nothing).
+struct LastUpload {          // one upload remembered for all streams
+    uint64_t stream = 0;
+    bool fresh = false;
+    void uploaded(size_t, uint64_t s) { stream = s; fresh = true; }
+    bool open(uint64_t s) const { return fresh && stream == s; }
+    void followed(uint64_t s) { if (stream == s) fresh = false; }
+};
+template <typename Order>
+static std::pair<uint32_t, uint32_t> wrong_launches(uint32_t seed)
+{
+    Order order;
+    uint32_t early = 0, late = 0, version = 0, latest[4] = {};
+    std::vector<std::pair<uint32_t, uint32_t>> behind[3];       // (region, version) uploaded behind the last kernel of a stream
+    for (int i = 0; i < 400; i++) {
+        seed = seed * 1664525u + 1013904223u;
+        const uint32_t s = (seed >> 8) % 3, r = (seed >> 16) % 4;
+        if ((seed >> 24) % 2) {
+            order.uploaded(r, 10 + s);
+            latest[r] = ++version;
+            behind[s].push_back({r, version});
+        } else {
+            bool must = false;
+            for (auto [region, v] : behind[s]) must = must || latest[region] == v;
+            early += must && !order.open(10 + s);
+            late += !must && order.open(10 + s);
+            order.followed(10 + s);
+            behind[s].clear();
+        }
+    }
+    return {early, late};
+}
+
+static void test_upload_order()
+{
+    UploadOrder<4> order;
+    CHECK(!order.open(0));                                   // 0 is a stream like any other
+    order.uploaded(0, 7);                                    // step_begin on one stream, a group of layers on another
+    order.uploaded(2, 8);
+    CHECK(order.open(7) && order.open(8) && !order.open(9));
+    order.followed(8);
+    CHECK(order.open(7) && !order.open(8));
+    order.uploaded(0, 8);                                    // the next step, on the other stream
+    CHECK(!order.open(7) && order.open(8));
+    order.followed(8);
+    CHECK(!order.open(7) && !order.open(8));
+    uint32_t early = 0;
+    for (uint32_t seed = 1; seed <= 500; seed++) {
+        CHECK(wrong_launches<UploadOrder<4>>(seed) == std::make_pair(0u, 0u));
+        early += wrong_launches<LastUpload>(seed).first;
+    }
+    CHECK(early > 0);
+}
+
 static void test_wrapper_without_gpu()
 {
     LatentKVCacheConfig cfg;
@@ -399,6 +456,7 @@ int main(int argc, char** argv)
         test_planner();
         test_absorb_ring();
         test_few_ring();
+        test_upload_order();
         test_wrapper_without_gpu();
         std::puts("host units ok");
         return 0;

@@ -1096,6 +1096,51 @@ def test_calls_of_a_step_on_streams_of_their_own(torch):
     ctx.close()
 
 
+@pytest.mark.parametrize("how", ["another stream", "another handle"])
+def test_the_first_call_behind_an_upload_waits_for_it_whatever_went_elsewhere(torch, how):
+    """step_begin behind a busy stream, then a group of layers on a stream ordered behind it, whose own upload has its first launch
+    there, then an append on the first stream with nothing between it and the step's upload.  And the default stream by its other handle
+    (cudaStreamLegacy).  The rows of a step in between are what a call that is too early would write to."""
+    ctx, seqs, lens, kv, q = _step_ctx(torch)
+    L, B, H = q.shape[:3]
+    last = L - 1
+    ctx.step_begin(seqs)
+    ctx.step_append(last, kv[last])
+    ctx.step_end()
+    want = [ctx.read_rows(last, s, n, 1).copy() for s, n in zip(seqs, lens)]
+    ctx.rollback(seqs, lens)
+    other = ctx.seq_create()
+    ctx.step_begin([other])
+    ctx.step_append(last, kv[last, :1].contiguous())
+    ctx.step_end()
+    stale = ctx.read_rows(last, other, 0, 1).copy()
+    for s, n in zip(seqs, lens):
+        ctx.write_rows(last, s, n, torch.zeros((1, 576), dtype=torch.int16, device="cuda"))
+    ctx.write_rows(last, other, 0, torch.zeros((1, 576), dtype=torch.int16, device="cuda"))
+    out = torch.zeros((last, B, H, 128), dtype=torch.int16, device="cuda")
+    torch.cuda.synchronize()
+    a, b = torch.cuda.default_stream() if how == "another handle" else torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(a):
+        torch.cuda._sleep(20_000_000)              # about 10 ms
+        ctx.step_begin(seqs)
+    if how == "another stream":
+        b.wait_stream(a)
+        with torch.cuda.stream(b):
+            ctx.step_layers(0, last, kv[:last], q[:last], out)
+        with torch.cuda.stream(a):
+            ctx.step_append(last, kv[last])
+    else:
+        assert a.cuda_stream == 0
+        assert ctx.lib.mla_step_append(ctx.h, last, kv[last].data_ptr(), 1) == capi.OK
+    torch.cuda.synchronize()
+    ctx.step_end()
+    assert ctx.status() == 0
+    for s, n, w in zip(seqs, lens, want):
+        assert np.array_equal(ctx.read_rows(last, s, n, 1)[0], w[0])
+    assert not ctx.read_rows(last, other, 0, 1).any() and stale.any()
+    ctx.close()
+
+
 @pytest.mark.parametrize("how", ["layers", "calls"])
 def test_the_calls_of_an_open_step_can_be_captured(torch, how):
     """step_begin uploads; the calls behind it are launches alone, also inside a stream capture.  The graph is replayed over other
