@@ -184,6 +184,16 @@ uint64_t stream_key(cudaStream_t st)
     return st == cudaStreamLegacy ? 0 : uint64_t(reinterpret_cast<uintptr_t>(st));
 }
 
+bool capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
 size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
 // Sequences that take at least this many new tokens in a step go through the prefill kernels.
@@ -461,8 +471,12 @@ int build_plan(mla_ctx* c, Plan& plan, int region, const std::vector<uint32_t>& 
             c->chunk_groups.push_back({g.rows, g.n_tiles, reinterpret_cast<const uint32_t*>(d + o_cpg) + g.page0,
                                        reinterpret_cast<const mla::PrefillTile*>(d + o_ctl) + g.tile0});
     }
-    CU_TRY(c, cudaError_t(mla::launch_fetch(h, d, uint32_t(off / 16), st)));
-    c->uploads.uploaded(size_t(region), stream_key(st));
+    if (capturing(st)) {
+        CU_TRY(c, cudaMemcpyAsync(d, h, off, cudaMemcpyHostToDevice, st));       // a graph's kernels follow a copy without further care
+    } else {
+        CU_TRY(c, cudaError_t(mla::launch_fetch(h, d, uint32_t(off / 16), st)));
+        c->uploads.uploaded(size_t(region), stream_key(st));
+    }
     CU_TRY(c, cudaEventRecord(mb.done, st));
     mb.in_flight = true;
 
@@ -518,18 +532,12 @@ int rest_plan(mla_ctx* c, cudaStream_t st)
     return build_plan(c, c->plan_rest, kPlanRest, c->step_seqs, c->rows, &rest, &att_row, 1, st, &cm);
 }
 
-bool capturing(cudaStream_t st)
+// The stream of a launch that may be the first behind an upload of metadata.  A captured launch keeps its overlap: a graph starts when
+// what lies ahead of it in its stream is done, and inside a capture uploads are copies (build_plan).
+mla::LaunchStream launch_stream(const mla_ctx* c, cudaStream_t st)
 {
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return status != cudaStreamCaptureStatusNone;
+    return mla::LaunchStream(st, c->uploads.open(stream_key(st)) && !capturing(st));
 }
-
-// the stream of a launch that may be the first behind an upload of metadata
-mla::LaunchStream launch_stream(const mla_ctx* c, cudaStream_t st) { return mla::LaunchStream(st, c->uploads.open(stream_key(st))); }
 // ... and once it is in the stream (a captured launch is not)
 void launched(mla_ctx* c, cudaStream_t st) { if (c->uploads.open(stream_key(st)) && !capturing(st)) c->uploads.followed(stream_key(st)); }
 

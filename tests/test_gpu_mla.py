@@ -1185,6 +1185,117 @@ def test_the_calls_of_an_open_step_can_be_captured(torch, how):
     ctx.close()
 
 
+@pytest.mark.parametrize("how", ["layers", "calls", "block"])
+def test_calls_captured_on_the_stream_of_step_begin_keep_their_overlap(torch, how):
+    """Captured with nothing between them and the step's upload, the launches of a step follow each other by programmatic edges, all of
+    them.  Replayed at once behind the upload of a step, with another step's metadata in its place before and the stream
+    busy, the graph writes this step's rows and outputs."""
+    import ctypes as C
+    ctx, seqs, lens, kv, q = _step_ctx(torch)
+    L, B, H = q.shape[:3]
+    bits = lambda t: t.view(torch.int16).cpu().numpy().view(np.uint16)
+    E = 256
+    rn = lambda *shape: (torch.randn(shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(len(shape))) * 0.05).half()
+    for l in range(L if how == "block" else 0):
+        ctx.set_block_weights(l, attn_norm=bits(1 + rn(E)), kv_a_mqa=bits(rn(576, E)), wo=bits(rn(E, H * 128)), q=bits(rn(H * 192, E)))
+    ctx.set_q_rope(how == "block")
+    hidden, start = rn(B, E), rn(B, E)
+    out = torch.zeros((L, B, H, 128), dtype=torch.int16, device="cuda")
+
+    def calls():
+        if how == "layers":
+            ctx.step_layers(0, L, kv, q, out)
+        for l in range(L if how == "calls" else 0):
+            ctx.step_append(l, kv[l])
+            ctx.step_attend(l, q[l], out[l])
+        for l in range(L if how == "block" else 0):
+            ctx.step_block(l, hidden)
+
+    def end():
+        """Closes the step: its rows and outputs, which are zeros again behind it."""
+        got = [ctx.read_rows(l, s, n, 1).copy() for l in range(L) for s, n in zip(seqs, lens)], (hidden if how == "block" else out).clone()
+        ctx.step_end()
+        ctx.rollback(seqs, lens)
+        for l in range(L):
+            for s, n in zip(seqs, lens):
+                ctx.write_rows(l, s, n, torch.zeros((1, 576), dtype=torch.int16, device="cuda"))
+        hidden.copy_(start)
+        out.zero_()
+        return got
+
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        hidden.copy_(start)
+        for _ in range(2):                         # workspaces are there, kernels are loaded
+            ctx.step_begin(seqs)
+            calls()
+            end()
+        ctx.step_begin(seqs)
+        g = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(g, stream=stream):
+            before = ctx.launch_count()
+            calls()
+            n = ctx.launch_count() - before
+        # an edge's data are 8 bytes: ports of either end, kind of dependency (1: programmatic), nothing
+        edges, data = C.c_size_t(n - 1), (C.c_uint8 * 8 * (n - 1))()
+        ends = [(C.c_void_p * (n - 1))() for _ in range(2)]
+        assert C.CDLL("libcuda.so.1").cuGraphGetEdges_v2(C.c_void_p(g.raw_cuda_graph()), *ends, data, C.byref(edges)) == 0
+        assert edges.value == n - 1 and all(ends[1]) and [d[2] for d in data] == [1] * (n - 1)
+        g.instantiate()
+        stream.synchronize()
+        g.replay()
+        want = end()
+        for _ in range(3):
+            other = ctx.seq_create()
+            ctx.step_begin([other])
+            ctx.step_append(0, kv[0, :1].contiguous())
+            ctx.step_end()
+            ctx.seq_free(other)
+            torch.cuda._sleep(2_000_000)           # about a millisecond
+            ctx.step_begin(seqs)
+            g.replay()
+            got = end()
+            assert torch.equal(got[1], want[1]) and got[1].any() and all(np.array_equal(x, y) and x.any() for x, y in zip(got[0], want[0]))
+        assert ctx.status() == 0
+    del g
+    ctx.close()
+
+
+def test_a_step_that_is_captured_whole(torch):
+    """step_begin inside the capture as well (which waits for its turn in the upload ring: a relaxed capture lets it): its upload is
+    part of the graph, and the launches behind it find it complete."""
+    ctx, seqs, lens, kv, q = _step_ctx(torch)
+    L, B, H = q.shape[:3]
+    out, want = (torch.zeros((L, B, H, 128), dtype=torch.int16, device="cuda") for _ in range(2))
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        ctx.step_begin(seqs)
+        for l in range(L):
+            ctx.step_append(l, kv[l])
+            ctx.step_attend(l, q[l], want[l])
+        rows = [ctx.read_rows(l, s, n, 1).copy() for l in range(L) for s, n in zip(seqs, lens)]
+        ctx.step_end()
+        ctx.rollback(seqs, lens)
+        for l in range(L):
+            for s, n in zip(seqs, lens):
+                ctx.write_rows(l, s, n, torch.zeros((1, 576), dtype=torch.int16, device="cuda"))
+        stream.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream, capture_error_mode="relaxed"):
+            ctx.step_begin(seqs)
+            for l in range(L):
+                ctx.step_append(l, kv[l])
+                ctx.step_attend(l, q[l], out[l])
+        torch.cuda._sleep(2_000_000)
+        g.replay()
+        got = [ctx.read_rows(l, s, n, 1).copy() for l in range(L) for s, n in zip(seqs, lens)]
+        ctx.step_end()
+        assert ctx.status() == 0
+    assert torch.equal(out, want) and all(np.array_equal(x, y) and x.any() for x, y in zip(got, rows))
+    del g
+    ctx.close()
+
+
 def test_a_context_on_a_device_with_little_room_left(torch, oracle):
     """The workspace for groups of layers is a matter of speed: where it does not fit any more the context is created without it,
     and its steps give the same."""
