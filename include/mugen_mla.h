@@ -174,7 +174,8 @@ int mla_step_attend(mla_ctx* ctx, uint32_t layer, const void* q, void* out, void
  * [n_layers][rows][576], q DEVICE [n_layers][rows][n_heads][192], out DEVICE
  * [n_layers][rows][n_heads][128].  Appended rows are bit-identical to the per-layer calls'.  Layers of steps with few rows
  * are launched in groups, planned together: their KV ranges may be cut elsewhere, so outputs agree with the per-layer calls'
- * (and mla_step_layer_host's) within rounding, not bit for bit; the same call repeats its bits. */
+ * (and mla_step_layer_host's) within rounding, not bit for bit; the same call repeats its bits, also in another context of the
+ * same configuration (unless the device was nearly full when that one was made: then its groups are smaller). */
 int mla_step_layers(mla_ctx* ctx, uint32_t layer_begin, uint32_t n_layers, const void* kv_a,
                     const void* q, void* out, void* stream);
 /* Same two calls with HOST buffers: copies kv_a and q in, runs append + attend on `stream`, copies

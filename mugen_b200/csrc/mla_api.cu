@@ -204,10 +204,12 @@ constexpr uint32_t kPrefillMin = 64;
 // 40 single rows 201 -> 176, 128 of 2000 tokens 1470 -> 1415; 6 layers of 64 heads x 120 ragged sequences 334 -> 287; 3 layers of 128
 // heads x 128 837 -> 830; slower in one of 27 shapes (4 layers of 128 heads, 30 sequences x 4 rows: 466 -> 468).  160 MB give no more.
 constexpr uint64_t kGroupRows = 4096, kGroupBytes = 96ull << 20;
-// The smaller ones where less of the device is free when a context is made: what it or its caller allocates later (expanded keys of a
-// long prompt, weights) has the room that it had.
+// The smaller ones where pool and weights leave less than kRoomForGroups of the device: what the caller allocates beside them has the
+// room that it had.  Which ones a context has goes by its configuration, so that a program cuts KV ranges alike, and gives the same
+// bits, whatever else is on the device; but where the larger workspace would leave less than kLeftByGroups, and a later step could fail
+// for want of it, the smaller one is taken.
 constexpr uint64_t kSmallGroupRows = 1024, kSmallGroupBytes = 48ull << 20;
-constexpr size_t kRoomForGroups = 16ull << 30;
+constexpr size_t kRoomForGroups = 16ull << 30, kLeftByGroups = 1ull << 30;
 // Expanded keys and values of the chunks that share a launch (a chunk that needs more has one of its own).
 constexpr uint64_t kExpandBytes = 256ull << 20;
 
@@ -832,9 +834,9 @@ int mla_create(const mla_config* cfg, mla_ctx** out)
         return std::max<uint32_t>(c->cfg.max_rows, uint32_t(std::min<uint64_t>({uint64_t(c->cfg.max_rows) * cfg->n_layers, rows,
                                                                                 std::max<uint64_t>(1, bytes / row_bytes)})));
     };
-    size_t free_bytes = 0, total_bytes = 0;
-    CR_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
-    c->ws_rows = free_bytes >= kRoomForGroups ? group_rows(kGroupRows, kGroupBytes) : group_rows(kSmallGroupRows, kSmallGroupBytes);
+    const uint32_t small_groups = group_rows(kSmallGroupRows, kSmallGroupBytes);
+    const size_t own_bytes = pool_bytes + 3 * weight_bytes(cp) * cfg->n_layers;
+    c->ws_rows = prop.totalGlobalMem >= own_bytes + kRoomForGroups ? group_rows(kGroupRows, kGroupBytes) : small_groups;
     CR_TRY(cudaMalloc(&c->status_dev, sizeof(uint32_t)));
     CR_TRY(cudaMemset(c->status_dev, 0, sizeof(uint32_t)));
     c->meta_cap = meta_capacity(cp);
@@ -869,24 +871,34 @@ int mla_create(const mla_config* cfg, mla_ctx** out)
         cp->err = std::string("tcgen05 merge kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));
         return bail(MLA_ERR_CUDA);
     }
-    // The last allocations.  Where the device is too full for groups of layers and of rows, one layer of max_rows rows must do:
-    // steps then go layer by layer, and rows of one sequence share a stream of its pages as far as the records hold them.
-    auto workspace = [&](uint32_t rows, bool groups) -> cudaError_t {
+    // The last allocations.  Where the device is too full for groups of layers and of rows, smaller ones or one layer of max_rows rows
+    // must do: with the last of them steps go layer by layer, and rows of one sequence share a stream of its pages as far as the
+    // records hold them.
+    auto workspace = [&](uint32_t rows, bool groups, size_t left) -> cudaError_t {
         c->ws_rows = rows;
         // a plan has at most one segment per query group more than it has workers, each of up to group_heads (or H) records
         c->rec_cap = (size_t(workers_of(cp, c->kernel, H)) + rows) * H;
         if (groups && group_heads(cp) >= 2 * H) c->rec_cap += size_t(c->sm_count) * group_heads(cp) + size_t(rows) * H;
         // 64 spare rows: the tcgen05 kernels fetch queries in boxes of 64 head rows
         const size_t q_bytes = (size_t(rows) * H + 64) * mla::kRow * 2;
+        size_t free_bytes = 0, total_bytes = 0;
         cudaError_t e = cudaMalloc(&c->q_abs, q_bytes);
         if (e == cudaSuccess) e = cudaMalloc(&c->recs, c->rec_cap * mla::kPart * sizeof(float));
+        if (e == cudaSuccess) e = cudaMemGetInfo(&free_bytes, &total_bytes);
+        if (e == cudaSuccess && free_bytes < left) e = cudaErrorMemoryAllocation;
         if (e == cudaSuccess) return cudaMemset(c->q_abs, 0, q_bytes);
         cudaGetLastError();
         cudaFree(c->q_abs);
+        cudaFree(c->recs);
         c->q_abs = nullptr;
+        c->recs = nullptr;
         return e;
     };
-    if (workspace(c->ws_rows, true) == cudaErrorMemoryAllocation) CR_TRY(workspace(c->cfg.max_rows, false));
+    cudaError_t we = cudaErrorMemoryAllocation;
+    if (c->ws_rows > small_groups) we = workspace(c->ws_rows, true, kLeftByGroups);
+    if (we == cudaErrorMemoryAllocation) we = workspace(small_groups, true, 0);
+    if (we == cudaErrorMemoryAllocation) we = workspace(c->cfg.max_rows, false, 0);
+    CR_TRY(we);
     if (int rc = make_tensor_maps(cp)) return bail(rc);
     if (int ce = mla::decode_tc5_pair128_configure()) {
         cp->err = std::string("tcgen05 pair128 kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));

@@ -1346,6 +1346,39 @@ def test_a_context_on_a_device_with_little_room_left(torch, oracle):
     ctx.close()
 
 
+@pytest.mark.parametrize("room, groups", [(12 << 30, 1), (1 << 29, 3)])
+def test_what_else_is_on_the_device_does_not_change_the_groups(torch, room, groups):
+    """A context made with `room` bytes of the device left behind it, beside one with all of it: 27 layers of 101 rows are one group
+    whether 12 or 180 GB are free, and give the same bits.  Only where less than a gigabyte is left the groups are smaller."""
+    make = lambda: _step_ctx(torch, L=27, lens=[(29 * i) % 150 for i in range(101)])
+    outs = []
+    for full in (False, True):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        if full:
+            filler = torch.empty(torch.cuda.mem_get_info()[0] - need - room, dtype=torch.uint8, device="cuda")
+        else:
+            free = torch.cuda.mem_get_info()[0]
+        ctx, seqs, lens, kv, q = make()
+        if full:
+            del filler
+        else:
+            torch.cuda.synchronize()
+            need = free - torch.cuda.mem_get_info()[0]
+        out = torch.zeros((27, 101, 16, 128), dtype=torch.int16, device="cuda")
+        before = ctx.launch_count()
+        ctx.step_begin(seqs)
+        ctx.step_layers(0, 27, kv, q, out)
+        ctx.step_end()
+        assert ctx.status() == 0 and ctx.launch_count() - before == 3 * (groups if full else 1)
+        outs.append(_host(out))
+        ctx.close()
+    if groups == 1:
+        assert np.array_equal(outs[0], outs[1])
+    for l in (0, 13, 26):
+        check_close(outs[1][l], outs[0][l], synth.DT_F16, f"layer {l}")
+
+
 @pytest.mark.parametrize("n_seq, pages", [(1, 1), (85, 1), (86, 1), (300, 1), (40, 120)])
 def test_step_metadata_of_any_size_reaches_the_kernels(torch, n_seq, pages):
     """The metadata goes up in pieces of 16 bytes, 1,024 to a block: a step of many rows, or of many pages, writes the same cache rows
