@@ -745,7 +745,7 @@ def test_block_tables_are_permuted_pages(torch):
 @pytest.mark.parametrize("H,dt,L,lens", [
     (16, synth.DT_F16, 5, [200]),                                   # one row per layer: all layers in one group
     (40, synth.DT_BF16, 3, [1, 64, 65, 700, 0]),                    # tile edges and an empty sequence
-    (128, synth.DT_BF16, 7, [(37 * i) % 190 for i in range(100)]),  # 700 rows: groups of 3 layers and a tail of one
+    (128, synth.DT_BF16, 7, [(37 * i) % 190 for i in range(100)]),  # 700 rows: a group of 4 layers and one of 3
 ])
 def test_step_layers_in_groups_of_layers(torch, H, dt, L, lens):
     """step_layers plans groups of layers as one launch series; its cuts may differ from the per-layer calls', so outputs
@@ -1408,11 +1408,25 @@ def test_step_metadata_of_any_size_reaches_the_kernels(torch, n_seq, pages):
     assert np.array_equal(rows[0], rows[1]) and rows[0].any(axis=(1, 2)).all()
 
 
-@pytest.mark.parametrize("H,dt,L,rows", [
-    (5, synth.DT_F16, 27, 60),         # 1,620 rows: one group
-    (16, synth.DT_BF16, 27, 101),      # 2,727 of the 2,730 that 96 MB of queries hold
-    (16, synth.DT_F16, 9, 304),        # 2,736: five layers and four
-    (5, synth.DT_BF16, 9, 456),        # 4,104 of 4,096: five and four
+@pytest.mark.parametrize("H,dt,L,rows,groups", [
+    (5, synth.DT_F16, 27, 60, 1),          # 1,620 rows
+    (16, synth.DT_BF16, 27, 101, 1),       # 2,727
+    (5, synth.DT_BF16, 9, 455, 1),         # 4,095 of the 4,096 that a group may have
+    (5, synth.DT_BF16, 9, 456, 2),         # 4,104: five layers and four
+    (64, synth.DT_BF16, 5, 273, 1),        # 1,365 rows of 73,728 bytes: as many as 96 MB of queries hold
+    (64, synth.DT_F16, 5, 274, 2),         # 1,370: three layers and two
+    (128, synth.DT_BF16, 3, 227, 1),       # 681 of 682
+    (128, synth.DT_BF16, 3, 228, 2),       # 684: two layers and one
 ])
-def test_groups_of_layers_of_thousands_of_rows(torch, H, dt, L, rows):
+def test_groups_of_layers_of_thousands_of_rows(torch, monkeypatch, H, dt, L, rows, groups):
+    from mugen_b200.mla import MlaContext
+    launches, step_layers = [], MlaContext.step_layers
+
+    def counted(ctx, *args):
+        before = ctx.launch_count()
+        step_layers(ctx, *args)
+        launches.append(ctx.launch_count() - before)
+
+    monkeypatch.setattr(MlaContext, "step_layers", counted)
     test_step_layers_in_groups_of_layers(torch, H, dt, L, [(29 * i) % 150 for i in range(rows)])
+    assert launches == [3 * groups]                # absorb, attention, merge
