@@ -1535,8 +1535,9 @@ namespace {
 
 // out_i[rows][N_i] = act[rows][K] . W_i[N_i][K]^T, rounded to the storage type; residual: added to what out holds
 // norm_w: act's rows go through the RMSNorm first, by way of norm_out where the projection does not do it itself
+// exchanged: of the projection before, then of this one (launch_gemm_tc5)
 int project(mla_ctx* c, const void* act, uint32_t rows, uint32_t K, std::initializer_list<mla::GemmWeight> weights, bool residual, cudaStream_t st,
-            const void* norm_w = nullptr, void* norm_out = nullptr)
+            const void* norm_w = nullptr, void* norm_out = nullptr, bool* exchanged = nullptr)
 {
     mla::GemmCall g;
     g.A = act;
@@ -1548,7 +1549,8 @@ int project(mla_ctx* c, const void* act, uint32_t rows, uint32_t K, std::initial
     g.norm_w = norm_w;
     g.norm_out = norm_out;
     g.eps = c->cfg.rms_norm_eps;
-    const int rc = mla::launch_gemm_tc5(int(c->cfg.dtype), g, c->gemm_ws, c->status_dev, launch_stream(c, st), c->launches);
+    g.exchange_near = exchanged && *exchanged;
+    const int rc = mla::launch_gemm_tc5(int(c->cfg.dtype), g, c->gemm_ws, c->status_dev, launch_stream(c, st), c->launches, exchanged);
     if (rc == -1) return fail(c, MLA_ERR_INVALID, "projection operands must be 16-byte aligned with row lengths that are multiples of 8");
     if (rc != 0) return fail(c, MLA_ERR_CUDA, std::string("projection launch: ") + cudaGetErrorString(cudaError_t(rc)));
     if (rows) launched(c, st);
@@ -1570,8 +1572,9 @@ int project_in(mla_ctx* c, const BlockW& b, uint32_t rows, const void* hidden, v
     const mla::GemmWeight kv = gemm_weight(b.kv_a_map, uint32_t(mla::kRow), kv_a);
     if (!b.q_lora) return project(c, hidden, rows, E, {gemm_weight(b.q_map, QD, q), kv}, false, st, b.attn_norm, c->blk_hidden2);
     if (int e = grow(c, &c->blk_qa, &c->blk_qa_cap, size_t(rows) * b.q_lora * 2)) return e;
-    if (int e = project(c, hidden, rows, E, {gemm_weight(b.q_a_map, b.q_lora, c->blk_qa), kv}, false, st, b.attn_norm, c->blk_hidden2)) return e;
-    return project(c, c->blk_qa, rows, b.q_lora, {gemm_weight(b.q_b_map, QD, q)}, false, st, b.q_a_norm, c->blk_qa);
+    bool exchanged = false;
+    if (int e = project(c, hidden, rows, E, {gemm_weight(b.q_a_map, b.q_lora, c->blk_qa), kv}, false, st, b.attn_norm, c->blk_hidden2, &exchanged)) return e;
+    return project(c, c->blk_qa, rows, b.q_lora, {gemm_weight(b.q_b_map, QD, q)}, false, st, b.q_a_norm, c->blk_qa, &exchanged);
 }
 
 }  // namespace

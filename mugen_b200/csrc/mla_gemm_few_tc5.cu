@@ -407,12 +407,7 @@ int launch_type(const GemmCall& g, uint32_t cs, uint32_t* status, const LaunchSt
         return int(cudaLaunchKernelEx(&cfg, kernel, *g.w[0].map, *g.w[last].map, static_cast<const T*>(g.A), static_cast<const T*>(g.norm_w),
                                       static_cast<T*>(g.w[0].out), static_cast<T*>(g.w[last].out), a, status));
     };
-    // A warp's whole rows are a trip to L2 for every 256 pieces of 8 values of them, the exchange is one trip and one through the cluster:
-    // (16 heads, hidden 2048, input projections of 1 / 8 / 16 / 32 rows: 7.0 / 7.1 / 7.9 / 9.9 us by exchange, 5.7 / 5.8 / 7.0 / 8.6
-    // whole.)  Short rows of more than 8, where it matters least, use the exchange because the kernel for it has just run for the
-    // longer rows of q_a (16 blocks of 32 heads x 20 rows, hidden 4096, q_lora 512: 848 us whole, 840).
-    const bool whole = g.M <= 8 ? g.K <= 4096 : g.K >= 1024 && g.K <= 2048;
-    const int norm = !g.norm_w ? kNoNorm : whole ? kWhole : kExchange;
+    const int norm = !g.norm_w ? kNoNorm : gemm_few_tc5_exchanges(g) ? kExchange : kWhole;
     a.whole = norm == kWhole;
     auto pick = [&](auto none, auto exchange, auto whole) { return norm == kNoNorm ? go(none) : norm == kWhole ? go(whole) : go(exchange); };
     if (g.M <= 8) return go(gemm_few_kernel<T, 16, 1, kAny>);
@@ -476,6 +471,19 @@ uint32_t gemm_few_tc5_cluster(const GemmCall& g, const uint32_t (&resident)[4])
         return cs > 1 && kb - kbs >= spared && (cs > 2 || g.M <= 16 || blocks <= 96) ? cs : 0;
     }
     return 0;
+}
+
+// Whether the cluster's blocks exchange their shares of a row's squares; otherwise every warp sums its whole rows itself.
+// A warp's whole rows are a trip to L2 for every 256 pieces of 8 values of them, the exchange is one trip and one through the cluster:
+// (16 heads, hidden 2048, input projections of 1 / 8 / 16 / 32 rows: 7.0 / 7.1 / 7.9 / 9.9 us by exchange, 5.7 / 5.8 / 7.0 / 8.6
+// whole.)  For short rows of more than 8, where it matters least, the kernel is the better one whose instructions the projection just
+// before has fetched.  Blocks, us per layer, q_b by exchange / whole, 12 and 32 rows: 16 heads, hidden 2048, q_lora 512 (whole rows before)
+// 33.9 / 32.3 and 41.8 / 37.8; 32 heads, hidden 4096, q_lora 512 (exchange before) 41.7 / 41.6 and 52.9 / 53.9; 16 heads, hidden 7168, q_lora 768,
+// 32 rows (the general kernel before) 53.9 / 51.7.
+bool gemm_few_tc5_exchanges(const GemmCall& g)
+{
+    if (!g.norm_w) return false;
+    return g.M <= 8 ? g.K > 4096 : g.K > 2048 || (g.K < 1024 && g.exchange_near);
 }
 
 int launch_gemm_few_tc5(int dtype, const GemmCall& g, uint32_t cs, uint32_t* status, const LaunchStream& st)

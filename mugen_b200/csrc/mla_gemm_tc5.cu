@@ -924,8 +924,9 @@ bool gemm_tc5_weight_maps(GemmWeightMaps* maps, int dtype, const void* W, uint64
 
 // Returns a cudaError_t value, or -1 when the operands cannot be addressed (pointers must be 16-byte aligned, row lengths
 // multiples of 8).
-int launch_gemm_tc5(int dtype, const GemmCall& call, const GemmWorkspace& ws, uint32_t* status, const LaunchStream& st, uint64_t& launched)
+int launch_gemm_tc5(int dtype, const GemmCall& call, const GemmWorkspace& ws, uint32_t* status, const LaunchStream& st, uint64_t& launched, bool* exchanged)
 {
+    if (exchanged) *exchanged = false;
     if (call.M == 0 || call.n_weights == 0) return 0;
     GemmCall g = call;
     const bool aligned = (reinterpret_cast<uintptr_t>(g.A) & 15u) == 0;
@@ -939,6 +940,7 @@ int launch_gemm_tc5(int dtype, const GemmCall& call, const GemmWorkspace& ws, ui
     if (g.A && g.K % 8 == 0 && aligned && apart)
         if (const uint32_t cs = gemm_few_tc5_cluster(g, ws.clusters)) {
             launched++;
+            if (exchanged) *exchanged = gemm_few_tc5_exchanges(g);
             return launch_gemm_few_tc5(dtype, g, cs, status, st);
         }
     if (g.norm_w) {

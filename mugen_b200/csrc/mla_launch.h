@@ -128,6 +128,7 @@ struct GemmCall {
     const void* norm_w = nullptr;              // not null: A's rows go through the RMSNorm with this weight first, ...
     float eps = 0.0f;
     void* norm_out = nullptr;                  // ... rounded to the storage type here [M][K] where the kernel does not do it itself
+    bool exchange_near = false;                // the projection just before this one was one that gemm_few_tc5_exchanges
 };
 struct GemmWorkspace {
     float* partial;            // gemm_tc5_partial_bytes(blocks)
@@ -135,10 +136,12 @@ struct GemmWorkspace {
     uint32_t blocks, max_tiles;
     uint32_t clusters[4];      // gemm_few_tc5_clusters
 };
-// launched: kernels launched are added to it
-int launch_gemm_tc5(int dtype, const GemmCall& g, const GemmWorkspace& ws, uint32_t* status, const LaunchStream& st, uint64_t& launched);
+// launched: kernels launched are added to it.  exchanged: whether blocks traded sums of squares (gemm_few_tc5_exchanges)
+int launch_gemm_tc5(int dtype, const GemmCall& g, const GemmWorkspace& ws, uint32_t* status, const LaunchStream& st, uint64_t& launched,
+                    bool* exchanged = nullptr);
 // The same for few rows and weights that fit the SMs in one go, the norm included (mla_gemm_few_tc5.cu); launch_gemm_tc5 picks.
 uint32_t gemm_few_tc5_cluster(const GemmCall& g, const uint32_t (&resident)[4]);
+bool gemm_few_tc5_exchanges(const GemmCall& g);
 int launch_gemm_few_tc5(int dtype, const GemmCall& g, uint32_t cs, uint32_t* status, const LaunchStream& st);
 int gemm_few_tc5_clusters(int dtype, uint32_t (&n)[4]);
 int gemm_few_tc5_configure(int dtype);

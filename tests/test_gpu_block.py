@@ -466,8 +466,9 @@ def test_projections_whose_tiles_have_fewer_k_blocks_than_issuers(torch, E, rows
 @pytest.mark.parametrize("dt", ["f16", "bf16"])
 @pytest.mark.parametrize("rows,H,E,R", [
     (1, 2, 4096, 0), (1, 2, 4104, 0), (4, 2, 7168, 0), (8, 5, 6144, 136),         # up to 8 rows: whole rows up to 4,096 values, exchanged sums behind that
-    (9, 2, 1016, 0), (9, 2, 1024, 0), (16, 5, 2048, 0), (16, 2, 2056, 256),       # up to 16: whole from 1,024 to 2,048
+    (9, 2, 1016, 0), (9, 2, 1024, 0), (16, 5, 2048, 0), (16, 2, 2056, 256),       # up to 16: whole up to 2,048
     (17, 2, 1016, 0), (25, 2, 1032, 0), (32, 5, 2048, 1024), (31, 2, 2056, 0),    # up to 32
+    (10, 3, 1032, 72), (16, 5, 4096, 264), (18, 2, 2048, 1016), (32, 5, 2056, 264),      # short rows of q_a: as the projection before
 ])
 def test_projections_of_few_rows_in_every_form_of_the_norm(torch, rows, H, E, R, dt):
     test_projections_of_few_rows_in_every_cluster_size(torch, rows, H, E, R, dt)
