@@ -1362,6 +1362,7 @@ def test_what_else_is_on_the_device_does_not_change_the_groups(torch, room, grou
         ctx, seqs, lens, kv, q = make()
         if full:
             del filler
+            torch.cuda.empty_cache()
         else:
             torch.cuda.synchronize()
             need = free - torch.cuda.mem_get_info()[0]
