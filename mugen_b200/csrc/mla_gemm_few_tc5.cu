@@ -440,21 +440,28 @@ int gemm_few_tc5_clusters(int dtype, uint32_t (&n)[4])
 // of 2 835).
 // What a cluster gains over the general kernel are the k-blocks that a tile's block does not walk itself, and the hand-over of a cut
 // tile; what it loses is the way of the sums from block to block, more with more blocks and with more rows that each must finish.
-// One projection from packed weights in a chain of such launches, general kernel -> this one (us; - / +: the rule refuses / takes):
+// One projection from packed weights in a chain of launches of the same kernel, general kernel -> this one (us; - / +: the rule
+// refuses / takes):
 //   k-blocks  tiles  cluster  blocks    4 rows         16 rows        32 rows
-//      4       16       4       64     2.9 -> 2.9     3.0 -> 3.3     3.7 -> 4.2     -
-//      8       32       4      128     3.8 -> 4.2     4.0 -> 4.5     4.7 -> 5.5     -
-//     10       16       4       64     4.1 -> 3.0     4.3 -> 3.5     5.0 -> 4.6     +
-//     10       24       4       96     4.3 -> 3.9     4.4 -> 4.3     5.2 -> 5.3     + up to 8 rows
-//     10       72       2      144     4.5 -> 5.1     4.7 -> 5.6     5.5 -> 6.8     -
-//     16       48       2       96     5.6 -> 4.7     5.8 -> 5.3     6.6 -> 6.5     +
-//     16       72       2      144     6.5 -> 6.3     6.6 -> 6.8     7.4 -> 8.0     + up to 16 rows
-//     16       96       1       96     7.3 -> 7.6     7.5 -> 8.6                    -
-//     32       24       4       96     7.2 -> 5.0     7.4 -> 5.4     9.7 -> 6.4     +
-//     32       56       2      112     9.8 -> 7.8     9.9 -> 8.6                    +
+//      4       16       4       64     2.6 -> 2.9     2.8 -> 3.2     3.2 -> 3.8     -
+//      8       32       4      128     3.1 -> 4.2     3.2 -> 4.5     3.8 -> 5.0     -
+//     10       16       8      128     3.2 -> 3.1     3.4 -> 3.5     4.1 -> 4.1     +
+//     10       24       4       96     3.5 -> 4.0     3.8 -> 4.2     4.5 -> 4.8     + up to 8 rows
+//     10       72       2      144     4.5 -> 5.1     4.7 -> 5.6     5.4 -> 6.1     -
+//     16       48       2       96     5.1 -> 4.7     5.3 -> 5.2     6.0 -> 5.9     +
+//     16       72       2      144     5.9 -> 6.3     6.0 -> 6.7     6.6 -> 7.3     + up to 16 rows
+//     16       96       1       96     6.8 -> 7.6     7.0 -> 8.5                    -
+//     32       24       4       96     7.0 -> 5.0     7.4 -> 5.3     8.6 -> 5.8     +
+//     32       56       2      112     9.3 -> 8.0     9.6 -> 8.5                    +
+// In a block the rule takes it a little earlier than this chain says, because there the instructions of the one kernel are near, and
+// those of the other are fetched.  With limits as the chain has them (8 k-blocks spared in clusters of 8, 9 to 12 in those of 4, 8 and at most 112
+// blocks in those of 2) blocks of 4 to 8 heads, hidden 1024 to 7168, take 0.93 to 1.07 of their time, 1.005 in the mean, and more
+// where it is a user's common case: 5 heads, hidden 2048, 2 / 8 / 17 rows 24.7 / 24.4 / 28.0 us per layer, 25.5 / 25.8 / 29.7.
 // With the norm in front the general kernel has a launch more, and only single blocks with more than 8 rows lose: 64 heads, hidden
-// 4096, q_lora 512, all by the general kernel / both projections here / as the rule has it: 8 rows 14.7 / 12.9 / 12.9, 16 rows 14.7 /
-// 15.3 / 14.0, 32 rows 18.1 / 20.1 / 17.3.  16 heads x 4 rows: hidden 4096 13.0 -> 11.2, hidden 7168 with q_lora 1536 20.4 -> 17.3.
+// 4096, q_lora 512, all by the general kernel / both projections here / as the rule has it: 8 rows 13.0 / 10.6 / 10.6, 16 rows 13.2 /
+// 14.3 / 12.7, 32 rows 15.5 / 19.0 / 15.7.  16 heads x 4 rows: hidden 4096 10.8 -> 9.3, hidden 7168 with q_lora 1536 18.4 -> 15.1.
+// q_b alone by the general kernel where q_a exchanges (hidden 3072 and 4096, q_lora 512 and 768, 9 to 32 rows): slower in 31 of 36 blocks,
+// 0.97 to 1.05.
 uint32_t gemm_few_tc5_cluster(const GemmCall& g, const uint32_t (&resident)[4])
 {
     if (!g.packed || g.M > 32 || g.M == 0) return 0;

@@ -104,7 +104,6 @@ struct GemmArgs {
     uint32_t group_m;                   // tiles along A's rows that stand side by side in the line of tiles
     uint32_t packed;                    // weights in the layout of gemm_tc5_pack
     uint32_t residual;                  // out = T(float(out) + float(T(x))) instead of T(x)
-    uint32_t tile_store;                // pairs: outputs leave by TMA
     uint32_t vec_io;                    // outputs start on a 16-byte boundary
     const uint32_t* table;              // paged A: page of every 64 rows, else nullptr
     uint32_t layer, n_pages;
@@ -830,7 +829,7 @@ int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t*
     a.stride = std::max(1u, std::min(whole_tiles - sh.cut_tiles, ws.blocks / 2));          // all pairs where tiles are cut and others are whole
     const uint32_t workers = rows_kernel || sh.cut_tiles == whole_tiles ? (a.units + a.run - 1) / a.run : a.stride;
     a.residual = g.residual ? 1u : 0u;
-    a.tile_store = rows_kernel ? 0u : 1u;
+    bool tile_store = !rows_kernel;                          // pairs: outputs leave by TMA
     a.vec_io = 1u;
     a.packed = g.packed ? 1u : 0u;
     a.partial = ws.partial;
@@ -843,9 +842,12 @@ int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t*
         a.N[i] = w.N;
         a.w_row0[i] = w.row0;
         out[i] = static_cast<T*>(w.out);
-        if (reinterpret_cast<uintptr_t>(w.out) & 15u) a.vec_io = a.tile_store = 0u;
+        if (reinterpret_cast<uintptr_t>(w.out) & 15u) {
+            a.vec_io = 0u;
+            tile_store = false;
+        }
         // storage-type output with rows that TMA can address: the epilogue stores tiles (see the kernel)
-        if (a.tile_store && !make_matrix_map(&mc[i], dtype, w.out, g.M, w.N, 32)) a.tile_store = 0u;
+        if (tile_store && !make_matrix_map(&mc[i], dtype, w.out, g.M, w.N, 32)) tile_store = false;
     }
     if (g.paged_map) {
         a.table = g.table;
@@ -862,7 +864,7 @@ int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t*
         return nt == 16 ? go(gemm_rows_kernel<T, 16>) : nt == 32 ? go(gemm_rows_kernel<T, 32>)
              : nt == 64 ? go(gemm_rows_kernel<T, 64>) : go(gemm_rows_kernel<T, 128>);
     }
-    const CUtensorMap &c0 = a.tile_store ? mc[0] : m0, &c1 = a.tile_store ? mc[last] : m0;
+    const CUtensorMap &c0 = tile_store ? mc[0] : m0, &c1 = tile_store ? mc[last] : m0;
     auto go = [&](auto kernel) {
         return int(launch_pdl(kernel, dim3(2 * workers), dim3(PAIR_THREADS), size_t(pair_smem(int(nt))), st, pa, m0, m1, c0, c1, out[0], out[1], a, status));
     };
@@ -871,10 +873,10 @@ int launch_type(const GemmCall& g, const GemmWorkspace& ws, int dtype, uint32_t*
     };
     const bool cut = sh.cut_tiles != 0;
     if (g.paged_map) {                                   // outputs in the library's own buffers
-        if (!a.tile_store) return -1;
+        if (!tile_store) return -1;
         return cut ? width.template operator()<true, true, false, true>() : width.template operator()<true, false, false, true>();
     }
-    if (!a.tile_store) return width.template operator()<false, true, true, false>();
+    if (!tile_store) return width.template operator()<false, true, true, false>();
     if (g.residual) return cut ? width.template operator()<false, true, true, true>() : width.template operator()<false, false, true, true>();
     return cut ? width.template operator()<false, true, false, true>() : width.template operator()<false, false, false, true>();
 }
