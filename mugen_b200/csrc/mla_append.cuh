@@ -37,7 +37,7 @@ constexpr int kAppendRowSmem = kRank * 4;      // the row's squares: 2,048 bytes
 // pairs (i, i + 32) meet by a shuffle): only its squares go through shared memory, to the lane that adds them.
 // What bounds it is that sum, a chain of 512 dependent additions: 1.1 us, 1.3 to 2.5 measured.  (The whole row through shared memory in
 // 16-bit values, then its squares, a value at a time, and the sum without the loads ahead of it: 4.1 us for the sum, 5.5 in all; 27
-// blocks over a 777-token prompt 1806 -> 1725 us, 8 layers of 128 heads x 8 sequences by calls 456 -> 454.)
+// blocks over a 777-token prompt 1806 -> 1725 us.)
 template <typename T>
 struct AppendRow {
     bool live = false;
