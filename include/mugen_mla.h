@@ -51,8 +51,8 @@ enum { MLA_W_F16 = 1, MLA_W_Q4_0 = 2, MLA_W_Q8_0 = 8, MLA_W_BF16 = 30 };
 /* Split-KV attention kernel family (mla_config.kernel).  AUTO picks, by the head rows that one stream of a
  * sequence's pages serves (n_heads, or several new tokens of one sequence x n_heads where they fit 128), PAIR128 above
  * 64 (SM pairs, tcgen05.mma.cta_group::2, 128-token tiles), TCGEN05_T16 up to 16 (tcgen05 in the transposed form: the
- * tokens of a page are the rows of the tile, groups of 16 heads its columns) and TCGEN05 between (one SM per group of
- * up to 64).  MMA (mma.sync m16n8k16, any head count) stays selectable.  All give
+ * tokens of a page are the rows of the tile, groups of 16 heads its columns) and TCGEN05 between (the same form with
+ * 32, 48 or 64 columns).  MMA (mma.sync m16n8k16, any head count) stays selectable.  All give
  * the same results within the attention tolerance; each is bit-reproducible from run to run. */
 enum { MLA_KERNEL_AUTO = 0, MLA_KERNEL_MMA = 1, MLA_KERNEL_TCGEN05 = 2, MLA_KERNEL_TCGEN05_PAIR128 = 3,
        MLA_KERNEL_TCGEN05_T16 = 4 };

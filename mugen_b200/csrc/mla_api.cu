@@ -294,10 +294,8 @@ uint32_t workers_of(const mla_ctx* c, uint32_t kernel, uint32_t heads)
 }
 
 // The attention kernel for `heads` head rows over one stream of the cache.  More than 64 rows go to the SM-pair kernel,
-// which streams the cache once for 128 of them at the same rate whether all are live or not (a second pass of the 64-row
-// kernel costs more than the padding); up to 16 take the transposed tcgen05 form (tokens as rows, the heads as 16
-// columns); everything between fills (part of) the 64-row tiles of the single-block kernel (measured at 32 heads, 64
-// sequences x 8192 tokens: 128 us against 186 us for two passes of the 16-column form and 300 us for mma.sync).
+// which streams the cache once for 128 of them at the same rate whether all are live or not (a second pass of the 64-column
+// kernel costs more than the padding); up to 64 take the transposed form with 16 columns (T16) or as many as the rows need.
 uint32_t kernel_for(const mla_ctx* c, uint32_t heads)
 {
     if (c->cfg.kernel != MLA_KERNEL_AUTO) return c->cfg.kernel;
@@ -595,9 +593,9 @@ int run_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, float* expo
         e = mla::launch_decode_tc5_pair128(dt, c->tmaps, c->pool, layer, c->cfg.n_pages, m, c->recs, H, p.max_pages <= 64 ? 1u : 0u,
                                            next_w, next_w ? uint32_t(weight_bytes(c)) : 0u, c->status_dev, st);
     else if (p.kernel == MLA_KERNEL_TCGEN05)
-        e = mla::launch_decode_tc5(dt, c->tmaps, c->pool, layer, c->cfg.n_pages, m, c->recs, H, c->status_dev, st);
+        e = mla::launch_decode_tc5(dt, mla::decode_tc5_columns(m.rec_stride), c->tmaps, c->pool, layer, c->cfg.n_pages, m, c->recs, H, c->status_dev, st);
     else if (p.kernel == MLA_KERNEL_TCGEN05_T16)
-        e = mla::launch_decode_tc5_t16(dt, c->tmaps, c->pool, layer, c->cfg.n_pages, m, c->recs, H, c->status_dev, st);
+        e = mla::launch_decode_tc5(dt, 16, c->tmaps, c->pool, layer, c->cfg.n_pages, m, c->recs, H, c->status_dev, st);
     else
         e = mla::launch_decode_mma(dt, c->q_abs, layer_pool(c, layer), c->cfg.n_pages, m, c->recs, H, c->status_dev, st);
     if (e != 0) return fail(c, MLA_ERR_CUDA, std::string("attention launch: ") + cudaGetErrorString(cudaError_t(e)));
@@ -749,16 +747,15 @@ int make_tensor_maps(mla_ctx* c)
     {
         const cuuint64_t dims[4] = {64, c->pool_slots, 9, c->cfg.n_layers};
         const cuuint64_t strides[3] = {cuuint64_t(mla::kRow) * 2, 128, c->pool_slots * mla::kRow * 2};
-        const cuuint32_t box_v[4] = {64, 64, 2, 1}, box_page[4] = {64, 64, 9, 1};
+        const cuuint32_t box_v[4] = {64, 64, 2, 1};
         if (int e = encode(mla::kMapPoolV, "cache pool, two chunks of a page", 4, c->pool, dims, strides, box_v)) return e;
-        if (int e = encode(mla::kMapPoolPage, "cache pool, whole page", 4, c->pool, dims, strides, box_page)) return e;
-        // 64 spare rows behind the queries: boxes of 64 head rows may start at the last row's heads
+        // 64 spare rows behind the queries: boxes of up to 64 head rows may start at the last row's heads
         const cuuint64_t qdims[3] = {64, cuuint64_t(c->ws_rows) * c->cfg.n_heads + 64, 9};
         const cuuint64_t qstrides[2] = {cuuint64_t(mla::kRow) * 2, 128};
-        const cuuint32_t qbox[3] = {64, 64, 9};
-        if (int e = encode(mla::kMapQueries, "absorbed queries", 3, c->q_abs, qdims, qstrides, qbox)) return e;
-        const cuuint32_t qbox16[3] = {64, 16, 9};
-        if (int e = encode(mla::kMapQueries16, "absorbed queries, 16 heads", 3, c->q_abs, qdims, qstrides, qbox16)) return e;
+        for (int head_rows : {16, 32, 48, 64}) {
+            const cuuint32_t qbox[3] = {64, cuuint32_t(head_rows), 9};
+            if (int e = encode(mla::query_map(head_rows), "absorbed queries", 3, c->q_abs, qdims, qstrides, qbox)) return e;
+        }
     }
     return MLA_OK;
 }
@@ -904,12 +901,8 @@ int mla_create(const mla_config* cfg, mla_ctx** out)
         cp->err = std::string("tcgen05 pair128 kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));
         return bail(MLA_ERR_CUDA);
     }
-    if (int ce = mla::decode_tc5_configure()) {
+    if (int ce = mla::decode_tc5_configure(int(cfg->dtype))) {
         cp->err = std::string("tcgen05 kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));
-        return bail(MLA_ERR_CUDA);
-    }
-    if (int ce = mla::decode_tc5_t16_configure()) {
-        cp->err = std::string("tcgen05 16-head kernel configuration: ") + cudaGetErrorString(cudaError_t(ce));
         return bail(MLA_ERR_CUDA);
     }
 #undef CR_TRY

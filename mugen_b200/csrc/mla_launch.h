@@ -53,30 +53,31 @@ int launch_decode_mma(int dtype, const void* q_abs, const void* layer_pool, uint
                       const StepMeta& m, float* recs, uint32_t H, uint32_t* status, cudaStream_t st);
 int decode_mma_configure();   // the *_configure() functions set kernel attributes on the CURRENT device: once per device
 
-// Split-KV attention on the 5th-generation tensor cores (tcgen05.mma, accumulators in TMEM,
-// cache tiles staged by TMA): grid (persistent blocks, ceil(H/64)).  tmaps points at the context's
-// host CUtensorMap array (kMap* below), pool at the whole cache pool; this kernel uses kMapPoolPage and kMapQueries.
-int launch_decode_tc5(int dtype, const void* tmaps, const void* pool, uint32_t layer0, uint32_t n_pages, const StepMeta& m,
+// Split-KV attention on the 5th-generation tensor cores (tcgen05.mma, accumulators in TMEM, cache tiles staged by TMA), tokens as M
+// rows, `columns` (16, 32, 48 or 64) head rows as columns: grid (persistent blocks, groups of head rows).  tmaps points at the
+// context's host CUtensorMap array (kMap* below), pool at the whole cache pool; uses kMapPoolV, kMapPoolSub and query_map(columns).
+int launch_decode_tc5(int dtype, uint32_t columns, const void* tmaps, const void* pool, uint32_t layer0, uint32_t n_pages, const StepMeta& m,
                       float* recs, uint32_t H, uint32_t* status, cudaStream_t st);
-int decode_tc5_configure();   // sets the kernel's attributes on the current device
-
-// The transposed form for narrow head counts (mla_decode_tc5_t16.cu): tokens are the M rows, groups of 16 heads the N
-// columns; grid (persistent blocks, ceil(H/16)).  Uses kMapPoolV, kMapPoolSub and kMapQueries16.
-int launch_decode_tc5_t16(int dtype, const void* tmaps, const void* pool, uint32_t layer0, uint32_t n_pages, const StepMeta& m, float* recs,
-                          uint32_t H, uint32_t* status, cudaStream_t st);
-int decode_tc5_t16_configure();
+int decode_tc5_configure(int dtype);   // sets the kernels' attributes on the current device
+// columns for a launch whose largest query group has `heads` head rows
+inline uint32_t decode_tc5_columns(uint32_t heads) { return heads <= 32 ? 32 : heads <= 48 ? 48 : 64; }
 
 // Tensor maps a context builds once (mla_api.cu, make_tensor_maps), by index into its array.
 enum : int {
     kMapPoolSub = 0,      // cache pool [layers][slots][576]: box 64 values x 64 tokens (one K sub-tile)
     kMapPoolV = 1,        // cache pool, whole-row view (64 values, slots, 9 chunks, layers): box 64 tokens x 2 chunks
     kMapQueries = 2,      // absorbed queries, whole-row view: box 64 head rows x 9 chunks
-    kMapPoolPage = 3,     // cache pool, whole-row view: box 64 tokens x 9 chunks (one page in one instruction)
-    kMapQueries16 = 4,    // absorbed queries, whole-row view: box 16 head rows x 9 chunks
-    kMapCount = 5
+    kMapQueries16 = 3,    // the same with 16, 32 and 48 head rows
+    kMapQueries32 = 4,
+    kMapQueries48 = 5,
+    kMapCount = 6
 };
+constexpr int query_map(uint32_t head_rows)
+{
+    return head_rows == 16 ? kMapQueries16 : head_rows == 32 ? kMapQueries32 : head_rows == 48 ? kMapQueries48 : kMapQueries;
+}
 
-// The same on a pair of SMs (cluster of 2, tcgen05.mma.cta_group::2), 128-token tiles (two pages per score
+// Split-KV attention on a pair of SMs (cluster of 2, tcgen05.mma.cta_group::2), 128-token tiles (two pages per score
 // MMA series): grid (2 x persistent pairs, ceil(H/128)).  Uses kMapPoolSub, kMapPoolV, kMapQueries and the
 // whole pool.
 int launch_decode_tc5_pair128(int dtype, const void* tmaps, const void* pool, uint32_t layer0, uint32_t n_pages,

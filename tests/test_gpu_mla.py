@@ -829,6 +829,33 @@ def test_rows_of_one_sequence_share_a_stream(torch, oracle, H, dt, spec):
     ctx.close()
 
 
+@pytest.mark.parametrize("H,dt", [(16, synth.DT_BF16), (17, synth.DT_F16), (32, synth.DT_BF16), (33, synth.DT_F16), (48, synth.DT_BF16),
+                                  (49, synth.DT_F16), (64, synth.DT_BF16)])
+def test_transposed_attention_at_the_edges_of_its_widths(torch, oracle, H, dt):
+    """Both sides of every width of the transposed kernel: rows of one token, a full page, one token more, and long ones whose scores rise
+    from page to page, so that references move on later pages; 320 rows, so that a block walks several segments and its rings of
+    pages wrap many times.  Bounds as everywhere here."""
+    lens = [1, 64, 65, 1100]
+    case = synth.make_layer_case(9100 + H, H, lens, dt, q_scale=3.0)
+    for i, n in enumerate(lens):
+        ramp = np.linspace(0.2, 2.0, n, dtype=np.float32)[:, None]
+        case.caches[i] = synth.to_bits(synth.from_bits(case.caches[i], dt) * ramp, dt)
+    times = 80
+    ctx = make_ctx(case, capi.KERNEL_AUTO, shuffle=5, max_rows=len(lens) * times)
+    seqs = fill(torch, ctx, case)
+    want = [oracle_out(oracle, case, b) for b in range(len(lens))]
+    out = torch.zeros((len(lens) * times, H, 128), dtype=torch.int16, device="cuda")
+    ctx.attend_rows(0, seqs * times, lens * times, _dev(torch, np.tile(case.q, (times, 1, 1))), out)
+    got = _host(out)
+    assert ctx.status() == 0 and ctx.kernel_name() == ("tcgen05-t16" if H <= 16 else "tcgen05")
+    for r in range(len(lens) * times):
+        check_close(got[r], want[r % len(lens)], dt, f"row {r}")
+    again = torch.zeros_like(out)
+    ctx.attend_rows(0, seqs * times, lens * times, _dev(torch, np.tile(case.q, (times, 1, 1))), again)
+    assert np.array_equal(_host(again), got)
+    ctx.close()
+
+
 @pytest.mark.parametrize("H,dt,lens", [
     (5, synth.DT_F16, [6000]),                             # one row in 94 parts: sixteen warps share its dims
     (32, synth.DT_BF16, [2100]),
