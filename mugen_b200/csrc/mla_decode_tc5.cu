@@ -85,6 +85,9 @@ struct Plan {
     static_assert(SMEM_BYTES <= SMEM_MAX && PAIRS >= 6, "shared memory of one block");
     static_assert(OFF_PAIRS % 1024 == 0 && OFF_ROPE % 1024 == 0 && OFF_P % 1024 == 0, "swizzled tiles need 1 KB alignment");
     static_assert((4 + S_TILES * PARTS) * NH <= 512, "tensor memory");
+    // A barrier wait names its phase by one bit: an issuer may wait for a slot's next filling only when the one before has landed, although
+    // another issuer waited for that one.  It works on page t when all have worked on page t - S_TILES; a filling earlier is PAIRS pairs back.
+    static_assert(PAIRS >= 4 * S_TILES, "phases of the pair ring");
     static_assert(B_COUNT * 8 <= M_TMEM, "barriers overflow their area");
 };
 

@@ -1,43 +1,34 @@
 // Split-KV absorbed MLA attention for 128-head groups on a PAIR of SMs, 128-token super-tiles
 // (thread-block cluster of 2, tcgen05.mma.cta_group::2), sm_100a.
 //
-// Same division of labour as mla_decode_tc5_pair.cu (each block: 64 heads, its 256 latent dims of
-// V, O^T for its dims x all 128 heads), but a tile is TWO pages and the pair's score MMA has
-// N = 128: block r stages the whole K of page r (the B operand's rows 64r .. 64r+63).  Measured on
-// B200 with four issuing warps, a cta_group::2 M128 N64 K16 MMA occupies the tensor pipe for 33
-// cycles and the N128 one for 44, so the 72 score MMAs of two pages (2,380 cycles) become 36
-// (1,580); with the 16 value MMAs (M256 N128 K16, 77 cycles each) a 128-token tile needs ~2,800
-// pipe cycles instead of ~3,600, which is below the time HBM needs to deliver it.
+// Each block has 64 heads, its 256 latent dims of V, and O^T for its dims x all 128 heads.  A tile is two pages, and the pair's score
+// MMA has N = 128: block r stages the whole K of page r (the B operand's rows 64r .. 64r+63).
 //
-// Shared memory is exactly full (Q' 72 KB, K 72 KB, V 64 KB, P 16 KB, 3 KB of barriers and
-// scratch), so K and V are not double-buffered as a whole.  Every K sub-tile [64 tokens][64 dims]
-// and every V buffer [page][128-dim chunk] has its own "full" barrier and is re-loaded as soon as
-// the MMAs that read it have completed; the "empty" side is signalled per release round (K
-// sub-tiles {0-3}, {4-7}, {8}; V per page) so that a producer thread pays one shared-memory round
-// trip (~300 cycles while the MMAs stream their operands) per round, not per buffer.  The dynamic
-// shared segment must start 1 KB-aligned because there is no slack to round up (checked; the
-// status word says so if not).
+// Shared memory is exactly full (Q' 72 KB, K 72 KB, V 64 KB, P 16 KB, 3 KB of barriers and scratch), so K and V are not double-buffered
+// as a whole: every pair of K sub-tiles [64 tokens][2 x 64 dims], the rope sub-tile and every V buffer [page][128-dim chunk] is
+// re-loaded as soon as the MMAs that read it have completed.  The dynamic shared segment must start 1 KB-aligned because there is
+// no slack to round up (checked; the status word says so if not).
 //
-// TMEM: O^T 2 x 128 columns; four partial score tiles of 64 columns, one per issuing warp (a warp
-// waits ~50-100 cycles per MMA it issues, so four of them are needed to keep the pipe busy).  Each
-// accumulator has ONE issuing thread and the softmax adds the partials in a fixed order, so the
-// result is bit-reproducible from run to run and under any page permutation.  (A variant with two
-// partials shared by two issuers each and the score tile double-buffered took the same time and
-// lost that property: the order of the accumulations then depends on timing.)
+// TMEM: O^T 2 x 128 columns; two score tiles of two partial sums of 64 columns, one per issuing warp.  Each accumulator has ONE
+// issuing thread and the softmax adds the partials in a fixed order, so the result is bit-reproducible from run to run and under any
+// page permutation.
 //
-// Warps: 0 K producer, 1-4 score issuers (sub-tiles {0,4,8} {1,5} {2,6} {3,7}), 5-6 value issuers
-// (one per chunk), 7 V producer (+ optional linear L2 prefetch of later pages), 8-15 softmax.  The
-// softmax computes its exponentials optimistically against the current reference maximum while the
-// cluster round that tells whether any head of the pair must move its maximum is in flight; only
-// in that rare case they are redone and O^T rescaled.  Waiting threads sleep in the barrier unit
-// (try_wait with a time hint) rather than re-poll: shared-memory bandwidth is what the MMA operand
-// fetches and the TMA fills compete for.  All waits are bounded.
+// Warps: 0 K producer, 1-2 score issuers (pairs {0,2}, {1,3} and the rope sub-tile), 3-4 value issuers (one per chunk), 5 V producer,
+// 6-13 softmax.  The softmax computes its exponentials optimistically against the current reference maximum while the
+// cluster round that tells whether any head of the pair must move its maximum is in flight; only in that rare case they are redone
+// and O^T rescaled.  Waiting threads sleep in the barrier unit (try_wait with a time hint) rather than re-poll: shared-memory
+// bandwidth is what the MMA operand fetches and the TMA fills compete for.  All waits are bounded.
 //
-// What bounds it, measured with clock64 and %globaltimer inside a traced build of the kernel: about
-// 400k SM cycles per launch at batch 64 x ctx 16384 at an effective SM clock of 1.55 GHz, although
-// nvidia-smi reports 1.97 GHz around a short run: the clock is throttled within the kernel, and
-// variants of this kernel that need fewer or more cycles (prefetch on or off, polling hints, score
-// double-buffering, producer layouts) all take the same 260-275 us.
+// What bounds it, from clock64 marks in a traced build (32 sequences x 8191 tokens): the period of a tile is 2,900 cycles, of which the
+// MMAs (36 of 44 cycles, 16 of 77) need 2,816; HBM needs 1.67 us for it, 3,280 cycles at 1.965 GHz.  Before, K was released in three
+// rounds of four sub-tiles and the softmax read four partial score tiles, and the period was 3,530: a K load takes 2,200 cycles and
+// nothing waited for it but the next tile.  Long lists run into the power cap (SM clock 1.2 to 1.5 GHz) and follow energy
+// instead: with a quarter of the score MMAs / of the value MMAs / without the V loads / the exponentials 4 layers of 64 x 16383 take
+// 1,144 / 1,165 / 1,229 / 1,276 us instead of 1,305.  Before / now: 4 layers of 64 x 16383 tokens 1,317 / 1,272 us, eight
+// launches of 8 x 16383 tokens 492 / 468, one sequence of 131,072 tokens 243 / 231 (4 %, 1.5 % and 2 % of it because no array is
+// indexed by the tile's parity and no wait ends with a vote: they sat on the chain from scores to P).
+// Not better: K 6 pairs deep with 2 V buffers (period 5,040) or 5 with 3 (3,710), where V, 1,400 cycles from L2, holds P up; the
+// other block's V loaded over K pairs that have been read, two tiles in flight (4,010).
 #include "mla_launch.h"
 #include "mla_tc5.cuh"
 
@@ -53,13 +44,14 @@ constexpr int HG = 64;                              // heads per block (128 per 
 constexpr int NSUB = kRow / 64;                     // 9
 constexpr int SUB_BYTES = kPage * 128;              // 8,192: [64 tokens or heads][64 values]
 constexpr int Q_BYTES = NSUB * SUB_BYTES;           // 73,728
-constexpr int K_BYTES = NSUB * SUB_BYTES;           // 73,728: the whole K of this block's page
-constexpr int VBUF_BYTES = 2 * SUB_BYTES;           // 16,384: 64 tokens x 128 dims (one page, one chunk)
+constexpr int PAIR_BYTES = 2 * SUB_BYTES;           // 16,384: sub-tiles 2i, 2i+1 of a page
 constexpr int P_BYTES = HG * 128;                   // 8,192 per page
+constexpr int PAGE_BYTES = kPage * kRow * 2;
 constexpr int OFF_Q = 0;
 constexpr int OFF_K = OFF_Q + Q_BYTES;
-constexpr int OFF_V = OFF_K + K_BYTES;                      // [page][chunk]
-constexpr int OFF_P = OFF_V + PAGES * 2 * VBUF_BYTES;       // [page]
+constexpr int OFF_V = OFF_K + 4 * PAIR_BYTES;                  // [page][chunk]
+constexpr int OFF_ROPE = OFF_V + PAGES * 2 * PAIR_BYTES;
+constexpr int OFF_P = OFF_ROPE + SUB_BYTES;                 // [page]
 constexpr int OFF_MISC = OFF_P + PAGES * P_BYTES;
 constexpr int MISC_BYTES = 3072;
 constexpr int SMEM_BYTES = OFF_MISC + MISC_BYTES;           // 232,448 = all of it: no alignment slack
@@ -77,24 +69,20 @@ constexpr int M_LSUM = 1536;      // [3][64] floats: the other quarters' partial
 
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t COL_O = 0;       // 2 chunks x 128 head columns
-constexpr uint32_t COL_S = 256;     // 4 partial score tiles x 64 columns
+constexpr uint32_t COL_S = 256;     // 2 score tiles x 2 partial sums x 64 columns
 
-constexpr int N_QK = 4, N_PV = 2;
-constexpr int NUM_THREADS = 32 * (2 + N_QK + N_PV + 8);   // 512
+constexpr int N_QK = 2, N_PV = 2;
+constexpr int FIRST_SOFTMAX_WARP = 2 + N_QK + N_PV;
+constexpr int NUM_THREADS = 32 * (FIRST_SOFTMAX_WARP + 8);
 constexpr int SOFTMAX_THREADS = 256;
 constexpr int PAIR_SOFTMAX_WARPS = 16;
 constexpr float RESCALE_THRESHOLD = 8.0f;
 
-// L2 prefetch (kernel argument prefetch_tiles, 0 = off): every block pulls "its" whole page towards L2 that many
-// tiles ahead as ONE linear request of 73,728 contiguous bytes.  Each K sub-tile buffer is re-loaded as soon as the
-// MMAs that read it complete and is needed again one tile later, so the re-load's latency sits on the tile loop:
-// with few sequences per GPU (HBM far from saturated) turning an HBM miss into an L2 hit shortens the tile period
-// (8 sequences: 47.7 -> 45.3 us per launch at distance 1; distances 2 and 4 queue more requests in front of the
-// demand loads and lose again), while at batch 64, where HBM bandwidth is the co-limit, it changes nothing
-// (267 -> 268 us), so the host turns it on only for short work lists.
-constexpr int K_ROUNDS = (NSUB + N_QK - 1) / N_QK;   // 3: the issuers free sub-tiles {0-3}, {4-7}, {8} together
-enum { B_QFULL = 0, B_QEMPTY, B_KFULL, B_KEMPTY = B_KFULL + NSUB, B_VFULL = B_KEMPTY + K_ROUNDS, B_VEMPTY = B_VFULL + 4,
-       B_SFULL = B_VEMPTY + PAGES, B_SEMPTY, B_PFULL, B_PEMPTY, B_OFULL, B_SYNCA0, B_SYNCA1, B_SYNCB0, B_SYNCB1, B_COUNT };
+// L2 prefetch (kernel argument prefetch_tiles, 0 = off): every block pulls "its" page towards L2 that many tiles ahead, a quarter
+// (contiguous bytes) with every pair it loads.  Only for short work lists: one sequence of 131,072 tokens takes 237 us with it and
+// 240 without, 4 layers of 32 x 8191 tokens 375 and 365.
+enum { B_QFULL = 0, B_QEMPTY, B_KFULL, B_KEMPTY = B_KFULL + 4, B_VFULL = B_KEMPTY + 4, B_VEMPTY = B_VFULL + 4, B_RFULL = B_VEMPTY + 4,
+       B_REMPTY, B_SFULL, B_SEMPTY = B_SFULL + 2, B_PFULL = B_SEMPTY + 2, B_PEMPTY, B_OFULL, B_SYNCA0, B_SYNCA1, B_SYNCB0, B_SYNCB1, B_COUNT };
 static_assert(B_COUNT * 8 <= M_TMEM, "barriers overflow their area");
 
 
@@ -119,7 +107,7 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
 {
     extern __shared__ __align__(1024) unsigned char sm[];
     const uint32_t base = smem_u32(sm);
-    const uint32_t sQ = base + OFF_Q, sK = base + OFF_K, sV = base + OFF_V, sP = base + OFF_P;
+    const uint32_t sQ = base + OFF_Q, sK = base + OFF_K, sV = base + OFF_V, sRope = base + OFF_ROPE, sP = base + OFF_P;
     const uint32_t sBar = base + OFF_MISC + M_BAR;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + OFF_MISC + M_TMEM);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + M_ABORT);
@@ -146,30 +134,20 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
     }
 
     if (tid == 64) { prefetch_map(&map_q); prefetch_map(&map_sub); prefetch_map(&map_kv64); }
-    // one barrier per thread of warp 0 (31 of them): initialised in one step instead of 31 by a single thread
     if (warp == 0) {
         if (lane == 0) {
             *abort_flag = 0;
             need_flag[0] = 0;
             need_flag[1] = 0;
         }
-        if (lane < B_COUNT) {
-            const int i = int(lane);
-            const uint32_t count = i == B_QFULL ? 1u
-                                 : i == B_QEMPTY ? uint32_t(N_QK)
-                                 : i < B_KEMPTY ? 1u                                                          // KFULL
-                                 : i < B_VFULL ? uint32_t(min(N_QK, NSUB - N_QK * (i - B_KEMPTY)))           // KEMPTY rounds
-                                 : i < B_VEMPTY ? 1u                                                          // VFULL
-                                 : i < B_SFULL ? uint32_t(N_PV)                                               // VEMPTY
-                                 : i == B_SFULL ? uint32_t(N_QK)
-                                 : (i == B_PEMPTY || i == B_OFULL) ? uint32_t(N_PV)
-                                 : uint32_t(PAIR_SOFTMAX_WARPS);                    // SEMPTY, PFULL, SYNCA0/1, SYNCB0/1
+        for (int i = int(lane); i < B_COUNT; i += 32) {
+            const uint32_t count = i == B_QEMPTY || i == B_SFULL || i == B_SFULL + 1 ? uint32_t(N_QK)
+                                 : i == B_PEMPTY || i == B_OFULL ? uint32_t(N_PV)
+                                 : i < B_SEMPTY ? 1u : uint32_t(PAIR_SOFTMAX_WARPS);          // SEMPTY, PFULL, SYNCA0/1, SYNCB0/1
             mbar_init(bar(i), count);
         }
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        mbar_init_fence();
     }
-    static_assert(B_COUNT <= 32, "one barrier per lane of the initialising warp");
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n"
                      ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
@@ -216,7 +194,7 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
     // the score tile).  A segment with an odd page count repeats its last page in the second half:
     // finite data whose scores the softmax masks.
     auto page_of = [&](const uint32_t* tbl, const SegInfo& s, uint32_t j, uint32_t r) -> uint32_t {
-        if (tbl == tbl0 && j == 0) return page0[r];
+        if (tbl == tbl0 && j == 0) return r ? page0[1] : page0[0];
         const uint32_t i = min(PAGES * j + r, s.n_pages - 1);
         return tbl[i];
     };
@@ -225,7 +203,7 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
         // ===================== TMA producer for Q' and K =====================
         if (lane == 0) {
             const uint32_t leader_qfull = map_to_rank(bar(B_QFULL), 0);
-            const uint32_t leader_kfull = map_to_rank(bar(B_KFULL), 0);
+            const uint32_t leader_kfull = map_to_rank(bar(B_KFULL), 0), leader_rfull = map_to_rank(bar(B_RFULL), 0);
             uint32_t t = 0, nseg = 0;
             bool ok = true;
             for (uint32_t seg = seg_begin; seg < seg_end && ok; seg++) {
@@ -238,24 +216,25 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                 tma_load_3d_pair(sQ, &map_q, leader_qfull, 0, int(s.q_row * H + h0), 0);      // all 9 sub-tiles at once
                 for (uint32_t j = 0; j < s.n_tiles && ok; j++, t++) {
                     uint32_t page = page_of(tbl, s, j, rank);
+                    const uint32_t ahead = prefetch_tiles > 0 && j + prefetch_tiles < s.n_tiles ? page_of(tbl, s, j + prefetch_tiles, rank) : n_pages;
                     if (page >= n_pages) {
                         atomicOr(status, ST_BAD_PAGE);
                         page = 0;
                     }
-                    const int slot0 = int(page * kPage);
-                    // The score issuers release the sub-tiles in rounds ({0-3}, {4-7}, {8}); one wait per round
-                    // instead of one per sub-tile: a shared-memory round trip costs this thread ~300 cycles while
-                    // the MMAs stream their operands, and nine of them per tile made it the slowest stage.
+                    const int slot0 = int(page * kPage), layer = int(layer0 + s.layer);
 #pragma unroll 1
-                    for (int rd = 0; rd < K_ROUNDS && ok; rd++) {
-                        ok = mbar_wait<kSleep>(bar(B_KEMPTY + rd), (t & 1) ^ 1, abort_flag, status);
+                    for (uint32_t i = 0; i < 4; i++) {
+                        if (ahead < n_pages) bulk_prefetch_l2(page_ptr(s, ahead) + i * (PAGE_BYTES / 4), PAGE_BYTES / 4);
+                        ok = mbar_wait<kSleep>(bar(B_KEMPTY + i), (t & 1) ^ 1, abort_flag, status);
                         if (!ok) break;
-#pragma unroll 1
-                        for (int c = N_QK * rd; c < min(N_QK * (rd + 1), NSUB); c++) {
-                            if (rank == 0) mbar_expect_tx(bar(B_KFULL + c), 2 * SUB_BYTES);
-                            tma_load_3d_pair(sK + c * SUB_BYTES, &map_sub, leader_kfull + 8 * c, 64 * c, slot0, int(layer0 + s.layer));
-                        }
+                        if (rank == 0) mbar_expect_tx(bar(B_KFULL + i), 2 * PAIR_BYTES);
+                        tma_load_4d_pair(sK + i * PAIR_BYTES, &map_kv64, leader_kfull + 8 * i, 0, slot0, int(2 * i), layer);
                     }
+                    if (!ok) break;
+                    ok = mbar_wait<kSleep>(bar(B_REMPTY), (t & 1) ^ 1, abort_flag, status);
+                    if (!ok) break;
+                    if (rank == 0) mbar_expect_tx(bar(B_RFULL), 2 * SUB_BYTES);
+                    tma_load_3d_pair(sRope, &map_sub, leader_rfull, kRank, slot0, layer);
                 }
                 nseg++;
             }
@@ -270,30 +249,17 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                 const SegInfo s = seg_info(seg);
                 if (s.n_tiles == 0 || s.heads <= hpair) continue;
                 const uint32_t* tbl = seg_table(seg, s);
-                // tile 0 is demand-loaded right now; tiles 1 .. prefetch_tiles-1 have no earlier tile to ride on
-                for (uint32_t jj = 1; jj < min(prefetch_tiles, s.n_tiles); jj++) {
-                    const uint32_t pgid = page_of(tbl, s, jj, rank);
-                    if (pgid < n_pages) bulk_prefetch_l2(page_ptr(s, pgid), kPage * kRow * 2);
-                }
                 for (uint32_t j = 0; j < s.n_tiles && ok; j++, t++) {
-                    if (prefetch_tiles > 0 && j + prefetch_tiles < s.n_tiles) {
-                        const uint32_t pgid = page_of(tbl, s, j + prefetch_tiles, rank);
-                        if (pgid < n_pages) bulk_prefetch_l2(page_ptr(s, pgid), kPage * kRow * 2);
-                    }
 #pragma unroll 1
-                    for (uint32_t pg = 0; pg < uint32_t(PAGES) && ok; pg++) {     // both chunk issuers release a page together
-                        uint32_t page = page_of(tbl, s, j, pg);
+                    for (uint32_t v = 0; v < 4; v++) {           // page v / 2, chunk v % 2
+                        uint32_t page = page_of(tbl, s, j, v / 2);
                         if (page >= n_pages) page = 0;           // flagged by the K producer
-                        ok = mbar_wait<kSleep>(bar(B_VEMPTY + pg), (t & 1) ^ 1, abort_flag, status);
+                        ok = mbar_wait<kSleep>(bar(B_VEMPTY + v), (t & 1) ^ 1, abort_flag, status);
                         if (!ok) break;
-#pragma unroll 1
-                        for (uint32_t ch = 0; ch < 2; ch++) {
-                            const uint32_t v = 2 * pg + ch;
-                            if (rank == 0) mbar_expect_tx(bar(B_VFULL + v), 2 * VBUF_BYTES);
-                            // all 64 tokens of the page, this block's 128 dims of chunk ch = sub-tiles 4*ch + 2r, +1
-                            tma_load_4d_pair(sV + v * VBUF_BYTES, &map_kv64, leader_vfull + 8 * v, 0, int(page * kPage),
-                                             4 * int(ch) + 2 * int(rank), int(layer0 + s.layer));
-                        }
+                        if (rank == 0) mbar_expect_tx(bar(B_VFULL + v), 2 * PAIR_BYTES);
+                        // all 64 tokens of the page, this block's 128 dims of the chunk = sub-tiles 4 * chunk + 2r, +1
+                        tma_load_4d_pair(sV + v * PAIR_BYTES, &map_kv64, leader_vfull + 8 * v, 0, int(page * kPage),
+                                         int(4 * (v % 2) + 2 * rank), int(layer0 + s.layer));
                     }
                 }
             }
@@ -316,8 +282,7 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
             constexpr uint32_t HI = desc_hi(1024);
             const bool is_qk = warp <= N_QK;
             const uint32_t part = is_qk ? warp - 1 : warp - 1 - N_QK;
-            const uint32_t qk_a = desc_lo(sQ, 16), qk_b = desc_lo(sK, 16);
-            const uint32_t pv_a = desc_lo(sV, SUB_BYTES), pv_b = desc_lo(sP, 16);
+            const uint32_t qk_a = desc_lo(sQ, 16), pv_b = desc_lo(sP, 16);
             uint32_t t = 0, nseg = 0;
             bool ok = true;
             for (uint32_t seg = seg_begin; seg < seg_end && ok; seg++) {
@@ -326,44 +291,63 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                 if (is_qk) ok = mbar_wait<kSleepCluster>(bar(B_QFULL), nseg & 1, abort_flag, status);
                 for (uint32_t j = 0; j < s.n_tiles && ok; j++, t++) {
                     if (is_qk) {
-                        // sub-tiles part, part+4 (, part+8): partial scores into this warp's own 64 columns
-                        ok = mbar_wait<kSleepCluster>(bar(B_SEMPTY), (t & 1) ^ 1, abort_flag, status);
-                        if (!ok) break;
-                        const uint32_t d = tmem + COL_S + part * (TILE / 2);
-#pragma unroll 1
-                        for (uint32_t c = part; c < uint32_t(NSUB); c += N_QK) {
-                            ok = mbar_wait<kSleepCluster>(bar(B_KFULL + c), t & 1, abort_flag, status);
+                        // score issuer p: pairs p, p + 2, the last one also the rope sub-tile, into its own 64 columns
+                        ok = mbar_wait<kSleepCluster>(bar(B_SEMPTY + (t & 1)), ((t >> 1) & 1) ^ 1, abort_flag, status);
+                        const uint32_t d = tmem + COL_S + ((t & 1) * N_QK + part) * (TILE / 2);
+#pragma unroll
+                        for (uint32_t e = 0; e < 4 / N_QK; e++) {
+                            const uint32_t i = part + N_QK * e;
+                            ok = ok && mbar_wait<kSleep>(bar(B_KFULL + i), t & 1, abort_flag, status);
                             if (!ok) break;
                             tc_fence_after();
+                            const uint32_t b0 = desc_lo(sK + i * PAIR_BYTES, 16);
                             if (elect_one()) {
 #pragma unroll
-                                for (int k = 0; k < 4; k++)
-                                    tc_mma_pair(d, qk_a + ((c * SUB_BYTES + k * 32) >> 4), HI, qk_b + ((c * SUB_BYTES + k * 32) >> 4),
-                                                HI, IDESC_QK, (c == part && k == 0) ? 0u : 1u);
-                                tc_commit_pair(bar(B_KEMPTY + c / N_QK));
-                                if (c + N_QK >= uint32_t(NSUB)) {      // same thread as the MMAs it covers
-                                    tc_commit_pair(bar(B_SFULL));
-                                    if (j + 1 == s.n_tiles) tc_commit_pair(bar(B_QEMPTY));
-                                }
+                                for (int cc = 0; cc < 2; cc++)
+#pragma unroll
+                                    for (int k = 0; k < 4; k++)
+                                        tc_mma_pair(d, qk_a + (((2 * i + cc) * SUB_BYTES + k * 32) >> 4), HI, b0 + ((cc * SUB_BYTES + k * 32) >> 4),
+                                                    HI, IDESC_QK, (e == 0 && cc == 0 && k == 0) ? 0u : 1u);
+                                tc_commit_pair(bar(B_KEMPTY + i));
                             }
                             __syncwarp();
                         }
+                        if (!ok) break;
+                        const bool last = part == uint32_t(N_QK - 1);
+                        if (last) {
+                            ok = mbar_wait<kSleep>(bar(B_RFULL), t & 1, abort_flag, status);
+                            if (!ok) break;
+                            tc_fence_after();
+                        }
+                        const uint32_t br = desc_lo(sRope, 16);
+                        if (elect_one()) {
+                            if (last) {
+#pragma unroll
+                                for (int k = 0; k < 4; k++)
+                                    tc_mma_pair(d, qk_a + ((8 * SUB_BYTES + k * 32) >> 4), HI, br + ((k * 32) >> 4), HI, IDESC_QK, 1u);
+                                tc_commit_pair(bar(B_REMPTY));
+                            }
+                            tc_commit_pair(bar(B_SFULL + (t & 1)));
+                            if (j + 1 == s.n_tiles) tc_commit_pair(bar(B_QEMPTY));
+                        }
+                        __syncwarp();
                     } else {
                         // chunk `part` of O^T += V^T P^T over the tile's two pages
                         ok = mbar_wait<kSleepCluster>(bar(B_PFULL), t & 1, abort_flag, status);
 #pragma unroll 1
                         for (uint32_t pg = 0; pg < uint32_t(PAGES) && ok; pg++) {
                             const uint32_t v = 2 * pg + part;
-                            ok = mbar_wait<kSleepCluster>(bar(B_VFULL + v), t & 1, abort_flag, status);
+                            ok = mbar_wait<kSleep>(bar(B_VFULL + v), t & 1, abort_flag, status);
                             if (!ok) break;
                             tc_fence_after();
+                            const uint32_t a0 = desc_lo(sV + v * PAIR_BYTES, SUB_BYTES);
                             const uint32_t fresh = (j == 0 && pg == 0) ? 0u : 1u;
                             if (elect_one()) {
 #pragma unroll
                                 for (int k = 0; k < kPage / 16; k++)
-                                    tc_mma_pair(tmem + COL_O + part * (2 * HG), pv_a + ((v * VBUF_BYTES + k * 2048) >> 4), HI,
+                                    tc_mma_pair(tmem + COL_O + part * (2 * HG), a0 + ((k * 2048) >> 4), HI,
                                                 pv_b + ((pg * P_BYTES + k * 32) >> 4), HI, IDESC_PV, k == 0 ? fresh : 1u);
-                                tc_commit_pair(bar(B_VEMPTY + pg));
+                                tc_commit_pair(bar(B_VEMPTY + v));
                                 if (pg + 1 == uint32_t(PAGES)) {
                                     tc_commit_pair(bar(B_PEMPTY));
                                     if (j + 1 == s.n_tiles) tc_commit_pair(bar(B_OFULL));
@@ -381,7 +365,7 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
         // S of a pair MMA with 64 rows per block: head row r sits in TMEM lane r (tokens of the first
         // page) and lane 64+r (second page), 64 columns each.  Two warps share each lane quarter and
         // split its columns, so a thread owns (head, 32 tokens): token quarter tq = 2*page + group.
-        const uint32_t sw_id = warp - (2 + N_QK + N_PV);      // 0..7
+        const uint32_t sw_id = warp - FIRST_SOFTMAX_WARP;      // 0..7
         const uint32_t grp = sw_id / 4;                       // column group within the lane quarter
         const uint32_t q4 = warp % 4;
         const uint32_t lane_base = (q4 * 32u) << 16;
@@ -390,22 +374,21 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
         const uint32_t hl = 32 * (q4 % 2) + lane;             // head within this block's 64
         const uint32_t st_id = tid - (NUM_THREADS - SOFTMAX_THREADS);
         const uint32_t peer = rank ^ 1;
-        const uint32_t r_sempty = map_to_rank(bar(B_SEMPTY), 0);
+        const uint32_t r_sempty = map_to_rank(bar(B_SEMPTY), 0);          // and the second one 8 bytes on
         const uint32_t r_pfull = map_to_rank(bar(B_PFULL), 0);
-        const uint32_t r_synca[2] = {map_to_rank(bar(B_SYNCA0), peer), map_to_rank(bar(B_SYNCA1), peer)};
-        const uint32_t r_syncb[2] = {map_to_rank(bar(B_SYNCB0), peer), map_to_rank(bar(B_SYNCB1), peer)};
+        const uint32_t r_synca = map_to_rank(bar(B_SYNCA0), peer), r_syncb = map_to_rank(bar(B_SYNCB0), peer);     // likewise
         const uint32_t r_flag = map_to_rank(base + OFF_MISC + M_FLAG, peer);
         const uint32_t r_alpha = map_to_rank(base + OFF_MISC + M_ALPHA, peer);
         float m_used = -INFINITY, l_part = 0.0f;
-        uint32_t t = 0, nseg = 0, na[2] = {0, 0}, nb[2] = {0, 0};   // na / nb: uses of SYNCA[par] / SYNCB[par] so far
+        uint32_t t = 0, nseg = 0, na = 0, nb = 0;         // na / nb, bit par: phase of SYNCA[par] / SYNCB[par]
         bool fail = false;
         auto wait_w = [&](uint32_t b, uint32_t parity) {              // completion of tensor-core / TMA work
-            if (!fail) fail = !mbar_wait<kSleep>(b, parity, abort_flag, status);
-            fail = __any_sync(0xffffffffu, fail);
+            fail |= !mbar_wait<kSleep>(b, parity, abort_flag, status);
+            __syncwarp();
         };
         auto wait_x = [&](uint32_t b, uint32_t parity) {              // rounds that carry the twin's DSMEM writes
-            if (!fail) fail = !mbar_wait<kSleepCluster>(b, parity, abort_flag, status);
-            fail = __any_sync(0xffffffffu, fail);
+            fail |= !mbar_wait<kSleepCluster>(b, parity, abort_flag, status);
+            __syncwarp();
         };
         auto group_or = [&](bool pred) -> bool {              // barrier over this block's softmax threads + OR
             uint32_t r;
@@ -437,35 +420,23 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
             const int lim = seg_visible(s, h0 + hl, H);
             for (uint32_t j = 0; j < s.n_tiles; j++, t++) {
                 const uint32_t par = t & 1;
-                wait_w(bar(B_SFULL), t & 1);
+                wait_w(bar(B_SFULL + par), (t >> 1) & 1);
                 uint32_t sv[32];
-                if (!fail) {
-                    tc_fence_after();
-                    {
-                        uint32_t sw[32];
-                        tc_ld32(tmem + lane_base + COL_S + grp * 32, sv);
-                        tc_ld32(tmem + lane_base + COL_S + (TILE / 2) + grp * 32, sw);
-                        tc_wait_ld();
+                tc_fence_after();
+                {
+                    uint32_t sw[32];
+                    const uint32_t col = tmem + lane_base + COL_S + par * N_QK * (TILE / 2) + grp * 32;
+                    tc_ld32(col, sv);
+                    tc_ld32(col + TILE / 2, sw);
+                    tc_wait_ld();
 #pragma unroll
-                        for (int i = 0; i < 32; i++) sv[i] = __float_as_uint(__uint_as_float(sv[i]) + __uint_as_float(sw[i]));
-                    }
-#pragma unroll 1
-                    for (int p = 2; p < N_QK; p++) {
-                        uint32_t sw[32];
-                        tc_ld32(tmem + lane_base + COL_S + p * (TILE / 2) + grp * 32, sw);
-                        tc_wait_ld();
-#pragma unroll
-                        for (int i = 0; i < 32; i++) sv[i] = __float_as_uint(__uint_as_float(sv[i]) + __uint_as_float(sw[i]));
-                    }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) {                       // orders only TMEM reads: no memory release needed
-                        if (rank == 0) mbar_arrive(bar(B_SEMPTY));
-                        else mbar_arrive_cluster_relaxed(r_sempty);
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; i++) sv[i] = 0u;
+                    for (int i = 0; i < 32; i++) sv[i] = __float_as_uint(__uint_as_float(sv[i]) + __uint_as_float(sw[i]));
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {                       // orders only TMEM reads: no memory release needed
+                    if (rank == 0) mbar_arrive(bar(B_SEMPTY + par));
+                    else mbar_arrive_cluster_relaxed(r_sempty + 8 * par);
                 }
                 // Scores stay unscaled in registers: the scale rides in the FMA in front of each exponential, and
                 // the mask pass runs only on a segment's last, partly filled tile.
@@ -492,15 +463,15 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                 // does any head of the pair have to move its reference maximum on this tile?
                 const bool need = !first && (mx > m_used + RESCALE_THRESHOLD);
                 const bool warp_need = __any_sync(0xffffffffu, need);
-                if (lane == 0 && !fail && !first) {
+                if (lane == 0 && !first) {
                     if (warp_need) {
                         atomicOr(const_cast<uint32_t*>(&need_flag[par]), 1u);
                         asm volatile("red.relaxed.cluster.shared::cluster.or.b32 [%0], %1;\n" ::"r"(r_flag + 4 * par), "r"(1u) : "memory");
                         mbar_arrive_local_release_cluster(bar(B_SYNCA0 + par));
-                        mbar_arrive_cluster(r_synca[par]);
+                        mbar_arrive_cluster(r_synca + 8 * par);
                     } else {
                         mbar_arrive(bar(B_SYNCA0 + par));
-                        mbar_arrive_cluster_relaxed(r_synca[par]);
+                        mbar_arrive_cluster_relaxed(r_synca + 8 * par);
                     }
                 }
                 // a row that has seen no token yet (a segment that only later rows of its group reach): p = 0
@@ -518,8 +489,8 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                 }
                 bool slow = false;
                 if (!first) {
-                    wait_x(bar(B_SYNCA0 + par), na[par] & 1);
-                    na[par]++;
+                    wait_x(bar(B_SYNCA0 + par), (na >> par) & 1);
+                    na ^= 1u << par;
                     if (group_or(fail)) { stop = true; break; }
                     slow = need_flag[par] != 0;
                 }
@@ -539,10 +510,10 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                     __syncwarp();
                     if (lane == 0) {
                         mbar_arrive_local_release_cluster(bar(B_SYNCB0 + par));
-                        mbar_arrive_cluster(r_syncb[par]);
+                        mbar_arrive_cluster(r_syncb + 8 * par);
                     }
-                    wait_x(bar(B_SYNCB0 + par), nb[par] & 1);
-                    nb[par]++;
+                    wait_x(bar(B_SYNCB0 + par), (nb >> par) & 1);
+                    nb ^= 1u << par;
                     l_part *= alpha;
                     m_eff = m_used == -INFINITY ? 0.0f : m_used;
                     sum = 0.0f;
@@ -557,7 +528,6 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                 l_part += sum;
                 // PV of the previous tile must be complete: O is stable and P is free
                 wait_w(bar(B_PEMPTY), (t - 1) & 1);
-                if (fail) continue;            // carried to the next barrier
                 tc_fence_after();
                 if (slow) {
                     // O^T[this block's dims][128 heads] *= alpha[head]; each warp group takes one chunk
