@@ -177,7 +177,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constan
     } else {
         const uint32_t e = warp - FIRST_ROW_WARP, t = tid - FIRST_ROW_WARP * 32;
         T* out = second ? out1 : out0;
-        const uint32_t N = a.N[second], o = tn * BM + t % BM;
+        const uint32_t N = second ? a.N[1] : a.N[0], o = tn * BM + t % BM;       // (indexed, the arguments are copied to the stack)
         const uint32_t pieces = kbs * 8, p0 = kb0 * 8, n_pieces = a.K / 8;
         // this warp's rows: e, e + 8, .., or with few of them a share of one row
         const uint32_t part = e & (a.split - 1), my_rows = e < a.M * a.split ? (a.split > 1 ? 1 : (a.M - e + ROW_WARPS - 1) / ROW_WARPS) : 0;
