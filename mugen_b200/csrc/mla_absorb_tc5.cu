@@ -219,64 +219,77 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
                 mbar_arrive(acc_empty(b));
             }
         }
-    } else if (warp >= FIRST_APPEND) {
-        append(blockIdx.x * APPEND_WARPS + warp - FIRST_APPEND, a.blocks * APPEND_WARPS, app_inside, sm + off_append(NT) + (warp - FIRST_APPEND) * kAppendRowSmem);
     } else {
-        // ---- query rows: q_nope -> operand rows, q_rope -> behind the absorbed dims (by the unit that has d-tile 0)
+        // ---- query rows: q_nope -> operand rows, q_rope -> behind the absorbed dims (by the unit that has d-tile 0).  A block with several
+        // row tiles leaves the rope part to the append warps: it took the query warps 2,000 to 3,000 cycles per tile, and everything
+        // waited for the operand rows of the next one.  From the wait to the last output of 27 layers x 16 heads x 80 rows 51,500 ->
+        // 31,600 cycles; 16 sequences x 5 verify rows 322 -> 317 us, 64 x 8 985 -> 907, 4 layers of 128 heads x 100 sequences of 300 tokens 190 -> 172.
+        // With a single tile the rope part is not in the way, and the append warps may be busy for longer.
+        const uint32_t t = (tid - FIRST_QUERY * 32) % 128;
         Unit x = unit_of(u0);                      // the divisions not behind the wait
-        // Rows of many steps lie far apart and have not been touched for a pass over the cache: the first load of a tile took 5 us from the
-        // wait on, W_UK was there after 2 (16 sequences x 5 rows to verify, with the epilogue's wider stores 324.6 -> 320.2 us; 32
-        // sequences through three blocks of 128 heads 375 -> 372).  L2 is the point of coherence, so asking ahead of the wait is safe.  (Not with one tile of up to
-        // 16 rows, which the kernel before may just be writing: 27 blocks of 4 sequences 757 -> 761 us.)
-        if constexpr (NT > 16) {
-            for (uint32_t u = u0; u < u1; u++) {
-                const Unit y = unit_of(u);
-                const uint32_t ra = y.rt0 * NT, n = min(a.rows, y.rt1 * NT) - ra;
-                for (uint32_t i = tid - FIRST_QUERY * 32; i < 3 * n; i += 128) {
-                    const uint32_t r = ra + i / 3;
-                    const T* p = q + ((size_t(y.li) * a.rows + (a.att_row ? a.att_row[r] : r)) * a.H + y.h) * kQDim + (i % 3) * 64;
-                    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));
+        const bool several = u1 - u0 > 1 || x.rt1 - x.rt0 > 1;
+        if (warp >= FIRST_APPEND) {
+            append(blockIdx.x * APPEND_WARPS + warp - FIRST_APPEND, a.blocks * APPEND_WARPS, app_inside, sm + off_append(NT) + (warp - FIRST_APPEND) * kAppendRowSmem);
+        } else {
+            // Rows of many steps lie far apart and have not been touched for a pass over the cache: the first load of a tile took 5 us from the
+            // wait on, W_UK was there after 2 (16 sequences x 5 rows to verify, with the epilogue's wider stores 324.6 -> 320.2 us; 32
+            // sequences through three blocks of 128 heads 375 -> 372).  L2 is the point of coherence, so asking ahead of the wait is safe.  (Not with one tile of up to
+            // 16 rows, which the kernel before may just be writing: 27 blocks of 4 sequences 757 -> 761 us.)
+            if constexpr (NT > 16) {
+                for (uint32_t u = u0; u < u1; u++) {
+                    const Unit y = unit_of(u);
+                    const uint32_t ra = y.rt0 * NT, n = min(a.rows, y.rt1 * NT) - ra;
+                    for (uint32_t i = t; i < 3 * n; i += 128) {
+                        const uint32_t r = ra + i / 3;
+                        const T* p = q + ((size_t(y.li) * a.rows + (a.att_row ? a.att_row[r] : r)) * a.H + y.h) * kQDim + (i % 3) * 64;
+                        asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));
+                    }
+                }
+            }
+            grid_dependency_wait();
+            bool ok = true;
+            uint32_t n = 0;
+            for (uint32_t u = u0; u < u1; u++, x = unit_of(u)) {
+                const T* ql = q + size_t(x.li) * a.rows * a.H * kQDim;
+                for (uint32_t rt = x.rt0; rt < x.rt1; rt++, n++) {
+                    const uint32_t b = n & 1, r0 = rt * NT;
+                    ok = ok && mbar_wait(a_empty(b), ((n >> 1) & 1) ^ 1, abort_flag, status);
+                    unsigned char* dst = sm + OFF_A + b * a_bytes(NT);
+                    auto q_row = [&](uint32_t r) -> const T* { return ql + (size_t(a.att_row ? a.att_row[r] : r) * a.H + x.h) * kQDim; };
+                    uint4 v[NT / 8];                                          // 16 chunks of 16 bytes per row
+#pragma unroll
+                    for (int k = 0; k < NT / 8; k++) {
+                        const uint32_t c = t + 128 * k, rr = c / 16;
+                        v[k] = r0 + rr < a.rows ? reinterpret_cast<const uint4*>(q_row(r0 + rr))[c % 16] : make_uint4(0, 0, 0, 0);
+                    }
+#pragma unroll
+                    for (int k = 0; k < NT / 8; k++) {
+                        const uint32_t c = t + 128 * k, rr = c / 16, ch = c % 16;
+                        *reinterpret_cast<uint4*>(dst + (ch / 8) * (NT * 128) + rr * 128 + (((ch % 8) ^ (rr & 7)) << 4)) = v[k];
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                    mbar_arrive(a_full(b));
                 }
             }
         }
-        grid_dependency_wait();
-        const uint32_t t = tid - FIRST_QUERY * 32;
-        bool ok = true;
-        uint32_t n = 0;
-        for (uint32_t u = u0; u < u1; u++, x = unit_of(u)) {
-            const T* ql = q + size_t(x.li) * a.rows * a.H * kQDim;
-            for (uint32_t rt = x.rt0; rt < x.rt1; rt++, n++) {
-                const uint32_t b = n & 1, r0 = rt * NT;
-                ok = ok && mbar_wait(a_empty(b), ((n >> 1) & 1) ^ 1, abort_flag, status);
-                unsigned char* dst = sm + OFF_A + b * a_bytes(NT);
-                auto q_row = [&](uint32_t r) -> const T* { return ql + (size_t(a.att_row ? a.att_row[r] : r) * a.H + x.h) * kQDim; };
-                uint4 v[NT / 8];                                          // 16 chunks of 16 bytes per row
-#pragma unroll
-                for (int k = 0; k < NT / 8; k++) {
-                    const uint32_t c = t + 128 * k, rr = c / 16;
-                    v[k] = r0 + rr < a.rows ? reinterpret_cast<const uint4*>(q_row(r0 + rr))[c % 16] : make_uint4(0, 0, 0, 0);
-                }
-#pragma unroll
-                for (int k = 0; k < NT / 8; k++) {
-                    const uint32_t c = t + 128 * k, rr = c / 16, ch = c % 16;
-                    *reinterpret_cast<uint4*>(dst + (ch / 8) * (NT * 128) + rr * 128 + (((ch % 8) ^ (rr & 7)) << 4)) = v[k];
-                }
-                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                mbar_arrive(a_full(b));
+        if ((warp >= FIRST_APPEND) == several) {
+            for (uint32_t u = u0; u < u1; u++) {
+                x = unit_of(u);
                 if (x.d0 != 0) continue;
+                const T* ql = q + size_t(x.li) * a.rows * a.H * kQDim;
+                auto q_row = [&](uint32_t r) -> const T* { return ql + (size_t(a.att_row ? a.att_row[r] : r) * a.H + x.h) * kQDim; };
+                const uint32_t ra = x.rt0 * NT, n_rows = min(a.rows, x.rt1 * NT) - ra;
                 T* qa = q_abs + (size_t(x.li) * a.rows * a.H + x.h) * kRow + kRank;
                 if (a.cos_sin == nullptr) {
-                    for (uint32_t c = t; c < NT * 8; c += 128) {          // already rotated: 8 chunks per row
-                        const uint32_t r = r0 + c / 8;
-                        if (r < a.rows)
-                            reinterpret_cast<uint4*>(qa + size_t(r) * a.H * kRow)[c % 8] = reinterpret_cast<const uint4*>(q_row(r) + kNope)[c % 8];
+                    for (uint32_t c = t; c < n_rows * 8; c += 128) {      // already rotated: 8 chunks per row
+                        const uint32_t r = ra + c / 8;
+                        reinterpret_cast<uint4*>(qa + size_t(r) * a.H * kRow)[c % 8] = reinterpret_cast<const uint4*>(q_row(r) + kNope)[c % 8];
                     }
                 } else {
                     // q-side RoPE (reference: transformer.cpp:3882-3921, NeoX pairs (i, i+32), YaRN frequencies): the same
                     // table and the same separately rounded products as the k_rope rotation of the append; eight pairs at a time
-                    for (uint32_t c = t; c < NT * 4; c += 128) {
-                        const uint32_t r = r0 + c / 4, i = (c % 4) * 8;
-                        if (r >= a.rows) continue;
+                    for (uint32_t c = t; c < n_rows * 4; c += 128) {
+                        const uint32_t r = ra + c / 4, i = (c % 4) * 8;
                         const uint32_t pos = a.q_pos[r];
                         const uint4* src = reinterpret_cast<const uint4*>(q_row(r) + kNope + i);
                         const uint4 v0 = src[0], v1 = src[4];
