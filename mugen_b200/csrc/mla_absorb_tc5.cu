@@ -53,6 +53,10 @@ struct AbsorbArgs {
     const float* cos_sin;               // not null: rotate the last 64 dims of every head with the row's position
     const uint32_t *q_pos, *att_row;
     uint32_t cs_rows, app_layers;
+    // The kernel just ahead uploads this launch's metadata.  Nothing of it is read, and no kernel behind is let start, before the wait; W
+    // does not depend on it (16 heads x 27 layers, one sequence: 43.7 -> 40.6 us a step against a launch that starts when the upload
+    // is over; 128 heads x 8 layers, one sequence 80.3 -> 75.6).
+    uint32_t behind_upload;
 };
 
 template <typename T, int NT>
@@ -64,7 +68,7 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
     constexpr AbsorbRing RING{STAGES / ISSUERS};
     constexpr uint32_t TMEM_COLS = 8 * NT;                      // two sets of four d-tiles x NT columns
     extern __shared__ unsigned char absorb_tc5_smem[];
-    grid_launch_dependents();
+    if (!a.behind_upload) grid_launch_dependents();
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     // Apart from kv_a the append touches nothing that an earlier kernel of the stream still reads or writes: constant
     // tables, the step metadata (uploaded before the step's first kernel), and slots of this layer's pool, last read by
@@ -75,6 +79,11 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
     const uint32_t app_total = app.rows * a.app_layers, app_inside = min(app_total, a.blocks * APPEND_WARPS * APPEND_PER_WARP);
     auto append = [&](uint32_t i0, uint32_t step, uint32_t end, unsigned char* smem) {
         bool waited = !app.wait_first;
+        if (a.behind_upload) {
+            grid_dependency_wait();
+            grid_launch_dependents();
+            waited = true;
+        }
         for (uint32_t i = i0; i < end; i += step) {
             AppendRow<T> row;
             row.prepare(app, i / app.rows, i % app.rows, status);
@@ -235,6 +244,7 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
             // wait on, W_UK was there after 2 (16 sequences x 5 rows to verify, with the epilogue's wider stores 324.6 -> 320.2 us; 32
             // sequences through three blocks of 128 heads 375 -> 372).  L2 is the point of coherence, so asking ahead of the wait is safe.  (Not with one tile of up to
             // 16 rows, which the kernel before may just be writing: 27 blocks of 4 sequences 757 -> 761 us.)
+            if (a.behind_upload && a.att_row) grid_dependency_wait();
             if constexpr (NT > 16) {
                 for (uint32_t u = u0; u < u1; u++) {
                     const Unit y = unit_of(u);
@@ -247,6 +257,7 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
                 }
             }
             grid_dependency_wait();
+            if (a.behind_upload) grid_launch_dependents();
             bool ok = true;
             uint32_t n = 0;
             for (uint32_t u = u0; u < u1; u++, x = unit_of(u)) {
@@ -350,17 +361,17 @@ int absorb_tc5_configure()
 // w_map: host CUtensorMap over W_UK^T of all layers ([layers*H*512 d][128 i], box 64 i x 128 d, 128-byte swizzle).  q, q_abs
 // and (with kv_a != nullptr: the launch also appends) kv_a hold m.layers consecutive layers from layer0; layer_pool and
 // norm_w point at layer0's slices.  With rotate_q the last 64 dims of every query head are rotated with the row's
-// position (m.row_pos) before they are stored.
+// position (m.row_pos) before they are stored.  behind_upload: see AbsorbArgs; the launch is then not plain.
 int launch_absorb_tc5(int dtype, const void* q, const void* w_map, void* q_abs, uint32_t H, uint32_t layer0, const void* kv_a,
                       void* layer_pool, uint64_t pool_slots, const void* norm_w, const float* cos_sin, uint32_t cs_rows,
-                      float eps, const StepMeta& m, bool rotate_q, bool append_waits, uint32_t sm_count, uint32_t* status, const LaunchStream& st)
+                      float eps, const StepMeta& m, bool rotate_q, bool append_waits, bool behind_upload, uint32_t sm_count, uint32_t* status, const LaunchStream& st)
 {
     if (m.rows == 0) return 0;
     const CUtensorMap* map = static_cast<const CUtensorMap*>(w_map);
     AppendArgs app{};
     if (kv_a) app = AppendArgs{kv_a, layer_pool, pool_slots, norm_w, cos_sin, cs_rows, eps, m.app_pos, m.app_slot, m.app_rows, append_waits ? 1u : 0u};
     const uint32_t nt = m.rows <= 16 ? 16 : m.rows <= 32 ? 32 : 64, row_tiles = (m.rows + nt - 1) / nt, heads = m.layers * H;
-    AbsorbArgs a{m.rows, H, layer0, 1, 1, 0, 0, 0, rotate_q ? cos_sin : nullptr, m.row_pos, m.att_row, cs_rows, m.layers};
+    AbsorbArgs a{m.rows, H, layer0, 1, 1, 0, 0, 0, rotate_q ? cos_sin : nullptr, m.row_pos, m.att_row, cs_rows, m.layers, behind_upload ? 1u : 0u};
     // a head is cut while its parts still leave SMs idle: along d first (the weights are then still read once)
     while (a.d_parts < 4 && heads * a.d_parts * 2 <= sm_count) a.d_parts *= 2;
     a.r_parts = std::max(1u, std::min(row_tiles, sm_count / (heads * a.d_parts)));

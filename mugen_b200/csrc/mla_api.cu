@@ -570,8 +570,10 @@ int run_append(mla_ctx* c, uint32_t layer, const void* kv_a, const mla::StepMeta
 
 // absorb -> split-KV attention -> merge (+ W_UV, or export of the merged partial state) of the plan's layers from `layer` on
 // With fused_kv_a the absorb launch also appends the step's new rows (the caller then skips run_append).
+// own_upload: the caller has just uploaded p, and nobody else can have launched anything on st since; the absorb then starts before the
+// upload is over, and holds back the kernels behind it until it is.
 int run_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, float* exported, const Plan& p, cudaStream_t st,
-               const void* fused_kv_a = nullptr, bool kv_a_settled = false)
+               const void* fused_kv_a = nullptr, bool kv_a_settled = false, bool own_upload = false)
 {
     const mla::StepMeta& m = p.m;
     if (m.rows == 0) return MLA_OK;
@@ -579,7 +581,8 @@ int run_attend(mla_ctx* c, uint32_t layer, const void* q, void* out, float* expo
     const int dt = int(c->cfg.dtype);
     const int ae = mla::launch_absorb_tc5(dt, q, &c->w_uk_map, c->q_abs, H, layer, fused_kv_a, layer_pool(c, layer), c->pool_slots,
                                           layer_norm(c, layer), c->cos_sin, c->cs_rows, c->cfg.rms_norm_eps, m, c->q_rope_in_kernel,
-                                          !kv_a_settled, uint32_t(c->sm_count), c->status_dev, launch_stream(c, st));
+                                          !kv_a_settled, own_upload, uint32_t(c->sm_count), c->status_dev,
+                                          own_upload ? mla::LaunchStream(st) : launch_stream(c, st));
     if (ae != 0) return fail(c, MLA_ERR_CUDA, std::string("absorb launch: ") + cudaGetErrorString(cudaError_t(ae)));
     launched(c, st);
     int e;
@@ -1217,14 +1220,17 @@ int mla_step_layers(mla_ctx* c, uint32_t layer_begin, uint32_t n_layers, const v
         group = (n_layers + n_groups - 1) / n_groups;
         // both plans go up ahead of the first launch: an upload between two launches ends their overlap
         auto plan_of = [&](uint32_t n) -> Plan& { return n == group ? c->stack : c->stack_tail; };
+        bool own_upload = false;               // by this call, so that nothing stands between it and the first launch
         for (uint32_t n : {group, n_layers % group})
-            if (Plan& p = plan_of(n); n && (!p.ready || p.m.layers != n))
+            if (Plan& p = plan_of(n); n && (!p.ready || p.m.layers != n)) {
                 if (int e = build_plan(c, p, n == group ? kPlanStack : kPlanStackTail, c->step_seqs, c->rows, nullptr, nullptr, n, st)) return e;
+                own_upload = true;
+            }
         for (uint32_t i = 0; i < n_layers; i += group) {
             const uint32_t n = std::min(group, n_layers - i);
             Plan& p = plan_of(n);
             if (int e = run_attend(c, layer_begin + i, static_cast<const char*>(q) + i * q_b, static_cast<char*>(out) + i * o_b, nullptr, p, st,
-                                   static_cast<const char*>(kv_a) + i * kv_b, i > 0))
+                                   static_cast<const char*>(kv_a) + i * kv_b, i > 0, own_upload && i == 0))
                 return e;
         }
         return MLA_OK;

@@ -96,9 +96,11 @@ int merge_mma_configure();
 // new rows (launch_append's arguments) in extra blocks.  rotate_q: q arrives before its RoPE; the kernel rotates
 // the last 64 dims of every head with the row's position (m.row_pos) and the cos/sin table.  append_waits: kv_a may
 // have been written by the kernel launched just before this one (the append blocks then wait for it before reading).
+// behind_upload: that kernel is the upload (launch_fetch) of m, and st is not plain: the weights are loaded while it runs, everything else,
+// and the start of the kernels behind, waits for it.
 int launch_absorb_tc5(int dtype, const void* q, const void* w_map, void* q_abs, uint32_t H, uint32_t layer0, const void* kv_a,
                       void* layer_pool, uint64_t pool_slots, const void* norm_w, const float* cos_sin, uint32_t cs_rows,
-                      float eps, const StepMeta& m, bool rotate_q, bool append_waits, uint32_t sm_count, uint32_t* status, const LaunchStream& st);
+                      float eps, const StepMeta& m, bool rotate_q, bool append_waits, bool behind_upload, uint32_t sm_count, uint32_t* status, const LaunchStream& st);
 int absorb_tc5_configure();
 
 // The same merge + projection on tcgen05; w_map: host CUtensorMap over W_UV of

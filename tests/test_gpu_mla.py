@@ -1168,6 +1168,37 @@ def test_the_first_call_behind_an_upload_waits_for_it_whatever_went_elsewhere(to
     ctx.close()
 
 
+@pytest.mark.parametrize("H,dt", [(16, synth.DT_F16), (128, synth.DT_BF16)])
+def test_groups_of_layers_start_early_behind_their_own_upload(torch, H, dt):
+    """Steps over other sequences in turn, enqueued behind a busy stream without a wait in between: the first kernel of a group starts
+    before its upload has stored anything, and neither it nor a kernel behind it may use what the step before had left there."""
+    ctx, seqs, lens, kv, q = _step_ctx(torch, H=H, dt=dt, lens=(100, 700, 64, 1, 333, 129))
+    L, B = kv.shape[:2]
+    picks = [[0, 1, 2], [5, 4], [3], [1, 5, 0, 2], [2, 0]]
+
+    def step(p, out):
+        rows = torch.tensor(p, device="cuda")
+        k, x = kv[:, rows].contiguous(), q[:, rows].contiguous()
+        ctx.step_begin([seqs[i] for i in p])
+        ctx.step_layers(0, L, k, x, out)
+        ctx.step_end()
+        ctx.rollback([seqs[i] for i in p], [lens[i] for i in p])
+        return k, x
+
+    outs = [[torch.zeros((L, len(p), H, 128), dtype=torch.int16, device="cuda") for p in picks] for _ in range(3)]
+    for p, o in zip(picks, outs[0]):
+        step(p, o)
+        torch.cuda.synchronize()
+    torch.cuda._sleep(20_000_000)              # about 10 ms
+    keep = [step(p, o) for r in outs[1:] for p, o in zip(picks, r)]
+    torch.cuda.synchronize()
+    assert ctx.status() == 0 and len(keep) == 2 * len(picks)
+    for r in outs[1:]:
+        for want, got in zip(outs[0], r):
+            assert np.array_equal(_host(got), _host(want))
+    ctx.close()
+
+
 @pytest.mark.parametrize("how", ["layers", "calls"])
 def test_the_calls_of_an_open_step_can_be_captured(torch, how):
     """step_begin uploads; the calls behind it are launches alone, also inside a stream capture.  The graph is replayed over other
