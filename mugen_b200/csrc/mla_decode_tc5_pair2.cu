@@ -40,12 +40,12 @@ using namespace tc5;
 
 constexpr int PAGES = 2;                            // pages per super-tile
 constexpr int TILE = PAGES * kPage;                 // 128 tokens
-constexpr int HG = 64;                              // heads per block (128 per pair)
+constexpr int ROWS = 64;                            // rows of a block's operand tiles: tokens of a page, heads
 constexpr int NSUB = kRow / 64;                     // 9
 constexpr int SUB_BYTES = kPage * 128;              // 8,192: [64 tokens or heads][64 values]
 constexpr int Q_BYTES = NSUB * SUB_BYTES;           // 73,728
 constexpr int PAIR_BYTES = 2 * SUB_BYTES;           // 16,384: sub-tiles 2i, 2i+1 of a page
-constexpr int P_BYTES = HG * 128;                   // 8,192 per page
+constexpr int P_BYTES = ROWS * 128;                 // 8,192 per page
 constexpr int PAGE_BYTES = kPage * kRow * 2;
 constexpr int OFF_Q = 0;
 constexpr int OFF_K = OFF_Q + Q_BYTES;
@@ -97,7 +97,10 @@ __device__ __forceinline__ SegInfo load_seg(const StepMeta& m, uint32_t seg) {
     return s;
 }
 
-template <typename T>
+// HG: heads per block, 64 or 48.  With up to 96 head rows (launch_decode_tc5_pair128) P and O^T have 96 columns instead of 128, which is a
+// quarter less for the value MMAs and the states: 80 heads, 4 layers of 32 x 8191 tokens 337 -> 327 us, 64 x 16383 1,290 -> 1,254; 16 heads x 16
+// sequences x 5 verify rows 316 -> 309, x 6 331 -> 321; 96 heads 343 -> 335, and no call slower by more than runs differ.
+template <typename T, int HG>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __grid_constant__ CUtensorMap map_kv64,
                           const __grid_constant__ CUtensorMap map_q, const unsigned char* __restrict__ pool,
@@ -120,8 +123,8 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const uint32_t rank = cluster_rank();                 // 0 = pair leader (issues the MMAs)
     const uint32_t worker = blockIdx.x / 2;
-    const uint32_t hpair = blockIdx.y * (2 * HG);        // first head of the pair's 128
-    const uint32_t h0 = hpair + rank * HG;               // first head of this block's 64
+    const uint32_t hpair = blockIdx.y * (2 * HG);        // first head of the pair's 128 (96)
+    const uint32_t h0 = hpair + rank * HG;               // first head of this block's 64 (48)
     const uint32_t seg_begin = m.cta_seg_begin[worker], seg_end = m.cta_seg_begin[worker + 1];
 
     // The swizzled operand tiles need 1 KB alignment and the plan leaves no room to round up.
@@ -417,7 +420,8 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
             }
             m_used = -INFINITY;
             l_part = 0.0f;
-            const int lim = seg_visible(s, h0 + hl, H);
+            const bool mine = HG == ROWS || hl < uint32_t(HG);          // with 48 heads the last rows of the score tile are the twin's
+            const int lim = mine ? seg_visible(s, h0 + hl, H) : 0;
             for (uint32_t j = 0; j < s.n_tiles; j++, t++) {
                 const uint32_t par = t & 1;
                 wait_w(bar(B_SFULL + par), (t >> 1) & 1);
@@ -456,9 +460,9 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                 // of a pair walk the same segments, so they skip the same rounds.
                 const bool first = j == 0;
                 if (first) {
-                    half_max[tq * HG + hl] = mx;
+                    half_max[tq * ROWS + hl] = mx;
                     if (group_or(fail)) { stop = true; break; }
-                    m_used = fmaxf(fmaxf(half_max[hl], half_max[HG + hl]), fmaxf(half_max[2 * HG + hl], half_max[3 * HG + hl]));
+                    m_used = fmaxf(fmaxf(half_max[hl], half_max[ROWS + hl]), fmaxf(half_max[2 * ROWS + hl], half_max[3 * ROWS + hl]));
                 }
                 // does any head of the pair have to move its reference maximum on this tile?
                 const bool need = !first && (mx > m_used + RESCALE_THRESHOLD);
@@ -498,11 +502,11 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                     // exchange the token quarters' maxima inside the block, decide per head, publish the
                     // scale factors to both blocks, and redo the exponentials
                     float alpha = 1.0f;
-                    half_max[tq * HG + hl] = mx;
+                    half_max[tq * ROWS + hl] = mx;
                     group_or(false);
-                    const float mrow = fmaxf(fmaxf(half_max[hl], half_max[HG + hl]), fmaxf(half_max[2 * HG + hl], half_max[3 * HG + hl]));
+                    const float mrow = fmaxf(fmaxf(half_max[hl], half_max[ROWS + hl]), fmaxf(half_max[2 * ROWS + hl], half_max[3 * ROWS + hl]));
                     if (mrow > m_used + RESCALE_THRESHOLD) { alpha = fast_ex2(m_used - mrow); m_used = mrow; }
-                    if (tq == 0) {
+                    if (tq == 0 && mine) {
                         alpha_all[par * 128 + rank * HG + hl] = alpha;
                         asm volatile("st.relaxed.cluster.shared::cluster.f32 [%0], %1;\n"
                                      ::"r"(r_alpha + 4 * (par * 128 + rank * HG + hl)), "f"(alpha) : "memory");
@@ -532,9 +536,9 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                 if (slow) {
                     // O^T[this block's dims][128 heads] *= alpha[head]; each warp group takes one chunk
 #pragma unroll 1
-                    for (int c = 0; c < 4; c++) {
+                    for (int c = 0; c < 2 * HG / 32; c++) {
                         uint32_t o[32];
-                        const uint32_t col = COL_O + grp * 128 + c * 32;
+                        const uint32_t col = COL_O + grp * (2 * HG) + c * 32;
                         tc_ld32(tmem + lane_base + col, o);
                         tc_wait_ld();
                         const float* al = alpha_all + par * 128 + c * 32;
@@ -568,13 +572,13 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
             // ---- epilogue: O^T (this block's 256 dims x 128 heads) -> acc[head][dim]; (m, l) of own heads
             wait_w(bar(B_OFULL), nseg & 1);
             group_or(false);                   // the maxima scratch is free: its bytes now carry the partial sums
-            if (tq != 0) l_other[(tq - 1) * HG + hl] = l_part;
+            if (tq != 0) l_other[(tq - 1) * ROWS + hl] = l_part;
             if (group_or(fail)) { stop = true; break; }
             tc_fence_after();
 #pragma unroll 1
-            for (int c = 0; c < 4; c++) {                      // warp group `grp` owns chunk `grp`
+            for (int c = 0; c < 2 * HG / 32; c++) {                      // warp group `grp` owns chunk `grp`
                 uint32_t o[32];
-                tc_ld32(tmem + lane_base + COL_O + grp * 128 + c * 32, o);
+                tc_ld32(tmem + lane_base + COL_O + grp * (2 * HG) + c * 32, o);
                 tc_wait_ld();
                 const uint32_t dim = grp * 256 + rank * 128 + q4 * 32 + lane;
                 const uint32_t hb = hpair + c * 32;
@@ -583,10 +587,10 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                     if (hb + i < s.heads) recs[(size_t(seg) * m.rec_stride + hb + i) * kPart + 2 + dim] = __uint_as_float(o[i]);
                 }
             }
-            if (tq == 0 && h0 + hl < s.heads) {
+            if (tq == 0 && mine && h0 + hl < s.heads) {
                 float* rc = recs + (size_t(seg) * m.rec_stride + h0 + hl) * kPart;
                 rc[0] = m_used;
-                rc[1] = l_part + l_other[hl] + l_other[HG + hl] + l_other[2 * HG + hl];
+                rc[1] = l_part + l_other[hl] + l_other[ROWS + hl] + l_other[2 * ROWS + hl];
             }
             tc_fence_before();
             group_or(false);                   // the scratch is reused by the next segment
@@ -608,17 +612,16 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
 
 int decode_tc5_pair128_configure()
 {
-    cudaError_t e = cudaFuncSetAttribute(decode_tc5_pair128_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         SMEM_BYTES);
-    if (e != cudaSuccess) return int(e);
-    e = cudaFuncSetAttribute(decode_tc5_pair128_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             SMEM_BYTES);
-    if (e != cudaSuccess) return int(e);
-    // every kernel of a layer-step asks for the same (maximal) shared-memory carve-out, so the SMs are not
-    // re-partitioned between consecutive launches
-    e = cudaFuncSetAttribute(decode_tc5_pair128_kernel<__half>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return int(e);
-    e = cudaFuncSetAttribute(decode_tc5_pair128_kernel<__nv_bfloat16>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    auto set = [](auto kernel) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        // every kernel of a layer-step asks for the same (maximal) shared-memory carve-out, so the SMs are not
+        // re-partitioned between consecutive launches
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    };
+    cudaError_t e = set(decode_tc5_pair128_kernel<__half, 64>);
+    if (e == cudaSuccess) e = set(decode_tc5_pair128_kernel<__half, 48>);
+    if (e == cudaSuccess) e = set(decode_tc5_pair128_kernel<__nv_bfloat16, 64>);
+    if (e == cudaSuccess) e = set(decode_tc5_pair128_kernel<__nv_bfloat16, 48>);
     return int(e);
 }
 
@@ -631,14 +634,15 @@ int launch_decode_tc5_pair128(int dtype, const void* tmaps, const void* pool, ui
     if (m.ctas == 0) return 0;
     const CUtensorMap* maps = static_cast<const CUtensorMap*>(tmaps);
     const float scale_log2 = 1.4426950408889634f / sqrtf(float(kQDim));
-    dim3 grid(2 * m.ctas, (m.rec_stride + 2 * HG - 1) / (2 * HG));          // clusters of 2 along x
-    if (dtype == 0)
-        return int(launch_pdl(decode_tc5_pair128_kernel<__half>, grid, dim3(NUM_THREADS), SMEM_BYTES, st, maps[kMapPoolSub], maps[kMapPoolV], maps[kMapQueries],
+    const bool narrow = m.rec_stride <= 96;
+    dim3 grid(2 * m.ctas, narrow ? 1 : (m.rec_stride + 127) / 128);          // clusters of 2 along x
+    auto go = [&](auto kernel) {
+        return int(launch_pdl(kernel, grid, dim3(NUM_THREADS), SMEM_BYTES, st, maps[kMapPoolSub], maps[kMapPoolV], maps[kMapQueries],
                               static_cast<const unsigned char*>(pool), layer0, n_pages, m, recs, H, scale_log2, prefetch_tiles,
                               static_cast<const unsigned char*>(next_weights), next_weights_bytes, status));
-    return int(launch_pdl(decode_tc5_pair128_kernel<__nv_bfloat16>, grid, dim3(NUM_THREADS), SMEM_BYTES, st, maps[kMapPoolSub], maps[kMapPoolV],
-                          maps[kMapQueries], static_cast<const unsigned char*>(pool), layer0, n_pages, m, recs, H, scale_log2, prefetch_tiles,
-                              static_cast<const unsigned char*>(next_weights), next_weights_bytes, status));
+    };
+    if (dtype == 0) return narrow ? go(decode_tc5_pair128_kernel<__half, 48>) : go(decode_tc5_pair128_kernel<__half, 64>);
+    return narrow ? go(decode_tc5_pair128_kernel<__nv_bfloat16, 48>) : go(decode_tc5_pair128_kernel<__nv_bfloat16, 64>);
 }
 
 }  // namespace mla

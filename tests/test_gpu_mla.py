@@ -830,9 +830,9 @@ def test_rows_of_one_sequence_share_a_stream(torch, oracle, H, dt, spec):
 
 
 @pytest.mark.parametrize("H,dt", [(16, synth.DT_BF16), (17, synth.DT_F16), (32, synth.DT_BF16), (33, synth.DT_F16), (48, synth.DT_BF16),
-                                  (49, synth.DT_F16), (64, synth.DT_BF16)])
-def test_transposed_attention_at_the_edges_of_its_widths(torch, oracle, H, dt):
-    """Both sides of every width of the transposed kernel: rows of one token, a full page, one token more, and long ones whose scores rise
+                                  (49, synth.DT_F16), (64, synth.DT_BF16), (65, synth.DT_F16), (96, synth.DT_BF16), (97, synth.DT_BF16)])
+def test_attention_at_the_edges_of_its_widths(torch, oracle, H, dt):
+    """Both sides of every width of the transposed kernel and of the SM-pair kernel: rows of one token, a full page, one token more, and long ones whose scores rise
     from page to page, so that references move on later pages; 320 rows, so that a block walks several segments and its rings of
     pages wrap many times.  Bounds as everywhere here."""
     lens = [1, 64, 65, 1100]
@@ -847,7 +847,7 @@ def test_transposed_attention_at_the_edges_of_its_widths(torch, oracle, H, dt):
     out = torch.zeros((len(lens) * times, H, 128), dtype=torch.int16, device="cuda")
     ctx.attend_rows(0, seqs * times, lens * times, _dev(torch, np.tile(case.q, (times, 1, 1))), out)
     got = _host(out)
-    assert ctx.status() == 0 and ctx.kernel_name() == ("tcgen05-t16" if H <= 16 else "tcgen05")
+    assert ctx.status() == 0 and ctx.kernel_name() == ("tcgen05-t16" if H <= 16 else "tcgen05" if H <= 64 else "tcgen05-pair128")
     for r in range(len(lens) * times):
         check_close(got[r], want[r % len(lens)], dt, f"row {r}")
     again = torch.zeros_like(out)
