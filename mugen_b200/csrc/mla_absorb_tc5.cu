@@ -30,8 +30,8 @@ namespace {
 using namespace tc5;
 
 constexpr int PIECE = 128 * 128;                // 16,384: [128 d][64 i]
-// A tcgen05.mma costs its issuing warp about a hundred cycles whatever its size and a head takes 32 of them per row tile: an
-// issuer per d-tile (with the merge's issuers: 8 layers x 128 heads x 8 sequences, layer by layer, 514.6 -> 508.4 us).
+// An issuer per d-tile: one warp could issue a head's 32 MMAs as fast as the tensor core takes them, but its waits for eight pieces of W
+// stand one behind the other (with the merge's issuers: 8 layers x 128 heads x 8 sequences, layer by layer, 514.6 -> 508.4 us).
 constexpr int ISSUERS = 4, FIRST_EPI = 1 + ISSUERS, FIRST_QUERY = FIRST_EPI + 4;
 constexpr int APPEND_WARPS = 4, FIRST_APPEND = FIRST_QUERY + 4;
 constexpr int NUM_WARPS = FIRST_APPEND + APPEND_WARPS, NUM_THREADS = 32 * NUM_WARPS;   // W producer, MMA issuers, 4 epilogue, 4 query, 4 append warps

@@ -38,8 +38,8 @@ constexpr int OFF_MISC = OFF_A + 2 * NSUB * 32 * 128;
 constexpr int MISC_BYTES = 256;
 constexpr int SMEM_BYTES = OFF_MISC + MISC_BYTES + 1024;   // + slack to round the base up to 1 KB
 constexpr int RED_WARPS = 16;
-// A tcgen05.mma costs its issuing warp about a hundred cycles whatever its size, and a tile takes 32 of them.  With
-// few rows that is longer than the tile's loads: four issuers take two sub-tiles each into accumulators of their own, which the
+// A tile takes 32 MMAs of 40 cycles (their 128 weight rows from shared memory), whoever issues them; what an issuer adds is its waits
+// and its code, which comes in cold.  With few rows four issuers take two sub-tiles each into accumulators of their own, which the
 // epilogue adds in a fixed order (27 blocks of 16 heads x 4 rows: 996 -> 970 us with the absorb's issuers).  With more than 8
 // rows (G = 1) the reduction takes longer and needs the registers: two issuers there (3 layers x 128 heads x 128 sequences of 64
 // tokens: one 218 us, two 205, four 244 with 160 bytes of spills; 2 layers x 128 heads x 128 verify rows: 305, 297, 324).
