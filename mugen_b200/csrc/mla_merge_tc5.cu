@@ -75,7 +75,8 @@ __device__ __forceinline__ void reduce_row(const MergeArgs& a, const RowParts& r
     const Index stride = Index(a.rec_stride) * kPart;
     const float* rec0 = a.recs + size_t(rp.rec_off + h) * kPart;
     if (DL == 16 && rp.end - rp.begin == 1) {
-        // One part, as most rows of a large step have: no weights, nothing to exchange, the sums are those of the path below.  Only where a
+        // One part, as most rows of a large step have: nothing to exchange, and the bits of the path below for every state (an empty part
+        // adds nothing, whatever its sums hold; a maximum of infinity makes NaN).  Only where a
         // block has many rows (a warp per row): 27 layers of 64 sequences x 8 verify rows of 16 heads 1,070 -> 998 us, 4 layers of 128 heads x
         // 100 sequences of 300 tokens 206 -> 190.  With fewer rows per block 8 x 128 heads by calls take 0.7 % longer.
         const float* rec = rec0 + size_t(rp.begin) * stride;
@@ -87,9 +88,10 @@ __device__ __forceinline__ void reduce_row(const MergeArgs& a, const RowParts& r
             acc[2 * k] = f.x;
             acc[2 * k + 1] = f.y;
         }
-        const float one = ml.x != -INFINITY && ml.y > 0.0f ? 1.0f / ml.y : 0.0f;
+        const bool live = ml.x > -INFINITY;                    // not so for NaN either
+        const float w = 1.0f + (ml.x - ml.x), l = w * ml.y, inv = l > 0.0f ? 1.0f / l : 0.0f;
 #pragma unroll
-        for (int k = 0; k < DL; k++) acc[k] *= one;
+        for (int k = 0; k < DL; k++) acc[k] = live ? fmaf(w, acc[k], 0.0f) * inv : 0.0f;
         return;
     }
     for (uint32_t c0 = rp.begin; c0 < rp.end; c0 += 32) {

@@ -998,6 +998,40 @@ def test_merge_of_partials_beyond_4g_floats(torch):
     ctx.close()
 
 
+@pytest.mark.parametrize("rows", [2, 8, 12])
+def test_merge_of_one_part_is_the_merge_of_parts(torch, rows):
+    """A row with one part takes a path of its own where a block has many rows (12 rows of 128 heads): it must give the bits of the
+    general one, here the same part beside one that is empty, also for states that finite scores do not leave.  An empty part
+    (m = -inf) adds nothing, whatever lies behind it."""
+    from mugen_b200.mla import MlaContext
+    H = 128
+    ctx = MlaContext(n_layers=1, n_heads=H, dtype=synth.DT_F16, n_pages=2, max_seqs=1, max_seq_len=64, **YARN)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(2)
+    w_uv = (torch.randn(H, 128, 512, device="cuda", generator=gen) * 0.05).half()
+    bits = w_uv.view(torch.int16).cpu().numpy().view(np.uint16)
+    ctx.set_layer_weights(0, bits, bits, synth.W_F16, np.full(512, 0x3C00, np.uint16))
+    inf, nan = float("inf"), float("nan")
+    p = torch.randn((1, rows, H, 514), device="cuda", generator=gen)
+    p[..., 1] = p[..., 1].abs() + 0.5
+    empty = [(0, 0), (1, 3), (rows - 1, 127)]
+    for (r, h), acc in zip(empty, (nan, inf, -inf)):
+        p[0, r, h, 0], p[0, r, h, 1], p[0, r, h, 2:] = -inf, 0.0, acc
+    for h, (m, l) in zip((10, 11, 12, 13), ((inf, 1.0), (nan, 1.0), (0.5, 0.0), (0.5, nan))):
+        p[0, 1, h, 0], p[0, 1, h, 1] = m, l
+    beside = torch.zeros_like(p)
+    beside[..., 0] = -inf
+    one, two = (torch.full((rows, H, 128), 7.0, device="cuda", dtype=torch.float16) for _ in range(2))
+    ctx.merge_partials(0, 1, rows, p, one)
+    ctx.merge_partials(0, 2, rows, torch.cat([p, beside]), two)
+    assert ctx.status() == 0
+    for r, h in empty:
+        assert not one[r, h].any(), f"empty part of row {r}, head {h}"
+    assert torch.equal(one.isnan(), two.isnan())
+    assert torch.equal(one.nan_to_num(), two.nan_to_num())
+    ctx.close()
+
+
 def test_bounded_waits_do_not_run_while_an_earlier_kernel_does(torch, oracle):
     """A kernel ahead of the absorb and the merge that lets them start early and then runs for longer than the limit of their
     barrier waits (about two seconds): the limits must start when it ends, and the results must stand."""
