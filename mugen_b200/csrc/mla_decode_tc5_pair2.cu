@@ -504,6 +504,10 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                     float alpha = 1.0f;
                     half_max[tq * ROWS + hl] = mx;
                     group_or(false);
+                    // Everyone here has read the flag, and the twin's writes of this round have landed.  It is cleared ahead of this thread's
+                    // arrival below: whoever next raises it, two tiles from now, the twin too, has waited for that arrival first.  (The
+                    // arrival for P does not order it: on a segment's last tile the twin may pass a first tile, which has no round, and be there.)
+                    if (st_id == 0) need_flag[par] = 0;
                     const float mrow = fmaxf(fmaxf(half_max[hl], half_max[ROWS + hl]), fmaxf(half_max[2 * ROWS + hl], half_max[3 * ROWS + hl]));
                     if (mrow > m_used + RESCALE_THRESHOLD) { alpha = fast_ex2(m_used - mrow); m_used = mrow; }
                     if (tq == 0 && mine) {
@@ -564,9 +568,6 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
                     if (rank == 0) mbar_arrive(bar(B_PFULL));
                     else mbar_arrive_remote(r_pfull);
                 }
-                // the flag of this parity is next written two tiles from now: clear it once every
-                // thread of the block has read it (they all passed the barrier of the slow path)
-                if (st_id == 0 && slow) need_flag[par] = 0;
             }
             if (stop) break;
             // ---- epilogue: O^T (this block's 256 dims x 128 heads) -> acc[head][dim]; (m, l) of own heads

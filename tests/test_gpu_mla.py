@@ -856,6 +856,39 @@ def test_attention_at_the_edges_of_its_widths(torch, oracle, H, dt):
     ctx.close()
 
 
+@pytest.mark.parametrize("H,dt", [(128, synth.DT_F16), (96, synth.DT_BF16)])
+def test_references_move_on_the_last_tile_of_every_segment(torch, oracle, H, dt):
+    """Segments of two and three tiles of the SM-pair kernel, several per pair, whose scores rise by more than 2^8 from tile to tile: the request to
+    move a reference comes on a segment's last tile, and again on the second one of the next segment, with one flag for both and no
+    round between the blocks on the first tile in between."""
+    lens, times = [256, 384, 130, 257], 80
+    case = synth.make_layer_case(9300 + H, H, lens, dt, q_scale=3.0)
+    for i, n in enumerate(lens):
+        steps = np.asarray([0.05, 1.0, 2.2], np.float32)[np.arange(n) // 128][:, None]
+        case.caches[i] = synth.to_bits(synth.from_bits(case.caches[i], dt) * steps, dt)
+    w_uk = synth.from_bits(case.w_uk, dt).reshape(H, 128, 512)
+    for i, n in enumerate(lens):
+        q, c = synth.from_bits(case.q[i], dt), synth.from_bits(case.caches[i], dt)
+        s = (np.einsum("hi,hid,td->ht", q[:, :128], w_uk, c[:, :512], optimize=True) + q[:, 128:] @ c[:, 512:].T) / np.sqrt(192) * np.log2(np.e)
+        tops = np.stack([s[:, t:t + 128].max(1) for t in range(0, n, 128)])
+        assert i > 1 or (np.diff(tops, axis=0).max(1) > 9).all()             # some head moves on every tile but the first
+    ctx = make_ctx(case, capi.KERNEL_AUTO, shuffle=5, max_rows=len(lens) * times)
+    seqs = fill(torch, ctx, case)
+    want = [oracle_out(oracle, case, b) for b in range(len(lens))]
+    q = _dev(torch, np.tile(case.q, (times, 1, 1)))
+    first = None
+    for _ in range(4):
+        out = torch.zeros((len(lens) * times, H, 128), dtype=torch.int16, device="cuda")
+        ctx.attend_rows(0, seqs * times, lens * times, q, out)
+        got = _host(out)
+        assert ctx.status() == 0 and ctx.kernel_name() == "tcgen05-pair128"
+        assert first is None or np.array_equal(got, first)
+        first = got
+    for r in range(len(lens) * times):
+        check_close(first[r], want[r % len(lens)], dt, f"row {r}")
+    ctx.close()
+
+
 @pytest.mark.parametrize("H,dt,lens", [
     (5, synth.DT_F16, [6000]),                             # one row in 94 parts: sixteen warps share its dims
     (32, synth.DT_BF16, [2100]),
