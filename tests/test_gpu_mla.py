@@ -798,6 +798,9 @@ def test_step_layers_in_groups_of_layers(torch, H, dt, L, lens):
     (32, synth.DT_BF16, [(125, 7)]),                                # 7 rows in groups of 4 and 3
     (16, synth.DT_F16, [(10, 1)] * 40 + [(300, 40)]),               # many single rows beside a long run
     (100, synth.DT_BF16, [(130, 2), (64, 1)]),                      # no grouping; heads between 64 and 128
+    (16, synth.DT_BF16, [(62, 5), (500, 1), (1000, 2)]),            # 80 head rows, 48 per block of the pair, beside groups of 16 and 32
+    (16, synth.DT_F16, [(300, 6), (0, 1)]),                         # 96 beside 16: the second block's queries reach past the last row
+    (16, synth.DT_F16, [(40, 2), (700, 3), (129, 1)]),              # 48 columns of the transposed kernel, groups of 32, 48 and 16
 ])
 def test_rows_of_one_sequence_share_a_stream(torch, oracle, H, dt, spec):
     """Several new tokens of a sequence in one step are attended over one stream of its pages; every row against the CPU
