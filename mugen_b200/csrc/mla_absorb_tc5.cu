@@ -53,9 +53,10 @@ struct AbsorbArgs {
     const float* cos_sin;               // not null: rotate the last 64 dims of every head with the row's position
     const uint32_t *q_pos, *att_row;
     uint32_t cs_rows, app_layers;
-    // The kernel just ahead uploads this launch's metadata.  Nothing of it is read, and no kernel behind is let start, before the wait; W
-    // does not depend on it (16 heads x 27 layers, one sequence: 43.7 -> 40.6 us a step against a launch that starts when the upload
-    // is over; 128 heads x 8 layers, one sequence 80.3 -> 75.6).
+    // The kernel just ahead uploads this launch's metadata, that of a group of layers (att_row is null).  Nothing of it is read, and no
+    // kernel behind is let start, before the wait: the kernels behind read metadata ahead of theirs.  W does not depend on it (16 heads x
+    // 27 layers, one sequence: 43.7 -> 40.6 us a step against a launch that starts when the upload is over; 128 heads x 8 layers, one
+    // sequence 80.3 -> 75.6).
     uint32_t behind_upload;
 };
 
@@ -71,7 +72,7 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
     if (!a.behind_upload) grid_launch_dependents();
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     // Apart from kv_a the append touches nothing that an earlier kernel of the stream still reads or writes: constant
-    // tables, the step metadata (uploaded before the step's first kernel), and slots of this layer's pool, last read by
+    // tables, the step metadata (in place when this kernel starts, or behind_upload), and slots of this layer's pool, last read by
     // this layer's attention in the PREVIOUS step.  Where the host knows that kv_a was complete before the kernel ahead of
     // this one started (the later layers of a multi-layer call, whose kv_a the caller handed over with the first layer's),
     // the append works first and waits last; the wait then only keeps "this kernel completes after its predecessors", which
@@ -244,7 +245,6 @@ absorb_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const T* __restrict
             // wait on, W_UK was there after 2 (16 sequences x 5 rows to verify, with the epilogue's wider stores 324.6 -> 320.2 us; 32
             // sequences through three blocks of 128 heads 375 -> 372).  L2 is the point of coherence, so asking ahead of the wait is safe.  (Not with one tile of up to
             // 16 rows, which the kernel before may just be writing: 27 blocks of 4 sequences 757 -> 761 us.)
-            if (a.behind_upload && a.att_row) grid_dependency_wait();
             if constexpr (NT > 16) {
                 for (uint32_t u = u0; u < u1; u++) {
                     const Unit y = unit_of(u);

@@ -31,12 +31,14 @@ enum : uint32_t {
 // first access to memory that any earlier kernel of the stream reads or writes (the wait returns
 // once the previous grid has completed and flushed; completion is transitive because every kernel
 // of the chain waits before it completes).  grid_launch_dependents() lets the next kernel's blocks
-// start as soon as this kernel's blocks have all begun.  Both are no-ops in a plain launch.
+// start as soon as this kernel's blocks have all called it.  Both are no-ops in a plain launch.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
-// The first kernel behind an upload of step metadata is launched plain: it starts when the upload is done and flushed, and so does
-// every kernel behind it, all of which read the metadata ahead of their wait.
+// Step metadata is read ahead of the wait by most kernels, so none of those may start before the upload is done and flushed.  The first
+// kernel behind an upload sees to that, in one of two ways: it is launched plain, and so starts when the upload is over; or it
+// reads no metadata ahead of its wait and calls grid_launch_dependents() only behind it (AbsorbArgs::behind_upload).  Either
+// way every kernel further on starts with the metadata in place.
 struct LaunchStream {
     cudaStream_t st;
     bool plain;

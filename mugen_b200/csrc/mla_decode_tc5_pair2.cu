@@ -162,7 +162,7 @@ decode_tc5_pair128_kernel(const __grid_constant__ CUtensorMap map_sub, const __g
     asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-    // The step's metadata was complete before the step's first kernel started (that one is launched plain), so it may be
+    // The step's metadata is in place when this kernel starts (the rule stands in mla_common.cuh), so it may be
     // read ahead of the wait: the dependent loads that describe the first segment (descriptor -> page ids) then overlap
     // the previous kernel's tail instead of delaying the first TMA.
     SegInfo seg0{};

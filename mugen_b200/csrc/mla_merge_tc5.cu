@@ -269,7 +269,7 @@ merge_outproj_tc5_kernel(const __grid_constant__ CUtensorMap map_w, T* __restric
         // ---- reduction of the partial states into the operand tiles
         const uint32_t rw = warp - FIRST_RED;
         // a row's part p: a segment of the plan (its RowParts say which, and where in the segment's records the row is), or
-        // shard p of a KV-range-sharded sequence.  The plan was uploaded before the step's first kernel.
+        // shard p of a KV-range-sharded sequence.  The plan is in place when this kernel starts (mla_common.cuh).
         auto row_parts = [&](uint32_t li, uint32_t r) -> RowParts {
             if (!a.parts) return RowParts{0, a.n_parts, r * a.H, 0};
             const uint4 v = __ldg(reinterpret_cast<const uint4*>(a.parts + size_t(li) * a.rows + r));

@@ -102,7 +102,7 @@ prefill_tc5_kernel(const T* __restrict__ q, const __grid_constant__ CUtensorMap 
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + M_ABORT);
 
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-    // the list is sorted, tiles that see the most keys first; the step's metadata was uploaded before its first kernel
+    // the list is sorted, tiles that see the most keys first; the step's metadata is in place when this kernel starts (mla_common.cuh)
     PrefillTile a;
     {
         const uint4* p = reinterpret_cast<const uint4*>(tiles + blockIdx.x);

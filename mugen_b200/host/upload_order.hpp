@@ -2,7 +2,7 @@
 //
 // The kernel that uploads lets the next launch on its stream start before it has stored anything, and the library's kernels read
 // metadata ahead of their own wait.  So the first of them behind an upload, on the upload's stream, is launched without
-// that overlap.  Uploads of one step can stand on several streams at once (mla_step_begin on one, the plan of a group of layers on
+// that overlap, or it is one that waits before it reads metadata and before it lets the next kernel start.  Uploads of one step can stand on several streams at once (mla_step_begin on one, the plan of a group of layers on
 // another), so each region of the metadata buffer remembers its own; a region that is written anew forgets the
 // upload before, which the caller has ordered ahead of this one.
 #pragma once
