@@ -14,9 +14,9 @@
 //                                A = the SAME cache sub-tiles read MN-major, B = P^T [NH][64 tok] (K-major)
 //
 // What bounds it: HBM brings a page to every SM in 1.67 us (73.7 KB x 148 at 6.54 TB/s).  The MMAs of a page take 1,450 (16 rows) to
-// 1,920 cycles (64; measured alone an MMA takes the larger of N/2 cycles and its operands' bytes / 128).  From the request of a
-// pair to the end of the PV MMAs that free its slot it is 5,000 to 7,000 cycles, about 2,300 of them the load; so the pages that fit
-// beside Q' and P set the pace where they are few (2.75 pages with 16 rows, 2.5, 2.25, 2 with 64).  A page does not sit in one stage
+// 1,920 cycles (64; measured alone an MMA takes the larger of N/2 cycles and its operands' bytes / 128, with 16 columns 3 more).  From the
+// request of a pair to the end of the PV MMAs that free its slot it is 5,000 to 7,000 cycles, about 2,300 of them the load; so the pages
+// that fit beside Q' and P set the pace where they are few (2.75 pages with 16 rows, 2.5, 2.25, 2 with 64).  A page does not sit in one stage
 // buffer: whole-page stages leave one load in flight while the other page is consumed.  With pair slots a score MMA starts as soon as
 // its pair has landed and a slot is free as soon as the PV MMAs of its chunk are done.
 // 8 layers of 32 sequences x 8191 tokens, bf16, absorb and merge included: 16 heads 410 -> 382 us (0.97 of the HBM rate), 32 heads 567 ->
@@ -154,8 +154,8 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid_con
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     // The first pages of the block's first segment towards L2 while the absorb launch ends: L2 is the point of coherence, so this is
     // safe even for the page that the append is still writing.  8 layers of 64 heads x 16 sequences, one launch series each: 375 ->
-    // 365 us.  The first segment's descriptor is read here too, not behind the wait (the step's metadata was uploaded ahead of its
-    // first kernel).
+    // 365 us.  The first segment's descriptor is read here too, not behind the wait (the step's metadata is in place when this kernel
+    // starts: the rule stands in mla_common.cuh).
     SegInfo seg0{};
     if (seg_begin < seg_end) seg0 = load_seg(m, seg_begin);
     auto seg_info = [&](uint32_t seg) -> SegInfo { return seg == seg_begin ? seg0 : load_seg(m, seg); };
@@ -167,8 +167,7 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid_con
             if (page < n_pages) bulk_prefetch_l2(page_at(s, page), PAGE_BYTES);
         }
     }
-    // queries, new cache rows and the state records belong to earlier kernels of the stream (the step's metadata does not:
-    // it was uploaded before the first of them started)
+    // queries, new cache rows and the state records belong to earlier kernels of the stream, which may still run
     grid_dependency_wait();
 
     if (warp == 0) {
@@ -370,8 +369,8 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid_con
             }
             return top > over_by;
         };
-        // A row that has seen no token yet (a segment that only later rows of its group reach) has p = 0 against a reference of 0; its
-        // thread takes the slow path on every page, so that a first score, wherever it comes, becomes the reference.
+        // A row without a maximum (one that sees no token of the segment, or only scores of -infinity so far) has p = 0 against a reference of
+        // 0.  Its thread takes the slow path on every page with a score above -infinity, so that the row's first one becomes its reference.
         auto set_ref = [&](int v, float mt) {
             const bool empty = mt == -INFINITY;
             m_ref[v] = empty ? 0.0f : mt;
