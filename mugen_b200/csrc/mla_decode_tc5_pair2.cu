@@ -24,8 +24,9 @@
 // rounds of four sub-tiles and the softmax read four partial score tiles, and the period was 3,530: a K load takes 2,200 cycles and
 // nothing waited for it but the next tile.  Long lists run into the power cap (SM clock 1.2 to 1.5 GHz) and follow energy
 // instead: with a quarter of the score MMAs / of the value MMAs / without the V loads / the exponentials 4 layers of 64 x 16383 take
-// 1,144 / 1,165 / 1,229 / 1,276 us instead of 1,305.  Before / now: 4 layers of 64 x 16383 tokens 1,317 / 1,272 us, eight
-// launches of 8 x 16383 tokens 492 / 468, one sequence of 131,072 tokens 243 / 231 (4 %, 1.5 % and 2 % of it because no array is
+// 1,144 / 1,165 / 1,229 / 1,276 us instead of 1,305.  Before / now: the kernel alone at full clocks, one layer of 64 x 16384 tokens, 262 /
+// 241 us; under the cap 4 layers of 64 x 16383 1,332 to 1,374 / 1,281 to 1,305 on three GPUs, where runs of one side differ by 1 to 5 %; eight
+// launches of 8 x 16383 tokens 492 / 468, one sequence of 131,072 tokens 243 / 231 (1.5 % and 2 % of it because no array is
 // indexed by the tile's parity and no wait ends with a vote: they sat on the chain from scores to P).
 // Not better: K 6 pairs deep with 2 V buffers (period 5,040) or 5 with 3 (3,710), where V, 1,400 cycles from L2, holds P up; the
 // other block's V loaded over K pairs that have been read, two tiles in flight (4,010).
