@@ -315,6 +315,8 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid_con
         const uint32_t tok_a = 16 * q4 + tr;
         // where this lane's row of a stored 8 x 8 block lies: blocks come as (k, tokens 0-7), (k, 8-15), (k+1, 0-7), (k+1, 8-15)
         const uint32_t p_row = sP + (grp * NW + 8 * (lane >> 4) + (lane & 7)) * 128 + (((2 * q4 + ((lane >> 3) & 1)) ^ (lane & 7)) << 4);
+        // References are scores as they are, unscaled, so that the difference to the largest one is exactly 0 however large they are: with the scale
+        // in an FMA against a scaled reference it was the rounding of that, beyond 2^32 an exponential of infinity or 0 (and no faster).
         float m_ref[NV], psum[NV];                            // m_ref: 0 for the rows of `none`, whose reference is -infinity
         uint32_t none = 0, t = 0, nseg = 0, sb = 0, sph = 0;
         float over_by = RESCALE_THRESHOLD;
@@ -334,14 +336,14 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid_con
             return r != 0;
         };
         uint32_t sv[NW / 2];                                  // scores, unscaled: sv[4k + 2e' + e]: head 8k + 2qd + e, token tok_a + 8e'
-        auto publish_max = [&] {                              // maxima of this warp's 16 tokens, scaled
+        auto publish_max = [&] {                              // maxima of this warp's 16 tokens
 #pragma unroll
             for (int v = 0; v < NV; v++) {
                 float x = fmaxf(__uint_as_float(sv[4 * (v >> 1) + (v & 1)]), __uint_as_float(sv[4 * (v >> 1) + 2 + (v & 1)]));
                 x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 4));
                 x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 8));
                 x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 16));
-                if (tr == 0) hmax_s[q4 * NH + head_of(v)] = x * scale_log2;
+                if (tr == 0) hmax_s[q4 * NH + head_of(v)] = x;
             }
         };
         auto tile_max = [&](int v) {
@@ -358,7 +360,7 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid_con
 #pragma unroll
                 for (int e = 0; e < 2; e++) {
                     const float me = m_ref[2 * k + e];
-                    const float xa = fmaf(__uint_as_float(sv[4 * k + e]), scale_log2, -me), xb = fmaf(__uint_as_float(sv[4 * k + 2 + e]), scale_log2, -me);
+                    const float xa = (__uint_as_float(sv[4 * k + e]) - me) * scale_log2, xb = (__uint_as_float(sv[4 * k + 2 + e]) - me) * scale_log2;
                     top = fmaxf(top, fmaxf(xa, xb));
                     p[e] = fast_ex2(xa);
                     p[2 + e] = fast_ex2(xb);
@@ -447,7 +449,8 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid_con
                         for (int v = 0; v < NV; v++) {
                             const float mt = tile_max(v), mr = (none >> v) & 1 ? -INFINITY : m_ref[v];
                             float alpha = 1.0f;
-                            if (mt > mr + RESCALE_THRESHOLD) { alpha = fast_ex2(mr - mt); set_ref(v, mt); }
+                            const float up = (mt - mr) * scale_log2;
+                            if (up > RESCALE_THRESHOLD) { alpha = fast_ex2(-up); set_ref(v, mt); }
                             psum[v] *= alpha;
                             if (q4 == 0 && tr == 0) alpha_s[head_of(v)] = alpha;
                         }
@@ -519,7 +522,7 @@ decode_tc5_kernel(const __grid_constant__ CUtensorMap map_pair, const __grid_con
                     const uint32_t h = head_of(v);
                     if (h0 + h < s.heads) {
                         float* rc = recs + (rec + h) * kPart;
-                        rc[0] = (none >> v) & 1 ? -INFINITY : m_ref[v];
+                        rc[0] = (none >> v) & 1 ? -INFINITY : m_ref[v] * scale_log2;
                         rc[1] = (hmax_s[h] + hmax_s[NH + h]) + (hmax_s[2 * NH + h] + hmax_s[3 * NH + h]);
                     }
                 }

@@ -859,6 +859,43 @@ def test_attention_at_the_edges_of_its_widths(torch, oracle, H, dt):
     ctx.close()
 
 
+@pytest.mark.parametrize("H", [5, 16, 32, 48, 64])
+def test_scores_far_beyond_the_precision_of_their_exponents(torch, H):
+    """Finite scores of 2^36 and more, where one step of a float is thousands: the largest score's distance to the reference is 0 all
+    the same, and the softmax picks its token.  All rows of a sequence lie along one direction u, one of them is u, one -u,
+    the others at most half as long: the output is W_UV u, with the sign of the head's score."""
+    from mugen_b200.mla import MlaContext
+    lens = [1, 64, 65, 130, 1100]
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(H)
+    rn = lambda *shape, s=1.0: (torch.randn(shape, device="cuda", generator=gen) * s).bfloat16()
+    bits = lambda t: t.view(torch.int16).cpu().numpy().view(np.uint16)
+    ctx = MlaContext(n_layers=1, n_heads=H, dtype=synth.DT_BF16, n_pages=64, max_seqs=len(lens), max_seq_len=2048, max_rows=len(lens), **YARN)
+    w_uk, w_uv = rn(H * 128, 512, s=0.02), rn(H * 128, 512, s=0.02)
+    ctx.set_layer_weights(0, bits(w_uk), bits(w_uv), synth.W_BF16, np.full(512, 0x3F80, np.uint16))
+    u, q = rn(576), rn(len(lens), H, 192, s=1e13)
+    seqs = []
+    for n in lens:
+        a = (torch.rand(n, device="cuda", generator=gen) - 0.5).double()
+        a[-1], a[n // 3] = (-1.0, 1.0) if n > 1 else (1.0, 1.0)
+        s = ctx.seq_create()
+        ctx.write_rows(0, s, 0, (a[:, None] * u.double()).bfloat16().view(torch.int16))
+        ctx.advance_seq_len(s, n)
+        seqs.append(s)
+    out = torch.zeros((len(lens), H, 128), dtype=torch.int16, device="cuda")
+    ctx.attend_rows(0, seqs, lens, q.view(torch.int16), out)
+    got = out.view(torch.bfloat16).double()
+    assert ctx.status() == 0
+    score = torch.einsum("rhi,hid,d->rh", q[..., :128].double(), w_uk.double().view(H, 128, 512), u[:512].double()) + q[..., 128:].double() @ u[512:].double()
+    sure = score.abs() > 0.02 * score.square().mean().sqrt()               # the absorbed queries' rounding cannot turn the sign
+    assert sure.double().mean() > 0.9 and score.abs()[sure].min() > 2.0 ** 36 / (1.4427 / 192 ** 0.5)
+    sign = torch.where(torch.tensor(lens, device="cuda")[:, None] > 1, score.sign(), torch.ones_like(score))
+    want = sign[..., None] * (w_uv.double().view(H, 128, 512) @ u[:512].double())
+    err = (got - want).norm(dim=-1) / want.norm(dim=-1)
+    assert err[sure].max().item() <= 2.0 ** -8                             # the outputs' rounding to 8 bits
+    ctx.close()
+
+
 @pytest.mark.parametrize("H,dt", [(128, synth.DT_F16), (96, synth.DT_BF16)])
 def test_references_move_on_the_last_tile_of_every_segment(torch, oracle, H, dt):
     """Segments of two and three tiles of the SM-pair kernel, several per pair, whose scores rise by more than 2^8 from tile to tile: the request to
