@@ -27,6 +27,7 @@ from __future__ import annotations
 
 import argparse
 import json
+import math
 import os
 import subprocess
 import sys
@@ -46,12 +47,25 @@ METRIC, UNIT = "mla_decode_tokens_per_s", "tokens/s"
 # value below (otherwise `traffic` is null until the capture is repeated).
 NCU_TRAFFIC = {"kernel": "tcgen05-pair128", "source": "mugen_b200/csrc/mla_decode_tc5_pair2.cu",
                "source_sha256_16": "b387cc17b8ebb270", "bytes_per_layer": 1.2650e9}
-# The attention kernel is timed live by CUDA events inside the library on every 7th launch of the timed region
-# (61 layers are 13 launches of five layers each and a last of one; 7 is coprime to 13, so every group gets sampled over
-# the steps): an event between two kernels stops
+# The attention kernel is timed live by CUDA events inside the library, not on every launch: an event between two kernels stops
 # the next one from becoming resident while the previous drains, and bracketing every launch would slow the
 # step that `value` reports by about 3 %.
-KERNEL_EVENT_STRIDE = 7
+MIN_EVENT_STRIDE = 7
+
+
+def event_stride(launches_per_step: int) -> int:
+    """Every so many launches one is timed: coprime to a step's launches, so that over the steps each group of layers is."""
+    stride = MIN_EVENT_STRIDE
+    while math.gcd(stride, launches_per_step) != 1:
+        stride += 1
+    return stride
+
+
+def timed_layers(layers: int, launches_per_step: int, stride: int, timed: int) -> int:
+    """Layers in the timed launches: a step's launches hold equal groups of them, the last one what is left."""
+    group = -(-layers // launches_per_step)
+    last = layers - group * (launches_per_step - 1)
+    return sum(last if k * stride % launches_per_step == launches_per_step - 1 else group for k in range(timed))
 
 
 def parse_args():
@@ -325,12 +339,16 @@ def run_ours(a):
         ctx.step_end()
 
     clocks = ClockSampler(local) if rank == 0 else None
+    launches0 = ctx.launch_count()
     for _ in range(a.warmup):
         one_step()
     torch.cuda.synchronize()
     lens_sum = 0
+    # step_layers launches groups of layers, three kernels per group
+    groups = max(1, (ctx.launch_count() - launches0) // (3 * max(1, a.warmup)))
     launches0 = ctx.launch_count()
-    ctx.profile_enable(KERNEL_EVENT_STRIDE if L >= KERNEL_EVENT_STRIDE else 1)
+    stride = event_stride(groups) if L >= MIN_EVENT_STRIDE else 1
+    ctx.profile_enable(stride)
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     barrier(); torch.cuda.synchronize()
     if clocks:
@@ -344,7 +362,7 @@ def run_ours(a):
     ms = ev0.elapsed_time(ev1)
     ctx.profile_enable(False)
     n_attn, attn_ms = ctx.profile_read()
-    launches = own_launches = ctx.launch_count() - launches0
+    launches = ctx.launch_count() - launches0
     clk = clocks.stop() if clocks else None
     assert ctx.status() == 0, "a kernel flagged a fault during the timed region"
 
@@ -360,8 +378,8 @@ def run_ours(a):
 
     # ---- roofline of the dominant kernel (split-KV attention), this rank's launches
     peak, peak_src = measured_peak_gbs()
-    # step_layers launches groups of layers, three kernels per group: a timed launch holds so many layers in the mean
-    layers_per_launch = L * a.steps / max(1, own_launches / 3)
+    # a timed launch holds so many layers in the mean
+    layers_per_launch = timed_layers(L, groups, stride, n_attn) / max(1, n_attn)
     rows_per_launch = lens_sum / max(1, a.steps) * layers_per_launch  # cache rows streamed per launch
     algo_bytes = rows_per_launch * 576 * 2 + layers_per_launch * B * H * 576 * 2 + (rows_per_launch / 64) * 4
     per_launch_s = (attn_ms * 1e-3) / max(1, n_attn)
